@@ -75,7 +75,8 @@ enum GcaStatus {
  *
  *   q, out   (N, J, Hq, S, D)      addressed with *_stride = {n, j, h, s}
  *   k_cache, v_cache (N, C, L, Hkv, D) addressed with *_stride = {n, c, l, h}
- *   indices  (N, J, K) int32, contiguous; < 0 marks a padding slot (skipped)
+ *   indices  (N, J, K) int32, contiguous; < 0 marks a padding slot (skipped).  NULL with J = 1 and
+ *            C = K: slot k reads chunk k (the pre-gathered call below)
  *   weights  (N, J, K) float32, contiguous (shared by all heads)
  *   lse      (N*J, Hq, K, S) float32 base-2 log-sum-exp per slot, or NULL
  *
@@ -83,7 +84,7 @@ enum GcaStatus {
  *   K_k = k_cache[n, indices[n,j,k], :, h / (Hq/Hkv), :].
  *
  * The pre-gathered call of the reference (k of shape (Z, Hkv, K, L, D)) is the same
- * kernel with N=Z, J=1, C=K, indices = 0..K-1 and the matching strides.
+ * kernel with N=Z, J=1, C=K, indices = 0..K-1 (or NULL) and the matching strides.
  * `off_by_one` > 0 adds a virtual zero logit of that weight to every softmax; 0 gives
  * the behaviour of the reference kernels (whose `sm_n` argument has no effect).
  */
@@ -405,6 +406,18 @@ typedef struct LinearArgs {
 int gca_row_rms(const RowRmsArgs* args, void* stream);
 int gca_linear(const LinearArgs* args, void* stream);
 
+/* gca_linear over `batches` blocks of one.M rows each, the blocks *_batch_stride elements apart (x, out,
+ * residual; row_scale by values): the rows of several sequences when something else -- a first chunk that
+ * retrieves nothing -- lies between them.  lead_rows > 0: the lead_rows rows of `out` in FRONT of every block
+ * (out - lead_rows * out_stride ...) are written as the same rows of `residual`, or as zeros without one. */
+typedef struct LinearBatchedArgs {
+  LinearArgs one;
+  int64_t x_batch_stride, out_batch_stride, residual_batch_stride, scale_batch_stride;
+  int32_t batches, lead_rows;
+} LinearBatchedArgs;
+
+int gca_linear_batched(const LinearBatchedArgs* args, void* stream);
+
 /* out[m, c] = silu(gate_up[m, c]) * gate_up[m, I + c] for c < I: the activation between ONE gate|up
  * projection (weights stacked) and down_proj -- the reference's fused SwiGLU, model/llama.py:290-300.
  * bf16; gate_up (M, 2 I) and out (M, I) by row strides in elements (multiples of 8); I % 8 == 0. */
@@ -511,7 +524,8 @@ int gca_vmem_free(void* va, size_t bytes);
 const char* gca_strerror(int code);
 int gca_abi_version(void);
 /* sizeof() of an argument block as the library was compiled (0 GcaFwdArgs, 1 GcaBwdArgs,
- * 2 LmkTopkArgs, 3 LmkMergeArgs, 4 CacheAppendArgs, 5 LmkExchangeArgs, 6 KvProjectArgs, 7 RowRmsArgs, 8 LinearArgs, 9 WindowDecodeArgs, 10 LinearCeArgs, 11 WindowAppendArgs, 12 WindowRingDecodeArgs): lets a foreign-language binding verify
+ * 2 LmkTopkArgs, 3 LmkMergeArgs, 4 CacheAppendArgs, 5 LmkExchangeArgs, 6 KvProjectArgs, 7 RowRmsArgs, 8 LinearArgs, 9 WindowDecodeArgs, 10 LinearCeArgs, 11 WindowAppendArgs, 12 WindowRingDecodeArgs,
+ * 13 LinearBatchedArgs): lets a foreign-language binding verify
  * its struct layout before the first call. */
 size_t gca_sizeof(int which);
 

@@ -1,4 +1,5 @@
-"""ctypes binding of libgca_b200.so (the C ABI declared in include/gca_b200.h).
+"""ctypes binding of libgca_b200.so (the C ABI declared in include/gca_b200.h) and the loader of the compiled
+host path in front of it (``host()``).
 
 The library is built in-tree by ``long_context_modeling_b200.build``.  There is no
 fallback of any kind: if the shared object is missing, or a call is rejected, an
@@ -117,6 +118,11 @@ class LinearArgs(C.Structure):
     ]
 
 
+class LinearBatchedArgs(C.Structure):
+    _fields_ = [("one", LinearArgs), ("x_batch_stride", C.c_int64), ("out_batch_stride", C.c_int64), ("residual_batch_stride", C.c_int64),
+                ("scale_batch_stride", C.c_int64), ("batches", C.c_int32), ("lead_rows", C.c_int32)]
+
+
 class WindowDecodeArgs(C.Structure):
     _fields_ = [
         ("q", C.c_void_p), ("k", C.c_void_p), ("v", C.c_void_p), ("alibi_slopes", C.c_void_p), ("out", C.c_void_p),
@@ -157,6 +163,7 @@ EXPORTS = {
     "gca_kv_project_append": (C.c_int, [C.POINTER(KvProjectArgs), C.c_void_p]),
     "gca_row_rms": (C.c_int, [C.POINTER(RowRmsArgs), C.c_void_p]),
     "gca_linear": (C.c_int, [C.POINTER(LinearArgs), C.c_void_p]),
+    "gca_linear_batched": (C.c_int, [C.POINTER(LinearBatchedArgs), C.c_void_p]),
     "gca_silu_mul": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int64, C.c_int32, C.c_int64, C.c_int64, C.c_void_p]),
     "gca_window_decode": (C.c_int, [C.POINTER(WindowDecodeArgs), C.c_void_p]),
     "gca_window_shift_append": (C.c_int, [C.POINTER(WindowAppendArgs), C.c_void_p]),
@@ -200,7 +207,7 @@ def lib() -> C.CDLL:
             raise RuntimeError("libgca_b200.so has an unexpected ABI version")
         for which, struct in enumerate((GcaFwdArgs, GcaBwdArgs, LmkTopkArgs, LmkMergeArgs, CacheAppendArgs, LmkExchangeArgs,
                                        KvProjectArgs, RowRmsArgs, LinearArgs, WindowDecodeArgs, LinearCeArgs, WindowAppendArgs,
-                                       WindowRingDecodeArgs)):
+                                       WindowRingDecodeArgs, LinearBatchedArgs)):
             if handle.gca_sizeof(which) != C.sizeof(struct):
                 raise RuntimeError(f"struct layout mismatch for {struct.__name__}: "
                                    f"library {handle.gca_sizeof(which)} vs binding {C.sizeof(struct)}")
@@ -212,7 +219,34 @@ class GcaError(RuntimeError):
     pass
 
 
-_nvtx = False
+_host = None
+
+
+def host():
+    """The compiled host path (csrc/host_binding.cpp), bound to the entry points of the loaded library."""
+    global _host
+    if _host is None:
+        try:
+            from . import _host as module
+        except ImportError as e:
+            raise RuntimeError("the compiled host path is missing: build it with `python -m long_context_modeling_b200.build` "
+                               "(there is no fallback path)") from e
+        handle = lib()
+        module.bind({name: C.cast(getattr(handle, name), C.c_void_p).value for name in EXPORTS}, GcaError)
+        module.set_switches(_nvtx, _check)
+        _host = module
+    return _host
+
+
+_nvtx = _check = False
+
+
+def set_check(enabled: bool) -> None:
+    """Status check after every call of the compiled host path (``gca.set_status_checks``)."""
+    global _check
+    _check = bool(enabled)
+    if _host is not None:
+        _host.set_switches(_nvtx, _check)
 
 
 def set_nvtx(enabled: bool) -> None:
@@ -220,6 +254,8 @@ def set_nvtx(enabled: bool) -> None:
     a host program; off by default)."""
     global _nvtx
     _nvtx = bool(enabled)
+    if _host is not None:
+        _host.set_switches(_nvtx, _check)
 
 
 def call(name: str, *args) -> None:

@@ -235,17 +235,7 @@ class ChunkKVManager:
         self._reserve(self._len + count, x, x[:, :, -1])
         if self._k.dtype != torch.bfloat16 or self._lmk.dtype != torch.bfloat16:
             raise ValueError("append_projected writes a bf16 cache")
-        a = _lib.KvProjectArgs()
-        a.x, a.wk, a.wv = x.data_ptr(), k_weight.contiguous().data_ptr(), v_weight.contiguous().data_ptr()
-        a.k_cache, a.v_cache, a.lmk_cache = self._k.data_ptr(), self._v.data_ptr(), self._lmk.data_ptr()
-        from .gca import _status
-        a.status = _status(x.device).data_ptr()
-        a.cache_batch_stride, a.lmk_cache_batch_stride = self._k.stride(0), self._lmk.stride(0)
-        a.N, a.count, a.pos, a.D = n, count, self._len, dim
-        a.capacity, a.lmk_capacity = self._capacity(), self._lmk.shape[1]
-        a.zero_landmark = 1 if self._zero_landmark else 0
-        with torch.cuda.device(x.device):
-            _lib.call("gca_kv_project_append", C.byref(a), torch.cuda.current_stream().cuda_stream)
+        _lib.host().kv_project_append(x, k_weight, v_weight, self._k, self._v, self._lmk, self._len, self._capacity(), self._zero_landmark)
         self._len += count
 
     # ------------------------------------------------------------------ retrieval state

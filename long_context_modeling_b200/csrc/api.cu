@@ -15,7 +15,7 @@ int launch_cache_append(const CacheAppendArgs& a, cudaStream_t stream);
 int launch_kv_project_append(const KvProjectArgs& a, int sms, cudaStream_t stream);
 int launch_row_rms(const RowRmsArgs& a, cudaStream_t stream);
 int launch_silu_mul(const void* gu, void* out, long long M, int I, long long in_stride, long long out_stride, cudaStream_t stream);
-int launch_linear(const LinearArgs& a, int sms, cudaStream_t stream);
+int launch_linear(const LinearBatchedArgs& a, int sms, cudaStream_t stream);
 int launch_window_decode(const WindowDecodeArgs& a, cudaStream_t stream);
 int launch_window_ring_decode(const WindowRingDecodeArgs& a, cudaStream_t stream);
 int launch_linear_ce(const LinearCeArgs& a, int sms, cudaStream_t stream);
@@ -68,7 +68,8 @@ int check_strides(const int64_t s[4], int esize, const int32_t dims[4]) {
 
 int check_common(const void* q, const void* k, const void* v, const int32_t* idx, const float* w, int dtype, int N,
                  int J, int Hq, int Hkv, int S, int L, int D, int K, int C) {
-  if (!q || !k || !v || !idx || !w) return GCA_ERR_NULL;
+  if (!q || !k || !v || !w) return GCA_ERR_NULL;
+  if (!idx && (J != 1 || C != K)) return GCA_ERR_NULL;        // no index array: the pre-gathered call only
   if (esize_of(dtype) == 0) return GCA_ERR_DTYPE;
   if (N < 0 || J < 0 || Hq <= 0 || Hkv <= 0 || Hq % Hkv != 0) return GCA_ERR_SHAPE;
   if (L != 64 || D != 64 || S < 1 || S > 64 || K < 1 || K > 32 || C < 1) return GCA_ERR_SHAPE;
@@ -124,6 +125,7 @@ size_t gca_sizeof(int which) {
     case 10: return sizeof(LinearCeArgs);
     case 11: return sizeof(WindowAppendArgs);
     case 12: return sizeof(WindowRingDecodeArgs);
+    case 13: return sizeof(LinearBatchedArgs);
     default: return 0;
   }
 }
@@ -426,18 +428,29 @@ int gca_window_ring_decode(const WindowRingDecodeArgs* a, void* stream) {
   return gca::launch_window_ring_decode(*a, (cudaStream_t)stream);
 }
 
-int gca_linear(const LinearArgs* a, void* stream) {
-  if (!a) return GCA_ERR_NULL;
+int gca_linear_batched(const LinearBatchedArgs* b, void* stream) {
+  if (!b) return GCA_ERR_NULL;
+  const LinearArgs* a = &b->one;
   if (!a->x || !a->w || !a->out) return GCA_ERR_NULL;
   if (a->M < 0 || a->N < 16 || a->N % 16 != 0 || a->K < 64 || a->K % 64 != 0) return GCA_ERR_SHAPE;
+  if (b->batches < 0 || b->lead_rows < 0) return GCA_ERR_SHAPE;
   if (a->x_stride % 8 || a->w_stride % 8 || a->out_stride % 8 || (a->residual && a->residual_stride % 8) ||
       a->x_stride < a->K || a->w_stride < a->K || a->out_stride < a->N || (a->residual && a->residual_stride < a->N))
     return GCA_ERR_STRIDE;
+  if (b->batches > 1 && (b->x_batch_stride % 8 || b->out_batch_stride % 8 || (a->residual && b->residual_batch_stride % 8))) return GCA_ERR_STRIDE;
   if (!aligned16(a->x) || !aligned16(a->w) || !aligned16(a->out) || (a->residual && !aligned16(a->residual))) return GCA_ERR_ALIGN;
-  if (a->M == 0) return 0;
+  if (a->M == 0 || b->batches == 0) return 0;
   gca::DeviceScope scope(a->out);
   if (scope.rc) return scope.rc;
-  return gca::launch_linear(*a, gca::sm_count(scope.dev), (cudaStream_t)stream);
+  return gca::launch_linear(*b, gca::sm_count(scope.dev), (cudaStream_t)stream);
+}
+
+int gca_linear(const LinearArgs* a, void* stream) {
+  if (!a) return GCA_ERR_NULL;
+  LinearBatchedArgs b = {};
+  b.one = *a;
+  b.batches = 1;
+  return gca_linear_batched(&b, stream);
 }
 
 }  // extern "C"

@@ -171,7 +171,7 @@ __device__ __forceinline__ QInfo q_info(const BwdQParams& p, int hp) {
 }
 __device__ __forceinline__ int q_load_row(const BwdQParams& p, int u, int zj, int lane) {
   if (u >= p.units || lane >= p.K) return -1;
-  return p.indices[(long long)zj * p.K + lane];
+  return slot_chunk(p.indices, zj, p.K, lane);
 }
 __device__ __forceinline__ unsigned q_valid(const BwdQParams& p, int idx) {
   return __ballot_sync(0xffffffffu, idx >= 0 && idx < p.C);

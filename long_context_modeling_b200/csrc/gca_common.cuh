@@ -29,6 +29,11 @@ template <> __device__ __forceinline__ void st_f<__nv_bfloat16>(__nv_bfloat16* p
   *p = __float2bfloat16_rn(v);
 }
 
+// The chunk that slot k of query chunk zj reads; no index array = the pre-gathered call, slot k reads chunk k.
+__device__ __forceinline__ int slot_chunk(const int32_t* __restrict__ indices, long long zj, int K, int k) {
+  return indices ? indices[zj * K + k] : k;
+}
+
 // Problem geometry shared by forward and backward kernels (passed by value).
 struct Geom {
   int N, J, Hq, Hkv, S, L, D, K, C, G;

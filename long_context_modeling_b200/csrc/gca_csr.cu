@@ -173,6 +173,17 @@ csr_small_kernel(const int32_t* __restrict__ indices, unsigned long long* __rest
   }
 }
 
+// The pre-gathered call: chunk c of row block n is read by its slot c and nothing else.
+__global__ void csr_identity_kernel(unsigned long long* __restrict__ keys_out, int* __restrict__ offsets, int4* __restrict__ unit_tab, int NC,
+                                    int C) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i > NC) return;
+  offsets[i] = i;
+  if (i == NC) return;
+  keys_out[i] = ((unsigned long long)i << 32) | (unsigned)(i % C);
+  unit_tab[i] = make_int4(i, i + 1, i, 0);
+}
+
 size_t small_smem_bytes(int C) { return (size_t)(32 * C + (C + 1) + C + SMALL_C + 33) * 4; }
 
 bool small_path(int N, int JK, int C) {
@@ -231,7 +242,10 @@ int build_csr(const int32_t* indices, int N, int J, int K, int C, void* workspac
   const long long cmax = (long long)J * K;
   const int cbits = bits_for(cmax), nbits = bits_for(N);
   if (cbits + nbits > 32) return GCA_ERR_TOO_LARGE;
-  if (launch && NC > 0 && total > 0 && !by_sort && small_path(N, J * K, C)) {
+  if (launch && !indices && NC > 0) {
+    csr_identity_kernel<<<(unsigned)((NC + 1 + 255) / 256), 256, 0, stream>>>(keys_out, offsets, uvals_out, (int)NC, C);
+    GCA_CUDA_CHECK(cudaGetLastError());
+  } else if (launch && NC > 0 && total > 0 && !by_sort && small_path(N, J * K, C)) {
     const size_t smem = small_smem_bytes(C);
     GCA_CUDA_CHECK(cudaFuncSetAttribute(csr_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     csr_small_kernel<<<N, SMALL_THREADS, smem, stream>>>(indices, keys_out, offsets, uvals_out, N, J * K, C);

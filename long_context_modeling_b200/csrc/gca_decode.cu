@@ -72,7 +72,7 @@ decode_kernel(const __grid_constant__ DecParams p) {
   struct Slot { int item, k, idx; };
   auto load_idx = [&](int item, int k) -> int {
     const int zj = item / g.Hkv;
-    const int v = p.indices[(long long)zj * g.K + k];
+    const int v = slot_chunk(p.indices, zj, g.K, k);
     if (v >= g.C) { if (p.status && lane == 0) atomicOr(p.status, GCA_STATUS_BAD_INDEX); return -1; }
     return v;
   };
@@ -274,7 +274,7 @@ decode_rows_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
 #pragma unroll
     for (int e = 0; e < 8; ++e) o[r][e] = 0.f;
   for (int k = warp; k < g.K; k += NWARPS) {
-    const int idx = indices[(long long)zj * g.K + k];
+    const int idx = slot_chunk(indices, zj, g.K, k);
     if (idx < 0) continue;                                       // padding slot (warp-uniform)
     if (idx >= g.C) { if (status && lane == 0) atomicOr(status, GCA_STATUS_BAD_INDEX); continue; }
     const float w = weights[(long long)zj * g.K + k];

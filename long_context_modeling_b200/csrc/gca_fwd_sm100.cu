@@ -184,7 +184,7 @@ __device__ __forceinline__ UnitInfo unit_info(const FwdTcParams& p, int hp) {
 // Lane-parallel read of one row of retrieved indices; every role prefetches the next row.
 __device__ __forceinline__ int load_index_row(const FwdTcParams& p, int u, int zj, int lane) {
   if (u >= p.units || lane >= p.K) return -1;
-  return p.indices[(long long)zj * p.K + lane];
+  return slot_chunk(p.indices, zj, p.K, lane);
 }
 __device__ __forceinline__ unsigned valid_mask(const FwdTcParams& p, int idx) {
   return __ballot_sync(0xffffffffu, idx >= 0 && idx < p.C);

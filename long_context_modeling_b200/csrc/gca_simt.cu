@@ -114,7 +114,7 @@ fwd_simt_kernel(const E* __restrict__ q, const E* __restrict__ kc, const E* __re
   const float c2 = g.sm_scale * GCA_LOG2E;
 
   for (int k = 0; k < g.K; ++k) {
-    const int idx = indices[(long long)zj * g.K + k];
+    const int idx = slot_chunk(indices, zj, g.K, k);
     const float w = weights[(long long)zj * g.K + k];
     float* lse_row = lse ? lse + (((long long)zj * g.Hq + h) * g.K + k) * g.S : nullptr;
     if (idx < 0 || idx >= g.C) {
@@ -289,7 +289,7 @@ bwd_q_simt_kernel(const E* __restrict__ q, const E* __restrict__ kc, const E* __
     for (int b = 0; b < 4; ++b) aQ[a][b] = 0.f;
 
   for (int k = 0; k < g.K; ++k) {
-    const int idx = indices[(long long)zj * g.K + k];
+    const int idx = slot_chunk(indices, zj, g.K, k);
     float* dwp = dw_part + ((long long)zj * g.Hq + h) * g.K + k;
     if (idx < 0 || idx >= g.C) {
       if (threadIdx.x == 0) *dwp = 0.f;

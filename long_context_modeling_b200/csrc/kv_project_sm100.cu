@@ -58,7 +58,11 @@ struct ProjParams {
   int zero_landmark;
   int tiles_m, tiles_n;     // tiles_n = ceil(output columns / BN)
   int nmat;                 // 2: K and V projection with append epilogue; 1: linear mode
-  // linear mode
+  // linear mode: `batches` blocks of M rows, each cut in 64-row blocks (a 128-row tile is two of them, whatever
+  // batch they belong to)
+  int batches, blocks_per_batch;
+  int lead_rows, lead_tiles;          // rows in front of every batch that get the residual alone; copy tiles for them
+  long long out_bs, res_bs, scale_bs; // elements (values) between batches
   __nv_bfloat16* out;
   const __nv_bfloat16* residual;      // or nullptr
   const float* row_scale;             // or nullptr
@@ -70,6 +74,11 @@ struct ProjParams {
   const long long* targets;           // (M) class ids; negative = ignored row
 };
 
+__device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* m, uint64_t* bar, int c0, int c1, int c2) {
+  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+               ::"r"(smem_u32(smem_dst)), "l"(m), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
+               : "memory");
+}
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m, uint64_t* bar, int c0, int c1) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
                ::"r"(smem_u32(smem_dst)), "l"(m), "r"(smem_u32(bar)), "r"(c0), "r"(c1)
@@ -121,7 +130,13 @@ kv_project_append_kernel(const __grid_constant__ ProjParams p) {
           if (!ok) break;
           uint8_t* dst = smem + ring.st * STAGE_BYTES;
           mbar_arrive_expect_tx(&bars[FULL + ring.st], STAGE_BYTES);
-          tma_load_2d(dst, &p.tm_x, &bars[FULL + ring.st], ks * BK, tm * BM);          // rows past M are zero-filled
+          if (p.blocks_per_batch) {                            // linear mode: two 64-row blocks (rows past the end are zero-filled)
+            const int b0 = (2 * tm) / p.blocks_per_batch, b1 = (2 * tm + 1) / p.blocks_per_batch;
+            tma_load_3d(dst, &p.tm_x, &bars[FULL + ring.st], ks * BK, (2 * tm - b0 * p.blocks_per_batch) * 64, b0);
+            tma_load_3d(dst + A_BYTES / 2, &p.tm_x, &bars[FULL + ring.st], ks * BK, (2 * tm + 1 - b1 * p.blocks_per_batch) * 64, b1);
+          } else {
+            tma_load_2d(dst, &p.tm_x, &bars[FULL + ring.st], ks * BK, tm * BM);        // rows past M are zero-filled
+          }
           tma_load_2d(dst + A_BYTES, tw, &bars[FULL + ring.st], ks * BK, tn * BN);
           ring.next();
           ++issued;
@@ -163,15 +178,26 @@ kv_project_append_kernel(const __grid_constant__ ProjParams p) {
     const uint32_t tlane = tmem_base + ((uint32_t)(quad * 32) << 16);
     bool ok = true;
     uint32_t tcount = 0;
-    for (int t = blockIdx.x; t < total && ok; t += gridDim.x, ++tcount) {
+    for (int t = blockIdx.x; t < total + p.lead_tiles && ok; t += gridDim.x, ++tcount) {
+      if (t >= total) {                                  // the lead rows of one batch, 256 columns: residual or zeros
+        const int b = (t - total) / p.tiles_n, c0 = (t - total - b * p.tiles_n) * BN, vecs = min(BN, p.ncols - c0) / 8;
+        __nv_bfloat16* dst = p.out + b * p.out_bs - p.lead_rows * p.out_stride + c0;
+        const __nv_bfloat16* src = p.residual + b * p.res_bs - p.lead_rows * p.res_stride + c0;
+        for (int i = (warp - 2) * 32 + lane; i < p.lead_rows * vecs; i += 128) {
+          const int r = i / vecs, v = i - r * vecs;
+          *reinterpret_cast<uint4*>(dst + r * p.out_stride + v * 8) =
+              p.residual ? *reinterpret_cast<const uint4*>(src + r * p.res_stride + v * 8) : make_uint4(0, 0, 0, 0);
+        }
+        continue;
+      }
       int which, tm, tn;
       tile_of(p, t, which, tm, tn);
       const uint32_t ab = tcount & 1;
       ok = mbar_wait_bounded(&bars[ACC_FULL + ab], (tcount >> 1) & 1, abort_flag);
       if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
       tc_fence_after();
-      const long long m = (long long)tm * BM + row_in_tile;
-      const bool live = m < p.M;
+      long long m = (long long)tm * BM + row_in_tile;
+      bool live = m < p.M;
       if (p.nmat == 1 && p.ce_part) {
         // cross-entropy mode: per row, the maximum and the sum of exponentials of this column
         // tile's logits (base 2, logits scaled by log2 e) and the target's logit if it lies here
@@ -210,9 +236,12 @@ kv_project_append_kernel(const __grid_constant__ ProjParams p) {
       }
       if (p.nmat == 1) {
         // linear mode: out = row_scale * acc + residual, 16 columns per pass
-        const float sc = (live && p.row_scale) ? p.row_scale[m] : 1.0f;
-        __nv_bfloat16* orow = p.out + m * p.out_stride + tn * BN;
-        const __nv_bfloat16* rrow = p.residual ? p.residual + m * p.res_stride + tn * BN : nullptr;
+        const int block = 2 * tm + (row_in_tile >> 6), b = block / p.blocks_per_batch;
+        m = (block - b * p.blocks_per_batch) * 64 + (row_in_tile & 63);
+        live = b < p.batches && m < p.M;
+        const float sc = (live && p.row_scale) ? p.row_scale[b * p.scale_bs + m] : 1.0f;
+        __nv_bfloat16* orow = p.out + b * p.out_bs + m * p.out_stride + tn * BN;
+        const __nv_bfloat16* rrow = p.residual ? p.residual + b * p.res_bs + m * p.res_stride + tn * BN : nullptr;
         const int cols = min(BN, p.ncols - tn * BN);
 #pragma unroll 1
         for (int c0 = 0; c0 < cols; c0 += 16) {
@@ -278,6 +307,23 @@ int make_matrix_map(CUtensorMap* map, const void* base, long long rows, long lon
   const cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
   const cuuint32_t estr[2] = {1, 1};
   CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : GCA_ERR_TMA;
+}
+
+// The same for linear mode's x: (columns, rows, batches), boxes of 64 columns x 64 rows of one batch.
+int make_rows_map(CUtensorMap* map, const void* base, long long batches, long long rows, long long cols, long long row_stride,
+                  long long batch_stride) {
+  EncodeTiledFn fn = encode_tiled_fn();
+  if (!fn) return GCA_ERR_TMA;
+  if (batches == 1) batch_stride = row_stride;            // never advanced; any legal stride does
+  if (row_stride % 8 != 0 || batch_stride % 8 != 0 || batch_stride <= 0) return GCA_ERR_STRIDE;
+  const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)batches};
+  const cuuint64_t strides[2] = {(cuuint64_t)row_stride * 2, (cuuint64_t)batch_stride * 2};
+  const cuuint32_t box[3] = {64, 64, 1};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : GCA_ERR_TMA;
@@ -380,6 +426,7 @@ int launch_linear_ce(const LinearCeArgs& a, int sms, cudaStream_t stream) {
   p.tiles_m = (int)((a.M + BM - 1) / BM); p.tiles_n = (a.N + BN - 1) / BN; p.nmat = 1;
   p.out = nullptr; p.residual = nullptr; p.row_scale = a.row_scale; p.out_stride = p.res_stride = 0; p.ncols = a.N;
   // workspace: partials (M, tiles_n) float2, then the target logits (M) float
+  p.batches = 1; p.blocks_per_batch = 0; p.lead_rows = p.lead_tiles = 0; p.out_bs = p.res_bs = p.scale_bs = 0;
   p.ce_part = reinterpret_cast<float2*>(a.workspace);
   p.ce_target = reinterpret_cast<float*>(p.ce_part + a.M * p.tiles_n);
   p.targets = reinterpret_cast<const long long*>(a.targets);
@@ -412,24 +459,37 @@ int launch_silu_mul(const void* gu, void* out, long long M, int I, long long in_
   return (int)cudaGetLastError();
 }
 
-int launch_linear(const LinearArgs& a, int sms, cudaStream_t stream) {
+int launch_linear(const LinearBatchedArgs& ba, int sms, cudaStream_t stream) {
+  LinearBatchedArgs args = ba;
+  LinearArgs& a = args.one;
+  // batches that lie back to back are one block of rows
+  if (args.batches > 1 && args.lead_rows == 0 && args.x_batch_stride == a.M * a.x_stride && args.out_batch_stride == a.M * a.out_stride &&
+      (!a.residual || args.residual_batch_stride == a.M * a.residual_stride) && (!a.row_scale || args.scale_batch_stride == a.M)) {
+    a.M *= args.batches;
+    args.batches = 1;
+  }
   ProjParams p;
   int rc;
-  if ((rc = make_matrix_map(&p.tm_x, a.x, a.M, a.K, a.x_stride, BM)) || (rc = make_matrix_map(&p.tm_wk, a.w, a.N, a.K, a.w_stride, BN)))
+  if ((rc = make_rows_map(&p.tm_x, a.x, args.batches, a.M, a.K, a.x_stride, args.x_batch_stride)) ||
+      (rc = make_matrix_map(&p.tm_wk, a.w, a.N, a.K, a.w_stride, BN)))
     return rc;
   p.tm_wv = p.tm_wk;
   p.k_cache = p.v_cache = nullptr; p.status = a.status; p.cache_bs = 0;
+  const long long per_batch = (a.M + 63) / 64, blocks = per_batch * args.batches, lead = args.lead_rows > 0 ? args.batches : 0;
+  p.tiles_n = (a.N + BN - 1) / BN;
+  const long long total = (blocks + 1) / 2 * p.tiles_n;
+  if (total + lead * p.tiles_n >= (1ll << 30) || a.M >= (1ll << 31)) return GCA_ERR_TOO_LARGE;
   p.M = (int)a.M; p.D = a.K; p.rows_per_seq = 1; p.pos = 0; p.zero_landmark = 0;
-  p.tiles_m = (int)((a.M + BM - 1) / BM); p.tiles_n = (a.N + BN - 1) / BN; p.nmat = 1;
+  p.tiles_m = (int)((blocks + 1) / 2); p.nmat = 1;
+  p.batches = args.batches; p.blocks_per_batch = (int)per_batch;
+  p.lead_rows = args.lead_rows; p.lead_tiles = (int)(lead * p.tiles_n);
+  p.out_bs = args.out_batch_stride; p.res_bs = args.residual_batch_stride; p.scale_bs = args.scale_batch_stride;
   p.out = (__nv_bfloat16*)a.out; p.residual = (const __nv_bfloat16*)a.residual; p.row_scale = a.row_scale;
   p.out_stride = a.out_stride; p.res_stride = a.residual_stride; p.ncols = a.N;
   p.ce_part = nullptr; p.ce_target = nullptr; p.targets = nullptr;
-  const long long total = (long long)p.tiles_m * p.tiles_n;
-  if (total >= (1ll << 31) || a.M >= (1ll << 31)) return GCA_ERR_TOO_LARGE;
-  if (total == 0) return 0;
   GCA_CUDA_CHECK(cudaFuncSetAttribute(kv_project_append_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-  const unsigned grid = (unsigned)(total < sms ? total : sms);
-  kv_project_append_kernel<<<grid, NTHREADS, SMEM_BYTES, stream>>>(p);
+  const long long tiles = total + p.lead_tiles;
+  kv_project_append_kernel<<<(unsigned)(tiles < sms ? tiles : sms), NTHREADS, SMEM_BYTES, stream>>>(p);
   GCA_CUDA_CHECK(cudaGetLastError());
   return 0;
 }
@@ -446,6 +506,7 @@ int launch_kv_project_append(const KvProjectArgs& a, int sms, cudaStream_t strea
   p.zero_landmark = a.zero_landmark;
   p.tiles_m = (int)((M + BM - 1) / BM); p.tiles_n = a.D / BN; p.nmat = 2;
   p.out = nullptr; p.residual = nullptr; p.row_scale = nullptr; p.out_stride = p.res_stride = 0; p.ncols = a.D;
+  p.batches = 1; p.blocks_per_batch = 0; p.lead_rows = p.lead_tiles = 0; p.out_bs = p.res_bs = p.scale_bs = 0;
   p.ce_part = nullptr; p.ce_target = nullptr; p.targets = nullptr;
   const long long total = (long long)p.tiles_m * p.tiles_n * 2;
   if (total >= (1ll << 31)) return GCA_ERR_TOO_LARGE;

@@ -37,44 +37,13 @@ def _require(t: torch.Tensor, name: str) -> None:
 
 def row_rms(x: torch.Tensor, eps: float) -> torch.Tensor:
     """1 / sqrt(mean(x^2, -1) + eps) per row of x (..., D) bf16 -> float32 (M,)."""
-    _require(x, "row_rms")
-    x2 = _rows(x)
-    out = torch.empty(x2.shape[0], dtype=torch.float32, device=x.device)
-    a = _lib.RowRmsArgs()
-    a.x, a.row_scale, a.M, a.x_stride, a.D, a.eps = x2.data_ptr(), out.data_ptr(), x2.shape[0], x2.stride(0), x2.shape[1], eps
-    _lib.call("gca_row_rms", C.byref(a), _stream())
-    return out
+    return _lib.host().row_rms(x, eps)
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, row_scale: Optional[torch.Tensor] = None,
            residual: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """out[m] = row_scale[m] * (x[m] @ weight.T) + residual[m]; x (..., K), weight (N, K), bf16."""
-    _require(x, "linear")
-    _require(weight, "linear weight")
-    x2, n = _rows(x), weight.shape[0]
-    shape = x.shape[:-1] + (n,)
-    if out is None:
-        out = torch.empty(shape, dtype=torch.bfloat16, device=x.device)
-    o2 = _rows(out)
-    if o2.data_ptr() != out.data_ptr():
-        raise ValueError("linear: `out` must be viewable as (M, N) rows")
-    a = _lib.LinearArgs()
-    a.x, a.w, a.out = x2.data_ptr(), weight.data_ptr(), o2.data_ptr()
-    a.M, a.N, a.K = x2.shape[0], n, x2.shape[1]
-    a.x_stride, a.w_stride, a.out_stride = x2.stride(0), weight.stride(0), o2.stride(0)
-    if residual is not None:
-        _require(residual, "linear residual")
-        r2 = _rows(residual)
-        if r2.shape != o2.shape:
-            raise ValueError(f"linear: residual {tuple(residual.shape)} does not match the output {tuple(shape)}")
-        a.residual, a.residual_stride = r2.data_ptr(), r2.stride(0)
-    if row_scale is not None:
-        if row_scale.dtype != torch.float32 or row_scale.numel() != x2.shape[0] or not row_scale.is_contiguous():
-            raise ValueError("linear: row_scale must be contiguous float32 with one value per row")
-        a.row_scale = row_scale.data_ptr()
-    a.status = _status(x.device).data_ptr()
-    _lib.call("gca_linear", C.byref(a), _stream())
-    return out
+    return _lib.host().linear(x, weight, row_scale, residual, out)
 
 
 def fold_gain(weight: torch.Tensor, gain: torch.Tensor) -> torch.Tensor:
@@ -91,14 +60,7 @@ def rmsnorm_linear(x: torch.Tensor, folded_weight: torch.Tensor, eps: float) -> 
 def silu_mul(gate_up: torch.Tensor) -> torch.Tensor:
     """silu(gate_up[..., :I]) * gate_up[..., I:] for the output (..., 2 I) of one stacked gate|up projection
     (the reference's fused SwiGLU activation, ``model/llama.py:290-300``): one launch, one rounding."""
-    _require(gate_up, "silu_mul")
-    x2 = _rows(gate_up)
-    inter = x2.shape[1] // 2
-    if x2.shape[1] != 2 * inter:
-        raise ValueError("silu_mul: the last dimension must hold gate and up halves of equal width")
-    out = torch.empty((x2.shape[0], inter), dtype=torch.bfloat16, device=gate_up.device)
-    _lib.call("gca_silu_mul", x2.data_ptr(), out.data_ptr(), x2.shape[0], inter, x2.stride(0), out.stride(0), _stream())
-    return out.view(*gate_up.shape[:-1], inter)
+    return _lib.host().silu_mul(gate_up)
 
 
 def window_decode(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, window: int, slopes: Optional[torch.Tensor] = None,
@@ -107,30 +69,7 @@ def window_decode(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, window: int
     (``flash_attn_with_kvcache(..., causal=True, window_size=(window, 0), alibi_slopes=slopes)``,
     ``model/llama.py:684-688``).  q (N, Hq, Sq, 64), k / v (N, Hkv, T, 64) bf16 -- any strides with the
     head dimension contiguous; the query rows stand at positions T - Sq .. T - 1.  Returns (N, Hq, Sq, 64)."""
-    a = _lib.WindowDecodeArgs()
-    out = _fill_window_args(a, q, k, v, window, slopes, sm_scale)
-    _lib.call("gca_window_decode", C.byref(a), _stream())
-    return out
-
-
-def _fill_window_args(a, q, k, v, window, slopes, sm_scale) -> torch.Tensor:
-    for t, name in ((q, "q"), (k, "k"), (v, "v")):
-        _require(t, f"window_decode {name}")
-        if t.dim() != 4 or t.shape[-1] != 64 or t.stride(-1) != 1:
-            raise ValueError(f"window_decode: {name} must be (N, H, L, 64) with contiguous head dimension")
-    n, hq, sq, _ = q.shape
-    hkv, t_len = k.shape[1], k.shape[2]
-    out = torch.empty((n, hq, sq, 64), dtype=torch.bfloat16, device=q.device)
-    a.q, a.k, a.v, a.out = q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr()
-    if slopes is not None:
-        if slopes.dtype != torch.float32 or slopes.numel() != hq or not slopes.is_contiguous() or not slopes.is_cuda:
-            raise ValueError("window_decode: slopes must be contiguous float32 (Hq,) on the device")
-        a.alibi_slopes = slopes.data_ptr()
-    for i in range(3):
-        a.q_stride[i], a.o_stride[i], a.k_stride[i], a.v_stride[i] = q.stride(i), out.stride(i), k.stride(i), v.stride(i)
-    a.N, a.Hq, a.Hkv, a.Sq, a.T, a.window = n, hq, hkv, sq, t_len, int(window)
-    a.sm_scale = float(sm_scale) if sm_scale is not None else 0.125
-    return out
+    return _lib.host().window_decode(q, k, v, window, slopes, 0.125 if sm_scale is None else sm_scale)
 
 
 def window_ring_decode(q: torch.Tensor, k_ring: torch.Tensor, v_ring: torch.Tensor, k_new: torch.Tensor, v_new: torch.Tensor,
@@ -144,22 +83,8 @@ def window_ring_decode(q: torch.Tensor, k_ring: torch.Tensor, v_ring: torch.Tens
     captured CUDA graph can replay the step; it must stay below 2^32 (subtract a multiple of T long before).
     q (N, Hq, 1, 64).  ``torch.roll(ring, -(rows_written % T), 2)``
     gives the window back in order."""
-    for t, name in ((k_new, "k_new"), (v_new, "v_new")):
-        _require(t, f"window_ring_decode {name}")
-    if not rows_written.is_cuda:
-        raise RuntimeError("window_ring_decode rows_written: the fused projections run on a CUDA device only (no CPU fallback)")
-    if rows_written.dtype != torch.int64 or rows_written.numel() != 1:
-        raise ValueError("window_ring_decode: rows_written must be one int64 on the device")
-    n, hkv = k_ring.shape[0], k_ring.shape[1]
-    kn, vn = k_new.reshape(n, hkv, 64) if k_new.dim() == 4 else k_new, v_new.reshape(n, hkv, 64) if v_new.dim() == 4 else v_new
-    if kn.stride(2) != 1 or vn.stride(2) != 1 or kn.stride()[:2] != vn.stride()[:2]:
-        raise ValueError("window_ring_decode: new rows must be bf16 with a contiguous head dimension and equal strides")
-    a = _lib.WindowRingDecodeArgs()
-    out = _fill_window_args(a.attn, q, k_ring, v_ring, window, slopes, sm_scale)
-    a.k_new, a.v_new, a.rows_written = kn.data_ptr(), vn.data_ptr(), rows_written.data_ptr()
-    a.new_stride[0], a.new_stride[1] = kn.stride(0), kn.stride(1)
-    _lib.call("gca_window_ring_decode", C.byref(a), _stream())
-    return out
+    return _lib.host().window_ring_decode(q, k_ring, v_ring, k_new, v_new, rows_written, window, slopes,
+                                          0.125 if sm_scale is None else sm_scale)
 
 
 def linear_cross_entropy(x: torch.Tensor, weight: torch.Tensor, targets: torch.Tensor,

@@ -16,7 +16,7 @@ import math
 import torch
 import torch.nn as nn
 
-from . import fused_ops, gca
+from . import _lib, fused_ops, gca
 
 
 class RMSNorm(nn.Module):
@@ -135,31 +135,8 @@ class TritonGroupCrossAttention(nn.Module):
         as in ``model/DRT.py:387-394``."""
         if self.q_proj.bias is not None or self.o_proj.bias is not None:
             raise ValueError("forward_fused: projection biases are not supported")
-        n, dd, s, dim = hidden_states.shape
-        q = fused_ops.rmsnorm_linear(hidden_states, self._folded_q_weight(), self.pre_norm.eps)
-        skip_first = dd > 1 and not first_chunk_retrieves
-        out = torch.empty((n, dd * s, dim), dtype=torch.bfloat16, device=hidden_states.device)
-        if skip_first or indices.shape[1] * indices.shape[2] == 0:
-            lead = s if indices.shape[1] * indices.shape[2] else dd * s
-            if residual is None:
-                out[:, :lead].zero_()
-            else:
-                out[:, :lead] = residual[:, :lead]
-            if lead == dd * s:
-                return out
-        q5 = q.view(n, dd, s, self.num_heads, self.head_dim).permute(0, 1, 3, 2, 4)
-        if skip_first:
-            q5 = q5[:, 1:]
-        vals = gca.gca_indexed_nograd(q5, k_cache, v_cache, indices, weights, 1.0 / math.sqrt(self.head_dim), self.sm_n)
-        vals = vals.permute(0, 1, 3, 2, 4).reshape(n, -1, self.hidden_size)
-        first = s if skip_first else 0
-        w = self.o_proj.weight.detach()
-        if first == 0:                           # no skipped chunk: all rows share one row stride, one GEMM
-            fused_ops.linear(vals, w, residual=residual, out=out)
-            return out
-        for b in range(n):                       # one GEMM per sequence: a sequence's rows share one row stride
-            fused_ops.linear(vals[b], w, residual=None if residual is None else residual[b, first:], out=out[b, first:])
-        return out
+        return _lib.host().layer_fused(hidden_states, self._folded_q_weight(), self.pre_norm.eps, k_cache, v_cache, indices, weights,
+                                       self.o_proj.weight, residual, first_chunk_retrieves, self.num_heads, 1.0 / math.sqrt(self.head_dim))
 
     def forward_indexed(self, hidden_states: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
                         indices: torch.Tensor, weights: torch.Tensor, first_chunk_retrieves: bool = False) -> torch.Tensor:
@@ -182,7 +159,7 @@ class TritonGroupCrossAttention(nn.Module):
         if torch.is_grad_enabled() and (q5.requires_grad or k_cache.requires_grad or weights.requires_grad):
             vals = gca.gca_indexed(q5, k_cache, v_cache, indices, weights, scale, self.sm_n, token_major_out=True)
         else:
-            vals = gca.gca_indexed_nograd(q5, k_cache, v_cache, indices, weights, scale, self.sm_n)
+            vals = gca.gca_indexed_nograd(q5, k_cache, v_cache, indices, weights, scale, self.sm_n, token_major_out=True)
         vals = vals.permute(0, 1, 3, 2, 4).reshape(n, -1, self.hidden_size)
         o = self.o_proj(vals)
         return self._pad_first_chunk(hidden_states, o) if skip_first else o

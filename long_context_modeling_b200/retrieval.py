@@ -25,26 +25,15 @@ import torch
 from . import _lib
 
 
+_SCORE_ROUND = {"fp32": 0, "bf16": 1}
+
+
 class Retrieval(NamedTuple):
     keys: torch.Tensor       # (R.., K) int64 view of the packed uint64 candidates, descending
     indices: torch.Tensor    # (R.., K) int32 global chunk ids, -1 = padding
     scores: torch.Tensor     # (R.., K) float32 noise-free scores
     weights: torch.Tensor    # (R.., K) float32 softmax over valid slots, padding 0
     n_valid: torch.Tensor    # (R..)    int32
-
-
-def _bf16_rows(t: torch.Tensor, require_bf16: bool = False) -> torch.Tensor:
-    """The scan kernel reads bf16 landmarks.  Landmarks in another dtype are ROUNDED to bf16 first:
-    that is what the reference's scoring einsum sees under the trainer's bf16 autocast
-    (``trainer/slidewindow_trainer.py:198``, ``model/DRT.py:612``), but a float32 run of the
-    reference scores in float32 and may pick another chunk on a near tie.  ``require_bf16``
-    turns the rounding into an error."""
-    if t.dtype != torch.bfloat16:
-        if require_bf16:
-            raise ValueError(f"landmarks are {t.dtype}: the scan kernel scores bf16 landmarks and would round them "
-                             "(pass bf16 tensors, or drop require_bf16 to accept the rounding)")
-        t = t.to(torch.bfloat16)
-    return t if t.stride(-1) == 1 else t.contiguous()
 
 
 def lmk_score_topk(lmk_q: torch.Tensor, lmk_k: torch.Tensor, topk: int, *, q_pos0: Optional[int] = None,
@@ -55,49 +44,15 @@ def lmk_score_topk(lmk_q: torch.Tensor, lmk_k: torch.Tensor, topk: int, *, q_pos
     Row ``i`` sees cached chunk ``e`` iff ``e_base + e < q_pos0 + i``; the default
     ``q_pos0 = E - Cq`` is the reference's causal chunk mask (``model/DRT.py:590-607``).
     ``head_dim`` = 64 switches to one score / one top-k per head (outputs (N, Cq, H, K)).
-    Landmarks that are not bf16 are rounded to bf16 before scoring (see ``_bf16_rows``);
-    ``require_bf16=True`` raises instead.
+    The scan kernel reads bf16 landmarks.  Landmarks in another dtype are ROUNDED to bf16 first: that is
+    what the reference's scoring einsum sees under the trainer's bf16 autocast
+    (``trainer/slidewindow_trainer.py:198``, ``model/DRT.py:612``), but a float32 run of the reference
+    scores in float32 and may pick another chunk on a near tie.  ``require_bf16=True`` raises instead.
     """
-    if not (lmk_q.is_cuda and lmk_k.is_cuda):
-        raise RuntimeError("landmark retrieval runs on CUDA tensors only (there is no CPU path)")
-    if lmk_q.dim() != 3 or lmk_k.dim() != 3 or lmk_q.shape[0] != lmk_k.shape[0] or lmk_q.shape[2] != lmk_k.shape[2]:
-        raise ValueError("expected lmk_q (N, Cq, D) and lmk_k (N, E, D)")
-    lq, lk = _bf16_rows(lmk_q.detach(), require_bf16), _bf16_rows(lmk_k.detach(), require_bf16)
-    n, cq, d = lq.shape
-    e = lk.shape[1]
-    heads = d // head_dim if head_dim else 1
-    rows_shape = (n, cq, heads) if head_dim else (n, cq)
-    dev = lq.device
-    keys = torch.empty(rows_shape + (topk,), dtype=torch.int64, device=dev)
-    indices = torch.empty(rows_shape + (topk,), dtype=torch.int32, device=dev)
-    scores = torch.empty(rows_shape + (topk,), dtype=torch.float32, device=dev)
-    weights = torch.empty(rows_shape + (topk,), dtype=torch.float32, device=dev)
-    n_valid = torch.empty(rows_shape, dtype=torch.int32, device=dev)
-    if n * cq == 0:
-        return Retrieval(keys, indices, scores, weights, n_valid)
-    a = _lib.LmkTopkArgs()
-    a.lmk_q, a.lmk_k = lq.data_ptr(), lk.data_ptr()
-    if noise is not None:
-        noise = noise.to(torch.float32).contiguous()
-        if noise.shape != (n, cq, e):
-            raise ValueError("noise must be (N, Cq, E)")
-        a.noise = noise.data_ptr()
-    a.out_keys, a.out_indices, a.out_scores = keys.data_ptr(), indices.data_ptr(), scores.data_ptr()
-    a.out_weights, a.out_nvalid = weights.data_ptr(), n_valid.data_ptr()
-    a.q_batch_stride, a.q_row_stride = lq.stride(0), lq.stride(1)
-    a.k_batch_stride, a.k_row_stride = lk.stride(0), lk.stride(1)
-    a.q_pos0 = (e - cq) if q_pos0 is None else int(q_pos0)
-    a.e_base = int(e_base)
-    a.N, a.Cq, a.E, a.D, a.K = n, cq, e, d, int(topk)
-    a.head_dim = int(head_dim)
-    a.score_round = {"fp32": 0, "bf16": 1}[score_round]
-    a.splits = int(splits)
-    with torch.cuda.device(dev):
-        nbytes = _lib.lib().lmk_topk_workspace_bytes(C.byref(a))
-        ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=dev)
-        a.workspace, a.workspace_bytes = ws.data_ptr(), nbytes
-        _lib.call("lmk_score_topk", C.byref(a), torch.cuda.current_stream().cuda_stream)
-    return Retrieval(keys, indices, scores, weights, n_valid)
+    if require_bf16 and not (lmk_q.dtype == lmk_k.dtype == torch.bfloat16):
+        raise ValueError(f"landmarks are {lmk_q.dtype} / {lmk_k.dtype}: the scan kernel scores bf16 landmarks and would round them "
+                         "(pass bf16 tensors, or drop require_bf16 to accept the rounding)")
+    return Retrieval(*_lib.host().lmk_score_topk(lmk_q, lmk_k, topk, q_pos0, e_base, noise, head_dim, _SCORE_ROUND[score_round], splits))
 
 
 def merge_topk(keys: torch.Tensor, topk: int) -> Retrieval:
