@@ -234,6 +234,33 @@ int lmk_score_topk(const LmkTopkArgs* args, void* stream);
 size_t lmk_topk_workspace_bytes(const LmkTopkArgs* args);
 
 /*
+ * Gradient of the retrieval weights into the landmarks: what autograd does behind
+ * `softmax(scores.gather(...))` of model/DRT.py:626 (einsum backward, gather backward, index_put with
+ * accumulation), per-sequence mode.  With ds = w (dw - sum_k w dw) / sqrt(D):
+ *   dlmk_q[n, c] = sum_k ds[n, c, k] lmk_k[n, idx(n, c, k)],   dlmk_k[n, e] = sum over the (c, k) that chose e of ds lmk_q[n, c]
+ * lmk_q, lmk_k, dlmk_q (N, Cq, D), dlmk_k (N, E, D) bf16 (the gradients contiguous, either may be NULL); indices (N, Cq, K)
+ * int32 with -1 = padding and weights (N, Cq, K) float32 as lmk_score_topk wrote them with the same q_pos0 and e_base = 0.
+ * The incoming gradient is dw_rows for the first `rows` query rows plus dw_all for all of them (float32 by
+ * strides n, c, k; either may be NULL): the weights are handed out whole and without their last row.
+ */
+typedef struct LmkGradArgs {
+  const void* lmk_q;
+  const void* lmk_k;
+  const int32_t* indices;
+  const float* weights;
+  const float* dw_rows;
+  const float* dw_all;
+  void* dlmk_q;
+  void* dlmk_k;
+  int64_t q_batch_stride, q_row_stride, k_batch_stride, k_row_stride;
+  int64_t dw_rows_stride[3], dw_all_stride[3];
+  int64_t q_pos0;
+  int32_t N, Cq, E, D, K, rows;
+} LmkGradArgs;
+
+int lmk_weights_backward(const LmkGradArgs* args, void* stream);
+
+/*
  * lmk_score_topk for callers that cannot provide device scratch.  (No counterpart in the
  * reference: it exists for hosts that must not allocate device memory around the call -- a
  * server that handed all HBM to its own pools, a plugin inside someone else's allocator, a
@@ -242,8 +269,9 @@ size_t lmk_topk_workspace_bytes(const LmkTopkArgs* args);
  * Same arguments, same results, bit for bit; args->workspace / workspace_bytes are ignored.
  * The per-block candidate lists go into an array compiled into the library
  * (LMK_STATIC_SCRATCH_BYTES of device memory on every GPU that loads it, held until exit).
- * Limit: lmk_topk_workspace_bytes(args) must not exceed LMK_STATIC_SCRATCH_BYTES, i.e.
- * rows * splits * K * 8 bytes <= 1 MiB (rows = N*Cq, times D/64 in per-head mode); a larger
+ * Limit: the row scan's lists must not exceed LMK_STATIC_SCRATCH_BYTES, i.e.
+ * rows * splits * K * 8 bytes <= 1 MiB (rows = N*Cq, times D/64 in per-head mode; this entry always takes
+ * the row scan, lmk_score_topk has another form with a larger workspace for many rows); a larger
  * problem is refused with GCA_ERR_STATIC_SCRATCH and nothing is launched.  Passing
  * args->splits lets the caller shrink the need.
  * The call allocates nothing, on the host or on the device.  Its first use on a device looks
@@ -525,7 +553,7 @@ const char* gca_strerror(int code);
 int gca_abi_version(void);
 /* sizeof() of an argument block as the library was compiled (0 GcaFwdArgs, 1 GcaBwdArgs,
  * 2 LmkTopkArgs, 3 LmkMergeArgs, 4 CacheAppendArgs, 5 LmkExchangeArgs, 6 KvProjectArgs, 7 RowRmsArgs, 8 LinearArgs, 9 WindowDecodeArgs, 10 LinearCeArgs, 11 WindowAppendArgs, 12 WindowRingDecodeArgs,
- * 13 LinearBatchedArgs): lets a foreign-language binding verify
+ * 13 LinearBatchedArgs, 14 LmkGradArgs): lets a foreign-language binding verify
  * its struct layout before the first call. */
 size_t gca_sizeof(int which);
 

@@ -64,6 +64,16 @@ class LmkTopkArgs(C.Structure):
     ]
 
 
+class LmkGradArgs(C.Structure):
+    _fields_ = [
+        ("lmk_q", C.c_void_p), ("lmk_k", C.c_void_p), ("indices", C.c_void_p), ("weights", C.c_void_p),
+        ("dw_rows", C.c_void_p), ("dw_all", C.c_void_p), ("dlmk_q", C.c_void_p), ("dlmk_k", C.c_void_p),
+        ("q_batch_stride", C.c_int64), ("q_row_stride", C.c_int64), ("k_batch_stride", C.c_int64), ("k_row_stride", C.c_int64),
+        ("dw_rows_stride", C.c_int64 * 3), ("dw_all_stride", C.c_int64 * 3), ("q_pos0", C.c_int64),
+        ("N", C.c_int32), ("Cq", C.c_int32), ("E", C.c_int32), ("D", C.c_int32), ("K", C.c_int32), ("rows", C.c_int32),
+    ]
+
+
 class LmkMergeArgs(C.Structure):
     _fields_ = [
         ("keys", C.c_void_p), ("out_keys", C.c_void_p), ("out_indices", C.c_void_p),
@@ -158,6 +168,7 @@ EXPORTS = {
     "lmk_score_topk": (C.c_int, [C.POINTER(LmkTopkArgs), C.c_void_p]),
     "lmk_topk_workspace_bytes": (C.c_size_t, [C.POINTER(LmkTopkArgs)]),
     "lmk_score_topk_static": (C.c_int, [C.POINTER(LmkTopkArgs), C.c_void_p]),
+    "lmk_weights_backward": (C.c_int, [C.POINTER(LmkGradArgs), C.c_void_p]),
     "lmk_topk_merge": (C.c_int, [C.POINTER(LmkMergeArgs), C.c_void_p]),
     "gca_cache_append": (C.c_int, [C.POINTER(CacheAppendArgs), C.c_void_p]),
     "gca_kv_project_append": (C.c_int, [C.POINTER(KvProjectArgs), C.c_void_p]),
@@ -207,7 +218,7 @@ def lib() -> C.CDLL:
             raise RuntimeError("libgca_b200.so has an unexpected ABI version")
         for which, struct in enumerate((GcaFwdArgs, GcaBwdArgs, LmkTopkArgs, LmkMergeArgs, CacheAppendArgs, LmkExchangeArgs,
                                        KvProjectArgs, RowRmsArgs, LinearArgs, WindowDecodeArgs, LinearCeArgs, WindowAppendArgs,
-                                       WindowRingDecodeArgs, LinearBatchedArgs)):
+                                       WindowRingDecodeArgs, LinearBatchedArgs, LmkGradArgs)):
             if handle.gca_sizeof(which) != C.sizeof(struct):
                 raise RuntimeError(f"struct layout mismatch for {struct.__name__}: "
                                    f"library {handle.gca_sizeof(which)} vs binding {C.sizeof(struct)}")

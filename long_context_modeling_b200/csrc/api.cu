@@ -7,6 +7,7 @@
 namespace gca {
 int launch_decode(const GcaFwdArgs& a, int sms, cudaStream_t stream);
 int launch_lmk_score_topk(const LmkTopkArgs& a, void* scratch, int sms, cudaStream_t stream);
+int launch_lmk_grad(const LmkGradArgs& a, cudaStream_t stream);
 int launch_lmk_merge(const LmkMergeArgs& a, cudaStream_t stream);
 size_t lmk_topk_workspace_bytes_impl(const LmkTopkArgs& a, int sms);
 bool bwd_tc_available();
@@ -126,6 +127,7 @@ size_t gca_sizeof(int which) {
     case 11: return sizeof(WindowAppendArgs);
     case 12: return sizeof(WindowRingDecodeArgs);
     case 13: return sizeof(LinearBatchedArgs);
+    case 14: return sizeof(LmkGradArgs);
     default: return 0;
   }
 }
@@ -286,6 +288,21 @@ int lmk_score_topk(const LmkTopkArgs* a, void* stream) {
   const size_t need = gca::lmk_topk_workspace_bytes_impl(*a, sms);
   if (a->workspace_bytes < need) return GCA_ERR_WORKSPACE;
   return gca::launch_lmk_score_topk(*a, a->workspace, sms, (cudaStream_t)stream);
+}
+
+int lmk_weights_backward(const LmkGradArgs* a, void* stream) {
+  if (!a) return GCA_ERR_NULL;
+  if (!a->lmk_q || !a->lmk_k || !a->indices || !a->weights) return GCA_ERR_NULL;
+  if (a->N < 0 || a->Cq < 0 || a->E < 0 || a->D < 8 || a->D % 8 != 0 || a->D > 1024 || a->K < 1 || a->K > 32 || a->rows < 0 || a->rows > a->Cq)
+    return GCA_ERR_SHAPE;
+  if (a->q_row_stride % 8 || a->k_row_stride % 8 || a->q_batch_stride % 8 || a->k_batch_stride % 8) return GCA_ERR_STRIDE;
+  if (!aligned16(a->lmk_q) || !aligned16(a->lmk_k) || (a->dlmk_q && !aligned16(a->dlmk_q)) || (a->dlmk_k && !aligned16(a->dlmk_k)))
+    return GCA_ERR_ALIGN;
+  if ((long long)a->Cq * a->K >= (1ll << 31) - 64) return GCA_ERR_TOO_LARGE;
+  if (a->N == 0) return 0;
+  gca::DeviceScope scope(a->lmk_q);
+  if (scope.rc) return scope.rc;
+  return gca::launch_lmk_grad(*a, (cudaStream_t)stream);
 }
 
 int lmk_topk_merge(const LmkMergeArgs* a, void* stream) {

@@ -34,6 +34,23 @@ __device__ __forceinline__ int slot_chunk(const int32_t* __restrict__ indices, l
   return indices ? indices[zj * K + k] : k;
 }
 
+// Programmatic dependent launch: a kernel launched with `launch_dependent` may start while the one before it on the
+// stream still runs (once every block of that one has called pdl_trigger or left); pdl_wait returns when
+// everything before it on the stream is complete and visible.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... Params, class... Args>
+inline cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr; cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+}
+
 // Problem geometry shared by forward and backward kernels (passed by value).
 struct Geom {
   int N, J, Hq, Hkv, S, L, D, K, C, G;

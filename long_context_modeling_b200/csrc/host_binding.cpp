@@ -43,7 +43,7 @@ struct Api {
 #define GCA_API(name) decltype(&::name) name = nullptr;
 #define GCA_API_LIST                                                                                          \
   GCA_API(gca_fwd) GCA_API(gca_decode) GCA_API(gca_bwd_stages) GCA_API(gca_bwd_workspace_bytes)               \
-  GCA_API(lmk_score_topk) GCA_API(lmk_topk_workspace_bytes) GCA_API(gca_kv_project_append) GCA_API(gca_row_rms) \
+  GCA_API(lmk_score_topk) GCA_API(lmk_topk_workspace_bytes) GCA_API(lmk_weights_backward) GCA_API(gca_kv_project_append) GCA_API(gca_row_rms) \
   GCA_API(gca_linear) GCA_API(gca_linear_batched) GCA_API(gca_silu_mul) GCA_API(gca_window_decode)            \
   GCA_API(gca_window_ring_decode) GCA_API(gca_strerror)
   GCA_API_LIST
@@ -666,6 +666,82 @@ Retrieved score_topk(const Tensor& q_in, const Tensor& k_in, int64_t topk, bool 
   return r;
 }
 
+// A tensor over the storage of `t` without its last row (axis 1 of a contiguous (N, Cq, K)).
+Tensor without_last_row(const Tensor& t) {
+  Tensor s = carve(t.storage(), (size_t)t.storage_offset() * t.element_size(), {0}, t.scalar_type());
+  const int64_t cq = t.size(1);
+  s.unsafeGetTensorImpl()->set_sizes_and_strides({t.size(0), cq > 0 ? cq - 1 : 0, t.size(2)}, t.strides());
+  return s;
+}
+
+// The retrieval weights as a function of the landmarks: outputs the weights without the last row, then whole.
+struct WeightsBackward : public Node {
+  SavedVariable q, k, w;
+  Tensor indices;
+  bool released = false;
+  std::mutex mu;
+
+  std::string name() const override { return "RetrievalWeightsBackward"; }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mu);
+    released = true;
+    for (SavedVariable* s : {&q, &k, &w}) s->reset_data();
+    indices = Tensor();
+  }
+  variable_list apply(variable_list&& grads) override {
+    std::lock_guard<std::mutex> lock(mu);
+    TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
+    variable_list out(2);
+    if (!grads[0].defined() && !grads[1].defined()) return out;
+    const Tensor tq = q.unpack(), tk = k.unpack(), tw = w.unpack(shared_from_this());
+    at::AutoDispatchBelowADInplaceOrView below;
+    const Tensor cq = inner_contiguous(tq), ck = inner_contiguous(tk);
+    Launch on(cq);
+    LmkGradArgs a{};
+    a.lmk_q = cq.const_data_ptr(); a.lmk_k = ck.const_data_ptr();
+    a.indices = indices.const_data_ptr<int32_t>(); a.weights = tw.const_data_ptr<float>();
+    if (grads[0].defined()) {
+      a.dw_rows = grads[0].const_data_ptr<float>(); a.rows = (int32_t)grads[0].size(1);
+      for (int i = 0; i < 3; ++i) a.dw_rows_stride[i] = grads[0].stride(i);
+    }
+    if (grads[1].defined()) {
+      a.dw_all = grads[1].const_data_ptr<float>();
+      for (int i = 0; i < 3; ++i) a.dw_all_stride[i] = grads[1].stride(i);
+    }
+    if (task_should_compute_output(0)) { out[0] = at::empty(cq.sizes(), cq.options()); a.dlmk_q = out[0].mutable_data_ptr(); }
+    if (task_should_compute_output(1)) { out[1] = at::empty(ck.sizes(), ck.options()); a.dlmk_k = out[1].mutable_data_ptr(); }
+    a.q_batch_stride = cq.stride(0); a.q_row_stride = cq.stride(1); a.k_batch_stride = ck.stride(0); a.k_row_stride = ck.stride(1);
+    a.N = (int32_t)cq.size(0); a.Cq = (int32_t)cq.size(1); a.E = (int32_t)ck.size(1); a.D = (int32_t)cq.size(2); a.K = (int32_t)indices.size(2);
+    a.q_pos0 = ck.size(1) - cq.size(1);
+    try {
+      call("lmk_weights_backward", [&] { return api.lmk_weights_backward(&a, on.stream); });
+    } catch (const LibraryError& e) { GcaBackward::raise(e); }
+    return out;
+  }
+};
+
+struct Retrieving { Tensor indices, weights; Retrieved full; };
+
+// Selection and weights for query chunks 1 .. Cq - 1 (row i serves query chunk i + 1), recorded for autograd when a landmark
+// needs a gradient.
+Retrieving retrieve(const Tensor& q, const Tensor& k, int64_t topk, const Tensor& noise, int64_t score_round) {
+  Retrieving r;
+  r.full = score_topk(q, k, topk, false, 0, 0, noise, 0, score_round, 0);
+  r.indices = without_last_row(r.full.indices);
+  r.weights = without_last_row(r.full.weights);
+  if (torch::autograd::compute_requires_grad(q, k)) {
+    auto node = std::shared_ptr<WeightsBackward>(new WeightsBackward(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(q, k));
+    node->q = SavedVariable(q, false); node->k = SavedVariable(k, false);
+    node->indices = r.full.indices;
+    torch::autograd::impl::set_version_counter(r.weights, torch::autograd::impl::version_counter(r.full.weights));
+    torch::autograd::set_history(r.weights, node);
+    torch::autograd::set_history(r.full.weights, node);
+    node->w = SavedVariable(r.full.weights, true);
+  }
+  return r;
+}
+
 // The projection + append of `count` chunks at chunk position `pos` of the caches.
 void kv_project_append(const Tensor& x, const Tensor& wk, const Tensor& wv, const Tensor& k_cache, const Tensor& v_cache, const Tensor& lmk,
                        int64_t pos, int64_t capacity, bool zero_landmark) {
@@ -834,6 +910,17 @@ ENTRY(linear, 5)
   return wrap(unlocked([&] { return linear(x, w, scale, residual, out); }));
 ENTRY_END
 
+// (q, landmarks, topk, noise or None, score_round) -> (indices[:, :-1], weights[:, :-1], keys, indices, scores, weights, n_valid)
+ENTRY(retrieve, 5)
+  const Tensor &q = a.tensor(0), &k = a.tensor(1);
+  TORCH_CHECK(q.is_cuda() && k.is_cuda(), "landmark retrieval runs on CUDA tensors only (there is no CPU path)");
+  TORCH_CHECK_VALUE(q.dim() == 3 && k.dim() == 3 && q.size(0) == k.size(0) && q.size(2) == k.size(2), "expected lmk_q (N, Cq, D) and lmk_k (N, E, D)");
+  const int64_t topk = a.integer(2), round = a.integer(4);
+  const Tensor noise = a.maybe(3);
+  const Retrieving r = unlocked([&] { return retrieve(q, k, topk, noise, round); });
+  return wrap_tuple({r.indices, r.weights, r.full.keys, r.full.indices, r.full.scores, r.full.weights, r.full.n_valid});
+ENTRY_END
+
 // (hidden, q weight with the norm's gain, eps, k, v, idx, w, o weight, residual or None, first chunk retrieves, heads, scale)
 ENTRY(layer_fused, 12)
   const Tensor &x = a.tensor(0), &qw = a.tensor(1), &k = a.tensor(3), &v = a.tensor(4), &idx = a.tensor(5), &w = a.tensor(6), &ow = a.tensor(7);
@@ -924,7 +1011,7 @@ ENTRY_END
 PyMethodDef methods[] = {
     METHOD(bind), METHOD(set_switches), METHOD(status_word), METHOD(gca_indexed), METHOD(attention), METHOD(gca_nograd), METHOD(gca_kv_cache),
     METHOD(gca_forward_lse), METHOD(gca_backward), METHOD(row_rms), METHOD(linear), METHOD(layer_fused), METHOD(silu_mul),
-    METHOD(window_decode), METHOD(window_ring_decode), METHOD(lmk_score_topk), METHOD(kv_project_append), {nullptr, nullptr, 0, nullptr}};
+    METHOD(window_decode), METHOD(window_ring_decode), METHOD(lmk_score_topk), METHOD(retrieve), METHOD(kv_project_append), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_host", "Host path of the hot entry points.", -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

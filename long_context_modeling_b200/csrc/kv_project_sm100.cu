@@ -74,17 +74,6 @@ struct ProjParams {
   const long long* targets;           // (M) class ids; negative = ignored row
 };
 
-__device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* m, uint64_t* bar, int c0, int c1, int c2) {
-  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-               ::"r"(smem_u32(smem_dst)), "l"(m), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
-               : "memory");
-}
-__device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m, uint64_t* bar, int c0, int c1) {
-  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-               ::"r"(smem_u32(smem_dst)), "l"(m), "r"(smem_u32(bar)), "r"(c0), "r"(c1)
-               : "memory");
-}
-
 // tile t of this CTA -> (which matrix, row tile, column tile)
 __device__ __forceinline__ void tile_of(const ProjParams& p, int t, int& which, int& tm, int& tn) {
   tn = t % p.tiles_n;
@@ -297,38 +286,6 @@ kv_project_append_kernel(const __grid_constant__ ProjParams p) {
   if (threadIdx.x == 0 && *abort_flag && p.status) atomicOr(p.status, GCA_STATUS_TIMEOUT);
 }
 
-// 2-D bf16 matrix (rows x cols, row stride in elements), boxes of (64 columns x box_rows rows), 128-byte swizzle.
-int make_matrix_map(CUtensorMap* map, const void* base, long long rows, long long cols, long long row_stride, int box_rows) {
-  EncodeTiledFn fn = encode_tiled_fn();
-  if (!fn) return GCA_ERR_TMA;
-  if (row_stride % 8 != 0) return GCA_ERR_STRIDE;
-  const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)row_stride * 2};
-  const cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
-  const cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? 0 : GCA_ERR_TMA;
-}
-
-// The same for linear mode's x: (columns, rows, batches), boxes of 64 columns x 64 rows of one batch.
-int make_rows_map(CUtensorMap* map, const void* base, long long batches, long long rows, long long cols, long long row_stride,
-                  long long batch_stride) {
-  EncodeTiledFn fn = encode_tiled_fn();
-  if (!fn) return GCA_ERR_TMA;
-  if (batches == 1) batch_stride = row_stride;            // never advanced; any legal stride does
-  if (row_stride % 8 != 0 || batch_stride % 8 != 0 || batch_stride <= 0) return GCA_ERR_STRIDE;
-  const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)batches};
-  const cuuint64_t strides[2] = {(cuuint64_t)row_stride * 2, (cuuint64_t)batch_stride * 2};
-  const cuuint32_t box[3] = {64, 64, 1};
-  const cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? 0 : GCA_ERR_TMA;
-}
-
 __global__ void lmk_rows_kernel(const uint4* __restrict__ x, uint4* __restrict__ lmk, long long lmk_bs, int pos, int count,
                                 int row_vecs, long long total) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -470,7 +427,7 @@ int launch_linear(const LinearBatchedArgs& ba, int sms, cudaStream_t stream) {
   }
   ProjParams p;
   int rc;
-  if ((rc = make_rows_map(&p.tm_x, a.x, args.batches, a.M, a.K, a.x_stride, args.x_batch_stride)) ||
+  if ((rc = make_rows_map(&p.tm_x, a.x, args.batches, a.M, a.K, a.x_stride, args.x_batch_stride, 64)) ||
       (rc = make_matrix_map(&p.tm_wk, a.w, a.N, a.K, a.w_stride, BN)))
     return rc;
   p.tm_wv = p.tm_wk;

@@ -1,0 +1,409 @@
+// Landmark top-k for many query rows per sequence (a training step, a prefill) on the tensor cores, with the bits of
+// the row scan.
+//
+// Scoring every (row, landmark) pair is a matrix product, but the selection is defined on float32 sums in ONE fixed order
+// (lmk_topk.cu), which a tensor core does not follow.  So the product only SCREENS: it gives every score to within a bound, a
+// row keeps its KC = K + 4 best approximate scores per range of landmarks, and the merge computes the exact score of
+// those that can still be among the K best -- K of them, rarely one more -- in the scan's own order.
+//
+//   |approximate - exact| <= 2^-15 |q| |k| / sqrt(D) =: eps.   Either sum of exact bf16 products is off by at most a few dozen
+//   roundings of 2^-24 of sum |q_i k_i| <= |q| |k|; tensor cores align and truncate at 2^-22 or better per addition, 48 of
+//   them for D = 768.  The bound is ~8e-4 of the spread of the scores of one row, so it costs next to nothing.
+//   With T the K-th best approximate score of the row, whatever lies below T - 2 eps cannot win.  A range whose KC
+//   entries are all above that line may hide more (copies of one landmark): that row is scanned exactly by its warp.
+//
+// Screening: one CTA per (128 rows, range of landmarks), tiles of 64 landmarks; warp 16 issues the TMA copies of a 4-stage ring
+// (128 x 64 of q, 64 x 64 of the landmarks), warp 17 the 128 x 64 x 16 MMAs; 16 worker warps add up the squared norms
+// from the same stages while they pass, then take the tile from tensor memory and select with warp-wide maxima, one row
+// per warp at a time.  Every wait is bounded; when one runs out the error bound of the block's rows is written as infinite, which
+// sends them through the exact scan.  What bounds it is latency (12 K steps, one selection round after another): 8 x 260 rows x 260
+// landmarks x 768 take ~15 us for both kernels, against 190 us for the row scan and its merge.
+#include "lmk_common.cuh"
+#include "sm100_ptx.cuh"
+#include "tma_host.cuh"
+
+namespace gca {
+
+namespace {
+
+using namespace sm100;
+
+constexpr int BM = 128, BN = 64, BK = 64, STAGES = 4;
+constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
+constexpr int WORKERS = 16, THREADS = (WORKERS + 2) * 32, NORM_WARPS = (BM + BN) / 32;
+constexpr int LDS_ROW = BN + 1;
+constexpr int OFF_SCORE = STAGES * STAGE_BYTES, OFF_NORM = OFF_SCORE + BM * LDS_ROW * 4, OFF_BAR = OFF_NORM + (BM + BN) * 4;
+constexpr int SMEM_BYTES = OFF_BAR + 256 + 1024;
+constexpr int EXTRA = 4, MAX_LISTS = 32;
+constexpr float BOUND = 1.0f / 32768.0f;
+enum Bar { FULL = 0, EMPTY = FULL + STAGES, ACC_FULL = EMPTY + STAGES, ACC_EMPTY, NUM_BARS };
+constexpr uint32_t IDESC = umma_idesc_bf16(BM, BN, 0, 0);
+
+struct ScreenParams {
+  CUtensorMap tm_q, tm_k;
+  const float* noise;
+  unsigned long long* part;      // (rows, lists, KC) approximate keys, descending
+  float* eps;                    // (rows, lists)
+  long long q_pos0, e_base;
+  int Cq, E, D, KC, lists, tiles_per_list;
+  float scale;
+};
+
+__global__ void __launch_bounds__(THREADS, 1)
+lmk_screen_kernel(const __grid_constant__ ScreenParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  float* score = reinterpret_cast<float*>(smem + OFF_SCORE);
+  float* norm = reinterpret_cast<float*>(smem + OFF_NORM);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + NUM_BARS);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + NUM_BARS + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int list = blockIdx.x, t0 = blockIdx.y * BM, n = blockIdx.z;
+  const int rows = min(BM, p.Cq - t0), ksteps = p.D / BK;
+  // tiles of this list that some row of the block can see
+  const int tiles_all = (p.E + BN - 1) / BN, first = list * p.tiles_per_list;
+  const long long seen = p.q_pos0 + t0 + rows - 1 - p.e_base;             // landmarks visible to the last row
+  const int last = (int)min((long long)min(tiles_all, first + p.tiles_per_list), seen <= 0 ? 0ll : (seen + BN - 1) / BN);
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < STAGES; ++i) { mbar_init(&bars[FULL + i], 1); mbar_init(&bars[EMPTY + i], 1 + NORM_WARPS); }
+    mbar_init(&bars[ACC_FULL], 1);
+    mbar_init(&bars[ACC_EMPTY], WORKERS);
+    *abort_flag = 0;
+    fence_barrier_init();
+  }
+  if (warp == WORKERS + 1) { tmem_alloc(tmem_slot, 64); tmem_relinquish(); }
+  if (warp == WORKERS && lane == 0) { tma_prefetch_desc(&p.tm_q); tma_prefetch_desc(&p.tm_k); }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  pdl_trigger();
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp == WORKERS) {
+    if (lane == 0) {
+      uint32_t it = 0;
+      bool ok = true;
+      for (int t = first; t < last && ok; ++t)
+        for (int ks = 0; ks < ksteps; ++ks, ++it) {
+          const uint32_t st = it % STAGES;
+          ok = mbar_wait_bounded(&bars[EMPTY + st], ((it / STAGES) & 1) ^ 1, abort_flag);
+          if (!ok) break;
+          mbar_arrive_expect_tx(&bars[FULL + st], STAGE_BYTES);
+          tma_load_3d(smem + st * STAGE_BYTES, &p.tm_q, &bars[FULL + st], ks * BK, t0, n);
+          tma_load_3d(smem + st * STAGE_BYTES + A_BYTES, &p.tm_k, &bars[FULL + st], ks * BK, t * BN, n);
+        }
+      if (*abort_flag)          // nothing may land in shared memory after the block has gone
+        for (uint32_t back = 0; back < (uint32_t)STAGES && back < it; ++back) {
+          const uint32_t g = it - 1 - back;
+          for (int i = 0; i < (1 << 20); ++i)
+            if (mbar_try_wait(&bars[FULL + g % STAGES], (g / STAGES) & 1)) break;
+        }
+    }
+  } else if (warp == WORKERS + 1) {
+    uint32_t it = 0, tile = 0;
+    bool ok = true;
+    for (int t = first; t < last && ok; ++t, ++tile) {
+      ok = mbar_wait_warp(&bars[ACC_EMPTY], (tile & 1) ^ 1, abort_flag, lane);
+      for (int ks = 0; ks < ksteps && ok; ++ks, ++it) {
+        const uint32_t st = it % STAGES;
+        ok = mbar_wait_warp(&bars[FULL + st], (it / STAGES) & 1, abort_flag, lane);
+        if (!ok) break;
+        tc_fence_after();
+        const uint64_t da = umma_desc_sw128(smem_u32(smem + st * STAGE_BYTES)), db = umma_desc_sw128(smem_u32(smem + st * STAGE_BYTES + A_BYTES));
+#pragma unroll
+        for (int kk = 0; kk < BK / 16; ++kk) umma_bf16_ss_elect(tmem, da + kk * 2, db + kk * 2, IDESC, (uint32_t)(ks > 0 || kk > 0));
+        umma_commit_elect(&bars[EMPTY + st]);
+      }
+      if (ok) umma_commit_elect(&bars[ACC_FULL]);
+    }
+  } else {
+    bool ok = true;
+    uint32_t it = 0, tile = 0;
+    float eps_max = 0.f;                                     // of this warp's rows: row i of the warp in lane i
+    for (int t = first; t < last && ok; ++t, ++tile) {
+      if (warp < NORM_WARPS) {
+        float ss = 0.f;
+        for (int ks = 0; ks < ksteps && ok; ++ks, ++it) {
+          const uint32_t st = it % STAGES;
+          ok = mbar_wait_warp(&bars[FULL + st], (it / STAGES) & 1, abort_flag, lane);
+          if (!ok) break;
+          const uint8_t* row = smem + st * STAGE_BYTES + threadIdx.x * 128;        // A rows, then B rows right behind them
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            float f[8];
+            unpack8(*reinterpret_cast<const uint4*>(row + ((c ^ (lane & 7)) << 4)), f);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) ss = fmaf(f[i], f[i], ss);
+          }
+          mbar_arrive_warp(&bars[EMPTY + st], lane);
+        }
+        norm[threadIdx.x] = ss;
+      }
+      if (ok) ok = mbar_wait_warp(&bars[ACC_FULL], tile & 1, abort_flag, lane);
+      if (ok) {
+        tc_fence_after();
+        const int quad = warp & 3, c0 = (warp >> 2) * 16, r = quad * 32 + lane;
+        uint32_t v[16];
+        tmem_ld_32x32b_x16(tmem + ((uint32_t)(quad * 32) << 16) + c0, v);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 16; ++i) score[r * LDS_ROW + c0 + i] = __uint_as_float(v[i]) * p.scale;
+        tc_fence_before();
+        mbar_arrive_warp(&bars[ACC_EMPTY], lane);
+      }
+      // one decision for all workers: whether any of them gave up
+      int failed = !ok || *abort_flag;
+      asm volatile(
+          "{\n\t.reg .pred p, q;\n\t"
+          "setp.ne.s32 q, %0, 0;\n\t"
+          "barrier.cta.red.or.pred p, 1, %1, q;\n\t"
+          "selp.s32 %0, 1, 0, p;\n\t}"
+          : "+r"(failed)
+          : "r"(WORKERS * 32)
+          : "memory");
+      if (failed) { ok = false; break; }
+      const float kn = fmaxf(norm[BM + lane], norm[BM + 32 + lane]);
+      const float kmax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(kn)));     // squared norms: never negative
+      // two rows of the warp at a time: a round is a chain of dependent warp-wide operations
+      for (int i = 0; i < BM / WORKERS; i += 2) {
+        if (warp + i * WORKERS >= rows) break;
+        unsigned o0[2], o1[2];
+        unsigned long long run[2], mine[2] = {0ull, 0ull};
+        unsigned long long* dst[2];
+        bool live[2];
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          const int lr = warp + (i + x) * WORKERS, row = t0 + lr;
+          const long long grow = (long long)n * p.Cq + row;
+          live[x] = lr < rows;
+          if (lane == i + x && live[x]) eps_max = fmaxf(eps_max, BOUND * p.scale * sqrtf(norm[lr]) * sqrtf(kmax) * 1.001f);
+          float s0 = score[lr * LDS_ROW + lane], s1 = score[lr * LDS_ROW + 32 + lane];
+          const int e0 = t * BN + lane, e1 = e0 + 32;
+          const bool v0 = live[x] && e0 < p.E && p.e_base + e0 < p.q_pos0 + row, v1 = live[x] && e1 < p.E && p.e_base + e1 < p.q_pos0 + row;
+          if (p.noise) {
+            if (v0) s0 += p.noise[grow * p.E + e0];
+            if (v1) s1 += p.noise[grow * p.E + e1];
+          }
+          o0[x] = v0 ? orderable(s0) : 0u;
+          o1[x] = v1 ? orderable(s1) : 0u;
+          dst[x] = p.part + (grow * p.lists + list) * p.KC;
+          run[x] = live[x] && t > first && lane < p.KC ? dst[x][lane] : 0ull;         // the list so far (this warp wrote it)
+        }
+#pragma unroll 1
+        for (int k = 0; k < p.KC; ++k) {
+#pragma unroll
+          for (int x = 0; x < 2; ++x) {
+            const unsigned rh = (unsigned)(run[x] >> 32);
+            const unsigned m = __reduce_max_sync(0xffffffffu, max(rh, max(o0[x], o1[x])));
+            const unsigned br = __ballot_sync(0xffffffffu, rh == m), b0 = __ballot_sync(0xffffffffu, o0[x] == m),
+                           b1 = __ballot_sync(0xffffffffu, o1[x] == m);
+            // equal scores: the lower id first, so the list's own entries, then the tile's two halves
+            const unsigned from = br ? br : b0 ? b0 : b1;
+            const int src = __ffs(from) - 1;
+            unsigned long long best = __shfl_sync(0xffffffffu, run[x], src);
+            if (!br) best = ((unsigned long long)m << 32) | (0xffffffffu - (unsigned)(p.e_base + t * BN + src + (b0 ? 0 : 32)));
+            if (lane == src) { if (br) run[x] = 0ull; else if (b0) o0[x] = 0u; else o1[x] = 0u; }
+            if (lane == k) mine[x] = m ? best : 0ull;
+          }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+          if (live[x] && lane < p.KC) dst[x][lane] = mine[x];
+      }
+      asm volatile("bar.sync 1, %0;" ::"r"(WORKERS * 32) : "memory");     // scores and norms are free for the next tile
+    }
+    for (int lr = warp, i = 0; lr < rows; lr += WORKERS, ++i) {
+      const long long at = ((long long)n * p.Cq + t0 + lr) * p.lists + list;
+      if (lane == i) p.eps[at] = ok ? eps_max : INFINITY;      // a wait ran out: the merge scans the row itself
+      if (last <= first && lane < p.KC) p.part[at * p.KC + lane] = 0ull;
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == WORKERS + 1) tmem_dealloc(tmem, 64);
+}
+
+struct SettleParams {
+  FinalParams fin;
+  const unsigned long long* part;
+  const float* eps;
+  const float* noise;
+  long long q_pos0;
+  int KC, lists, E;
+};
+
+constexpr int SETTLE_WARPS = 8;
+
+// One warp per row: the candidates that can win get their exact scores and are put in order.
+template <int NP>
+__global__ void __launch_bounds__(SETTLE_WARPS * 32)
+lmk_settle_kernel(const __grid_constant__ SettleParams p) {
+  __shared__ unsigned long long won_key[SETTLE_WARPS][32];
+  __shared__ float won_score[SETTLE_WARPS][32];
+  const FinalParams& f = p.fin;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long row = (long long)blockIdx.x * SETTLE_WARPS + warp;
+  pdl_wait();
+  if (row >= f.R) return;
+  const long long n = row / f.Cq, r = row % f.Cq;
+  const __nv_bfloat16* q = f.lq + n * f.qbs + r * f.qrs;
+  const __nv_bfloat16* kb = f.lk + n * f.kbs;
+  const int pieces = f.D >> 3;
+  const unsigned long long* src = p.part + (row * p.lists + lane) * p.KC;
+  const bool have = lane < p.lists;
+  unsigned long long head = have ? src[0] : 0ull, next = have ? src[1] : 0ull, c0 = 0ull, c1 = 0ull;
+  const unsigned eb = __reduce_max_sync(0xffffffffu, have ? __float_as_uint(p.eps[row * p.lists + lane]) : 0u);
+  const float eps = __uint_as_float(eb);
+  bool slow = !(eps < 1e30f);
+  float line = -INFINITY;
+  int at = 1, count = 0;
+  while (!slow) {
+    const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(head >> 32));
+    if (hi == 0u) break;
+    const float s = from_orderable(hi);
+    if (count >= f.K && s < line) break;
+    if (count == 64 || !(fabsf(s) < 1e30f)) { slow = true; break; }
+    const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(head >> 32) == hi ? (unsigned)head : 0u);
+    const unsigned long long best = ((unsigned long long)hi << 32) | lo;
+    if (lane == (count & 31)) { if (count < 32) c0 = best; else c1 = best; }
+    ++count;
+    if (count == f.K) line = s - 2.0f * eps - fabsf(s) * 4.8e-7f;           // 2^-21: the roundings of scale and noise
+    bool spent = false;
+    if (head == best) { head = next; ++at; next = at < p.KC ? src[at] : 0ull; spent = at > p.KC; }
+    slow = __any_sync(0xffffffffu, spent);                                   // a full list used up: it may hide more
+  }
+  const bool want_sel = p.noise != nullptr;
+  if (slow) {
+    unsigned long long m = 0ull, th = 0ull;
+    const long long seen = min((long long)p.E, p.q_pos0 + r - f.e_base);
+    for (long long e = 0; e < seen; ++e) {
+      float s = exact_dot(q, kb + e * f.krs, pieces, lane) * f.scale;
+      if (want_sel) s += p.noise[row * p.E + e];
+      const unsigned long long key = make_key(s, (unsigned)(f.e_base + e));
+      if (key > th) {
+        list_insert(m, key, lane);
+        th = __shfl_sync(0xffffffffu, m, f.K - 1);
+      }
+    }
+    float clean = from_orderable((unsigned)(m >> 32));
+    if (want_sel)
+      for (int i = 0; i < f.K; ++i) {
+        const unsigned long long key = __shfl_sync(0xffffffffu, m, i);
+        const long long e = key ? (long long)(0xffffffffu - (unsigned)key) - f.e_base : 0;
+        const float s = exact_dot(q, kb + e * f.krs, pieces, lane) * f.scale;
+        if (lane == i) clean = s;
+      }
+    emit_scored(f, row, m, clean, lane);
+    return;
+  }
+  // exact scores; the rows of four candidates are requested together
+  unsigned long long k0 = 0ull, k1 = 0ull;
+  float s0 = 0.f, s1 = 0.f;
+  uint4 qv[NP];
+#pragma unroll
+  for (int pp = 0; pp < NP; ++pp) qv[pp] = lane + 32 * pp < pieces ? *reinterpret_cast<const uint4*>(q + (lane + 32 * pp) * 8) : make_uint4(0, 0, 0, 0);
+  for (int i0 = 0; i0 < count; i0 += 4) {
+    uint4 kv[4][NP];
+    unsigned id[4];
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      const int i = min(i0 + x, count - 1);
+      id[x] = 0xffffffffu - (unsigned)__shfl_sync(0xffffffffu, i < 32 ? c0 : c1, i & 31);
+      const __nv_bfloat16* kr = kb + ((long long)id[x] - f.e_base) * f.krs;
+#pragma unroll
+      for (int pp = 0; pp < NP; ++pp)
+        kv[x][pp] = lane + 32 * pp < pieces ? *reinterpret_cast<const uint4*>(kr + (lane + 32 * pp) * 8) : make_uint4(0, 0, 0, 0);
+    }
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      float acc = 0.f;
+#pragma unroll
+      for (int pp = 0; pp < NP; ++pp) {                      // absent pieces add 0 * 0: the sums never are -0
+        float af[8], bf[8];
+        unpack8(qv[pp], af);
+        unpack8(kv[x][pp], bf);
+#pragma unroll
+        for (int jj = 0; jj < 8; ++jj) acc = fmaf(af[jj], bf[jj], acc);
+      }
+#pragma unroll
+      for (int of = 16; of > 0; of >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, of);
+      const float s = acc * f.scale;
+      const int i = i0 + x;
+      if (i < count && lane == (i & 31)) {
+        const unsigned long long key = make_key(want_sel ? s + p.noise[row * p.E + (long long)id[x] - f.e_base] : s, id[x]);
+        if (i < 32) { k0 = key; s0 = s; } else { k1 = key; s1 = s; }
+      }
+    }
+  }
+  int r0 = 0, r1 = 0;
+  for (int i = 0; i < count; ++i) {
+    const unsigned long long o = __shfl_sync(0xffffffffu, i < 32 ? k0 : k1, i & 31);
+    r0 += o > k0;
+    r1 += o > k1;
+  }
+  won_key[warp][lane] = 0ull;
+  __syncwarp();
+  if (k0 && r0 < 32) { won_key[warp][r0] = k0; won_score[warp][r0] = s0; }
+  if (k1 && r1 < 32) { won_key[warp][r1] = k1; won_score[warp][r1] = s1; }
+  __syncwarp();
+  emit_scored(f, row, lane < f.K ? won_key[warp][lane] : 0ull, won_score[warp][lane], lane);
+}
+
+// Landmark ranges per row: enough CTAs to fill the GPU, at most one list per lane of the merging warp.
+int screen_lists(const LmkTopkArgs& a, int sms, int* tiles_per_list) {
+  const int tiles = (a.E + BN - 1) / BN;
+  const long long blocks = (long long)a.N * ((a.Cq + BM - 1) / BM);
+  long long lists = (2ll * sms + blocks - 1) / blocks;
+  if (lists > MAX_LISTS) lists = MAX_LISTS;
+  if (lists > tiles) lists = tiles;
+  if (lists < 1) lists = 1;
+  *tiles_per_list = (int)((tiles + lists - 1) / lists);
+  return (tiles + *tiles_per_list - 1) / *tiles_per_list;
+}
+
+}  // namespace
+
+// float32 scores without per-head lists, whole 64-element K steps, room for K + 4 candidates in a warp; below a few thousand pairs
+// per sequence the row scan is as fast.
+bool lmk_screen_applies(const LmkTopkArgs& a) {
+  return a.head_dim == 0 && a.score_round == 0 && a.splits == 0 && a.D % BK == 0 && a.K <= 32 - EXTRA && a.Cq >= 64 && a.E >= 64 &&
+         (a.N == 1 || (a.q_batch_stride > 0 && a.k_batch_stride > 0)) && a.q_row_stride > 0 && a.k_row_stride > 0;
+}
+
+size_t lmk_screen_workspace_bytes(const LmkTopkArgs& a, int sms) {
+  int tpl;
+  const size_t lists = (size_t)screen_lists(a, sms, &tpl), rows = (size_t)a.N * a.Cq;
+  return align_up(rows * lists * (a.K + EXTRA) * 8, 256) + align_up(rows * lists * 4, 256);
+}
+
+int launch_lmk_screen(const LmkTopkArgs& a, void* scratch, int sms, const FinalParams& fin, cudaStream_t stream) {
+  ScreenParams p;
+  int rc;
+  if ((rc = make_rows_map(&p.tm_q, a.lmk_q, a.N, a.Cq, a.D, a.q_row_stride, a.q_batch_stride, BM)) ||
+      (rc = make_rows_map(&p.tm_k, a.lmk_k, a.N, a.E, a.D, a.k_row_stride, a.k_batch_stride, BN)))
+    return rc;
+  p.KC = a.K + EXTRA;
+  p.lists = screen_lists(a, sms, &p.tiles_per_list);
+  const size_t rows = (size_t)a.N * a.Cq;
+  p.part = static_cast<unsigned long long*>(scratch);
+  p.eps = reinterpret_cast<float*>(static_cast<char*>(scratch) + align_up(rows * p.lists * p.KC * 8, 256));
+  p.noise = a.noise; p.q_pos0 = a.q_pos0; p.e_base = a.e_base;
+  p.Cq = a.Cq; p.E = a.E; p.D = a.D; p.scale = fin.scale;
+  GCA_CUDA_CHECK(cudaFuncSetAttribute(lmk_screen_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+  lmk_screen_kernel<<<dim3((unsigned)p.lists, (unsigned)((a.Cq + BM - 1) / BM), (unsigned)a.N), THREADS, SMEM_BYTES, stream>>>(p);
+  GCA_CUDA_CHECK(cudaGetLastError());
+  SettleParams sp;
+  sp.fin = fin; sp.part = p.part; sp.eps = p.eps; sp.noise = a.noise; sp.q_pos0 = a.q_pos0; sp.KC = p.KC; sp.lists = p.lists; sp.E = a.E;
+  const dim3 grid((unsigned)((rows + SETTLE_WARPS - 1) / SETTLE_WARPS)), block(SETTLE_WARPS * 32);
+  switch ((a.D + 255) / 256) {
+    case 1: return (int)launch_dependent(lmk_settle_kernel<1>, grid, block, 0, stream, sp);
+    case 2: return (int)launch_dependent(lmk_settle_kernel<2>, grid, block, 0, stream, sp);
+    case 3: return (int)launch_dependent(lmk_settle_kernel<3>, grid, block, 0, stream, sp);
+    case 4: return (int)launch_dependent(lmk_settle_kernel<4>, grid, block, 0, stream, sp);
+    default: return GCA_ERR_SHAPE;
+  }
+}
+
+}  // namespace gca

@@ -15,42 +15,20 @@
 // (lane i holds the i-th best).  Blocks write their lists to a scratch buffer; a second,
 // tiny kernel merges the lists of all blocks of a row and emits indices, noise-free scores,
 // softmax weights and the number of valid slots.
-#include "gca_common.cuh"
+#include "lmk_common.cuh"
+
+namespace gca {
+// lmk_tc_sm100.cu: many query rows per sequence
+bool lmk_screen_applies(const LmkTopkArgs& a);
+size_t lmk_screen_workspace_bytes(const LmkTopkArgs& a, int sms);
+int launch_lmk_screen(const LmkTopkArgs& a, void* scratch, int sms, const FinalParams& fin, cudaStream_t stream);
+}  // namespace gca
 
 namespace gca {
 
 namespace {
 
 constexpr int SCAN_WARPS = 8;
-constexpr int MAXK = 32;
-
-__device__ __forceinline__ unsigned orderable(float s) {
-  const unsigned u = __float_as_uint(s);
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-__device__ __forceinline__ float from_orderable(unsigned o) {
-  return __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o);
-}
-__device__ __forceinline__ unsigned long long make_key(float score, unsigned gidx) {
-  return ((unsigned long long)orderable(score) << 32) | (unsigned long long)(0xffffffffu - gidx);
-}
-__device__ __forceinline__ float round_bf16(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
-
-// Insert `key` into the descending list held one element per lane.  Warp-uniform call.
-__device__ __forceinline__ void list_insert(unsigned long long& mine, unsigned long long key, int lane) {
-  const bool lower = mine < key;
-  const unsigned long long up = __shfl_up_sync(0xffffffffu, mine, 1);
-  const int lower_prev = __shfl_up_sync(0xffffffffu, (int)lower, 1);
-  if (lower) mine = (lane > 0 && lower_prev) ? up : key;
-}
-
-__device__ __forceinline__ void unpack8(const uint4& v, float f[8]) {
-  f[0] = __uint_as_float(v.x << 16); f[1] = __uint_as_float(v.x & 0xffff0000u);
-  f[2] = __uint_as_float(v.y << 16); f[3] = __uint_as_float(v.y & 0xffff0000u);
-  f[4] = __uint_as_float(v.z << 16); f[5] = __uint_as_float(v.z & 0xffff0000u);
-  f[6] = __uint_as_float(v.w << 16); f[7] = __uint_as_float(v.w & 0xffff0000u);
-}
-
 struct ScanParams {
   const __nv_bfloat16* lq;
   const __nv_bfloat16* lk;
@@ -71,6 +49,7 @@ __global__ void __launch_bounds__(SCAN_WARPS * 32)
 lmk_scan_kernel(ScanParams p) {
   constexpr int NL = PER_HEAD ? NP * 4 : TQ;
   __shared__ unsigned long long sL[SCAN_WARPS][NL][MAXK];
+  pdl_trigger();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int split = blockIdx.x, t0 = blockIdx.y * TQ, n = blockIdx.z;
   const int pieces = p.D >> 3;
@@ -201,22 +180,6 @@ lmk_scan_kernel(ScanParams p) {
   }
 }
 
-struct FinalParams {
-  const unsigned long long* keys;   // (R, P)
-  unsigned long long* out_keys;
-  int32_t* out_indices;
-  float* out_scores;
-  float* out_weights;
-  int32_t* out_nvalid;
-  // optional recompute of noise-free scores (per-sequence mode with noise)
-  const __nv_bfloat16* lq;
-  const __nv_bfloat16* lk;
-  long long qbs, qrs, kbs, krs, e_base;
-  int Cq, D, score_round;
-  float scale;
-  int R, P, K;
-};
-
 constexpr int FIN_WARPS = 8;
 
 // The merge of one row's P candidates (src) by one block of FIN_WARPS warps (sL: FIN_WARPS x MAXK
@@ -252,50 +215,76 @@ __device__ void finalize_row(const FinalParams& p, long long row, const unsigned
       list_insert(m, key, lane);
       th = __shfl_sync(0xffffffffu, m, p.K - 1);
     }
-  const bool valid = lane < p.K && m != 0ull;
-  const int idx = valid ? (int)(0xffffffffu - (unsigned)(m & 0xffffffffull)) : -1;
-  float score = valid ? from_orderable((unsigned)(m >> 32)) : -INFINITY;
-  if (p.lq) {
-    // selection used noisy scores: recompute the noise-free score of every winner in the
-    // same fixed order as the scan
-    const long long n = row / p.Cq, r = row % p.Cq;
-    const int pieces = p.D >> 3;
-    for (int i = 0; i < p.K; ++i) {
-      const int wi = __shfl_sync(0xffffffffu, idx, i);
-      if (wi < 0) continue;
-      float acc = 0.f;
-      for (int c = lane; c < pieces; c += 32) {
-        const uint4 a = *reinterpret_cast<const uint4*>(p.lq + n * p.qbs + r * p.qrs + c * 8);
-        const uint4 b = *reinterpret_cast<const uint4*>(p.lk + n * p.kbs + (wi - p.e_base) * p.krs + c * 8);
-        float af[8], bf[8];
-        unpack8(a, af); unpack8(b, bf);
-#pragma unroll
-        for (int jj = 0; jj < 8; ++jj) acc = fmaf(af[jj], bf[jj], acc);
-      }
-#pragma unroll
-      for (int of = 16; of > 0; of >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, of);
-      const float s = p.score_round ? round_bf16(round_bf16(acc) * p.scale) : acc * p.scale;
-      if (lane == i) score = s;
+  emit_row(p, row, m, lane);
+}
+
+// The scan's lists of a row merged by one warp (up to 32 lists; eight rows per block): lane l stands at the head of list
+// l, and K times the best head is taken by a warp-wide maximum and its list moves on.
+__global__ void __launch_bounds__(FIN_WARPS * 32)
+lmk_merge_rows_kernel(FinalParams p) {
+  const int lane = threadIdx.x & 31;
+  const long long row = (long long)blockIdx.x * FIN_WARPS + (threadIdx.x >> 5);
+  pdl_wait();
+  if (row >= p.R) return;
+  const unsigned long long* src = p.keys + row * p.P + (long long)lane * p.K;
+  unsigned long long head = lane < p.lists ? src[0] : 0ull, next = lane < p.lists && p.K > 1 ? src[1] : 0ull, mine = 0ull;
+  int at = 1;
+  for (int i = 0; i < p.K; ++i) {
+    const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(head >> 32));
+    if (hi == 0u) break;
+    const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(head >> 32) == hi ? (unsigned)head : 0u);
+    const unsigned long long best = ((unsigned long long)hi << 32) | lo;
+    if (lane == i) mine = best;
+    if (head == best) { head = next; ++at; next = at < p.K ? src[at] : 0ull; }
+  }
+  emit_row(p, row, mine, lane);
+}
+
+// Many lists per row (a long cache scanned by every SM): one block per row, no serial insertion.  An entry e of a
+// list can be among the K best only if fewer than K - e list heads are better than its own; so the heads are ranked by counting,
+// the K best lists are lined up by rank, and their K (K + 1) / 2 possible entries are ranked by counting again.
+// 296 lists, K = 8: 12.9 us of warp-serial insertions before.
+constexpr int RANK_LISTS = 1024;
+
+__global__ void __launch_bounds__(FIN_WARPS * 32)
+lmk_rank_merge_kernel(FinalParams p) {
+  __shared__ __align__(16) unsigned long long heads[RANK_LISTS];
+  __shared__ int by_rank[MAXK];
+  __shared__ unsigned long long cand[MAXK * (MAXK + 1) / 2 + 1], best[MAXK];
+  const int tid = threadIdx.x, lists = p.lists, K = p.K;
+  const int padded = (lists + 1) & ~1;
+  const unsigned long long* src = p.keys + (long long)blockIdx.x * p.P;
+  if (tid < MAXK) { by_rank[tid] = -1; best[tid] = 0ull; }
+  pdl_wait();
+  for (int i = tid; i < padded; i += FIN_WARPS * 32) heads[i] = i < lists ? src[(long long)i * K] : 0ull;
+  __syncthreads();
+  for (int i = tid; i < lists; i += FIN_WARPS * 32) {
+    const unsigned long long mine = heads[i];
+    if (mine == 0ull) continue;
+    int rank = 0;
+    for (int j = 0; j < padded; j += 2) {
+      const ulonglong2 h = *reinterpret_cast<const ulonglong2*>(&heads[j]);
+      rank += (h.x > mine) + (h.y > mine);
     }
+    if (rank < K) by_rank[rank] = i;                      // keys are distinct: one list per rank
   }
-  // softmax over the valid slots
-  float mx = valid ? score : -INFINITY;
-#pragma unroll
-  for (int of = 16; of > 0; of >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, of));
-  float ex = valid ? expf(score - mx) : 0.f;
-  float sum = ex;
-#pragma unroll
-  for (int of = 16; of > 0; of >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, of);
-  const float wgt = (valid && sum > 0.f) ? ex / sum : 0.f;
-  const unsigned nv = __popc(__ballot_sync(0xffffffffu, valid));
-  if (lane < p.K) {
-    const long long o = row * p.K + lane;
-    if (p.out_keys) p.out_keys[o] = m;
-    if (p.out_indices) p.out_indices[o] = idx;
-    if (p.out_scores) p.out_scores[o] = score;
-    if (p.out_weights) p.out_weights[o] = wgt;
+  __syncthreads();
+  // candidate (r, e), r + e < K, at position e of the list of rank r
+  const int total = K * (K + 1) / 2;
+  for (int i = tid; i < K * K; i += FIN_WARPS * 32) {
+    const int r = i / K, e = i - r * K;
+    if (r + e < K) cand[r * K - r * (r - 1) / 2 + e] = by_rank[r] >= 0 ? src[(long long)by_rank[r] * K + e] : 0ull;
   }
-  if (lane == 0 && p.out_nvalid) p.out_nvalid[row] = (int)nv;
+  __syncthreads();
+  for (int i = tid; i < total; i += FIN_WARPS * 32) {
+    const unsigned long long mine = cand[i];
+    if (mine == 0ull) continue;
+    int rank = 0;
+    for (int j = 0; j < total; ++j) rank += cand[j] > mine;
+    if (rank < K) best[rank] = mine;
+  }
+  __syncthreads();
+  if (tid < 32) emit_row(p, blockIdx.x, tid < K ? best[tid] : 0ull, tid);
 }
 
 __global__ void __launch_bounds__(FIN_WARPS * 32)
@@ -398,9 +387,13 @@ lmk_exchange_kernel(ExchangeParams p) {
   if (tid == 0) epochs[row] = e;
 }
 
+int pick_tq(const LmkTopkArgs& a) { return (a.head_dim > 0 || a.Cq < 4) ? 1 : 4; }
+
+}  // namespace
+
 // Two CTAs per SM when the query tile count alone does not fill the GPU.
-int choose_splits(const LmkTopkArgs& a, int tq, int sms) {
-  if (a.splits > 0) return a.splits;
+int scan_splits(const LmkTopkArgs& a, int sms) {
+  const int tq = pick_tq(a);
   const long long blocks = (long long)a.N * ((a.Cq + tq - 1) / tq);
   long long s = (2 * (long long)sms + blocks - 1) / blocks;
   const long long max_s = (a.E + 255) / 256;              // keep at least 256 rows per split
@@ -409,7 +402,9 @@ int choose_splits(const LmkTopkArgs& a, int tq, int sms) {
   return (int)s;
 }
 
-int pick_tq(const LmkTopkArgs& a) { return (a.head_dim > 0 || a.Cq < 4) ? 1 : 4; }
+namespace {
+
+int choose_splits(const LmkTopkArgs& a, int sms) { return a.splits > 0 ? a.splits : scan_splits(a, sms); }
 
 template <int NP>
 void launch_scan(const ScanParams& sp, int tq, bool per_head, dim3 grid, cudaStream_t stream) {
@@ -426,31 +421,36 @@ size_t lmk_topk_rows(const LmkTopkArgs& a) {
 }
 
 size_t lmk_topk_workspace_bytes_impl(const LmkTopkArgs& a, int sms) {
-  const int splits = choose_splits(a, pick_tq(a), sms);
-  return align_up(lmk_topk_rows(a) * (size_t)splits * a.K * sizeof(unsigned long long), 256);
+  if (lmk_screen_applies(a)) return lmk_screen_workspace_bytes(a, sms);
+  return align_up(lmk_topk_rows(a) * (size_t)choose_splits(a, sms) * a.K * sizeof(unsigned long long), 256);
 }
 
-// Scan + finalize on caller-provided scratch.  `scratch` must hold
+// Scan + merge on caller-provided scratch.  `scratch` must hold
 // lmk_topk_workspace_bytes_impl(a, sms) bytes.
 int launch_lmk_score_topk(const LmkTopkArgs& a, void* scratch, int sms, cudaStream_t stream) {
+  const size_t rows = lmk_topk_rows(a);
+  if (rows == 0) return 0;
   const bool per_head = a.head_dim > 0;
-  const int H = per_head ? a.D / a.head_dim : 1;
-  const int tq = pick_tq(a);
-  const int splits = choose_splits(a, tq, sms);
+  const float scale = (float)(1.0 / sqrt((double)(per_head ? a.head_dim : a.D)));
+  FinalParams fp;
+  fp.keys = (unsigned long long*)scratch; fp.out_keys = (unsigned long long*)a.out_keys; fp.out_indices = a.out_indices;
+  fp.out_scores = a.out_scores; fp.out_weights = a.out_weights; fp.out_nvalid = a.out_nvalid;
+  fp.lq = (const __nv_bfloat16*)a.lmk_q; fp.lk = (const __nv_bfloat16*)a.lmk_k;
+  fp.qbs = a.q_batch_stride; fp.qrs = a.q_row_stride; fp.kbs = a.k_batch_stride; fp.krs = a.k_row_stride; fp.e_base = a.e_base;
+  fp.Cq = a.Cq; fp.D = a.D; fp.score_round = a.score_round; fp.scale = scale;
+  fp.R = (int)rows; fp.P = 0; fp.K = a.K; fp.lists = 0;
+  if (lmk_screen_applies(a)) return launch_lmk_screen(a, scratch, sms, fp, stream);
+  const int tq = pick_tq(a), splits = choose_splits(a, sms);
   ScanParams sp;
-  sp.lq = (const __nv_bfloat16*)a.lmk_q; sp.lk = (const __nv_bfloat16*)a.lmk_k; sp.noise = a.noise;
+  sp.lq = fp.lq; sp.lk = fp.lk; sp.noise = a.noise;
   sp.part = (unsigned long long*)scratch;
   sp.qbs = a.q_batch_stride; sp.qrs = a.q_row_stride; sp.kbs = a.k_batch_stride; sp.krs = a.k_row_stride;
   sp.q_pos0 = a.q_pos0; sp.e_base = a.e_base;
-  sp.N = a.N; sp.Cq = a.Cq; sp.E = a.E; sp.D = a.D; sp.K = a.K; sp.H = H;
+  sp.N = a.N; sp.Cq = a.Cq; sp.E = a.E; sp.D = a.D; sp.K = a.K; sp.H = per_head ? a.D / a.head_dim : 1;
   sp.splits = splits; sp.e_per_split = (a.E + splits - 1) / splits;
-  sp.score_round = a.score_round;
-  sp.scale = (float)(1.0 / sqrt((double)(per_head ? a.head_dim : a.D)));
-  const size_t rows = lmk_topk_rows(a);
-  if (rows == 0) return 0;
-  dim3 grid((unsigned)splits, (unsigned)((a.Cq + tq - 1) / tq), (unsigned)a.N);
-  const int np = (a.D + 255) / 256;
-  switch (np) {
+  sp.score_round = a.score_round; sp.scale = scale;
+  const dim3 grid((unsigned)splits, (unsigned)((a.Cq + tq - 1) / tq), (unsigned)a.N);
+  switch ((a.D + 255) / 256) {
     case 1: launch_scan<1>(sp, tq, per_head, grid, stream); break;
     case 2: launch_scan<2>(sp, tq, per_head, grid, stream); break;
     case 3: launch_scan<3>(sp, tq, per_head, grid, stream); break;
@@ -458,14 +458,12 @@ int launch_lmk_score_topk(const LmkTopkArgs& a, void* scratch, int sms, cudaStre
     default: return GCA_ERR_SHAPE;
   }
   GCA_CUDA_CHECK(cudaGetLastError());
-  FinalParams fp;
-  fp.keys = sp.part; fp.out_keys = (unsigned long long*)a.out_keys; fp.out_indices = a.out_indices; fp.out_scores = a.out_scores;
-  fp.out_weights = a.out_weights; fp.out_nvalid = a.out_nvalid;
-  const bool recompute = a.noise != nullptr && !per_head;
-  fp.lq = recompute ? sp.lq : nullptr; fp.lk = sp.lk;
-  fp.qbs = sp.qbs; fp.qrs = sp.qrs; fp.kbs = sp.kbs; fp.krs = sp.krs; fp.e_base = a.e_base;
-  fp.Cq = a.Cq; fp.D = a.D; fp.score_round = a.score_round; fp.scale = sp.scale;
-  fp.R = (int)rows; fp.P = splits * a.K; fp.K = a.K;
+  if (a.noise == nullptr || per_head) fp.lq = nullptr;          // the keys hold the noise-free scores
+  fp.P = splits * a.K; fp.lists = splits;
+  // a warp per row up to 32 lists, a block per row beyond
+  if (splits <= 32)
+    return (int)launch_dependent(lmk_merge_rows_kernel, dim3((unsigned)((rows + FIN_WARPS - 1) / FIN_WARPS)), dim3(FIN_WARPS * 32), 0, stream, fp);
+  if (splits <= RANK_LISTS) return (int)launch_dependent(lmk_rank_merge_kernel, dim3((unsigned)rows), dim3(FIN_WARPS * 32), 0, stream, fp);
   lmk_finalize_kernel<<<(unsigned)rows, FIN_WARPS * 32, 0, stream>>>(fp);
   return (int)cudaGetLastError();
 }
@@ -477,7 +475,7 @@ int launch_lmk_merge(const LmkMergeArgs& a, cudaStream_t stream) {
   fp.out_weights = a.out_weights; fp.out_nvalid = a.out_nvalid;
   fp.lq = nullptr; fp.lk = nullptr; fp.qbs = fp.qrs = fp.kbs = fp.krs = fp.e_base = 0;
   fp.Cq = 1; fp.D = 0; fp.score_round = 0; fp.scale = 1.f;
-  fp.R = a.R; fp.P = a.P; fp.K = a.K;
+  fp.R = a.R; fp.P = a.P; fp.K = a.K; fp.lists = 0;
   lmk_finalize_kernel<<<(unsigned)a.R, FIN_WARPS * 32, 0, stream>>>(fp);
   return (int)cudaGetLastError();
 }
@@ -543,7 +541,10 @@ extern "C" int lmk_score_topk_static(const LmkTopkArgs* a, void* stream) {
   gca::DeviceScope scope(a->lmk_k);        // the array of the GPU that holds the landmarks
   if (scope.rc) return scope.rc;
   const int sms = gca::sm_count(scope.dev);
-  // rows x splits x K candidate keys of 8 bytes must fit the built-in array
+  // rows x splits x K candidate keys of 8 bytes must fit the built-in array: the row scan needs the fewest lists
+  LmkTopkArgs b = *a;
+  if (b.splits == 0) b.splits = gca::scan_splits(b, sms);
+  a = &b;
   if (gca::lmk_topk_workspace_bytes_impl(*a, sms) > (size_t)LMK_STATIC_SCRATCH_BYTES) return GCA_ERR_STATIC_SCRATCH;
   void* scratch = nullptr;
   rc = gca::static_scratch_ptr(scope.dev, &scratch);
@@ -618,7 +619,7 @@ extern "C" int lmk_topk_exchange(const LmkExchangeArgs* a, void* stream) {
   fp.out_scores = a->out_scores; fp.out_weights = a->out_weights; fp.out_nvalid = a->out_nvalid;
   fp.lq = nullptr; fp.lk = nullptr; fp.qbs = fp.qrs = fp.kbs = fp.krs = fp.e_base = 0;
   fp.Cq = 1; fp.D = 0; fp.score_round = 0; fp.scale = 1.f;
-  fp.R = a->R; fp.P = a->world * gca::MAXK; fp.K = a->K;
+  fp.R = a->R; fp.P = a->world * gca::MAXK; fp.K = a->K; fp.lists = 0;
   gca::lmk_exchange_kernel<<<(unsigned)a->R, gca::FIN_WARPS * 32, 0, (cudaStream_t)stream>>>(p);
   return (int)cudaGetLastError();
 }

@@ -110,4 +110,36 @@ inline int make_tile_map_5d(CUtensorMap* map, const void* base, int d0, int d1, 
   return 0;
 }
 
+// 2-D bf16 matrix (rows x cols, row stride in elements), boxes of (64 columns x box_rows rows), 128-byte swizzle.
+inline int make_matrix_map(CUtensorMap* map, const void* base, long long rows, long long cols, long long row_stride, int box_rows) {
+  EncodeTiledFn fn = encode_tiled_fn();
+  if (!fn) return GCA_ERR_TMA;
+  if (row_stride % 8 != 0) return GCA_ERR_STRIDE;
+  const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  const cuuint64_t strides[1] = {(cuuint64_t)row_stride * 2};
+  const cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
+  const cuuint32_t estr[2] = {1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : GCA_ERR_TMA;
+}
+
+// The same for `batches` such matrices: (columns, rows, batches), boxes of 64 columns x box_rows rows of one batch.
+inline int make_rows_map(CUtensorMap* map, const void* base, long long batches, long long rows, long long cols, long long row_stride,
+                         long long batch_stride, int box_rows) {
+  EncodeTiledFn fn = encode_tiled_fn();
+  if (!fn) return GCA_ERR_TMA;
+  if (batches == 1) batch_stride = row_stride;            // never advanced; any legal stride does
+  if (row_stride % 8 != 0 || batch_stride % 8 != 0 || batch_stride <= 0) return GCA_ERR_STRIDE;
+  const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)batches};
+  const cuuint64_t strides[2] = {(cuuint64_t)row_stride * 2, (cuuint64_t)batch_stride * 2};
+  const cuuint32_t box[3] = {64, (cuuint32_t)box_rows, 1};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : GCA_ERR_TMA;
+}
+
 }  // namespace gca

@@ -100,11 +100,13 @@ def retrieve(lmk_q: torch.Tensor, chunk_kvs, topk: int, *, training: bool = Fals
     if training and noise is None:
         # Gumbel noise as in model/DRT.py:616-620
         noise = -torch.empty(lmk_q.shape[0], lmk_q.shape[1], past.shape[1], device=lmk_q.device).exponential_().log()
+    wants_grad = lmk_q.requires_grad or past.requires_grad
+    if not wants_grad or (lmk_q.dtype == past.dtype == torch.bfloat16):
+        # bf16 landmarks: the scan's own scores are what the weights are made of, and their gradient is one kernel
+        idx, w, *full = _lib.host().retrieve(lmk_q, past, topk, noise, _SCORE_ROUND[score_round])
+        return idx, w, Retrieval(*full)
     res = lmk_score_topk(lmk_q, past, topk, noise=noise, score_round=score_round)
-    if lmk_q.requires_grad or past.requires_grad:
-        weights = differentiable_weights(lmk_q, past, res.indices)
-    else:
-        weights = res.weights
+    weights = differentiable_weights(lmk_q, past, res.indices)
     return res.indices[:, :-1], weights[:, :-1], res._replace(weights=weights)
 
 

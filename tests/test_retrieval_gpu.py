@@ -335,3 +335,53 @@ def test_virtual_memory_cache_grows_in_place():
     virt.close()
     assert len(virt) == 0
     assert torch.cuda.mem_get_info(dev)[0] > free0 - used + 2 * n * (1 << 21)        # the mapped pages were released
+
+
+@pytest.mark.parametrize("n,cq,e,d,k,noisy", [(1, 64, 64, 768, 3, False), (2, 65, 129, 64, 28, True), (3, 64, 640, 256, 1, False),
+                                              (1, 70, 2200, 768, 8, True), (2, 130, 130, 1024, 16, True), (9, 200, 191, 128, 5, False)])
+def test_tensor_core_screening_bit_exact_vs_canonical_oracle(lcm, n, cq, e, d, k, noisy):
+    """Many query rows: approximate scores choose the candidates, exact ones decide.  Ragged tiles in both axes,
+    several tiles per candidate list, rows that see fewer chunks than K."""
+    lq, lk = cases.landmark_case(31, n, cq, e, d=d)
+    q_pos0 = max(0, e - cq)
+    noise = -torch.empty(n, cq, e).exponential_(generator=torch.Generator().manual_seed(5)).log() if noisy else None
+    res = lcm.lmk_score_topk(lq.cuda(), lk.cuda(), k, q_pos0=q_pos0, noise=None if noise is None else noise.cuda())
+    check(res, oracle_rows(lq, lk, k, q_pos0=q_pos0, noise=noise))
+
+
+@pytest.mark.parametrize("copies", [2, 40, 200])
+def test_tensor_core_screening_with_copies_of_landmarks(lcm, copies):
+    """Ties that the candidate lists cannot hold (copies of one landmark) and near ties: the exact scan takes over, ties go to
+    the lower id."""
+    lq, lk = cases.landmark_case(34, 2, 80, 300, d=192)
+    lk[0, 3:3 + copies] = lq[0, 7]
+    lk[1, ::2] = lk[1, 0]
+    lk[1, 1::4, 5] += 0.015625
+    res = lcm.lmk_score_topk(lq.cuda(), lk.cuda(), 8, q_pos0=260)
+    check(res, oracle_rows(lq, lk, 8, q_pos0=260))
+
+
+@pytest.mark.parametrize("e,k,splits", [(9000, 32, 33), (70001, 1, 0), (5000, 7, 1024), (3000, 8, 1500)])
+def test_many_candidate_lists_per_row(lcm, e, k, splits):
+    lq, lk = cases.landmark_case(32, 1, 1, e, d=128)
+    res = lcm.lmk_score_topk(lq.cuda(), lk.cuda(), k, splits=splits)
+    check(res, oracle_rows(lq, lk, k))
+
+
+@pytest.mark.parametrize("n,c,d,k", [(1, 3, 64, 2), (2, 37, 768, 8), (1, 150, 1024, 32), (3, 65, 264, 5)])
+def test_retrieval_weight_gradients_against_float32(lcm, n, c, d, k):
+    """``retrieve`` on bf16 landmarks that require grad: weights and both gradients against float32 autograd over the
+    same selection; both outputs (whole, without the last row) carry gradient."""
+    lq, lk = cases.landmark_case(33, n, c, c, d=d, std=0.5)
+    q, m = lq.cuda().requires_grad_(), lk.cuda().requires_grad_()
+    chunks = type("Chunks", (), {"past_lmk_embeds": m})
+    idx, w, full = lcm.retrieve(q, chunks, min(k, c))
+    g = torch.Generator().manual_seed(2)
+    probe, probe_all = (torch.randn(x.shape, generator=g).cuda() for x in (w, full.weights))
+    dq, dm = torch.autograd.grad([w, full.weights], [q, m], [probe, probe_all])
+    qf, mf = lq.cuda().float().requires_grad_(), lk.cuda().float().requires_grad_()
+    ref = lcm.differentiable_weights(qf, mf, full.indices)
+    rq, rm = torch.autograd.grad([ref[:, :-1], ref], [qf, mf], [probe, probe_all])
+    assert torch.equal(idx, full.indices[:, :-1]) and torch.allclose(w, ref[:, :-1], atol=1e-5)
+    for got, want in ((dq, rq), (dm, rm)):
+        assert (got.float() - want).norm() <= 4e-3 * want.norm() + 1e-6
