@@ -245,7 +245,7 @@ int gca_bwd_stages(const GcaBwdArgs* a, unsigned stages, void* stream) {
   if (algo == GCA_ALGO_AUTO) algo = tc_ok ? GCA_ALGO_TC : GCA_ALGO_SIMT;
   if (algo == GCA_ALGO_TC)
     rc = tc_ok ? gca::launch_bwd_tc(*a, csr, dw_part, rowterm, gca::sm_count(scope.dev), s, stages & GCA_BWD_STAGE_ALL) : GCA_ERR_ALGO;
-  else if (algo == GCA_ALGO_SIMT) rc = gca::launch_bwd_simt(*a, csr, dw_part, s, stages & GCA_BWD_STAGE_ALL);
+  else if (algo == GCA_ALGO_SIMT) rc = gca::launch_bwd_simt(*a, csr, dw_part, reinterpret_cast<float*>(rowterm), s, stages & GCA_BWD_STAGE_ALL);
   else rc = GCA_ERR_ALGO;
   if (rc) return rc;
   if (!(stages & GCA_BWD_STAGE_Q)) return 0;

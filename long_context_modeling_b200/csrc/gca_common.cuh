@@ -85,7 +85,8 @@ size_t csr_workspace_bytes(int N, int J, int K, int C);
 // SIMT (CUDA-core, fp32 accumulate) kernels: every dtype, S <= 64, L = D = 64.
 int launch_fwd_simt(const GcaFwdArgs& a, cudaStream_t stream);
 // stages: GCA_BWD_STAGE_KV and / or GCA_BWD_STAGE_Q
-int launch_bwd_simt(const GcaBwdArgs& a, const Csr& csr, float* dw_part, cudaStream_t stream, unsigned stages);
+// row_di: (N*J, Hq, K, 64) floats of scratch, Di of every row: the q-major stage writes it, the kv-major stage reads it
+int launch_bwd_simt(const GcaBwdArgs& a, const Csr& csr, float* dw_part, float* row_di, cudaStream_t stream, unsigned stages);
 
 // tcgen05 / TMEM / TMA kernels: bf16, S = L = D = 64.
 int launch_fwd_tc(const GcaFwdArgs& a, int sms, cudaStream_t stream);

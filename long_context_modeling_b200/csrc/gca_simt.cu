@@ -1,338 +1,416 @@
-// CUDA-core GCA kernels with float32 accumulation.  They serve float32 data (the
-// accuracy path: tensor cores would round the operands) and any shape the tensor-core
-// kernels do not take (S < 64 query rows).  Tiles are 64 keys x 64 dims; one block owns
-// one (sequence, query chunk, head) in the q-major kernels and one (sequence, cache
-// chunk, kv head) in the kv-major backward kernel, so no atomics are needed and results
-// are bit-reproducible.
+// CUDA-core GCA kernels with float32 arithmetic throughout.  They serve float32 data (the accuracy path: tensor cores
+// would round the operands) and any shape the tensor-core kernels do not take (S < 64 query rows).  One block of four
+// warps owns one (sequence, query chunk, head) in the q-major kernels and one (sequence, cache chunk, kv head) in the
+// kv-major backward kernel, so no atomics are needed and results are bit-reproducible.
+//
+// Bound: the FMA pipe (73 TFLOP/s measured on this part; the packed form is no faster).  A product of two 64 x 64
+// tiles is 64 steps of 64 x 64 FMA, so what matters is how few other instructions go with them: a warp owns 16
+// rows x 64 columns of every product, a thread 4 x 8, which is 12 16-byte shared loads per 128 FMA (a 4 x 4 tile with scalar
+// loads: 64 per 128).  A warp owns whole rows, so the softmax stays inside it, and the rows it writes as the A
+// operand of the next product are read by nobody else: blocks synchronise only for the K / V (Q / dO) tiles,
+// which cp.async brings in one step ahead.  The kv-major kernel works on TRANSPOSED scores (rows = keys) for the same
+// reason; what it needs per query row, Di = rowsum(P dP), comes from the q-major kernel.
+// 2 x 64 chunks x 12 heads, top-8, float32: forward 477 -> 371 us, q-major 689 -> 481 us, kv-major 1031 -> 785 us.
 #include "gca_common.cuh"
 
 namespace gca {
 
 namespace {
 
-constexpr int T = 64;          // tile edge (keys per chunk, head dim, max query rows)
-constexpr int LD = T + 1;      // padded leading dimension in shared memory
-constexpr int NTHREADS = 256;
+constexpr int T = 64;            // tile edge (keys per chunk, head dim, max query rows)
+constexpr int LD = T + 4;        // row pitch of operand tiles: eight rows of 16 bytes hit all banks once
+constexpr int LDP = T + 8;       // row pitch of tiles written by (4 rows x 8 columns) lanes
+constexpr int NTHREADS = 128;
+constexpr int TILE = T * LD, TILE_P = T * LDP;
 
-// Load a (rows x 64) tile whose rows are `row_stride` elements apart into padded smem.
+__device__ __forceinline__ void cp_async16(float* dst, const float* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int LEFT>
+__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory"); }
+
+// A (rows x 64) tile whose rows are `row_stride` elements apart; rows past `rows` become zeros.  float32 arrives
+// asynchronously (one commit group, taken by the caller), bf16 is widened on the way.
+__device__ __forceinline__ void load_tile(float* dst, const float* src, long long row_stride, int rows) {
+  for (int i = threadIdx.x; i < T * (T / 4); i += NTHREADS) {
+    const int r = i >> 4, c = (i & 15) * 4;
+    if (r < rows) cp_async16(dst + r * LD + c, src + r * row_stride + c);
+    else *reinterpret_cast<float4*>(dst + r * LD + c) = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+}
+__device__ __forceinline__ void load_tile(float* dst, const __nv_bfloat16* src, long long row_stride, int rows) {
+  for (int i = threadIdx.x; i < T * (T / 8); i += NTHREADS) {
+    const int r = i >> 3, c = (i & 7) * 8;
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (r < rows) v = *reinterpret_cast<const uint4*>(src + r * row_stride + c);
+    const unsigned w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      *reinterpret_cast<float4*>(dst + r * LD + c + 4 * h) =
+          make_float4(__uint_as_float(w[2 * h] << 16), __uint_as_float(w[2 * h] & 0xffff0000u), __uint_as_float(w[2 * h + 1] << 16),
+                      __uint_as_float(w[2 * h + 1] & 0xffff0000u));
+  }
+}
+
+// What a thread owns of a product: rows row0 + 4 i (i < 4) and columns tx + 8 j (NT products) or tx * 4 + 32 (j / 4) + j % 4 (NN).
+struct Own {
+  int row0, tx;
+  __device__ __forceinline__ Own() {
+    const int lane = threadIdx.x & 31;
+    row0 = (threadIdx.x >> 5) * 16 + (lane >> 3);
+    tx = lane & 7;
+  }
+};
+
+// acc[i][j] = sum_d A[row_i][d] B[col_j][d]
+__device__ __forceinline__ void mma_nt(const float* A, const float* B, const Own& o, float acc[4][8]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+  const float* a0 = A + o.row0 * LD;
+  const float* b0 = B + o.tx * LD;
+#pragma unroll 2
+  for (int d = 0; d < T; d += 4) {
+    float4 a[4], b[8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(a0 + 4 * i * LD + d);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) b[j] = *reinterpret_cast<const float4*>(b0 + 8 * j * LD + d);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        acc[i][j] = fmaf(a[i].x, b[j].x, acc[i][j]); acc[i][j] = fmaf(a[i].y, b[j].y, acc[i][j]);
+        acc[i][j] = fmaf(a[i].z, b[j].z, acc[i][j]); acc[i][j] = fmaf(a[i].w, b[j].w, acc[i][j]);
+      }
+  }
+}
+
+// acc[i][j] += sum_r A[row_i][r] B[r][col_j]   (A: pitch LDP, this warp's own rows)
+__device__ __forceinline__ void mma_nn_acc(const float* A, const float* B, const Own& o, float acc[4][8]) {
+  const float* a0 = A + o.row0 * LDP;
+  const float* b0 = B + o.tx * 4;
+#pragma unroll 2
+  for (int r = 0; r < T; r += 4) {
+    float4 a[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(a0 + 4 * i * LDP + r);
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      const float4 b = *reinterpret_cast<const float4*>(b0 + (r + x) * LD), c = *reinterpret_cast<const float4*>(b0 + (r + x) * LD + 32);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float av = x == 0 ? a[i].x : x == 1 ? a[i].y : x == 2 ? a[i].z : a[i].w;
+        acc[i][0] = fmaf(av, b.x, acc[i][0]); acc[i][1] = fmaf(av, b.y, acc[i][1]);
+        acc[i][2] = fmaf(av, b.z, acc[i][2]); acc[i][3] = fmaf(av, b.w, acc[i][3]);
+        acc[i][4] = fmaf(av, c.x, acc[i][4]); acc[i][5] = fmaf(av, c.y, acc[i][5]);
+        acc[i][6] = fmaf(av, c.z, acc[i][6]); acc[i][7] = fmaf(av, c.w, acc[i][7]);
+      }
+    }
+  }
+}
+
+// Write a thread's NT-shaped values as rows of the next product's A operand.
+__device__ __forceinline__ void put_rows(float* P, const Own& o, const float v[4][8]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) P[(o.row0 + 4 * i) * LDP + o.tx + 8 * j] = v[i][j];
+}
+
+__device__ __forceinline__ void store4(float* dst, const float* v, float s) {
+  *reinterpret_cast<float4*>(dst) = make_float4(v[0] * s, v[1] * s, v[2] * s, v[3] * s);
+}
+__device__ __forceinline__ void store4(__nv_bfloat16* dst, const float* v, float s) {
+  const __nv_bfloat162 a = __floats2bfloat162_rn(v[0] * s, v[1] * s), b = __floats2bfloat162_rn(v[2] * s, v[3] * s);
+  *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const unsigned*>(&a), *reinterpret_cast<const unsigned*>(&b));
+}
 template <typename E>
-__device__ __forceinline__ void load_tile(float* dst, const E* src, long long row_stride, int rows) {
-  for (int i = threadIdx.x; i < T * T; i += NTHREADS) {
-    int r = i >> 6, c = i & 63;
-    dst[r * LD + c] = (r < rows) ? ld_f<E>(src + r * row_stride + c) : 0.f;
+__device__ __forceinline__ void store_rows(E* base, long long row_stride, int rows, const Own& o, const float acc[4][8], float s) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = o.row0 + 4 * i;
+    if (r >= rows) continue;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) store4(base + r * row_stride + o.tx * 4 + 32 * h, &acc[i][4 * h], s);
   }
 }
 
-// acc[a][b] = sum_d A[(4*ty+a)][d] * B[(tx+16*b)][d]      (A, B padded tiles, "NT" product)
-__device__ __forceinline__ void mma_nt(const float* A, const float* B, int ty, int tx, float acc[4][4]) {
+// Reduce over the 8 lanes that share a row.
+__device__ __forceinline__ float row_max(float v) {
 #pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b) acc[a][b] = 0.f;
-#pragma unroll 8
-  for (int d = 0; d < T; ++d) {
-    float av[4], bv[4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a) av[a] = A[(4 * ty + a) * LD + d];
-#pragma unroll
-    for (int b = 0; b < 4; ++b) bv[b] = B[(tx + 16 * b) * LD + d];
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) acc[a][b] = fmaf(av[a], bv[b], acc[a][b]);
-  }
-}
-
-// acc[a][b] += sum_r A[(4*ty+a)][r] * B[r][(tx+16*b)]     ("NN" product)
-__device__ __forceinline__ void mma_nn_acc(const float* A, const float* B, int ty, int tx, float acc[4][4]) {
-#pragma unroll 8
-  for (int r = 0; r < T; ++r) {
-    float av[4], bv[4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a) av[a] = A[(4 * ty + a) * LD + r];
-#pragma unroll
-    for (int b = 0; b < 4; ++b) bv[b] = B[r * LD + tx + 16 * b];
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) acc[a][b] = fmaf(av[a], bv[b], acc[a][b]);
-  }
-}
-
-// acc[a][b] += sum_r A[r][(4*ty+a)] * B[r][(tx+16*b)]     ("TN" product: A used transposed)
-__device__ __forceinline__ void mma_tn_acc(const float* A, const float* B, int ty, int tx, float acc[4][4]) {
-#pragma unroll 8
-  for (int r = 0; r < T; ++r) {
-    float av[4], bv[4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a) av[a] = A[r * LD + 4 * ty + a];
-#pragma unroll
-    for (int b = 0; b < 4; ++b) bv[b] = B[r * LD + tx + 16 * b];
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) acc[a][b] = fmaf(av[a], bv[b], acc[a][b]);
-  }
-}
-
-// Reduce over the 16 lanes that share a row (lanes with equal ty inside a half warp).
-__device__ __forceinline__ float row_max16(float v) {
-#pragma unroll
-  for (int o = 8; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+  for (int of = 4; of > 0; of >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, of));
   return v;
 }
-__device__ __forceinline__ float row_sum16(float v) {
+__device__ __forceinline__ float row_sum(float v) {
 #pragma unroll
-  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  for (int of = 4; of > 0; of >>= 1) v += __shfl_xor_sync(0xffffffffu, v, of);
   return v;
+}
+
+// The next slot from k on that reads a chunk (K if none).
+__device__ __forceinline__ int next_slot(const int32_t* indices, long long zj, const Geom& g, int k, int& idx) {
+  for (; k < g.K; ++k) {
+    idx = slot_chunk(indices, zj, g.K, k);
+    if (idx >= 0 && idx < g.C) break;
+  }
+  return k;
 }
 
 // ------------------------------------------------------------------------------------
 // forward
 // ------------------------------------------------------------------------------------
 template <typename E>
-__global__ void __launch_bounds__(NTHREADS)
+__global__ void __launch_bounds__(NTHREADS, 3)
 fwd_simt_kernel(const E* __restrict__ q, const E* __restrict__ kc, const E* __restrict__ vc,
                 const int32_t* __restrict__ indices, const float* __restrict__ weights,
                 E* __restrict__ out, float* __restrict__ lse, int32_t* status, Geom g) {
-  extern __shared__ float smem[];
-  float* sQ = smem;
-  float* sK = sQ + T * LD;
-  float* sV = sK + T * LD;
-  float* sP = sV + T * LD;
-
+  extern __shared__ __align__(16) float smem[];
+  float *sQ = smem, *sK = sQ + TILE, *sV = sK + TILE, *sP = sV + TILE;
   const int zj = blockIdx.x, h = blockIdx.y;
   const int n = zj / g.J, j = zj % g.J, hk = h / g.G;
-  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-
-  load_tile<E>(sQ, q + n * g.qs[0] + j * g.qs[1] + h * g.qs[2], g.qs[3], g.S);
-  float o[4][4];
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b) o[a][b] = 0.f;
-  const float c2 = g.sm_scale * GCA_LOG2E;
-
+  const Own own;
+  // padding slots and ids outside the cache
   for (int k = 0; k < g.K; ++k) {
     const int idx = slot_chunk(indices, zj, g.K, k);
-    const float w = weights[(long long)zj * g.K + k];
-    float* lse_row = lse ? lse + (((long long)zj * g.Hq + h) * g.K + k) * g.S : nullptr;
-    if (idx < 0 || idx >= g.C) {
-      if (idx >= g.C && status && threadIdx.x == 0) atomicOr(status, GCA_STATUS_BAD_INDEX);
-      if (lse_row) for (int r = threadIdx.x; r < g.S; r += NTHREADS) lse_row[r] = 0.f;
-      continue;
-    }
-    __syncthreads();
-    load_tile<E>(sK, kc + n * g.ks[0] + idx * g.ks[1] + hk * g.ks[3], g.ks[2], T);
-    load_tile<E>(sV, vc + n * g.vs[0] + idx * g.vs[1] + hk * g.vs[3], g.vs[2], T);
-    __syncthreads();
-    float s[4][4];
-    mma_nt(sQ, sK, ty, tx, s);
+    if (idx >= 0 && idx < g.C) continue;
+    if (idx >= g.C && status && threadIdx.x == 0) atomicOr(status, GCA_STATUS_BAD_INDEX);
+    if (lse) for (int r = threadIdx.x; r < g.S; r += NTHREADS) lse[(((long long)zj * g.Hq + h) * g.K + k) * g.S + r] = 0.f;
+  }
+  auto k_tile = [&](int idx) { load_tile(sK, kc + n * g.ks[0] + idx * g.ks[1] + hk * g.ks[3], g.ks[2], T); };
+  auto v_tile = [&](int idx) { load_tile(sV, vc + n * g.vs[0] + idx * g.vs[1] + hk * g.vs[3], g.vs[2], T); };
+  float acc[4][8];
 #pragma unroll
-    for (int a = 0; a < 4; ++a) {
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int b = 0; b < 8; ++b) acc[i][b] = 0.f;
+  const float c2 = g.sm_scale * GCA_LOG2E;
+
+  int idx = -1, k = next_slot(indices, zj, g, 0, idx);
+  if (k < g.K) {
+    load_tile(sQ, q + n * g.qs[0] + j * g.qs[1] + h * g.qs[2], g.qs[3], g.S);
+    k_tile(idx);
+    cp_commit();
+    v_tile(idx);
+    cp_commit();
+  }
+  while (k < g.K) {
+    int idx_next = -1;
+    const int k_next = next_slot(indices, zj, g, k + 1, idx_next);
+    const float w = weights[(long long)zj * g.K + k];
+    cp_wait<1>();                              // Q and K are here, V may still be on its way
+    __syncthreads();
+    float s[4][8];
+    mma_nt(sQ, sK, own, s);
+    __syncthreads();                           // every warp is done with K
+    if (k_next < g.K) k_tile(idx_next);
+    cp_commit();
+    float* lse_row = lse ? lse + (((long long)zj * g.Hq + h) * g.K + k) * g.S : nullptr;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
       float m = -INFINITY;
 #pragma unroll
-      for (int b = 0; b < 4; ++b) { s[a][b] *= c2; m = fmaxf(m, s[a][b]); }
-      m = row_max16(m);
+      for (int b = 0; b < 8; ++b) { s[i][b] *= c2; m = fmaxf(m, s[i][b]); }
+      m = row_max(m);
       if (g.off_by_one > 0.f) m = fmaxf(m, 0.f);
       float l = 0.f;
 #pragma unroll
-      for (int b = 0; b < 4; ++b) { s[a][b] = exp2f(s[a][b] - m); l += s[a][b]; }
-      l = row_sum16(l);
+      for (int b = 0; b < 8; ++b) { s[i][b] = exp2f(s[i][b] - m); l += s[i][b]; }
+      l = row_sum(l);
       if (g.off_by_one > 0.f) l += g.off_by_one * exp2f(-m);
-      const int r = 4 * ty + a;
-      if (lse_row && tx == 0 && r < g.S) lse_row[r] = m + log2f(l);
+      const int r = own.row0 + 4 * i;
+      if (lse_row && own.tx == 0 && r < g.S) lse_row[r] = m + log2f(l);
       const float f = w / l;
 #pragma unroll
-      for (int b = 0; b < 4; ++b) sP[r * LD + tx + 16 * b] = s[a][b] * f;
+      for (int b = 0; b < 8; ++b) s[i][b] *= f;
     }
+    put_rows(sP, own, s);
+    cp_wait<1>();                              // V is here, the next K may still be on its way
     __syncthreads();
-    mma_nn_acc(sP, sV, ty, tx, o);
+    mma_nn_acc(sP, sV, own, acc);
+    __syncthreads();                           // every warp is done with V
+    if (k_next < g.K) v_tile(idx_next);
+    cp_commit();
+    k = k_next;
+    idx = idx_next;
   }
-  E* op = out + n * g.os[0] + j * g.os[1] + h * g.os[2];
-#pragma unroll
-  for (int a = 0; a < 4; ++a) {
-    const int r = 4 * ty + a;
-    if (r < g.S)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) st_f<E>(op + r * g.os[3] + tx + 16 * b, o[a][b]);
-  }
+  store_rows(out + n * g.os[0] + j * g.os[1] + h * g.os[2], g.os[3], g.S, own, acc, 1.0f);
 }
 
 // ------------------------------------------------------------------------------------
-// backward, shared per-slot math: given Q, dO, K, V tiles in smem and the row LSE,
-// produce P*w (sPw) and dS (sdS) tiles in smem and return the per-thread partial of
-// sum_rows Di (for dw).  Rows >= S hold zeros.
+// backward, q-major: one block per (sequence, query chunk, q head): dQ, the per-head part of dw, and Di = rowsum(P dP) of
+// every (row, slot) for the kv-major kernel.
 // ------------------------------------------------------------------------------------
-__device__ __forceinline__ float slot_backward_core(const float* sQ, const float* sdO, const float* sK, const float* sV,
-                                                    float* sPw, float* sdS, const float* lse_row, float w, float c2,
-                                                    int S, int ty, int tx) {
-  float s[4][4], dp[4][4];
-  mma_nt(sQ, sK, ty, tx, s);
-  mma_nt(sdO, sV, ty, tx, dp);
-  float di_sum = 0.f;
-#pragma unroll
-  for (int a = 0; a < 4; ++a) {
-    const int r = 4 * ty + a;
-    const bool live = r < S;
-    const float m = live ? lse_row[r] : 0.f;
-    float di = 0.f;
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      s[a][b] = live ? exp2f(s[a][b] * c2 - m) : 0.f;
-      di = fmaf(s[a][b], dp[a][b], di);
-    }
-    di = row_sum16(di);
-    if (tx == 0) di_sum += di;
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      const float pw = s[a][b] * w;
-      sPw[r * LD + tx + 16 * b] = pw;
-      sdS[r * LD + tx + 16 * b] = pw * (dp[a][b] - di);
-    }
-  }
-  return di_sum;
-}
-
-// kv-major: one block per (sequence n, cache chunk c, kv head).  Loops over every
-// (query chunk j, slot k) that retrieved the chunk and over the q heads of the group.
 template <typename E>
-__global__ void __launch_bounds__(NTHREADS)
-bwd_kv_simt_kernel(const E* __restrict__ q, const E* __restrict__ kc, const E* __restrict__ vc,
-                   const float* __restrict__ weights, const E* __restrict__ dout, const float* __restrict__ lse,
-                   E* __restrict__ dk, E* __restrict__ dv, Csr csr, Geom g,
-                   long long dos0, long long dos1, long long dos2, long long dos3,
-                   long long dks0, long long dks1, long long dks2, long long dks3,
-                   long long dvs0, long long dvs1, long long dvs2, long long dvs3) {
-  extern __shared__ float smem[];
-  float* sK = smem;
-  float* sV = sK + T * LD;
-  float* sQ = sV + T * LD;
-  float* sdO = sQ + T * LD;
-  float* sPw = sdO + T * LD;
-  float* sdS = sPw + T * LD;
-
-  const int nc = blockIdx.x, hk = blockIdx.y;
-  const int n = nc / g.C, c = nc % g.C;
-  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-  const float c2 = g.sm_scale * GCA_LOG2E;
-
-  float aK[4][4], aV[4][4];
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b) { aK[a][b] = 0.f; aV[a][b] = 0.f; }
-
-  const int beg = csr.offsets[nc], end = csr.offsets[nc + 1];
-  if (end > beg) {
-    load_tile<E>(sK, kc + n * g.ks[0] + c * g.ks[1] + hk * g.ks[3], g.ks[2], T);
-    load_tile<E>(sV, vc + n * g.vs[0] + c * g.vs[1] + hk * g.vs[3], g.vs[2], T);
-  }
-  for (int e = beg; e < end; ++e) {
-    const int entry = (int)(csr.sorted_keys[e] & 0xffffffffull);
-    const int j = entry / g.K, k = entry % g.K;
-    const long long zj = (long long)n * g.J + j;
-    const float w = weights[zj * g.K + k];
-    for (int gi = 0; gi < g.G; ++gi) {
-      const int h = hk * g.G + gi;
-      __syncthreads();
-      load_tile<E>(sQ, q + n * g.qs[0] + j * g.qs[1] + h * g.qs[2], g.qs[3], g.S);
-      load_tile<E>(sdO, dout + n * dos0 + j * dos1 + h * dos2, dos3, g.S);
-      __syncthreads();
-      const float* lse_row = lse + ((zj * g.Hq + h) * g.K + k) * g.S;
-      slot_backward_core(sQ, sdO, sK, sV, sPw, sdS, lse_row, w, c2, g.S, ty, tx);
-      __syncthreads();
-      mma_tn_acc(sPw, sdO, ty, tx, aV);   // dV[key][d] += sum_row (w P)[row][key] dO[row][d]
-      mma_tn_acc(sdS, sQ, ty, tx, aK);    // dK[key][d] += sum_row dS[row][key] Q[row][d]
-    }
-  }
-  E* dkp = dk + n * dks0 + c * dks1 + hk * dks3;
-  E* dvp = dv + n * dvs0 + c * dvs1 + hk * dvs3;
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      const int r = 4 * ty + a, col = tx + 16 * b;
-      st_f<E>(dkp + r * dks2 + col, aK[a][b] * g.sm_scale);
-      st_f<E>(dvp + r * dvs2 + col, aV[a][b]);
-    }
-}
-
-// q-major: one block per (sequence, query chunk, q head): dQ and the per-head part of dw.
-template <typename E>
-__global__ void __launch_bounds__(NTHREADS)
+__global__ void __launch_bounds__(NTHREADS, 2)
 bwd_q_simt_kernel(const E* __restrict__ q, const E* __restrict__ kc, const E* __restrict__ vc,
                   const int32_t* __restrict__ indices, const float* __restrict__ weights,
                   const E* __restrict__ dout, const float* __restrict__ lse, E* __restrict__ dq,
-                  float* __restrict__ dw_part, Geom g,
+                  float* __restrict__ dw_part, float* __restrict__ row_di, Geom g,
                   long long dos0, long long dos1, long long dos2, long long dos3) {
-  extern __shared__ float smem[];
-  float* sQ = smem;
-  float* sdO = sQ + T * LD;
-  float* sK = sdO + T * LD;
-  float* sV = sK + T * LD;
-  float* sPw = sV + T * LD;
-  float* sdS = sPw + T * LD;
-  __shared__ float red[NTHREADS / 32];
-
+  extern __shared__ __align__(16) float smem[];
+  float *sQ = smem, *sdO = sQ + TILE, *sK = sdO + TILE, *sV = sK + TILE, *sdS = sV + TILE;
+  __shared__ float red[2][NTHREADS / 32];
   const int zj = blockIdx.x, h = blockIdx.y;
   const int n = zj / g.J, j = zj % g.J, hk = h / g.G;
-  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+  const Own own;
   const float c2 = g.sm_scale * GCA_LOG2E;
-
-  load_tile<E>(sQ, q + n * g.qs[0] + j * g.qs[1] + h * g.qs[2], g.qs[3], g.S);
-  load_tile<E>(sdO, dout + n * dos0 + j * dos1 + h * dos2, dos3, g.S);
-  float aQ[4][4];
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b) aQ[a][b] = 0.f;
-
-  for (int k = 0; k < g.K; ++k) {
+  for (int k = threadIdx.x; k < g.K; k += NTHREADS) {
     const int idx = slot_chunk(indices, zj, g.K, k);
-    float* dwp = dw_part + ((long long)zj * g.Hq + h) * g.K + k;
-    if (idx < 0 || idx >= g.C) {
-      if (threadIdx.x == 0) *dwp = 0.f;
-      continue;
-    }
+    if (idx < 0 || idx >= g.C) dw_part[((long long)zj * g.Hq + h) * g.K + k] = 0.f;
+  }
+  auto k_tile = [&](int idx) { load_tile(sK, kc + n * g.ks[0] + idx * g.ks[1] + hk * g.ks[3], g.ks[2], T); };
+  auto v_tile = [&](int idx) { load_tile(sV, vc + n * g.vs[0] + idx * g.vs[1] + hk * g.vs[3], g.vs[2], T); };
+  float acc[4][8];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int b = 0; b < 8; ++b) acc[i][b] = 0.f;
+  int idx = -1, k = next_slot(indices, zj, g, 0, idx), turn = 0;
+  if (k < g.K) {
+    load_tile(sQ, q + n * g.qs[0] + j * g.qs[1] + h * g.qs[2], g.qs[3], g.S);
+    load_tile(sdO, dout + n * dos0 + j * dos1 + h * dos2, dos3, g.S);
+    v_tile(idx);
+    cp_commit();
+    k_tile(idx);
+    cp_commit();
+  }
+  while (k < g.K) {
+    int idx_next = -1;
+    const int k_next = next_slot(indices, zj, g, k + 1, idx_next);
+    const long long slot = ((long long)zj * g.Hq + h) * g.K + k;
     const float w = weights[(long long)zj * g.K + k];
-    __syncthreads();
-    load_tile<E>(sK, kc + n * g.ks[0] + idx * g.ks[1] + hk * g.ks[3], g.ks[2], T);
-    load_tile<E>(sV, vc + n * g.vs[0] + idx * g.vs[1] + hk * g.vs[3], g.vs[2], T);
-    __syncthreads();
-    const float* lse_row = lse + (((long long)zj * g.Hq + h) * g.K + k) * g.S;
-    // dw wants sum_rows <dO, O_k> = sum_rows rowsum(P * dP): use weight 1 for Di, then scale.
-    float di = slot_backward_core(sQ, sdO, sK, sV, sPw, sdS, lse_row, 1.0f, c2, g.S, ty, tx);
-    // block reduction of di in a fixed order
+    float m[4];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) di += __shfl_xor_sync(0xffffffffu, di, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = di;
+    for (int i = 0; i < 4; ++i) { const int r = own.row0 + 4 * i; m[i] = r < g.S ? lse[slot * g.S + r] : 0.f; }
+    float s[4][8], dp[4][8];
+    cp_wait<1>();                              // Q, dO and V are here
     __syncthreads();
-    if (threadIdx.x == 0) {
-      float t = 0.f;
-      for (int i = 0; i < NTHREADS / 32; ++i) t += red[i];
-      *dwp = t;
+    mma_nt(sdO, sV, own, dp);
+    cp_wait<0>();                              // K is here
+    __syncthreads();                           // and every warp is done with V
+    if (k_next < g.K) v_tile(idx_next);
+    cp_commit();
+    mma_nt(sQ, sK, own, s);
+    float di_sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = own.row0 + 4 * i;
+      const bool live = r < g.S;
+      float di = 0.f;
+#pragma unroll
+      for (int b = 0; b < 8; ++b) {
+        s[i][b] = live ? exp2f(s[i][b] * c2 - m[i]) : 0.f;
+        di = fmaf(s[i][b], dp[i][b], di);
+      }
+      di = row_sum(di);
+      if (own.tx == 0) {
+        di_sum += di;
+        row_di[slot * T + r] = di;
+      }
+#pragma unroll
+      for (int b = 0; b < 8; ++b) s[i][b] = s[i][b] * w * (dp[i][b] - di);
     }
-    // dQ[row][d] += w * sum_key dS1[row][key] K[key][d]   (dS1 computed with weight 1)
-    float t[4][4];
+    put_rows(sdS, own, s);
+    // dw: the rows of a warp, then the warps, in a fixed order
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) t[a][b] = 0.f;
-    mma_nn_acc(sdS, sK, ty, tx, t);
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) aQ[a][b] = fmaf(w, t[a][b], aQ[a][b]);
+    for (int of = 16; of >= 8; of >>= 1) di_sum += __shfl_xor_sync(0xffffffffu, di_sum, of);
+    if ((threadIdx.x & 31) == 0) red[turn][threadIdx.x >> 5] = di_sum;
+    __syncwarp();
+    mma_nn_acc(sdS, sK, own, acc);
+    __syncthreads();                           // every warp is done with K
+    if (threadIdx.x == 0) dw_part[slot] = ((red[turn][0] + red[turn][1]) + red[turn][2]) + red[turn][3];
+    if (k_next < g.K) k_tile(idx_next);
+    cp_commit();
+    k = k_next;
+    idx = idx_next;
+    turn ^= 1;
   }
-  E* dqp = dq + n * g.os[0] + j * g.os[1] + h * g.os[2];
+  store_rows(dq + n * g.os[0] + j * g.os[1] + h * g.os[2], g.os[3], g.S, own, acc, g.sm_scale);
+}
+
+// ------------------------------------------------------------------------------------
+// backward, kv-major: one block per (sequence n, cache chunk c, kv head).  Loops over every (query chunk j, slot k) that
+// retrieved the chunk and over the q heads of the group, on transposed scores: rows = the chunk's keys.
+// ------------------------------------------------------------------------------------
+template <typename E>
+__global__ void __launch_bounds__(NTHREADS, 2)
+bwd_kv_simt_kernel(const E* __restrict__ q, const E* __restrict__ kc, const E* __restrict__ vc,
+                   const float* __restrict__ weights, const E* __restrict__ dout, const float* __restrict__ lse,
+                   const float* __restrict__ row_di, E* __restrict__ dk, E* __restrict__ dv, Csr csr, Geom g,
+                   long long dos0, long long dos1, long long dos2, long long dos3,
+                   long long dks0, long long dks1, long long dks2, long long dks3,
+                   long long dvs0, long long dvs1, long long dvs2, long long dvs3) {
+  extern __shared__ __align__(16) float smem[];
+  float *sK = smem, *sV = sK + TILE, *sQ = sV + TILE, *sdO = sQ + TILE, *sP = sdO + TILE;
+  const int4 unit = csr.unit_tab[blockIdx.x];         // the chunks with the most retrievers of a sequence first
+  const int nc = unit.z, hk = blockIdx.y;
+  const int n = nc / g.C, c = nc % g.C;
+  const Own own;
+  const float c2 = g.sm_scale * GCA_LOG2E;
+  float aK[4][8], aV[4][8];
 #pragma unroll
-  for (int a = 0; a < 4; ++a) {
-    const int r = 4 * ty + a;
-    if (r < g.S)
+  for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int b = 0; b < 4; ++b) st_f<E>(dqp + r * g.os[3] + tx + 16 * b, aQ[a][b] * g.sm_scale);
+    for (int b = 0; b < 8; ++b) { aK[i][b] = 0.f; aV[i][b] = 0.f; }
+  // steps: (entry, q head of the group)
+  const int steps = (unit.y - unit.x) * g.G;
+  auto step_of = [&](int t, int& j, int& k, int& h) {
+    const int e = t / g.G, entry = (int)(csr.sorted_keys[unit.x + e] & 0xffffffffull);
+    j = entry / g.K;
+    k = entry - j * g.K;
+    h = hk * g.G + (t - e * g.G);
+  };
+  auto q_tile = [&](int j, int h) { load_tile(sQ, q + n * g.qs[0] + j * g.qs[1] + h * g.qs[2], g.qs[3], g.S); };
+  auto o_tile = [&](int j, int h) { load_tile(sdO, dout + n * dos0 + j * dos1 + h * dos2, dos3, g.S); };
+  int j = 0, k = 0, h = 0;
+  if (steps > 0) {
+    step_of(0, j, k, h);
+    load_tile(sK, kc + n * g.ks[0] + c * g.ks[1] + hk * g.ks[3], g.ks[2], T);
+    load_tile(sV, vc + n * g.vs[0] + c * g.vs[1] + hk * g.vs[3], g.vs[2], T);
+    q_tile(j, h);
+    o_tile(j, h);
+    cp_commit();
   }
+  for (int t = 0; t < steps; ++t) {
+    const long long zj = (long long)n * g.J + j, slot = (zj * g.Hq + h) * g.K + k;
+    const float w = weights[zj * g.K + k];
+    float m[8], di[8];
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+      const int r = own.tx + 8 * b;
+      m[b] = r < g.S ? lse[slot * g.S + r] : INFINITY;            // exp2(x - inf) = 0: rows past the end do not count
+      di[b] = r < g.S ? row_di[slot * T + r] : 0.f;
+    }
+    if (t + 1 < steps) step_of(t + 1, j, k, h);
+    cp_wait<0>();
+    __syncthreads();
+    float p[4][8], dp[4][8];
+    mma_nt(sK, sQ, own, p);
+    mma_nt(sV, sdO, own, dp);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int b = 0; b < 8; ++b) {
+        p[i][b] = exp2f(p[i][b] * c2 - m[b]) * w;
+        dp[i][b] = p[i][b] * (dp[i][b] - di[b]);
+      }
+    put_rows(sP, own, p);
+    __syncwarp();
+    mma_nn_acc(sP, sdO, own, aV);              // dV[key][d] += sum_row (w P)[row][key] dO[row][d]
+    __syncthreads();                           // every warp is done with dO
+    if (t + 1 < steps) o_tile(j, h);
+    put_rows(sP, own, dp);
+    __syncwarp();
+    mma_nn_acc(sP, sQ, own, aK);               // dK[key][d] += sum_row dS[row][key] Q[row][d]
+    __syncthreads();
+    if (t + 1 < steps) q_tile(j, h);
+    cp_commit();
+  }
+  store_rows(dk + n * dks0 + c * dks1 + hk * dks3, dks2, T, own, aK, g.sm_scale);
+  store_rows(dv + n * dvs0 + c * dvs1 + hk * dvs3, dvs2, T, own, aV, 1.0f);
 }
 
 __global__ void dw_reduce_kernel(const float* __restrict__ part, float* __restrict__ dw, int ZJ, int Hq, int K,
@@ -367,7 +445,7 @@ Geom make_geom(const GcaBwdArgs& a) {
 
 template <typename E>
 int fwd_simt_typed(const GcaFwdArgs& a, cudaStream_t stream) {
-  const size_t smem = 4 * T * LD * sizeof(float);
+  const size_t smem = (3 * TILE + TILE_P) * sizeof(float);
   GCA_CUDA_CHECK(cudaFuncSetAttribute(fwd_simt_kernel<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   dim3 grid((unsigned)(a.N * a.J), (unsigned)a.Hq);
   fwd_simt_kernel<E><<<grid, NTHREADS, smem, stream>>>((const E*)a.q, (const E*)a.k_cache, (const E*)a.v_cache,
@@ -376,26 +454,30 @@ int fwd_simt_typed(const GcaFwdArgs& a, cudaStream_t stream) {
 }
 
 template <typename E>
-int bwd_simt_typed(const GcaBwdArgs& a, const Csr& csr, float* dw_part, cudaStream_t stream, unsigned stages) {
-  const size_t smem = 6 * T * LD * sizeof(float);
-  GCA_CUDA_CHECK(cudaFuncSetAttribute(bwd_kv_simt_kernel<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  GCA_CUDA_CHECK(cudaFuncSetAttribute(bwd_q_simt_kernel<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  Geom g = make_geom(a);
-  dim3 gkv((unsigned)(a.N * a.C), (unsigned)a.Hkv);
-  if (stages & GCA_BWD_STAGE_KV)
-  bwd_kv_simt_kernel<E><<<gkv, NTHREADS, smem, stream>>>(
-      (const E*)a.q, (const E*)a.k_cache, (const E*)a.v_cache, a.weights, (const E*)a.dout, a.lse,
-      (E*)a.dk_cache, (E*)a.dv_cache, csr, g,
-      a.do_stride[0], a.do_stride[1], a.do_stride[2], a.do_stride[3],
-      a.dk_stride[0], a.dk_stride[1], a.dk_stride[2], a.dk_stride[3],
-      a.dv_stride[0], a.dv_stride[1], a.dv_stride[2], a.dv_stride[3]);
-  GCA_CUDA_CHECK(cudaGetLastError());
-  dim3 gq((unsigned)(a.N * a.J), (unsigned)a.Hq);
-  if (stages & GCA_BWD_STAGE_Q)
-  bwd_q_simt_kernel<E><<<gq, NTHREADS, smem, stream>>>(
-      (const E*)a.q, (const E*)a.k_cache, (const E*)a.v_cache, a.indices, a.weights, (const E*)a.dout, a.lse,
-      (E*)a.dq, dw_part, g, a.do_stride[0], a.do_stride[1], a.do_stride[2], a.do_stride[3]);
-  return (int)cudaGetLastError();
+int bwd_simt_typed(const GcaBwdArgs& a, const Csr& csr, float* dw_part, float* row_di, cudaStream_t stream, unsigned stages) {
+  const size_t smem = (4 * TILE + TILE_P) * sizeof(float);
+  const Geom g = make_geom(a);
+  if (stages & GCA_BWD_STAGE_Q) {
+    GCA_CUDA_CHECK(cudaFuncSetAttribute(bwd_q_simt_kernel<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const dim3 grid((unsigned)(a.N * a.J), (unsigned)a.Hq);
+    if (grid.x > 0)
+      bwd_q_simt_kernel<E><<<grid, NTHREADS, smem, stream>>>(
+          (const E*)a.q, (const E*)a.k_cache, (const E*)a.v_cache, a.indices, a.weights, (const E*)a.dout, a.lse,
+          (E*)a.dq, dw_part, row_di, g, a.do_stride[0], a.do_stride[1], a.do_stride[2], a.do_stride[3]);
+    GCA_CUDA_CHECK(cudaGetLastError());
+  }
+  if (stages & GCA_BWD_STAGE_KV) {
+    GCA_CUDA_CHECK(cudaFuncSetAttribute(bwd_kv_simt_kernel<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const dim3 grid((unsigned)(a.N * a.C), (unsigned)a.Hkv);
+    bwd_kv_simt_kernel<E><<<grid, NTHREADS, smem, stream>>>(
+        (const E*)a.q, (const E*)a.k_cache, (const E*)a.v_cache, a.weights, (const E*)a.dout, a.lse, row_di,
+        (E*)a.dk_cache, (E*)a.dv_cache, csr, g,
+        a.do_stride[0], a.do_stride[1], a.do_stride[2], a.do_stride[3],
+        a.dk_stride[0], a.dk_stride[1], a.dk_stride[2], a.dk_stride[3],
+        a.dv_stride[0], a.dv_stride[1], a.dv_stride[2], a.dv_stride[3]);
+    GCA_CUDA_CHECK(cudaGetLastError());
+  }
+  return 0;
 }
 
 }  // namespace
@@ -406,9 +488,9 @@ int launch_fwd_simt(const GcaFwdArgs& a, cudaStream_t stream) {
   return GCA_ERR_DTYPE;
 }
 
-int launch_bwd_simt(const GcaBwdArgs& a, const Csr& csr, float* dw_part, cudaStream_t stream, unsigned stages) {
-  if (a.dtype == GCA_BF16) return bwd_simt_typed<__nv_bfloat16>(a, csr, dw_part, stream, stages);
-  if (a.dtype == GCA_F32) return bwd_simt_typed<float>(a, csr, dw_part, stream, stages);
+int launch_bwd_simt(const GcaBwdArgs& a, const Csr& csr, float* dw_part, float* row_di, cudaStream_t stream, unsigned stages) {
+  if (a.dtype == GCA_BF16) return bwd_simt_typed<__nv_bfloat16>(a, csr, dw_part, row_di, stream, stages);
+  if (a.dtype == GCA_F32) return bwd_simt_typed<float>(a, csr, dw_part, row_di, stream, stages);
   return GCA_ERR_DTYPE;
 }
 
