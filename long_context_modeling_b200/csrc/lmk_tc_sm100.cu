@@ -78,6 +78,7 @@ lmk_screen_kernel(const __grid_constant__ ScreenParams p) {
   __syncthreads();
   tc_fence_after();
   pdl_trigger();
+  pdl_wait();
   const uint32_t tmem = *tmem_slot;
 
   if (warp == WORKERS) {
@@ -245,6 +246,7 @@ lmk_settle_kernel(const __grid_constant__ SettleParams p) {
   const FinalParams& f = p.fin;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long row = (long long)blockIdx.x * SETTLE_WARPS + warp;
+  pdl_trigger();
   pdl_wait();
   if (row >= f.R) return;
   const long long n = row / f.Cq, r = row % f.Cq;
@@ -392,8 +394,8 @@ int launch_lmk_screen(const LmkTopkArgs& a, void* scratch, int sms, const FinalP
   p.noise = a.noise; p.q_pos0 = a.q_pos0; p.e_base = a.e_base;
   p.Cq = a.Cq; p.E = a.E; p.D = a.D; p.scale = fin.scale;
   GCA_CUDA_CHECK(cudaFuncSetAttribute(lmk_screen_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-  lmk_screen_kernel<<<dim3((unsigned)p.lists, (unsigned)((a.Cq + BM - 1) / BM), (unsigned)a.N), THREADS, SMEM_BYTES, stream>>>(p);
-  GCA_CUDA_CHECK(cudaGetLastError());
+  GCA_CUDA_CHECK(launch_dependent(lmk_screen_kernel, dim3((unsigned)p.lists, (unsigned)((a.Cq + BM - 1) / BM), (unsigned)a.N), dim3(THREADS), SMEM_BYTES,
+                                  stream, p));
   SettleParams sp;
   sp.fin = fin; sp.part = p.part; sp.eps = p.eps; sp.noise = a.noise; sp.q_pos0 = a.q_pos0; sp.KC = p.KC; sp.lists = p.lists; sp.E = a.E;
   const dim3 grid((unsigned)((rows + SETTLE_WARPS - 1) / SETTLE_WARPS)), block(SETTLE_WARPS * 32);

@@ -15,6 +15,8 @@
 // (lane i holds the i-th best).  Blocks write their lists to a scratch buffer; a second,
 // tiny kernel merges the lists of all blocks of a row and emits indices, noise-free scores,
 // softmax weights and the number of valid slots.
+#include <algorithm>
+
 #include "lmk_common.cuh"
 
 namespace gca {
@@ -42,13 +44,180 @@ struct ScanParams {
   float scale;
 };
 
-// NP: pieces per lane (D <= 256*NP).  TQ: query rows per block (per-sequence mode).
-// PER_HEAD: head_dim == 64, one list per head, TQ must be 1.
-template <int NP, int TQ, bool PER_HEAD>
+// Merge a batch of 64 scores (lane i: ids id0 + i and id0 + 32 + i; orderable, 0 = none; all ids above those of the list) into a
+// list of K keys held one per lane; `kth` is the list's K-th key.
+__device__ __forceinline__ void select_batch(unsigned long long& mine, unsigned long long& kth, unsigned o0, unsigned o1, unsigned id0, int K,
+                                             int lane) {
+  const unsigned th = (unsigned)(kth >> 32);                 // 0 while the list is not full
+  unsigned b0 = __ballot_sync(0xffffffffu, o0 > th), b1 = __ballot_sync(0xffffffffu, o1 > th);
+  const int found = __popc(b0) + __popc(b1);
+  if (found == 0) return;
+  if (found < K) {                                           // a few: one insertion each, lower ids first
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      unsigned b = h ? b1 : b0;
+      while (b) {
+        const int src = __ffs(b) - 1;
+        b &= b - 1;
+        const unsigned o = __shfl_sync(0xffffffffu, h ? o1 : o0, src);
+        const unsigned long long key = ((unsigned long long)o << 32) | (0xffffffffu - (id0 + 32 * h + src));
+        if (key > kth) {
+          list_insert(mine, key, lane);
+          kth = __shfl_sync(0xffffffffu, mine, K - 1);
+        }
+      }
+    }
+    return;
+  }
+  unsigned long long run = mine, best_mine = 0ull;           // many: the K best of list and batch by K warp-wide maxima
+  for (int k = 0; k < K; ++k) {
+    const unsigned rh = (unsigned)(run >> 32);
+    const unsigned m = __reduce_max_sync(0xffffffffu, max(rh, max(o0, o1)));
+    if (m == 0u) break;
+    const unsigned br = __ballot_sync(0xffffffffu, rh == m);
+    b0 = __ballot_sync(0xffffffffu, o0 == m);
+    b1 = __ballot_sync(0xffffffffu, o1 == m);
+    const int src = __ffs(br ? br : b0 ? b0 : b1) - 1;       // equal scores: the lower id first
+    unsigned long long best = __shfl_sync(0xffffffffu, run, src);
+    if (!br) best = ((unsigned long long)m << 32) | (0xffffffffu - (id0 + src + (b0 ? 0 : 32)));
+    if (lane == src) { if (br) run = 0ull; else if (b0) o0 = 0u; else o1 = 0u; }
+    if (lane == k) best_mine = best;
+  }
+  mine = lane < K ? best_mine : 0ull;
+  kth = __shfl_sync(0xffffffffu, mine, K - 1);
+}
+
+// ---------------------------------------------------------------------------------------------
+// One query row (a decode step), or one row and head at a time: the landmarks are streamed once, HBM-bound.
+//
+// Every lane copies the 16-byte pieces it will need itself to shared memory (cp.async), RING rows ahead of the
+// arithmetic, so 196 KB per SM are on their way without a register or a barrier.  Scores of 64 rows at a time go to shared
+// memory; list l (one per head, or the only one) is kept by warp l % 16, which looks at the 64 scores with two
+// votes and inserts what beats its K-th entry: one list per block instead of one per warp to merge at the end, and
+// no list code in the scoring loop (per head it was 12 lists in every warp, each with a serial insertion: 60 us for
+// 2 x 16,411 landmarks, now 16; 262,144 landmarks, one list: 68 -> 63 us = 6.3 TB/s).
+constexpr int BATCH = 64, STREAM_WARPS = 16;
+template <int NP> constexpr int RING_ROWS = NP > 3 ? 6 : 8;       // 196 KB per SM
+
+template <int NP, bool PER_HEAD>
+__global__ void __launch_bounds__(STREAM_WARPS * 32, 1)
+lmk_stream_kernel(ScanParams p) {
+  constexpr int RING = RING_ROWS<NP>, NL = PER_HEAD ? NP * 4 : 1, MINE = (NL + STREAM_WARPS - 1) / STREAM_WARPS, ROW_BYTES = NP * 512;
+  extern __shared__ __align__(16) unsigned char ring_all[];            // [STREAM_WARPS][RING][ROW_BYTES]
+  __shared__ float score[2][NL][BATCH];
+  pdl_trigger();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int split = blockIdx.x, t0 = blockIdx.y, n = blockIdx.z;
+  const int pieces = p.D >> 3;
+  unsigned char* ring = ring_all + warp * RING * ROW_BYTES + lane * 16;
+  const int e_lo = split * p.e_per_split;
+  // the causal mask is a limit on the landmark id
+  const long long seen = p.q_pos0 + t0 - p.e_base;
+  const int e_hi = (int)max((long long)e_lo, min((long long)min(p.E, e_lo + p.e_per_split), seen));
+  const __nv_bfloat16* kb = p.lk + n * p.kbs + lane * 8;
+  // this warp's i-th row is e_lo + 16 i + warp
+  auto fetch = [&](int i) {
+    const int e = e_lo + i * STREAM_WARPS + warp;
+    if (e < e_hi) {
+      const __nv_bfloat16* src = kb + (long long)e * p.krs;
+      const unsigned dst = (unsigned)__cvta_generic_to_shared(ring + (i % RING) * ROW_BYTES);
+#pragma unroll
+      for (int pp = 0; pp < NP; ++pp)
+        if (lane + 32 * pp < pieces) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + pp * 512), "l"(src + pp * 256) : "memory");
+    }
+  };
+  pdl_wait();
+#pragma unroll
+  for (int i = 0; i < RING; i += 2) {
+    fetch(i);
+    fetch(i + 1);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  float qf[NP][8];
+#pragma unroll
+  for (int pp = 0; pp < NP; ++pp) {
+    const int c = lane + 32 * pp;
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (c < pieces) v = *reinterpret_cast<const uint4*>(p.lq + n * p.qbs + (long long)t0 * p.qrs + c * 8);
+    unpack8(v, qf[pp]);
+  }
+  unsigned long long mine[MINE], kth[MINE];
+#pragma unroll
+  for (int x = 0; x < MINE; ++x) mine[x] = kth[x] = 0ull;
+
+  const int batches = (e_hi - e_lo + BATCH - 1) / BATCH;
+  for (int b = 0; b < batches; ++b) {
+    float (*sc)[BATCH] = score[b & 1];
+#pragma unroll 2
+    for (int i = 0; i < BATCH / STREAM_WARPS; i += 2) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(RING / 2 - 1) : "memory");       // a lane reads only what it copied itself
+      const int i0 = b * (BATCH / STREAM_WARPS) + i;
+      uint4 kv[2][NP];
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int pp = 0; pp < NP; ++pp)
+          kv[u][pp] = lane + 32 * pp < pieces ? *reinterpret_cast<const uint4*>(ring + ((i0 + u) % RING) * ROW_BYTES + pp * 512) : make_uint4(0, 0, 0, 0);
+      float acc[2][PER_HEAD ? NP : 1];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+#pragma unroll
+        for (int x = 0; x < (PER_HEAD ? NP : 1); ++x) acc[u][x] = 0.f;
+#pragma unroll
+        for (int pp = 0; pp < NP; ++pp) {                    // absent pieces add 0 * 0: the sums never are -0
+          float kf[8];
+          unpack8(kv[u][pp], kf);
+#pragma unroll
+          for (int jj = 0; jj < 8; ++jj) acc[u][PER_HEAD ? pp : 0] = fmaf(qf[pp][jj], kf[jj], acc[u][PER_HEAD ? pp : 0]);
+        }
+      }
+      fetch(i0 + RING);
+      fetch(i0 + RING + 1);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+#pragma unroll
+      for (int of = PER_HEAD ? 4 : 16; of > 0; of >>= 1)
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+          for (int x = 0; x < (PER_HEAD ? NP : 1); ++x) acc[u][x] += __shfl_xor_sync(0xffffffffu, acc[u][x], of);
+      if ((lane & (PER_HEAD ? 7 : 31)) == 0)
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+          for (int x = 0; x < (PER_HEAD ? NP : 1); ++x)
+            sc[PER_HEAD ? x * 4 + (lane >> 3) : 0][(i + u) * STREAM_WARPS + warp] =
+                p.score_round ? round_bf16(round_bf16(acc[u][x]) * p.scale) : acc[u][x] * p.scale;
+    }
+    __syncthreads();
+    const int e0 = e_lo + b * BATCH + lane, e1 = e0 + 32;
+#pragma unroll
+    for (int x = 0; x < MINE; ++x) {
+      const int l = warp + x * STREAM_WARPS;
+      if (l >= NL || (PER_HEAD && l >= p.H)) continue;
+      float s0 = sc[l][lane], s1 = sc[l][lane + 32];
+      if (p.noise) {
+        if (e0 < e_hi) s0 += p.noise[((long long)n * p.Cq + t0) * p.E + e0];
+        if (e1 < e_hi) s1 += p.noise[((long long)n * p.Cq + t0) * p.E + e1];
+      }
+      select_batch(mine[x], kth[x], e0 < e_hi ? orderable(s0) : 0u, e1 < e_hi ? orderable(s1) : 0u, (unsigned)(p.e_base + e_lo + b * BATCH), p.K, lane);
+    }
+  }
+#pragma unroll
+  for (int x = 0; x < MINE; ++x) {
+    const int l = warp + x * STREAM_WARPS;
+    if (l >= NL || (PER_HEAD && l >= p.H)) continue;
+    const long long row = ((long long)n * p.Cq + t0) * p.H + l;
+    if (lane < p.K) p.part[(row * p.splits + split) * p.K + lane] = mine[x];
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
+// A few query rows per sequence (TQ per block): one warp scores one landmark row against all of them.
+// NP: pieces per lane (D <= 256*NP).
+template <int NP, int TQ>
 __global__ void __launch_bounds__(SCAN_WARPS * 32)
 lmk_scan_kernel(ScanParams p) {
-  constexpr int NL = PER_HEAD ? NP * 4 : TQ;
-  __shared__ unsigned long long sL[SCAN_WARPS][NL][MAXK];
+  __shared__ unsigned long long sL[SCAN_WARPS][TQ][MAXK];
   pdl_trigger();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int split = blockIdx.x, t0 = blockIdx.y * TQ, n = blockIdx.z;
@@ -66,22 +235,20 @@ lmk_scan_kernel(ScanParams p) {
       unpack8(v, qf[t][pp]);
     }
 
-  unsigned long long mine[NL];
+  unsigned long long mine[TQ];
   // Admission test: a candidate enters a full list only if its score beats the list's K-th
   // score (rows arrive in increasing index order inside a warp, so an equal score loses the
   // tie; scores are never -0).  NaN while the list is not full: "!(s <= NaN)" admits everything.
-  float thr_s[PER_HEAD ? NP : TQ];
+  float thr_s[TQ];
 #pragma unroll
-  for (int l = 0; l < NL; ++l) mine[l] = 0ull;
-#pragma unroll
-  for (int l = 0; l < (PER_HEAD ? NP : TQ); ++l) thr_s[l] = __int_as_float(0x7fc00000);
+  for (int l = 0; l < TQ; ++l) { mine[l] = 0ull; thr_s[l] = __int_as_float(0x7fc00000); }
 
   const int e_lo = split * p.e_per_split;
   const int e_hi = min(p.E, e_lo + p.e_per_split);
   const __nv_bfloat16* kb = p.lk + n * p.kbs;
   // the last query row of the tile sees the most chunks: rows past that limit are skipped
   const long long tile_limit = p.q_pos0 + min(t0 + TQ, p.Cq) - 1;
-  constexpr int U = (TQ == 1 && !PER_HEAD) ? 4 : 2;   // landmark rows in flight per warp iteration
+  constexpr int U = 2;                                // landmark rows in flight per warp iteration
 
   for (int e = e_lo + warp; e < e_hi; e += U * SCAN_WARPS) {
     uint4 kv[U][NP];
@@ -104,54 +271,25 @@ lmk_scan_kernel(ScanParams p) {
       float kf[NP][8];
 #pragma unroll
       for (int pp = 0; pp < NP; ++pp) unpack8(kv[u][pp], kf[pp]);
-      if (!PER_HEAD) {
 #pragma unroll
-        for (int t = 0; t < TQ; ++t) {
-          float acc = 0.f;
+      for (int t = 0; t < TQ; ++t) {
+        float acc = 0.f;
 #pragma unroll
-          for (int pp = 0; pp < NP; ++pp)
-            if (lane + 32 * pp < pieces) {
-#pragma unroll
-              for (int jj = 0; jj < 8; ++jj) acc = fmaf(qf[t][pp][jj], kf[pp][jj], acc);
-            }
-#pragma unroll
-          for (int of = 16; of > 0; of >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, of);
-          float s = p.score_round ? round_bf16(round_bf16(acc) * p.scale) : acc * p.scale;
-          const int row = t0 + t;
-          const bool vis = row < p.Cq && eg < p.q_pos0 + row;
-          if (p.noise && vis) s += p.noise[((long long)n * p.Cq + row) * p.E + eu];
-          if (vis && !(s <= thr_s[t])) {
-            list_insert(mine[t], make_key(s, (unsigned)eg), lane);
-            const unsigned long long kth = __shfl_sync(0xffffffffu, mine[t], p.K - 1);
-            if (kth != 0ull) thr_s[t] = from_orderable((unsigned)(kth >> 32));
-          }
-        }
-      } else {
-        const bool vis = eg < p.q_pos0 + t0;
-#pragma unroll
-        for (int pp = 0; pp < NP; ++pp) {
-          float acc = 0.f;
+        for (int pp = 0; pp < NP; ++pp)
           if (lane + 32 * pp < pieces) {
 #pragma unroll
-            for (int jj = 0; jj < 8; ++jj) acc = fmaf(qf[0][pp][jj], kf[pp][jj], acc);
+            for (int jj = 0; jj < 8; ++jj) acc = fmaf(qf[t][pp][jj], kf[pp][jj], acc);
           }
 #pragma unroll
-          for (int of = 4; of > 0; of >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, of);
-          // lanes 8g..8g+7 now hold the score of head 4*pp + g; each lane group tests it against
-          // its own head's threshold, and only rows with a candidate take the uniform path
-          const float s_loc = p.score_round ? round_bf16(round_bf16(acc) * p.scale) : acc * p.scale;
-          const unsigned cand = __ballot_sync(0xffffffffu, vis && !(s_loc <= thr_s[pp]));
-          if (cand == 0) continue;
-#pragma unroll
-          for (int hg = 0; hg < 4; ++hg) {
-            if (!((cand >> (8 * hg)) & 1u)) continue;
-            const int l = pp * 4 + hg;
-            if (l >= p.H) continue;
-            const float s = __shfl_sync(0xffffffffu, s_loc, hg * 8);
-            list_insert(mine[l], make_key(s, (unsigned)eg), lane);
-            const unsigned long long kth = __shfl_sync(0xffffffffu, mine[l], p.K - 1);
-            if (kth != 0ull && (lane >> 3) == hg) thr_s[pp] = from_orderable((unsigned)(kth >> 32));
-          }
+        for (int of = 16; of > 0; of >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, of);
+        float s = p.score_round ? round_bf16(round_bf16(acc) * p.scale) : acc * p.scale;
+        const int row = t0 + t;
+        const bool vis = row < p.Cq && eg < p.q_pos0 + row;
+        if (p.noise && vis) s += p.noise[((long long)n * p.Cq + row) * p.E + eu];
+        if (vis && !(s <= thr_s[t])) {
+          list_insert(mine[t], make_key(s, (unsigned)eg), lane);
+          const unsigned long long kth = __shfl_sync(0xffffffffu, mine[t], p.K - 1);
+          if (kth != 0ull) thr_s[t] = from_orderable((unsigned)(kth >> 32));
         }
       }
     }
@@ -159,15 +297,14 @@ lmk_scan_kernel(ScanParams p) {
 
   // merge the 8 per-warp lists of every row of the tile; list l is merged by warp l % 8
 #pragma unroll
-  for (int l = 0; l < NL; ++l)
+  for (int l = 0; l < TQ; ++l)
     if (lane < p.K) sL[warp][l][lane] = mine[l];
   __syncthreads();
 #pragma unroll
-  for (int l = 0; l < NL; ++l) {
+  for (int l = 0; l < TQ; ++l) {
     if ((l % SCAN_WARPS) != warp) continue;
-    long long row;
-    if (PER_HEAD) { if (l >= p.H) continue; row = ((long long)n * p.Cq + t0) * p.H + l; }
-    else          { if (t0 + l >= p.Cq) continue; row = (long long)n * p.Cq + t0 + l; }
+    if (t0 + l >= p.Cq) continue;
+    const long long row = (long long)n * p.Cq + t0 + l;
     unsigned long long m = 0ull, th = 0ull;
     for (int w = 0; w < SCAN_WARPS; ++w)
       for (int i = 0; i < p.K; ++i) {
@@ -224,6 +361,7 @@ __global__ void __launch_bounds__(FIN_WARPS * 32)
 lmk_merge_rows_kernel(FinalParams p) {
   const int lane = threadIdx.x & 31;
   const long long row = (long long)blockIdx.x * FIN_WARPS + (threadIdx.x >> 5);
+  pdl_trigger();
   pdl_wait();
   if (row >= p.R) return;
   const unsigned long long* src = p.keys + row * p.P + (long long)lane * p.K;
@@ -255,6 +393,7 @@ lmk_rank_merge_kernel(FinalParams p) {
   const int padded = (lists + 1) & ~1;
   const unsigned long long* src = p.keys + (long long)blockIdx.x * p.P;
   if (tid < MAXK) { by_rank[tid] = -1; best[tid] = 0ull; }
+  pdl_trigger();
   pdl_wait();
   for (int i = tid; i < padded; i += FIN_WARPS * 32) heads[i] = i < lists ? src[(long long)i * K] : 0ull;
   __syncthreads();
@@ -404,13 +543,38 @@ int scan_splits(const LmkTopkArgs& a, int sms) {
 
 namespace {
 
-int choose_splits(const LmkTopkArgs& a, int sms) { return a.splits > 0 ? a.splits : scan_splits(a, sms); }
+// Landmark ranges of the streaming form: one block per SM at a time, so what counts is whole waves; a block costs about as much
+// again as reading 96 rows before and after its stream.
+int stream_splits(const LmkTopkArgs& a, int sms) {
+  const long long blocks = (long long)a.N * a.Cq;
+  const int most = (int)std::min<long long>((a.E + BATCH - 1) / BATCH, 2 * sms);
+  int best = 1;
+  long long best_cost = -1;
+  for (int s = 1; s <= most; ++s) {
+    const long long cost = (blocks * s + sms - 1) / sms * ((a.E + s - 1) / s + 96);
+    if (best_cost < 0 || cost < best_cost) { best = s; best_cost = cost; }
+  }
+  return best;
+}
+
+int choose_splits(const LmkTopkArgs& a, int sms) {
+  return a.splits > 0 ? a.splits : pick_tq(a) == 1 ? stream_splits(a, sms) : scan_splits(a, sms);
+}
+
+template <int NP, bool PER_HEAD>
+int launch_stream(const ScanParams& sp, dim3 grid, cudaStream_t stream) {
+  constexpr int smem = STREAM_WARPS * RING_ROWS<NP> * NP * 512;
+  GCA_CUDA_CHECK(cudaFuncSetAttribute(lmk_stream_kernel<NP, PER_HEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  return (int)launch_dependent(lmk_stream_kernel<NP, PER_HEAD>, grid, dim3(STREAM_WARPS * 32), smem, stream, sp);
+}
 
 template <int NP>
-void launch_scan(const ScanParams& sp, int tq, bool per_head, dim3 grid, cudaStream_t stream) {
-  if (per_head) lmk_scan_kernel<NP, 1, true><<<grid, SCAN_WARPS * 32, 0, stream>>>(sp);
-  else if (tq == 1) lmk_scan_kernel<NP, 1, false><<<grid, SCAN_WARPS * 32, 0, stream>>>(sp);
-  else lmk_scan_kernel<NP, 4, false><<<grid, SCAN_WARPS * 32, 0, stream>>>(sp);
+int launch_scan(const ScanParams& sp, int tq, bool per_head, cudaStream_t stream) {
+  const dim3 grid((unsigned)sp.splits, (unsigned)((sp.Cq + tq - 1) / tq), (unsigned)sp.N);
+  if (per_head) return launch_stream<NP, true>(sp, grid, stream);
+  if (tq == 1) return launch_stream<NP, false>(sp, grid, stream);
+  lmk_scan_kernel<NP, 4><<<grid, SCAN_WARPS * 32, 0, stream>>>(sp);
+  return (int)cudaGetLastError();
 }
 
 }  // namespace
@@ -449,15 +613,15 @@ int launch_lmk_score_topk(const LmkTopkArgs& a, void* scratch, int sms, cudaStre
   sp.N = a.N; sp.Cq = a.Cq; sp.E = a.E; sp.D = a.D; sp.K = a.K; sp.H = per_head ? a.D / a.head_dim : 1;
   sp.splits = splits; sp.e_per_split = (a.E + splits - 1) / splits;
   sp.score_round = a.score_round; sp.scale = scale;
-  const dim3 grid((unsigned)splits, (unsigned)((a.Cq + tq - 1) / tq), (unsigned)a.N);
+  int rc;
   switch ((a.D + 255) / 256) {
-    case 1: launch_scan<1>(sp, tq, per_head, grid, stream); break;
-    case 2: launch_scan<2>(sp, tq, per_head, grid, stream); break;
-    case 3: launch_scan<3>(sp, tq, per_head, grid, stream); break;
-    case 4: launch_scan<4>(sp, tq, per_head, grid, stream); break;
-    default: return GCA_ERR_SHAPE;
+    case 1: rc = launch_scan<1>(sp, tq, per_head, stream); break;
+    case 2: rc = launch_scan<2>(sp, tq, per_head, stream); break;
+    case 3: rc = launch_scan<3>(sp, tq, per_head, stream); break;
+    case 4: rc = launch_scan<4>(sp, tq, per_head, stream); break;
+    default: rc = GCA_ERR_SHAPE;
   }
-  GCA_CUDA_CHECK(cudaGetLastError());
+  if (rc) return rc;
   if (a.noise == nullptr || per_head) fp.lq = nullptr;          // the keys hold the noise-free scores
   fp.P = splits * a.K; fp.lists = splits;
   // a warp per row up to 32 lists, a block per row beyond
