@@ -442,7 +442,10 @@ typedef struct LinearBatchedArgs {
   LinearArgs one;
   int64_t x_batch_stride, out_batch_stride, residual_batch_stride, scale_batch_stride;
   int32_t batches, lead_rows;
+  float rms_eps;              /* > 0: scale the rows by rsqrt(mean(x^2) + rms_eps), computed on the way (row_scale NULL);
+                                 for up to GCA_SKINNY_ROWS rows in all, lying back to back, else GCA_ERR_SHAPE */
 } LinearBatchedArgs;
+#define GCA_SKINNY_ROWS 128   /* up to this many rows take the latency-bound form of gca_linear */
 
 int gca_linear_batched(const LinearBatchedArgs* args, void* stream);
 

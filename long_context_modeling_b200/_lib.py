@@ -130,7 +130,7 @@ class LinearArgs(C.Structure):
 
 class LinearBatchedArgs(C.Structure):
     _fields_ = [("one", LinearArgs), ("x_batch_stride", C.c_int64), ("out_batch_stride", C.c_int64), ("residual_batch_stride", C.c_int64),
-                ("scale_batch_stride", C.c_int64), ("batches", C.c_int32), ("lead_rows", C.c_int32)]
+                ("scale_batch_stride", C.c_int64), ("batches", C.c_int32), ("lead_rows", C.c_int32), ("rms_eps", C.c_float)]
 
 
 class WindowDecodeArgs(C.Structure):

@@ -51,6 +51,20 @@ inline cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 b
   return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
 }
 
+// The same as pairs of CTAs (clusters of two along x).
+template <class... Params, class... Args>
+inline cudaError_t launch_dependent_pairs(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = 2; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = 2;
+  return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+}
+
 // Problem geometry shared by forward and backward kernels (passed by value).
 struct Geom {
   int N, J, Hq, Hkv, S, L, D, K, C, G;

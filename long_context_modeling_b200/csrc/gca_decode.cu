@@ -255,6 +255,8 @@ decode_rows_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
   const int n = zj / g.J, j = zj - n * g.J;
   const int rows = g.G * g.S;                                    // <= R
   const float c2 = g.sm_scale * GCA_LOG2E;
+  pdl_trigger();
+  pdl_wait();
   float qv[R][8];
 #pragma unroll
   for (int r = 0; r < R; ++r) {
@@ -366,6 +368,124 @@ decode_rows_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
   }
 }
 
+// The same for so few (sequence, kv head) items that the SMs are not all busy: WPS warps share a slot (64 / WPS keys each, all
+// their loads in flight at once), the partial softmax states meet in shared memory.  One sequence, 12 heads, K = 8, behind the
+// projection it depends on: 6.0 -> ~4 us.
+template <int R, int WPS>
+__global__ void __launch_bounds__(NWARPS * WPS * 32)
+decode_split_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ kc, const __nv_bfloat16* __restrict__ vc,
+                    const int32_t* __restrict__ indices, const float* __restrict__ weights, __nv_bfloat16* __restrict__ out,
+                    int32_t* status, const Geom g) {
+  constexpr int STEPS = 16 / WPS, PITCH = 66;                    // (maximum, sum, 64 outputs)
+  extern __shared__ float part[];                                // [K][WPS][R][PITCH]
+  __shared__ float slot_w[32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = lane >> 3, sub = lane & 7;
+  const int item = blockIdx.x;
+  const int zj = item / g.Hkv, hk = item - zj * g.Hkv;
+  const int n = zj / g.J, j = zj - n * g.J;
+  const int rows = g.G * g.S;
+  const float c2 = g.sm_scale * GCA_LOG2E;
+  pdl_trigger();
+  pdl_wait();
+  uint4 qv[R];                                                   // this lane's 8 query values of every row, as they came
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    qv[r] = make_uint4(0, 0, 0, 0);
+    if (r < rows) {
+      const int gi = r / g.S, s = r - gi * g.S;
+      qv[r] = *reinterpret_cast<const uint4*>(q + n * g.qs[0] + j * g.qs[1] + (hk * g.G + gi) * g.qs[2] + s * g.qs[3] + sub * 8);
+    }
+  }
+  const int share = warp % WPS;
+  for (int k = warp / WPS; k < g.K; k += NWARPS) {
+    const int idx = slot_chunk(indices, zj, g.K, k);
+    const bool live = idx >= 0 && idx < g.C;
+    if (share == 0 && lane == 0) {
+      if (idx >= g.C && status) atomicOr(status, GCA_STATUS_BAD_INDEX);
+      slot_w[k] = live ? weights[(long long)zj * g.K + k] : 0.f;
+    }
+    if (!live) continue;
+    const int key0 = share * (64 / WPS) + grp;
+    const __nv_bfloat16* kb = kc + n * g.ks[0] + idx * g.ks[1] + hk * g.ks[3] + sub * 8;
+    const __nv_bfloat16* vb = vc + n * g.vs[0] + idx * g.vs[1] + hk * g.vs[3] + sub * 8;
+    uint4 kq[STEPS], vq[STEPS];
+#pragma unroll
+    for (int s = 0; s < STEPS; ++s) {
+      kq[s] = *reinterpret_cast<const uint4*>(kb + (key0 + s * 4) * g.ks[2]);
+      vq[s] = *reinterpret_cast<const uint4*>(vb + (key0 + s * 4) * g.vs[2]);
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      float sc[STEPS], m = -INFINITY;
+      const unsigned qw[4] = {qv[r].x, qv[r].y, qv[r].z, qv[r].w};
+#pragma unroll
+      for (int s = 0; s < STEPS; ++s) {
+        const unsigned kw[4] = {kq[s].x, kq[s].y, kq[s].z, kq[s].w};
+        float t = 0.f;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { t = fmaf(bf_lo(qw[e]), bf_lo(kw[e]), t); t = fmaf(bf_hi(qw[e]), bf_hi(kw[e]), t); }
+        sc[s] = t * c2;
+      }
+#pragma unroll
+      for (int of = 1; of < 8; of <<= 1)
+#pragma unroll
+        for (int s = 0; s < STEPS; ++s) sc[s] += __shfl_xor_sync(0xffffffffu, sc[s], of);
+#pragma unroll
+      for (int s = 0; s < STEPS; ++s) m = fmaxf(m, sc[s]);
+      m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
+      m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16));
+      float l = 0.f, acc[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[e] = 0.f;
+#pragma unroll
+      for (int s = 0; s < STEPS; ++s) {
+        const float pr = ex2f(sc[s] - m);
+        l += pr;
+        const unsigned vw[4] = {vq[s].x, vq[s].y, vq[s].z, vq[s].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { acc[2 * e] = fmaf(pr, bf_lo(vw[e]), acc[2 * e]); acc[2 * e + 1] = fmaf(pr, bf_hi(vw[e]), acc[2 * e + 1]); }
+      }
+#pragma unroll
+      for (int of = 8; of <= 16; of <<= 1) {
+        l += __shfl_xor_sync(0xffffffffu, l, of);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], of);
+      }
+      float* dst = part + ((k * WPS + share) * R + r) * PITCH;
+      if (lane == 0) { dst[0] = m; dst[1] = l; }
+      if (grp == 0) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) dst[2 + sub * 8 + e] = acc[e];
+      }
+    }
+  }
+  __syncthreads();
+  // out = sum over slots of w * (merged numerator) / (merged sum), in slot order
+  for (int i = threadIdx.x; i < rows * 64; i += NWARPS * WPS * 32) {
+    const int r = i >> 6, d = i & 63;
+    float t = 0.f;
+    for (int k = 0; k < g.K; ++k) {
+      const float w = slot_w[k];
+      const int idx = slot_chunk(indices, zj, g.K, k);
+      if (idx < 0 || idx >= g.C) continue;
+      const float* src = part + (k * WPS * R + r) * PITCH;
+      float m = g.off_by_one > 0.f ? 0.f : -INFINITY;
+#pragma unroll
+      for (int x = 0; x < WPS; ++x) m = fmaxf(m, src[x * R * PITCH]);
+      float l = g.off_by_one > 0.f ? g.off_by_one * ex2f(-m) : 0.f, o = 0.f;
+#pragma unroll
+      for (int x = 0; x < WPS; ++x) {
+        const float c = ex2f(src[x * R * PITCH] - m);
+        l = fmaf(src[x * R * PITCH + 1], c, l);
+        o = fmaf(src[x * R * PITCH + 2 + d], c, o);
+      }
+      t = fmaf(o, w / l, t);
+    }
+    const int gi = r / g.S, s = r - gi * g.S;
+    out[n * g.os[0] + j * g.os[1] + (hk * g.G + gi) * g.os[2] + s * g.os[3] + d] = __float2bfloat16_rn(t);
+  }
+}
+
 template <int R>
 int launch_decode_r(const DecParams& p, int blocks, int sms, cudaStream_t stream) {
   const size_t smem = NWARPS * 2 * TILE_BYTES + 2 * (1 + NWARPS) * R * T * sizeof(float) + 256 + 1024;
@@ -397,10 +517,19 @@ int launch_decode(const GcaFwdArgs& a, int sms, cudaStream_t stream) {
   if (rows <= 4 && blocks > 0 && a.D == 64 && a.L == 64 && vec16) {
     auto q = (const __nv_bfloat16*)a.q; auto kc = (const __nv_bfloat16*)a.k_cache; auto vc = (const __nv_bfloat16*)a.v_cache;
     auto out = (__nv_bfloat16*)a.out;
-    if (rows <= 1) decode_rows_kernel<1><<<(unsigned)blocks, NWARPS * 32, 0, stream>>>(q, kc, vc, a.indices, a.weights, out, a.status, g);
-    else if (rows <= 2) decode_rows_kernel<2><<<(unsigned)blocks, NWARPS * 32, 0, stream>>>(q, kc, vc, a.indices, a.weights, out, a.status, g);
-    else decode_rows_kernel<4><<<(unsigned)blocks, NWARPS * 32, 0, stream>>>(q, kc, vc, a.indices, a.weights, out, a.status, g);
-    return (int)cudaGetLastError();
+    // warps per slot while whole SMs would be idle (the states of all slots fit 48 KB of shared memory)
+    const int wps = rows <= 2 && blocks <= sms ? 4 : rows <= 2 && blocks <= 2 * sms ? 2 : 1;
+    const size_t smem = (size_t)a.K * wps * (rows <= 1 ? 1 : 2) * 66 * sizeof(float);
+    auto run = [&](auto kernel, int threads, size_t bytes) {
+      return (int)launch_dependent(kernel, dim3((unsigned)blocks), dim3(threads), bytes, stream, q, kc, vc, a.indices, a.weights, out, a.status, g);
+    };
+    if (wps > 1 && smem <= 48 * 1024) {
+      if (rows <= 1) return wps == 4 ? run(decode_split_kernel<1, 4>, NWARPS * 128, smem) : run(decode_split_kernel<1, 2>, NWARPS * 64, smem);
+      return wps == 4 ? run(decode_split_kernel<2, 4>, NWARPS * 128, smem) : run(decode_split_kernel<2, 2>, NWARPS * 64, smem);
+    }
+    if (rows <= 1) return run(decode_rows_kernel<1>, NWARPS * 32, 0);
+    if (rows <= 2) return run(decode_rows_kernel<2>, NWARPS * 32, 0);
+    return run(decode_rows_kernel<4>, NWARPS * 32, 0);
   }
   int rc;
   if ((rc = make_tile_map_5d(&p.tm_k, a.k_cache, 64, 64, a.Hkv, a.C, a.N, a.k_stride[2], a.k_stride[3], a.k_stride[1], a.k_stride[0], 1, true))) return rc;

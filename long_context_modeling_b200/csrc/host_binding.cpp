@@ -451,6 +451,24 @@ Tensor linear(const Tensor& x, const Tensor& weight, const Tensor& row_scale, co
   return out;
 }
 
+// RMSNorm(x) w^T with the norm's gain in w: a few rows are one launch, more take a row reduction and the GEMM's epilogue.
+Tensor rmsnorm_linear(const Tensor& x, const Tensor& weight, double eps) {
+  at::AutoDispatchBelowADInplaceOrView below;
+  const Rows r = rows_of(x);
+  if (r.m > GCA_SKINNY_ROWS) return linear(x, weight, row_rms(x, eps), Tensor(), Tensor());
+  Launch on(x);
+  c10::SmallVector<int64_t, 6> shape(x.sizes().begin(), x.sizes().end());
+  shape.back() = weight.size(0);
+  const Tensor out = at::empty(shape, x.options());
+  LinearBatchedArgs lp{};
+  lp.one.x = r.hold.const_data_ptr(); lp.one.w = weight.const_data_ptr(); lp.one.out = out.mutable_data_ptr();
+  lp.one.M = r.m; lp.one.N = (int32_t)weight.size(0); lp.one.K = (int32_t)x.size(-1);
+  lp.one.x_stride = r.stride; lp.one.w_stride = weight.stride(0); lp.one.out_stride = weight.size(0);
+  lp.batches = 1; lp.rms_eps = (float)eps;
+  call("gca_linear", [&] { return api.gca_linear_batched(&lp, on.stream); });
+  return out;
+}
+
 // One GCA sub-layer for inference: residual + o_proj(GCA(q_proj(RMSNorm(hidden)))) on hidden (n, chunks, s, dim).
 // The q rows and the attention's output are token-major buffers, so nothing is re-laid out between the
 // three steps, and the rows of a skipped first chunk (nothing retrieved: the residual alone, or zeros) are written by
@@ -477,19 +495,24 @@ Tensor layer_fused(const Tensor& hidden_in, const Tensor& q_weight, double eps, 
   }
   const int64_t skip = chunks > 1 && !first_chunk_retrieves ? 1 : 0, J = chunks - skip, rows = J * s;
   const Tensor idx = as_int32(idx_in), w = as_float(w_in);
-  const Tensor scale = at::empty({n * chunks * s}, hidden.options().dtype(at::kFloat));
+  const bool few = n * rows <= GCA_SKINNY_ROWS && skip == 0;             // the norm rides on the projection
   const Tensor q = at::empty({2, n, J, s, dim}, hidden.options());      // [0]: q, [1]: the attention's output
   void* const vals = static_cast<char*>(q.mutable_data_ptr()) + q.stride(0) * 2;
-  RowRmsArgs rr;
-  rr.x = hidden.const_data_ptr(); rr.row_scale = scale.mutable_data_ptr<float>(); rr.M = n * chunks * s; rr.x_stride = dim;
-  rr.D = (int32_t)dim; rr.eps = (float)eps;
-  call("gca_row_rms", [&] { return api.gca_row_rms(&rr, on.stream); });
+  Tensor scale;
+  if (!few) {
+    scale = at::empty({n * chunks * s}, hidden.options().dtype(at::kFloat));
+    RowRmsArgs rr;
+    rr.x = hidden.const_data_ptr(); rr.row_scale = scale.mutable_data_ptr<float>(); rr.M = n * chunks * s; rr.x_stride = dim;
+    rr.D = (int32_t)dim; rr.eps = (float)eps;
+    call("gca_row_rms", [&] { return api.gca_row_rms(&rr, on.stream); });
+  }
   LinearBatchedArgs lp{};
   LinearArgs& a = lp.one;
   a.x = static_cast<const char*>(hidden.const_data_ptr()) + skip * s * dim * 2; a.w = q_weight.const_data_ptr(); a.out = q.mutable_data_ptr();
   a.M = rows; a.N = (int32_t)q_weight.size(0); a.K = (int32_t)dim;
   a.x_stride = dim; a.w_stride = q_weight.stride(0); a.out_stride = dim;
-  a.row_scale = scale.const_data_ptr<float>() + skip * s;
+  if (few) lp.rms_eps = (float)eps;
+  else a.row_scale = scale.const_data_ptr<float>() + skip * s;
   a.status = status_ptr(on.dev);
   lp.batches = (int32_t)n; lp.x_batch_stride = chunks * s * dim; lp.out_batch_stride = rows * dim; lp.scale_batch_stride = chunks * s;
   call("gca_linear", [&] { return api.gca_linear_batched(&lp, on.stream); });
@@ -515,6 +538,7 @@ Tensor layer_fused(const Tensor& hidden_in, const Tensor& q_weight, double eps, 
   a.x = vals; a.w = o_weight.const_data_ptr(); a.w_stride = o_weight.stride(0); a.N = (int32_t)o_weight.size(0);
   a.out = static_cast<char*>(out.mutable_data_ptr()) + skip * s * dim * 2;
   a.row_scale = nullptr;
+  lp.rms_eps = 0.f;
   lp.x_batch_stride = rows * dim; lp.out_batch_stride = chunks * s * dim;
   lp.lead_rows = (int32_t)(skip * s);
   if (residual.defined()) {
@@ -921,6 +945,14 @@ ENTRY(retrieve, 5)
   return wrap_tuple({r.indices, r.weights, r.full.keys, r.full.indices, r.full.scores, r.full.weights, r.full.n_valid});
 ENTRY_END
 
+ENTRY(rmsnorm_linear, 3)
+  const Tensor &x = a.tensor(0), &w = a.tensor(1);
+  require_bf16(x, "linear");
+  require_bf16(w, "linear weight");
+  const double eps = a.real(2);
+  return wrap(unlocked([&] { return rmsnorm_linear(x, w, eps); }));
+ENTRY_END
+
 // (hidden, q weight with the norm's gain, eps, k, v, idx, w, o weight, residual or None, first chunk retrieves, heads, scale)
 ENTRY(layer_fused, 12)
   const Tensor &x = a.tensor(0), &qw = a.tensor(1), &k = a.tensor(3), &v = a.tensor(4), &idx = a.tensor(5), &w = a.tensor(6), &ow = a.tensor(7);
@@ -1010,7 +1042,7 @@ ENTRY_END
 #define METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(&py_##name)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
     METHOD(bind), METHOD(set_switches), METHOD(status_word), METHOD(gca_indexed), METHOD(attention), METHOD(gca_nograd), METHOD(gca_kv_cache),
-    METHOD(gca_forward_lse), METHOD(gca_backward), METHOD(row_rms), METHOD(linear), METHOD(layer_fused), METHOD(silu_mul),
+    METHOD(gca_forward_lse), METHOD(gca_backward), METHOD(row_rms), METHOD(linear), METHOD(rmsnorm_linear), METHOD(layer_fused), METHOD(silu_mul),
     METHOD(window_decode), METHOD(window_ring_decode), METHOD(lmk_score_topk), METHOD(retrieve), METHOD(kv_project_append), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_host", "Host path of the hot entry points.", -1, methods, nullptr, nullptr, nullptr, nullptr};
 

@@ -10,11 +10,17 @@
 //   Wk, Wv (D x D) bf16 in nn.Linear layout (out, in) = K-major B operand
 //   K_cache[n, pos + c, s, :] = X[(n, c, s), :] Wk^T   (zeros for s = 63 when zero_landmark)
 //
-// tcgen05 GEMM, one CTA per SM, persistent over (row tile of 128, column tile of 256, K|V):
-// warp 0 issues the TMA copies of a 4-stage ring (A 128 x 64, B 256 x 64 per stage), warp 1 issues
-// 128 x 256 x 16 MMAs into one of two 256-column accumulators in tensor memory, warps 2-5 turn a
-// finished accumulator into bf16 rows of the cache while the next tile is being multiplied.
-// Every wait is bounded (GCA_STATUS_TIMEOUT on expiry).
+// tcgen05 GEMM, one CTA per SM, persistent over (row tile, column tile, K|V): warp 0 issues the TMA copies of a ring of
+// 64-deep stages, warp 1 the MMAs into one of two accumulators in tensor memory, eight epilogue warps (two per lane quarter,
+// half of the columns each) turn a finished accumulator into bf16 rows of the cache while the next tile is being multiplied;
+// the warp that has a chunk's last row also copies it to the landmark cache.  Every wait is bounded
+// (GCA_STATUS_TIMEOUT on expiry).
+// Tiles (chosen by choose_tile): PAIRS of CTAs on 256 x 256 (cta_group::2) for large products, where each CTA loads half of the
+// weight rows: per product a third less shared-memory and L2 traffic than 128 x 256, and power is what a large
+// product is bound by (SM clock 1.3-1.6 GHz of 1.97 within milliseconds).  8 x 260 chunks x 64 rows, 768 -> 2 x 768: 307 -> 287 us
+// back to back, 255 -> 231 us for a single launch; cuBLAS needs 298 / 266 us for the bare product.  Smaller products take the width of 64,
+// 128 or 256 columns whose waves cost least: 6,912 rows 768 -> 768 on 148 SMs are 162 tiles of 256 columns (two
+// waves, the second nearly empty) but 324 of 128: 33 -> 19 us.
 //
 // The same kernel in LINEAR mode is the projection either side of GCA (model/DRT.py:352-355,385):
 //   out[m, :] = row_scale[m] * (x[m, :] W^T) + residual[m, :]
@@ -38,14 +44,21 @@ namespace {
 
 using namespace sm100;
 
-constexpr int BM = 128, BN = 256, BK = 64;
-constexpr int STAGES = 4;
-constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
-constexpr int OFF_BAR = STAGES * STAGE_BYTES;
-constexpr int SMEM_BYTES = OFF_BAR + 256 + 1024;
-constexpr int NTHREADS = 6 * 32;
-enum Bar { FULL = 0, EMPTY = FULL + STAGES, ACC_FULL = EMPTY + STAGES, ACC_EMPTY = ACC_FULL + 2, NUM_BARS = ACC_EMPTY + 2 };
-constexpr uint32_t IDESC = umma_idesc_bf16(BM, BN, 0, 0);
+constexpr int BM = 128, BK = 64;                      // rows of a CTA's accumulator, K step
+constexpr int EPI_WARPS = 8, NTHREADS = (2 + EPI_WARPS) * 32;
+
+// BN: columns of a tile.  PAIR: two CTAs share a tile of 256 rows (cta_group::2), each loading half of the weight rows.
+template <int BN, bool PAIR>
+struct Cfg {
+  static constexpr int B_ROWS = PAIR ? BN / 2 : BN;
+  static constexpr int A_BYTES = BM * BK * 2, STAGE_BYTES = A_BYTES + B_ROWS * BK * 2;
+  static constexpr int STAGES = 196608 / STAGE_BYTES;
+  static constexpr int OFF_BAR = STAGES * STAGE_BYTES, SMEM_BYTES = OFF_BAR + 256 + 1024;
+  static constexpr int FULL = 0, EMPTY = FULL + STAGES, ACC_FULL = EMPTY + STAGES, ACC_EMPTY = ACC_FULL + 2, NUM_BARS = ACC_EMPTY + 2;
+  static constexpr uint32_t IDESC = umma_idesc_bf16(PAIR ? 2 * BM : BM, BN, 0, 0);
+  static constexpr int TM = PAIR ? 2 * BM : BM;        // rows of a tile
+  static_assert(NUM_BARS * 8 + 8 <= 256, "barriers fit their space");
+};
 
 struct ProjParams {
   CUtensorMap tm_x, tm_wk, tm_wv;
@@ -55,7 +68,11 @@ struct ProjParams {
   long long cache_bs;       // elements between sequences in the caches
   int M, D, rows_per_seq;   // D = contraction length; rows_per_seq = count * 64
   int pos;                  // first chunk position written
+  const uint4* x_rows;      // append: x itself and the landmark cache its chunks' last rows go to (or nullptr)
+  uint4* lmk;
+  long long lmk_bs;         // 16-byte vectors between sequences
   int zero_landmark;
+  int wide;                 // output rows start on 32-byte boundaries
   int tiles_m, tiles_n;     // tiles_n = ceil(output columns / BN)
   int nmat;                 // 2: K and V projection with append epilogue; 1: linear mode
   // linear mode: `batches` blocks of M rows, each cut in 64-row blocks (a 128-row tile is two of them, whatever
@@ -82,8 +99,12 @@ __device__ __forceinline__ void tile_of(const ProjParams& p, int t, int& which, 
   else { which = 0; tm = r; }
 }
 
+template <int BN, bool PAIR>
 __global__ void __launch_bounds__(NTHREADS, 1)
 kv_project_append_kernel(const __grid_constant__ ProjParams p) {
+  using C = Cfg<BN, PAIR>;
+  constexpr int STAGES = C::STAGES, STAGE_BYTES = C::STAGE_BYTES, A_BYTES = C::A_BYTES, OFF_BAR = C::OFF_BAR, NUM_BARS = C::NUM_BARS;
+  constexpr int FULL = C::FULL, EMPTY = C::EMPTY, ACC_FULL = C::ACC_FULL, ACC_EMPTY = C::ACC_EMPTY, TMEM_COLS = 2 * BN;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
@@ -92,25 +113,34 @@ kv_project_append_kernel(const __grid_constant__ ProjParams p) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int total = p.tiles_m * p.tiles_n * p.nmat;
   const int ksteps = p.D / BK;
+  const uint32_t rank = PAIR ? cluster_rank() : 0u;
+  const int first = PAIR ? blockIdx.x / 2 : blockIdx.x, step = PAIR ? gridDim.x / 2 : gridDim.x;
   if (threadIdx.x == 0) {
     for (int i = 0; i < STAGES; ++i) { mbar_init(&bars[FULL + i], 1); mbar_init(&bars[EMPTY + i], 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&bars[ACC_FULL + i], 1); mbar_init(&bars[ACC_EMPTY + i], 128); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&bars[ACC_FULL + i], 1); mbar_init(&bars[ACC_EMPTY + i], (PAIR ? 2 : 1) * EPI_WARPS); }
     *abort_flag = 0;
     fence_barrier_init();
   }
-  if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  if (warp == 1) {
+    if (PAIR) tmem_alloc_pair(tmem_slot, TMEM_COLS);
+    else { tmem_alloc(tmem_slot, TMEM_COLS); tmem_relinquish(); }
+  }
   if (warp == 0 && lane == 0) { tma_prefetch_desc(&p.tm_x); tma_prefetch_desc(&p.tm_wk); tma_prefetch_desc(&p.tm_wv); }
   tc_fence_before();
-  __syncthreads();
+  __syncwarp();
+  if (PAIR) cluster_sync();
+  else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_trigger();
+  pdl_wait();
 
   if (warp == 0) {
     if (lane == 0) {
       Ring ring; ring.init(STAGES);
       uint32_t issued = 0;
       bool ok = true;
-      for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+      for (int t = first; t < total && ok; t += step) {
         int which, tm, tn;
         tile_of(p, t, which, tm, tn);
         const CUtensorMap* tw = which ? &p.tm_wv : &p.tm_wk;
@@ -118,20 +148,30 @@ kv_project_append_kernel(const __grid_constant__ ProjParams p) {
           ok = mbar_wait_bounded(&bars[EMPTY + ring.st], ring.ph ^ 1, abort_flag);
           if (!ok) break;
           uint8_t* dst = smem + ring.st * STAGE_BYTES;
-          mbar_arrive_expect_tx(&bars[FULL + ring.st], STAGE_BYTES);
+          uint64_t* full = &bars[FULL + ring.st];
+          if (rank == 0) mbar_arrive_expect_tx(full, (PAIR ? 2 : 1) * STAGE_BYTES);
           if (p.blocks_per_batch) {                            // linear mode: two 64-row blocks (rows past the end are zero-filled)
-            const int b0 = (2 * tm) / p.blocks_per_batch, b1 = (2 * tm + 1) / p.blocks_per_batch;
-            tma_load_3d(dst, &p.tm_x, &bars[FULL + ring.st], ks * BK, (2 * tm - b0 * p.blocks_per_batch) * 64, b0);
-            tma_load_3d(dst + A_BYTES / 2, &p.tm_x, &bars[FULL + ring.st], ks * BK, (2 * tm + 1 - b1 * p.blocks_per_batch) * 64, b1);
+            const int blk = (C::TM / 64) * tm + 2 * (int)rank, b0 = blk / p.blocks_per_batch, b1 = (blk + 1) / p.blocks_per_batch;
+            const int r0 = (blk - b0 * p.blocks_per_batch) * 64, r1 = (blk + 1 - b1 * p.blocks_per_batch) * 64;
+            if (PAIR) {
+              tma_load_3d_pair(dst, &p.tm_x, full, ks * BK, r0, b0);
+              tma_load_3d_pair(dst + A_BYTES / 2, &p.tm_x, full, ks * BK, r1, b1);
+            } else {
+              tma_load_3d(dst, &p.tm_x, full, ks * BK, r0, b0);
+              tma_load_3d(dst + A_BYTES / 2, &p.tm_x, full, ks * BK, r1, b1);
+            }
+          } else if (PAIR) {
+            tma_load_2d_pair(dst, &p.tm_x, full, ks * BK, tm * C::TM + (int)rank * BM);      // rows past M are zero-filled
           } else {
-            tma_load_2d(dst, &p.tm_x, &bars[FULL + ring.st], ks * BK, tm * BM);        // rows past M are zero-filled
+            tma_load_2d(dst, &p.tm_x, full, ks * BK, tm * BM);
           }
-          tma_load_2d(dst + A_BYTES, tw, &bars[FULL + ring.st], ks * BK, tn * BN);
+          if (PAIR) tma_load_2d_pair(dst + A_BYTES, tw, full, ks * BK, tn * BN + (int)rank * C::B_ROWS);
+          else tma_load_2d(dst + A_BYTES, tw, full, ks * BK, tn * BN);
           ring.next();
           ++issued;
         }
       }
-      if (*abort_flag)          // nothing may land in shared memory after the block has gone
+      if (*abort_flag && rank == 0)          // nothing may land in shared memory after the block (or its pair) has gone
         for (uint32_t back = 0; back < (uint32_t)STAGES && back < issued; ++back) {
           const uint32_t g = issued - 1 - back;
           for (int i = 0; i < (1 << 20); ++i)
@@ -139,13 +179,14 @@ kv_project_append_kernel(const __grid_constant__ ProjParams p) {
         }
     }
   } else if (warp == 1) {
-    // all lanes run the issuing code; elect.sync inside the wrappers picks the issuing lane
+    // all lanes run the issuing code; elect.sync inside the wrappers picks the issuing lane (of the pair's leader)
     Ring ring; ring.init(STAGES);
     bool ok = true;
     uint32_t tcount = 0;
-    for (int t = blockIdx.x; t < total && ok; t += gridDim.x, ++tcount) {
+    for (int t = first; t < total && ok && rank == 0; t += step, ++tcount) {
       const uint32_t ab = tcount & 1;
       ok = mbar_wait_warp(&bars[ACC_EMPTY + ab], ((tcount >> 1) & 1) ^ 1, abort_flag, lane);
+      if (ok) tc_fence_after();
       for (int ks = 0; ks < ksteps && ok; ++ks) {
         ok = mbar_wait_warp(&bars[FULL + ring.st], ring.ph, abort_flag, lane);
         if (!ok) break;
@@ -153,26 +194,40 @@ kv_project_append_kernel(const __grid_constant__ ProjParams p) {
         const uint64_t da = umma_desc_sw128(smem_u32(smem + ring.st * STAGE_BYTES));
         const uint64_t db = umma_desc_sw128(smem_u32(smem + ring.st * STAGE_BYTES + A_BYTES));
 #pragma unroll
-        for (int kk = 0; kk < BK / 16; ++kk)
-          umma_bf16_ss_elect(tmem_base + ab * BN, da + kk * 2, db + kk * 2, IDESC, (uint32_t)(ks > 0 || kk > 0));
-        umma_commit_elect(&bars[EMPTY + ring.st]);
+        for (int kk = 0; kk < BK / 16; ++kk) {
+          if (PAIR) umma_bf16_ss_pair_elect(tmem_base + ab * BN, da + kk * 2, db + kk * 2, C::IDESC, (uint32_t)(ks > 0 || kk > 0));
+          else umma_bf16_ss_elect(tmem_base + ab * BN, da + kk * 2, db + kk * 2, C::IDESC, (uint32_t)(ks > 0 || kk > 0));
+        }
+        if (PAIR) umma_commit_pair_elect(&bars[EMPTY + ring.st]);
+        else umma_commit_elect(&bars[EMPTY + ring.st]);
         ring.next();
       }
-      if (ok) umma_commit_elect(&bars[ACC_FULL + ab]);
+      if (ok) {
+        if (PAIR) umma_commit_pair_elect(&bars[ACC_FULL + ab]);
+        else umma_commit_elect(&bars[ACC_FULL + ab]);
+      }
     }
   } else {
     // epilogue: thread = accumulator lane = row of the tile
-    const int quad = warp & 3;                           // warps 2..5 -> TMEM lane quarters 2, 3, 0, 1
+    const int quad = warp & 3, half = (warp - 2) >> 2;   // warps 2..9: every TMEM lane quarter twice, one half of the columns each
     const int row_in_tile = quad * 32 + lane;
     const uint32_t tlane = tmem_base + ((uint32_t)(quad * 32) << 16);
+    auto release = [&](uint32_t ab) {                  // this warp has read its part of the accumulator
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        if (PAIR) mbar_arrive_leader(&bars[ACC_EMPTY + ab]);
+        else mbar_arrive(&bars[ACC_EMPTY + ab]);
+      }
+    };
     bool ok = true;
     uint32_t tcount = 0;
-    for (int t = blockIdx.x; t < total + p.lead_tiles && ok; t += gridDim.x, ++tcount) {
+    for (int t = first; t < total + p.lead_tiles && ok; t += step, ++tcount) {
       if (t >= total) {                                  // the lead rows of one batch, 256 columns: residual or zeros
         const int b = (t - total) / p.tiles_n, c0 = (t - total - b * p.tiles_n) * BN, vecs = min(BN, p.ncols - c0) / 8;
         __nv_bfloat16* dst = p.out + b * p.out_bs - p.lead_rows * p.out_stride + c0;
         const __nv_bfloat16* src = p.residual + b * p.res_bs - p.lead_rows * p.res_stride + c0;
-        for (int i = (warp - 2) * 32 + lane; i < p.lead_rows * vecs; i += 128) {
+        for (int i = ((warp - 2) + EPI_WARPS * (int)rank) * 32 + lane; i < p.lead_rows * vecs; i += (PAIR ? 2 : 1) * EPI_WARPS * 32) {
           const int r = i / vecs, v = i - r * vecs;
           *reinterpret_cast<uint4*>(dst + r * p.out_stride + v * 8) =
               p.residual ? *reinterpret_cast<const uint4*>(src + r * p.res_stride + v * 8) : make_uint4(0, 0, 0, 0);
@@ -182,12 +237,22 @@ kv_project_append_kernel(const __grid_constant__ ProjParams p) {
       int which, tm, tn;
       tile_of(p, t, which, tm, tn);
       const uint32_t ab = tcount & 1;
+      if (p.nmat == 2 && p.lmk && which == 0 && tn == 0 && half == 0 && (quad & 1)) {
+        // the landmark embedding of a chunk is its last row: copied by the warp that has that row
+        const long long last = (long long)tm * C::TM + (int)rank * BM + quad * 32 + 31;
+        if (last < p.M) {
+          const long long n = last / p.rows_per_seq, c = (last - n * p.rows_per_seq) / 64;
+          const int vecs = p.D / 8;
+          for (int v = lane; v < vecs; v += 32) p.lmk[n * p.lmk_bs + (p.pos + c) * vecs + v] = p.x_rows[last * vecs + v];
+        }
+      }
       ok = mbar_wait_bounded(&bars[ACC_FULL + ab], (tcount >> 1) & 1, abort_flag);
       if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
       tc_fence_after();
-      long long m = (long long)tm * BM + row_in_tile;
+      long long m = (long long)tm * C::TM + (int)rank * BM + row_in_tile;
       bool live = m < p.M;
       if (p.nmat == 1 && p.ce_part) {
+        if (half) { release(ab); continue; }             // a row's tile is reduced by one thread
         // cross-entropy mode: per row, the maximum and the sum of exponentials of this column
         // tile's logits (base 2, logits scaled by log2 e) and the target's logit if it lies here
         const float sc = ((live && p.row_scale) ? p.row_scale[m] : 1.0f) * GCA_LOG2E;
@@ -219,82 +284,74 @@ kv_project_append_kernel(const __grid_constant__ ProjParams p) {
           mx = nm;
         }
         if (live) p.ce_part[m * p.tiles_n + tn] = make_float2(mx, sum);
-        tc_fence_before();
-        mbar_arrive(&bars[ACC_EMPTY + ab]);
+        release(ab);
         continue;
       }
+      // a row of the output: linear mode out = scale * acc + residual, append mode a cache row (zeros for a landmark row)
+      __nv_bfloat16* dst;
+      const __nv_bfloat16* res = nullptr;
+      float sc = 1.0f;
+      bool zero = false;
+      int cols = BN;
       if (p.nmat == 1) {
-        // linear mode: out = row_scale * acc + residual, 16 columns per pass
-        const int block = 2 * tm + (row_in_tile >> 6), b = block / p.blocks_per_batch;
+        const int block = (C::TM / 64) * tm + 2 * (int)rank + (row_in_tile >> 6), b = block / p.blocks_per_batch;
         m = (block - b * p.blocks_per_batch) * 64 + (row_in_tile & 63);
         live = b < p.batches && m < p.M;
-        const float sc = (live && p.row_scale) ? p.row_scale[b * p.scale_bs + m] : 1.0f;
-        __nv_bfloat16* orow = p.out + b * p.out_bs + m * p.out_stride + tn * BN;
-        const __nv_bfloat16* rrow = p.residual ? p.residual + b * p.res_bs + m * p.res_stride + tn * BN : nullptr;
-        const int cols = min(BN, p.ncols - tn * BN);
-#pragma unroll 1
-        for (int c0 = 0; c0 < cols; c0 += 16) {
-          uint32_t v[16];
-          tmem_ld_32x32b_x16(tlane + ab * BN + c0, v);
-          // the residual's 32 bytes are requested before the accumulator read is waited for
-          uint4 r0 = make_uint4(0, 0, 0, 0), r1 = r0;
-          if (live && rrow) { r0 = *reinterpret_cast<const uint4*>(rrow + c0); r1 = *reinterpret_cast<const uint4*>(rrow + c0 + 8); }
-          tmem_ld_wait();
-          if (live) {
-            uint32_t w[8];
-            if (rrow) {
-              const uint32_t rr[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
-#pragma unroll
-              for (int i = 0; i < 8; ++i)
-                w[i] = pack_bf16x2(fmaf(__uint_as_float(v[2 * i]), sc, __uint_as_float(rr[i] << 16)),
-                                   fmaf(__uint_as_float(v[2 * i + 1]), sc, __uint_as_float(rr[i] & 0xffff0000u)));
-            } else {
-#pragma unroll
-              for (int i = 0; i < 8; ++i) w[i] = pack_bf16x2(__uint_as_float(v[2 * i]) * sc, __uint_as_float(v[2 * i + 1]) * sc);
-            }
-            reinterpret_cast<uint4*>(orow + c0)[0] = make_uint4(w[0], w[1], w[2], w[3]);
-            reinterpret_cast<uint4*>(orow + c0)[1] = make_uint4(w[4], w[5], w[6], w[7]);
-          }
-        }
-        tc_fence_before();
-        mbar_arrive(&bars[ACC_EMPTY + ab]);
-        continue;
+        if (live && p.row_scale) sc = p.row_scale[b * p.scale_bs + m];
+        dst = p.out + b * p.out_bs + m * p.out_stride + tn * BN;
+        if (live && p.residual) res = p.residual + b * p.res_bs + m * p.res_stride + tn * BN;
+        cols = min(BN, p.ncols - tn * BN);
+      } else {
+        const int n = live ? (int)(m / p.rows_per_seq) : 0;
+        const int r = live ? (int)(m - (long long)n * p.rows_per_seq) : 0;       // (chunk, row) inside the appended block
+        zero = p.zero_landmark && (r & 63) == 63;
+        dst = (which ? p.v_cache : p.k_cache) + n * p.cache_bs + ((long long)p.pos * 64 + r) * p.D + tn * BN;
       }
-      const int n = live ? (int)(m / p.rows_per_seq) : 0;
-      const int r = live ? (int)(m - (long long)n * p.rows_per_seq) : 0;       // (chunk, row) inside the appended block
-      const bool zero = p.zero_landmark && (r & 63) == 63;
-      __nv_bfloat16* dst = (which ? p.v_cache : p.k_cache) + n * p.cache_bs + ((long long)p.pos * 64 + r) * p.D + tn * BN;
-      // one small loop body (16 columns: TMEM -> bf16 -> one 32-byte store), 16 passes
+      // passes of 32 columns (or the last 16) of one small loop body; the residual is asked for before the accumulator
+      const int c_end = min(cols, (half + 1) * (BN / 2));
 #pragma unroll 1
-      for (int c0 = 0; c0 < BN; c0 += 16) {
-        uint32_t v[16];
-        tmem_ld_32x32b_x16(tlane + ab * BN + c0, v);
+      for (int c0 = half * (BN / 2); c0 < c_end; c0 += 32) {
+        uint32_t v[32];
+        uint4 rr[4];
+        const bool two = c0 + 16 < c_end;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) rr[i] = (res && (i < 2 || two)) ? *reinterpret_cast<const uint4*>(res + c0 + 8 * i) : make_uint4(0, 0, 0, 0);
+        tmem_ld_32x32b_x32(tlane + ab * BN + c0, v);
         tmem_ld_wait();
         if (zero) {
 #pragma unroll
-          for (int i = 0; i < 16; ++i) v[i] = 0u;
+          for (int i = 0; i < 32; ++i) v[i] = 0u;
         }
-        if (live) store16_bf16(reinterpret_cast<uint8_t*>(dst + c0), v, 1.0f, true);
+        if (!live) continue;
+        const uint32_t rw[16] = {rr[0].x, rr[0].y, rr[0].z, rr[0].w, rr[1].x, rr[1].y, rr[1].z, rr[1].w,
+                                 rr[2].x, rr[2].y, rr[2].z, rr[2].w, rr[3].x, rr[3].y, rr[3].z, rr[3].w};
+        uint32_t w[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          w[i] = pack_bf16x2(fmaf(__uint_as_float(v[2 * i]), sc, __uint_as_float(rw[i] << 16)),
+                             fmaf(__uint_as_float(v[2 * i + 1]), sc, __uint_as_float(rw[i] & 0xffff0000u)));
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          if (h && !two) break;
+          if (p.wide) st_global_256(dst + c0 + 16 * h, w[8 * h], w[8 * h + 1], w[8 * h + 2], w[8 * h + 3], w[8 * h + 4], w[8 * h + 5], w[8 * h + 6], w[8 * h + 7]);
+          else {
+            reinterpret_cast<uint4*>(dst + c0 + 16 * h)[0] = make_uint4(w[8 * h], w[8 * h + 1], w[8 * h + 2], w[8 * h + 3]);
+            reinterpret_cast<uint4*>(dst + c0 + 16 * h)[1] = make_uint4(w[8 * h + 4], w[8 * h + 5], w[8 * h + 6], w[8 * h + 7]);
+          }
+        }
       }
-      tc_fence_before();
-      mbar_arrive(&bars[ACC_EMPTY + ab]);
+      release(ab);
     }
   }
   tc_fence_before();
-  __syncthreads();
-  if (warp == 1) tmem_dealloc(tmem_base, 512);
+  __syncwarp();
+  if (PAIR) cluster_sync();                            // neither CTA leaves while the other's MMAs or arrivals may touch it
+  else __syncthreads();
+  if (warp == 1) {
+    if (PAIR) tmem_dealloc_pair(tmem_base, TMEM_COLS);
+    else tmem_dealloc(tmem_base, TMEM_COLS);
+  }
   if (threadIdx.x == 0 && *abort_flag && p.status) atomicOr(p.status, GCA_STATUS_TIMEOUT);
-}
-
-__global__ void lmk_rows_kernel(const uint4* __restrict__ x, uint4* __restrict__ lmk, long long lmk_bs, int pos, int count,
-                                int row_vecs, long long total) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= total) return;
-  const int v = (int)(i % row_vecs);
-  const long long cn = i / row_vecs;                      // n * count + c
-  const int c = (int)(cn % count);
-  const long long n = cn / count;
-  lmk[n * lmk_bs + (long long)(pos + c) * row_vecs + v] = x[(cn * 64 + 63) * row_vecs + v];
 }
 
 // row_scale[m] = rsqrt(mean(x[m, :]^2) + eps): one warp per row, 16-byte loads.
@@ -372,28 +429,71 @@ __global__ void ce_combine_kernel(const float2* __restrict__ part, const float* 
 
 }  // namespace
 
+int launch_skinny_linear(const LinearArgs& a, float rms_eps, cudaStream_t stream);
+
+namespace {
+
+// Which tile: wide pairs once every pair of SMs has one (they read the least shared memory and L2 per product, and power is what a
+// large product runs into), else the width whose waves cost least.  In units of column-steps of one CTA: a tile costs its
+// width plus ~64 for its prologue and epilogue tail.
+struct TileChoice { int bn; bool pair; };
+TileChoice choose_tile(long long rows64, int ncols, int nmat, int sms) {
+  auto ceil_div = [](long long a, long long b) { return (a + b - 1) / b; };
+  TileChoice best = {256, true};
+  long long best_cost = ceil_div(ceil_div(rows64, 4) * ceil_div(ncols, 256) * nmat, sms / 2) * (256 + 48);
+  for (int bn : {256, 128, 64}) {
+    const long long cost = ceil_div(ceil_div(rows64, 2) * ceil_div(ncols, bn) * nmat, sms) * (bn + 64);
+    if (cost < best_cost) { best_cost = cost; best = {bn, false}; }
+  }
+  return best;
+}
+
+template <int BN, bool PAIR>
+int launch_tiles(const ProjParams& p, int sms, cudaStream_t stream) {
+  using C = Cfg<BN, PAIR>;
+  GCA_CUDA_CHECK(cudaFuncSetAttribute(kv_project_append_kernel<BN, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
+  const long long tiles = (long long)p.tiles_m * p.tiles_n * p.nmat + p.lead_tiles;
+  if (PAIR) {
+    const unsigned pairs = (unsigned)(tiles < sms / 2 ? tiles : sms / 2);
+    return (int)launch_dependent_pairs(kv_project_append_kernel<BN, PAIR>, dim3(2 * pairs), dim3(NTHREADS), C::SMEM_BYTES, stream, p);
+  }
+  return (int)launch_dependent(kv_project_append_kernel<BN, PAIR>, dim3((unsigned)(tiles < sms ? tiles : sms)), dim3(NTHREADS), C::SMEM_BYTES, stream, p);
+}
+
+// rows64: 64-row blocks of x (of all batches).  Fills in the tile counts; the weight maps are made here because their box is the tile's.
+int launch_product(ProjParams& p, const void* wk, const void* wv, long long w_stride, long long rows64, TileChoice tile, int sms, cudaStream_t stream) {
+  const int tm = tile.pair ? 4 : 2, box = tile.pair ? tile.bn / 2 : tile.bn;
+  int rc;
+  if ((rc = make_matrix_map(&p.tm_wk, wk, p.ncols, p.D, w_stride, box)) || (rc = make_matrix_map(&p.tm_wv, wv, p.ncols, p.D, w_stride, box))) return rc;
+  p.tiles_m = (int)((rows64 + tm - 1) / tm);
+  p.tiles_n = (p.ncols + tile.bn - 1) / tile.bn;
+  p.lead_tiles = p.lead_rows > 0 ? p.batches * p.tiles_n : 0;
+  if ((long long)p.tiles_m * p.tiles_n * p.nmat + p.lead_tiles >= (1ll << 30)) return GCA_ERR_TOO_LARGE;
+  if (tile.pair) return launch_tiles<256, true>(p, sms, stream);
+  if (tile.bn == 256) return launch_tiles<256, false>(p, sms, stream);
+  if (tile.bn == 128) return launch_tiles<128, false>(p, sms, stream);
+  return launch_tiles<64, false>(p, sms, stream);
+}
+
+}  // namespace
+
 int launch_linear_ce(const LinearCeArgs& a, int sms, cudaStream_t stream) {
   ProjParams p;
+  if (a.M >= (1ll << 31)) return GCA_ERR_TOO_LARGE;
   int rc;
-  if ((rc = make_matrix_map(&p.tm_x, a.x, a.M, a.K, a.x_stride, BM)) || (rc = make_matrix_map(&p.tm_wk, a.w, a.N, a.K, a.w_stride, BN)))
-    return rc;
-  p.tm_wv = p.tm_wk;
+  if ((rc = make_matrix_map(&p.tm_x, a.x, a.M, a.K, a.x_stride, BM))) return rc;
   p.k_cache = p.v_cache = nullptr; p.status = a.status; p.cache_bs = 0;
-  p.M = (int)a.M; p.D = a.K; p.rows_per_seq = 1; p.pos = 0; p.zero_landmark = 0;
-  p.tiles_m = (int)((a.M + BM - 1) / BM); p.tiles_n = (a.N + BN - 1) / BN; p.nmat = 1;
+  p.M = (int)a.M; p.D = a.K; p.rows_per_seq = 1; p.pos = 0; p.zero_landmark = 0; p.nmat = 1;
   p.out = nullptr; p.residual = nullptr; p.row_scale = a.row_scale; p.out_stride = p.res_stride = 0; p.ncols = a.N;
-  // workspace: partials (M, tiles_n) float2, then the target logits (M) float
-  p.batches = 1; p.blocks_per_batch = 0; p.lead_rows = p.lead_tiles = 0; p.out_bs = p.res_bs = p.scale_bs = 0;
+  p.batches = 1; p.blocks_per_batch = 0; p.lead_rows = 0; p.out_bs = p.res_bs = p.scale_bs = 0;
+  // workspace: partials (M, 256-column tiles) float2, then the target logits (M) float
+  const long long tiles = (a.N + 255) / 256;
   p.ce_part = reinterpret_cast<float2*>(a.workspace);
-  p.ce_target = reinterpret_cast<float*>(p.ce_part + a.M * p.tiles_n);
+  p.ce_target = reinterpret_cast<float*>(p.ce_part + a.M * tiles);
   p.targets = reinterpret_cast<const long long*>(a.targets);
-  const long long total = (long long)p.tiles_m * p.tiles_n;
-  if (total >= (1ll << 31) || a.M >= (1ll << 31)) return GCA_ERR_TOO_LARGE;
-  if (total == 0) return 0;
-  GCA_CUDA_CHECK(cudaFuncSetAttribute(kv_project_append_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-  const unsigned grid = (unsigned)(total < sms ? total : sms);
-  kv_project_append_kernel<<<grid, NTHREADS, SMEM_BYTES, stream>>>(p);
-  GCA_CUDA_CHECK(cudaGetLastError());
+  TileChoice tile = choose_tile((a.M + 63) / 64, a.N, 1, sms);
+  tile.bn = 256;                                       // the workspace counts 256-column tiles
+  if ((rc = launch_product(p, a.w, a.w, a.w_stride, (a.M + 63) / 64, tile, sms, stream))) return rc;
   const int warps = 8;
   ce_combine_kernel<<<(unsigned)((a.M + warps - 1) / warps), warps * 32, 0, stream>>>(p.ce_part, p.ce_target, p.targets, a.loss, a.lse, a.M,
                                                                                     p.tiles_n);
@@ -425,60 +525,40 @@ int launch_linear(const LinearBatchedArgs& ba, int sms, cudaStream_t stream) {
     a.M *= args.batches;
     args.batches = 1;
   }
+  if (args.batches == 1 && args.lead_rows == 0 && a.M <= GCA_SKINNY_ROWS) return launch_skinny_linear(a, args.rms_eps, stream);
+  if (args.rms_eps > 0.f) return GCA_ERR_SHAPE;
   ProjParams p;
+  if (a.M >= (1ll << 31)) return GCA_ERR_TOO_LARGE;
   int rc;
-  if ((rc = make_rows_map(&p.tm_x, a.x, args.batches, a.M, a.K, a.x_stride, args.x_batch_stride, 64)) ||
-      (rc = make_matrix_map(&p.tm_wk, a.w, a.N, a.K, a.w_stride, BN)))
-    return rc;
-  p.tm_wv = p.tm_wk;
+  if ((rc = make_rows_map(&p.tm_x, a.x, args.batches, a.M, a.K, a.x_stride, args.x_batch_stride, 64))) return rc;
   p.k_cache = p.v_cache = nullptr; p.status = a.status; p.cache_bs = 0;
-  const long long per_batch = (a.M + 63) / 64, blocks = per_batch * args.batches, lead = args.lead_rows > 0 ? args.batches : 0;
-  p.tiles_n = (a.N + BN - 1) / BN;
-  const long long total = (blocks + 1) / 2 * p.tiles_n;
-  if (total + lead * p.tiles_n >= (1ll << 30) || a.M >= (1ll << 31)) return GCA_ERR_TOO_LARGE;
-  p.M = (int)a.M; p.D = a.K; p.rows_per_seq = 1; p.pos = 0; p.zero_landmark = 0;
-  p.tiles_m = (int)((blocks + 1) / 2); p.nmat = 1;
-  p.batches = args.batches; p.blocks_per_batch = (int)per_batch;
-  p.lead_rows = args.lead_rows; p.lead_tiles = (int)(lead * p.tiles_n);
+  const long long per_batch = (a.M + 63) / 64;
+  p.M = (int)a.M; p.D = a.K; p.rows_per_seq = 1; p.pos = 0; p.zero_landmark = 0; p.nmat = 1;
+  p.batches = args.batches; p.blocks_per_batch = (int)per_batch; p.lead_rows = args.lead_rows;
   p.out_bs = args.out_batch_stride; p.res_bs = args.residual_batch_stride; p.scale_bs = args.scale_batch_stride;
   p.out = (__nv_bfloat16*)a.out; p.residual = (const __nv_bfloat16*)a.residual; p.row_scale = a.row_scale;
   p.out_stride = a.out_stride; p.res_stride = a.residual_stride; p.ncols = a.N;
+  p.wide = (reinterpret_cast<uintptr_t>(a.out) & 31u) == 0 && a.out_stride % 16 == 0 && args.out_batch_stride % 16 == 0;
   p.ce_part = nullptr; p.ce_target = nullptr; p.targets = nullptr;
-  GCA_CUDA_CHECK(cudaFuncSetAttribute(kv_project_append_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-  const long long tiles = total + p.lead_tiles;
-  kv_project_append_kernel<<<(unsigned)(tiles < sms ? tiles : sms), NTHREADS, SMEM_BYTES, stream>>>(p);
-  GCA_CUDA_CHECK(cudaGetLastError());
-  return 0;
+  const long long blocks = per_batch * args.batches;
+  if (blocks >= (1ll << 30)) return GCA_ERR_TOO_LARGE;
+  return launch_product(p, a.w, a.w, a.w_stride, blocks, choose_tile(blocks, a.N, 1, sms), sms, stream);
 }
 
 int launch_kv_project_append(const KvProjectArgs& a, int sms, cudaStream_t stream) {
   ProjParams p;
   const long long M = (long long)a.N * a.count * 64;
   int rc;
-  if ((rc = make_matrix_map(&p.tm_x, a.x, M, a.D, a.D, BM)) || (rc = make_matrix_map(&p.tm_wk, a.wk, a.D, a.D, a.D, BN)) ||
-      (rc = make_matrix_map(&p.tm_wv, a.wv, a.D, a.D, a.D, BN)))
-    return rc;
+  if ((rc = make_matrix_map(&p.tm_x, a.x, M, a.D, a.D, BM))) return rc;
   p.k_cache = (__nv_bfloat16*)a.k_cache; p.v_cache = (__nv_bfloat16*)a.v_cache; p.status = a.status;
   p.cache_bs = a.cache_batch_stride; p.M = (int)M; p.D = a.D; p.rows_per_seq = a.count * 64; p.pos = a.pos;
-  p.zero_landmark = a.zero_landmark;
-  p.tiles_m = (int)((M + BM - 1) / BM); p.tiles_n = a.D / BN; p.nmat = 2;
+  p.zero_landmark = a.zero_landmark; p.nmat = 2;
   p.out = nullptr; p.residual = nullptr; p.row_scale = nullptr; p.out_stride = p.res_stride = 0; p.ncols = a.D;
-  p.batches = 1; p.blocks_per_batch = 0; p.lead_rows = p.lead_tiles = 0; p.out_bs = p.res_bs = p.scale_bs = 0;
   p.ce_part = nullptr; p.ce_target = nullptr; p.targets = nullptr;
-  const long long total = (long long)p.tiles_m * p.tiles_n * 2;
-  if (total >= (1ll << 31)) return GCA_ERR_TOO_LARGE;
-  GCA_CUDA_CHECK(cudaFuncSetAttribute(kv_project_append_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-  const unsigned grid = (unsigned)(total < sms ? total : sms);
-  kv_project_append_kernel<<<grid, NTHREADS, SMEM_BYTES, stream>>>(p);
-  GCA_CUDA_CHECK(cudaGetLastError());
-  if (a.lmk_cache) {
-    const int row_vecs = a.D / 8;
-    const long long tot = (long long)a.N * a.count * row_vecs;
-    lmk_rows_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, stream>>>((const uint4*)a.x, (uint4*)a.lmk_cache,
-                                                                      a.lmk_cache_batch_stride / 8, a.pos, a.count, row_vecs, tot);
-    GCA_CUDA_CHECK(cudaGetLastError());
-  }
-  return 0;
+  p.batches = 1; p.blocks_per_batch = 0; p.lead_rows = 0; p.out_bs = p.res_bs = p.scale_bs = 0;
+  p.wide = 1;                                          // the entry point asks for 32-byte aligned caches
+  p.x_rows = (const uint4*)a.x; p.lmk = (uint4*)a.lmk_cache; p.lmk_bs = a.lmk_cache_batch_stride / 8;
+  return launch_product(p, a.wk, a.wv, a.D, M / 64, choose_tile(M / 64, a.D, 2, sms), sms, stream);
 }
 
 }  // namespace gca

@@ -76,6 +76,8 @@ win_decode_kernel(const WinParams p) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = lane >> 3, sub = lane & 7;
   const int n = blockIdx.x / p.Hkv, hk = blockIdx.x - n * p.Hkv;
   const int rows = p.G * p.Sq;                       // <= R
+  pdl_trigger();
+  pdl_wait();
   // this lane's 8 query values of every row, pre-scaled; the row's ALiBi slope (in log2 units) and position
   float qv[R][8], slope[R];
   int pos[R];
@@ -277,16 +279,11 @@ static int launch_window(const WindowDecodeArgs& a, const WindowRingDecodeArgs* 
   const int rows = p.G * a.Sq;
   const unsigned grid = (unsigned)(a.N * a.Hkv);
   if (grid == 0) return 0;
-  if (ring) {                                      // one new position: G rows per kv head
-    if (rows <= 1) win_decode_kernel<1, true><<<grid, NWARPS * 32, 0, stream>>>(p);
-    else if (rows <= 2) win_decode_kernel<2, true><<<grid, NWARPS * 32, 0, stream>>>(p);
-    else if (rows <= 4) win_decode_kernel<4, true><<<grid, NWARPS * 32, 0, stream>>>(p);
-    else return GCA_ERR_SHAPE;
-  } else if (rows <= 1) win_decode_kernel<1, false><<<grid, NWARPS * 32, 0, stream>>>(p);
-  else if (rows <= 2) win_decode_kernel<2, false><<<grid, NWARPS * 32, 0, stream>>>(p);
-  else if (rows <= 4) win_decode_kernel<4, false><<<grid, NWARPS * 32, 0, stream>>>(p);
-  else return GCA_ERR_SHAPE;
-  return (int)cudaGetLastError();
+  auto run = [&](auto kernel) { return (int)launch_dependent(kernel, dim3(grid), dim3(NWARPS * 32), 0, stream, p); };
+  if (rows > 4) return GCA_ERR_SHAPE;
+  if (ring)                                        // one new position: G rows per kv head
+    return rows <= 1 ? run(win_decode_kernel<1, true>) : rows <= 2 ? run(win_decode_kernel<2, true>) : run(win_decode_kernel<4, true>);
+  return rows <= 1 ? run(win_decode_kernel<1, false>) : rows <= 2 ? run(win_decode_kernel<2, false>) : run(win_decode_kernel<4, false>);
 }
 
 int launch_window_decode(const WindowDecodeArgs& a, cudaStream_t stream) { return launch_window(a, nullptr, stream); }

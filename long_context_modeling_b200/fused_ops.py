@@ -53,8 +53,8 @@ def fold_gain(weight: torch.Tensor, gain: torch.Tensor) -> torch.Tensor:
 
 def rmsnorm_linear(x: torch.Tensor, folded_weight: torch.Tensor, eps: float) -> torch.Tensor:
     """RMSNorm(x) @ W.T with ``folded_weight = fold_gain(W, norm.weight)``: one row reduction over x
-    and one GEMM over the raw x whose epilogue applies 1 / rms."""
-    return linear(x, folded_weight, row_scale=row_rms(x, eps))
+    and one GEMM over the raw x whose epilogue applies 1 / rms (one launch for a handful of rows)."""
+    return _lib.host().rmsnorm_linear(x, folded_weight, eps)
 
 
 def silu_mul(gate_up: torch.Tensor) -> torch.Tensor:

@@ -314,3 +314,57 @@ def test_silu_mul_against_float32(m, inter):
     assert torch.equal(F.silu_mul(gu.view(1, m, 2 * inter).contiguous()).view(m, inter), got)
     with pytest.raises(ValueError):
         F.silu_mul(gu[:, :2 * inter - 8].contiguous()[:, :2 * inter - 12])   # halves not a multiple of 8 wide
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 16, 64), (16, 768, 768), (17, 48, 2080), (33, 512, 96 * 2), (65, 768, 768), (128, 1024, 1024)])
+@pytest.mark.parametrize("with_res", [False, True])
+def test_few_row_linear_and_fused_norm_against_float32(m, n, k, with_res):
+    """The latency-bound form (up to 128 rows): every number of 16-row tiles, contractions that do not split evenly over the
+    warps, and RMSNorm fused into the projection."""
+    need_gpu()
+    from long_context_modeling_b200 import fused_ops as F
+    k = k // 64 * 64
+    g = torch.Generator().manual_seed(m + n)
+    x, w, r = ((torch.randn(*s, generator=g) * c).bfloat16().cuda() for s, c in (((m, k), 1.0), ((n, k), k ** -0.5), ((m, n), 1.0)))
+    y = F.linear(x, w, residual=r if with_res else None)
+    ref = x.float() @ w.float().t() + (r.float() if with_res else 0)
+    assert (y.float() - ref).abs().max() <= 2e-2 * ref.abs().max()
+    z = F.rmsnorm_linear(x * 3, w, 1e-5)
+    xf = (x * 3).float()
+    ref = (xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + 1e-5)) @ w.float().t()
+    assert (z.float() - ref).abs().max() <= 2e-2 * ref.abs().max()
+
+
+@pytest.mark.parametrize("m,n,k", [(200, 768, 768), (3000, 272, 128), (6912, 768, 768), (20011, 784, 192), (40000, 768, 768)])
+def test_linear_tile_widths_against_float32(m, n, k):
+    """Every tile the GEMM chooses from (64 to 256 columns, pairs of CTAs on 256 x 256), ragged in rows and columns, with the
+    row scale and the residual."""
+    need_gpu()
+    from long_context_modeling_b200 import fused_ops as F
+    g = torch.Generator(device="cuda").manual_seed(m)
+    x, w, r = ((torch.randn(*s, generator=g, device="cuda") * c).bfloat16() for s, c in (((m, k), 1.0), ((n, k), k ** -0.5), ((m, n), 1.0)))
+    sc = torch.rand(m, generator=g, device="cuda") + 0.5
+    y = F.linear(x, w, row_scale=sc, residual=r)
+    ref = (x.float() @ w.float().t()) * sc[:, None] + r.float()
+    assert (y.float() - ref).abs().max() <= 2e-2 * ref.abs().max()
+    assert torch.equal(y, F.linear(x, w, row_scale=sc, residual=r))
+
+
+@pytest.mark.parametrize("n,c,dim", [(1, 1, 256), (3, 5, 512), (5, 61, 768), (2, 300, 1024)])
+def test_projection_append_tile_widths(n, c, dim):
+    """K, V and landmark rows of an append at a position behind earlier chunks, against float32, small and large products."""
+    need_gpu()
+    import long_context_modeling_b200 as lcm
+    g = torch.Generator(device="cuda").manual_seed(c)
+    x = torch.randn(n, c, 64, dim, generator=g, device="cuda").bfloat16()
+    wk, wv = ((torch.randn(dim, dim, generator=g, device="cuda") * dim ** -0.5).bfloat16() for _ in range(2))
+    cache = lcm.ChunkKVManager(zero_landmark=True, capacity=c + 3)
+    with torch.no_grad():
+        cache.append_projected(x[:, :1], wk, wv)
+        cache.append_projected(x, wk, wv)
+    for got, w in ((cache.chunk_k, wk), (cache.chunk_v, wv)):
+        ref = x.float() @ w.float().t()
+        ref[:, :, -1] = 0
+        ref = torch.cat([ref[:, :1], ref], 1)
+        assert (got.float() - ref).abs().max() <= 2e-2 * ref.abs().max()
+    assert torch.equal(cache.past_lmk_embeds, torch.cat([x[:, :1, -1], x[:, :, -1]], 1))

@@ -417,3 +417,21 @@ def test_full_size_config_properties(lcm):
         used[b, idx[b][idx[b] >= 0]] = True
     assert kg.grad.view(n, c, -1)[~used.to(dev)].abs().max().item() == 0
     assert lcm.read_status() == 0
+
+
+@pytest.mark.parametrize("n,hq,hkv,sq,k,obo", [(1, 12, 12, 1, 8, False), (2, 6, 6, 2, 13, True), (20, 12, 12, 1, 5, False), (14, 12, 6, 1, 32, True),
+                                               (30, 12, 12, 1, 8, False), (26, 12, 12, 2, 3, True)])
+def test_decode_warps_per_slot(lcm, n, hq, hkv, sq, k, obo):
+    """One to four warps per retrieved slot, chosen by how many (sequence, kv head) items there are: padding slots, one that
+    lies outside the cache, the extra softmax logit, more slots than warps."""
+    g = torch.Generator().manual_seed(n)
+    c = 40
+    kc, vc = (torch.randn(n, c, 64, hkv * 64, generator=g).bfloat16() for _ in range(2))
+    q = torch.randn(n, 1, hq, sq, 64, generator=g).bfloat16()
+    idx = torch.stack([torch.randperm(c, generator=g)[:k] for _ in range(n)]).view(n, 1, k)
+    if k > 3:
+        idx[:, :, 2] = -1
+    w = torch.softmax(torch.randn(n, 1, k, generator=g), -1)
+    ref = G.gca_indexed(q.float(), kc.float(), vc.float(), idx, torch.where(idx < 0, torch.zeros_like(w), w), 0.125, off_by_one=1.0 if obo else 0.0)
+    got = lcm.gca_indexed_nograd(q.cuda(), kc.cuda(), vc.cuda(), idx.cuda(), w.cuda(), 0.125, softmax_off_by_one=obo).float().cpu()
+    assert (got - ref).abs().max() <= 1e-2 * ref.abs().max()
