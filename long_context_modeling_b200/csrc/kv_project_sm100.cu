@@ -10,8 +10,8 @@
 //   Wk, Wv (D x D) bf16 in nn.Linear layout (out, in) = K-major B operand
 //   K_cache[n, pos + c, s, :] = X[(n, c, s), :] Wk^T   (zeros for s = 63 when zero_landmark)
 //
-// tcgen05 GEMM, one CTA per SM, persistent over (row tile, column tile, K|V): warp 0 issues the TMA copies of a ring of
-// 64-deep stages, warp 1 the MMAs into one of two accumulators in tensor memory, eight epilogue warps (two per lane quarter,
+// tcgen05 GEMM, one CTA per SM, persistent over (row tile, column tile, K|V): two warps issue the TMA copies of a ring of
+// 64-deep stages (rows of x, rows of the weights), warp 1 the MMAs into one of two accumulators in tensor memory, eight epilogue warps (two per lane quarter,
 // half of the columns each) turn a finished accumulator into bf16 rows of the cache while the next tile is being multiplied;
 // the warp that has a chunk's last row also copies it to the landmark cache.  Every wait is bounded
 // (GCA_STATUS_TIMEOUT on expiry).
@@ -45,7 +45,7 @@ namespace {
 using namespace sm100;
 
 constexpr int BM = 128, BK = 64;                      // rows of a CTA's accumulator, K step
-constexpr int EPI_WARPS = 8, NTHREADS = (2 + EPI_WARPS) * 32;
+constexpr int EPI_WARPS = 8, W_WARP = 2 + EPI_WARPS, NTHREADS = (3 + EPI_WARPS) * 32;
 
 // BN: columns of a tile.  PAIR: two CTAs share a tile of 256 rows (cta_group::2), each loading half of the weight rows.
 template <int BN, bool PAIR>
@@ -57,6 +57,7 @@ struct Cfg {
   static constexpr int FULL = 0, EMPTY = FULL + STAGES, ACC_FULL = EMPTY + STAGES, ACC_EMPTY = ACC_FULL + 2, NUM_BARS = ACC_EMPTY + 2;
   static constexpr uint32_t IDESC = umma_idesc_bf16(PAIR ? 2 * BM : BM, BN, 0, 0);
   static constexpr int TM = PAIR ? 2 * BM : BM;        // rows of a tile
+  static constexpr int ACC_COLS = BN > 128 ? 256 : BN;  // tensor-memory columns of an accumulator
   static_assert(NUM_BARS * 8 + 8 <= 256, "barriers fit their space");
 };
 
@@ -104,19 +105,19 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 kv_project_append_kernel(const __grid_constant__ ProjParams p) {
   using C = Cfg<BN, PAIR>;
   constexpr int STAGES = C::STAGES, STAGE_BYTES = C::STAGE_BYTES, A_BYTES = C::A_BYTES, OFF_BAR = C::OFF_BAR, NUM_BARS = C::NUM_BARS;
-  constexpr int FULL = C::FULL, EMPTY = C::EMPTY, ACC_FULL = C::ACC_FULL, ACC_EMPTY = C::ACC_EMPTY, TMEM_COLS = 2 * BN;
+  constexpr int FULL = C::FULL, EMPTY = C::EMPTY, ACC_FULL = C::ACC_FULL, ACC_EMPTY = C::ACC_EMPTY, ACC_COLS = C::ACC_COLS, TMEM_COLS = 2 * ACC_COLS;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + NUM_BARS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + NUM_BARS + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int total = p.tiles_m * p.tiles_n * p.nmat;
   const int ksteps = p.D / BK;
   const uint32_t rank = PAIR ? cluster_rank() : 0u;
   const int first = PAIR ? blockIdx.x / 2 : blockIdx.x, step = PAIR ? gridDim.x / 2 : gridDim.x;
   if (threadIdx.x == 0) {
-    for (int i = 0; i < STAGES; ++i) { mbar_init(&bars[FULL + i], 1); mbar_init(&bars[EMPTY + i], 1); }
+    for (int i = 0; i < STAGES; ++i) { mbar_init(&bars[FULL + i], 2); mbar_init(&bars[EMPTY + i], 1); }
     for (int i = 0; i < 2; ++i) { mbar_init(&bars[ACC_FULL + i], 1); mbar_init(&bars[ACC_EMPTY + i], (PAIR ? 2 : 1) * EPI_WARPS); }
     *abort_flag = 0;
     fence_barrier_init();
@@ -135,49 +136,50 @@ kv_project_append_kernel(const __grid_constant__ ProjParams p) {
   pdl_trigger();
   pdl_wait();
 
-  if (warp == 0) {
-    if (lane == 0) {
-      Ring ring; ring.init(STAGES);
-      uint32_t issued = 0;
-      bool ok = true;
-      for (int t = first; t < total && ok; t += step) {
-        int which, tm, tn;
-        tile_of(p, t, which, tm, tn);
-        const CUtensorMap* tw = which ? &p.tm_wv : &p.tm_wk;
-        for (int ks = 0; ks < ksteps; ++ks) {
-          ok = mbar_wait_bounded(&bars[EMPTY + ring.st], ring.ph ^ 1, abort_flag);
-          if (!ok) break;
-          uint8_t* dst = smem + ring.st * STAGE_BYTES;
-          uint64_t* full = &bars[FULL + ring.st];
-          if (rank == 0) mbar_arrive_expect_tx(full, (PAIR ? 2 : 1) * STAGE_BYTES);
-          if (p.blocks_per_batch) {                            // linear mode: two 64-row blocks (rows past the end are zero-filled)
-            const int blk = (C::TM / 64) * tm + 2 * (int)rank, b0 = blk / p.blocks_per_batch, b1 = (blk + 1) / p.blocks_per_batch;
-            const int r0 = (blk - b0 * p.blocks_per_batch) * 64, r1 = (blk + 1 - b1 * p.blocks_per_batch) * 64;
-            if (PAIR) {
-              tma_load_3d_pair(dst, &p.tm_x, full, ks * BK, r0, b0);
-              tma_load_3d_pair(dst + A_BYTES / 2, &p.tm_x, full, ks * BK, r1, b1);
-            } else {
-              tma_load_3d(dst, &p.tm_x, full, ks * BK, r0, b0);
-              tma_load_3d(dst + A_BYTES / 2, &p.tm_x, full, ks * BK, r1, b1);
-            }
-          } else if (PAIR) {
-            tma_load_2d_pair(dst, &p.tm_x, full, ks * BK, tm * C::TM + (int)rank * BM);      // rows past M are zero-filled
-          } else {
-            tma_load_2d(dst, &p.tm_x, full, ks * BK, tm * BM);
-          }
-          if (PAIR) tma_load_2d_pair(dst + A_BYTES, tw, full, ks * BK, tn * BN + (int)rank * C::B_ROWS);
-          else tma_load_2d(dst + A_BYTES, tw, full, ks * BK, tn * BN);
-          ring.next();
-          ++issued;
-        }
+  if (warp == 0 || warp == W_WARP) {
+    // two producers: the rows of x and the rows of the weights, each with its own arrival on FULL (the leader's, for a pair)
+    Ring ring; ring.init(STAGES);
+    uint32_t issued = 0;
+    bool ok = true;
+    for (int t = first; t < total && ok; t += step) {
+      int which, tm, tn;
+      tile_of(p, t, which, tm, tn);
+      const CUtensorMap* tw = which ? &p.tm_wv : &p.tm_wk;
+      // the CTA's 128 rows in one box, or (several batches) as two 64-row blocks; rows past the end are zero-filled
+      int b0 = 0, b1 = 0, r0 = tm * C::TM + (int)rank * BM, r1 = 0;
+      const bool blocks = p.batches > 1;
+      if (blocks) {
+        const int blk = (C::TM / 64) * tm + 2 * (int)rank;
+        b0 = blk / p.blocks_per_batch; b1 = (blk + 1) / p.blocks_per_batch;
+        r0 = (blk - b0 * p.blocks_per_batch) * 64; r1 = (blk + 1 - b1 * p.blocks_per_batch) * 64;
       }
-      if (*abort_flag && rank == 0)          // nothing may land in shared memory after the block (or its pair) has gone
-        for (uint32_t back = 0; back < (uint32_t)STAGES && back < issued; ++back) {
-          const uint32_t g = issued - 1 - back;
-          for (int i = 0; i < (1 << 20); ++i)
-            if (mbar_try_wait(&bars[FULL + g % STAGES], (g / STAGES) & 1)) break;
+      for (int ks = 0; ks < ksteps; ++ks) {
+        ok = mbar_wait_warp(&bars[EMPTY + ring.st], ring.ph ^ 1, abort_flag, lane);
+        if (!ok) break;
+        uint8_t* dst = smem + ring.st * STAGE_BYTES;
+        uint64_t* full = &bars[FULL + ring.st];
+        if (warp == 0) {
+          if (rank == 0) mbar_expect_tx_elect(full, (PAIR ? 2 : 1) * A_BYTES);
+          if (blocks) {
+            tma_load_3d_elect<PAIR>(dst, &p.tm_x, full, ks * BK, r0, b0);
+            tma_load_3d_elect<PAIR>(dst + A_BYTES / 2, &p.tm_x, full, ks * BK, r1, b1);
+          } else {
+            tma_load_2d_elect<PAIR>(dst, &p.tm_x, full, ks * BK, r0);
+          }
+        } else {
+          if (rank == 0) mbar_expect_tx_elect(full, (PAIR ? 2 : 1) * (STAGE_BYTES - A_BYTES));
+          tma_load_2d_elect<PAIR>(dst + A_BYTES, tw, full, ks * BK, tn * BN + (int)rank * C::B_ROWS);
         }
+        ring.next();
+        ++issued;
+      }
     }
+    if (*abort_flag && rank == 0)          // nothing may land in shared memory after the block (or its pair) has gone
+      for (uint32_t back = 0; back < (uint32_t)STAGES && back < issued; ++back) {
+        const uint32_t g = issued - 1 - back;
+        for (int i = 0; i < (1 << 20); ++i)
+          if (mbar_try_wait(&bars[FULL + g % STAGES], (g / STAGES) & 1)) break;
+      }
   } else if (warp == 1) {
     // all lanes run the issuing code; elect.sync inside the wrappers picks the issuing lane (of the pair's leader)
     Ring ring; ring.init(STAGES);
@@ -195,8 +197,8 @@ kv_project_append_kernel(const __grid_constant__ ProjParams p) {
         const uint64_t db = umma_desc_sw128(smem_u32(smem + ring.st * STAGE_BYTES + A_BYTES));
 #pragma unroll
         for (int kk = 0; kk < BK / 16; ++kk) {
-          if (PAIR) umma_bf16_ss_pair_elect(tmem_base + ab * BN, da + kk * 2, db + kk * 2, C::IDESC, (uint32_t)(ks > 0 || kk > 0));
-          else umma_bf16_ss_elect(tmem_base + ab * BN, da + kk * 2, db + kk * 2, C::IDESC, (uint32_t)(ks > 0 || kk > 0));
+          if (PAIR) umma_bf16_ss_pair_elect(tmem_base + ab * ACC_COLS, da + kk * 2, db + kk * 2, C::IDESC, (uint32_t)(ks > 0 || kk > 0));
+          else umma_bf16_ss_elect(tmem_base + ab * ACC_COLS, da + kk * 2, db + kk * 2, C::IDESC, (uint32_t)(ks > 0 || kk > 0));
         }
         if (PAIR) umma_commit_pair_elect(&bars[EMPTY + ring.st]);
         else umma_commit_elect(&bars[EMPTY + ring.st]);
@@ -262,7 +264,7 @@ kv_project_append_kernel(const __grid_constant__ ProjParams p) {
 #pragma unroll 1
         for (int c0 = 0; c0 < cols; c0 += 16) {
           uint32_t v[16];
-          tmem_ld_32x32b_x16(tlane + ab * BN + c0, v);
+          tmem_ld_32x32b_x16(tlane + ab * ACC_COLS + c0, v);
           tmem_ld_wait();
           float x[16];
           float pm = -INFINITY;
@@ -316,7 +318,7 @@ kv_project_append_kernel(const __grid_constant__ ProjParams p) {
         const bool two = c0 + 16 < c_end;
 #pragma unroll
         for (int i = 0; i < 4; ++i) rr[i] = (res && (i < 2 || two)) ? *reinterpret_cast<const uint4*>(res + c0 + 8 * i) : make_uint4(0, 0, 0, 0);
-        tmem_ld_32x32b_x32(tlane + ab * BN + c0, v);
+        tmem_ld_32x32b_x32(tlane + ab * ACC_COLS + c0, v);
         tmem_ld_wait();
         if (zero) {
 #pragma unroll
@@ -441,7 +443,7 @@ TileChoice choose_tile(long long rows64, int ncols, int nmat, int sms) {
   auto ceil_div = [](long long a, long long b) { return (a + b - 1) / b; };
   TileChoice best = {256, true};
   long long best_cost = ceil_div(ceil_div(rows64, 4) * ceil_div(ncols, 256) * nmat, sms / 2) * (256 + 48);
-  for (int bn : {256, 128, 64}) {
+  for (int bn : {256, 192, 128, 64}) {
     const long long cost = ceil_div(ceil_div(rows64, 2) * ceil_div(ncols, bn) * nmat, sms) * (bn + 64);
     if (cost < best_cost) { best_cost = cost; best = {bn, false}; }
   }
@@ -471,6 +473,7 @@ int launch_product(ProjParams& p, const void* wk, const void* wv, long long w_st
   if ((long long)p.tiles_m * p.tiles_n * p.nmat + p.lead_tiles >= (1ll << 30)) return GCA_ERR_TOO_LARGE;
   if (tile.pair) return launch_tiles<256, true>(p, sms, stream);
   if (tile.bn == 256) return launch_tiles<256, false>(p, sms, stream);
+  if (tile.bn == 192) return launch_tiles<192, false>(p, sms, stream);
   if (tile.bn == 128) return launch_tiles<128, false>(p, sms, stream);
   return launch_tiles<64, false>(p, sms, stream);
 }
@@ -530,7 +533,9 @@ int launch_linear(const LinearBatchedArgs& ba, int sms, cudaStream_t stream) {
   ProjParams p;
   if (a.M >= (1ll << 31)) return GCA_ERR_TOO_LARGE;
   int rc;
-  if ((rc = make_rows_map(&p.tm_x, a.x, args.batches, a.M, a.K, a.x_stride, args.x_batch_stride, 64))) return rc;
+  rc = args.batches > 1 ? make_rows_map(&p.tm_x, a.x, args.batches, a.M, a.K, a.x_stride, args.x_batch_stride, 64)
+                        : make_matrix_map(&p.tm_x, a.x, a.M, a.K, a.x_stride, BM);
+  if (rc) return rc;
   p.k_cache = p.v_cache = nullptr; p.status = a.status; p.cache_bs = 0;
   const long long per_batch = (a.M + 63) / 64;
   p.M = (int)a.M; p.D = a.K; p.rows_per_seq = 1; p.pos = 0; p.zero_landmark = 0; p.nmat = 1;

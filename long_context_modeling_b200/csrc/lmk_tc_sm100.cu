@@ -58,7 +58,7 @@ lmk_screen_kernel(const __grid_constant__ ScreenParams p) {
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + NUM_BARS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + NUM_BARS + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int list = blockIdx.x, t0 = blockIdx.y * BM, n = blockIdx.z;
   const int rows = min(BM, p.Cq - t0), ksteps = p.D / BK;
   // tiles of this list that some row of the block can see
@@ -82,25 +82,23 @@ lmk_screen_kernel(const __grid_constant__ ScreenParams p) {
   const uint32_t tmem = *tmem_slot;
 
   if (warp == WORKERS) {
-    if (lane == 0) {
-      uint32_t it = 0;
-      bool ok = true;
-      for (int t = first; t < last && ok; ++t)
-        for (int ks = 0; ks < ksteps; ++ks, ++it) {
-          const uint32_t st = it % STAGES;
-          ok = mbar_wait_bounded(&bars[EMPTY + st], ((it / STAGES) & 1) ^ 1, abort_flag);
-          if (!ok) break;
-          mbar_arrive_expect_tx(&bars[FULL + st], STAGE_BYTES);
-          tma_load_3d(smem + st * STAGE_BYTES, &p.tm_q, &bars[FULL + st], ks * BK, t0, n);
-          tma_load_3d(smem + st * STAGE_BYTES + A_BYTES, &p.tm_k, &bars[FULL + st], ks * BK, t * BN, n);
-        }
-      if (*abort_flag)          // nothing may land in shared memory after the block has gone
-        for (uint32_t back = 0; back < (uint32_t)STAGES && back < it; ++back) {
-          const uint32_t g = it - 1 - back;
-          for (int i = 0; i < (1 << 20); ++i)
-            if (mbar_try_wait(&bars[FULL + g % STAGES], (g / STAGES) & 1)) break;
-        }
-    }
+    uint32_t it = 0;
+    bool ok = true;
+    for (int t = first; t < last && ok; ++t)
+      for (int ks = 0; ks < ksteps; ++ks, ++it) {
+        const uint32_t st = it % STAGES;
+        ok = mbar_wait_warp(&bars[EMPTY + st], ((it / STAGES) & 1) ^ 1, abort_flag, lane);
+        if (!ok) break;
+        mbar_expect_tx_elect(&bars[FULL + st], STAGE_BYTES);
+        tma_load_3d_elect(smem + st * STAGE_BYTES, &p.tm_q, &bars[FULL + st], ks * BK, t0, n);
+        tma_load_3d_elect(smem + st * STAGE_BYTES + A_BYTES, &p.tm_k, &bars[FULL + st], ks * BK, t * BN, n);
+      }
+    if (*abort_flag)          // nothing may land in shared memory after the block has gone
+      for (uint32_t back = 0; back < (uint32_t)STAGES && back < it; ++back) {
+        const uint32_t g = it - 1 - back;
+        for (int i = 0; i < (1 << 20); ++i)
+          if (mbar_try_wait(&bars[FULL + g % STAGES], (g / STAGES) & 1)) break;
+      }
   } else if (warp == WORKERS + 1) {
     uint32_t it = 0, tile = 0;
     bool ok = true;

@@ -1,7 +1,7 @@
 // out[m, :] = scale[m] * (x[m, :] . w^T) + residual[m, :] for a handful of rows (a decode step: one or two per sequence).
 //
 // Bound: latency.  768 x 768 weights are 1.2 MB, 0.2 us of HBM time; the 128 x 256-tile GEMM keeps 3 SMs busy with
-// them for 9 us.  Here a block owns 8 output columns (96 blocks for 768), its 8 warps split the contraction, and every
+// them for 9 us.  Here a block owns 8 or 16 output columns (96 blocks for 768), its 8 warps split the contraction, and every
 // operand goes from global memory straight into mma.sync fragments: a 16-byte load per lane covers 8 consecutive k of one
 // column (or row), and since a dot product does not care about the order of k, those 8 serve as the fragment's k slots
 // of two steps -- the same permutation on both sides, no shared memory, no shuffles.  Partial sums of the warps are
@@ -44,40 +44,50 @@ __device__ __forceinline__ float sum_sq(const uint4& v, float s) {
   return s;
 }
 
-// MT: 16-row tiles (M <= 16 MT)
-template <int MT>
+// A block: 16 MT rows x 8 NT columns.
+template <int MT, int NT>
 __global__ void __launch_bounds__(WARPS * 32)
 skinny_linear_kernel(const SkinnyParams p) {
-  __shared__ float part[WARPS][MT * 16][8];
+  constexpr int COLS = 8 * NT;
+  __shared__ float part[WARPS][MT * 16][COLS];
   __shared__ float part_ss[WARPS][MT * 16];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = lane >> 2, quad = lane & 3;
-  const int n0 = blockIdx.x * 8, blocks = p.K / 32;
+  const int n0 = blockIdx.x * COLS, m0 = blockIdx.y * MT * 16, rows = min(MT * 16, p.M - m0), blocks = p.K / 32;
   const __nv_bfloat16* wrow = p.w + (long long)(n0 + grp) * p.w_stride + quad * 8;
-  for (int kb = warp; kb < blocks; kb += WARPS) asm volatile("prefetch.global.L2 [%0];" ::"l"(wrow + kb * 32));
+  const __nv_bfloat16* x = p.x + m0 * p.x_stride + quad * 8;
+  for (int kb = warp; kb < blocks; kb += WARPS)
+#pragma unroll
+    for (int t = 0; t < NT; ++t) asm volatile("prefetch.global.L2 [%0];" ::"l"(wrow + 8 * t * p.w_stride + kb * 32));
   pdl_trigger();
   pdl_wait();
-  float acc[MT][4], ss[MT][2];
+  float acc[MT][NT][4], ss[MT][2];
 #pragma unroll
   for (int m = 0; m < MT; ++m) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) acc[m][i] = 0.f;
+    for (int t = 0; t < NT; ++t)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc[m][t][i] = 0.f;
     ss[m][0] = ss[m][1] = 0.f;
   }
 #pragma unroll 3
   for (int kb = warp; kb < blocks; kb += WARPS) {
-    const uint4 b = *reinterpret_cast<const uint4*>(wrow + kb * 32);
-    uint4 a[MT][2];
+    uint4 b[NT], a[MT][2];
+#pragma unroll
+    for (int t = 0; t < NT; ++t) b[t] = *reinterpret_cast<const uint4*>(wrow + 8 * t * p.w_stride + kb * 32);
 #pragma unroll
     for (int m = 0; m < MT; ++m)
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int r = m * 16 + h * 8 + grp;
-        a[m][h] = r < p.M ? *reinterpret_cast<const uint4*>(p.x + r * p.x_stride + kb * 32 + quad * 8) : make_uint4(0, 0, 0, 0);
+        a[m][h] = r < rows ? *reinterpret_cast<const uint4*>(x + r * p.x_stride + kb * 32) : make_uint4(0, 0, 0, 0);
       }
 #pragma unroll
     for (int m = 0; m < MT; ++m) {
-      mma_bf16(acc[m], a[m][0].x, a[m][1].x, a[m][0].y, a[m][1].y, b.x, b.y);
-      mma_bf16(acc[m], a[m][0].z, a[m][1].z, a[m][0].w, a[m][1].w, b.z, b.w);
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        mma_bf16(acc[m][t], a[m][0].x, a[m][1].x, a[m][0].y, a[m][1].y, b[t].x, b[t].y);
+        mma_bf16(acc[m][t], a[m][0].z, a[m][1].z, a[m][0].w, a[m][1].w, b[t].z, b[t].w);
+      }
       if (p.rms_eps > 0.f) {
         ss[m][0] = sum_sq(a[m][0], ss[m][0]);
         ss[m][1] = sum_sq(a[m][1], ss[m][1]);
@@ -89,7 +99,9 @@ skinny_linear_kernel(const SkinnyParams p) {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const int r = m * 16 + h * 8 + grp;
-      *reinterpret_cast<float2*>(&part[warp][r][quad * 2]) = make_float2(acc[m][2 * h], acc[m][2 * h + 1]);
+#pragma unroll
+      for (int t = 0; t < NT; ++t)
+        *reinterpret_cast<float2*>(&part[warp][r][t * 8 + quad * 2]) = make_float2(acc[m][t][2 * h], acc[m][t][2 * h + 1]);
       if (p.rms_eps > 0.f) {
         float s = ss[m][h];
         s += __shfl_xor_sync(0xffffffffu, s, 1);
@@ -99,8 +111,9 @@ skinny_linear_kernel(const SkinnyParams p) {
     }
   __syncthreads();
   // a thread finishes two neighbouring columns of a row
-  for (int i = threadIdx.x; i < p.M * 4; i += WARPS * 32) {
-    const int r = i >> 2, c = (i & 3) * 2;
+  for (int i = threadIdx.x; i < rows * (COLS / 2); i += WARPS * 32) {
+    const int r = i / (COLS / 2), c = (i % (COLS / 2)) * 2;
+    const long long row = m0 + r;
     float2 t = make_float2(0.f, 0.f);
 #pragma unroll
     for (int wv = 0; wv < WARPS; ++wv) {
@@ -114,14 +127,14 @@ skinny_linear_kernel(const SkinnyParams p) {
 #pragma unroll
       for (int wv = 0; wv < WARPS; ++wv) s += part_ss[wv][r];
       sc = rsqrtf(s / (float)p.K + p.rms_eps);
-    } else if (p.row_scale) sc = p.row_scale[r];
+    } else if (p.row_scale) sc = p.row_scale[row];
     float2 res = make_float2(0.f, 0.f);
     if (p.residual) {
-      const unsigned v = *reinterpret_cast<const unsigned*>(p.residual + r * p.res_stride + n0 + c);
+      const unsigned v = *reinterpret_cast<const unsigned*>(p.residual + row * p.res_stride + n0 + c);
       res = make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
     }
     const __nv_bfloat162 o = __floats2bfloat162_rn(fmaf(t.x, sc, res.x), fmaf(t.y, sc, res.y));
-    *reinterpret_cast<__nv_bfloat162*>(p.out + r * p.out_stride + n0 + c) = o;
+    *reinterpret_cast<__nv_bfloat162*>(p.out + row * p.out_stride + n0 + c) = o;
   }
 }
 
@@ -134,11 +147,9 @@ int launch_skinny_linear(const LinearArgs& a, float rms_eps, cudaStream_t stream
   p.residual = (const __nv_bfloat16*)a.residual; p.row_scale = a.row_scale;
   p.x_stride = a.x_stride; p.w_stride = a.w_stride; p.out_stride = a.out_stride; p.res_stride = a.residual_stride;
   p.M = (int)a.M; p.K = a.K; p.rms_eps = rms_eps;
-  const dim3 grid((unsigned)(a.N / 8)), block(WARPS * 32);
-  if (a.M <= 16) return (int)launch_dependent(skinny_linear_kernel<1>, grid, block, 0, stream, p);
-  if (a.M <= 32) return (int)launch_dependent(skinny_linear_kernel<2>, grid, block, 0, stream, p);
-  if (a.M <= 64) return (int)launch_dependent(skinny_linear_kernel<4>, grid, block, 0, stream, p);
-  return (int)launch_dependent(skinny_linear_kernel<8>, grid, block, 0, stream, p);
+  // more rows: 32 x 16 per block, so that neither operand is read by more blocks than needed to fill the SMs
+  if (a.M <= 16) return (int)launch_dependent(skinny_linear_kernel<1, 1>, dim3((unsigned)(a.N / 8)), dim3(WARPS * 32), 0, stream, p);
+  return (int)launch_dependent(skinny_linear_kernel<2, 2>, dim3((unsigned)(a.N / 16), (unsigned)((a.M + 31) / 32)), dim3(WARPS * 32), 0, stream, p);
 }
 
 }  // namespace gca
