@@ -249,6 +249,7 @@ int gca_bwd_stages(const GcaBwdArgs* a, unsigned stages, void* stream) {
   else rc = GCA_ERR_ALGO;
   if (rc) return rc;
   if (!(stages & GCA_BWD_STAGE_Q)) return 0;
+  if (algo == GCA_ALGO_TC && (stages & GCA_BWD_STAGE_KV)) return 0;      // the kv-major kernel has reduced dw
   return gca::launch_dw_reduce(dw_part, a->dw, a->N * a->J, a->Hq, a->K, algo == GCA_ALGO_TC ? gca::bwd_tc_dw_parts() : 1, s);
 }
 

@@ -146,7 +146,27 @@ struct BwdKvParams {
   int N, J, Hq, Hkv, G, K, C, HP;
   int wide_store;           // dk / dv rows are 32-byte aligned: 256-bit stores
   float c2, sm_scale;
+  const float4* dw_part;    // (N*J, Hq, K): the q-major pass's four partials of every (head, slot) of dw, or nullptr
+  float* dw;                // (N*J, K)
 };
+
+// dw[zj, k] = the partials of all heads in a fixed order (the same as dw_reduce_kernel's).  A launch of its own for these few
+// additions took 10 us between the passes; here the worker warps do it while the first K / V and Q / dO tiles are on their way.
+__device__ __forceinline__ void reduce_dw(const BwdKvParams& p) {
+  if (!p.dw_part) return;
+  const int total = p.N * p.J * p.K;
+  for (int i = blockIdx.x * (4 * NG * 32) + threadIdx.x; i < total; i += gridDim.x * (4 * NG * 32)) {
+    const int zj = i / p.K, k = i - zj * p.K;
+    const float4* src = p.dw_part + (long long)zj * p.Hq * p.K + k;
+    float t = 0.f;
+#pragma unroll 4
+    for (int h = 0; h < p.Hq; ++h) {
+      const float4 v = src[(long long)h * p.K];
+      t += v.x; t += v.y; t += v.z; t += v.w;
+    }
+    p.dw[i] = t;
+  }
+}
 
 // One lane: K + V per unit; per iteration Q + dO, the two heads' row-term tiles and the weight.
 __device__ void kv_producer(const BwdKvParams& p, uint8_t* smem, uint64_t* bars, volatile int* abort_flag) {
@@ -473,7 +493,7 @@ bwd_kv_tc_kernel(const __grid_constant__ BwdKvParams p) {
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + NUM_BARS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + NUM_BARS + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int i = 0; i < NBUF; ++i) {
       mbar_init(&bars[SP_FULL + i], 2);                              // S^T commit + dP^T commit
@@ -502,8 +522,10 @@ bwd_kv_tc_kernel(const __grid_constant__ BwdKvParams p) {
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  if (warp < 4 * NG) kv_worker(p, smem, bars, abort_flag, warp >> 2, warp & 3, lane, tmem_base);
-  else if (warp == PROD_WARP) { if (lane == 0) kv_producer(p, smem, bars, abort_flag); }
+  if (warp < 4 * NG) {
+    reduce_dw(p);                        // while the first tiles are on their way
+    kv_worker(p, smem, bars, abort_flag, warp >> 2, warp & 3, lane, tmem_base);
+  } else if (warp == PROD_WARP) { if (lane == 0) kv_producer(p, smem, bars, abort_flag); }
   else if (warp == ISSUE_S) kv_issuer<0>(p, smem, bars, abort_flag, lane, tmem_base);
   else if (warp == ISSUE_DP) kv_issuer<1>(p, smem, bars, abort_flag, lane, tmem_base);
   else if (warp == ISSUE_DV) kv_issuer<2>(p, smem, bars, abort_flag, lane, tmem_base);
@@ -525,8 +547,8 @@ bool rows_32b_aligned(const void* base, const int64_t* stride) {
 }  // namespace
 
 // rowterm: the per-row term tiles as the q-major pass wrote them into the workspace (1 KB per
-// (row block, head, slot)).
-int launch_bwd_kv_tc(const GcaBwdArgs& a, const Csr& csr, const uint4* rowterm, int sms, cudaStream_t stream) {
+// (row block, head, slot)).  dw_part: reduce these partials into a.dw on the way, or nullptr.
+int launch_bwd_kv_tc(const GcaBwdArgs& a, const Csr& csr, const uint4* rowterm, const float* dw_part, int sms, cudaStream_t stream) {
   BwdKvParams p;
   int rc;
   auto qmap = [&](CUtensorMap* m, const void* base, const int64_t* st, int box) {
@@ -553,6 +575,7 @@ int launch_bwd_kv_tc(const GcaBwdArgs& a, const Csr& csr, const uint4* rowterm, 
   if (p.units == 0) return 0;
   GCA_CUDA_CHECK(cudaFuncSetAttribute(bwd_kv_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
   const unsigned grid = (unsigned)(p.units < sms ? p.units : sms);
+  p.dw_part = reinterpret_cast<const float4*>(dw_part); p.dw = a.dw;
   bwd_kv_tc_kernel<<<grid, NTHREADS, SMEM_BYTES, stream>>>(p);
   GCA_CUDA_CHECK(cudaGetLastError());
   return 0;

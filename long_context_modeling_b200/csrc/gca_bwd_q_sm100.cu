@@ -140,6 +140,7 @@ __device__ __forceinline__ void drain(uint64_t* bars, int full0, uint32_t issued
 
 struct BwdQParams {
   CUtensorMap tm_q, tm_do, tm_k2, tm_v2, tm_k1, tm_v1;
+  int beside_index;         // launched while the index is being built (everything before THAT is complete): wait at the end, not here
   const int32_t* indices;
   const float* weights;
   const float* lse;
@@ -515,7 +516,7 @@ bwd_q_tc_kernel(const __grid_constant__ BwdQParams p) {
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + NUM_BARS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + NUM_BARS + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) {
       mbar_init(&bars[QDO_FULL + i], 1);
@@ -541,12 +542,15 @@ bwd_q_tc_kernel(const __grid_constant__ BwdQParams p) {
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_trigger();
+  if (!p.beside_index) pdl_wait();
   if (warp < 4 * NWG) q_worker(p, smem, bars, abort_flag, warp >> 2, warp & 3, lane, tmem_base);
   else if (warp == PROD_WARP) q_producer(p, smem, bars, abort_flag, lane);
   else if (warp >= WRITER_WARP) q_writer(p, bars, abort_flag, warp & 3, lane, tmem_base);
   else if (warp == ISSUE_S) q_issuer<0>(p, smem, bars, abort_flag, lane, tmem_base);
   else if (warp == ISSUE_DP) q_issuer<1>(p, smem, bars, abort_flag, lane, tmem_base);
   else if (warp == ISSUE_DQ) q_issuer<2>(p, smem, bars, abort_flag, lane, tmem_base);
+  if (p.beside_index) pdl_wait();        // the index is complete before this kernel is
   tc_fence_before();
   __syncthreads();
   if (warp == ISSUE_S) tmem_dealloc(tmem_base, TMEM_COLS);
@@ -564,7 +568,7 @@ bool rows_32b_aligned(const void* base, const int64_t* stride) {
 }  // namespace
 
 // dw_part: (N*J, Hq, K, 4) float32 partials; rowterm: (N*J, Hq, K, 64) x 16 bytes (see BwdQParams).
-int launch_bwd_q_tc(const GcaBwdArgs& a, float* dw_part, uint4* rowterm, int sms, cudaStream_t stream) {
+int launch_bwd_q_tc(const GcaBwdArgs& a, float* dw_part, uint4* rowterm, bool beside_index, int sms, cudaStream_t stream) {
   const float c2 = a.sm_scale * GCA_LOG2E;
   int rc;
   auto qmap = [&](CUtensorMap* m, const void* base, const int64_t* st, int box) {
@@ -592,9 +596,8 @@ int launch_bwd_q_tc(const GcaBwdArgs& a, float* dw_part, uint4* rowterm, int sms
   if (p.units == 0) return 0;
   GCA_CUDA_CHECK(cudaFuncSetAttribute(bwd_q_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
   const unsigned grid = (unsigned)(p.units < sms ? p.units : sms);
-  bwd_q_tc_kernel<<<grid, NTHREADS, SMEM_BYTES, stream>>>(p);
-  GCA_CUDA_CHECK(cudaGetLastError());
-  return 0;
+  p.beside_index = beside_index;
+  return (int)launch_dependent(bwd_q_tc_kernel, dim3(grid), dim3(NTHREADS), SMEM_BYTES, stream, p);
 }
 
 }  // namespace gca

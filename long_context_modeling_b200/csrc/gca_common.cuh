@@ -76,18 +76,18 @@ struct Geom {
   float off_by_one;
 };
 
-// Inverse retrieval index: for every cache chunk (n, c) the sorted list of (j*K + k)
-// entries that retrieved it.  `offsets` has N*C + 1 entries into `sorted_keys`, whose low
-// 32 bits hold the entry.
-// `unit_tab` lists the chunks in the order the kv-major tensor-core kernel walks them: sequence
+// Inverse retrieval index: for every cache chunk (n, c) the list of (j*K + k) entries that retrieved it, in order: the low
+// 32 bits of `sorted_keys`.
+// `unit_tab` lists the chunks in the order the kv-major kernels walk them: sequence
 // by sequence, and inside a sequence by DECREASING number of retrievers (x = first entry,
 // y = one past the last, z = chunk id n*C + c).  CTAs take units round-robin, so every CTA gets
 // chunks of every size class; in chunk order the busiest CTA had 8 % more work than the average
 // (chunks near the start of a sequence are retrieved by many more queries than late ones).
+// `overlaps`: the kernel that builds it was just launched and lets the next kernel on the stream start before it is done.
 struct Csr {
-  const int* offsets;
   const unsigned long long* sorted_keys;
   const int4* unit_tab;
+  bool overlaps;
 };
 
 // launch == false: only lay the index out in `workspace` (it was built by an earlier call)

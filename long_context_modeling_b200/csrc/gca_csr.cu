@@ -5,8 +5,8 @@
 // Each valid entry becomes the 64-bit key  (n*C + c) << 32 | (j*K + k); a stable radix sort
 // on the chunk field gives the lists back to back (two 8-bit passes at N*C = 2048 instead of
 // the eight of a full 64-bit sort), and a binary search per chunk finds where each list starts.
-// Padding slots (index < 0) and out-of-range indices sort to the end.  Small problems take a
-// single-launch counting sort with the same result (csr_small_kernel).
+// Padding slots (index < 0) and out-of-range indices sort to the end.  Problems of a training step's size take a
+// single launch with the same result (csr_list_kernel).
 #include <cstdlib>
 
 #include <cub/device/device_radix_sort.cuh>
@@ -56,138 +56,100 @@ __global__ void csr_offsets_kernel(const unsigned long long* __restrict__ sorted
 }
 
 // ---------------------------------------------------------------------------------------------
-// Small problems (C <= 1024 chunks per sequence; the training shapes): the whole index in ONE
-// launch, one CTA per sequence, bit-identical to the radix-sort path below, which costs nine
-// launches (~85 us, against ~2 ms for the whole backward at the 16K-token shape).
-//   1. every warp histograms its own contiguous range of the sequence's J*K entries (shared memory)
-//   2. per chunk, an exclusive prefix over the 32 warps; a block scan over the chunks
-//   3. every warp walks its range again IN ORDER and places each entry at
-//        base(sequence) + start(chunk) + entries of earlier warps + entries earlier in this warp
-//      (rank inside a round of 32 by __match_any_sync), i.e. a stable counting sort
-//   4. the sequence's chunks sorted by decreasing count (bitonic, shared memory) -> unit table
-// base(sequence) = number of valid entries of all earlier sequences, counted by every CTA itself
-// (no CTA waits for another).
-constexpr int SMALL_C = 1024, SMALL_THREADS = 1024;
+// Problems of a training step's size: the whole index in ONE launch of small blocks, bit-identical to the radix-sort path
+// below, which costs nine launches (~85 us).  A block handles eight chunks of a sequence; its warps read a section of the
+// sequence's J*K entries each, twice:
+//   1. counting the retrievers of ALL the sequence's chunks (shared-memory histogram; redundant between blocks, but J*K
+//      reads from L2 are nothing) and of the block's own chunks per section.  That gives every list its start -- lists of
+//      a sequence lie back to back from entry n * J * K --, its place in the walking order (chunks by decreasing count,
+//      ties by id), and every section its first entry of every list;
+//   2. writing the entries that name one of the block's chunks, in order.
+// What bounds it is the chain of loads: 16 are in flight per lane.  Few registers, 4 bytes of shared memory per chunk: its
+// blocks run BESIDE the q-major pass, which is launched while they work (nothing in it depends on the index) and fills
+// the SMs to all but this.  In front of the q-major pass (one block per sequence, 145 KB of shared memory) it took 14 us
+// at 8 x 256 chunks, K = 8, and 34 us at 1,024 chunks, K = 16.
+constexpr int LIST_WARPS = 8, LIST_MAX_C = 2048, LIST_LOADS = 16;
 
-__global__ void __launch_bounds__(SMALL_THREADS, 1)
-csr_small_kernel(const int32_t* __restrict__ indices, unsigned long long* __restrict__ keys_out, int* __restrict__ offsets,
-                 int4* __restrict__ unit_tab, int N, int JK, int C) {
-  extern __shared__ int sm[];
-  int* hw = sm;                         // [32][C]
-  int* start = hw + 32 * C;             // [C + 1]
-  int* cnt = start + C + 1;             // [C]
-  unsigned* skey = reinterpret_cast<unsigned*>(cnt + C);   // [Cp2]
-  int* red = reinterpret_cast<int*>(skey + SMALL_C);       // [33]
-  const int n = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+__global__ void __launch_bounds__(LIST_WARPS * 32)
+csr_list_kernel(const int32_t* __restrict__ indices, unsigned long long* __restrict__ keys_out, int4* __restrict__ unit_tab, int JK, int C) {
+  __shared__ int cnt[LIST_MAX_C];
+  __shared__ int sect[LIST_WARPS][LIST_WARPS];       // [section][chunk of this block]: entries, then the first one's place
+  const int n = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int32_t* row = indices + (long long)n * JK;
-  for (int i = tid; i < 32 * C; i += SMALL_THREADS) hw[i] = 0;
-  // valid entries of the sequences before this one
-  int before = 0;
-  for (long long i = tid; i < (long long)n * JK; i += SMALL_THREADS) {
-    const int v = indices[i];
-    before += (v >= 0 && v < C);
-  }
+  for (int i = threadIdx.x; i < C; i += LIST_WARPS * 32) cnt[i] = 0;
+  if (threadIdx.x < LIST_WARPS * LIST_WARPS) (&sect[0][0])[threadIdx.x] = 0;
+  pdl_wait();
+  pdl_trigger();                         // everything before this kernel is complete: the next one may start
+  __syncthreads();
+  const int c0 = blockIdx.x * LIST_WARPS, c1 = min(c0 + LIST_WARPS, C);
+  const int per = ((JK + LIST_WARPS * 32 - 1) / (LIST_WARPS * 32)) * 32, first = warp * per, last = min(first + per, JK);
+  for (int t0 = first; t0 < last; t0 += 32 * LIST_LOADS) {
+    int v[LIST_LOADS];
 #pragma unroll
-  for (int of = 16; of > 0; of >>= 1) before += __shfl_xor_sync(0xffffffffu, before, of);
-  if (lane == 0) red[warp] = before;
-  __syncthreads();
-  if (warp == 0) {
-    int v = red[lane];
+    for (int x = 0; x < LIST_LOADS; ++x) v[x] = t0 + 32 * x + lane < last ? row[t0 + 32 * x + lane] : -1;
 #pragma unroll
-    for (int of = 16; of > 0; of >>= 1) v += __shfl_xor_sync(0xffffffffu, v, of);
-    if (lane == 0) red[32] = v;
-  }
-  // 1. per-warp histograms; warp w owns entries [w * per, (w + 1) * per), per a multiple of 32
-  const int per = (((JK + 31) / 32) + 31) / 32 * 32;
-  const int t0 = warp * per, t1 = min(JK, t0 + per);
-  for (int t = t0 + lane; t < t1; t += 32) {
-    const int v = row[t];
-    if (v >= 0 && v < C) atomicAdd(&hw[warp * C + v], 1);
-  }
-  __syncthreads();
-  const int gbase = red[32];
-  // 2. exclusive prefix over the warps per chunk, then over the chunks
-  int mine = 0;
-  if (tid < C) {
-    int run = 0;
-    for (int w = 0; w < 32; ++w) { const int v = hw[w * C + tid]; hw[w * C + tid] = run; run += v; }
-    cnt[tid] = run;
-    mine = run;
-  }
-  int incl = mine;
-#pragma unroll
-  for (int of = 1; of < 32; of <<= 1) { const int v = __shfl_up_sync(0xffffffffu, incl, of); if (lane >= of) incl += v; }
-  __syncthreads();                       // red[] is read above by everybody before it is reused
-  if (lane == 31) red[warp] = incl;
-  __syncthreads();
-  if (warp == 0) {
-    int v = red[lane], s = v;
-#pragma unroll
-    for (int of = 1; of < 32; of <<= 1) { const int u = __shfl_up_sync(0xffffffffu, s, of); if (lane >= of) s += u; }
-    red[lane] = s - v;                   // exclusive prefix of the warp totals
-    if (lane == 31) start[C] = s;        // the sequence's number of valid entries (C <= 1024: all chunks covered)
-  }
-  __syncthreads();
-  if (tid < C) start[tid] = red[warp] + incl - mine;
-  __syncthreads();
-  // 3. stable placement
-  for (int t = t0 + lane; t < t0 + per; t += 32) {      // whole rounds: every lane takes part in the votes
-    const int v = t < t1 ? row[t] : -1;
-    const bool valid = v >= 0 && v < C;
-    const unsigned peers = __match_any_sync(0xffffffffu, valid ? v : -1 - lane);
-    const int rank = __popc(peers & ((1u << lane) - 1u));
-    int pos = 0;
-    if (valid) pos = gbase + start[v] + hw[warp * C + v] + rank;
-    __syncwarp();
-    if (valid) {
-      keys_out[pos] = (((unsigned long long)((long long)n * C + v)) << 32) | (unsigned)t;
-      if (rank == 0) hw[warp * C + v] += __popc(peers);
+    for (int x = 0; x < LIST_LOADS; ++x) {
+      if (v[x] >= 0 && v[x] < C) atomicAdd(&cnt[v[x]], 1);
+      if (v[x] >= c0 && v[x] < c1) atomicAdd(&sect[warp][v[x] - c0], 1);
     }
-    __syncwarp();
   }
-  // offsets
-  if (tid < C) offsets[(long long)n * C + tid] = gbase + start[tid];
-  if (n == N - 1 && tid == 0) offsets[(long long)N * C] = gbase + start[C];
-  // 4. walking order of the sequence's chunks: by decreasing count, ties by chunk id
-  int cp2 = 1;
-  while (cp2 < C) cp2 <<= 1;
-  for (int i = tid; i < cp2; i += SMALL_THREADS)
-    skey[i] = i < C ? (((unsigned)(JK - cnt[i])) << 10) | (unsigned)i : 0xffffffffu;
   __syncthreads();
-  for (int k = 2; k <= cp2; k <<= 1)
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int i = tid; i < cp2; i += SMALL_THREADS) {
-        const int ixj = i ^ j;
-        if (ixj > i) {
-          const unsigned a = skey[i], b = skey[ixj];
-          const bool up = (i & k) == 0;
-          if ((a > b) == up) { skey[i] = b; skey[ixj] = a; }
-        }
+  const int c = c0 + warp;
+  if (c < c1) {
+    const int mine = cnt[c];
+    int start = 0, rank = 0;
+    for (int i = lane; i < C; i += 32) {
+      const int v = cnt[i];
+      start += i < c ? v : 0;
+      rank += v > mine || (v == mine && i < c);
+    }
+#pragma unroll
+    for (int of = 16; of > 0; of >>= 1) {
+      start += __shfl_xor_sync(0xffffffffu, start, of);
+      rank += __shfl_xor_sync(0xffffffffu, rank, of);
+    }
+    start += n * JK;
+    if (lane == 0) {
+      unit_tab[(long long)n * C + rank] = make_int4(start, start + mine, n * C + c, 0);
+      for (int w = 0; w < LIST_WARPS; ++w) {
+        const int here = sect[w][warp];
+        sect[w][warp] = start;
+        start += here;
       }
-      __syncthreads();
     }
-  if (tid < C) {
-    const int c = (int)(skey[tid] & 1023u);
-    const int beg = gbase + start[c];
-    unit_tab[(long long)n * C + tid] = make_int4(beg, beg + cnt[c], n * C + c, 0);
   }
+  __syncthreads();
+  for (int t0 = first; t0 < last; t0 += 32 * LIST_LOADS) {
+    int v[LIST_LOADS];
+#pragma unroll
+    for (int x = 0; x < LIST_LOADS; ++x) v[x] = t0 + 32 * x + lane < last ? row[t0 + 32 * x + lane] : -1;
+#pragma unroll
+    for (int x = 0; x < LIST_LOADS; ++x) {
+      const bool hit = v[x] >= c0 && v[x] < c1;
+      if (!__any_sync(0xffffffffu, hit)) continue;
+      const unsigned same = __match_any_sync(0xffffffffu, hit ? v[x] : -1), before = same & ((1u << lane) - 1u);
+      const int at = hit ? sect[warp][v[x] - c0] : 0;
+      if (hit) keys_out[at + __popc(before)] = (unsigned long long)((long long)n * C + v[x]) << 32 | (unsigned)(t0 + 32 * x + lane);
+      __syncwarp();
+      if (hit && before == 0) sect[warp][v[x] - c0] = at + __popc(same);
+      __syncwarp();
+    }
+  }
+}
+
+// Beyond 2^27 (blocks x entries x 8, a few tens of microseconds of L2 reads) or 2,048 chunks per sequence: the sort.
+bool small_path(int N, int JK, int C) {
+  return C <= LIST_MAX_C && (long long)N * JK < (1ll << 31) && (long long)N * C * JK <= (1ll << 27) && N <= 65535;
 }
 
 // The pre-gathered call: chunk c of row block n is read by its slot c and nothing else.
-__global__ void csr_identity_kernel(unsigned long long* __restrict__ keys_out, int* __restrict__ offsets, int4* __restrict__ unit_tab, int NC,
-                                    int C) {
+__global__ void csr_identity_kernel(unsigned long long* __restrict__ keys_out, int4* __restrict__ unit_tab, int NC, int C) {
+  pdl_wait();
+  pdl_trigger();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i > NC) return;
-  offsets[i] = i;
-  if (i == NC) return;
+  if (i >= NC) return;
   keys_out[i] = ((unsigned long long)i << 32) | (unsigned)(i % C);
   unit_tab[i] = make_int4(i, i + 1, i, 0);
-}
-
-size_t small_smem_bytes(int C) { return (size_t)(32 * C + (C + 1) + C + SMALL_C + 33) * 4; }
-
-bool small_path(int N, int JK, int C) {
-  return C <= SMALL_C && JK < (1 << 21) && (long long)N * JK <= (1ll << 18);
 }
 
 size_t cub_temp_bytes(long long total) {
@@ -242,14 +204,14 @@ int build_csr(const int32_t* indices, int N, int J, int K, int C, void* workspac
   const long long cmax = (long long)J * K;
   const int cbits = bits_for(cmax), nbits = bits_for(N);
   if (cbits + nbits > 32) return GCA_ERR_TOO_LARGE;
+  out->overlaps = false;
   if (launch && !indices && NC > 0) {
-    csr_identity_kernel<<<(unsigned)((NC + 1 + 255) / 256), 256, 0, stream>>>(keys_out, offsets, uvals_out, (int)NC, C);
-    GCA_CUDA_CHECK(cudaGetLastError());
+    GCA_CUDA_CHECK(launch_dependent(csr_identity_kernel, dim3((unsigned)((NC + 255) / 256)), dim3(256), 0, stream, keys_out, uvals_out, (int)NC, C));
+    out->overlaps = true;
   } else if (launch && NC > 0 && total > 0 && !by_sort && small_path(N, J * K, C)) {
-    const size_t smem = small_smem_bytes(C);
-    GCA_CUDA_CHECK(cudaFuncSetAttribute(csr_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    csr_small_kernel<<<N, SMALL_THREADS, smem, stream>>>(indices, keys_out, offsets, uvals_out, N, J * K, C);
-    GCA_CUDA_CHECK(cudaGetLastError());
+    GCA_CUDA_CHECK(launch_dependent(csr_list_kernel, dim3((unsigned)((C + LIST_WARPS - 1) / LIST_WARPS), (unsigned)N), dim3(LIST_WARPS * 32), 0,
+                                    stream, indices, keys_out, uvals_out, J * K, C));
+    out->overlaps = true;
   } else if (launch) {
     if (total > 0) {
       csr_keys_kernel<<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(indices, keys_in, N, J * K, C);
@@ -270,7 +232,6 @@ int build_csr(const int32_t* indices, int N, int J, int K, int C, void* workspac
                                                      cbits + nbits, stream));
     }
   }
-  out->offsets = offsets;
   out->sorted_keys = keys_out;
   out->unit_tab = uvals_out;
   *used_bytes = need;

@@ -633,7 +633,7 @@ fwd_tc_kernel(const __grid_constant__ FwdTcParams p) {
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + NUM_BARS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + NUM_BARS + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) { mbar_init(&bars[Q_FULL + i], 1); mbar_init(&bars[Q_EMPTY + i], 1); }
@@ -652,6 +652,8 @@ fwd_tc_kernel(const __grid_constant__ FwdTcParams p) {
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_trigger();
+  pdl_wait();
 
   if (warp < 4 * NWG) softmax_role(p, smem, bars, abort_flag, warp >> 2, warp & 3, lane, tmem_base);
   else if (warp == KPROD_WARP) kproducer_role(p, smem, bars, abort_flag, lane);
@@ -703,8 +705,7 @@ int launch_fwd_tc(const GcaFwdArgs& a, int sms, cudaStream_t stream) {
   if (p.units == 0) return 0;
   GCA_CUDA_CHECK(cudaFuncSetAttribute(fwd_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
   const unsigned grid = (unsigned)(p.units < sms ? p.units : sms);
-  fwd_tc_kernel<<<grid, NTHREADS, SMEM_BYTES, stream>>>(p);
-  return (int)cudaGetLastError();
+  return (int)launch_dependent(fwd_tc_kernel, dim3(grid), dim3(NTHREADS), SMEM_BYTES, stream, p);
 }
 
 }  // namespace gca

@@ -272,6 +272,13 @@ def test_inverse_index_single_launch_equals_radix_sort(lcm, shape):
     assert lcm.read_status() == 0
 
 
+@pytest.mark.parametrize("shape", [(1, 301, 2, 16), (2, 3, 2, 1), (1, 2048, 2, 2), (1, 2049, 2, 2)])
+def test_inverse_index_sections_equal_radix_sort(lcm, shape):
+    """The block-wise index at its edges: several rounds of loads per section with a remainder, fewer entries than warps,
+    chunk counts that are no multiple of a block's eight, the most chunks it takes and one more."""
+    test_inverse_index_single_launch_equals_radix_sort(lcm, shape)
+
+
 def test_host_pipeline_matches_direct_calls(lcm):
     """HostGcaPipeline (upload / kernels / download of consecutive steps overlapped on three
     streams) returns, step by step and in order, the bits of the plain calls."""
