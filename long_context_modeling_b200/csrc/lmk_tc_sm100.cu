@@ -28,11 +28,13 @@ namespace {
 
 using namespace sm100;
 
-constexpr int BM = 128, BN = 64, BK = 64, STAGES = 4;
+constexpr int BM = 128, BN = 64, BK = 64, STAGES = 7;
 constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int WORKERS = 16, THREADS = (WORKERS + 2) * 32, NORM_WARPS = (BM + BN) / 32;
-constexpr int LDS_ROW = BN + 1;
-constexpr int OFF_SCORE = STAGES * STAGE_BYTES, OFF_NORM = OFF_SCORE + BM * LDS_ROW * 4, OFF_BAR = OFF_NORM + (BM + BN) * 4;
+constexpr int COLS = 16;                          // score columns per worker thread
+constexpr int OFF_X1 = STAGES * STAGE_BYTES;      // [2 tiles][2 pairs of column groups][COLS][BM] keys
+constexpr int OFF_X2 = OFF_X1 + 4 * COLS * BM * 4, OFF_NORM = OFF_X2 + 32 * BM * 4, OFF_BAR = OFF_NORM + 2 * (BM + BN) * 4;
+static_assert(OFF_BAR + 256 + 1024 <= 227 * 1024, "shared memory");
 constexpr int SMEM_BYTES = OFF_BAR + 256 + 1024;
 constexpr int EXTRA = 4, MAX_LISTS = 32;
 constexpr float BOUND = 1.0f / 32768.0f;
@@ -46,15 +48,53 @@ struct ScreenParams {
   float* eps;                    // (rows, lists)
   long long q_pos0, e_base;
   int Cq, E, D, KC, lists, tiles_per_list;
+  int noise_vec;                 // the noise can be read as float4
   float scale;
 };
 
+// Sorting networks on a thread's own registers, descending; every index is a constant.
+template <class T>
+__device__ __forceinline__ void order(T& hi, T& lo) {
+  const T a = hi, b = lo;
+  hi = a > b ? a : b;
+  lo = a > b ? b : a;
+}
+template <int LO, int N, int R, class T>
+__device__ __forceinline__ void odd_even_merge(T* v) {
+  if constexpr (2 * R < N) {
+    odd_even_merge<LO, N, 2 * R>(v);
+    odd_even_merge<LO + R, N, 2 * R>(v);
+#pragma unroll
+    for (int i = LO + R; i + R < LO + N; i += 2 * R) order(v[i], v[i + R]);
+  } else {
+    order(v[LO], v[LO + R]);
+  }
+}
+template <int LO, int N, class T>
+__device__ __forceinline__ void odd_even_sort(T* v) {      // Batcher's odd-even merge sort: 63 exchanges for 16 keys
+  if constexpr (N > 1) {
+    odd_even_sort<LO, N / 2>(v);
+    odd_even_sort<LO + N / 2, N / 2>(v);
+    odd_even_merge<LO, N, 1>(v);
+  }
+}
+template <int N, class T>
+__device__ __forceinline__ void bitonic_merge(T* v) {      // v: a descending run followed by an ascending one
+#pragma unroll
+  for (int d = N / 2; d > 0; d /= 2)
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      if (!(i & d)) order(v[i], v[i + d]);
+}
+
+template <int LEN>                // entries a thread keeps: KC <= LEN
 __global__ void __launch_bounds__(THREADS, 1)
 lmk_screen_kernel(const __grid_constant__ ScreenParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  float* score = reinterpret_cast<float*>(smem + OFF_SCORE);
-  float* norm = reinterpret_cast<float*>(smem + OFF_NORM);
+  unsigned* x1 = reinterpret_cast<unsigned*>(smem + OFF_X1);
+  unsigned* x2 = reinterpret_cast<unsigned*>(smem + OFF_X2);
+  float* norms = reinterpret_cast<float*>(smem + OFF_NORM);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + NUM_BARS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + NUM_BARS + 1);
@@ -119,37 +159,71 @@ lmk_screen_kernel(const __grid_constant__ ScreenParams p) {
   } else {
     bool ok = true;
     uint32_t it = 0, tile = 0;
-    float eps_max = 0.f;                                     // of this warp's rows: row i of the warp in lane i
+    // thread: one row of the tile, COLS of its columns
+    const int quad = warp & 3, group = warp >> 2, r = quad * 32 + lane, row = t0 + r, c0 = group * COLS;
+    const bool live = r < rows;
+    const long long grow = (long long)n * p.Cq + row;
+    float eps_max = 0.f;                                     // of the row (group 0)
+    unsigned long long* dst = p.part + (grow * p.lists + list) * p.KC;
     for (int t = first; t < last && ok; ++t, ++tile) {
+      float* norm = norms + (tile & 1) * (BM + BN);
       if (warp < NORM_WARPS) {
-        float ss = 0.f;
+        float ss[4] = {0.f, 0.f, 0.f, 0.f};
         for (int ks = 0; ks < ksteps && ok; ++ks, ++it) {
           const uint32_t st = it % STAGES;
           ok = mbar_wait_warp(&bars[FULL + st], (it / STAGES) & 1, abort_flag, lane);
           if (!ok) break;
-          const uint8_t* row = smem + st * STAGE_BYTES + threadIdx.x * 128;        // A rows, then B rows right behind them
+          const uint8_t* src = smem + st * STAGE_BYTES + threadIdx.x * 128;        // A rows, then B rows right behind them
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
             float f[8];
-            unpack8(*reinterpret_cast<const uint4*>(row + ((c ^ (lane & 7)) << 4)), f);
+            unpack8(*reinterpret_cast<const uint4*>(src + ((c ^ (lane & 7)) << 4)), f);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) ss = fmaf(f[i], f[i], ss);
+            for (int i = 0; i < 8; ++i) ss[i & 3] = fmaf(f[i], f[i], ss[i & 3]);
           }
           mbar_arrive_warp(&bars[EMPTY + st], lane);
         }
-        norm[threadIdx.x] = ss;
+        norm[threadIdx.x] = (ss[0] + ss[1]) + (ss[2] + ss[3]);
+      }
+      // the row's noise while the products are being formed; columns the row cannot see become key 0
+      const long long e0 = (long long)t * BN + c0;
+      const int see = live ? (int)max(0ll, min((long long)COLS, min((long long)p.E - e0, p.q_pos0 + row - p.e_base - e0))) : 0;
+      float add[COLS];
+#pragma unroll
+      for (int i = 0; i < COLS; ++i) add[i] = 0.f;
+      if (p.noise) {
+        const float* src = p.noise + grow * p.E + e0;
+        if (p.noise_vec) {
+#pragma unroll
+          for (int i = 0; i < COLS; i += 4)
+            if (i < see) {                                   // whole groups of four lie inside the row or outside
+              const float4 v = *reinterpret_cast<const float4*>(src + i);
+              add[i] = v.x; add[i + 1] = v.y; add[i + 2] = v.z; add[i + 3] = v.w;
+            }
+        } else {
+#pragma unroll
+          for (int i = 0; i < COLS; ++i)
+            if (i < see) add[i] = src[i];
+        }
       }
       if (ok) ok = mbar_wait_warp(&bars[ACC_FULL], tile & 1, abort_flag, lane);
+      unsigned key[LEN];
       if (ok) {
         tc_fence_after();
-        const int quad = warp & 3, c0 = (warp >> 2) * 16, r = quad * 32 + lane;
-        uint32_t v[16];
+        uint32_t v[COLS];
         tmem_ld_32x32b_x16(tmem + ((uint32_t)(quad * 32) << 16) + c0, v);
         tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 16; ++i) score[r * LDS_ROW + c0 + i] = __uint_as_float(v[i]) * p.scale;
         tc_fence_before();
         mbar_arrive_warp(&bars[ACC_EMPTY], lane);
+        // key: the score without its last six bits, then the column, lower columns above; never equal inside a tile
+#pragma unroll
+        for (int i = 0; i < COLS; ++i)
+          key[i] = i < see ? (orderable(__uint_as_float(v[i]) * p.scale + add[i]) & ~63u) | (unsigned)(BN - 1 - c0 - i) : 0u;
+        odd_even_sort<0, COLS>(key);
+        if (group & 1) {
+#pragma unroll
+          for (int i = 0; i < COLS; ++i) x1[(((tile & 1) * 2 + (group >> 1)) * COLS + i) * BM + r] = key[i];
+        }
       }
       // one decision for all workers: whether any of them gave up
       int failed = !ok || *abort_flag;
@@ -162,61 +236,54 @@ lmk_screen_kernel(const __grid_constant__ ScreenParams p) {
           : "r"(WORKERS * 32)
           : "memory");
       if (failed) { ok = false; break; }
+      if (group & 1) continue;
+      // two sorted runs of 16 -> the LEN best, sorted
+#pragma unroll
+      for (int i = 0; i < COLS; ++i) {
+        const unsigned o = x1[(((tile & 1) * 2 + (group >> 1)) * COLS + COLS - 1 - i) * BM + r];
+        if (LEN == COLS) key[i] = max(key[i], o);
+        else key[LEN - COLS + i] = o;
+      }
+      bitonic_merge<LEN>(key);
+      if (group == 2) {
+#pragma unroll
+        for (int i = 0; i < LEN; ++i) x2[i * BM + r] = key[i];
+      }
+      asm volatile("bar.sync 2, %0;" ::"r"(WORKERS * 16) : "memory");
+      if (group == 2) continue;
+#pragma unroll
+      for (int i = 0; i < LEN; ++i) key[i] = max(key[i], x2[(LEN - 1 - i) * BM + r]);
+      bitonic_merge<LEN>(key);
       const float kn = fmaxf(norm[BM + lane], norm[BM + 32 + lane]);
       const float kmax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(kn)));     // squared norms: never negative
-      // two rows of the warp at a time: a round is a chain of dependent warp-wide operations
-      for (int i = 0; i < BM / WORKERS; i += 2) {
-        if (warp + i * WORKERS >= rows) break;
-        unsigned o0[2], o1[2];
-        unsigned long long run[2], mine[2] = {0ull, 0ull};
-        unsigned long long* dst[2];
-        bool live[2];
+      if (live) {
+        eps_max = fmaxf(eps_max, BOUND * p.scale * sqrtf(norm[r]) * sqrtf(kmax) * 1.001f);
+        auto entry = [&](unsigned k) {
+          return k ? (unsigned long long)(k & ~63u) << 32 | (0xffffffffu - (unsigned)(p.e_base + t * BN + (BN - 1) - (int)(k & 63u))) : 0ull;
+        };
+        if (t == first) {
 #pragma unroll
-        for (int x = 0; x < 2; ++x) {
-          const int lr = warp + (i + x) * WORKERS, row = t0 + lr;
-          const long long grow = (long long)n * p.Cq + row;
-          live[x] = lr < rows;
-          if (lane == i + x && live[x]) eps_max = fmaxf(eps_max, BOUND * p.scale * sqrtf(norm[lr]) * sqrtf(kmax) * 1.001f);
-          float s0 = score[lr * LDS_ROW + lane], s1 = score[lr * LDS_ROW + 32 + lane];
-          const int e0 = t * BN + lane, e1 = e0 + 32;
-          const bool v0 = live[x] && e0 < p.E && p.e_base + e0 < p.q_pos0 + row, v1 = live[x] && e1 < p.E && p.e_base + e1 < p.q_pos0 + row;
-          if (p.noise) {
-            if (v0) s0 += p.noise[grow * p.E + e0];
-            if (v1) s1 += p.noise[grow * p.E + e1];
+          for (int i = 0; i < LEN; ++i)
+            if (i < p.KC) dst[i] = entry(key[i]);
+        } else {                                                 // with the list so far (this thread wrote it)
+          unsigned long long run[LEN];
+#pragma unroll
+          for (int i = 0; i < LEN; ++i) {
+            const unsigned long long o = i < p.KC ? dst[i] : 0ull, e = entry(key[LEN - 1 - i]);
+            run[i] = o > e ? o : e;
           }
-          o0[x] = v0 ? orderable(s0) : 0u;
-          o1[x] = v1 ? orderable(s1) : 0u;
-          dst[x] = p.part + (grow * p.lists + list) * p.KC;
-          run[x] = live[x] && t > first && lane < p.KC ? dst[x][lane] : 0ull;         // the list so far (this warp wrote it)
-        }
-#pragma unroll 1
-        for (int k = 0; k < p.KC; ++k) {
+          bitonic_merge<LEN>(run);
 #pragma unroll
-          for (int x = 0; x < 2; ++x) {
-            const unsigned rh = (unsigned)(run[x] >> 32);
-            const unsigned m = __reduce_max_sync(0xffffffffu, max(rh, max(o0[x], o1[x])));
-            const unsigned br = __ballot_sync(0xffffffffu, rh == m), b0 = __ballot_sync(0xffffffffu, o0[x] == m),
-                           b1 = __ballot_sync(0xffffffffu, o1[x] == m);
-            // equal scores: the lower id first, so the list's own entries, then the tile's two halves
-            const unsigned from = br ? br : b0 ? b0 : b1;
-            const int src = __ffs(from) - 1;
-            unsigned long long best = __shfl_sync(0xffffffffu, run[x], src);
-            if (!br) best = ((unsigned long long)m << 32) | (0xffffffffu - (unsigned)(p.e_base + t * BN + src + (b0 ? 0 : 32)));
-            if (lane == src) { if (br) run[x] = 0ull; else if (b0) o0[x] = 0u; else o1[x] = 0u; }
-            if (lane == k) mine[x] = m ? best : 0ull;
-          }
+          for (int i = 0; i < LEN; ++i)
+            if (i < p.KC) dst[i] = run[i];
         }
-        __syncwarp();
-#pragma unroll
-        for (int x = 0; x < 2; ++x)
-          if (live[x] && lane < p.KC) dst[x][lane] = mine[x];
       }
-      asm volatile("bar.sync 1, %0;" ::"r"(WORKERS * 32) : "memory");     // scores and norms are free for the next tile
+      __syncwarp();
     }
-    for (int lr = warp, i = 0; lr < rows; lr += WORKERS, ++i) {
-      const long long at = ((long long)n * p.Cq + t0 + lr) * p.lists + list;
-      if (lane == i) p.eps[at] = ok ? eps_max : INFINITY;      // a wait ran out: the merge scans the row itself
-      if (last <= first && lane < p.KC) p.part[at * p.KC + lane] = 0ull;
+    if (group == 0 && live) {
+      p.eps[grow * p.lists + list] = ok ? eps_max : INFINITY;      // a wait ran out: the merge scans the row itself
+      if (last <= first)
+        for (int i = 0; i < p.KC; ++i) dst[i] = 0ull;
     }
   }
   tc_fence_before();
@@ -269,7 +336,7 @@ lmk_settle_kernel(const __grid_constant__ SettleParams p) {
     const unsigned long long best = ((unsigned long long)hi << 32) | lo;
     if (lane == (count & 31)) { if (count < 32) c0 = best; else c1 = best; }
     ++count;
-    if (count == f.K) line = s - 2.0f * eps - fabsf(s) * 4.8e-7f;           // 2^-21: the roundings of scale and noise
+    if (count == f.K) line = s - 2.001f * eps - fabsf(s) * 8.2e-6f;         // 2^-17: the bits a key leaves out; roundings of scale and noise
     bool spent = false;
     if (head == best) { head = next; ++at; next = at < p.KC ? src[at] : 0ull; spent = at > p.KC; }
     slow = __any_sync(0xffffffffu, spent);                                   // a full list used up: it may hide more
@@ -391,8 +458,10 @@ int launch_lmk_screen(const LmkTopkArgs& a, void* scratch, int sms, const FinalP
   p.eps = reinterpret_cast<float*>(static_cast<char*>(scratch) + align_up(rows * p.lists * p.KC * 8, 256));
   p.noise = a.noise; p.q_pos0 = a.q_pos0; p.e_base = a.e_base;
   p.Cq = a.Cq; p.E = a.E; p.D = a.D; p.scale = fin.scale;
-  GCA_CUDA_CHECK(cudaFuncSetAttribute(lmk_screen_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-  GCA_CUDA_CHECK(launch_dependent(lmk_screen_kernel, dim3((unsigned)p.lists, (unsigned)((a.Cq + BM - 1) / BM), (unsigned)a.N), dim3(THREADS), SMEM_BYTES,
+  p.noise_vec = a.E % 4 == 0 && (reinterpret_cast<uintptr_t>(a.noise) & 15u) == 0;
+  auto screen = p.KC <= 16 ? lmk_screen_kernel<16> : lmk_screen_kernel<32>;
+  GCA_CUDA_CHECK(cudaFuncSetAttribute(screen, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+  GCA_CUDA_CHECK(launch_dependent(screen, dim3((unsigned)p.lists, (unsigned)((a.Cq + BM - 1) / BM), (unsigned)a.N), dim3(THREADS), SMEM_BYTES,
                                   stream, p));
   SettleParams sp;
   sp.fin = fin; sp.part = p.part; sp.eps = p.eps; sp.noise = a.noise; sp.q_pos0 = a.q_pos0; sp.KC = p.KC; sp.lists = p.lists; sp.E = a.E;

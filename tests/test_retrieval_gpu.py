@@ -349,6 +349,12 @@ def test_tensor_core_screening_bit_exact_vs_canonical_oracle(lcm, n, cq, e, d, k
     check(res, oracle_rows(lq, lk, k, q_pos0=q_pos0, noise=noise))
 
 
+@pytest.mark.parametrize("e,k,noisy", [(2101, 28, True), (4200, 12, False), (2240, 13, True)])
+def test_tensor_core_screening_merges_tiles(lcm, e, k, noisy):
+    """Several tiles per candidate list, lists of up to 16 and of up to 32 entries, noise rows aligned to 16 bytes and not."""
+    test_tensor_core_screening_bit_exact_vs_canonical_oracle(lcm, 1, 66, e, 64, k, noisy)
+
+
 @pytest.mark.parametrize("copies", [2, 40, 200])
 def test_tensor_core_screening_with_copies_of_landmarks(lcm, copies):
     """Ties that the candidate lists cannot hold (copies of one landmark) and near ties: the exact scan takes over, ties go to
