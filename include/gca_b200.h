@@ -449,6 +449,31 @@ typedef struct LinearBatchedArgs {
 
 int gca_linear_batched(const LinearBatchedArgs* args, void* stream);
 
+/* The GCA sub-layer of a decode step for a few sequences as one launch (model/DRT.py:345-394):
+ *   out[n, s] = residual[n, s] + Wo attention(rmsnorm(x[n, s]) Wq^T, the chunks in indices[n]) .
+ * x and out (N, S, H * 64) contiguous, Wq (with the norm's gain) and Wo (H * 64, H * 64) by row strides, caches bf16 with
+ * chunks of 64 rows (strides n, c, l, h), indices and weights (N, K).  N up to what runs at a time (7), S 1 or 2, H 4, 8, 12 or 16,
+ * H * K up to 192; anything else is GCA_ERR_ALGO, nothing having been launched: run the three steps. */
+typedef struct LayerDecodeArgs {
+  const void* x;
+  const void* wq;
+  const void* wo;
+  const void* k_cache;
+  const void* v_cache;
+  const int32_t* indices;
+  const float* weights;
+  const void* residual;       /* may be NULL */
+  void* out;
+  int32_t* status;            /* may be NULL */
+  int64_t wq_stride, wo_stride, residual_batch_stride, residual_stride;
+  int64_t k_stride[4];
+  int64_t v_stride[4];
+  int32_t N, S, H, Hkv, K, C;
+  float eps, sm_scale;
+} LayerDecodeArgs;
+
+int gca_layer_decode(const LayerDecodeArgs* args, void* stream);
+
 /* out[m, c] = silu(gate_up[m, c]) * gate_up[m, I + c] for c < I: the activation between ONE gate|up
  * projection (weights stacked) and down_proj -- the reference's fused SwiGLU, model/llama.py:290-300.
  * bf16; gate_up (M, 2 I) and out (M, I) by row strides in elements (multiples of 8); I % 8 == 0. */
@@ -556,7 +581,7 @@ const char* gca_strerror(int code);
 int gca_abi_version(void);
 /* sizeof() of an argument block as the library was compiled (0 GcaFwdArgs, 1 GcaBwdArgs,
  * 2 LmkTopkArgs, 3 LmkMergeArgs, 4 CacheAppendArgs, 5 LmkExchangeArgs, 6 KvProjectArgs, 7 RowRmsArgs, 8 LinearArgs, 9 WindowDecodeArgs, 10 LinearCeArgs, 11 WindowAppendArgs, 12 WindowRingDecodeArgs,
- * 13 LinearBatchedArgs, 14 LmkGradArgs): lets a foreign-language binding verify
+ * 13 LinearBatchedArgs, 14 LmkGradArgs, 15 LayerDecodeArgs): lets a foreign-language binding verify
  * its struct layout before the first call. */
 size_t gca_sizeof(int which);
 

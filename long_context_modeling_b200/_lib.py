@@ -74,6 +74,17 @@ class LmkGradArgs(C.Structure):
     ]
 
 
+class LayerDecodeArgs(C.Structure):
+    _fields_ = [
+        ("x", C.c_void_p), ("wq", C.c_void_p), ("wo", C.c_void_p), ("k_cache", C.c_void_p), ("v_cache", C.c_void_p),
+        ("indices", C.c_void_p), ("weights", C.c_void_p), ("residual", C.c_void_p), ("out", C.c_void_p), ("status", C.c_void_p),
+        ("wq_stride", C.c_int64), ("wo_stride", C.c_int64), ("residual_batch_stride", C.c_int64), ("residual_stride", C.c_int64),
+        ("k_stride", C.c_int64 * 4), ("v_stride", C.c_int64 * 4),
+        ("N", C.c_int32), ("S", C.c_int32), ("H", C.c_int32), ("Hkv", C.c_int32), ("K", C.c_int32), ("C", C.c_int32),
+        ("eps", C.c_float), ("sm_scale", C.c_float),
+    ]
+
+
 class LmkMergeArgs(C.Structure):
     _fields_ = [
         ("keys", C.c_void_p), ("out_keys", C.c_void_p), ("out_indices", C.c_void_p),
@@ -169,6 +180,7 @@ EXPORTS = {
     "lmk_topk_workspace_bytes": (C.c_size_t, [C.POINTER(LmkTopkArgs)]),
     "lmk_score_topk_static": (C.c_int, [C.POINTER(LmkTopkArgs), C.c_void_p]),
     "lmk_weights_backward": (C.c_int, [C.POINTER(LmkGradArgs), C.c_void_p]),
+    "gca_layer_decode": (C.c_int, [C.POINTER(LayerDecodeArgs), C.c_void_p]),
     "lmk_topk_merge": (C.c_int, [C.POINTER(LmkMergeArgs), C.c_void_p]),
     "gca_cache_append": (C.c_int, [C.POINTER(CacheAppendArgs), C.c_void_p]),
     "gca_kv_project_append": (C.c_int, [C.POINTER(KvProjectArgs), C.c_void_p]),
@@ -218,7 +230,7 @@ def lib() -> C.CDLL:
             raise RuntimeError("libgca_b200.so has an unexpected ABI version")
         for which, struct in enumerate((GcaFwdArgs, GcaBwdArgs, LmkTopkArgs, LmkMergeArgs, CacheAppendArgs, LmkExchangeArgs,
                                        KvProjectArgs, RowRmsArgs, LinearArgs, WindowDecodeArgs, LinearCeArgs, WindowAppendArgs,
-                                       WindowRingDecodeArgs, LinearBatchedArgs, LmkGradArgs)):
+                                       WindowRingDecodeArgs, LinearBatchedArgs, LmkGradArgs, LayerDecodeArgs)):
             if handle.gca_sizeof(which) != C.sizeof(struct):
                 raise RuntimeError(f"struct layout mismatch for {struct.__name__}: "
                                    f"library {handle.gca_sizeof(which)} vs binding {C.sizeof(struct)}")

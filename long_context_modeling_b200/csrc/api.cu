@@ -17,6 +17,7 @@ int launch_kv_project_append(const KvProjectArgs& a, int sms, cudaStream_t strea
 int launch_row_rms(const RowRmsArgs& a, cudaStream_t stream);
 int launch_silu_mul(const void* gu, void* out, long long M, int I, long long in_stride, long long out_stride, cudaStream_t stream);
 int launch_linear(const LinearBatchedArgs& a, int sms, cudaStream_t stream);
+int launch_layer_decode(const LayerDecodeArgs& a, cudaStream_t stream);
 int launch_window_decode(const WindowDecodeArgs& a, cudaStream_t stream);
 int launch_window_ring_decode(const WindowRingDecodeArgs& a, cudaStream_t stream);
 int launch_linear_ce(const LinearCeArgs& a, int sms, cudaStream_t stream);
@@ -128,6 +129,7 @@ size_t gca_sizeof(int which) {
     case 12: return sizeof(WindowRingDecodeArgs);
     case 13: return sizeof(LinearBatchedArgs);
     case 14: return sizeof(LmkGradArgs);
+    case 15: return sizeof(LayerDecodeArgs);
     default: return 0;
   }
 }
@@ -289,6 +291,20 @@ int lmk_score_topk(const LmkTopkArgs* a, void* stream) {
   const size_t need = gca::lmk_topk_workspace_bytes_impl(*a, sms);
   if (a->workspace_bytes < need) return GCA_ERR_WORKSPACE;
   return gca::launch_lmk_score_topk(*a, a->workspace, sms, (cudaStream_t)stream);
+}
+
+int gca_layer_decode(const LayerDecodeArgs* a, void* stream) {
+  if (!a) return GCA_ERR_NULL;
+  if (!a->x || !a->wq || !a->wo || !a->k_cache || !a->v_cache || !a->indices || !a->weights || !a->out) return GCA_ERR_NULL;
+  if (a->N < 0 || a->S < 1 || a->H < 1 || a->Hkv < 1 || a->H % a->Hkv || a->K < 1 || a->C < 0) return GCA_ERR_SHAPE;
+  if (a->wq_stride % 8 || a->wo_stride % 8) return GCA_ERR_STRIDE;
+  for (int i = 0; i < 4; ++i)
+    if (a->k_stride[i] % 8 || a->v_stride[i] % 8) return GCA_ERR_STRIDE;
+  if (!aligned16(a->x) || !aligned16(a->wq) || !aligned16(a->wo) || !aligned16(a->k_cache) || !aligned16(a->v_cache)) return GCA_ERR_ALIGN;
+  if (a->N == 0) return 0;
+  gca::DeviceScope scope(a->x);
+  if (scope.rc) return scope.rc;
+  return gca::launch_layer_decode(*a, (cudaStream_t)stream);
 }
 
 int lmk_weights_backward(const LmkGradArgs* a, void* stream) {

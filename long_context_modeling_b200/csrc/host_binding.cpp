@@ -44,7 +44,7 @@ struct Api {
 #define GCA_API_LIST                                                                                          \
   GCA_API(gca_fwd) GCA_API(gca_decode) GCA_API(gca_bwd_stages) GCA_API(gca_bwd_workspace_bytes)               \
   GCA_API(lmk_score_topk) GCA_API(lmk_topk_workspace_bytes) GCA_API(lmk_weights_backward) GCA_API(gca_kv_project_append) GCA_API(gca_row_rms) \
-  GCA_API(gca_linear) GCA_API(gca_linear_batched) GCA_API(gca_silu_mul) GCA_API(gca_window_decode)            \
+  GCA_API(gca_linear) GCA_API(gca_linear_batched) GCA_API(gca_layer_decode) GCA_API(gca_silu_mul) GCA_API(gca_window_decode)            \
   GCA_API(gca_window_ring_decode) GCA_API(gca_strerror)
   GCA_API_LIST
 #undef GCA_API
@@ -495,6 +495,41 @@ Tensor layer_fused(const Tensor& hidden_in, const Tensor& q_weight, double eps, 
   }
   const int64_t skip = chunks > 1 && !first_chunk_retrieves ? 1 : 0, J = chunks - skip, rows = J * s;
   const Tensor idx = as_int32(idx_in), w = as_float(w_in);
+  Problem p;
+  int64_t kd[4], vd[4];
+  cache_view(k, head_dim, kd, p.ks);
+  cache_view(v, head_dim, vd, p.vs);
+  for (int i = 0; i < 4; ++i) TORCH_CHECK_VALUE(kd[i] == vd[i], "k_cache and v_cache must have the same shape");
+  TORCH_CHECK_VALUE(k.scalar_type() == at::kBFloat16 && v.scalar_type() == at::kBFloat16, "q, k_cache and v_cache must share one dtype");
+  TORCH_CHECK_VALUE(idx.dim() == 3 && idx.size(0) == n && idx.size(1) == J && w.sizes() == idx.sizes() && kd[0] == n,
+                    "indices/weights must be (N, J, K) = (", n, ", ", J, ", K); got ", idx.sizes(), ", ", w.sizes());
+  TORCH_CHECK_VALUE(kd[3] > 0 && heads % kd[3] == 0, "number of q heads must be a multiple of the number of kv heads");
+  p.N = n; p.J = J; p.Hq = heads; p.S = s; p.D = head_dim; p.C = kd[1]; p.L = kd[2]; p.Hkv = kd[3]; p.K = idx.size(2);
+  // a decode step of a few sequences is one launch
+  if (chunks == 1 && skip == 0 && s <= 2 && head_dim == 64 && dim == heads * 64 && p.L == 64 && q_weight.size(0) == dim && o_weight.size(0) == dim) {
+    LayerDecodeArgs d;
+    d.x = hidden.const_data_ptr(); d.wq = q_weight.const_data_ptr(); d.wo = o_weight.const_data_ptr();
+    d.k_cache = k.const_data_ptr(); d.v_cache = v.const_data_ptr(); d.indices = idx.const_data_ptr<int32_t>(); d.weights = w.const_data_ptr<float>();
+    d.residual = nullptr; d.residual_batch_stride = d.residual_stride = 0;
+    if (residual.defined()) {
+      d.residual = residual.const_data_ptr(); d.residual_batch_stride = residual.stride(0); d.residual_stride = residual.stride(1);
+    }
+    d.out = out.mutable_data_ptr(); d.status = status_ptr(on.dev);
+    d.wq_stride = q_weight.stride(0); d.wo_stride = o_weight.stride(0);
+    copy4(d.k_stride, p.ks); copy4(d.v_stride, p.vs);
+    d.N = (int32_t)n; d.S = (int32_t)s; d.H = (int32_t)heads; d.Hkv = (int32_t)p.Hkv; d.K = (int32_t)p.K; d.C = (int32_t)p.C;
+    d.eps = (float)eps; d.sm_scale = (float)sm_scale;
+    bool done = true;
+    call("gca_layer_decode", [&] {
+      const int rc = api.gca_layer_decode(&d, on.stream);
+      done = rc != GCA_ERR_ALGO;
+      return done ? rc : 0;
+    });
+    if (done) {
+      maybe_check(on.dev);
+      return out;
+    }
+  }
   const bool few = n * rows <= GCA_SKINNY_ROWS && skip == 0;             // the norm rides on the projection
   const Tensor q = at::empty({2, n, J, s, dim}, hidden.options());      // [0]: q, [1]: the attention's output
   void* const vals = static_cast<char*>(q.mutable_data_ptr()) + q.stride(0) * 2;
@@ -517,16 +552,6 @@ Tensor layer_fused(const Tensor& hidden_in, const Tensor& q_weight, double eps, 
   lp.batches = (int32_t)n; lp.x_batch_stride = chunks * s * dim; lp.out_batch_stride = rows * dim; lp.scale_batch_stride = chunks * s;
   call("gca_linear", [&] { return api.gca_linear_batched(&lp, on.stream); });
   // q as (n, J, heads, s, head_dim) by strides
-  Problem p;
-  int64_t kd[4], vd[4];
-  cache_view(k, head_dim, kd, p.ks);
-  cache_view(v, head_dim, vd, p.vs);
-  for (int i = 0; i < 4; ++i) TORCH_CHECK_VALUE(kd[i] == vd[i], "k_cache and v_cache must have the same shape");
-  TORCH_CHECK_VALUE(k.scalar_type() == at::kBFloat16 && v.scalar_type() == at::kBFloat16, "q, k_cache and v_cache must share one dtype");
-  TORCH_CHECK_VALUE(idx.dim() == 3 && idx.size(0) == n && idx.size(1) == J && w.sizes() == idx.sizes() && kd[0] == n,
-                    "indices/weights must be (N, J, K) = (", n, ", ", J, ", K); got ", idx.sizes(), ", ", w.sizes());
-  TORCH_CHECK_VALUE(kd[3] > 0 && heads % kd[3] == 0, "number of q heads must be a multiple of the number of kv heads");
-  p.N = n; p.J = J; p.Hq = heads; p.S = s; p.D = head_dim; p.C = kd[1]; p.L = kd[2]; p.Hkv = kd[3]; p.K = idx.size(2);
   p.qs[0] = rows * dim; p.qs[1] = s * dim; p.qs[2] = head_dim; p.qs[3] = dim;
   GcaFwdArgs f = fwd_args(p, q, k, v, idx, w, q, p.qs, nullptr, sm_scale, 0.0, GCA_ALGO_AUTO, on.dev);
   f.out = vals;

@@ -140,6 +140,34 @@ def test_fused_module_path_matches_reference_class(golden_dir):
         close(o1, g["triton_decode_o"], "decode")
 
 
+@pytest.mark.parametrize("n,heads,rows,k,chunks", [(1, 12, 1, 8, 64), (3, 4, 2, 1, 5), (7, 8, 1, 5, 9), (2, 16, 2, 12, 40), (1, 12, 2, 16, 30),
+                                                   (5, 16, 1, 3, 7), (9, 12, 1, 8, 20), (1, 16, 1, 13, 20)])
+def test_one_launch_decode_step(n, heads, rows, k, chunks):
+    """The whole sub-layer of a decode step as one launch -- (head, slot) tiles that do not divide evenly among the cluster's CTAs,
+    padding slots, a sequence without any, with and without residual -- against the unfused path; the last two are outside its
+    range and take the three launches."""
+    need_gpu()
+    import long_context_modeling_b200 as lcm
+    g = torch.Generator().manual_seed(7)
+    dim = heads * 64
+    mod = lcm.TritonGroupCrossAttention(dim, heads, chunk_topk=k).to("cuda", torch.bfloat16).eval()
+    hs = torch.randn(n, 1, rows, dim, generator=g).bfloat16().cuda()
+    kc, vc = (torch.randn(n, chunks, 64, dim, generator=g).bfloat16().cuda() for _ in range(2))
+    idx = torch.stack([torch.randperm(max(chunks, k), generator=g)[:k] for _ in range(n)]).view(n, 1, k).to(torch.int32)
+    idx[idx >= chunks] = -1
+    idx[0, 0, k // 2:] = -1
+    if n > 2:
+        idx[2] = -1
+    w = torch.softmax(torch.randn(n, 1, k, generator=g), -1).masked_fill(idx < 0, 0.0).cuda()
+    idx = idx.cuda()
+    res = torch.randn(n, rows, dim, generator=g).bfloat16().cuda()
+    with torch.no_grad():
+        want = mod.forward_indexed(hs, kc, vc, idx, w).float()
+        close(mod.forward_fused(hs, kc, vc, idx, w), want, "no residual")
+        close(mod.forward_fused(hs, kc, vc, idx, w, residual=res), want + res.float(), "with residual")
+    assert lcm.read_status() == 0
+
+
 def _window_reference(q, k, v, window, slopes, scale):
     """float32: explicit scores, ALiBi bias, window + causal mask, softmax (model/llama.py:684-688 semantics)."""
     n, hq, sq, d = q.shape
