@@ -256,6 +256,18 @@ decode_rows_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
   const int rows = g.G * g.S;                                    // <= R
   const float c2 = g.sm_scale * GCA_LOG2E;
   pdl_trigger();
+  // While the kernel before is finishing, this warp's first K tile on its way into L2 (V as well, which fills the queues the
+  // loads behind the wait need: no gain left).  The index may not be final yet, so it is a hint here, read past L1 and read
+  // again below.
+  if (warp < g.K) {
+    int hint = warp;
+    if (indices) asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(hint) : "l"(indices + (long long)zj * g.K + warp) : "memory");
+    if (hint >= 0 && hint < g.C) {
+      const __nv_bfloat16* kt = kc + n * g.ks[0] + hint * g.ks[1] + hk * g.ks[3] + lane * g.ks[2];
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(kt));
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(kt + 32 * g.ks[2]));
+    }
+  }
   pdl_wait();
   float qv[R][8];
 #pragma unroll
@@ -280,8 +292,8 @@ decode_rows_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
     if (idx < 0) continue;                                       // padding slot (warp-uniform)
     if (idx >= g.C) { if (status && lane == 0) atomicOr(status, GCA_STATUS_BAD_INDEX); continue; }
     const float w = weights[(long long)zj * g.K + k];
-    const __nv_bfloat16* kb = kc + n * g.ks[0] + idx * g.ks[1] + hk * g.ks[3] + sub * 8;
-    const __nv_bfloat16* vb = vc + n * g.vs[0] + idx * g.vs[1] + hk * g.vs[3] + sub * 8;
+    const __nv_bfloat16* kb = kc + n * g.ks[0] + idx * g.ks[1] + hk * g.ks[3] + sub * 8 + grp * g.ks[2];
+    const __nv_bfloat16* vb = vc + n * g.vs[0] + idx * g.vs[1] + hk * g.vs[3] + sub * 8 + grp * g.vs[2];
     RowState st[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
@@ -289,42 +301,55 @@ decode_rows_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
 #pragma unroll
       for (int e = 0; e < 8; ++e) st[r].acc[e] = 0.f;
     }
-    // 16 steps of 4 keys; the loads run four steps ahead of the arithmetic in registers
+    // 16 steps of 4 keys, four steps at a time: the next four steps' rows are requested as soon as the registers are read, and
+    // the four steps share one maximum and one rescaling (a step of its own each was a chain of ~200 cycles)
     uint4 kq[4], vq[4];
 #pragma unroll
     for (int s = 0; s < 4; ++s) {
-      kq[s] = *reinterpret_cast<const uint4*>(kb + (s * 4 + grp) * g.ks[2]);
-      vq[s] = *reinterpret_cast<const uint4*>(vb + (s * 4 + grp) * g.vs[2]);
+      kq[s] = *reinterpret_cast<const uint4*>(kb); kb += 4 * g.ks[2];
+      vq[s] = *reinterpret_cast<const uint4*>(vb); vb += 4 * g.vs[2];
     }
 #pragma unroll 1
     for (int b4 = 0; b4 < 16; b4 += 4) {
+      float sc[R][4];
 #pragma unroll
       for (int s = 0; s < 4; ++s) {
-        const uint4 kcur = kq[s], vcur = vq[s];
-        if (b4 + 4 < 16) {
-          const int key = (b4 + 4 + s) * 4 + grp;
-          kq[s] = *reinterpret_cast<const uint4*>(kb + key * g.ks[2]);
-          vq[s] = *reinterpret_cast<const uint4*>(vb + key * g.vs[2]);
-        }
-        const unsigned kw[4] = {kcur.x, kcur.y, kcur.z, kcur.w}, vw[4] = {vcur.x, vcur.y, vcur.z, vcur.w};
-        float kf[8], vf[8];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) { kf[2 * e] = bf_lo(kw[e]); kf[2 * e + 1] = bf_hi(kw[e]); vf[2 * e] = bf_lo(vw[e]); vf[2 * e + 1] = bf_hi(vw[e]); }
+        const unsigned kw[4] = {kq[s].x, kq[s].y, kq[s].z, kq[s].w};
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-          float sc = 0.f;
+          float t = 0.f;
 #pragma unroll
-          for (int e = 0; e < 8; ++e) sc = fmaf(qv[r][e], kf[e], sc);
-          sc += __shfl_xor_sync(0xffffffffu, sc, 1);
-          sc += __shfl_xor_sync(0xffffffffu, sc, 2);
-          sc += __shfl_xor_sync(0xffffffffu, sc, 4);
-          const float m = fmaxf(st[r].m, sc);
-          const float corr = ex2f(st[r].m - m), pr = ex2f(sc - m);
-          st[r].l = st[r].l * corr + pr;
-#pragma unroll
-          for (int e = 0; e < 8; ++e) st[r].acc[e] = fmaf(pr, vf[e], st[r].acc[e] * corr);
-          st[r].m = m;
+          for (int e = 0; e < 4; ++e) { t = fmaf(qv[r][2 * e], bf_lo(kw[e]), t); t = fmaf(qv[r][2 * e + 1], bf_hi(kw[e]), t); }
+          sc[r][s] = t;
         }
+        if (b4 + 4 < 16) { kq[s] = *reinterpret_cast<const uint4*>(kb); kb += 4 * g.ks[2]; }
+      }
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+#pragma unroll
+        for (int of = 1; of < 8; of <<= 1)
+#pragma unroll
+          for (int s = 0; s < 4; ++s) sc[r][s] += __shfl_xor_sync(0xffffffffu, sc[r][s], of);
+        const float m = fmaxf(st[r].m, fmaxf(fmaxf(sc[r][0], sc[r][1]), fmaxf(sc[r][2], sc[r][3])));
+        const float corr = ex2f(st[r].m - m);
+        st[r].m = m;
+#pragma unroll
+        for (int s = 0; s < 4; ++s) sc[r][s] = ex2f(sc[r][s] - m);
+        st[r].l = st[r].l * corr + ((sc[r][0] + sc[r][1]) + (sc[r][2] + sc[r][3]));
+#pragma unroll
+        for (int e = 0; e < 8; ++e) st[r].acc[e] *= corr;
+      }
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        const unsigned vw[4] = {vq[s].x, vq[s].y, vq[s].z, vq[s].w};
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            st[r].acc[2 * e] = fmaf(sc[r][s], bf_lo(vw[e]), st[r].acc[2 * e]);
+            st[r].acc[2 * e + 1] = fmaf(sc[r][s], bf_hi(vw[e]), st[r].acc[2 * e + 1]);
+          }
+        if (b4 + 4 < 16) { vq[s] = *reinterpret_cast<const uint4*>(vb); vb += 4 * g.vs[2]; }
       }
     }
 #pragma unroll
