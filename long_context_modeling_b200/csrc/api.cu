@@ -235,7 +235,7 @@ int gca_bwd_stages(const GcaBwdArgs* a, unsigned stages, void* stream) {
   if (scope.rc) return scope.rc;
   gca::Csr csr;
   size_t used = 0;
-  rc = gca::build_csr(a->indices, a->N, a->J, a->K, a->C, a->workspace, a->workspace_bytes, &csr, &used, s,
+  rc = gca::build_csr(a->indices, a->N, a->J, a->K, a->C, a->workspace, a->workspace_bytes, gca::units_by_count(*a), &csr, &used, s,
                       (stages & GCA_BWD_STAGE_INDEX) != 0, (stages & GCA_BWD_INDEX_BY_SORT) != 0);
   if (rc) return rc;
   if (!(stages & (GCA_BWD_STAGE_KV | GCA_BWD_STAGE_Q))) return 0;

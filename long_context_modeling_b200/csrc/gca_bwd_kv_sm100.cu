@@ -38,6 +38,11 @@
 // every NBUF-th iteration), one TMA producer (Q, dO and the per-row term tiles of every
 // iteration; K, V per unit) and the MMA issuers (S^T, dP^T, dV, dK).  Every wait is bounded
 // (GCA_STATUS_TIMEOUT on expiry).
+//
+// Units go to CTAs on demand, in the order of the unit table: a warp draws tickets and publishes the units to the other roles.  A
+// chunk near the start of a sequence has many times the retrievers of one near its end; dealt out in turn, the busiest CTA
+// had 4 % more than the average at 8 x 256 chunks, K = 8, 7 % at 1,024, K = 16, 50 % at 2 x 64.  Which CTA has a unit does
+// not show in its result.
 #include "gca_common.cuh"
 #include "sm100_ptx.cuh"
 #include "tc_common.cuh"
@@ -80,7 +85,8 @@ static_assert(NBUF == 2 || NBUF == 3, "score buffers");
 #define GCA_KV_PREPROBE 0
 #endif
 constexpr int PROD_WARP = 4 * NG, ISSUE_S = PROD_WARP + 1, ISSUE_DP = ISSUE_S + 1, ISSUE_DV = ISSUE_DP + 1;       // dK issuer (GRAD2): ISSUE_DV + 1
-constexpr int NTHREADS = (ISSUE_DV + GRAD_ISSUERS) * 32;
+constexpr int SCHED_WARP = ISSUE_DV + GRAD_ISSUERS;
+constexpr int NTHREADS = (SCHED_WARP + 1) * 32;
 constexpr int WCOLS = 64 / SPLIT;                        // query columns of a key row that one group handles
 constexpr int TMEM_COLS = 512;
 constexpr uint32_t LANE16 = 16u << 16;            // TMEM lane offset of head B's 64-row tile
@@ -101,13 +107,16 @@ constexpr int OFF_RT = OFF_QDO + NQ * 2 * PAIR_BYTES;        // [NQ][head A tile
 constexpr int OFF_ONES_S = OFF_RT + NQ * 2 * RT_BYTES;       // 64 rows x (1 1 1 0 0 0 0 0): picks a0 + a1 + a2
 constexpr int OFF_ONES_DP = OFF_ONES_S + RT_BYTES;           // 64 rows x (0 0 0 1 1 1 0 0): picks b0 + b1 + b2
 constexpr int OFF_ZERO = OFF_ONES_DP + RT_BYTES;             // 64 rows x 16 bytes of zeros
+constexpr int ND = 8, AHEAD = 8;                             // units published ahead, until they have AHEAD iterations
 constexpr int OFF_W = OFF_ZERO + RT_BYTES;                   // [NQ] retrieval weight of the iteration (its sign is used)
-constexpr int OFF_BAR = OFF_W + 64;
+constexpr int OFF_UNIT = OFF_W + 64;                         // [ND] published units: first entry, one past the last (-1: no more work), chunk, head pair
+constexpr int OFF_BAR = OFF_UNIT + ND * 16;
 constexpr int SMEM_BYTES = OFF_BAR + 512 + 1024;
 static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
 enum Bar { KV_FULL = 0, KV_EMPTY = KV_FULL + NKV, QDO_FULL = KV_EMPTY + NKV, QDO_EMPTY = QDO_FULL + NQ,
            SP_FULL = QDO_EMPTY + NQ, PDS_FULL = SP_FULL + NBUF, BUF_FREE = PDS_FULL + NBUF, ACC_FULL = BUF_FREE + NBUF,
-           ACC_EMPTY = ACC_FULL + NBUF, NUM_BARS = ACC_EMPTY + 1 };
+           ACC_EMPTY = ACC_FULL + NBUF, UNIT_FULL = ACC_EMPTY + 1, UNIT_EMPTY = UNIT_FULL + ND, NUM_BARS = UNIT_EMPTY + ND };
+constexpr int UNIT_READERS = 4 * NG + 3 + GRAD_ISSUERS;        // warps
 static_assert(NUM_BARS * 8 + 16 <= 512, "barrier block");
 // Tensor-memory columns.  Buffer b (iteration g uses b = g % NBUF) = 128 columns: S^T at +0 and
 // dP^T at +64 as float32; afterwards |w| P^T at +0 and |w| dS^T at +64 as packed bf16 (32 columns
@@ -137,6 +146,7 @@ struct BwdKvParams {
   const uint4* rowterm;     // (N*J, Hq, K) tiles of 64 x 16 bytes, written by the q-major pass
   const int4* unit_tab;     // units in walking order: (first entry, one past the last, chunk id n*C + c)
   const unsigned long long* sorted_keys;
+  int* tickets;             // [units handed out beyond the first of every CTA, CTAs done]
   __nv_bfloat16* dk;
   __nv_bfloat16* dv;
   int32_t* status;
@@ -144,6 +154,8 @@ struct BwdKvParams {
   long long dks[4], dvs[4];
   int units;
   int N, J, Hq, Hkv, G, K, C, HP;
+  int div;                  // unit u: chunk u / div of the table, head pair u % div; heads_outside: pair u / div, chunk u % div
+  bool heads_outside, in_turn;
   int wide_store;           // dk / dv rows are 32-byte aligned: 256-bit stores
   float c2, sm_scale;
   const float4* dw_part;    // (N*J, Hq, K): the q-major pass's four partials of every (head, slot) of dw, or nullptr
@@ -168,21 +180,62 @@ __device__ __forceinline__ void reduce_dw(const BwdKvParams& p) {
   }
 }
 
+// One lane: draws tickets and publishes units ahead of the roles -- not too many, a unit that waits here is one that a free CTA could have taken,
+// but enough iterations for the copies in flight.  A warp of its own: the producer, whose copies bound the kernel, lost ~600
+// cycles per unit to the two dependent trips to L2.  It naps between its probes, which otherwise crowd the shared-memory path
+// of the MMAs' operands (682 against 658 us at 8 x 256 chunks).
+__device__ void kv_scheduler(const BwdKvParams& p, uint8_t* smem, uint64_t* bars, volatile int* abort_flag) {
+  int4* slots = reinterpret_cast<int4*>(smem + OFF_UNIT);
+  uint32_t head = 0, tail = 0;               // units published, units that all roles have read
+  int ahead = 0;                             // iterations between the two
+  for (int u = blockIdx.x;; u = p.in_turn ? u + (int)gridDim.x : (int)gridDim.x + atomicAdd(p.tickets, 1)) {
+    int4 unit = make_int4(0, -1, 0, 0);
+    if (u < p.units) {
+      const int q = u / p.div, r = u - q * p.div;
+      unit = p.unit_tab[p.heads_outside ? r : q];
+      unit.w = p.heads_outside ? q : r;
+    }
+    slots[head % ND] = unit;
+    mbar_arrive(&bars[UNIT_FULL + head % ND]);
+    if (u >= p.units) break;
+    ++head;
+    ahead += (unit.y - unit.x) * p.G;
+    while (head - tail == ND || ahead >= AHEAD) {
+      for (int i = 0; !mbar_test_wait(&bars[UNIT_EMPTY + tail % ND], (tail / ND) & 1); ++i) {
+        if (i >= (1 << 21)) *abort_flag = 1;
+        if (*abort_flag) return;
+        __nanosleep(400);
+      }
+      ahead -= (slots[tail % ND].y - slots[tail % ND].x) * p.G;
+      ++tail;
+    }
+  }
+}
+// The next published unit (y < 0: no more work), read by a whole warp.
+__device__ __forceinline__ bool next_unit(uint8_t* smem, uint64_t* bars, Ring& ur, int4& unit, volatile int* abort_flag, int lane) {
+  if (!mbar_wait_warp(&bars[UNIT_FULL + ur.st], ur.ph, abort_flag, lane)) return false;
+  unit = reinterpret_cast<const int4*>(smem + OFF_UNIT)[ur.st];
+  mbar_arrive_warp(&bars[UNIT_EMPTY + ur.st], lane);
+  ur.next();
+  return true;
+}
+
 // One lane: K + V per unit; per iteration Q + dO, the two heads' row-term tiles and the weight.
 __device__ void kv_producer(const BwdKvParams& p, uint8_t* smem, uint64_t* bars, volatile int* abort_flag) {
-  PairCursor c;
-  c.init(p.HP);
-  Ring ring; ring.init(NQ);
+  Ring ring, ur; ring.init(NQ); ur.init(ND);
   uint32_t ucnt = 0, issued = 0;
   bool ok = true;
   float* sw = reinterpret_cast<float*>(smem + OFF_W);
-  int4 nxt = c.u < p.units ? p.unit_tab[c.outer] : make_int4(0, 0, 0, 0);
-  for (; c.u < p.units && ok; c.advance()) {
-    const int beg = nxt.x, end = nxt.y, chunk = nxt.z;
-    if (c.u + (int)gridDim.x < p.units) nxt = p.unit_tab[c.next_outer()];
+  while (ok) {
+    ok = mbar_wait_bounded(&bars[UNIT_FULL + ur.st], ur.ph, abort_flag);
+    if (!ok) break;
+    const int4 unit = reinterpret_cast<const int4*>(smem + OFF_UNIT)[ur.st];
+    mbar_arrive(&bars[UNIT_EMPTY + ur.st]);
+    ur.next();
+    const int beg = unit.x, end = unit.y, chunk = unit.z, hk0 = 2 * unit.w;
+    if (end < 0) break;
     if (end == beg) continue;
     const uint32_t un = ucnt++;
-    const int hk0 = 2 * c.inner;
     const bool two = hk0 + 1 < p.Hkv;
     const int n = chunk / p.C, ch = chunk - n * p.C;
     {
@@ -252,16 +305,14 @@ __device__ void kv_issuer(const BwdKvParams& p, uint8_t* smem, uint64_t* bars, v
   const uint32_t ones_addr = smem_u32(smem + (ROLE == 0 ? OFF_ONES_S : OFF_ONES_DP));
   const uint64_t dOnes = umma_desc_nosw_k(ones_addr, zero_addr - ones_addr, 128);
   const float* sw = reinterpret_cast<const float*>(smem + OFF_W);
-  PairCursor c;
-  c.init(p.HP);
-  Ring ring; ring.init(NQ);
+  Ring ring, ur; ring.init(NQ); ur.init(ND);
   uint32_t ucnt = 0, g = 0;
   uint32_t b = 0, bph = 0;                                // g % NBUF and the parity of g / NBUF
   bool ok = true;
-  int4 nxt = c.u < p.units ? p.unit_tab[c.outer] : make_int4(0, 0, 0, 0);
-  for (; c.u < p.units && ok; c.advance()) {
-    const int beg = nxt.x, end = nxt.y;
-    if (c.u + (int)gridDim.x < p.units) nxt = p.unit_tab[c.next_outer()];
+  int4 unit;
+  while (ok && (ok = next_unit(smem, bars, ur, unit, abort_flag, lane))) {
+    const int beg = unit.x, end = unit.y;
+    if (end < 0) break;
     const int niter = (end - beg) * p.G;
     if (niter == 0) continue;
     const uint32_t un = ucnt++;
@@ -382,20 +433,18 @@ __device__ void kv_worker(const BwdKvParams& p, uint8_t* smem, uint64_t* bars, v
   const int row = quad * 16 + (lane & 15);
   const uint32_t tlane = tmem_base + ((uint32_t)(quad * 32) << 16);
   const bool elected = quad == 0 && lane == 0;
-  PairCursor c;
-  c.init(p.HP);
-  Ring ring; ring.init(NQ);
+  Ring ring, ur; ring.init(NQ); ur.init(ND);
   uint32_t ucnt = 0, g = 0;
   bool ok = true;
   uint32_t epi = 0;                             // units this group has helped to write out
   uint32_t b = 0, bph = 0;                      // g % NBUF and the parity of g / NBUF
   const int my_buf = wg / SPLIT, part = wg % SPLIT;
-  int4 nxt = c.u < p.units ? p.unit_tab[c.outer] : make_int4(0, 0, 0, 0);
-  for (; c.u < p.units && ok; c.advance()) {
-    const int beg = nxt.x, end = nxt.y, chunk = nxt.z;
-    if (c.u + (int)gridDim.x < p.units) nxt = p.unit_tab[c.next_outer()];
+  int4 unit;
+  while (ok && (ok = next_unit(smem, bars, ur, unit, abort_flag, lane))) {
+    const int beg = unit.x, end = unit.y, chunk = unit.z;
+    if (end < 0) break;
     if (end == beg) {                           // nobody retrieved this chunk: zero gradient
-      const int hk = 2 * c.inner + tile;
+      const int hk = 2 * unit.w + tile;
       if (wg == 0 && hk < p.Hkv) {
         const int n = chunk / p.C, ch = chunk - n * p.C;
         __nv_bfloat16* dk_row = p.dk + n * p.dks[0] + ch * p.dks[1] + row * p.dks[2] + hk * p.dks[3];
@@ -457,7 +506,7 @@ __device__ void kv_worker(const BwdKvParams& p, uint8_t* smem, uint64_t* bars, v
       if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
       if (elected && part == 0) GCA_TRACE_BUF(p.prof, 10, un);
       tc_fence_after();
-      const int hk = 2 * c.inner + tile;
+      const int hk = 2 * unit.w + tile;
       const bool live = hk < p.Hkv;
       const int n = chunk / p.C, ch = chunk - n * p.C;
       __nv_bfloat16* dk_row = p.dk + n * p.dks[0] + ch * p.dks[1] + row * p.dks[2] + hk * p.dks[3];
@@ -502,6 +551,7 @@ bwd_kv_tc_kernel(const __grid_constant__ BwdKvParams p) {
       mbar_init(&bars[ACC_FULL + i], GRAD_ISSUERS);
     }
     mbar_init(&bars[ACC_EMPTY], 128 * SPLIT);
+    for (int i = 0; i < ND; ++i) { mbar_init(&bars[UNIT_FULL + i], 1); mbar_init(&bars[UNIT_EMPTY + i], UNIT_READERS); }
     for (int i = 0; i < NKV; ++i) { mbar_init(&bars[KV_FULL + i], 1); mbar_init(&bars[KV_EMPTY + i], 1); }
     for (int i = 0; i < NQ; ++i) { mbar_init(&bars[QDO_FULL + i], 1); mbar_init(&bars[QDO_EMPTY + i], GRAD_ISSUERS); }
     *abort_flag = 0;
@@ -526,6 +576,7 @@ bwd_kv_tc_kernel(const __grid_constant__ BwdKvParams p) {
     reduce_dw(p);                        // while the first tiles are on their way
     kv_worker(p, smem, bars, abort_flag, warp >> 2, warp & 3, lane, tmem_base);
   } else if (warp == PROD_WARP) { if (lane == 0) kv_producer(p, smem, bars, abort_flag); }
+  else if (warp == SCHED_WARP) { if (lane == 0) kv_scheduler(p, smem, bars, abort_flag); }
   else if (warp == ISSUE_S) kv_issuer<0>(p, smem, bars, abort_flag, lane, tmem_base);
   else if (warp == ISSUE_DP) kv_issuer<1>(p, smem, bars, abort_flag, lane, tmem_base);
   else if (warp == ISSUE_DV) kv_issuer<2>(p, smem, bars, abort_flag, lane, tmem_base);
@@ -533,7 +584,13 @@ bwd_kv_tc_kernel(const __grid_constant__ BwdKvParams p) {
   tc_fence_before();
   __syncthreads();
   if (warp == ISSUE_S) tmem_dealloc(tmem_base, TMEM_COLS);
-  if (threadIdx.x == 0 && *abort_flag && p.status) atomicOr(p.status, GCA_STATUS_TIMEOUT);
+  if (threadIdx.x == 0) {
+    if (*abort_flag && p.status) atomicOr(p.status, GCA_STATUS_TIMEOUT);
+    if (atomicAdd(p.tickets + 1, 1) == (int)gridDim.x - 1) {       // the last CTA leaves the counters as it found them
+      p.tickets[0] = 0;
+      p.tickets[1] = 0;
+    }
+  }
 }
 
 // every 64-element bf16 row of the tensor starts on a 32-byte boundary
@@ -561,12 +618,20 @@ int launch_bwd_kv_tc(const GcaBwdArgs& a, const Csr& csr, const uint4* rowterm, 
       (rc = qmap(&p.tm_q1, a.q, a.q_stride, 1)) || (rc = qmap(&p.tm_do1, a.dout, a.do_stride, 1)) ||
       (rc = kmap(&p.tm_k2, a.k_cache, a.k_stride, 2)) || (rc = kmap(&p.tm_v2, a.v_cache, a.v_stride, 2)))
     return rc;
-  p.weights = a.weights; p.rowterm = rowterm; p.unit_tab = csr.unit_tab; p.sorted_keys = csr.sorted_keys;
+  p.weights = a.weights; p.rowterm = rowterm; p.unit_tab = csr.unit_tab; p.sorted_keys = csr.sorted_keys; p.tickets = csr.tickets;
   p.dk = (__nv_bfloat16*)a.dk_cache; p.dv = (__nv_bfloat16*)a.dv_cache; p.status = a.status;
   p.prof = profile_buffer();
   for (int i = 0; i < 4; ++i) { p.dks[i] = a.dk_stride[i]; p.dvs[i] = a.dv_stride[i]; }
   p.N = a.N; p.J = a.J; p.Hq = a.Hq; p.Hkv = a.Hkv; p.G = a.Hq / a.Hkv; p.K = a.K; p.C = a.C;
   p.HP = (a.Hkv + 1) / 2;
+  // A chunk's head pairs side by side, but for one long sequence whose Q and dO do not fit into L2 (126 MB): there one head pair
+  // after the other, which reads those of a pair only (1,024 chunks, 12 heads: 620 -> 590 us; where they do fit it costs 5 %).
+  p.heads_outside = a.N == 1 && (long long)a.J * a.Hq * PAIR_BYTES > (126ll << 20);
+  p.div = p.heads_outside ? a.C : p.HP;
+  // From eight sequences on, one after the other, units are dealt out in turn all the same.  CTAs that draw reach the end of a sequence
+  // together, where its units are short and the next one's tiles are not in L2 yet; dealt out they drift apart (8 x 256
+  // chunks: 628 against 664 us, 8 x 100: 187 against 195; 5 x 300: 420 against 393).
+  p.in_turn = a.N >= 8 && !units_by_count(a);
   const long long units = (long long)a.N * a.C * p.HP;
   if (units >= (1ll << 31) - 65536) return GCA_ERR_TOO_LARGE;
   p.units = (int)units;

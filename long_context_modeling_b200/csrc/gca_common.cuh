@@ -78,22 +78,23 @@ struct Geom {
 
 // Inverse retrieval index: for every cache chunk (n, c) the list of (j*K + k) entries that retrieved it, in order: the low
 // 32 bits of `sorted_keys`.
-// `unit_tab` lists the chunks in the order the kv-major kernels walk them: sequence
-// by sequence, and inside a sequence by DECREASING number of retrievers (x = first entry,
-// y = one past the last, z = chunk id n*C + c).  CTAs take units round-robin, so every CTA gets
-// chunks of every size class; in chunk order the busiest CTA had 8 % more work than the average
-// (chunks near the start of a sequence are retrieved by many more queries than late ones).
+// `unit_tab` lists the chunks in the order the kv-major kernels take them: by DECREASING number of
+// retrievers, sequence by sequence or of all sequences (units_by_count); x = first entry,
+// y = one past the last, z = chunk id n*C + c.
+// `tickets`: two counters, zero between launches: units handed out by the tensor-core kv-major kernel, CTAs that are done.
 // `overlaps`: the kernel that builds it was just launched and lets the next kernel on the stream start before it is done.
 struct Csr {
   const unsigned long long* sorted_keys;
   const int4* unit_tab;
+  int* tickets;
   bool overlaps;
 };
 
 // launch == false: only lay the index out in `workspace` (it was built by an earlier call)
+// by_count: the unit table's order (units_by_count)
 // by_sort: take the radix-sort path even where the single-launch path would do (same bits)
 int build_csr(const int32_t* indices, int N, int J, int K, int C, void* workspace, size_t workspace_bytes,
-              Csr* out, size_t* used_bytes, cudaStream_t stream, bool launch = true, bool by_sort = false);
+              bool by_count, Csr* out, size_t* used_bytes, cudaStream_t stream, bool launch = true, bool by_sort = false);
 size_t csr_workspace_bytes(int N, int J, int K, int C);
 
 // SIMT (CUDA-core, fp32 accumulate) kernels: every dtype, S <= 64, L = D = 64.
@@ -110,6 +111,13 @@ int launch_bwd_tc(const GcaBwdArgs& a, const Csr& csr, float* dw_part, uint4* ro
 // dw[zj, k] = sum over heads and `parts` partials of dw_part[zj, h, k, part], in a fixed order
 int launch_dw_reduce(const float* dw_part, float* dw, int ZJ, int Hq, int K, int parts, cudaStream_t stream);
 int bwd_tc_dw_parts();   // partials per (row block, head, slot) that the tensor-core q-major pass writes
+
+// Order of the kv-major kernels' units, the rows of the unit table.  A chunk near the start of a sequence has many times the retrievers of one near its end, so
+// the large units have to start first; over ALL sequences when what they read, Q and dO, stays in L2 whatever the order
+// (half of its 126 MB), else one sequence after the other, which reads each sequence's Q and dO from memory once.
+inline bool units_by_count(const GcaBwdArgs& a) {
+  return (long long)a.N * a.J * a.Hq * a.S * a.D * 2 * (a.dtype == GCA_F32 ? 4 : 2) <= (64ll << 20);
+}
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 

@@ -39,19 +39,20 @@ __device__ __forceinline__ long long csr_lower_bound(const unsigned long long* _
 }
 
 // offsets[c] = first sorted key of chunk c (or the end).  The same thread also emits the chunk's
-// entry of the kv-major walking order: key = sequence << cbits | (cmax - count), so that an
-// ascending sort lists a sequence's chunks by decreasing number of retrievers; value =
+// entry of the kv-major walking order: key = sequence (by_count: 0) << cbits | (cmax - count), so that an
+// ascending sort lists a sequence's (all) chunks by decreasing number of retrievers; value =
 // (first entry, one past the last, chunk id): what the kv-major kernel reads per unit.
-__global__ void csr_offsets_kernel(const unsigned long long* __restrict__ sorted, int* __restrict__ offsets,
+__global__ void csr_offsets_kernel(const unsigned long long* __restrict__ sorted, int* __restrict__ offsets, int* __restrict__ tickets,
                                    unsigned* __restrict__ ukeys, int4* __restrict__ uvals,
-                                   long long total, long long NC, int C, int cbits, unsigned cmax) {
+                                   long long total, long long NC, int C, int cbits, unsigned cmax, bool by_count) {
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (c > NC) return;
+  if (c < 2) tickets[c] = 0;
   const long long lo = csr_lower_bound(sorted, total, (unsigned long long)c << 32);
   offsets[c] = (int)lo;
   if (c == NC) return;
   const unsigned cnt = (unsigned)(csr_lower_bound(sorted, total, (unsigned long long)(c + 1) << 32) - lo);
-  ukeys[c] = ((unsigned)(c / C) << cbits) | (cmax - (cnt < cmax ? cnt : cmax));
+  ukeys[c] = (by_count ? 0u : (unsigned)(c / C) << cbits) | (cmax - (cnt < cmax ? cnt : cmax));
   uvals[c] = make_int4((int)lo, (int)lo + (int)cnt, (int)c, 0);
 }
 
@@ -71,7 +72,8 @@ __global__ void csr_offsets_kernel(const unsigned long long* __restrict__ sorted
 constexpr int LIST_WARPS = 8, LIST_MAX_C = 2048, LIST_LOADS = 16;
 
 __global__ void __launch_bounds__(LIST_WARPS * 32)
-csr_list_kernel(const int32_t* __restrict__ indices, unsigned long long* __restrict__ keys_out, int4* __restrict__ unit_tab, int JK, int C) {
+csr_list_kernel(const int32_t* __restrict__ indices, unsigned long long* __restrict__ keys_out, int4* __restrict__ unit_tab, int* __restrict__ tickets,
+                int JK, int C, bool by_count) {
   __shared__ int cnt[LIST_MAX_C];
   __shared__ int sect[LIST_WARPS][LIST_WARPS];       // [section][chunk of this block]: entries, then the first one's place
   const int n = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -80,6 +82,7 @@ csr_list_kernel(const int32_t* __restrict__ indices, unsigned long long* __restr
   if (threadIdx.x < LIST_WARPS * LIST_WARPS) (&sect[0][0])[threadIdx.x] = 0;
   pdl_wait();
   pdl_trigger();                         // everything before this kernel is complete: the next one may start
+  if (blockIdx.x == 0 && n == 0 && threadIdx.x < 2) tickets[threadIdx.x] = 0;
   __syncthreads();
   const int c0 = blockIdx.x * LIST_WARPS, c1 = min(c0 + LIST_WARPS, C);
   const int per = ((JK + LIST_WARPS * 32 - 1) / (LIST_WARPS * 32)) * 32, first = warp * per, last = min(first + per, JK);
@@ -110,7 +113,7 @@ csr_list_kernel(const int32_t* __restrict__ indices, unsigned long long* __restr
     }
     start += n * JK;
     if (lane == 0) {
-      unit_tab[(long long)n * C + rank] = make_int4(start, start + mine, n * C + c, 0);
+      unit_tab[by_count ? (long long)rank * gridDim.y + n : (long long)n * C + rank] = make_int4(start, start + mine, n * C + c, 0);
       for (int w = 0; w < LIST_WARPS; ++w) {
         const int here = sect[w][warp];
         sect[w][warp] = start;
@@ -143,10 +146,11 @@ bool small_path(int N, int JK, int C) {
 }
 
 // The pre-gathered call: chunk c of row block n is read by its slot c and nothing else.
-__global__ void csr_identity_kernel(unsigned long long* __restrict__ keys_out, int4* __restrict__ unit_tab, int NC, int C) {
+__global__ void csr_identity_kernel(unsigned long long* __restrict__ keys_out, int4* __restrict__ unit_tab, int* __restrict__ tickets, int NC, int C) {
   pdl_wait();
   pdl_trigger();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < 2) tickets[i] = 0;
   if (i >= NC) return;
   keys_out[i] = ((unsigned long long)i << 32) | (unsigned)(i % C);
   unit_tab[i] = make_int4(i, i + 1, i, 0);
@@ -178,11 +182,11 @@ size_t csr_workspace_bytes(int N, int J, int K, int C) {
   const long long total = (long long)N * J * K;
   const long long NC = (long long)N * C;
   return align_up(total * 8, 256) * 2 + align_up((NC + 1) * 4, 256) + align_up(cub_temp_bytes(total), 256) +
-         align_up(NC * 4, 256) * 2 + align_up(NC * 16, 256) * 2 + align_up(cub_pairs_temp_bytes(NC), 256);
+         align_up(NC * 4, 256) * 2 + align_up(NC * 16, 256) * 2 + align_up(cub_pairs_temp_bytes(NC), 256) + 256;
 }
 
 int build_csr(const int32_t* indices, int N, int J, int K, int C, void* workspace, size_t workspace_bytes,
-              Csr* out, size_t* used_bytes, cudaStream_t stream, bool launch, bool by_sort) {
+              bool by_count, Csr* out, size_t* used_bytes, cudaStream_t stream, bool launch, bool by_sort) {
   const long long total = (long long)N * J * K;
   const long long NC = (long long)N * C;
   if (total >= (1ll << 31) || NC >= (1ll << 31)) return GCA_ERR_TOO_LARGE;
@@ -199,18 +203,19 @@ int build_csr(const int32_t* indices, int N, int J, int K, int C, void* workspac
   int4* uvals_in = (int4*)p;                             p += align_up(NC * 16, 256);
   int4* uvals_out = (int4*)p;                            p += align_up(NC * 16, 256);
   size_t utemp = cub_pairs_temp_bytes(NC);
-  void* utemp_ptr = p;
+  void* utemp_ptr = p;                                   p += align_up(utemp, 256);
+  int* tickets = (int*)p;
   // a chunk has at most J*K retrievers; the unit key holds (J*K - count) below the sequence number
   const long long cmax = (long long)J * K;
   const int cbits = bits_for(cmax), nbits = bits_for(N);
   if (cbits + nbits > 32) return GCA_ERR_TOO_LARGE;
   out->overlaps = false;
   if (launch && !indices && NC > 0) {
-    GCA_CUDA_CHECK(launch_dependent(csr_identity_kernel, dim3((unsigned)((NC + 255) / 256)), dim3(256), 0, stream, keys_out, uvals_out, (int)NC, C));
+    GCA_CUDA_CHECK(launch_dependent(csr_identity_kernel, dim3((unsigned)((NC + 255) / 256)), dim3(256), 0, stream, keys_out, uvals_out, tickets, (int)NC, C));
     out->overlaps = true;
   } else if (launch && NC > 0 && total > 0 && !by_sort && small_path(N, J * K, C)) {
     GCA_CUDA_CHECK(launch_dependent(csr_list_kernel, dim3((unsigned)((C + LIST_WARPS - 1) / LIST_WARPS), (unsigned)N), dim3(LIST_WARPS * 32), 0,
-                                    stream, indices, keys_out, uvals_out, J * K, C));
+                                    stream, indices, keys_out, uvals_out, tickets, J * K, C, by_count));
     out->overlaps = true;
   } else if (launch) {
     if (total > 0) {
@@ -225,8 +230,8 @@ int build_csr(const int32_t* indices, int N, int J, int K, int C, void* workspac
       GCA_CUDA_CHECK(cub::DeviceRadixSort::SortKeys(temp_ptr, temp, keys_in, keys_out, (int)total, 32, end_bit, stream));
     }
     if (NC > 0) {
-      csr_offsets_kernel<<<(unsigned)((NC + 1 + 255) / 256), 256, 0, stream>>>(keys_out, offsets, ukeys_in, uvals_in, total,
-                                                                               NC, C, cbits, (unsigned)cmax);
+      csr_offsets_kernel<<<(unsigned)((NC + 1 + 255) / 256), 256, 0, stream>>>(keys_out, offsets, tickets, ukeys_in, uvals_in, total,
+                                                                               NC, C, cbits, (unsigned)cmax, by_count);
       GCA_CUDA_CHECK(cudaGetLastError());
       GCA_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(utemp_ptr, utemp, ukeys_in, ukeys_out, uvals_in, uvals_out, (int)NC, 0,
                                                      cbits + nbits, stream));
@@ -234,6 +239,7 @@ int build_csr(const int32_t* indices, int N, int J, int K, int C, void* workspac
   }
   out->sorted_keys = keys_out;
   out->unit_tab = uvals_out;
+  out->tickets = tickets;
   *used_bytes = need;
   return 0;
 }

@@ -10,7 +10,8 @@
 // operand of the next product are read by nobody else: blocks synchronise only for the K / V (Q / dO) tiles,
 // which cp.async brings in one step ahead.  The kv-major kernel works on TRANSPOSED scores (rows = keys) for the same
 // reason; what it needs per query row, Di = rowsum(P dP), comes from the q-major kernel.
-// 2 x 64 chunks x 12 heads, top-8, float32: forward 477 -> 371 us, q-major 689 -> 481 us, kv-major 1031 -> 785 us.
+// 2 x 64 chunks x 12 heads, top-8, float32: forward 477 -> 355 us, q-major 689 -> 481 us, kv-major 1031 -> 588 us (785 when its
+// blocks started in table order head by head, the longest units of the last head almost at the end).
 #include "gca_common.cuh"
 
 namespace gca {
@@ -71,7 +72,7 @@ __device__ __forceinline__ void mma_nt(const float* A, const float* B, const Own
     for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
   const float* a0 = A + o.row0 * LD;
   const float* b0 = B + o.tx * LD;
-#pragma unroll 2
+#pragma unroll 4
   for (int d = 0; d < T; d += 4) {
     float4 a[4], b[8];
 #pragma unroll
@@ -92,7 +93,7 @@ __device__ __forceinline__ void mma_nt(const float* A, const float* B, const Own
 __device__ __forceinline__ void mma_nn_acc(const float* A, const float* B, const Own& o, float acc[4][8]) {
   const float* a0 = A + o.row0 * LDP;
   const float* b0 = B + o.tx * 4;
-#pragma unroll 2
+#pragma unroll 4
   for (int r = 0; r < T; r += 4) {
     float4 a[4];
 #pragma unroll
@@ -163,12 +164,12 @@ __device__ __forceinline__ int next_slot(const int32_t* indices, long long zj, c
 // forward
 // ------------------------------------------------------------------------------------
 template <typename E>
-__global__ void __launch_bounds__(NTHREADS, 3)
+__global__ void __launch_bounds__(NTHREADS, 4)
 fwd_simt_kernel(const E* __restrict__ q, const E* __restrict__ kc, const E* __restrict__ vc,
                 const int32_t* __restrict__ indices, const float* __restrict__ weights,
                 E* __restrict__ out, float* __restrict__ lse, int32_t* status, Geom g) {
   extern __shared__ __align__(16) float smem[];
-  float *sQ = smem, *sK = sQ + TILE, *sV = sK + TILE, *sP = sV + TILE;
+  float *sQ = smem, *sV = sQ + TILE, *sK = sV + TILE, *sP = sK;      // P takes K's place: four blocks fit on an SM
   const int zj = blockIdx.x, h = blockIdx.y;
   const int n = zj / g.J, j = zj % g.J, hk = h / g.G;
   const Own own;
@@ -205,8 +206,6 @@ fwd_simt_kernel(const E* __restrict__ q, const E* __restrict__ kc, const E* __re
     float s[4][8];
     mma_nt(sQ, sK, own, s);
     __syncthreads();                           // every warp is done with K
-    if (k_next < g.K) k_tile(idx_next);
-    cp_commit();
     float* lse_row = lse ? lse + (((long long)zj * g.Hq + h) * g.K + k) * g.S : nullptr;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -227,12 +226,16 @@ fwd_simt_kernel(const E* __restrict__ q, const E* __restrict__ kc, const E* __re
       for (int b = 0; b < 8; ++b) s[i][b] *= f;
     }
     put_rows(sP, own, s);
-    cp_wait<1>();                              // V is here, the next K may still be on its way
+    cp_wait<0>();                              // V is here
     __syncthreads();
     mma_nn_acc(sP, sV, own, acc);
-    __syncthreads();                           // every warp is done with V
-    if (k_next < g.K) v_tile(idx_next);
-    cp_commit();
+    __syncthreads();                           // every warp is done with P and V
+    if (k_next < g.K) {
+      k_tile(idx_next);
+      cp_commit();
+      v_tile(idx_next);
+      cp_commit();
+    }
     k = k_next;
     idx = idx_next;
   }
@@ -345,8 +348,9 @@ bwd_kv_simt_kernel(const E* __restrict__ q, const E* __restrict__ kc, const E* _
                    long long dvs0, long long dvs1, long long dvs2, long long dvs3) {
   extern __shared__ __align__(16) float smem[];
   float *sK = smem, *sV = sK + TILE, *sQ = sV + TILE, *sdO = sQ + TILE, *sP = sdO + TILE;
-  const int4 unit = csr.unit_tab[blockIdx.x];         // the chunks with the most retrievers of a sequence first
-  const int nc = unit.z, hk = blockIdx.y;
+  const int hk = blockIdx.x % g.Hkv;
+  const int4 unit = csr.unit_tab[blockIdx.x / g.Hkv];
+  const int nc = unit.z;
   const int n = nc / g.C, c = nc % g.C;
   const Own own;
   const float c2 = g.sm_scale * GCA_LOG2E;
@@ -445,7 +449,7 @@ Geom make_geom(const GcaBwdArgs& a) {
 
 template <typename E>
 int fwd_simt_typed(const GcaFwdArgs& a, cudaStream_t stream) {
-  const size_t smem = (3 * TILE + TILE_P) * sizeof(float);
+  const size_t smem = (2 * TILE + TILE_P) * sizeof(float);
   GCA_CUDA_CHECK(cudaFuncSetAttribute(fwd_simt_kernel<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   dim3 grid((unsigned)(a.N * a.J), (unsigned)a.Hq);
   fwd_simt_kernel<E><<<grid, NTHREADS, smem, stream>>>((const E*)a.q, (const E*)a.k_cache, (const E*)a.v_cache,
@@ -468,7 +472,7 @@ int bwd_simt_typed(const GcaBwdArgs& a, const Csr& csr, float* dw_part, float* r
   }
   if (stages & GCA_BWD_STAGE_KV) {
     GCA_CUDA_CHECK(cudaFuncSetAttribute(bwd_kv_simt_kernel<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const dim3 grid((unsigned)(a.N * a.C), (unsigned)a.Hkv);
+    const unsigned grid = (unsigned)((long long)a.N * a.C * a.Hkv);
     bwd_kv_simt_kernel<E><<<grid, NTHREADS, smem, stream>>>(
         (const E*)a.q, (const E*)a.k_cache, (const E*)a.v_cache, a.weights, (const E*)a.dout, a.lse, row_di,
         (E*)a.dk_cache, (E*)a.dv_cache, csr, g,

@@ -279,6 +279,30 @@ def test_inverse_index_sections_equal_radix_sort(lcm, shape):
     test_inverse_index_single_launch_equals_radix_sort(lcm, shape)
 
 
+@pytest.mark.parametrize("shape", [(1, 820, 10, 2), (2, 420, 10, 2), (9, 100, 5, 3), (3, 5, 1, 2)])
+def test_unit_orders_of_the_kv_major_pass(lcm, shape):
+    """Every order in which the kv-major pass hands out its units -- one long sequence by head pairs, sequence by sequence, in turn from
+    eight sequences on, all sequences by count -- covers every chunk once: dK / dV against the CUDA-core kernels; repeated
+    launches (the ticket counters are back where they were) give the same bits."""
+    from long_context_modeling_b200 import gca as gmod
+    n, c, h, k = shape
+    q, kc, vc, idx, w, dout = (t.cuda() for t in cases.gca_indexed_case(43, n, c, h, k, dtype=torch.bfloat16))
+    _, lse = gmod.gca_forward_with_lse(q, kc, vc, idx, w, 0.125)
+    bufs = gmod.gca_backward_stages(q, kc, vc, idx, w, dout, lse, 0.125, stages=gmod.BWD_STAGE_INDEX | gmod.BWD_STAGE_Q)
+    first = None
+    for _ in range(3):
+        bufs[1].fill_(float("nan"))
+        bufs[2].fill_(float("nan"))
+        gmod.gca_backward_stages(q, kc, vc, idx, w, dout, lse, 0.125, stages=gmod.BWD_STAGE_KV, bufs=bufs)
+        got = [bufs[1].clone(), bufs[2].clone()]
+        first = first or got
+        assert all(torch.equal(x, y) for x, y in zip(got, first))
+    want = gmod.gca_backward_stages(q, kc, vc, idx, w, dout, lse, 0.125, algo=gmod.ALGO_SIMT)[1:3]
+    for x, y in zip(got, want):
+        assert (x.float() - y.float()).abs().max().item() <= 2e-2 * max(1e-3, y.float().abs().max().item())
+    assert lcm.read_status() == 0
+
+
 def test_host_pipeline_matches_direct_calls(lcm):
     """HostGcaPipeline (upload / kernels / download of consecutive steps overlapped on three
     streams) returns, step by step and in order, the bits of the plain calls."""
