@@ -64,19 +64,19 @@ class ChunkKVManager:
     def chunk_k(self) -> Optional[torch.Tensor]:
         if self._grad_mode:
             return self._gk
-        return None if self._k is None else self._k[:, :self._len]
+        return None if self._k is None else self._k.narrow(1, 0, self._len)
 
     @property
     def chunk_v(self) -> Optional[torch.Tensor]:
         if self._grad_mode:
             return self._gv
-        return None if self._v is None else self._v[:, :self._len]
+        return None if self._v is None else self._v.narrow(1, 0, self._len)
 
     @property
     def lmk_embs(self) -> Optional[torch.Tensor]:
         if self._grad_mode:
             return self._glmk
-        return None if self._lmk is None else self._lmk[:, :self._len]
+        return None if self._lmk is None else self._lmk.narrow(1, 0, self._len)
 
     def backed_views(self):
         """(chunk_k, chunk_v) over EVERY chunk slot that has memory behind it, filled or not: a view whose
@@ -165,10 +165,7 @@ class ChunkKVManager:
         if need <= cap:
             return
         new_cap = max(need, 2 * cap, self._capacity_hint, 16)
-        n, _, l, hd = like_k.shape
-        k = torch.empty((n, new_cap, l, hd), dtype=like_k.dtype, device=like_k.device)
-        v = torch.empty_like(k)
-        lmk = torch.empty((n, new_cap, like_lmk.shape[-1]), dtype=like_lmk.dtype, device=like_lmk.device)
+        k, v, lmk = _lib.host().cache_buffers(like_k, like_lmk, new_cap)
         if self._len:
             k[:, :self._len].copy_(self._k[:, :self._len])
             v[:, :self._len].copy_(self._v[:, :self._len])
@@ -231,8 +228,8 @@ class ChunkKVManager:
         if not enc_out.is_cuda:
             raise RuntimeError("ChunkKVManager holds device memory only (there is no CPU path)")
         x = enc_out.contiguous()
-        n, count, l, dim = x.shape
-        self._reserve(self._len + count, x, x[:, :, -1])
+        count = x.shape[1]
+        self._reserve(self._len + count, x, x)                  # landmarks: the last dimension and the type of x
         if self._k.dtype != torch.bfloat16 or self._lmk.dtype != torch.bfloat16:
             raise ValueError("append_projected writes a bf16 cache")
         _lib.host().kv_project_append(x, k_weight, v_weight, self._k, self._v, self._lmk, self._len, self._capacity(), self._zero_landmark)

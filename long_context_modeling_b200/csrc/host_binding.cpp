@@ -26,6 +26,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
 
+#include <array>
 #include <atomic>
 #include <mutex>
 
@@ -808,6 +809,16 @@ void kv_project_append(const Tensor& x, const Tensor& wk, const Tensor& wv, cons
   call("gca_kv_project_append", [&] { return api.gca_kv_project_append(&a, on.stream); });
 }
 
+// K, V (N, capacity, L, HD) like `k` (N, D, L, HD) and landmarks (N, capacity, Dm) like `lmk` (.., Dm).
+std::array<Tensor, 3> cache_buffers(const Tensor& k, const Tensor& lmk, int64_t capacity) {
+  TORCH_CHECK_VALUE(k.dim() == 4 && lmk.dim() > 0, "cache_buffers: expected (N, D, L, HD) and (.., Dm)");
+  at::AutoDispatchBelowADInplaceOrView below;
+  c10::cuda::OptionalCUDAGuard guard;
+  guard.set_index(k.device().index());
+  const int64_t shape[4] = {k.size(0), capacity, k.size(2), k.size(3)}, rows[3] = {k.size(0), capacity, lmk.size(-1)};
+  return {at::empty(shape, k.options()), at::empty(shape, k.options()), at::empty(rows, lmk.options())};
+}
+
 // ------------------------------------------------------------------------------------------- Python glue
 // Positional arguments only; the Python functions in front of these give them their names and defaults.
 struct Args {
@@ -1035,6 +1046,13 @@ ENTRY(kv_project_append, 9)
   Py_RETURN_NONE;
 ENTRY_END
 
+ENTRY(cache_buffers, 3)
+  const Tensor &k = a.tensor(0), &lmk = a.tensor(1);
+  const int64_t capacity = a.integer(2);
+  const auto t = unlocked([&] { return cache_buffers(k, lmk, capacity); });
+  return wrap_tuple({t[0], t[1], t[2]});
+ENTRY_END
+
 ENTRY(status_word, 1)
   const int64_t dev = a.integer(0);
   return wrap(unlocked([&] { return status_word((int)dev); }));
@@ -1068,7 +1086,7 @@ ENTRY_END
 PyMethodDef methods[] = {
     METHOD(bind), METHOD(set_switches), METHOD(status_word), METHOD(gca_indexed), METHOD(attention), METHOD(gca_nograd), METHOD(gca_kv_cache),
     METHOD(gca_forward_lse), METHOD(gca_backward), METHOD(row_rms), METHOD(linear), METHOD(rmsnorm_linear), METHOD(layer_fused), METHOD(silu_mul),
-    METHOD(window_decode), METHOD(window_ring_decode), METHOD(lmk_score_topk), METHOD(retrieve), METHOD(kv_project_append), {nullptr, nullptr, 0, nullptr}};
+    METHOD(window_decode), METHOD(window_ring_decode), METHOD(lmk_score_topk), METHOD(retrieve), METHOD(kv_project_append), METHOD(cache_buffers), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_host", "Host path of the hot entry points.", -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace
