@@ -352,7 +352,7 @@ def gpu_arm(args):
                                  "ceiling_value": flops_step * world / (ms_both * 1e-3) / 1e12,
                                  "e2e_frac_of_ceiling": ms_both / ms_e2e},
                 "host_binding": binding},
-        "gpu_launches": 5 * steps,      # fwd_tc, csr_small, bwd_kv_tc, bwd_q_tc, dw_reduce
+        "gpu_launches": 4 * steps,      # fwd_tc, csr_list, bwd_q_tc, bwd_kv_tc
         "kernels": kernels,
         "roofline": {"kernel": top, "bound": "tensor", "achieved": kernels[top]["achieved_tflops"],
                      "peak": peak, "unit": "TFLOP/s", "frac": kernels[top]["frac_of_peak"],
@@ -603,7 +603,7 @@ def measure_retrieval(dev, world, rank, local, per_head, steps, warmup, peaks, w
             "eager_ms_per_step": ms_eager, "eager_peer_exchange_ms_per_step": ms_p2p_eager,
             "sharded_gca_decode_ms_per_step": ms_gca,      # owner-computes decode over the sharded K/V cache + all-reduce, eager
             "gpu_launches": (2 if world == 1 else 3) * steps,      # scan, finalize (+ exchange-and-merge)
-            "roofline": {"kernel": "lmk_scan_kernel + lmk_finalize_kernel", "bound": "hbm", "achieved": achieved,
+            "roofline": {"kernel": "lmk_stream_kernel + merge", "bound": "hbm", "achieved": achieved,
                          "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": achieved / peaks["hbm_gbs"],
                          "peak_source": peaks["source"] + " copy bandwidth", "traffic": None,
                          "algorithmic_bytes_per_launch": bytes_local, "us_per_launch": ms_scan * 1e3},
@@ -865,7 +865,7 @@ def projection_arm(args):
             "clocks": clocks,
             "e2e": {"value": fl / (ms_e2e * 1e-3) / 1e12, "unit": "TFLOP/s", "h2d_bytes_per_step": x_host.numel() * 2,
                     "d2h_bytes_per_step": n * dim * 2, "ms_per_step": ms_e2e},
-            "gpu_launches": 2 * steps,
+            "gpu_launches": steps,
             "linear_mode": {"rows": m, "gemm_ms": ms_lin, "gemm_tflops": fl / 2 / (ms_lin * 1e-3) / 1e12,
                             "with_residual_ms": ms_res, "rmsnorm_row_scale_ms": ms_rms},
             "roofline": {"kernel": "kv_project_append_kernel", "bound": "tensor", "achieved": tf, "peak": peaks["bf16_tflops"],
