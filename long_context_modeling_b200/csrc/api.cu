@@ -1,8 +1,7 @@
 // extern "C" entry points of libgca_b200.so: argument validation on the host, kernel
 // selection, launches on the caller's stream.  Nothing here allocates device memory.
-#include <mutex>
-
 #include "gca_common.cuh"
+#include "per_device.cuh"
 
 namespace gca {
 int launch_decode(const GcaFwdArgs& a, int sms, cudaStream_t stream);
@@ -17,7 +16,7 @@ int launch_kv_project_append(const KvProjectArgs& a, int sms, cudaStream_t strea
 int launch_row_rms(const RowRmsArgs& a, cudaStream_t stream);
 int launch_silu_mul(const void* gu, void* out, long long M, int I, long long in_stride, long long out_stride, cudaStream_t stream);
 int launch_linear(const LinearBatchedArgs& a, int sms, cudaStream_t stream);
-int launch_layer_decode(const LayerDecodeArgs& a, cudaStream_t stream);
+int launch_layer_decode(const LayerDecodeArgs& a, int dev, cudaStream_t stream);
 int launch_window_decode(const WindowDecodeArgs& a, cudaStream_t stream);
 int launch_window_ring_decode(const WindowRingDecodeArgs& a, cudaStream_t stream);
 int launch_linear_ce(const LinearCeArgs& a, int sms, cudaStream_t stream);
@@ -37,17 +36,12 @@ DeviceScope::~DeviceScope() {
 }
 
 int sm_count(int dev) {
-  constexpr int MAXD = 64;
-  static std::mutex mu;
-  static int cached[MAXD] = {};
-  if (dev < 0 || dev >= MAXD) return 1;
-  std::lock_guard<std::mutex> lock(mu);
-  if (cached[dev] == 0) {
-    int n = 0;
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 1;
-    cached[dev] = n;
-  }
-  return cached[dev];
+  static PerDevice count;
+  int n = 1;
+  const bool known = count.get(dev, &n, [&](int* v) {
+    return cudaDeviceGetAttribute(v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && *v > 0;
+  });
+  return known ? n : 1;
 }
 }  // namespace gca
 
@@ -304,7 +298,7 @@ int gca_layer_decode(const LayerDecodeArgs* a, void* stream) {
   if (a->N == 0) return 0;
   gca::DeviceScope scope(a->x);
   if (scope.rc) return scope.rc;
-  return gca::launch_layer_decode(*a, (cudaStream_t)stream);
+  return gca::launch_layer_decode(*a, scope.dev, (cudaStream_t)stream);
 }
 
 int lmk_weights_backward(const LmkGradArgs* a, void* stream) {

@@ -11,6 +11,7 @@
 // One sequence, 12 heads, K = 8: 13.1 -> 8.4 us per call (8.4 on the device, of which 4.8 are launch, barriers and hand-overs, 8.2 on
 // the host); seven sequences 15 -> 9.
 #include "gca_common.cuh"
+#include "per_device.cuh"
 #include "sm100_ptx.cuh"
 
 namespace gca {
@@ -324,7 +325,7 @@ layer_decode_kernel(const __grid_constant__ LayerParams p) {
 }
 
 template <int HQ, int S>
-int launch(const LayerDecodeArgs& a, const LayerParams& p, cudaStream_t stream) {
+int launch(const LayerDecodeArgs& a, const LayerParams& p, int dev, cudaStream_t stream) {
   auto kernel = layer_decode_kernel<HQ, S>;
   const size_t smem = (size_t)p.units * 2 * TILE;
   cudaLaunchConfig_t cfg = {};
@@ -335,37 +336,40 @@ int launch(const LayerDecodeArgs& a, const LayerParams& p, cudaStream_t stream) 
   attr[1].id = cudaLaunchAttributeClusterDimension;
   attr[1].val.clusterDim.x = CL; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr; cfg.numAttrs = 2;
-  // how many clusters of the largest CTA run at a time (each needs 16 SMs of one GPC): asked once
-  static const int most = [&] {
+  // How many clusters of the largest CTA run at a time (each needs 16 SMs of one GPC), and the two limits raised: a device's own, so
+  // once per device.  If that fails the call takes three launches, and the next one tries again.
+  static PerDevice clusters;
+  int most = 0;
+  const bool known = clusters.get(dev, &most, [&](int* n) {
     cudaLaunchConfig_t largest = cfg;
     largest.dynamicSmemBytes = MAX_UNITS * 2 * TILE;
-    int clusters = 0;
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_UNITS * 2 * TILE) == cudaSuccess &&
-        cudaOccupancyMaxActiveClusters(&clusters, kernel, &largest) == cudaSuccess)
-      return clusters;
+        cudaOccupancyMaxActiveClusters(n, kernel, &largest) == cudaSuccess)
+      return true;
     cudaGetLastError();
-    return 0;
-  }();
-  if (a.N > most) return GCA_ERR_ALGO;
+    return false;
+  });
+  if (!known || a.N > most) return GCA_ERR_ALGO;
   return (int)cudaLaunchKernelEx(&cfg, kernel, p);
 }
 
 template <int S>
-int launch_heads(const LayerDecodeArgs& a, const LayerParams& p, cudaStream_t stream) {
+int launch_heads(const LayerDecodeArgs& a, const LayerParams& p, int dev, cudaStream_t stream) {
   switch (a.H) {
-    case 4: return launch<1, S>(a, p, stream);
-    case 8: return launch<2, S>(a, p, stream);
-    case 12: return launch<3, S>(a, p, stream);
-    default: return launch<4, S>(a, p, stream);
+    case 4: return launch<1, S>(a, p, dev, stream);
+    case 8: return launch<2, S>(a, p, dev, stream);
+    case 12: return launch<3, S>(a, p, dev, stream);
+    default: return launch<4, S>(a, p, dev, stream);
   }
 }
 
 }  // namespace
 
-// As many sequences as clusters run at a time, 7 on a B200 (a second wave takes longer than three launches: 16.9 against 14.4 us), 4, 8, 12 or 16 heads, and no more (head, slot) tiles per CTA than fit into its shared memory; anything
-// else is GCA_ERR_ALGO, before anything has been launched: more sequences fill the chip as three launches.
-int launch_layer_decode(const LayerDecodeArgs& a, cudaStream_t stream) {
+// As many sequences as clusters run at a time, 7 on a B200 (a second wave takes longer than three launches: 16.9 against 14.4 us), 4, 8,
+// 12 or 16 heads, and no more (head, slot) tiles per CTA than fit into its shared memory; anything else is GCA_ERR_ALGO, before
+// anything has been launched: more sequences fill the chip as three launches.  `dev`: the current device.
+int launch_layer_decode(const LayerDecodeArgs& a, int dev, cudaStream_t stream) {
   LayerParams p;
   p.units = (a.H * a.K + CL - 1) / CL;
   if (a.S < 1 || a.S > 2 || a.H % 4 != 0 || a.H < 4 || a.H > 16 || p.units > MAX_UNITS) return GCA_ERR_ALGO;
@@ -375,7 +379,7 @@ int launch_layer_decode(const LayerDecodeArgs& a, cudaStream_t stream) {
   p.wq_stride = a.wq_stride; p.wo_stride = a.wo_stride; p.res_batch = a.residual_batch_stride; p.res_row = a.residual_stride;
   for (int i = 0; i < 4; ++i) { p.ks[i] = a.k_stride[i]; p.vs[i] = a.v_stride[i]; }
   p.H = a.H; p.G = a.H / a.Hkv; p.K = a.K; p.C = a.C; p.eps = a.eps; p.c2 = a.sm_scale * GCA_LOG2E;
-  return a.S == 1 ? launch_heads<1>(a, p, stream) : launch_heads<2>(a, p, stream);
+  return a.S == 1 ? launch_heads<1>(a, p, dev, stream) : launch_heads<2>(a, p, dev, stream);
 }
 
 }  // namespace gca

@@ -5,6 +5,7 @@ CPU ranks over gloo."""
 import ctypes as C
 import os
 import re
+import subprocess
 import sys
 import datetime
 
@@ -297,3 +298,46 @@ def test_nvtx_switch_and_call_helper(lib):
     lib.set_nvtx(False)
     with pytest.raises(ValueError):                      # a negative return code from the library -> ValueError
         lib.call("gca_linear", None, None)
+
+
+PER_DEVICE_PROGRAM = r"""
+#include <cstdio>
+#include <thread>
+#include <vector>
+#include "per_device.cuh"
+int main() {
+  gca::PerDevice d;
+  int asked[3] = {0, 0, 0}, v = -1;
+  auto ask = [&](int dev, bool works) { return d.get(dev, &v, [&](int* n) { ++asked[dev]; *n = 10 + dev; return works; }); };
+  if (ask(1, false) || asked[1] != 1) return 1;                 // a failure is reported ...
+  if (!ask(1, true) || asked[1] != 2 || v != 11) return 2;      // ... and not kept
+  if (!ask(1, true) || asked[1] != 2 || v != 11) return 3;      // a value is
+  if (!ask(0, true) || asked[0] != 1 || v != 10) return 4;      // another device has its own
+  std::vector<std::thread> ts;
+  int wrong[8] = {};
+  for (int t = 0; t < 8; ++t)
+    ts.emplace_back([&, t] { int x = -1; wrong[t] = !d.get(2, &x, [&](int* n) { ++asked[2]; *n = 12; return true; }) || x != 12; });
+  for (auto& t : ts) t.join();
+  for (int w : wrong) if (w) return 5;
+  if (asked[2] != 1) return 6;
+  if (!d.get(1000, &v, [&](int* n) { *n = 7; return true; }) || v != 7) return 7;
+  return 0;
+}
+"""
+
+
+def test_numbers_of_a_device_are_asked_for_once_per_device(tmp_path):
+    """Launch limits (cluster size, shared memory) belong to a device and not to the process; a failed attempt to raise them
+    is tried again on the next call."""
+    src, exe = tmp_path / "per_device.cpp", tmp_path / "per_device"
+    src.write_text(PER_DEVICE_PROGRAM)
+    subprocess.check_call([os.environ.get("CXX", "g++"), "-std=c++17", "-pthread", "-I", os.path.join(ROOT, "long_context_modeling_b200", "csrc"),
+                           str(src), "-o", str(exe)])
+    assert subprocess.run([str(exe)], timeout=60).returncode == 0
+    # what a kernel's launch limits are raised by stands inside such a value or in front of every launch, never in a static of the process
+    csrc = os.path.join(ROOT, "long_context_modeling_b200", "csrc")
+    for name in os.listdir(csrc):
+        if name.endswith((".cu", ".cuh")):
+            text = open(os.path.join(csrc, name)).read()
+            for static in re.findall(r"\bstatic [^;={]*= *\[.*?\}\(\);", text, flags=re.S):
+                assert "cudaFuncSetAttribute" not in static, name
