@@ -672,9 +672,11 @@ Tensor carve(const c10::Storage& st, size_t byte_offset, at::IntArrayRef sizes, 
 }
 
 struct Retrieved { Tensor keys, indices, scores, weights, n_valid; };
+struct Selection { Tensor indices, weights; };       // a copy of the selection that the caller never sees
 
+// `kept`: the selection is copied for a backward pass, which the caller's in-place changes to its own tensors must not reach.
 Retrieved score_topk(const Tensor& q_in, const Tensor& k_in, int64_t topk, bool has_pos0, int64_t q_pos0, int64_t e_base, const Tensor& noise_in,
-                     int64_t head_dim, int64_t score_round, int64_t splits) {
+                     int64_t head_dim, int64_t score_round, int64_t splits, Selection* kept = nullptr) {
   at::AutoDispatchBelowADInplaceOrView below;
   const Tensor q = bf16_rows(q_in), k = bf16_rows(k_in);
   const int64_t n = q.size(0), cq = q.size(1), d = q.size(2), e = k.size(1);
@@ -685,14 +687,20 @@ Retrieved score_topk(const Tensor& q_in, const Tensor& k_in, int64_t topk, bool 
   const c10::SmallVector<int64_t, 4> row_shape = shape;
   shape.push_back(topk);
   const int64_t m = rows * topk;
-  const Tensor block = at::empty({m * 20 + rows * 4}, q.options().dtype(at::kByte));
+  // the selection lies together, so that one copy keeps it
+  const Tensor block = at::empty({m * (kept ? 28 : 20) + rows * 4}, q.options().dtype(at::kByte));
   const c10::Storage& st = block.storage();
   Retrieved r;
   r.keys = carve(st, 0, shape, at::kLong);
   r.indices = carve(st, (size_t)m * 8, shape, at::kInt);
-  r.scores = carve(st, (size_t)m * 12, shape, at::kFloat);
-  r.weights = carve(st, (size_t)m * 16, shape, at::kFloat);
+  r.weights = carve(st, (size_t)m * 12, shape, at::kFloat);
+  r.scores = carve(st, (size_t)m * 16, shape, at::kFloat);
   r.n_valid = carve(st, (size_t)m * 20, row_shape, at::kInt);
+  if (kept) {
+    const size_t at = (size_t)m * 20 + (size_t)rows * 4;
+    kept->indices = carve(st, at, shape, at::kInt);
+    kept->weights = carve(st, at + (size_t)m * 4, shape, at::kFloat);
+  }
   if (n * cq == 0) return r;
   LmkTopkArgs a{};
   Tensor noise;
@@ -713,21 +721,25 @@ Retrieved score_topk(const Tensor& q_in, const Tensor& k_in, int64_t topk, bool 
   const Tensor ws = at::empty({(int64_t)(need > 16 ? need : 16)}, q.options().dtype(at::kByte));
   a.workspace = ws.mutable_data_ptr(); a.workspace_bytes = need;
   call("lmk_score_topk", [&] { return api.lmk_score_topk(&a, on.stream); });
+  if (kept)
+    C10_CUDA_CHECK(cudaMemcpyAsync(kept->indices.mutable_data_ptr(), r.indices.const_data_ptr(), (size_t)m * 8, cudaMemcpyDeviceToDevice,
+                                   static_cast<cudaStream_t>(on.stream)));
   return r;
 }
 
-// A tensor over the storage of `t` without its last row (axis 1 of a contiguous (N, Cq, K)).
+// A tensor over the storage of `t` without its last row (axis 1 of a contiguous (N, Cq, K)); an in-place change to either counts for both.
 Tensor without_last_row(const Tensor& t) {
   Tensor s = carve(t.storage(), (size_t)t.storage_offset() * t.element_size(), {0}, t.scalar_type());
   const int64_t cq = t.size(1);
   s.unsafeGetTensorImpl()->set_sizes_and_strides({t.size(0), cq > 0 ? cq - 1 : 0, t.size(2)}, t.strides());
+  torch::autograd::impl::set_version_counter(s, torch::autograd::impl::version_counter(t));
   return s;
 }
 
-// The retrieval weights as a function of the landmarks: outputs the weights without the last row, then whole.
+// The retrieval weights as a function of the landmarks: outputs the whole weights, then those without the last row.  The selection is the
+// node's own copy.
 struct WeightsBackward : public Node {
-  SavedVariable q, k, w;
-  Tensor indices;
+  SavedVariable q, k, indices, w;
   bool released = false;
   std::mutex mu;
 
@@ -735,33 +747,32 @@ struct WeightsBackward : public Node {
   void release_variables() override {
     std::lock_guard<std::mutex> lock(mu);
     released = true;
-    for (SavedVariable* s : {&q, &k, &w}) s->reset_data();
-    indices = Tensor();
+    for (SavedVariable* s : {&q, &k, &indices, &w}) s->reset_data();
   }
   variable_list apply(variable_list&& grads) override {
     std::lock_guard<std::mutex> lock(mu);
     TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
     variable_list out(2);
     if (!grads[0].defined() && !grads[1].defined()) return out;
-    const Tensor tq = q.unpack(), tk = k.unpack(), tw = w.unpack(shared_from_this());
+    const Tensor tq = q.unpack(), tk = k.unpack(), ti = indices.unpack(), tw = w.unpack();
     at::AutoDispatchBelowADInplaceOrView below;
     const Tensor cq = inner_contiguous(tq), ck = inner_contiguous(tk);
     Launch on(cq);
     LmkGradArgs a{};
     a.lmk_q = cq.const_data_ptr(); a.lmk_k = ck.const_data_ptr();
-    a.indices = indices.const_data_ptr<int32_t>(); a.weights = tw.const_data_ptr<float>();
+    a.indices = ti.const_data_ptr<int32_t>(); a.weights = tw.const_data_ptr<float>();
     if (grads[0].defined()) {
-      a.dw_rows = grads[0].const_data_ptr<float>(); a.rows = (int32_t)grads[0].size(1);
-      for (int i = 0; i < 3; ++i) a.dw_rows_stride[i] = grads[0].stride(i);
+      a.dw_all = grads[0].const_data_ptr<float>();
+      for (int i = 0; i < 3; ++i) a.dw_all_stride[i] = grads[0].stride(i);
     }
     if (grads[1].defined()) {
-      a.dw_all = grads[1].const_data_ptr<float>();
-      for (int i = 0; i < 3; ++i) a.dw_all_stride[i] = grads[1].stride(i);
+      a.dw_rows = grads[1].const_data_ptr<float>(); a.rows = (int32_t)grads[1].size(1);
+      for (int i = 0; i < 3; ++i) a.dw_rows_stride[i] = grads[1].stride(i);
     }
     if (task_should_compute_output(0)) { out[0] = at::empty(cq.sizes(), cq.options()); a.dlmk_q = out[0].mutable_data_ptr(); }
     if (task_should_compute_output(1)) { out[1] = at::empty(ck.sizes(), ck.options()); a.dlmk_k = out[1].mutable_data_ptr(); }
     a.q_batch_stride = cq.stride(0); a.q_row_stride = cq.stride(1); a.k_batch_stride = ck.stride(0); a.k_row_stride = ck.stride(1);
-    a.N = (int32_t)cq.size(0); a.Cq = (int32_t)cq.size(1); a.E = (int32_t)ck.size(1); a.D = (int32_t)cq.size(2); a.K = (int32_t)indices.size(2);
+    a.N = (int32_t)cq.size(0); a.Cq = (int32_t)cq.size(1); a.E = (int32_t)ck.size(1); a.D = (int32_t)cq.size(2); a.K = (int32_t)ti.size(2);
     a.q_pos0 = ck.size(1) - cq.size(1);
     try {
       call("lmk_weights_backward", [&] { return api.lmk_weights_backward(&a, on.stream); });
@@ -776,18 +787,21 @@ struct Retrieving { Tensor indices, weights; Retrieved full; };
 // needs a gradient.
 Retrieving retrieve(const Tensor& q, const Tensor& k, int64_t topk, const Tensor& noise, int64_t score_round) {
   Retrieving r;
-  r.full = score_topk(q, k, topk, false, 0, 0, noise, 0, score_round, 0);
+  const bool record = torch::autograd::compute_requires_grad(q, k);
+  Selection kept;
+  r.full = score_topk(q, k, topk, false, 0, 0, noise, 0, score_round, 0, record ? &kept : nullptr);
   r.indices = without_last_row(r.full.indices);
   r.weights = without_last_row(r.full.weights);
-  if (torch::autograd::compute_requires_grad(q, k)) {
+  if (record) {
     auto node = std::shared_ptr<WeightsBackward>(new WeightsBackward(), torch::autograd::deleteNode);
     node->set_next_edges(torch::autograd::collect_next_edges(q, k));
     node->q = SavedVariable(q, false); node->k = SavedVariable(k, false);
-    node->indices = r.full.indices;
-    torch::autograd::impl::set_version_counter(r.weights, torch::autograd::impl::version_counter(r.full.weights));
-    torch::autograd::set_history(r.weights, node);
+    node->indices = SavedVariable(kept.indices, false); node->w = SavedVariable(kept.weights, false);
     torch::autograd::set_history(r.full.weights, node);
-    node->w = SavedVariable(r.full.weights, true);
+    // the rows are a view of the whole with an edge of their own: an in-place change to either is recorded for both
+    r.weights = torch::autograd::make_variable_differentiable_view(r.weights, torch::autograd::ViewInfo(r.full.weights, nullptr, nullptr),
+                                                                   std::nullopt, false, torch::autograd::CreationMeta::DEFAULT);
+    torch::autograd::set_history(r.weights, node);
   }
   return r;
 }

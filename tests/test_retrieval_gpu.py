@@ -391,3 +391,35 @@ def test_retrieval_weight_gradients_against_float32(lcm, n, c, d, k):
     assert torch.equal(idx, full.indices[:, :-1]) and torch.allclose(w, ref[:, :-1], atol=1e-5)
     for got, want in ((dq, rq), (dm, rm)):
         assert (got.float() - want).norm() <= 4e-3 * want.norm() + 1e-6
+
+
+def _retrieve_with_float32_twin(lcm, n, c, d, k, seed):
+    """(q, landmarks, ids, weights, whole result) of a bf16 retrieval that records gradients, and the same weights as float32
+    torch operations over the same selection: (q, landmarks, weights, whole weights)."""
+    lq, lk = cases.landmark_case(seed, n, c, c, d=d, std=0.5)
+    q, m = lq.cuda().requires_grad_(), lk.cuda().requires_grad_()
+    idx, w, full = lcm.retrieve(q, type("Chunks", (), {"past_lmk_embeds": m}), k)
+    qf, mf = lq.cuda().float().requires_grad_(), lk.cuda().float().requires_grad_()
+    ref = lcm.differentiable_weights(qf, mf, full.indices)
+    return (q, m, idx, w, full), (qf, mf, ref[:, :-1], ref)
+
+
+def test_in_place_changes_to_a_retrieval_and_its_gradients(lcm):
+    """The returned selection belongs to the caller: changed ids and scores do not reach the backward pass, a change to the weights
+    is recorded like that of any view (both results see it)."""
+    (q, m, idx, w, full), (qf, mf, wf, ref) = _retrieve_with_float32_twin(lcm, 2, 37, 768, 8, 35)
+    factor = torch.rand(w.shape, generator=torch.Generator().manual_seed(7)).cuda()
+    idx.fill_(0)
+    full.indices[:, -1] = 0
+    full.scores.zero_()
+    w.mul_(factor)
+    wf.mul_(factor)
+    full.weights.add_(w.sum())
+    ref.add_(wf.sum())
+    assert torch.allclose(full.weights, ref, atol=1e-4) and torch.equal(full.weights[:, :-1], w)
+    g = torch.Generator().manual_seed(8)
+    probe, probe_all = (torch.randn(x.shape, generator=g).cuda() for x in (w, full.weights))
+    got = torch.autograd.grad([w, full.weights], [q, m], [probe, probe_all])
+    want = torch.autograd.grad([wf, ref], [qf, mf], [probe, probe_all])
+    for a, b in zip(got, want):                              # each gradient is a float32 sum rounded to bf16 once (2^-9)
+        assert (a.float() - b).norm() <= 4e-3 * b.norm()
