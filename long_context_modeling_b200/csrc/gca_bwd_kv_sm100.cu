@@ -154,8 +154,8 @@ struct BwdKvParams {
   long long dks[4], dvs[4];
   int units;
   int N, J, Hq, Hkv, G, K, C, HP;
-  int div;                  // unit u: chunk u / div of the table, head pair u % div; heads_outside: pair u / div, chunk u % div
-  bool heads_outside, in_turn;
+  bool heads_outside;       // a sequence's units: one head pair after the other (else a chunk's head pairs side by side)
+  bool in_turn;
   int wide_store;           // dk / dv rows are 32-byte aligned: 256-bit stores
   float c2, sm_scale;
   const float4* dw_part;    // (N*J, Hq, K): the q-major pass's four partials of every (head, slot) of dw, or nullptr
@@ -191,9 +191,14 @@ __device__ void kv_scheduler(const BwdKvParams& p, uint8_t* smem, uint64_t* bars
   for (int u = blockIdx.x;; u = p.in_turn ? u + (int)gridDim.x : (int)gridDim.x + atomicAdd(p.tickets, 1)) {
     int4 unit = make_int4(0, -1, 0, 0);
     if (u < p.units) {
-      const int q = u / p.div, r = u - q * p.div;
-      unit = p.unit_tab[p.heads_outside ? r : q];
-      unit.w = p.heads_outside ? q : r;
+      int row = u / p.HP, pair = u - row * p.HP;
+      if (p.heads_outside) {
+        const int n = u / (p.C * p.HP), x = u - n * p.C * p.HP;
+        pair = x / p.C;
+        row = n * p.C + x - pair * p.C;
+      }
+      unit = p.unit_tab[row];
+      unit.w = pair;
     }
     slots[head % ND] = unit;
     mbar_arrive(&bars[UNIT_FULL + head % ND]);
@@ -624,10 +629,15 @@ int launch_bwd_kv_tc(const GcaBwdArgs& a, const Csr& csr, const uint4* rowterm, 
   for (int i = 0; i < 4; ++i) { p.dks[i] = a.dk_stride[i]; p.dvs[i] = a.dv_stride[i]; }
   p.N = a.N; p.J = a.J; p.Hq = a.Hq; p.Hkv = a.Hkv; p.G = a.Hq / a.Hkv; p.K = a.K; p.C = a.C;
   p.HP = (a.Hkv + 1) / 2;
-  // A chunk's head pairs side by side, but for one long sequence whose Q and dO do not fit into L2 (126 MB): there one head pair
-  // after the other, which reads those of a pair only (1,024 chunks, 12 heads: 620 -> 590 us; where they do fit it costs 5 %).
-  p.heads_outside = a.N == 1 && (long long)a.J * a.Hq * PAIR_BYTES > (126ll << 20);
-  p.div = p.heads_outside ? a.C : p.HP;
+  // The order inside a sequence: a chunk's head pairs side by side, or one head pair after the other.  The second reads the Q and dO of
+  // one pair at a time, which L2 (126 MB) holds where it does not hold those of all, but every pair ends with the short units of
+  // the late chunks (~4 us each).  So it pays where what misses L2 of a pass, iterations per CTA x share that does not fit, outweighs
+  // those ends, whatever the number of sequences.  12 heads, side by side / one after the other in us: 1 x 1,024 chunks K = 4: 226 / 242,
+  // K = 8: 355 / 365, K = 12: 486 / 488, K = 16: 621 / 609; 1 x 2,000 K = 4: 435 / 442, K = 8: 713 / 678; 1 x 1,400 K = 16: 869 / 816;
+  // 2 x 1,024 K = 8: 697 / 721, K = 16: 1248 / 1194; 4 x 1,024 K = 16: 2489 / 2378; 2 x 700 K = 16 (131 MB): 818 / 844.
+  // (Beyond 126 MB per sequence the unit table is always in sequence order.)
+  const long long l2 = 126ll << 20, seq_bytes = (long long)a.J * a.Hq * PAIR_BYTES;
+  p.heads_outside = seq_bytes > l2 && (long long)a.J * a.K * p.G * ((seq_bytes - l2) >> 20) > 32ll * sms * (seq_bytes >> 20);
   // From eight sequences on, one after the other, units are dealt out in turn all the same.  CTAs that draw reach the end of a sequence
   // together, where its units are short and the next one's tiles are not in L2 yet; dealt out they drift apart (8 x 256
   // chunks: 628 against 664 us, 8 x 100: 187 against 195; 5 x 300: 420 against 393).

@@ -281,7 +281,7 @@ def test_inverse_index_sections_equal_radix_sort(lcm, shape):
 
 @pytest.mark.parametrize("shape", [(1, 820, 10, 2), (2, 420, 10, 2), (9, 100, 5, 3), (3, 5, 1, 2)])
 def test_unit_orders_of_the_kv_major_pass(lcm, shape):
-    """Every order in which the kv-major pass hands out its units -- one long sequence by head pairs, sequence by sequence, in turn from
+    """Every order in which the kv-major pass hands out its units -- one long sequence, sequence by sequence, in turn from
     eight sequences on, all sequences by count -- covers every chunk once: dK / dV against the CUDA-core kernels; repeated
     launches (the ticket counters are back where they were) give the same bits."""
     from long_context_modeling_b200 import gca as gmod
@@ -300,6 +300,32 @@ def test_unit_orders_of_the_kv_major_pass(lcm, shape):
     want = gmod.gca_backward_stages(q, kc, vc, idx, w, dout, lse, 0.125, algo=gmod.ALGO_SIMT)[1:3]
     for x, y in zip(got, want):
         assert (x.float() - y.float()).abs().max().item() <= 2e-2 * max(1e-3, y.float().abs().max().item())
+    assert lcm.read_status() == 0
+
+
+@pytest.mark.parametrize("n,c,hq,hkv,k", [(1, 400, 32, 4, 12), (2, 360, 32, 4, 12), (3, 291, 30, 3, 32)])
+def test_head_pairs_one_after_the_other(lcm, n, c, hq, hkv, k):
+    """Sequences whose Q and dO exceed L2 with enough work per head pair: units in the order (sequence, head pair, chunk).  A sequence's
+    gradients do not depend on its neighbours: the bits of each sequence's own call with a chunk's head pairs side by side
+    (two head groups at a time fit L2), and no chunk missed."""
+    from long_context_modeling_b200 import gca as gmod
+    g = torch.Generator(device="cuda").manual_seed(44)
+    q, dout = (torch.empty(n, c - 1, hq, 64, 64, dtype=torch.bfloat16, device="cuda").normal_(generator=g) for _ in range(2))
+    kc, vc = (torch.empty(n, c, 64, hkv, 64, dtype=torch.bfloat16, device="cuda").normal_(generator=g) for _ in range(2))
+    idx = torch.rand(n, c - 1, c, generator=g, device="cuda").topk(k, dim=2).indices.int()
+    w = torch.softmax(torch.randn(n, c - 1, k, generator=g, device="cuda"), -1)
+    over = 1 - (126 << 20) / ((c - 1) * hq * 16384)
+    assert over > 0 and (c - 1) * k * hq // hkv * over > 32 * 148        # what the order is chosen by
+    _, lse = gmod.gca_forward_with_lse(q, kc, vc, idx, w, 0.125)
+    dk, dv = gmod.gca_backward_stages(q, kc, vc, idx, w, dout, lse, 0.125)[1:3]
+    group = hq // hkv
+    for i in range(n):
+        for h in range(0, hkv, 2):                       # a head pair (or the last head) by itself
+            hs, qs = slice(h, min(h + 2, hkv)), slice(h * group, min(h + 2, hkv) * group)
+            args = [t[i:i + 1].contiguous() for t in (q[:, :, qs], kc[:, :, :, hs], vc[:, :, :, hs], idx, w, dout[:, :, qs])]
+            _, l1 = gmod.gca_forward_with_lse(*args[:5], 0.125)
+            want = gmod.gca_backward_stages(*args, l1, 0.125)[1:3]
+            assert torch.equal(dk[i, :, :, hs], want[0][0]) and torch.equal(dv[i, :, :, hs], want[1][0])
     assert lcm.read_status() == 0
 
 
