@@ -155,7 +155,7 @@ struct BwdKvParams {
   int units;
   int N, J, Hq, Hkv, G, K, C, HP;
   bool heads_outside;       // a sequence's units: one head pair after the other (else a chunk's head pairs side by side)
-  bool in_turn;
+  int rotate;               // 0: units are drawn; else dealt out, every sequence from this many CTAs further on
   int wide_store;           // dk / dv rows are 32-byte aligned: 256-bit stores
   float c2, sm_scale;
   const float4* dw_part;    // (N*J, Hq, K): the q-major pass's four partials of every (head, slot) of dw, or nullptr
@@ -188,12 +188,22 @@ __device__ void kv_scheduler(const BwdKvParams& p, uint8_t* smem, uint64_t* bars
   int4* slots = reinterpret_cast<int4*>(smem + OFF_UNIT);
   uint32_t head = 0, tail = 0;               // units published, units that all roles have read
   int ahead = 0;                             // iterations between the two
-  for (int u = blockIdx.x;; u = p.in_turn ? u + (int)gridDim.x : (int)gridDim.x + atomicAdd(p.tickets, 1)) {
+  const int grid = (int)gridDim.x, per_seq = p.C * p.HP;
+  int seq = 0, first = (int)blockIdx.x, at = first;            // dealt out: sequence, this CTA's first place in it, its next place
+  auto dealt = [&] {
+    while (at >= per_seq && ++seq < p.N) {
+      first += p.rotate;
+      if (first >= grid) first -= grid;
+      at = first;
+    }
+    return seq < p.N ? seq * per_seq + at : p.units;
+  };
+  for (int u = p.rotate ? dealt() : first;;) {
     int4 unit = make_int4(0, -1, 0, 0);
     if (u < p.units) {
       int row = u / p.HP, pair = u - row * p.HP;
       if (p.heads_outside) {
-        const int n = u / (p.C * p.HP), x = u - n * p.C * p.HP;
+        const int n = u / per_seq, x = u - n * per_seq;
         pair = x / p.C;
         row = n * p.C + x - pair * p.C;
       }
@@ -214,6 +224,8 @@ __device__ void kv_scheduler(const BwdKvParams& p, uint8_t* smem, uint64_t* bars
       ahead -= (slots[tail % ND].y - slots[tail % ND].x) * p.G;
       ++tail;
     }
+    at += grid;
+    u = p.rotate ? dealt() : grid + atomicAdd(p.tickets, 1);
   }
 }
 // The next published unit (y < 0: no more work), read by a whole warp.
@@ -577,15 +589,17 @@ bwd_kv_tc_kernel(const __grid_constant__ BwdKvParams p) {
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  if (warp < 4 * NG) {
+  // The order of the roles is the order of their code, and the time depends on where the hot loops lie: 8 x 256 chunks, forward +
+  // backward, 1543 us with the issuers in front, 1565 with the workers in front, 1600 with scheduler and producer in front.
+  if (warp == ISSUE_S) kv_issuer<0>(p, smem, bars, abort_flag, lane, tmem_base);
+  else if (warp == ISSUE_DP) kv_issuer<1>(p, smem, bars, abort_flag, lane, tmem_base);
+  else if (warp == ISSUE_DV) kv_issuer<2>(p, smem, bars, abort_flag, lane, tmem_base);
+  else if (GRAD_ISSUERS == 2 && warp == ISSUE_DV + 1) kv_issuer<3>(p, smem, bars, abort_flag, lane, tmem_base);
+  else if (warp < 4 * NG) {
     reduce_dw(p);                        // while the first tiles are on their way
     kv_worker(p, smem, bars, abort_flag, warp >> 2, warp & 3, lane, tmem_base);
   } else if (warp == PROD_WARP) { if (lane == 0) kv_producer(p, smem, bars, abort_flag); }
-  else if (warp == SCHED_WARP) { if (lane == 0) kv_scheduler(p, smem, bars, abort_flag); }
-  else if (warp == ISSUE_S) kv_issuer<0>(p, smem, bars, abort_flag, lane, tmem_base);
-  else if (warp == ISSUE_DP) kv_issuer<1>(p, smem, bars, abort_flag, lane, tmem_base);
-  else if (warp == ISSUE_DV) kv_issuer<2>(p, smem, bars, abort_flag, lane, tmem_base);
-  else kv_issuer<3>(p, smem, bars, abort_flag, lane, tmem_base);
+  else if (lane == 0) kv_scheduler(p, smem, bars, abort_flag);
   tc_fence_before();
   __syncthreads();
   if (warp == ISSUE_S) tmem_dealloc(tmem_base, TMEM_COLS);
@@ -638,10 +652,6 @@ int launch_bwd_kv_tc(const GcaBwdArgs& a, const Csr& csr, const uint4* rowterm, 
   // (Beyond 126 MB per sequence the unit table is always in sequence order.)
   const long long l2 = 126ll << 20, seq_bytes = (long long)a.J * a.Hq * PAIR_BYTES;
   p.heads_outside = seq_bytes > l2 && (long long)a.J * a.K * p.G * ((seq_bytes - l2) >> 20) > 32ll * sms * (seq_bytes >> 20);
-  // From eight sequences on, one after the other, units are dealt out in turn all the same.  CTAs that draw reach the end of a sequence
-  // together, where its units are short and the next one's tiles are not in L2 yet; dealt out they drift apart (8 x 256
-  // chunks: 628 against 664 us, 8 x 100: 187 against 195; 5 x 300: 420 against 393).
-  p.in_turn = a.N >= 8 && !units_by_count(a);
   const long long units = (long long)a.N * a.C * p.HP;
   if (units >= (1ll << 31) - 65536) return GCA_ERR_TOO_LARGE;
   p.units = (int)units;
@@ -650,6 +660,18 @@ int launch_bwd_kv_tc(const GcaBwdArgs& a, const Csr& csr, const uint4* rowterm, 
   if (p.units == 0) return 0;
   GCA_CUDA_CHECK(cudaFuncSetAttribute(bwd_kv_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
   const unsigned grid = (unsigned)(p.units < sms ? p.units : sms);
+  // Several short sequences, one after the other, are dealt out instead of drawn.  CTAs that draw reach the end of every sequence
+  // together, where the units are short and the next sequence's tiles not in L2 yet; CTAs that are dealt to drift apart, which
+  // keeps two sequences in L2 at a time (hence half of its 126 MB) and takes some sequences to even out (four).  What a CTA is
+  // dealt depends on its first place in each sequence.  Without a rotation that place moves by the sequence's units modulo the CTAs,
+  // and where that is near 0 the same CTAs get all the long units (8 x 222 chunks, 12 heads, K = 8: 660 us).  0.38 of the CTAs, the
+  // golden section, spreads it for any length; an EVEN number, so that neighbours stay on two head pairs of one chunk: 57 instead
+  // of 56 of 148 loses all of the gain (8 x 256: 730 us), as does an odd number of pairs.
+  // Drawn / dealt out in us: 8 x 222: 594 / 570, 8 x 256: 680 / 658, 8 x 100: 283 / 265, 16 x 100: 556 / 506, 32 x 37: 404 / 355, 300 x 4
+  // (K = 2): 140 / 126, 4 x 222: 304 / 300.  Across the line: 3 x 300: 308 / 316, 8 x 512 (96 MB a sequence): 1328 / 1344, 8 x 256
+  // with 6 heads: 365 / 380, one query chunk per sequence (units all alike; 1,000 x 16 heads, K = 8, the step): 1859 / 1975.
+  const bool deal = a.N >= 4 && a.J > 1 && p.HP % 2 == 0 && 2 * seq_bytes <= l2 && !units_by_count(a);
+  p.rotate = deal ? 2 * ((191 * (int)grid + 500) / 1000) : 0;
   p.dw_part = reinterpret_cast<const float4*>(dw_part); p.dw = a.dw;
   bwd_kv_tc_kernel<<<grid, NTHREADS, SMEM_BYTES, stream>>>(p);
   GCA_CUDA_CHECK(cudaGetLastError());

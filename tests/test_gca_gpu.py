@@ -281,8 +281,8 @@ def test_inverse_index_sections_equal_radix_sort(lcm, shape):
 
 @pytest.mark.parametrize("shape", [(1, 820, 10, 2), (2, 420, 10, 2), (9, 100, 5, 3), (3, 5, 1, 2)])
 def test_unit_orders_of_the_kv_major_pass(lcm, shape):
-    """Every order in which the kv-major pass hands out its units -- one long sequence, sequence by sequence, in turn from
-    eight sequences on, all sequences by count -- covers every chunk once: dK / dV against the CUDA-core kernels; repeated
+    """Every order in which the kv-major pass hands out its units -- one long sequence, sequence by sequence,
+    all sequences by count -- covers every chunk once: dK / dV against the CUDA-core kernels; repeated
     launches (the ticket counters are back where they were) give the same bits."""
     from long_context_modeling_b200 import gca as gmod
     n, c, h, k = shape
@@ -301,6 +301,28 @@ def test_unit_orders_of_the_kv_major_pass(lcm, shape):
     for x, y in zip(got, want):
         assert (x.float() - y.float()).abs().max().item() <= 2e-2 * max(1e-3, y.float().abs().max().item())
     assert lcm.read_status() == 0
+
+
+@pytest.mark.parametrize("n,c,h,k", [(4, 520, 4, 2), (21, 100, 4, 3), (72, 40, 3, 1), (11, 76, 12, 5), (300, 5, 8, 2)])
+def test_sequences_dealt_out_in_rotation(lcm, n, c, h, k):
+    """Short sequences whose units are dealt out to the CTAs: many waves, about one, less than one and a few units per sequence, an odd
+    head.  Every chunk once: the bits of each sequence's own call, whose units are drawn."""
+    from long_context_modeling_b200 import gca as gmod
+    assert n >= 4 and c > 2 and (h + 1) // 2 % 2 == 0 and n * (c - 1) * h * 8192 > 64 << 20 and (c - 1) * h * 16384 <= 63 << 20
+    g = torch.Generator(device="cuda").manual_seed(45)
+    q, dout = (torch.empty(n, c - 1, h, 64, 64, dtype=torch.bfloat16, device="cuda").normal_(generator=g) for _ in range(2))
+    kc, vc = (torch.empty(n, c, 64, h * 64, dtype=torch.bfloat16, device="cuda").normal_(generator=g) for _ in range(2))
+    idx = torch.rand(n, c - 1, c, generator=g, device="cuda").topk(k, dim=2).indices.int()
+    idx[:, ::3, k - 1] = -1
+    w = torch.softmax(torch.randn(n, c - 1, k, generator=g, device="cuda"), -1)
+    _, lse = gmod.gca_forward_with_lse(q, kc, vc, idx, w, 0.125)
+    dk, dv = gmod.gca_backward_stages(q, kc, vc, idx, w, dout, lse, 0.125)[1:3]
+    for i in range(0, n, max(1, n // 7)):
+        args = [t[i:i + 1] for t in (q, kc, vc, idx, w, dout)]
+        _, l1 = gmod.gca_forward_with_lse(*args[:5], 0.125)
+        want = gmod.gca_backward_stages(*args, l1, 0.125)[1:3]
+        assert torch.equal(dk[i], want[0][0]) and torch.equal(dv[i], want[1][0])
+    assert torch.isfinite(dk).all() and torch.isfinite(dv).all() and lcm.read_status() == 0
 
 
 @pytest.mark.parametrize("n,c,hq,hkv,k", [(1, 400, 32, 4, 12), (2, 360, 32, 4, 12), (3, 291, 30, 3, 32)])
