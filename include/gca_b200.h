@@ -445,9 +445,13 @@ typedef struct LinearBatchedArgs {
   float rms_eps;              /* > 0: scale the rows by rsqrt(mean(x^2) + rms_eps), computed on the way (row_scale NULL);
                                  for up to GCA_SKINNY_ROWS rows in all, lying back to back, else GCA_ERR_SHAPE */
 } LinearBatchedArgs;
-#define GCA_SKINNY_ROWS 128   /* up to this many rows take the latency-bound form of gca_linear */
+#define GCA_SKINNY_ROWS 128   /* up to this many rows can take the latency-bound form of gca_linear */
 
 int gca_linear_batched(const LinearBatchedArgs* args, void* stream);
+
+/* 1 where M rows of K -> N are faster in the latency-bound form on the current device than as tiles of the tensor cores, which
+ * gca_linear goes by.  with_norm: RMSNorm + projection as one call with rms_eps against gca_row_rms and a call with row_scale. */
+int gca_linear_few_rows(int64_t M, int32_t N, int32_t K, int32_t with_norm);
 
 /* The GCA sub-layer of a decode step for a few sequences as one launch (model/DRT.py:345-394):
  *   out[n, s] = residual[n, s] + Wo attention(rmsnorm(x[n, s]) Wq^T, the chunks in indices[n]) .

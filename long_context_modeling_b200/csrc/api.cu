@@ -16,6 +16,7 @@ int launch_kv_project_append(const KvProjectArgs& a, int sms, cudaStream_t strea
 int launch_row_rms(const RowRmsArgs& a, cudaStream_t stream);
 int launch_silu_mul(const void* gu, void* out, long long M, int I, long long in_stride, long long out_stride, cudaStream_t stream);
 int launch_linear(const LinearBatchedArgs& a, int sms, cudaStream_t stream);
+bool few_rows(long long M, int N, int K, bool with_norm, int sms);
 int launch_layer_decode(const LayerDecodeArgs& a, int dev, cudaStream_t stream);
 int launch_window_decode(const WindowDecodeArgs& a, cudaStream_t stream);
 int launch_window_ring_decode(const WindowRingDecodeArgs& a, cudaStream_t stream);
@@ -471,6 +472,12 @@ int gca_linear_batched(const LinearBatchedArgs* b, void* stream) {
   gca::DeviceScope scope(a->out);
   if (scope.rc) return scope.rc;
   return gca::launch_linear(*b, gca::sm_count(scope.dev), (cudaStream_t)stream);
+}
+
+int gca_linear_few_rows(int64_t M, int32_t N, int32_t K, int32_t with_norm) {
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess) { (void)cudaGetLastError(); return 0; }
+  return gca::few_rows(M, N, K, with_norm != 0, gca::sm_count(dev));
 }
 
 int gca_linear(const LinearArgs* a, void* stream) {

@@ -45,7 +45,7 @@ struct Api {
 #define GCA_API_LIST                                                                                          \
   GCA_API(gca_fwd) GCA_API(gca_decode) GCA_API(gca_bwd_stages) GCA_API(gca_bwd_workspace_bytes)               \
   GCA_API(lmk_score_topk) GCA_API(lmk_topk_workspace_bytes) GCA_API(lmk_weights_backward) GCA_API(gca_kv_project_append) GCA_API(gca_row_rms) \
-  GCA_API(gca_linear) GCA_API(gca_linear_batched) GCA_API(gca_layer_decode) GCA_API(gca_silu_mul) GCA_API(gca_window_decode)            \
+  GCA_API(gca_linear) GCA_API(gca_linear_batched) GCA_API(gca_linear_few_rows) GCA_API(gca_layer_decode) GCA_API(gca_silu_mul) GCA_API(gca_window_decode)            \
   GCA_API(gca_window_ring_decode) GCA_API(gca_strerror)
   GCA_API_LIST
 #undef GCA_API
@@ -456,8 +456,8 @@ Tensor linear(const Tensor& x, const Tensor& weight, const Tensor& row_scale, co
 Tensor rmsnorm_linear(const Tensor& x, const Tensor& weight, double eps) {
   at::AutoDispatchBelowADInplaceOrView below;
   const Rows r = rows_of(x);
-  if (r.m > GCA_SKINNY_ROWS) return linear(x, weight, row_rms(x, eps), Tensor(), Tensor());
   Launch on(x);
+  if (!api.gca_linear_few_rows(r.m, (int32_t)weight.size(0), (int32_t)x.size(-1), 1)) return linear(x, weight, row_rms(x, eps), Tensor(), Tensor());
   c10::SmallVector<int64_t, 6> shape(x.sizes().begin(), x.sizes().end());
   shape.back() = weight.size(0);
   const Tensor out = at::empty(shape, x.options());
@@ -531,7 +531,7 @@ Tensor layer_fused(const Tensor& hidden_in, const Tensor& q_weight, double eps, 
       return out;
     }
   }
-  const bool few = n * rows <= GCA_SKINNY_ROWS && skip == 0;             // the norm rides on the projection
+  const bool few = skip == 0 && api.gca_linear_few_rows(n * rows, (int32_t)q_weight.size(0), (int32_t)dim, 1);       // the norm rides on the projection
   const Tensor q = at::empty({2, n, J, s, dim}, hidden.options());      // [0]: q, [1]: the attention's output
   void* const vals = static_cast<char*>(q.mutable_data_ptr()) + q.stride(0) * 2;
   Tensor scale;

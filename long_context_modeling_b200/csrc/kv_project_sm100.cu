@@ -432,6 +432,7 @@ __global__ void ce_combine_kernel(const float2* __restrict__ part, const float* 
 }  // namespace
 
 int launch_skinny_linear(const LinearArgs& a, float rms_eps, cudaStream_t stream);
+bool few_rows(long long M, int N, int K, bool with_norm, int sms);
 
 namespace {
 
@@ -528,7 +529,8 @@ int launch_linear(const LinearBatchedArgs& ba, int sms, cudaStream_t stream) {
     a.M *= args.batches;
     args.batches = 1;
   }
-  if (args.batches == 1 && args.lead_rows == 0 && a.M <= GCA_SKINNY_ROWS) return launch_skinny_linear(a, args.rms_eps, stream);
+  if (args.batches == 1 && args.lead_rows == 0 && a.M <= GCA_SKINNY_ROWS && (args.rms_eps > 0.f || few_rows(a.M, a.N, a.K, false, sms)))
+    return launch_skinny_linear(a, args.rms_eps, stream);
   if (args.rms_eps > 0.f) return GCA_ERR_SHAPE;
   ProjParams p;
   if (a.M >= (1ll << 31)) return GCA_ERR_TOO_LARGE;

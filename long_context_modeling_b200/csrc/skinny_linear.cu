@@ -140,7 +140,24 @@ skinny_linear_kernel(const SkinnyParams p) {
 
 }  // namespace
 
-// One block of rows (batches back to back), M <= SKINNY_ROWS.
+// Which products: what grows with rows and columns is the number of blocks, each of which reads its rows and its columns again, while
+// the 128-row tiles of the tensor cores take the same ~5-7 us whatever the rows (~10 at 8,192 columns and few rows).  The line is where
+// a wave of blocks is full: three per SM of 32 x 16, 14 per SM of 16 x 8 (which only read weights, once).  us, this form / tiles:
+//   M = 16: 768 -> 4,096 3.5 / 6.1, 1,024 -> 8,192 7.4 / 9.7, 768 -> 16,384 (2,048 blocks) 9.3 / 9.2, 768 -> 50,304 24.5 / 19.5
+//   M = 32: 768 -> 4,096 4.7 / 5.8, 1,024 -> 8,192 (512 blocks) 10.0 / 9.0, M = 17: 9.0 / 9.7; 768 -> 16,384 11.0 / 9.2
+//   M = 64: 1,024 -> 3,072 (384 blocks) 5.5 / 6.1, 768 -> 4,096 (512) 8.0 / 5.5;  M = 96: 768 -> 2,304 (432) 4.9 / 5.4, 1,024 -> 3,072 9.9 / 6.2
+//   M = 128: 768 -> 768 4.3 / 5.1, 768 -> 2,304 (576) 8.0 / 5.6, 768 -> 4,096 11.8 / 5.8
+// With the norm the tiles cost a launch more, and the blocks' work per wave decides: 768 -> 2,304, M = 128: 8.7 / 8.9, 768 -> 4,096, M = 64:
+// 8.7 / 8.8, 1,024 -> 3,072, M = 96: 10.4 / 8.5, 1,024 -> 4,096, M = 64: 10.4 / 9.3, 768 -> 4,096, M = 128: 12.8 / 9.1.
+bool few_rows(long long M, int N, int K, bool with_norm, int sms) {
+  if (M > GCA_SKINNY_ROWS) return false;
+  if (M <= 16) return N / 8 <= 14 * sms;
+  const long long blocks = N / 16 * ((M + 31) / 32);
+  if (M <= 32) return blocks <= 4 * sms;
+  return with_norm ? blocks * K <= 3ll * sms * 1024 : blocks <= 3 * sms;
+}
+
+// One block of rows (batches back to back), M <= GCA_SKINNY_ROWS.
 int launch_skinny_linear(const LinearArgs& a, float rms_eps, cudaStream_t stream) {
   SkinnyParams p;
   p.x = (const __nv_bfloat16*)a.x; p.w = (const __nv_bfloat16*)a.w; p.out = (__nv_bfloat16*)a.out;

@@ -396,3 +396,23 @@ def test_projection_append_tile_widths(n, c, dim):
         ref = torch.cat([ref[:, :1], ref], 1)
         assert (got.float() - ref).abs().max() <= 2e-2 * ref.abs().max()
     assert torch.equal(cache.past_lmk_embeds, torch.cat([x[:, :1, -1], x[:, :, -1]], 1))
+
+
+@pytest.mark.parametrize("m,n,k,few", [(16, 16576, 64, True), (16, 16592, 64, False), (32, 9472, 64, True), (32, 9488, 64, False),
+                                       (64, 3552, 128, True), (64, 3568, 128, False), (128, 2304, 768, False), (96, 3072, 1024, False)])
+def test_few_row_form_on_both_sides_of_its_line(m, n, k, few):
+    """Products on either side of the line between the latency-bound form and the tiles; RMSNorm + projection, whose line lies
+    elsewhere, at the same sizes."""
+    need_gpu()
+    from long_context_modeling_b200 import _lib
+    rows = _lib.lib().gca_linear_few_rows
+    assert rows(m, n, k, 0) == int(few) and rows(129, n, k, 1) == 0 and rows(1, 768, 768, 1) == 1
+    test_few_row_linear_and_fused_norm_against_float32(m, n, k, True)
+
+
+def test_decode_step_too_wide_for_the_few_row_form():
+    """64 sequences x 2 rows of a 2,048-wide sub-layer: row norms and tiled projections around the decode attention."""
+    need_gpu()
+    from long_context_modeling_b200 import _lib
+    assert _lib.lib().gca_linear_few_rows(128, 2048, 2048, 1) == 0
+    test_one_launch_decode_step(64, 32, 2, 2, 3)
