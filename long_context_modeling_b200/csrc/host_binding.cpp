@@ -16,7 +16,12 @@
 #include <ATen/ops/empty.h>
 #include <ATen/ops/empty_like.h>
 #include <ATen/ops/empty_strided.h>
+#include <ATen/ops/arange.h>
+#include <ATen/ops/constant_pad_nd.h>
+#include <ATen/ops/nan_to_num.h>
+#include <ATen/ops/softmax.h>
 #include <ATen/ops/zeros.h>
+#include <ATen/ops/zeros_like.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <nvtx3/nvToolsExt.h>
@@ -28,6 +33,7 @@
 
 #include <array>
 #include <atomic>
+#include <cmath>
 #include <mutex>
 
 #include "gca_b200.h"
@@ -755,6 +761,9 @@ struct WeightsBackward : public Node {
     variable_list out(2);
     if (!grads[0].defined() && !grads[1].defined()) return out;
     const Tensor tq = q.unpack(), tk = k.unpack(), ti = indices.unpack(), tw = w.unpack();
+    // gradients that are to be differentiated again, or come batched from vmap
+    const auto plain = [](const Tensor& t) { return !t.defined() || t.has_storage(); };
+    if (at::GradMode::is_enabled() || !plain(grads[0]) || !plain(grads[1])) return by_operations(tq, tk, ti, grads);
     at::AutoDispatchBelowADInplaceOrView below;
     const Tensor cq = inner_contiguous(tq), ck = inner_contiguous(tk);
     Launch on(cq);
@@ -777,6 +786,26 @@ struct WeightsBackward : public Node {
     try {
       call("lmk_weights_backward", [&] { return api.lmk_weights_backward(&a, on.stream); });
     } catch (const LibraryError& e) { GcaBackward::raise(e); }
+    return out;
+  }
+  // The same gradient as differentiable operations in float32, the weights among them.
+  variable_list by_operations(const Tensor& tq, const Tensor& tk, const Tensor& ti, const variable_list& grads) {
+    const double scale = 1.0 / std::sqrt((double)tq.size(2));
+    const Tensor lq = tq.to(at::kFloat), lk = tk.to(at::kFloat), padding = ti < 0;
+    const c10::List<std::optional<Tensor>> at_rows({at::arange(tq.size(0), ti.options().dtype(at::kLong)).view({-1, 1, 1}), ti.clamp_min(0).to(at::kLong)});
+    const Tensor rows = lk.index(at_rows);                                                       // (N, Cq, K, D)
+    const Tensor s = ((lq.unsqueeze(2) * rows).sum(-1) * scale).masked_fill(padding, -INFINITY);
+    const Tensor weights = at::nan_to_num(at::softmax(s, -1), 0.0);
+    Tensor dw = grads[0];
+    if (grads[1].defined()) {
+      const Tensor whole = at::constant_pad_nd(grads[1], {0, 0, 0, 1});                          // the last row is in the first output only
+      dw = dw.defined() ? dw + whole : whole;
+    }
+    const Tensor ds = weights * (dw - (dw * weights).sum(-1, true)) * scale;
+    variable_list out(2);
+    if (task_should_compute_output(0)) out[0] = (ds.unsqueeze(-1) * rows).sum(2).to(tq.scalar_type());
+    if (task_should_compute_output(1))
+      out[1] = at::zeros_like(lk).index_put(at_rows, ds.unsqueeze(-1) * lq.unsqueeze(2), true).to(tk.scalar_type());
     return out;
   }
 };

@@ -423,3 +423,26 @@ def test_in_place_changes_to_a_retrieval_and_its_gradients(lcm):
     want = torch.autograd.grad([wf, ref], [qf, mf], [probe, probe_all])
     for a, b in zip(got, want):                              # each gradient is a float32 sum rounded to bf16 once (2^-9)
         assert (a.float() - b).norm() <= 4e-3 * b.norm()
+
+
+def test_gradients_of_retrieval_weights_can_be_differentiated_and_batched(lcm):
+    """A gradient penalty (backward of the backward) and batched gradients (vmap), against float32 torch operations over the same
+    selection; two outputs, rows with fewer chunks than slots."""
+    (q, m, _, w, full), (qf, mf, wf, ref) = _retrieve_with_float32_twin(lcm, 2, 9, 64, 4, 36)
+    g = torch.Generator().manual_seed(9)
+    probe, probe_all = (torch.randn(x.shape, generator=g).cuda() for x in (w, full.weights))
+
+    def penalty(outs, ins, probes):
+        first = torch.autograd.grad(outs, ins, probes, create_graph=True)
+        return first, torch.autograd.grad(sum(x.float().pow(2).sum() for x in first), (*ins, *probes))
+
+    got = penalty([w, full.weights], [q, m], [probe.requires_grad_(), probe_all.requires_grad_()])
+    want = penalty([wf, ref], [qf, mf], [probe, probe_all])
+    # the first row sees no chunk: zeros here, where a softmax over nothing differentiated twice is NaN
+    for a, b in zip(got[0] + got[1], want[0] + want[1]):       # bf16 results of float32 sums, the second ones of rounded first ones
+        assert (a.float() - b.nan_to_num(0.0)).norm() <= 1e-2 * b.nan_to_num(0.0).norm() and torch.isfinite(a).all()
+    once = torch.autograd.grad(w, [q, m], probe, retain_graph=True)
+    several = torch.stack([probe, -2 * probe]).detach()
+    for x, y in zip(torch.autograd.grad(w, [q, m], several, is_grads_batched=True), once):
+        assert (x[0].float() - y.float()).norm() <= 8e-3 * y.float().norm()
+        assert (x[1].float() + 2 * y.float()).norm() <= 16e-3 * y.float().norm()
