@@ -134,6 +134,13 @@ struct Launch {
   }
 };
 
+// Dual numbers of forward-mode differentiation, which no kernel here knows about.
+bool has_tangent(std::initializer_list<const Tensor*> ts) {
+  for (const Tensor* t : ts)
+    if (t->_fw_grad(0).defined()) return true;
+  return false;
+}
+
 Tensor inner_contiguous(const Tensor& t) { return t.stride(-1) == 1 ? t : t.contiguous(); }
 Tensor as_int32(const Tensor& t) { return (t.scalar_type() == at::kInt ? t : t.to(at::kInt)).contiguous(); }
 Tensor as_float(const Tensor& t) { return (t.scalar_type() == at::kFloat ? t : t.to(at::kFloat)).contiguous(); }
@@ -323,6 +330,7 @@ struct GcaBackward : public Node {
 // gca_indexed / attention: forward, recorded for autograd when a gradient can be asked for.
 Tensor gca_autograd(Tensor q, Tensor k, Tensor v, const Tensor& idx_in, const Tensor& w_in, double sm_scale, double off_by_one, int64_t algo,
                     bool gathered, bool token_major) {
+  TORCH_CHECK_NOT_IMPLEMENTED(!has_tangent({&q, &k, &v, &w_in}), "GCA has no forward-mode derivative");
   q = inner_contiguous(q);
   k = inner_contiguous(k);
   v = inner_contiguous(v);
@@ -1013,13 +1021,15 @@ ENTRY(linear, 5)
   return wrap(unlocked([&] { return linear(x, w, scale, residual, out); }));
 ENTRY_END
 
-// (q, landmarks, topk, noise or None, score_round) -> (indices[:, :-1], weights[:, :-1], keys, indices, scores, weights, n_valid)
+// (q, landmarks, topk, noise or None, score_round) -> (indices[:, :-1], weights[:, :-1], keys, indices, scores, weights, n_valid);
+// None when the landmarks carry tangents
 ENTRY(retrieve, 5)
   const Tensor &q = a.tensor(0), &k = a.tensor(1);
   TORCH_CHECK(q.is_cuda() && k.is_cuda(), "landmark retrieval runs on CUDA tensors only (there is no CPU path)");
   TORCH_CHECK_VALUE(q.dim() == 3 && k.dim() == 3 && q.size(0) == k.size(0) && q.size(2) == k.size(2), "expected lmk_q (N, Cq, D) and lmk_k (N, E, D)");
   const int64_t topk = a.integer(2), round = a.integer(4);
   const Tensor noise = a.maybe(3);
+  if (has_tangent({&q, &k})) Py_RETURN_NONE;
   const Retrieving r = unlocked([&] { return retrieve(q, k, topk, noise, round); });
   return wrap_tuple({r.indices, r.weights, r.full.keys, r.full.indices, r.full.scores, r.full.weights, r.full.n_valid});
 ENTRY_END

@@ -103,8 +103,10 @@ def retrieve(lmk_q: torch.Tensor, chunk_kvs, topk: int, *, training: bool = Fals
     wants_grad = lmk_q.requires_grad or past.requires_grad
     if not wants_grad or (lmk_q.dtype == past.dtype == torch.bfloat16):
         # bf16 landmarks: the scan's own scores are what the weights are made of, and their gradient is one kernel
-        idx, w, *full = _lib.host().retrieve(lmk_q, past, topk, noise, _SCORE_ROUND[score_round])
-        return idx, w, Retrieval(*full)
+        res = _lib.host().retrieve(lmk_q, past, topk, noise, _SCORE_ROUND[score_round])
+        if res is not None:                                  # None: forward-mode differentiation, left to torch's operations
+            idx, w, *full = res
+            return idx, w, Retrieval(*full)
     res = lmk_score_topk(lmk_q, past, topk, noise=noise, score_round=score_round)
     weights = differentiable_weights(lmk_q, past, res.indices)
     return res.indices[:, :-1], weights[:, :-1], res._replace(weights=weights)

@@ -446,3 +446,31 @@ def test_gradients_of_retrieval_weights_can_be_differentiated_and_batched(lcm):
     for x, y in zip(torch.autograd.grad(w, [q, m], several, is_grads_batched=True), once):
         assert (x[0].float() - y.float()).norm() <= 8e-3 * y.float().norm()
         assert (x[1].float() + 2 * y.float()).norm() <= 16e-3 * y.float().norm()
+
+
+def test_forward_mode_differentiation_is_followed_or_refused(lcm):
+    """Tangents of the landmarks reach the retrieval weights (against the backward pass: <dw, J t> = <J^T dw, t>); GCA, which has
+    no forward-mode derivative, refuses them instead of dropping them."""
+    import torch.autograd.forward_ad as fwd
+    (q, m, _, w, _), (qf, mf, wf, _) = _retrieve_with_float32_twin(lcm, 2, 9, 64, 4, 37)
+    g = torch.Generator().manual_seed(10)
+    tq, tm, probe = (torch.randn(x.shape, generator=g).cuda() for x in (q, m, w))
+    dq, dm = torch.autograd.grad(wf, [qf, mf], probe)
+    with fwd.dual_level():
+        dual_q, dual_m = fwd.make_dual(q, tq.bfloat16()), fwd.make_dual(m, tm.bfloat16())
+        _, dual_w, _ = lcm.retrieve(dual_q, type("Chunks", (), {"past_lmk_embeds": dual_m}), 4)
+        tangent = fwd.unpack_dual(dual_w).tangent.clone()
+        tangent[:, 0] = 0                                    # the first row sees no chunk: torch's tangent of a softmax over nothing is NaN
+        got, want = (tangent * probe).sum(), (dq * tq.bfloat16()).sum() + (dm * tm.bfloat16()).sum()
+        # bf16 scores on the way: 2^-9 of each of the tangent's contributions
+        size = ((dq * tq.bfloat16()).abs().sum() + (dm * tm.bfloat16()).abs().sum())
+        assert (got - want).abs() <= 2 ** -7 * size
+        x = torch.randn(2, 3, 4, 64, 64, generator=g).bfloat16().cuda()
+        kv = torch.randn(2, 5, 64, 256, generator=g).bfloat16().cuda()
+        ids, wt = torch.zeros(2, 3, 2, dtype=torch.int32, device="cuda"), torch.ones(2, 3, 2, device="cuda")
+        for args in ((fwd.make_dual(x, x), kv, kv, ids, wt), (x, kv, fwd.make_dual(kv, kv), ids, wt), (x, kv, kv, ids, fwd.make_dual(wt, wt))):
+            with pytest.raises(NotImplementedError):
+                lcm.gca_indexed(*args, 0.125)
+        cr = kv.view(2, 5, 64, 4, 64).permute(0, 3, 1, 2, 4)
+        with pytest.raises(NotImplementedError):
+            lcm.attention(x[:, 0], fwd.make_dual(cr, cr), cr, torch.ones(2, 5, device="cuda"), 0.125)
