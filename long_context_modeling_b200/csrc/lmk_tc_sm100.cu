@@ -10,7 +10,7 @@
 //   roundings of 2^-24 of sum |q_i k_i| <= |q| |k|; tensor cores align and truncate at 2^-22 or better per addition, 48 of
 //   them for D = 768.  The bound is ~8e-4 of the spread of the scores of one row, so it costs next to nothing.
 //   With T the K-th best approximate score of the row, whatever lies below T - 2 eps cannot win.  A range whose KC
-//   entries are all above that line may hide more (copies of one landmark): that row is scanned exactly by its warp.
+//   entries are all above that line may hide more (copies of one landmark): that row is scanned exactly by its block.
 //
 // Screening: one CTA per (128 rows, range of landmarks), tiles of 64 landmarks; warp 16 issues the TMA copies of a 4-stage ring
 // (128 x 64 of q, 64 x 64 of the landmarks), warp 17 the 128 x 64 x 16 MMAs; 16 worker warps add up the squared norms
@@ -18,6 +18,8 @@
 // per warp at a time.  Every wait is bounded; when one runs out the error bound of the block's rows is written as infinite, which
 // sends them through the exact scan.  What bounds it is latency (12 K steps, one selection round after another): 8 x 260 rows x 260
 // landmarks x 768 take ~15 us for both kernels, against 190 us for the row scan and its merge.
+#include <algorithm>
+
 #include "lmk_common.cuh"
 #include "sm100_ptx.cuh"
 #include "tma_host.cuh"
@@ -298,24 +300,41 @@ struct SettleParams {
   const float* noise;
   long long q_pos0;
   int KC, lists, E;
+  int rows;                      // of a block, one per warp
 };
 
 constexpr int SETTLE_WARPS = 8;
 
-// One warp per row: the candidates that can win get their exact scores and are put in order.
+// Four landmark rows against the query row a warp holds: the scan's own sums, every lane gets them.
 template <int NP>
-__global__ void __launch_bounds__(SETTLE_WARPS * 32)
-lmk_settle_kernel(const __grid_constant__ SettleParams p) {
-  __shared__ unsigned long long won_key[SETTLE_WARPS][32];
-  __shared__ float won_score[SETTLE_WARPS][32];
+__device__ __forceinline__ void exact_dot4(float s[4], const uint4 (&qv)[NP], const uint4 (&kv)[4][NP]) {
+#pragma unroll
+  for (int x = 0; x < 4; ++x) {
+    float acc = 0.f;
+#pragma unroll
+    for (int pp = 0; pp < NP; ++pp) {                      // absent pieces add 0 * 0: the sums never are -0
+      float af[8], bf[8];
+      unpack8(qv[pp], af);
+      unpack8(kv[x][pp], bf);
+#pragma unroll
+      for (int jj = 0; jj < 8; ++jj) acc = fmaf(af[jj], bf[jj], acc);
+    }
+#pragma unroll
+    for (int of = 16; of > 0; of >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, of);
+    s[x] = acc;
+  }
+}
+template <int NP>
+__device__ __forceinline__ void load_row(uint4 (&v)[NP], const __nv_bfloat16* src, int pieces, int lane) {
+#pragma unroll
+  for (int pp = 0; pp < NP; ++pp) v[pp] = lane + 32 * pp < pieces ? *reinterpret_cast<const uint4*>(src + (lane + 32 * pp) * 8) : make_uint4(0, 0, 0, 0);
+}
+
+// One warp: the candidates of a row that can win get their exact scores and are put in order.  False: the lists may hide a winner.
+template <int NP>
+__device__ __forceinline__ bool settle_row(const SettleParams& p, long long row, unsigned long long* won_key, float* won_score, int lane) {
   const FinalParams& f = p.fin;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const long long row = (long long)blockIdx.x * SETTLE_WARPS + warp;
-  pdl_trigger();
-  pdl_wait();
-  if (row >= f.R) return;
   const long long n = row / f.Cq, r = row % f.Cq;
-  const __nv_bfloat16* q = f.lq + n * f.qbs + r * f.qrs;
   const __nv_bfloat16* kb = f.lk + n * f.kbs;
   const int pieces = f.D >> 3;
   const unsigned long long* src = p.part + (row * p.lists + lane) * p.KC;
@@ -323,15 +342,15 @@ lmk_settle_kernel(const __grid_constant__ SettleParams p) {
   unsigned long long head = have ? src[0] : 0ull, next = have ? src[1] : 0ull, c0 = 0ull, c1 = 0ull;
   const unsigned eb = __reduce_max_sync(0xffffffffu, have ? __float_as_uint(p.eps[row * p.lists + lane]) : 0u);
   const float eps = __uint_as_float(eb);
-  bool slow = !(eps < 1e30f);
+  if (!(eps < 1e30f)) return false;
   float line = -INFINITY;
   int at = 1, count = 0;
-  while (!slow) {
+  for (;;) {
     const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(head >> 32));
     if (hi == 0u) break;
     const float s = from_orderable(hi);
     if (count >= f.K && s < line) break;
-    if (count == 64 || !(fabsf(s) < 1e30f)) { slow = true; break; }
+    if (count == 64 || !(fabsf(s) < 1e30f)) return false;
     const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(head >> 32) == hi ? (unsigned)head : 0u);
     const unsigned long long best = ((unsigned long long)hi << 32) | lo;
     if (lane == (count & 31)) { if (count < 32) c0 = best; else c1 = best; }
@@ -339,38 +358,13 @@ lmk_settle_kernel(const __grid_constant__ SettleParams p) {
     if (count == f.K) line = s - 2.001f * eps - fabsf(s) * 8.2e-6f;         // 2^-17: the bits a key leaves out; roundings of scale and noise
     bool spent = false;
     if (head == best) { head = next; ++at; next = at < p.KC ? src[at] : 0ull; spent = at > p.KC; }
-    slow = __any_sync(0xffffffffu, spent);                                   // a full list used up: it may hide more
-  }
-  const bool want_sel = p.noise != nullptr;
-  if (slow) {
-    unsigned long long m = 0ull, th = 0ull;
-    const long long seen = min((long long)p.E, p.q_pos0 + r - f.e_base);
-    for (long long e = 0; e < seen; ++e) {
-      float s = exact_dot(q, kb + e * f.krs, pieces, lane) * f.scale;
-      if (want_sel) s += p.noise[row * p.E + e];
-      const unsigned long long key = make_key(s, (unsigned)(f.e_base + e));
-      if (key > th) {
-        list_insert(m, key, lane);
-        th = __shfl_sync(0xffffffffu, m, f.K - 1);
-      }
-    }
-    float clean = from_orderable((unsigned)(m >> 32));
-    if (want_sel)
-      for (int i = 0; i < f.K; ++i) {
-        const unsigned long long key = __shfl_sync(0xffffffffu, m, i);
-        const long long e = key ? (long long)(0xffffffffu - (unsigned)key) - f.e_base : 0;
-        const float s = exact_dot(q, kb + e * f.krs, pieces, lane) * f.scale;
-        if (lane == i) clean = s;
-      }
-    emit_scored(f, row, m, clean, lane);
-    return;
+    if (__any_sync(0xffffffffu, spent)) return false;                        // a full list used up: it may hide more
   }
   // exact scores; the rows of four candidates are requested together
   unsigned long long k0 = 0ull, k1 = 0ull;
   float s0 = 0.f, s1 = 0.f;
   uint4 qv[NP];
-#pragma unroll
-  for (int pp = 0; pp < NP; ++pp) qv[pp] = lane + 32 * pp < pieces ? *reinterpret_cast<const uint4*>(q + (lane + 32 * pp) * 8) : make_uint4(0, 0, 0, 0);
+  load_row<NP>(qv, f.lq + n * f.qbs + r * f.qrs, pieces, lane);
   for (int i0 = 0; i0 < count; i0 += 4) {
     uint4 kv[4][NP];
     unsigned id[4];
@@ -378,28 +372,16 @@ lmk_settle_kernel(const __grid_constant__ SettleParams p) {
     for (int x = 0; x < 4; ++x) {
       const int i = min(i0 + x, count - 1);
       id[x] = 0xffffffffu - (unsigned)__shfl_sync(0xffffffffu, i < 32 ? c0 : c1, i & 31);
-      const __nv_bfloat16* kr = kb + ((long long)id[x] - f.e_base) * f.krs;
-#pragma unroll
-      for (int pp = 0; pp < NP; ++pp)
-        kv[x][pp] = lane + 32 * pp < pieces ? *reinterpret_cast<const uint4*>(kr + (lane + 32 * pp) * 8) : make_uint4(0, 0, 0, 0);
+      load_row<NP>(kv[x], kb + ((long long)id[x] - f.e_base) * f.krs, pieces, lane);
     }
+    float acc[4];
+    exact_dot4<NP>(acc, qv, kv);
 #pragma unroll
     for (int x = 0; x < 4; ++x) {
-      float acc = 0.f;
-#pragma unroll
-      for (int pp = 0; pp < NP; ++pp) {                      // absent pieces add 0 * 0: the sums never are -0
-        float af[8], bf[8];
-        unpack8(qv[pp], af);
-        unpack8(kv[x][pp], bf);
-#pragma unroll
-        for (int jj = 0; jj < 8; ++jj) acc = fmaf(af[jj], bf[jj], acc);
-      }
-#pragma unroll
-      for (int of = 16; of > 0; of >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, of);
-      const float s = acc * f.scale;
+      const float s = acc[x] * f.scale;
       const int i = i0 + x;
       if (i < count && lane == (i & 31)) {
-        const unsigned long long key = make_key(want_sel ? s + p.noise[row * p.E + (long long)id[x] - f.e_base] : s, id[x]);
+        const unsigned long long key = make_key(p.noise ? s + p.noise[row * p.E + (long long)id[x] - f.e_base] : s, id[x]);
         if (i < 32) { k0 = key; s0 = s; } else { k1 = key; s1 = s; }
       }
     }
@@ -410,12 +392,90 @@ lmk_settle_kernel(const __grid_constant__ SettleParams p) {
     r0 += o > k0;
     r1 += o > k1;
   }
-  won_key[warp][lane] = 0ull;
+  won_key[lane] = 0ull;
   __syncwarp();
-  if (k0 && r0 < 32) { won_key[warp][r0] = k0; won_score[warp][r0] = s0; }
-  if (k1 && r1 < 32) { won_key[warp][r1] = k1; won_score[warp][r1] = s1; }
+  if (k0 && r0 < 32) { won_key[r0] = k0; won_score[r0] = s0; }
+  if (k1 && r1 < 32) { won_key[r1] = k1; won_score[r1] = s1; }
   __syncwarp();
-  emit_scored(f, row, lane < f.K ? won_key[warp][lane] : 0ull, won_score[warp][lane], lane);
+  emit_scored(f, row, lane < f.K ? won_key[lane] : 0ull, won_score[lane], lane);
+  return true;
+}
+
+// A whole block: every landmark the row can see, exactly.  Warp w takes landmarks w, w + 8, ..., four of them in flight.
+template <int NP>
+__device__ __forceinline__ void scan_row(const SettleParams& p, long long row, unsigned long long (*list)[32], int warp, int lane) {
+  const FinalParams& f = p.fin;
+  const long long n = row / f.Cq, r = row % f.Cq, seen = min((long long)p.E, p.q_pos0 + r - f.e_base);
+  const __nv_bfloat16* kb = f.lk + n * f.kbs;
+  const int pieces = f.D >> 3;
+  uint4 qv[NP];
+  load_row<NP>(qv, f.lq + n * f.qbs + r * f.qrs, pieces, lane);
+  unsigned long long m = 0ull, th = 0ull;
+  for (long long e0 = warp; e0 < seen; e0 += 4 * SETTLE_WARPS) {
+    uint4 kv[4][NP];
+    float add[4], acc[4];
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      const long long e = min(e0 + x * SETTLE_WARPS, seen - 1);
+      load_row<NP>(kv[x], kb + e * f.krs, pieces, lane);
+      add[x] = p.noise ? p.noise[row * p.E + e] : 0.f;
+    }
+    exact_dot4<NP>(acc, qv, kv);
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      const long long e = e0 + x * SETTLE_WARPS;
+      float s = acc[x] * f.scale;
+      if (p.noise) s += add[x];
+      const unsigned long long key = make_key(s, (unsigned)(f.e_base + e));
+      if (e < seen && key > th) {
+        list_insert(m, key, lane);
+        th = __shfl_sync(0xffffffffu, m, f.K - 1);
+      }
+    }
+  }
+  list[warp][lane] = m;
+  __syncthreads();
+  if (warp == 0) {
+    for (int w = 1; w < SETTLE_WARPS; ++w)
+      for (int i = 0; i < f.K; ++i) {
+        const unsigned long long key = list[w][i];
+        if (key <= th) break;                              // lists are descending
+        list_insert(m, key, lane);
+        th = __shfl_sync(0xffffffffu, m, f.K - 1);
+      }
+    float clean = from_orderable((unsigned)(m >> 32));
+    if (p.noise)
+      for (int i = 0; i < f.K; ++i) {
+        const unsigned long long key = __shfl_sync(0xffffffffu, m, i);
+        const long long e = key ? (long long)(0xffffffffu - (unsigned)key) - f.e_base : 0;
+        const float s = exact_dot(f.lq + n * f.qbs + r * f.qrs, kb + e * f.krs, pieces, lane) * f.scale;
+        if (lane == i) clean = s;
+      }
+    emit_scored(f, row, m, clean, lane);
+  }
+  __syncthreads();
+}
+
+// One warp per row; rows whose lists may hide a winner -- more copies of a landmark, or rows of equal scores, than the lists hold -- are
+// then scanned by the whole block.  One warp scanning alone, a landmark at a time, was up to 33 times slower than the row scan that
+// this path replaces (64 rows x 16,384 landmarks x 768, all rows tied: 13.1 ms against 0.4; now 0.5.  2,080 x 2,080: 1.69 -> 0.67 ms, the row
+// scan takes 0.79; 256 x 65,536: 76.7 -> 2.9, 6.1; worst against it: 8 x 260 x 260 x 1,024, 183 us against 121).
+template <int NP>
+__global__ void __launch_bounds__(SETTLE_WARPS * 32)
+lmk_settle_kernel(const __grid_constant__ SettleParams p) {
+  __shared__ unsigned long long won_key[SETTLE_WARPS][32];
+  __shared__ float won_score[SETTLE_WARPS][32];
+  __shared__ int hidden[SETTLE_WARPS];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long first = (long long)blockIdx.x * p.rows, row = first + warp;
+  pdl_trigger();
+  pdl_wait();
+  bool settled = true;
+  if (warp < p.rows && row < p.fin.R) settled = settle_row<NP>(p, row, won_key[warp], won_score[warp], lane);
+  if (lane == 0) hidden[warp] = !settled;
+  if (__syncthreads_or(!settled))
+    for (int w = 0; w < p.rows; ++w)
+      if (hidden[w]) scan_row<NP>(p, first + w, won_key, warp, lane);
 }
 
 // Landmark ranges per row: enough CTAs to fill the GPU, at most one list per lane of the merging warp.
@@ -465,7 +525,9 @@ int launch_lmk_screen(const LmkTopkArgs& a, void* scratch, int sms, const FinalP
                                   stream, p));
   SettleParams sp;
   sp.fin = fin; sp.part = p.part; sp.eps = p.eps; sp.noise = a.noise; sp.q_pos0 = a.q_pos0; sp.KC = p.KC; sp.lists = p.lists; sp.E = a.E;
-  const dim3 grid((unsigned)((rows + SETTLE_WARPS - 1) / SETTLE_WARPS)), block(SETTLE_WARPS * 32);
+  // fewer rows than two blocks per SM have warps: blocks of fewer rows, which share a scan among more SMs
+  sp.rows = (int)std::min<size_t>(SETTLE_WARPS, (rows + 2 * sms - 1) / (2 * sms));
+  const dim3 grid((unsigned)((rows + sp.rows - 1) / sp.rows)), block(SETTLE_WARPS * 32);
   switch ((a.D + 255) / 256) {
     case 1: return (int)launch_dependent(lmk_settle_kernel<1>, grid, block, 0, stream, sp);
     case 2: return (int)launch_dependent(lmk_settle_kernel<2>, grid, block, 0, stream, sp);

@@ -474,3 +474,20 @@ def test_forward_mode_differentiation_is_followed_or_refused(lcm):
         cr = kv.view(2, 5, 64, 4, 64).permute(0, 3, 1, 2, 4)
         with pytest.raises(NotImplementedError):
             lcm.attention(x[:, 0], fwd.make_dual(cr, cr), cr, torch.ones(2, 5, device="cuda"), 0.125)
+
+
+@pytest.mark.parametrize("n,cq,e,d,k,noisy", [(1, 64, 700, 768, 8, False), (2, 65, 300, 1024, 28, False), (3, 200, 331, 64, 1, True),
+                                              (9, 70, 64, 448, 5, False)])
+def test_rows_that_the_block_scans(lcm, n, cq, e, d, k, noisy):
+    """Rows whose candidate lists may hide a winner: all scores equal (a zero row), half of the landmarks one landmark; one row per
+    block and several, rows that see fewer landmarks than a block has warps.  Bits of the row scan (``splits`` takes it)."""
+    lq, lk = cases.landmark_case(38, n, cq, e, d=d)
+    lq[:, ::3] = 0
+    lk[:, 1::2] = lk[:, 1:2]
+    noise = None
+    if noisy:                                                # ties in the noisy scores too
+        noise = torch.randint(0, 2, (n, cq, e), generator=torch.Generator().manual_seed(3)).float().cuda()
+    for q_pos0 in (0, max(0, e - cq)):
+        res, want = (lcm.lmk_score_topk(lq.cuda(), lk.cuda(), k, q_pos0=q_pos0, noise=noise, splits=s) for s in (0, 1))
+        for a, b in zip(res, want):
+            assert torch.equal(a, b)
