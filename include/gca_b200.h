@@ -233,6 +233,10 @@ typedef struct LmkTopkArgs {
 int lmk_score_topk(const LmkTopkArgs* args, void* stream);
 size_t lmk_topk_workspace_bytes(const LmkTopkArgs* args);
 
+/* lmk_score_topk that writes the indices and weights a second time, for a backward pass that must not see what becomes of
+ * out_indices and out_weights: kept_indices, kept_weights laid out like those, both or neither NULL. */
+int lmk_score_topk_kept(const LmkTopkArgs* args, int32_t* kept_indices, float* kept_weights, void* stream);
+
 /*
  * Gradient of the retrieval weights into the landmarks: what autograd does behind
  * `softmax(scores.gather(...))` of model/DRT.py:626 (einsum backward, gather backward, index_put with

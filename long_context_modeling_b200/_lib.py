@@ -177,6 +177,7 @@ EXPORTS = {
     "gca_bwd_workspace_bytes": (C.c_size_t, [C.POINTER(GcaBwdArgs)]),
     "gca_bwd_stages": (C.c_int, [C.POINTER(GcaBwdArgs), C.c_uint, C.c_void_p]),
     "lmk_score_topk": (C.c_int, [C.POINTER(LmkTopkArgs), C.c_void_p]),
+    "lmk_score_topk_kept": (C.c_int, [C.POINTER(LmkTopkArgs), C.c_void_p, C.c_void_p, C.c_void_p]),
     "lmk_topk_workspace_bytes": (C.c_size_t, [C.POINTER(LmkTopkArgs)]),
     "lmk_score_topk_static": (C.c_int, [C.POINTER(LmkTopkArgs), C.c_void_p]),
     "lmk_weights_backward": (C.c_int, [C.POINTER(LmkGradArgs), C.c_void_p]),

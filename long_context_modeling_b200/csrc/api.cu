@@ -5,7 +5,7 @@
 
 namespace gca {
 int launch_decode(const GcaFwdArgs& a, int sms, cudaStream_t stream);
-int launch_lmk_score_topk(const LmkTopkArgs& a, void* scratch, int sms, cudaStream_t stream);
+int launch_lmk_score_topk(const LmkTopkArgs& a, void* scratch, int sms, cudaStream_t stream, int32_t* kept_indices, float* kept_weights);
 int launch_lmk_grad(const LmkGradArgs& a, cudaStream_t stream);
 int launch_lmk_merge(const LmkMergeArgs& a, cudaStream_t stream);
 size_t lmk_topk_workspace_bytes_impl(const LmkTopkArgs& a, int sms);
@@ -275,17 +275,20 @@ size_t lmk_topk_workspace_bytes(const LmkTopkArgs* a) {
   return gca::lmk_topk_workspace_bytes_impl(*a, scope.rc ? 256 : gca::sm_count(scope.dev));
 }
 
-int lmk_score_topk(const LmkTopkArgs* a, void* stream) {
+int lmk_score_topk(const LmkTopkArgs* a, void* stream) { return lmk_score_topk_kept(a, nullptr, nullptr, stream); }
+
+int lmk_score_topk_kept(const LmkTopkArgs* a, int32_t* kept_indices, float* kept_weights, void* stream) {
   int rc = gca::check_topk(a);
   if (rc) return rc;
   if (a->N == 0 || a->Cq == 0) return 0;
   if (!a->workspace) return GCA_ERR_WORKSPACE;
+  if (!kept_indices != !kept_weights) return GCA_ERR_NULL;
   gca::DeviceScope scope(a->lmk_k);
   if (scope.rc) return scope.rc;
   const int sms = gca::sm_count(scope.dev);
   const size_t need = gca::lmk_topk_workspace_bytes_impl(*a, sms);
   if (a->workspace_bytes < need) return GCA_ERR_WORKSPACE;
-  return gca::launch_lmk_score_topk(*a, a->workspace, sms, (cudaStream_t)stream);
+  return gca::launch_lmk_score_topk(*a, a->workspace, sms, (cudaStream_t)stream, kept_indices, kept_weights);
 }
 
 int gca_layer_decode(const LayerDecodeArgs* a, void* stream) {

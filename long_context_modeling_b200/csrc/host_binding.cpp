@@ -50,7 +50,7 @@ struct Api {
 #define GCA_API(name) decltype(&::name) name = nullptr;
 #define GCA_API_LIST                                                                                          \
   GCA_API(gca_fwd) GCA_API(gca_decode) GCA_API(gca_bwd_stages) GCA_API(gca_bwd_workspace_bytes)               \
-  GCA_API(lmk_score_topk) GCA_API(lmk_topk_workspace_bytes) GCA_API(lmk_weights_backward) GCA_API(gca_kv_project_append) GCA_API(gca_row_rms) \
+  GCA_API(lmk_score_topk_kept) GCA_API(lmk_topk_workspace_bytes) GCA_API(lmk_weights_backward) GCA_API(gca_kv_project_append) GCA_API(gca_row_rms) \
   GCA_API(gca_linear) GCA_API(gca_linear_batched) GCA_API(gca_linear_few_rows) GCA_API(gca_layer_decode) GCA_API(gca_silu_mul) GCA_API(gca_window_decode)            \
   GCA_API(gca_window_ring_decode) GCA_API(gca_strerror)
   GCA_API_LIST
@@ -686,9 +686,9 @@ Tensor carve(const c10::Storage& st, size_t byte_offset, at::IntArrayRef sizes, 
 }
 
 struct Retrieved { Tensor keys, indices, scores, weights, n_valid; };
-struct Selection { Tensor indices, weights; };       // a copy of the selection that the caller never sees
+struct Selection { Tensor indices, weights; };       // a selection that the caller never sees
 
-// `kept`: the selection is copied for a backward pass, which the caller's in-place changes to its own tensors must not reach.
+// `kept`: the selection is written twice, for a backward pass that the caller's in-place changes to its own tensors must not reach.
 Retrieved score_topk(const Tensor& q_in, const Tensor& k_in, int64_t topk, bool has_pos0, int64_t q_pos0, int64_t e_base, const Tensor& noise_in,
                      int64_t head_dim, int64_t score_round, int64_t splits, Selection* kept = nullptr) {
   at::AutoDispatchBelowADInplaceOrView below;
@@ -701,14 +701,13 @@ Retrieved score_topk(const Tensor& q_in, const Tensor& k_in, int64_t topk, bool 
   const c10::SmallVector<int64_t, 4> row_shape = shape;
   shape.push_back(topk);
   const int64_t m = rows * topk;
-  // the selection lies together, so that one copy keeps it
   const Tensor block = at::empty({m * (kept ? 28 : 20) + rows * 4}, q.options().dtype(at::kByte));
   const c10::Storage& st = block.storage();
   Retrieved r;
   r.keys = carve(st, 0, shape, at::kLong);
   r.indices = carve(st, (size_t)m * 8, shape, at::kInt);
-  r.weights = carve(st, (size_t)m * 12, shape, at::kFloat);
-  r.scores = carve(st, (size_t)m * 16, shape, at::kFloat);
+  r.scores = carve(st, (size_t)m * 12, shape, at::kFloat);
+  r.weights = carve(st, (size_t)m * 16, shape, at::kFloat);
   r.n_valid = carve(st, (size_t)m * 20, row_shape, at::kInt);
   if (kept) {
     const size_t at = (size_t)m * 20 + (size_t)rows * 4;
@@ -734,10 +733,10 @@ Retrieved score_topk(const Tensor& q_in, const Tensor& k_in, int64_t topk, bool 
   const size_t need = api.lmk_topk_workspace_bytes(&a);
   const Tensor ws = at::empty({(int64_t)(need > 16 ? need : 16)}, q.options().dtype(at::kByte));
   a.workspace = ws.mutable_data_ptr(); a.workspace_bytes = need;
-  call("lmk_score_topk", [&] { return api.lmk_score_topk(&a, on.stream); });
-  if (kept)
-    C10_CUDA_CHECK(cudaMemcpyAsync(kept->indices.mutable_data_ptr(), r.indices.const_data_ptr(), (size_t)m * 8, cudaMemcpyDeviceToDevice,
-                                   static_cast<cudaStream_t>(on.stream)));
+  call("lmk_score_topk", [&] {
+    return api.lmk_score_topk_kept(&a, kept ? kept->indices.mutable_data_ptr<int32_t>() : nullptr,
+                                   kept ? kept->weights.mutable_data_ptr<float>() : nullptr, on.stream);
+  });
   return r;
 }
 

@@ -41,6 +41,8 @@ struct FinalParams {
   float* out_scores;
   float* out_weights;
   int32_t* out_nvalid;
+  int32_t* kept_indices = nullptr;  // a second copy of indices and weights, or nullptr
+  float* kept_weights = nullptr;
   // optional recompute of noise-free scores (per-sequence mode with noise)
   const __nv_bfloat16* lq;
   const __nv_bfloat16* lk;
@@ -87,6 +89,7 @@ __device__ __forceinline__ void emit_scored(const FinalParams& p, long long row,
     if (p.out_indices) p.out_indices[o] = idx;
     if (p.out_scores) p.out_scores[o] = score;
     if (p.out_weights) p.out_weights[o] = wgt;
+    if (p.kept_indices) { p.kept_indices[o] = idx; p.kept_weights[o] = wgt; }
   }
   if (lane == 0 && p.out_nvalid) p.out_nvalid[row] = (int)nv;
 }

@@ -591,7 +591,7 @@ size_t lmk_topk_workspace_bytes_impl(const LmkTopkArgs& a, int sms) {
 
 // Scan + merge on caller-provided scratch.  `scratch` must hold
 // lmk_topk_workspace_bytes_impl(a, sms) bytes.
-int launch_lmk_score_topk(const LmkTopkArgs& a, void* scratch, int sms, cudaStream_t stream) {
+int launch_lmk_score_topk(const LmkTopkArgs& a, void* scratch, int sms, cudaStream_t stream, int32_t* kept_indices, float* kept_weights) {
   const size_t rows = lmk_topk_rows(a);
   if (rows == 0) return 0;
   const bool per_head = a.head_dim > 0;
@@ -599,6 +599,7 @@ int launch_lmk_score_topk(const LmkTopkArgs& a, void* scratch, int sms, cudaStre
   FinalParams fp;
   fp.keys = (unsigned long long*)scratch; fp.out_keys = (unsigned long long*)a.out_keys; fp.out_indices = a.out_indices;
   fp.out_scores = a.out_scores; fp.out_weights = a.out_weights; fp.out_nvalid = a.out_nvalid;
+  fp.kept_indices = kept_indices; fp.kept_weights = kept_weights;
   fp.lq = (const __nv_bfloat16*)a.lmk_q; fp.lk = (const __nv_bfloat16*)a.lmk_k;
   fp.qbs = a.q_batch_stride; fp.qrs = a.q_row_stride; fp.kbs = a.k_batch_stride; fp.krs = a.k_row_stride; fp.e_base = a.e_base;
   fp.Cq = a.Cq; fp.D = a.D; fp.score_round = a.score_round; fp.scale = scale;
@@ -713,7 +714,7 @@ extern "C" int lmk_score_topk_static(const LmkTopkArgs* a, void* stream) {
   void* scratch = nullptr;
   rc = gca::static_scratch_ptr(scope.dev, &scratch);
   if (rc) return rc;
-  return gca::launch_lmk_score_topk(*a, scratch, sms, (cudaStream_t)stream);
+  return gca::launch_lmk_score_topk(*a, scratch, sms, (cudaStream_t)stream, nullptr, nullptr);
 }
 
 // ---------------------------------------------------------------------------------------------
