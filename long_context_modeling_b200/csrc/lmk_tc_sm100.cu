@@ -256,10 +256,11 @@ lmk_screen_kernel(const __grid_constant__ ScreenParams p) {
 #pragma unroll
       for (int i = 0; i < LEN; ++i) key[i] = max(key[i], x2[(LEN - 1 - i) * BM + r]);
       bitonic_merge<LEN>(key);
-      const float kn = fmaxf(norm[BM + lane], norm[BM + 32 + lane]);
-      const float kmax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(kn)));     // squared norms: never negative
+      // squared norms are never negative: as whole numbers they are in order, and a NaN is above them all
+      const float kmax = __uint_as_float(__reduce_max_sync(0xffffffffu, max(__float_as_uint(norm[BM + lane]), __float_as_uint(norm[BM + 32 + lane]))));
       if (live) {
-        eps_max = fmaxf(eps_max, BOUND * p.scale * sqrtf(norm[r]) * sqrtf(kmax) * 1.001f);
+        const float bound = BOUND * p.scale * sqrtf(norm[r]) * sqrtf(kmax) * 1.001f;
+        eps_max = fmaxf(eps_max, bound < 1e30f ? bound : INFINITY);      // NaN too: nothing is known about the tile, the row is scanned
         auto entry = [&](unsigned k) {
           return k ? (unsigned long long)(k & ~63u) << 32 | (0xffffffffu - (unsigned)(p.e_base + t * BN + (BN - 1) - (int)(k & 63u))) : 0ull;
         };

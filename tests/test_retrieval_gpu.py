@@ -491,3 +491,25 @@ def test_rows_that_the_block_scans(lcm, n, cq, e, d, k, noisy):
         res, want = (lcm.lmk_score_topk(lq.cuda(), lk.cuda(), k, q_pos0=q_pos0, noise=noise, splits=s) for s in (0, 1))
         for a, b in zip(res, want):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("where", ["landmark", "query", "noise"])
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), -float("inf")])
+def test_screening_with_values_that_are_not_finite(lcm, where, value):
+    """NaN and infinities in a landmark (seen by some rows, and in the same tile as landmarks that others see), in a query row, in
+    the noise: keys, ids and scores of the row scan (``splits`` takes it)."""
+    lq, lk = cases.landmark_case(39, 2, 80, 300, d=128)
+    noise = torch.zeros(2, 80, 300)
+    lk[:, 200:240] *= 2.0 ** 12                              # the largest norms share the tile with the value
+    lk[:, 205:240] = lk[:, 200:201]                          # and tie
+    if where == "landmark":
+        lk[0, 250, 5] = value
+    elif where == "query":
+        lq[1, 3, 7] = value
+    else:
+        noise[0, 5, 100] = noise[1, 60, 3] = value
+    args = dict(q_pos0=205, noise=noise.cuda() if where == "noise" else None)
+    res, want = (lcm.lmk_score_topk(lq.cuda(), lk.cuda(), 8, splits=s, **args) for s in (0, 1))
+    assert torch.equal(res.keys, want.keys) and torch.equal(res.indices, want.indices) and torch.equal(res.n_valid, want.n_valid)
+    for a, b in ((res.scores, want.scores), (res.weights, want.weights)):
+        assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.nan_to_num(7.0), b.nan_to_num(7.0))
