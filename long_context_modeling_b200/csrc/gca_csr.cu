@@ -38,19 +38,15 @@ __device__ __forceinline__ long long csr_lower_bound(const unsigned long long* _
   return lo;
 }
 
-// offsets[c] = first sorted key of chunk c (or the end).  The same thread also emits the chunk's
-// entry of the kv-major walking order: key = sequence (by_count: 0) << cbits | (cmax - count), so that an
+// A thread emits a chunk's entry of the kv-major walking order: key = sequence (by_count: 0) << cbits | (cmax - count), so that an
 // ascending sort lists a sequence's (all) chunks by decreasing number of retrievers; value =
 // (first entry, one past the last, chunk id): what the kv-major kernel reads per unit.
-__global__ void csr_offsets_kernel(const unsigned long long* __restrict__ sorted, int* __restrict__ offsets, int* __restrict__ tickets,
-                                   unsigned* __restrict__ ukeys, int4* __restrict__ uvals,
-                                   long long total, long long NC, int C, int cbits, unsigned cmax, bool by_count) {
+__global__ void csr_units_kernel(const unsigned long long* __restrict__ sorted, int* __restrict__ tickets, unsigned* __restrict__ ukeys,
+                                 int4* __restrict__ uvals, long long total, long long NC, int C, int cbits, unsigned cmax, bool by_count) {
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c > NC) return;
   if (c < 2) tickets[c] = 0;
+  if (c >= NC) return;
   const long long lo = csr_lower_bound(sorted, total, (unsigned long long)c << 32);
-  offsets[c] = (int)lo;
-  if (c == NC) return;
   const unsigned cnt = (unsigned)(csr_lower_bound(sorted, total, (unsigned long long)(c + 1) << 32) - lo);
   ukeys[c] = (by_count ? 0u : (unsigned)(c / C) << cbits) | (cmax - (cnt < cmax ? cnt : cmax));
   uvals[c] = make_int4((int)lo, (int)lo + (int)cnt, (int)c, 0);
@@ -181,7 +177,7 @@ int bits_for(long long v) {       // smallest b with 2^b > v
 size_t csr_workspace_bytes(int N, int J, int K, int C) {
   const long long total = (long long)N * J * K;
   const long long NC = (long long)N * C;
-  return align_up(total * 8, 256) * 2 + align_up((NC + 1) * 4, 256) + align_up(cub_temp_bytes(total), 256) +
+  return align_up(total * 8, 256) * 2 + align_up(cub_temp_bytes(total), 256) +
          align_up(NC * 4, 256) * 2 + align_up(NC * 16, 256) * 2 + align_up(cub_pairs_temp_bytes(NC), 256) + 256;
 }
 
@@ -195,7 +191,6 @@ int build_csr(const int32_t* indices, int N, int J, int K, int C, void* workspac
   char* p = (char*)workspace;
   unsigned long long* keys_in = (unsigned long long*)p;  p += align_up(total * 8, 256);
   unsigned long long* keys_out = (unsigned long long*)p; p += align_up(total * 8, 256);
-  int* offsets = (int*)p;                                p += align_up((NC + 1) * 4, 256);
   size_t temp = cub_temp_bytes(total);
   void* temp_ptr = p;                                    p += align_up(temp, 256);
   unsigned* ukeys_in = (unsigned*)p;                     p += align_up(NC * 4, 256);
@@ -230,8 +225,8 @@ int build_csr(const int32_t* indices, int N, int J, int K, int C, void* workspac
       GCA_CUDA_CHECK(cub::DeviceRadixSort::SortKeys(temp_ptr, temp, keys_in, keys_out, (int)total, 32, end_bit, stream));
     }
     if (NC > 0) {
-      csr_offsets_kernel<<<(unsigned)((NC + 1 + 255) / 256), 256, 0, stream>>>(keys_out, offsets, tickets, ukeys_in, uvals_in, total,
-                                                                               NC, C, cbits, (unsigned)cmax, by_count);
+      csr_units_kernel<<<(unsigned)((NC + 255) / 256), 256, 0, stream>>>(keys_out, tickets, ukeys_in, uvals_in, total, NC, C, cbits,
+                                                                         (unsigned)cmax, by_count);
       GCA_CUDA_CHECK(cudaGetLastError());
       GCA_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(utemp_ptr, utemp, ukeys_in, ukeys_out, uvals_in, uvals_out, (int)NC, 0,
                                                      cbits + nbits, stream));
