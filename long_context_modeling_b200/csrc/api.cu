@@ -269,10 +269,10 @@ extern "C" {
 
 size_t lmk_topk_workspace_bytes(const LmkTopkArgs* a) {
   if (gca::check_topk(a)) return 0;
-  // A size query must not fail for lack of a device: when the landmark pointer cannot be
-  // attributed to one, 256 SMs are assumed, which can only over-estimate (more SMs = more splits).
+  // A size query must not fail for lack of a device: when the landmark pointer cannot be attributed to one, the answer
+  // holds for any of up to 256 SMs.
   gca::DeviceScope scope(a->lmk_k);
-  return gca::lmk_topk_workspace_bytes_impl(*a, scope.rc ? 256 : gca::sm_count(scope.dev));
+  return gca::lmk_topk_workspace_bytes_impl(*a, scope.rc ? 0 : gca::sm_count(scope.dev));
 }
 
 int lmk_score_topk(const LmkTopkArgs* a, void* stream) { return lmk_score_topk_kept(a, nullptr, nullptr, stream); }

@@ -545,9 +545,10 @@ namespace {
 
 // Landmark ranges of the streaming form: one block per SM at a time, so what counts is whole waves; a block costs about as much
 // again as reading 96 rows before and after its stream.
+int most_stream_splits(const LmkTopkArgs& a, int sms) { return (int)std::min<long long>((a.E + BATCH - 1) / BATCH, 2 * sms); }
 int stream_splits(const LmkTopkArgs& a, int sms) {
   const long long blocks = (long long)a.N * a.Cq;
-  const int most = (int)std::min<long long>((a.E + BATCH - 1) / BATCH, 2 * sms);
+  const int most = most_stream_splits(a, sms);
   int best = 1;
   long long best_cost = -1;
   for (int s = 1; s <= most; ++s) {
@@ -584,9 +585,13 @@ size_t lmk_topk_rows(const LmkTopkArgs& a) {
   return (size_t)a.N * a.Cq * H;
 }
 
+// sms = 0: what any device of up to 256 SMs needs.  Screening and the row scan take more lists the more SMs there are; the streaming
+// form does not (5 rows x 262,144: 59 lists for 148 SMs, 51 for 256), so there the most it tries counts.
 size_t lmk_topk_workspace_bytes_impl(const LmkTopkArgs& a, int sms) {
-  if (lmk_screen_applies(a)) return lmk_screen_workspace_bytes(a, sms);
-  return align_up(lmk_topk_rows(a) * (size_t)choose_splits(a, sms) * a.K * sizeof(unsigned long long), 256);
+  const int assumed = sms > 0 ? sms : 256;
+  if (lmk_screen_applies(a)) return lmk_screen_workspace_bytes(a, assumed);
+  const int splits = sms == 0 && a.splits == 0 && pick_tq(a) == 1 ? std::max(1, most_stream_splits(a, assumed)) : choose_splits(a, assumed);
+  return align_up(lmk_topk_rows(a) * (size_t)splits * a.K * sizeof(unsigned long long), 256);
 }
 
 // Scan + merge on caller-provided scratch.  `scratch` must hold

@@ -300,6 +300,25 @@ def test_nvtx_switch_and_call_helper(lib):
         lib.call("gca_linear", None, None)
 
 
+@pytest.mark.parametrize("n,e,head_dim", [(5, 262144, 0), (8, 65536, 0), (14, 65536, 64), (1, 100, 0), (3, 0, 0), (9, 262144, 0)])
+def test_workspace_query_without_a_device_is_enough_for_any(lib, n, e, head_dim):
+    """Landmark pointers that belong to no device: the size covers the lists that devices of up to 256 SMs take (the streaming form
+    tries every split count and takes the cheapest: blocks in waves x (rows of a block + 96))."""
+    if torch.cuda.is_available():
+        pytest.skip("a machine without a GPU is meant")
+    t = lib.LmkTopkArgs()
+    t.lmk_q = t.lmk_k = t.out_keys = 0x10000
+    t.N, t.Cq, t.E, t.D, t.K, t.head_dim = n, 1, e, 768, 8, head_dim
+    t.q_row_stride = t.k_row_stride = t.q_batch_stride = 768
+    t.k_batch_stride = 768 * e
+    got = lib.lib().lmk_topk_workspace_bytes(C.byref(t))
+    rows = n * (768 // head_dim if head_dim else 1)
+    for sms in (1, 64, 132, 148, 160, 256):
+        splits = range(1, min(-(-e // 64), 2 * sms) + 1)
+        best = min(splits, key=lambda s: (-(-n * s // sms) * (-(-e // s) + 96), s), default=1)
+        assert got >= rows * best * 8 * 8
+
+
 PER_DEVICE_PROGRAM = r"""
 #include <cstdio>
 #include <thread>
