@@ -294,7 +294,7 @@ kv_project_append_kernel(const __grid_constant__ ProjParams p) {
       const __nv_bfloat16* res = nullptr;
       float sc = 1.0f;
       bool zero = false;
-      int cols = BN;
+      const int cols = min(BN, p.ncols - tn * BN);       // 192 does not divide every width: the last tile is a narrow one
       if (p.nmat == 1) {
         const int block = (C::TM / 64) * tm + 2 * (int)rank + (row_in_tile >> 6), b = block / p.blocks_per_batch;
         m = (block - b * p.blocks_per_batch) * 64 + (row_in_tile & 63);
@@ -302,7 +302,6 @@ kv_project_append_kernel(const __grid_constant__ ProjParams p) {
         if (live && p.row_scale) sc = p.row_scale[b * p.scale_bs + m];
         dst = p.out + b * p.out_bs + m * p.out_stride + tn * BN;
         if (live && p.residual) res = p.residual + b * p.res_bs + m * p.res_stride + tn * BN;
-        cols = min(BN, p.ncols - tn * BN);
       } else {
         const int n = live ? (int)(m / p.rows_per_seq) : 0;
         const int r = live ? (int)(m - (long long)n * p.rows_per_seq) : 0;       // (chunk, row) inside the appended block

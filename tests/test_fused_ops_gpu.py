@@ -398,6 +398,33 @@ def test_projection_append_tile_widths(n, c, dim):
     assert torch.equal(cache.past_lmk_embeds, torch.cat([x[:, :1, -1], x[:, :, -1]], 1))
 
 
+@pytest.mark.parametrize("n,c,dim", [(1, 40, 512), (3, 32, 512), (2, 12, 1024), (1, 45, 1024), (1, 17, 1280), (5, 61, 768), (1, 2, 256)])
+def test_projection_append_stays_in_its_rows_and_chunks(n, c, dim):
+    """Widths that the column tile does not divide: the last tile must not run on into the next row (the tile that has those
+    columns writes them at the same time) or past the appended chunks.  Chunks before and behind keep their contents; launches that
+    follow each other into the same cache leave the bits of the last one."""
+    need_gpu()
+    from long_context_modeling_b200 import _lib
+    g = torch.Generator(device="cuda").manual_seed(dim + c)
+    xs = [torch.randn(n, c, 64, dim, generator=g, device="cuda").bfloat16() for _ in range(2)]
+    wk, wv = ((torch.randn(dim, dim, generator=g, device="cuda") * dim ** -0.5).bfloat16() for _ in range(2))
+    k, v = (torch.full((n, c + 2, 64, dim), 7.0, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    lmk = torch.full((n, c + 2, dim), 7.0, dtype=torch.bfloat16, device="cuda")
+    refs = [[(x.float() @ w.float().t()) for w in (wk, wv)] for x in xs]
+    bits = [None, None]
+    for i in range(12):
+        for _ in range(3):
+            _lib.host().kv_project_append(xs[1 - i % 2], wk, wv, k, v, lmk, 1, c + 2, False)
+        _lib.host().kv_project_append(xs[i % 2], wk, wv, k, v, lmk, 1, c + 2, False)
+        for got, ref in zip((k, v), refs[i % 2]):
+            assert (got[:, 1:c + 1].float() - ref).abs().max() <= 2e-2 * ref.abs().max()
+            assert (got[:, 0] == 7).all() and (got[:, c + 1:] == 7).all()
+        assert torch.equal(lmk[:, 1:c + 1], xs[i % 2][:, :, -1]) and (lmk[:, 0] == 7).all() and (lmk[:, c + 1:] == 7).all()
+        now = [k.clone(), v.clone()]
+        bits[i % 2] = bits[i % 2] or now
+        assert all(torch.equal(a, b) for a, b in zip(now, bits[i % 2]))
+
+
 @pytest.mark.parametrize("m,n,k,few", [(16, 16576, 64, True), (16, 16592, 64, False), (32, 9472, 64, True), (32, 9488, 64, False),
                                        (64, 3552, 128, True), (64, 3568, 128, False), (128, 2304, 768, False), (96, 3072, 1024, False)])
 def test_few_row_form_on_both_sides_of_its_line(m, n, k, few):
