@@ -17,10 +17,11 @@
 // (GCA_STATUS_TIMEOUT on expiry).
 // Tiles (chosen by choose_tile): PAIRS of CTAs on 256 x 256 (cta_group::2) for large products, where each CTA loads half of the
 // weight rows: per product a third less shared-memory and L2 traffic than 128 x 256, and power is what a large
-// product is bound by (SM clock 1.3-1.6 GHz of 1.97 within milliseconds).  8 x 260 chunks x 64 rows, 768 -> 2 x 768: 307 -> 287 us
-// back to back, 255 -> 231 us for a single launch; cuBLAS needs 298 / 266 us for the bare product.  Smaller products take the width of 64,
-// 128 or 256 columns whose waves cost least: 6,912 rows 768 -> 768 on 148 SMs are 162 tiles of 256 columns (two
-// waves, the second nearly empty) but 324 of 128: 33 -> 19 us.
+// product is bound by (SM clock 1.3-1.6 GHz of 1.97 within milliseconds).  8 x 260 chunks x 64 rows, 768 -> 2 x 768, as the call with the
+// allocation of its cache: 252 us after a rest, 289 in a row; cuBLAS, in the same run, 285 / 294 us for the bare product (with
+// 128 x 256 tiles in place of pairs the call took 7 % more).  Smaller products take the width of 64, 128, 192 or 256 columns
+// whose waves cost least: 6,912 rows 768 -> 768 on 148 SMs are 162 tiles of 256 columns (two waves, the second nearly
+// empty) but 216 of 192: 33 -> 19 us.
 //
 // The same kernel in LINEAR mode is the projection either side of GCA (model/DRT.py:352-355,385):
 //   out[m, :] = row_scale[m] * (x[m, :] W^T) + residual[m, :]

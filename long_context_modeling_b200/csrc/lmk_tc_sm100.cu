@@ -12,12 +12,13 @@
 //   With T the K-th best approximate score of the row, whatever lies below T - 2 eps cannot win.  A range whose KC
 //   entries are all above that line may hide more (copies of one landmark): that row is scanned exactly by its block.
 //
-// Screening: one CTA per (128 rows, range of landmarks), tiles of 64 landmarks; warp 16 issues the TMA copies of a 4-stage ring
-// (128 x 64 of q, 64 x 64 of the landmarks), warp 17 the 128 x 64 x 16 MMAs; 16 worker warps add up the squared norms
-// from the same stages while they pass, then take the tile from tensor memory and select with warp-wide maxima, one row
-// per warp at a time.  Every wait is bounded; when one runs out the error bound of the block's rows is written as infinite, which
-// sends them through the exact scan.  What bounds it is latency (12 K steps, one selection round after another): 8 x 260 rows x 260
-// landmarks x 768 take ~15 us for both kernels, against 190 us for the row scan and its merge.
+// Screening: one CTA per (128 rows, range of landmarks), tiles of 64 landmarks; warp 16 issues the TMA copies of a 7-stage ring
+// (128 x 64 of q, 64 x 64 of the landmarks), warp 17 the 128 x 64 x 16 MMAs.  Of 16 worker warps the first six add up the squared norms
+// from the same stages while they pass; then a thread takes 16 scores of one row from tensor memory and sorts them in its
+// registers, and the four runs of a row are merged in two steps through shared memory, the last with the row's list so far.
+// Every wait is bounded; when one runs out the error bound of the block's rows is written as infinite, which sends them through the
+// exact scan.  What bounds it is latency (12 K steps, one selection round after another): 8 x 260 rows x 260 landmarks x 768
+// take 15 us of screening and 14 of settling (each by itself, cold), 31 us as a call; the row scan and its merge 142.
 #include <algorithm>
 
 #include "lmk_common.cuh"

@@ -95,7 +95,8 @@ __device__ __forceinline__ void select_batch(unsigned long long& mine, unsigned 
 // memory; list l (one per head, or the only one) is kept by warp l % 16, which looks at the 64 scores with two
 // votes and inserts what beats its K-th entry: one list per block instead of one per warp to merge at the end, and
 // no list code in the scoring loop (per head it was 12 lists in every warp, each with a serial insertion: 60 us for
-// 2 x 16,411 landmarks, now 16; 262,144 landmarks, one list: 68 -> 63 us = 6.3 TB/s).
+// 2 x 16,411 landmarks, now 16; 262,144 landmarks, one list: 68 -> 63 us = 6.3 TB/s for the scan alone, 69.4 us = 5.8 TB/s with its
+// merge).
 constexpr int BATCH = 64, STREAM_WARPS = 16;
 template <int NP> constexpr int RING_ROWS = NP > 3 ? 6 : 8;       // 196 KB per SM
 

@@ -499,10 +499,11 @@ class GraphedDecoder:
         head = FO.fold_gain(self.model.embed_tokens.weight.detach(), self.model.norm.weight.detach())
         self.lm_w = F.pad(head, (0, 0, 0, -head.shape[0] % 64))
 
-    # With few rows (a decode step has one per sequence) the library's 128 x 256-tile GEMM keeps only a
-    # handful of CTAs busy, so below SMALL_M rows the products go to cuBLAS (whose small-M kernels split
-    # the work finer) and the fusion that remains is algebraic: one q|k|v and one gate|up product with
-    # the norm's gain folded into the weights, 1 / rms applied to the product's rows.
+    # With few rows (a decode step has one per sequence) the products go to cuBLAS, below SMALL_M rows, and the
+    # fusion that remains is algebraic: one q|k|v and one gate|up product with the norm's gain folded into the
+    # weights, 1 / rms applied to the product's rows.  The line was drawn when the library had 128 x 256 tiles
+    # only; its latency-bound form for few rows (gca_linear_few_rows) and the sub-layer as one launch
+    # (forward_fused) came later and have not been measured against cuBLAS in this loop.
     SMALL_M = 128
 
     def _norm_linear(self, x2, folded_w, eps):
