@@ -18,7 +18,7 @@ LIB = os.path.join(HERE, "libgca_b200.so")
 HOST_SOURCE = os.path.join(CSRC, "host_binding.cpp")
 HOST_LIB = os.path.join(HERE, "_host.so")              # a Python extension module: tensors in, C ABI calls out
 
-SOURCES = ["api.cu", "gca_simt.cu", "gca_csr.cu", "gca_decode.cu", "gca_cache.cu", "lmk_topk.cu", "lmk_tc_sm100.cu", "lmk_grad.cu",
+SOURCES = ["api.cu", "gca_simt.cu", "gca_f32_sm100.cu", "gca_csr.cu", "gca_decode.cu", "gca_cache.cu", "lmk_topk.cu", "lmk_tc_sm100.cu", "lmk_grad.cu",
            "gca_fwd_sm100.cu", "gca_bwd_sm100.cu", "gca_bwd_q_sm100.cu", "gca_bwd_kv_sm100.cu", "kv_project_sm100.cu", "skinny_linear.cu", "layer_decode.cu", "win_attn_decode.cu", "vmem.cu"]
 
 

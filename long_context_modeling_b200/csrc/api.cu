@@ -166,6 +166,7 @@ int gca_fwd(const GcaFwdArgs* a, void* stream) {
     b.algo = algo;
     return gca::launch_fwd_tc(b, gca::sm_count(scope.dev), s);
   }
+  if (a->algo == GCA_ALGO_AUTO && gca::f32_tc_takes(a->dtype, a->S, (long long)a->N * a->J * a->Hq)) return gca::launch_fwd_f32_tc(*a, s);
   if (algo == GCA_ALGO_SIMT) return gca::launch_fwd_simt(*a, s);
   return GCA_ERR_ALGO;
 }
@@ -240,14 +241,17 @@ int gca_bwd_stages(const GcaBwdArgs* a, unsigned stages, void* stream) {
   const bool tc_ok = a->dtype == GCA_BF16 && a->S == 64;
   if (algo == GCA_ALGO_TC_UNPAIRED) algo = GCA_ALGO_TC;
   if (algo == GCA_ALGO_AUTO) algo = tc_ok ? GCA_ALGO_TC : GCA_ALGO_SIMT;
+  const bool f32_tc = a->algo == GCA_ALGO_AUTO &&
+                      gca::f32_tc_takes(a->dtype, a->S, (long long)a->N * (a->J > a->C ? a->J : a->C) * a->Hq);
   if (algo == GCA_ALGO_TC)
     rc = tc_ok ? gca::launch_bwd_tc(*a, csr, dw_part, rowterm, gca::sm_count(scope.dev), s, stages & GCA_BWD_STAGE_ALL) : GCA_ERR_ALGO;
+  else if (f32_tc) rc = gca::launch_bwd_f32_tc(*a, csr, dw_part, reinterpret_cast<float*>(rowterm), s, stages & GCA_BWD_STAGE_ALL);
   else if (algo == GCA_ALGO_SIMT) rc = gca::launch_bwd_simt(*a, csr, dw_part, reinterpret_cast<float*>(rowterm), s, stages & GCA_BWD_STAGE_ALL);
   else rc = GCA_ERR_ALGO;
   if (rc) return rc;
   if (!(stages & GCA_BWD_STAGE_Q)) return 0;
   if (algo == GCA_ALGO_TC && (stages & GCA_BWD_STAGE_KV)) return 0;      // the kv-major kernel has reduced dw
-  return gca::launch_dw_reduce(dw_part, a->dw, a->N * a->J, a->Hq, a->K, algo == GCA_ALGO_TC ? gca::bwd_tc_dw_parts() : 1, s);
+  return gca::launch_dw_reduce(dw_part, a->dw, a->N * a->J, a->Hq, a->K, algo == GCA_ALGO_TC ? gca::bwd_tc_dw_parts() : f32_tc ? 4 : 1, s);
 }
 
 }  // extern "C"

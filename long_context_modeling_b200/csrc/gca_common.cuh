@@ -76,6 +76,24 @@ struct Geom {
   float off_by_one;
 };
 
+inline Geom make_geom(const GcaFwdArgs& a) {
+  Geom g;
+  g.N = a.N; g.J = a.J; g.Hq = a.Hq; g.Hkv = a.Hkv; g.S = a.S; g.L = a.L; g.D = a.D; g.K = a.K; g.C = a.C;
+  g.G = a.Hq / a.Hkv;
+  for (int i = 0; i < 4; ++i) { g.qs[i] = a.q_stride[i]; g.os[i] = a.o_stride[i]; g.ks[i] = a.k_stride[i]; g.vs[i] = a.v_stride[i]; }
+  g.sm_scale = a.sm_scale; g.off_by_one = a.off_by_one;
+  return g;
+}
+
+inline Geom make_geom(const GcaBwdArgs& a) {
+  Geom g;
+  g.N = a.N; g.J = a.J; g.Hq = a.Hq; g.Hkv = a.Hkv; g.S = a.S; g.L = a.L; g.D = a.D; g.K = a.K; g.C = a.C;
+  g.G = a.Hq / a.Hkv;
+  for (int i = 0; i < 4; ++i) { g.qs[i] = a.q_stride[i]; g.os[i] = a.dq_stride[i]; g.ks[i] = a.k_stride[i]; g.vs[i] = a.v_stride[i]; }
+  g.sm_scale = a.sm_scale; g.off_by_one = a.off_by_one;
+  return g;
+}
+
 // Inverse retrieval index: for every cache chunk (n, c) the list of (j*K + k) entries that retrieved it, in order: the low
 // 32 bits of `sorted_keys`.
 // `unit_tab` lists the chunks in the order the kv-major kernels take them: by DECREASING number of
@@ -102,6 +120,11 @@ int launch_fwd_simt(const GcaFwdArgs& a, cudaStream_t stream);
 // stages: GCA_BWD_STAGE_KV and / or GCA_BWD_STAGE_Q
 // row_di: (N*J, Hq, K, 64) floats of scratch, Di of every row: the q-major stage writes it, the kv-major stage reads it
 int launch_bwd_simt(const GcaBwdArgs& a, const Csr& csr, float* dw_part, float* row_di, cudaStream_t stream, unsigned stages);
+
+// float32 on the tensor cores, S = L = D = 64 (same scratch; four dw partials per (row block, head, slot)).
+bool f32_tc_takes(int dtype, int S, long long units);
+int launch_fwd_f32_tc(const GcaFwdArgs& a, cudaStream_t stream);
+int launch_bwd_f32_tc(const GcaBwdArgs& a, const Csr& csr, float* dw_part, float* row_di, cudaStream_t stream, unsigned stages);
 
 // tcgen05 / TMEM / TMA kernels: bf16, S = L = D = 64.
 int launch_fwd_tc(const GcaFwdArgs& a, int sms, cudaStream_t stream);

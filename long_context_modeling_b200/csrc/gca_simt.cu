@@ -1,5 +1,5 @@
-// CUDA-core GCA kernels with float32 arithmetic throughout.  They serve float32 data (the accuracy path: tensor cores
-// would round the operands) and any shape the tensor-core kernels do not take (S < 64 query rows).  One block of four
+// CUDA-core GCA kernels with float32 arithmetic throughout.  They serve what the tensor-core kernels do not take (fewer than 64 query
+// rows) and callers that ask for them; float32 with 64 rows goes to gca_f32_sm100.cu, which is faster and closer to 64 bits.  One block of four
 // warps owns one (sequence, query chunk, head) in the q-major kernels and one (sequence, cache chunk, kv head) in the
 // kv-major backward kernel, so no atomics are needed and results are bit-reproducible.
 //
@@ -417,34 +417,25 @@ bwd_kv_simt_kernel(const E* __restrict__ q, const E* __restrict__ kc, const E* _
   store_rows(dv + n * dvs0 + c * dvs1 + hk * dvs3, dvs2, T, own, aV, 1.0f);
 }
 
-__global__ void dw_reduce_kernel(const float* __restrict__ part, float* __restrict__ dw, int ZJ, int Hq, int K,
-                                 int parts) {
+// One thread per (row block, slot), whatever the order of the loads the same order of the sum.  Four heads' loads are in flight at a
+// time: one by one they cost 10 us for 12 heads x 4 partials, whatever the number of rows.
+template <int PARTS>
+__global__ void dw_reduce_kernel(const float* __restrict__ part, float* __restrict__ dw, int ZJ, int Hq, int K) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (long long)ZJ * K) return;
   const long long zj = i / K;
-  const int k = (int)(i % K);
+  const float* p = part + (zj * Hq * K + (i - zj * K)) * PARTS;
   float t = 0.f;
-  for (int h = 0; h < Hq; ++h)
-    for (int q = 0; q < parts; ++q) t += part[((zj * Hq + h) * K + k) * parts + q];
+#pragma unroll 4
+  for (int h = 0; h < Hq; ++h, p += K * PARTS) {
+    if (PARTS == 4) {
+      const float4 v = __ldg(reinterpret_cast<const float4*>(p));
+      t += v.x; t += v.y; t += v.z; t += v.w;
+    } else {
+      t += __ldg(p);
+    }
+  }
   dw[i] = t;
-}
-
-Geom make_geom(const GcaFwdArgs& a) {
-  Geom g;
-  g.N = a.N; g.J = a.J; g.Hq = a.Hq; g.Hkv = a.Hkv; g.S = a.S; g.L = a.L; g.D = a.D; g.K = a.K; g.C = a.C;
-  g.G = a.Hq / a.Hkv;
-  for (int i = 0; i < 4; ++i) { g.qs[i] = a.q_stride[i]; g.os[i] = a.o_stride[i]; g.ks[i] = a.k_stride[i]; g.vs[i] = a.v_stride[i]; }
-  g.sm_scale = a.sm_scale; g.off_by_one = a.off_by_one;
-  return g;
-}
-
-Geom make_geom(const GcaBwdArgs& a) {
-  Geom g;
-  g.N = a.N; g.J = a.J; g.Hq = a.Hq; g.Hkv = a.Hkv; g.S = a.S; g.L = a.L; g.D = a.D; g.K = a.K; g.C = a.C;
-  g.G = a.Hq / a.Hkv;
-  for (int i = 0; i < 4; ++i) { g.qs[i] = a.q_stride[i]; g.os[i] = a.dq_stride[i]; g.ks[i] = a.k_stride[i]; g.vs[i] = a.v_stride[i]; }
-  g.sm_scale = a.sm_scale; g.off_by_one = a.off_by_one;
-  return g;
 }
 
 template <typename E>
@@ -501,7 +492,9 @@ int launch_bwd_simt(const GcaBwdArgs& a, const Csr& csr, float* dw_part, float* 
 int launch_dw_reduce(const float* dw_part, float* dw, int ZJ, int Hq, int K, int parts, cudaStream_t stream) {
   const long long total = (long long)ZJ * K;
   if (total == 0) return 0;
-  dw_reduce_kernel<<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(dw_part, dw, ZJ, Hq, K, parts);
+  const unsigned blocks = (unsigned)((total + 63) / 64);
+  if (parts == 4) dw_reduce_kernel<4><<<blocks, 64, 0, stream>>>(dw_part, dw, ZJ, Hq, K);
+  else dw_reduce_kernel<1><<<blocks, 64, 0, stream>>>(dw_part, dw, ZJ, Hq, K);
   return (int)cudaGetLastError();
 }
 

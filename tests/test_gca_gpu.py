@@ -514,3 +514,62 @@ def test_decode_warps_per_slot(lcm, n, hq, hkv, sq, k, obo):
     ref = G.gca_indexed(q.float(), kc.float(), vc.float(), idx, torch.where(idx < 0, torch.zeros_like(w), w), 0.125, off_by_one=1.0 if obo else 0.0)
     got = lcm.gca_indexed_nograd(q.cuda(), kc.cuda(), vc.cuda(), idx.cuda(), w.cuda(), 0.125, softmax_off_by_one=obo).float().cpu()
     assert (got - ref).abs().max() <= 1e-2 * ref.abs().max()
+
+
+# ---- float32 on the tensor cores (S = 64), every operand as three bf16 values
+def _two_norm(a, b):
+    a, b = a.detach().double().cpu(), b.detach().double().cpu()
+    return ((a - b).norm() / (b.norm() + 1e-300)).item()
+
+
+F32_SPLIT_REL = 2.0 ** -20      # four errors of 2^-22: scores of |S c| < 8 carry 8 x 2^-25, exponentials, sums and the split 2^-24 each
+
+
+@pytest.mark.parametrize("n,c,hq,hkv,k,off_by_one,token_major", [
+    (1, 2, 1, 1, 1, False, False),       # no slot at all
+    (1, 3, 1, 1, 1, True, False),        # one slot: first and last at once
+    (1, 4, 2, 1, 2, False, True),        # two slots, one tile ring not filled
+    (3, 7, 3, 3, 5, True, False),        # rings wrap, odd number of heads, several sequences
+    (1, 12, 8, 2, 8, False, True),       # four q heads per kv head
+    (1, 40, 2, 2, 32, False, False),     # the most slots
+])
+def test_float32_split_products_vs_oracle(lcm, n, c, hq, hkv, k, off_by_one, token_major):
+    q, _, _, idx, w, dout = cases.gca_indexed_case(31, n, c, hq, k, dtype=torch.float32)
+    g = torch.Generator().manual_seed(32)
+    kc, vc = (torch.randn(n, c, 64, hkv * 64, generator=g) for _ in range(2))
+    for b in range(n):                   # padding anywhere among the slots
+        for j in range(c - 1):
+            perm = torch.randperm(k, generator=g)
+            idx[b, j], w[b, j] = idx[b, j, perm], w[b, j, perm]
+    if token_major:                      # views of a projection's output
+        q, dout = (t.transpose(2, 3).contiguous().transpose(2, 3) for t in (q, dout))
+    ref = G.gca_indexed_grads(q, kc, vc, idx, w, 0.125, dout, off_by_one=1.0 if off_by_one else 0.0, work_dtype=torch.float64)
+    got = run_indexed(lcm, q, kc, vc, idx, w, 0.125, dout=dout, softmax_off_by_one=off_by_one, token_major_out=token_major)
+    for name, g_, r_ in zip(("o", "dq", "dk", "dv", "dw"), got, ref):
+        assert g_.shape == r_.shape and _two_norm(g_, r_) <= F32_SPLIT_REL, (name, _two_norm(g_, r_))
+    again = run_indexed(lcm, q, kc, vc, idx, w, 0.125, dout=dout, softmax_off_by_one=off_by_one, token_major_out=token_major)
+    assert all(torch.equal(a, b) for a, b in zip(got, again))
+    assert lcm.read_status() == 0
+
+
+def test_float32_split_products_are_no_less_precise_than_fma(lcm):
+    q, kc, vc, idx, w, dout = cases.gca_indexed_case(33, 2, 20, 4, 8, dtype=torch.float32)
+    ref = G.gca_indexed_grads(q, kc, vc, idx, w, 0.125, dout, work_dtype=torch.float64)
+    tc, fma = (run_indexed(lcm, q, kc, vc, idx, w, 0.125, dout=dout, algo=algo) for algo in (0, 1))
+    for name, t_, f_, r_ in zip(("o", "dq", "dk", "dv"), tc, fma, ref):
+        assert _two_norm(t_, r_) <= _two_norm(f_, r_), name
+
+
+def test_float32_extremes_and_nan(lcm):
+    """The largest float32 numbers stay finite; NaN and infinities reach the rows and columns they belong to, and no others."""
+    q, kc, vc, idx, w, _ = cases.gca_indexed_case(34, 1, 6, 2, 2, dtype=torch.float32)
+    big = torch.finfo(torch.float32).max
+    vc[0, 0, 5, 7], kc[0, 1, 3, 9], q[..., 9] = -big, big, 0.0       # head 0: column 7; a score of 0 x big
+    out = run_indexed(lcm, q, kc, vc, idx, w, 0.125)
+    ref = G.gca_indexed(q.double(), kc.double(), vc.double(), idx, w.double(), 0.125)
+    assert torch.isfinite(out).all() and _two_norm(out[..., 7], ref[..., 7]) <= F32_SPLIT_REL
+    for bad in (float("nan"), float("inf")):
+        q2, v2 = q.clone(), vc.clone()
+        q2[0, 4, 1, 20, 3], v2[0, 2, 11, 30] = bad, bad             # a query row of head 1; column 30 of head 0 where chunk 2 is read
+        got, want = run_indexed(lcm, q2, kc, v2, idx, w, 0.125).cpu(), G.gca_indexed(q2, kc, v2, idx, w, 0.125)
+        assert torch.equal(torch.isfinite(got), torch.isfinite(want))
