@@ -573,3 +573,22 @@ def test_float32_extremes_and_nan(lcm):
         q2[0, 4, 1, 20, 3], v2[0, 2, 11, 30] = bad, bad             # a query row of head 1; column 30 of head 0 where chunk 2 is read
         got, want = run_indexed(lcm, q2, kc, v2, idx, w, 0.125).cpu(), G.gca_indexed(q2, kc, v2, idx, w, 0.125)
         assert torch.equal(torch.isfinite(got), torch.isfinite(want))
+
+
+@pytest.mark.parametrize("n,c,h,k", [(40, 30, 3, 1), (8, 60, 4, 2), (3, 30, 2, 32), (1, 3, 1, 4)])
+def test_forward_slot_records(lcm, n, c, h, k):
+    """Units of one slot, of few, of 32, and fewer slots in all than there are warpgroups; a third of the units empty: the forward's roles
+    follow slots, not units.  Same bits on every run and from one head per unit."""
+    g = torch.Generator(device="cuda").manual_seed(46)
+    q = torch.empty(n, c - 1, h, 64, 64, dtype=torch.bfloat16, device="cuda").normal_(generator=g)
+    kc, vc = (torch.empty(n, c, 64, h * 64, dtype=torch.bfloat16, device="cuda").normal_(generator=g) for _ in range(2))
+    idx = torch.randint(0, c, (n, c - 1, k), generator=g, device="cuda", dtype=torch.int32)
+    idx[:, ::3] = -1
+    idx[:, 1::3, k // 2] = -1
+    w = torch.softmax(torch.randn(n, c - 1, k, generator=g, device="cuda"), -1)
+    out = lcm.gca_indexed_nograd(q, kc, vc, idx, w, 0.125)
+    want = lcm.gca_indexed_nograd(q, kc, vc, idx, w, 0.125, algo=1)
+    assert (out.float() - want.float()).abs().max().item() <= BF16_REL * max(1e-3, want.float().abs().max().item())
+    for algo in (0, 3) * 10:
+        assert torch.equal(out, lcm.gca_indexed_nograd(q, kc, vc, idx, w, 0.125, algo=algo))
+    assert lcm.read_status() == 0
