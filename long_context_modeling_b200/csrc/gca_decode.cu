@@ -219,89 +219,97 @@ decode_kernel(const __grid_constant__ DecParams p) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// Up to four query rows per kv head (the model's decode step: one row): no shared-memory staging at
-// all.  One CTA per (sequence, query chunk, kv head), one warp per retrieved slot (slots k = warp,
-// warp + 8, ...).  A warp load covers FOUR key rows of the slot's tile (8 lanes x 16 bytes per
-// 128-byte row); every 8-lane group owns a stream of 16 keys with its own online-softmax state, the
-// loads run four steps ahead of the arithmetic in registers, and nothing is waited for except the
-// data itself.  Registers are capped so that three CTAs share an SM: 32 sequences x
-// 12 heads = 384 CTAs run as one wave, where the persistent TMA kernel below needs a ragged third
-// round of its 148 CTAs.  The four streams of a warp, then the slots in slot order, are merged in a
-// fixed order: the result does not depend on scheduling.
-struct RowState { float m, l, acc[8]; };
+// Up to four query rows per kv head (the model's decode step: one row): no shared-memory staging at all.  WPS warps per
+// retrieved slot (64 / WPS keys each), the slots of an item dealt out over the warps of a CTA or of a cluster of them.  A warp
+// load covers FOUR key rows of the slot's tile (8 lanes x 16 bytes per 128-byte row); every 8-lane group owns a stream of keys
+// with its own online-softmax state, the loads run four steps ahead of the arithmetic in registers, and nothing is waited for
+// except the data itself.  The streams of a warp, the warps of a slot, the slots and the CTAs of a cluster are merged in a fixed
+// order: the result does not depend on scheduling.
+// Bound: HBM for many items (32 sequences x 12 heads x 8 slots: 11.0 us, 7.7 at the copy rate; at most eight warps an item and a
+// step of its own for every four keys took 11.6), else latency: launch, one round of loads, the merges (one row, 132 items, K = 13:
+// 7.4 us against 8.7; two rows, 8 items, K = 16: 4.2 against 18.1, 96 items, K = 15: 7.8 against 17.9).  What each split gains is
+// said at decode_plan().
+struct RowState { float m, l; float2 acc[4]; };
 __device__ __forceinline__ float ex2f(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-__device__ __forceinline__ void merge_state(RowState& a, float m2, float l2, const float* acc2) {
-  const float m = fmaxf(a.m, m2);
-  const float ca = (a.m == -INFINITY) ? 0.f : ex2f(a.m - m), cb = (m2 == -INFINITY) ? 0.f : ex2f(m2 - m);
-  a.l = a.l * ca + l2 * cb;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) a.acc[i] = a.acc[i] * ca + acc2[i] * cb;
-  a.m = m;
+__device__ __forceinline__ float2 bf2(unsigned v) { return make_float2(bf_lo(v), bf_hi(v)); }
+__device__ __forceinline__ float2 splat(float x) { return make_float2(x, x); }
+__device__ __forceinline__ float ld_dsmem(const float* p, int rank) {        // the same variable in another CTA of the cluster
+  float v;
+  asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %1, %2;\n\tld.shared::cluster.f32 %0, [a];\n\t}" : "=f"(v) : "r"(smem_u32(p)), "r"(rank) : "memory");
+  return v;
 }
 
-template <int R>
-__global__ void __launch_bounds__(NWARPS * 32, R == 1 ? 3 : (R == 2 ? 2 : 1))
+// Registers a thread and the most warps a CTA of decode_rows_kernel<rows, wps> has.
+template <int R, int WPS> constexpr int ROW_REGS = R > 1 ? 128 : WPS == 4 ? 64 : 80;
+template <int R, int WPS> constexpr int ROW_WARPS = R > 1 ? 16 : WPS == 4 ? 32 : 24;
+constexpr int STATE = 66;                                        // maximum, sum, 64 outputs
+
+template <int R, int WPS>
+__global__ void __maxnreg__((ROW_REGS<R, WPS>))
 decode_rows_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ kc, const __nv_bfloat16* __restrict__ vc,
                    const int32_t* __restrict__ indices, const float* __restrict__ weights, __nv_bfloat16* __restrict__ out,
-                   int32_t* status, const Geom g) {
-  __shared__ float part[NWARPS][R][64];
+                   int32_t* status, const Geom g, int ctas) {
+  constexpr int BATCHES = 4 / WPS;                               // of four steps of four keys
+  constexpr int WARPS = ROW_WARPS<R, WPS>;
+  __shared__ float part[WARPS][R][WPS > 1 ? STATE : 64];        // a warp's weighted outputs over its slots; WPS > 1: its part of its slot's state
+  __shared__ float total[R][64];                                 // this CTA's sum
+  __shared__ float slot_w[WARPS];
+  __shared__ bool slot_reads[WARPS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = lane >> 3, sub = lane & 7;
-  const int item = blockIdx.x;
+  const int warps = blockDim.x >> 5, slots = warps / WPS;        // of the CTA
+  const int item = blockIdx.x / ctas, rank = blockIdx.x - item * ctas;
   const int zj = item / g.Hkv, hk = item - zj * g.Hkv;
   const int n = zj / g.J, j = zj - n * g.J;
-  const int rows = g.G * g.S;                                    // <= R
+  const int row0 = blockIdx.y * R, rows = min(R, g.G * g.S - row0);      // this CTA's rows of the kv head
   const float c2 = g.sm_scale * GCA_LOG2E;
+  const int k0 = rank * slots + warp / WPS, share = warp % WPS;
   pdl_trigger();
   // While the kernel before is finishing, this warp's first K tile on its way into L2 (V as well, which fills the queues the
   // loads behind the wait need: no gain left).  The index may not be final yet, so it is a hint here, read past L1 and read
   // again below.
-  if (warp < g.K) {
-    int hint = warp;
-    if (indices) asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(hint) : "l"(indices + (long long)zj * g.K + warp) : "memory");
+  if (k0 < g.K) {
+    int hint = k0;
+    if (indices) asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(hint) : "l"(indices + (long long)zj * g.K + k0) : "memory");
     if (hint >= 0 && hint < g.C) {
-      const __nv_bfloat16* kt = kc + n * g.ks[0] + hint * g.ks[1] + hk * g.ks[3] + lane * g.ks[2];
+      const __nv_bfloat16* kt = kc + n * g.ks[0] + hint * g.ks[1] + hk * g.ks[3] + (share * (64 / WPS) + lane % (64 / WPS)) * g.ks[2];
       asm volatile("prefetch.global.L2 [%0];" ::"l"(kt));
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(kt + 32 * g.ks[2]));
+      if (WPS == 1) asm volatile("prefetch.global.L2 [%0];" ::"l"(kt + 32 * g.ks[2]));
     }
   }
   pdl_wait();
-  float qv[R][8];
+  uint4 qv[R];                                                   // this lane's 8 query values of every row, as they came
 #pragma unroll
   for (int r = 0; r < R; ++r) {
-#pragma unroll
-    for (int e = 0; e < 8; ++e) qv[r][e] = 0.f;
+    qv[r] = make_uint4(0, 0, 0, 0);
     if (r < rows) {
-      const int gi = r / g.S, s = r - gi * g.S;
-      const uint4 t = *reinterpret_cast<const uint4*>(q + n * g.qs[0] + j * g.qs[1] + (hk * g.G + gi) * g.qs[2] + s * g.qs[3] + sub * 8);
-      const unsigned w4[4] = {t.x, t.y, t.z, t.w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) { qv[r][2 * e] = bf_lo(w4[e]) * c2; qv[r][2 * e + 1] = bf_hi(w4[e]) * c2; }
+      const int gi = (row0 + r) / g.S, s = row0 + r - gi * g.S;
+      qv[r] = *reinterpret_cast<const uint4*>(q + n * g.qs[0] + j * g.qs[1] + (hk * g.G + gi) * g.qs[2] + s * g.qs[3] + sub * 8);
     }
   }
-  float o[R][8];                                 // this warp's weighted outputs, 8 columns per lane
-#pragma unroll
-  for (int r = 0; r < R; ++r)
-#pragma unroll
-    for (int e = 0; e < 8; ++e) o[r][e] = 0.f;
-  for (int k = warp; k < g.K; k += NWARPS) {
+  if (WPS == 1) {
+    for (int i = lane; i < R * 64; i += 32) (&part[warp][0][0])[i] = 0.f;
+    __syncwarp();
+  } else if (share == 0 && lane == 0) slot_reads[warp / WPS] = false;
+  for (int k = k0; k < g.K; k += ctas * slots) {
     const int idx = slot_chunk(indices, zj, g.K, k);
     if (idx < 0) continue;                                       // padding slot (warp-uniform)
-    if (idx >= g.C) { if (status && lane == 0) atomicOr(status, GCA_STATUS_BAD_INDEX); continue; }
+    if (idx >= g.C) { if (status && share == 0 && lane == 0) atomicOr(status, GCA_STATUS_BAD_INDEX); continue; }
     const float w = weights[(long long)zj * g.K + k];
-    const __nv_bfloat16* kb = kc + n * g.ks[0] + idx * g.ks[1] + hk * g.ks[3] + sub * 8 + grp * g.ks[2];
-    const __nv_bfloat16* vb = vc + n * g.vs[0] + idx * g.vs[1] + hk * g.vs[3] + sub * 8 + grp * g.vs[2];
+    const int key0 = share * (64 / WPS) + grp;
+    const __nv_bfloat16* kb = kc + n * g.ks[0] + idx * g.ks[1] + hk * g.ks[3] + sub * 8 + key0 * g.ks[2];
+    const __nv_bfloat16* vb = vc + n * g.vs[0] + idx * g.vs[1] + hk * g.vs[3] + sub * 8 + key0 * g.vs[2];
     RowState st[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       st[r].m = -INFINITY; st[r].l = 0.f;
 #pragma unroll
-      for (int e = 0; e < 8; ++e) st[r].acc[e] = 0.f;
+      for (int e = 0; e < 4; ++e) st[r].acc[e] = splat(0.f);
     }
-    // 16 steps of 4 keys, four steps at a time: the next four steps' rows are requested as soon as the registers are read, and
+    // steps of 4 keys, four steps at a time: the next four steps' rows are requested as soon as the registers are read, and
     // the four steps share one maximum and one rescaling (a step of its own each was a chain of ~200 cycles)
     uint4 kq[4], vq[4];
 #pragma unroll
@@ -310,19 +318,20 @@ decode_rows_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
       vq[s] = *reinterpret_cast<const uint4*>(vb); vb += 4 * g.vs[2];
     }
 #pragma unroll 1
-    for (int b4 = 0; b4 < 16; b4 += 4) {
+    for (int b = 0; b < BATCHES; ++b) {
       float sc[R][4];
 #pragma unroll
       for (int s = 0; s < 4; ++s) {
-        const unsigned kw[4] = {kq[s].x, kq[s].y, kq[s].z, kq[s].w};
+        const float2 k2[4] = {bf2(kq[s].x), bf2(kq[s].y), bf2(kq[s].z), bf2(kq[s].w)};
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-          float t = 0.f;
-#pragma unroll
-          for (int e = 0; e < 4; ++e) { t = fmaf(qv[r][2 * e], bf_lo(kw[e]), t); t = fmaf(qv[r][2 * e + 1], bf_hi(kw[e]), t); }
-          sc[r][s] = t;
+          float2 t = __fmul2_rn(bf2(qv[r].x), k2[0]);
+          t = __ffma2_rn(bf2(qv[r].y), k2[1], t);
+          t = __ffma2_rn(bf2(qv[r].z), k2[2], t);
+          t = __ffma2_rn(bf2(qv[r].w), k2[3], t);
+          sc[r][s] = t.x + t.y;
         }
-        if (b4 + 4 < 16) { kq[s] = *reinterpret_cast<const uint4*>(kb); kb += 4 * g.ks[2]; }
+        if (b + 1 < BATCHES) { kq[s] = *reinterpret_cast<const uint4*>(kb); kb += 4 * g.ks[2]; }
       }
 #pragma unroll
       for (int r = 0; r < R; ++r) {
@@ -330,184 +339,154 @@ decode_rows_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
         for (int of = 1; of < 8; of <<= 1)
 #pragma unroll
           for (int s = 0; s < 4; ++s) sc[r][s] += __shfl_xor_sync(0xffffffffu, sc[r][s], of);
-        const float m = fmaxf(st[r].m, fmaxf(fmaxf(sc[r][0], sc[r][1]), fmaxf(sc[r][2], sc[r][3])));
+        const float m = fmaxf(st[r].m, fmaxf(fmaxf(sc[r][0], sc[r][1]), fmaxf(sc[r][2], sc[r][3])) * c2);
         const float corr = ex2f(st[r].m - m);
         st[r].m = m;
 #pragma unroll
-        for (int s = 0; s < 4; ++s) sc[r][s] = ex2f(sc[r][s] - m);
-        st[r].l = st[r].l * corr + ((sc[r][0] + sc[r][1]) + (sc[r][2] + sc[r][3]));
+        for (int s = 0; s < 4; ++s) sc[r][s] = ex2f(fmaf(sc[r][s], c2, -m));
+        st[r].l = fmaf(st[r].l, corr, (sc[r][0] + sc[r][1]) + (sc[r][2] + sc[r][3]));
+        if (BATCHES > 1) {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) st[r].acc[e] *= corr;
+          for (int e = 0; e < 4; ++e) st[r].acc[e] = __fmul2_rn(st[r].acc[e], splat(corr));
+        }
       }
 #pragma unroll
       for (int s = 0; s < 4; ++s) {
-        const unsigned vw[4] = {vq[s].x, vq[s].y, vq[s].z, vq[s].w};
+        const float2 v2[4] = {bf2(vq[s].x), bf2(vq[s].y), bf2(vq[s].z), bf2(vq[s].w)};
 #pragma unroll
         for (int r = 0; r < R; ++r)
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            st[r].acc[2 * e] = fmaf(sc[r][s], bf_lo(vw[e]), st[r].acc[2 * e]);
-            st[r].acc[2 * e + 1] = fmaf(sc[r][s], bf_hi(vw[e]), st[r].acc[2 * e + 1]);
-          }
-        if (b4 + 4 < 16) { vq[s] = *reinterpret_cast<const uint4*>(vb); vb += 4 * g.vs[2]; }
+          for (int e = 0; e < 4; ++e) st[r].acc[e] = __ffma2_rn(splat(sc[r][s]), v2[e], st[r].acc[e]);
+        if (b + 1 < BATCHES) { vq[s] = *reinterpret_cast<const uint4*>(vb); vb += 4 * g.vs[2]; }
       }
     }
+    if (WPS > 1 && share == 0 && lane == 0) { slot_w[warp / WPS] = w; slot_reads[warp / WPS] = true; }
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-#pragma unroll
-      for (int of = 8; of <= 16; of <<= 1) {
-        const float m2 = __shfl_xor_sync(0xffffffffu, st[r].m, of), l2 = __shfl_xor_sync(0xffffffffu, st[r].l, of);
-        float a2[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) a2[e] = __shfl_xor_sync(0xffffffffu, st[r].acc[e], of);
-        merge_state(st[r], m2, l2, a2);
-      }
-      // softmax over this slot's 64 keys (optionally with the off-by-one term), weighted by w
-      float mm = st[r].m, ll = st[r].l;
-      if (g.off_by_one > 0.f) {
-        const float m1 = fmaxf(mm, 0.f);
-        ll = ll * ex2f(mm - m1) + g.off_by_one * ex2f(-m1);
-        const float sc1 = ex2f(mm - m1);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) st[r].acc[e] *= sc1;
-      }
-      const float f = w / ll;
-#pragma unroll
-      for (int e = 0; e < 8; ++e) o[r][e] = fmaf(st[r].acc[e], f, o[r][e]);
-    }
-  }
-  if (grp == 0) {
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-#pragma unroll
-      for (int e = 0; e < 8; ++e) part[warp][r][sub * 8 + e] = o[r][e];
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < rows * 64; i += NWARPS * 32) {
-    const int r = i >> 6, d = i & 63;
-    float t = 0.f;
-#pragma unroll
-    for (int wv = 0; wv < NWARPS; ++wv) t += part[wv][r][d];
-    const int gi = r / g.S, s = r - gi * g.S;
-    out[n * g.os[0] + j * g.os[1] + (hk * g.G + gi) * g.os[2] + s * g.os[3] + d] = __float2bfloat16_rn(t);
-  }
-}
-
-// The same for so few (sequence, kv head) items that the SMs are not all busy: WPS warps share a slot (64 / WPS keys each, all
-// their loads in flight at once), the partial softmax states meet in shared memory.  One sequence, 12 heads, K = 8, behind the
-// projection it depends on: 6.0 -> ~4 us.
-template <int R, int WPS>
-__global__ void __launch_bounds__(NWARPS * WPS * 32)
-decode_split_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ kc, const __nv_bfloat16* __restrict__ vc,
-                    const int32_t* __restrict__ indices, const float* __restrict__ weights, __nv_bfloat16* __restrict__ out,
-                    int32_t* status, const Geom g) {
-  constexpr int STEPS = 16 / WPS, PITCH = 66;                    // (maximum, sum, 64 outputs)
-  extern __shared__ float part[];                                // [K][WPS][R][PITCH]
-  __shared__ float slot_w[32];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = lane >> 3, sub = lane & 7;
-  const int item = blockIdx.x;
-  const int zj = item / g.Hkv, hk = item - zj * g.Hkv;
-  const int n = zj / g.J, j = zj - n * g.J;
-  const int rows = g.G * g.S;
-  const float c2 = g.sm_scale * GCA_LOG2E;
-  pdl_trigger();
-  pdl_wait();
-  uint4 qv[R];                                                   // this lane's 8 query values of every row, as they came
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    qv[r] = make_uint4(0, 0, 0, 0);
-    if (r < rows) {
-      const int gi = r / g.S, s = r - gi * g.S;
-      qv[r] = *reinterpret_cast<const uint4*>(q + n * g.qs[0] + j * g.qs[1] + (hk * g.G + gi) * g.qs[2] + s * g.qs[3] + sub * 8);
-    }
-  }
-  const int share = warp % WPS;
-  for (int k = warp / WPS; k < g.K; k += NWARPS) {
-    const int idx = slot_chunk(indices, zj, g.K, k);
-    const bool live = idx >= 0 && idx < g.C;
-    if (share == 0 && lane == 0) {
-      if (idx >= g.C && status) atomicOr(status, GCA_STATUS_BAD_INDEX);
-      slot_w[k] = live ? weights[(long long)zj * g.K + k] : 0.f;
-    }
-    if (!live) continue;
-    const int key0 = share * (64 / WPS) + grp;
-    const __nv_bfloat16* kb = kc + n * g.ks[0] + idx * g.ks[1] + hk * g.ks[3] + sub * 8;
-    const __nv_bfloat16* vb = vc + n * g.vs[0] + idx * g.vs[1] + hk * g.vs[3] + sub * 8;
-    uint4 kq[STEPS], vq[STEPS];
-#pragma unroll
-    for (int s = 0; s < STEPS; ++s) {
-      kq[s] = *reinterpret_cast<const uint4*>(kb + (key0 + s * 4) * g.ks[2]);
-      vq[s] = *reinterpret_cast<const uint4*>(vb + (key0 + s * 4) * g.vs[2]);
-    }
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      float sc[STEPS], m = -INFINITY;
-      const unsigned qw[4] = {qv[r].x, qv[r].y, qv[r].z, qv[r].w};
-#pragma unroll
-      for (int s = 0; s < STEPS; ++s) {
-        const unsigned kw[4] = {kq[s].x, kq[s].y, kq[s].z, kq[s].w};
-        float t = 0.f;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) { t = fmaf(bf_lo(qw[e]), bf_lo(kw[e]), t); t = fmaf(bf_hi(qw[e]), bf_hi(kw[e]), t); }
-        sc[s] = t * c2;
-      }
-#pragma unroll
-      for (int of = 1; of < 8; of <<= 1)
-#pragma unroll
-        for (int s = 0; s < STEPS; ++s) sc[s] += __shfl_xor_sync(0xffffffffu, sc[s], of);
-#pragma unroll
-      for (int s = 0; s < STEPS; ++s) m = fmaxf(m, sc[s]);
-      m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
+      // the four streams: one maximum, then plain sums
+      float m = fmaxf(st[r].m, __shfl_xor_sync(0xffffffffu, st[r].m, 8));
       m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16));
-      float l = 0.f, acc[8];
+      const float corr = ex2f(st[r].m - m);
+      float l = st[r].l * corr;
 #pragma unroll
-      for (int e = 0; e < 8; ++e) acc[e] = 0.f;
-#pragma unroll
-      for (int s = 0; s < STEPS; ++s) {
-        const float pr = ex2f(sc[s] - m);
-        l += pr;
-        const unsigned vw[4] = {vq[s].x, vq[s].y, vq[s].z, vq[s].w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) { acc[2 * e] = fmaf(pr, bf_lo(vw[e]), acc[2 * e]); acc[2 * e + 1] = fmaf(pr, bf_hi(vw[e]), acc[2 * e + 1]); }
-      }
+      for (int e = 0; e < 4; ++e) st[r].acc[e] = __fmul2_rn(st[r].acc[e], splat(corr));
 #pragma unroll
       for (int of = 8; of <= 16; of <<= 1) {
         l += __shfl_xor_sync(0xffffffffu, l, of);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], of);
+        for (int e = 0; e < 4; ++e) {
+          st[r].acc[e].x += __shfl_xor_sync(0xffffffffu, st[r].acc[e].x, of);
+          st[r].acc[e].y += __shfl_xor_sync(0xffffffffu, st[r].acc[e].y, of);
+        }
       }
-      float* dst = part + ((k * WPS + share) * R + r) * PITCH;
-      if (lane == 0) { dst[0] = m; dst[1] = l; }
-      if (grp == 0) {
+      if (WPS > 1) {
+        float* dst = part[warp][r];
+        if (lane == 0) { dst[0] = m; dst[1] = l; }
+        if (grp == 0) {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) dst[2 + sub * 8 + e] = acc[e];
+          for (int e = 0; e < 4; ++e) { dst[2 + sub * 8 + 2 * e] = st[r].acc[e].x; dst[2 + sub * 8 + 2 * e + 1] = st[r].acc[e].y; }
+        }
+      } else {
+        // softmax over this slot's 64 keys (optionally with the off-by-one term), weighted by w
+        float f = 1.f;
+        if (g.off_by_one > 0.f) {
+          const float m1 = fmaxf(m, 0.f);
+          f = ex2f(m - m1);
+          l = l * f + g.off_by_one * ex2f(-m1);
+        }
+        f *= w / l;
+        if (grp == 0) {
+          float4* dst = reinterpret_cast<float4*>(&part[warp][r][sub * 8]);
+          const float4 a = dst[0], b = dst[1];
+          dst[0] = make_float4(fmaf(st[r].acc[0].x, f, a.x), fmaf(st[r].acc[0].y, f, a.y), fmaf(st[r].acc[1].x, f, a.z), fmaf(st[r].acc[1].y, f, a.w));
+          dst[1] = make_float4(fmaf(st[r].acc[2].x, f, b.x), fmaf(st[r].acc[2].y, f, b.y), fmaf(st[r].acc[3].x, f, b.z), fmaf(st[r].acc[3].y, f, b.w));
+        }
       }
     }
   }
   __syncthreads();
-  // out = sum over slots of w * (merged numerator) / (merged sum), in slot order
-  for (int i = threadIdx.x; i < rows * 64; i += NWARPS * WPS * 32) {
+  for (int i = threadIdx.x; i < rows * 64; i += blockDim.x) {
     const int r = i >> 6, d = i & 63;
     float t = 0.f;
-    for (int k = 0; k < g.K; ++k) {
-      const float w = slot_w[k];
-      const int idx = slot_chunk(indices, zj, g.K, k);
-      if (idx < 0 || idx >= g.C) continue;
-      const float* src = part + (k * WPS * R + r) * PITCH;
-      float m = g.off_by_one > 0.f ? 0.f : -INFINITY;
+    if (WPS == 1) {
+      for (int x = 0; x < warps; ++x) t += part[x][r][d];
+    } else {
+      for (int x = 0; x < slots; ++x) {
+        const float w = slot_w[x];
+        if (!slot_reads[x]) continue;                            // its parts hold no state
+        float m = g.off_by_one > 0.f ? 0.f : -INFINITY;
 #pragma unroll
-      for (int x = 0; x < WPS; ++x) m = fmaxf(m, src[x * R * PITCH]);
-      float l = g.off_by_one > 0.f ? g.off_by_one * ex2f(-m) : 0.f, o = 0.f;
+        for (int y = 0; y < WPS; ++y) m = fmaxf(m, part[x * WPS + y][r][0]);
+        float l = g.off_by_one > 0.f ? g.off_by_one * ex2f(-m) : 0.f, o = 0.f;
 #pragma unroll
-      for (int x = 0; x < WPS; ++x) {
-        const float c = ex2f(src[x * R * PITCH] - m);
-        l = fmaf(src[x * R * PITCH + 1], c, l);
-        o = fmaf(src[x * R * PITCH + 2 + d], c, o);
+        for (int y = 0; y < WPS; ++y) {
+          const float c = ex2f(part[x * WPS + y][r][0] - m);
+          l = fmaf(part[x * WPS + y][r][1], c, l);
+          o = fmaf(part[x * WPS + y][r][2 + d], c, o);
+        }
+        t = fmaf(o, w / l, t);
       }
-      t = fmaf(o, w / l, t);
     }
-    const int gi = r / g.S, s = r - gi * g.S;
-    out[n * g.os[0] + j * g.os[1] + (hk * g.G + gi) * g.os[2] + s * g.os[3] + d] = __float2bfloat16_rn(t);
+    if (ctas > 1) total[r][d] = t;
+    else {
+      const int gi = (row0 + r) / g.S, s = row0 + r - gi * g.S;
+      out[n * g.os[0] + j * g.os[1] + (hk * g.G + gi) * g.os[2] + s * g.os[3] + d] = __float2bfloat16_rn(t);
+    }
+  }
+  if (ctas > 1) {                                                // the first CTA adds the others' sums, in their order
+    cluster_sync();
+    if (rank == 0)
+      for (int i = threadIdx.x; i < rows * 64; i += blockDim.x) {
+        const int r = i >> 6, d = i & 63;
+        float t = total[r][d];
+        for (int x = 1; x < ctas; ++x) t += ld_dsmem(&total[r][d], x);
+        const int gi = (row0 + r) / g.S, s = row0 + r - gi * g.S;
+        out[n * g.os[0] + j * g.os[1] + (hk * g.G + gi) * g.os[2] + s * g.os[3] + d] = __float2bfloat16_rn(t);
+      }
+    cluster_sync();                                              // nobody leaves while its sums may be read
+  }
+}
+
+// How the slots of an item are dealt out: warps per slot, CTAs per item (a cluster), warps per CTA (a multiple of wps).
+//
+// What counts is that all CTAs run at once (a second wave nearly doubles the time: one row, K = 8, 384 items 10.3 us, 480 16.9 unless four
+// warps take two slots each: 15.4) and, within that, that as few steps as possible follow one another in a warp, and that an item is one CTA:
+// a cluster costs ~0.6 us.  So: the first of these that fits one wave, from the shortest chain to the longest.
+//   four warps a slot      K = 8, 100 items: 5.9 us in one CTA of 32 warps against 6.4 as two warps a slot and 7.7 as one.  Clusters of eight
+//                          warps each start sooner where every CTA has an SM to itself (12 items: 4.3 against 5.0), and clusters of
+//                          twelve or sixteen hold more than eight slots (K = 16, 64 items: 6.9 against 7.6 of a warp a slot)
+//   two warps a slot       one CTA: K = 8, 148 items 7.0 against 7.4.  In clusters only for two rows, whose chain is the longer one
+//                          (K = 16, 64 items: 7.7 against 8.6; one row 8.1 against 7.6), and for one row where a CTA cannot hold all slots
+//   a warp a slot          one CTA if it holds them (K = 13, 148 items: 8.4 against 10.2 of two CTAs), else a cluster of two to four
+//   two, three .. slots a warp, one CTA
+// Measured over rows 1, 2 x K 2 .. 32 x 4 .. 592 items (caches from memory): 1.0 % above the best of all splits on average.  Two rows at
+// 96 registers a thread instead of 128 fit more warps and lose 12 %: they spill.  Three and four rows are two pairs, whose second reading of
+// K and V hits L2: 250 registers left 8 warps an SM (K = 8, 184 items 16.7 us as four rows, 14.2 as pairs).
+struct DecodePlan { int wps, ctas, warps; };
+DecodePlan decode_plan(long long items, int K, int rows, int sms) {
+  const int cap4 = rows > 1 ? ROW_WARPS<2, 4> : ROW_WARPS<1, 4>, cap = rows > 1 ? ROW_WARPS<2, 1> : ROW_WARPS<1, 1>;
+  if (rows > 1) items *= (rows + 1) / 2;
+  DecodePlan plan = {0, 0, 0};
+  auto one_wave = [&](int wps, int ctas, int warps) {
+    const int sm_warps = 65536 / (32 * (rows > 1 ? ROW_REGS<2, 1> : wps == 4 ? ROW_REGS<1, 4> : ROW_REGS<1, 1>));
+    // clusters leave some places empty: all of a cluster's CTAs have to find theirs in one group of SMs
+    const int slack = ctas == 1 ? 0 : ctas < 5 ? 1 : ctas;
+    return warps <= (wps == 4 ? cap4 : cap) && items * ctas * (16 + slack) <= 16ll * sms * (sm_warps / warps);
+  };
+  auto take = [&](int wps, int ctas) {
+    const int slots = (K + ctas - 1) / ctas;
+    if (ctas > 8 || (K + slots - 1) / slots != ctas || !one_wave(wps, ctas, slots * wps)) return false;
+    plan = {wps, ctas, slots * wps};
+    return true;
+  };
+  const int by2 = (K + 1) / 2, by3 = (K + 2) / 3, by4 = (K + 3) / 4;
+  if (K > 6 && items * by2 <= sms && take(4, by2)) return plan;
+  if (take(4, 1) || (K > 4 && (take(4, by3) || take(4, by4))) || take(2, 1)) return plan;
+  if (rows > 1 && K > 8 && take(2, by4)) return plan;
+  if (take(1, 1) || (K > 8 && (take(2, by4) || take(1, 2) || take(1, 3) || take(1, 4)))) return plan;
+  for (int rounds = 2;; ++rounds) {
+    const int warps = (K + rounds - 1) / rounds;
+    if (warps <= 4 || one_wave(1, 1, warps)) return {1, 1, warps};
   }
 }
 
@@ -542,19 +521,21 @@ int launch_decode(const GcaFwdArgs& a, int sms, cudaStream_t stream) {
   if (rows <= 4 && blocks > 0 && a.D == 64 && a.L == 64 && vec16) {
     auto q = (const __nv_bfloat16*)a.q; auto kc = (const __nv_bfloat16*)a.k_cache; auto vc = (const __nv_bfloat16*)a.v_cache;
     auto out = (__nv_bfloat16*)a.out;
-    // warps per slot while whole SMs would be idle (the states of all slots fit 48 KB of shared memory)
-    const int wps = rows <= 2 && blocks <= sms ? 4 : rows <= 2 && blocks <= 2 * sms ? 2 : 1;
-    const size_t smem = (size_t)a.K * wps * (rows <= 1 ? 1 : 2) * 66 * sizeof(float);
-    auto run = [&](auto kernel, int threads, size_t bytes) {
-      return (int)launch_dependent(kernel, dim3((unsigned)blocks), dim3(threads), bytes, stream, q, kc, vc, a.indices, a.weights, out, a.status, g);
+    const DecodePlan plan = decode_plan(blocks, g.K, rows, sms);
+    auto run = [&](auto kernel) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3((unsigned)(blocks * plan.ctas), (unsigned)((rows + 1) / 2)); cfg.blockDim = dim3((unsigned)(plan.warps * 32)); cfg.stream = stream;
+      cudaLaunchAttribute attr[2];
+      attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[0].val.programmaticStreamSerializationAllowed = 1;
+      attr[1].id = cudaLaunchAttributeClusterDimension;
+      attr[1].val.clusterDim.x = (unsigned)plan.ctas; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+      cfg.attrs = attr; cfg.numAttrs = plan.ctas > 1 ? 2 : 1;
+      return (int)cudaLaunchKernelEx(&cfg, kernel, q, kc, vc, a.indices, a.weights, out, a.status, g, plan.ctas);
     };
-    if (wps > 1 && smem <= 48 * 1024) {
-      if (rows <= 1) return wps == 4 ? run(decode_split_kernel<1, 4>, NWARPS * 128, smem) : run(decode_split_kernel<1, 2>, NWARPS * 64, smem);
-      return wps == 4 ? run(decode_split_kernel<2, 4>, NWARPS * 128, smem) : run(decode_split_kernel<2, 2>, NWARPS * 64, smem);
-    }
-    if (rows <= 1) return run(decode_rows_kernel<1>, NWARPS * 32, 0);
-    if (rows <= 2) return run(decode_rows_kernel<2>, NWARPS * 32, 0);
-    return run(decode_rows_kernel<4>, NWARPS * 32, 0);
+    auto pick = [&](auto one, auto two, auto four) { return plan.wps == 1 ? run(one) : plan.wps == 2 ? run(two) : run(four); };
+    if (rows <= 1) return pick(decode_rows_kernel<1, 1>, decode_rows_kernel<1, 2>, decode_rows_kernel<1, 4>);
+    return pick(decode_rows_kernel<2, 1>, decode_rows_kernel<2, 2>, decode_rows_kernel<2, 4>);
   }
   int rc;
   if ((rc = make_tile_map_5d(&p.tm_k, a.k_cache, 64, 64, a.Hkv, a.C, a.N, a.k_stride[2], a.k_stride[3], a.k_stride[1], a.k_stride[0], 1, true))) return rc;

@@ -516,6 +516,36 @@ def test_decode_warps_per_slot(lcm, n, hq, hkv, sq, k, obo):
     assert (got - ref).abs().max() <= 1e-2 * ref.abs().max()
 
 
+@pytest.mark.parametrize("items,k,rows", [
+    (3, 7, 1), (9, 16, 2),               # four warps a slot, clusters of four and of eight CTAs
+    (60, 8, 1), (40, 4, 2), (30, 1, 4),  # ... all slots in one CTA
+    (40, 10, 1), (60, 16, 1), (40, 7, 2),  # ... clusters of CTAs of twelve and of sixteen warps, the last one not full
+    (147, 9, 1), (140, 12, 1), (140, 7, 2),  # two warps a slot in one CTA
+    (40, 14, 2), (20, 13, 4), (33, 29, 1),   # ... in clusters
+    (140, 16, 1), (400, 8, 1), (140, 6, 3),  # a warp a slot in one CTA
+    (90, 30, 1), (160, 16, 1), (100, 32, 1), (24, 31, 3),  # ... in clusters
+    (300, 32, 1), (520, 9, 1), (300, 17, 2), (1100, 5, 4),  # several slots a warp
+])
+def test_decode_splits(lcm, items, k, rows):
+    """How the slots are dealt out over warps, CTAs and clusters does not change the result: every split the decode kernel has,
+    with padding slots, one item that has nothing else, and the extra softmax logit."""
+    g = torch.Generator().manual_seed(items + k)
+    hkv = 3 if items % 3 == 0 else 1 if items % 2 else 2
+    n, c, obo = items // hkv, max(k, 5), items % 4 == 0
+    kc, vc = (torch.randn(n, c, 64, hkv * 64, generator=g).bfloat16() for _ in range(2))
+    q = torch.randn(n, 1, hkv, rows, 64, generator=g).bfloat16()
+    idx = torch.stack([torch.randperm(c, generator=g)[:k] for _ in range(n)]).view(n, 1, k)
+    idx[::3, :, k // 2] = -1
+    idx[n - 1] = -1
+    w = torch.softmax(torch.randn(n, 1, k, generator=g), -1)
+    ref = G.gca_indexed(q.float(), kc.float(), vc.float(), idx, torch.where(idx < 0, torch.zeros_like(w), w), 0.125, off_by_one=1.0 if obo else 0.0)
+    got = lcm.gca_indexed_nograd(q.cuda(), kc.cuda(), vc.cuda(), idx.cuda(), w.cuda(), 0.125, softmax_off_by_one=obo).float().cpu()
+    # the result's rounding to bf16: eight significant bits, a unit of the last place is at most 2^-7 of the value and the error half of
+    # one, 2^-8; the sums before it are float32 (K x 64 terms, 2^-24 each, seldom all in one direction: 2^-18 of the largest value)
+    assert ((got - ref).abs() <= ref.abs() * 2.0 ** -8 + 2.0 ** -18 * ref.abs().max()).all()
+    assert (got[n - 1] == 0).all() and lcm.read_status() == 0
+
+
 # ---- float32 on the tensor cores (S = 64), every operand as three bf16 values
 def _two_norm(a, b):
     a, b = a.detach().double().cpu(), b.detach().double().cpu()
