@@ -18,8 +18,8 @@ int launch_silu_mul(const void* gu, void* out, long long M, int I, long long in_
 int launch_linear(const LinearBatchedArgs& a, int sms, cudaStream_t stream);
 bool few_rows(long long M, int N, int K, bool with_norm, int sms);
 int launch_layer_decode(const LayerDecodeArgs& a, int dev, cudaStream_t stream);
-int launch_window_decode(const WindowDecodeArgs& a, cudaStream_t stream);
-int launch_window_ring_decode(const WindowRingDecodeArgs& a, cudaStream_t stream);
+int launch_window_decode(const WindowDecodeArgs& a, int sms, cudaStream_t stream);
+int launch_window_ring_decode(const WindowRingDecodeArgs& a, int sms, cudaStream_t stream);
 int launch_linear_ce(const LinearCeArgs& a, int sms, cudaStream_t stream);
 int launch_window_shift_append(const WindowAppendArgs& a, cudaStream_t stream);
 
@@ -448,7 +448,7 @@ int gca_window_decode(const WindowDecodeArgs* a, void* stream) {
   if (a->N == 0) return 0;
   gca::DeviceScope scope(a->out);
   if (scope.rc) return scope.rc;
-  return gca::launch_window_decode(*a, (cudaStream_t)stream);
+  return gca::launch_window_decode(*a, gca::sm_count(scope.dev), (cudaStream_t)stream);
 }
 
 int gca_window_ring_decode(const WindowRingDecodeArgs* a, void* stream) {
@@ -461,7 +461,7 @@ int gca_window_ring_decode(const WindowRingDecodeArgs* a, void* stream) {
   if (a->attn.N == 0) return 0;
   gca::DeviceScope scope(a->attn.out);
   if (scope.rc) return scope.rc;
-  return gca::launch_window_ring_decode(*a, (cudaStream_t)stream);
+  return gca::launch_window_ring_decode(*a, gca::sm_count(scope.dev), (cudaStream_t)stream);
 }
 
 int gca_linear_batched(const LinearBatchedArgs* b, void* stream) {

@@ -237,12 +237,6 @@ __device__ __forceinline__ float ex2f(float x) {
 }
 __device__ __forceinline__ float2 bf2(unsigned v) { return make_float2(bf_lo(v), bf_hi(v)); }
 __device__ __forceinline__ float2 splat(float x) { return make_float2(x, x); }
-__device__ __forceinline__ float ld_dsmem(const float* p, int rank) {        // the same variable in another CTA of the cluster
-  float v;
-  asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %1, %2;\n\tld.shared::cluster.f32 %0, [a];\n\t}" : "=f"(v) : "r"(smem_u32(p)), "r"(rank) : "memory");
-  return v;
-}
-
 // Registers a thread and the most warps a CTA of decode_rows_kernel<rows, wps> has.
 template <int R, int WPS> constexpr int ROW_REGS = R > 1 ? 128 : WPS == 4 ? 64 : 80;
 template <int R, int WPS> constexpr int ROW_WARPS = R > 1 ? 16 : WPS == 4 ? 32 : 24;

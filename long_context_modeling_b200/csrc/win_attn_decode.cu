@@ -7,36 +7,39 @@
 //   s[i, j] = scale * q_i . k_j  -  slope_h * (pos_i - j),   pos_i = T - Sq + i  (bottom-right aligned)
 //   visible: pos_i - W <= j <= pos_i;   out_i = softmax_j(s[i, :]) V
 //
-// One CTA per (sequence, kv head), 8 warps.  A warp load covers FOUR key rows: 8 lanes x 16 bytes
-// per 128-byte row, fully coalesced; each 8-lane group owns a stream of keys (j = 4 * step + group)
-// with its own online-softmax state (running maximum, sum, 8 output columns per lane), so the loop
-// has no cross-lane traffic except the 3-step dot-product reduction inside a group.  Loads run
-// PREFETCH steps ahead of the arithmetic (registers), which keeps ~64 KB per SM in flight.  At the
-// end the 4 streams of a warp and the 8 warps are merged in a fixed order: the result does not
-// depend on scheduling.
+// A CTA, or a cluster of them, per (sequence, kv head) and pair of rows; a warp takes sixteen keys at a time, straight from
+// registers.  Two kernels, chosen at window_plan(): `win_once_kernel` where there are warps for all sixteens at once,
+// `win_rounds_kernel` where several follow one another in a warp.  The warps' states and the CTAs' are merged in a fixed order:
+// the result does not depend on scheduling.
+//
+// Bound: HBM for many items, else latency (launch, one round of loads, the merges).  Eight warps an item, one key at a time and
+// multiply-adds took, us, one row: 512 keys, 4 items 6.9, now 4.8; 64 items 8.8, now 5.8; 384 items 13.3, now 12.7 (7.7 at the
+// copy rate); two rows, 384 items 23.0, now 12.6.  With multiply-adds in the second kernel too (four keys a step) 13.9 and 13.9: they
+// were ~400 instructions a warp for sixteen keys.  The same matrix instructions in the first kernel are slower (128 keys, 148
+// items 4.0 us against 3.4): their chain is the longer one.
 //
 // RING form (decode of one position per sequence against a FULL window): the window buffer is a
 // ring, the step's new K / V row arrives separately and replaces the oldest row.  With a
 // device-side count c of rows written so far, the new row goes to physical row p = c mod T, and
-// physical row j holds logical position (j - p - 1) mod T.  The CTA that owns the (sequence, kv head)
-// block takes row p from the new-row operands, stores it into the ring, and reads every other
-// row in place: the window never moves (shifting it costs a full read + write of the window per
+// physical row j holds logical position (j - p - 1) mod T.  The new row is taken from its own operands
+// and stored into row p; what a stream reads in row p itself, the oldest row or already the new one, is
+// masked; every other row is read in place: the window never moves (shifting it costs a full read + write of the window per
 // token and layer, more than the attention itself reads).
 #include "gca_common.cuh"
+#include "row_attn.cuh"
+#include "sm100_ptx.cuh"
+
+#include <algorithm>
 
 namespace gca {
 
 namespace {
 
-constexpr int NWARPS = 8, PREFETCH = 4;
-
-__device__ __forceinline__ float lo(uint32_t v) { return __uint_as_float(v << 16); }
-__device__ __forceinline__ float hi(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
+using row_attn::ex2;
+using row_attn::finite_max;
+using row_attn::high;
+using row_attn::load16;
+using row_attn::low;
 
 struct WinParams {
   const __nv_bfloat16* q;
@@ -55,170 +58,371 @@ struct WinParams {
   long long ns[2];
 };
 
-struct State { float m, l, acc[8]; };
+// Registers a thread and the most warps a CTA of the kernels has.
+template <int R, bool ROUNDS> constexpr int WIN_REGS = R > 1 ? 128 : ROUNDS ? 80 : 64;
+template <int R, bool ROUNDS> constexpr int WIN_WARPS = R > 1 ? 16 : ROUNDS ? 24 : 32;
 
-__device__ __forceinline__ void merge(State& a, float m2, float l2, const float* acc2) {
-  const float m = fmaxf(a.m, m2);
-  const float ca = (a.m == -INFINITY) ? 0.f : ex2(a.m - m), cb = (m2 == -INFINITY) ? 0.f : ex2(m2 - m);
-  a.l = a.l * ca + l2 * cb;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) a.acc[i] = a.acc[i] * ca + acc2[i] * cb;
-  a.m = m;
+template <int R> using WarpState = float[R][2 + 64];            // maximum, sum, 64 outputs of the rows
+
+// The warps' states (and a cluster's CTAs') to the outputs, in a fixed order.
+template <int R>
+__device__ __forceinline__ void merge_and_store(const WinParams& p, WarpState<R>* part, WarpState<R>& total, int ctas, int rank, int n, int hk, int row0, int rows) {
+  const int warps = blockDim.x >> 5;
+  __syncthreads();
+  auto store = [&](int r, int d, float l, float o) {
+    const int gi = (row0 + r) / p.Sq, i = row0 + r - gi * p.Sq, h = hk * p.G + gi;
+    p.out[n * p.os[0] + h * p.os[1] + i * p.os[2] + d] = __float2bfloat16_rn(p.T - p.Sq + i >= 0 ? o / l : 0.f);
+  };
+  for (int i = threadIdx.x; i < rows * 64; i += blockDim.x) {
+    const int r = i >> 6, d = i & 63;
+    float m = -INFINITY;
+    for (int w = 0; w < warps; ++w) m = fmaxf(m, part[w][r][0]);
+    const float mf = finite_max(m);
+    float l = 0.f, o = 0.f;
+    for (int w = 0; w < warps; ++w) {
+      const float c = ex2(part[w][r][0] - mf);
+      l = fmaf(part[w][r][1], c, l);
+      o = fmaf(part[w][r][2 + d], c, o);
+    }
+    if (ctas == 1) store(r, d, l, o);
+    else { total[r][2 + d] = o; if (d == 0) { total[r][0] = m; total[r][1] = l; } }
+  }
+  if (ctas > 1) {                                                // the first CTA merges the others' states, in their order
+    sm100::cluster_sync();
+    if (rank == 0)
+      for (int i = threadIdx.x; i < rows * 64; i += blockDim.x) {
+        const int r = i >> 6, d = i & 63;
+        float m = total[r][0];
+        for (int x = 1; x < ctas; ++x) m = fmaxf(m, sm100::ld_dsmem(&total[r][0], x));
+        const float mf = finite_max(m);
+        float l = 0.f, o = 0.f;
+        for (int x = 0; x < ctas; ++x) {
+          const float c = ex2(sm100::ld_dsmem(&total[r][0], x) - mf);
+          l = fmaf(sm100::ld_dsmem(&total[r][1], x), c, l);
+          o = fmaf(sm100::ld_dsmem(&total[r][2 + d], x), c, o);
+        }
+        store(r, d, l, o);
+      }
+    sm100::cluster_sync();                                       // nobody leaves while its state may be read
+  }
 }
 
-// Registers are capped so that three CTAs of the one-row kernel share an SM: 32 sequences x 12
-// heads = 384 CTAs then run as ONE wave on 148 SMs (with two per SM a second wave of 88 CTAs
-// doubled the kernel's duration).
+// One warp for sixteen keys, in one round: latency counts.  A warp load covers FOUR key rows: 8 lanes x 16 bytes per 128-byte row; each 8-lane
+// group has a stream of four keys, the streams are merged within the warp.  R rows of the kv head (blockIdx.y: which of its row pairs).  The
+// ring's new row and the window's last row stand beside the sixteens, in the first warp: a window of 512 is 513 rows.
 template <int R, bool RING>
-__global__ void __launch_bounds__(NWARPS * 32, R == 1 ? 3 : (R == 2 ? 2 : 1))
-win_decode_kernel(const WinParams p) {
-  __shared__ float part[NWARPS][R][2 + 64];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = lane >> 3, sub = lane & 7;
-  const int n = blockIdx.x / p.Hkv, hk = blockIdx.x - n * p.Hkv;
-  const int rows = p.G * p.Sq;                       // <= R
+__global__ void __maxnreg__((WIN_REGS<R, false>))
+win_once_kernel(const WinParams p, int ctas) {
+  __shared__ WarpState<R> part[WIN_WARPS<R, false>];
+  __shared__ WarpState<R> total;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = lane >> 3, sub = lane & 7, warps = blockDim.x >> 5;
+  const int item = blockIdx.x / ctas, rank = blockIdx.x - item * ctas;
+  const int n = item / p.Hkv, hk = item - n * p.Hkv;
+  const int row0 = blockIdx.y * R, rows = min(R, p.G * p.Sq - row0);
   pdl_trigger();
   pdl_wait();
-  // this lane's 8 query values of every row, pre-scaled; the row's ALiBi slope (in log2 units) and position
-  float qv[R][8], slope[R];
+  const int last = p.T - 1;
+  const int first = max(0, p.T - p.Sq - p.window);             // keys any row can see: [first, T)
+  const __nv_bfloat16* kb = p.k + n * p.ks[0] + hk * p.ks[1] + sub * 8;
+  const __nv_bfloat16* vb = p.v + n * p.vs[0] + hk * p.vs[1] + sub * 8;
+  const long long written = RING ? *p.ring : 0;
+  const int j0 = first + (rank * warps + warp) * 16 + grp;      // and 4, 8, 12 further on
+  const __nv_bfloat16 *kp = kb + j0 * p.ks[2], *vp = vb + j0 * p.vs[2];
+  uint4 kq[4], vq[4];
+#pragma unroll
+  for (int s = 0; s < 4; ++s) {
+    kq[s] = vq[s] = make_uint4(0, 0, 0, 0);
+    if (j0 + s * 4 < last) { kq[s] = load16(kp); vq[s] = load16(vp); }
+    kp += 4 * p.ks[2]; vp += 4 * p.vs[2];
+  }
+  const bool extra = rank == 0 && warp == 0;                     // group 0 has the ring's new row, group 1 the last row
+  uint4 kx = make_uint4(0, 0, 0, 0), vx = kx;
+  if (extra && grp < 2) {
+    if (RING && grp == 0) {
+      kx = load16(p.knew + n * p.ns[0] + hk * p.ns[1] + sub * 8); vx = load16(p.vnew + n * p.ns[0] + hk * p.ns[1] + sub * 8);
+    } else if (grp == 1) {
+      kx = load16(kb + last * p.ks[2]); vx = load16(vb + last * p.vs[2]);
+    }
+  }
+  uint4 qv[R];                                                   // this lane's 8 values of every row, the row's ALiBi slope (in log2 units) and position
+  float slope[R];
   int pos[R];
 #pragma unroll
   for (int r = 0; r < R; ++r) {
-    const int gi = r / p.Sq, i = r - gi * p.Sq, h = hk * p.G + gi;
+    const int gi = (row0 + r) / p.Sq, i = row0 + r - gi * p.Sq, h = hk * p.G + gi;
     pos[r] = p.T - p.Sq + i;
     slope[r] = 0.f;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) qv[r][e] = 0.f;
+    qv[r] = make_uint4(0, 0, 0, 0);
     if (r < rows) {
       slope[r] = p.slopes ? p.slopes[h] * GCA_LOG2E : 0.f;
-      const uint4 t = *reinterpret_cast<const uint4*>(p.q + n * p.qs[0] + h * p.qs[1] + i * p.qs[2] + sub * 8);
-      const uint32_t w[4] = {t.x, t.y, t.z, t.w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) { qv[r][2 * e] = lo(w[e]) * p.c2; qv[r][2 * e + 1] = hi(w[e]) * p.c2; }
+      qv[r] = load16(p.q + n * p.qs[0] + h * p.qs[1] + i * p.qs[2] + sub * 8);
     }
   }
-  State st[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    st[r].m = -INFINITY; st[r].l = 0.f;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) st[r].acc[e] = 0.f;
-  }
-  // keys any row can see: [first, T)
-  const int first = max(0, p.T - p.Sq - p.window);
-  const __nv_bfloat16* kb = p.k + n * p.ks[0] + hk * p.ks[1] + sub * 8;
-  const __nv_bfloat16* vb = p.v + n * p.vs[0] + hk * p.vs[1] + sub * 8;
-  const int stride = NWARPS * 4;                     // keys per CTA step
-  const int base = first + warp * 4;                 // warp-uniform: every lane runs the same steps
-  // Ring form: physical row `newest` is the slot of this step's new row.  The loop reads every row from
-  // the ring and skips that slot (it still holds the oldest row); the new row is visited afterwards from
-  // knew / vnew and stored into the slot.  The count is loaded first but needed only after the first
-  // loads have been issued.  The linear form is the ring whose newest row is the last one, nothing skipped.
-  const long long written = RING ? *p.ring : 0;
-  uint4 kq[PREFETCH], vq[PREFETCH];
-#pragma unroll
-  for (int s = 0; s < PREFETCH; ++s) {
-    const int j = base + grp + s * stride;
-    kq[s] = vq[s] = make_uint4(0, 0, 0, 0);
-    if (j < p.T) {
-      kq[s] = *reinterpret_cast<const uint4*>(kb + j * p.ks[2]);
-      vq[s] = *reinterpret_cast<const uint4*>(vb + j * p.vs[2]);
-    }
-  }
-  const int newest = RING ? (int)((unsigned)written % (unsigned)p.T) : p.T - 1;    // the count stays below 2^32 (caller's contract)
-  // one key against every row: `ok` = this lane's group counts it; dist[r] = back = pos[r] - (logical position)
-  auto visit = [&](const uint4& kc, const uint4& vc, bool ok, int back) {
-    const uint32_t kw[4] = {kc.x, kc.y, kc.z, kc.w}, vw[4] = {vc.x, vc.y, vc.z, vc.w};
-    float kf[8], vf[8];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) { kf[2 * e] = lo(kw[e]); kf[2 * e + 1] = hi(kw[e]); vf[2 * e] = lo(vw[e]); vf[2 * e + 1] = hi(vw[e]); }
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      float sc = 0.f;
-#pragma unroll
-      for (int e = 0; e < 8; ++e) sc = fmaf(qv[r][e], kf[e], sc);
-      sc += __shfl_xor_sync(0xffffffffu, sc, 1);
-      sc += __shfl_xor_sync(0xffffffffu, sc, 2);
-      sc += __shfl_xor_sync(0xffffffffu, sc, 4);
-      // linear form: `back` is the key's position j; ring form: the distance itself (one query position)
-      const int dist = RING ? back : pos[r] - back;
-      if (r < rows && ok && (RING || (dist >= 0 && dist <= p.window))) {
-        sc -= slope[r] * (float)dist;
-        const float m = fmaxf(st[r].m, sc);
-        const float corr = ex2(st[r].m - m), pr = ex2(sc - m);       // ex2(-inf) = 0 on the first key
-        st[r].l = st[r].l * corr + pr;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) st[r].acc[e] = fmaf(pr, vf[e], st[r].acc[e] * corr);
-        st[r].m = m;
-      }
-    }
+  // Ring: physical row `newest` is the new row's (the count stays below 2^32: caller's contract).  The linear form's newest row is the last one.
+  const int newest = RING ? (int)((unsigned)written % (unsigned)p.T) : last;
+  // how far key j lies behind row r's position, and whether the row sees it
+  auto distance = [&](int r, int j) {
+    const int d = (RING ? newest : pos[r]) - j;
+    return RING && d < 0 ? d + p.T : d;
   };
-  for (int jb = base; jb < p.T; jb += PREFETCH * stride) {
-#pragma unroll
-    for (int s = 0; s < PREFETCH; ++s) {
-      const int j = jb + grp + s * stride;
-      const uint4 kc = kq[s], vc = vq[s];
-      const int jn = j + PREFETCH * stride;             // refill this register slot
-      if (jn < p.T) {
-        kq[s] = *reinterpret_cast<const uint4*>(kb + jn * p.ks[2]);
-        vq[s] = *reinterpret_cast<const uint4*>(vb + jn * p.vs[2]);
-      }
-      // every lane of a warp runs the same number of steps (the reduction uses shuffles); keys past the
-      // end are masked, and so is the ring's slot of the new row
-      if (RING) {
-        int dist = newest - j;                          // rows behind the new one, around the ring
-        if (dist < 0) dist += p.T;
-        visit(kc, vc, j < p.T && dist != 0, dist);
-      } else {
-        visit(kc, vc, j < p.T, j);
-      }
-    }
-  }
-  if (RING && warp == 0) {
-    // the new row: attended to at distance 0 (counted by the warp's first stream), then stored over the oldest
-    // row -- no thread of this or another CTA reads that row of the ring
-    const long long noff = n * p.ns[0] + hk * p.ns[1] + sub * 8;        // this lane's 16 bytes of the new rows
-    const uint4 kc = *reinterpret_cast<const uint4*>(p.knew + noff), vc = *reinterpret_cast<const uint4*>(p.vnew + noff);
-    visit(kc, vc, grp == 0, 0);
-    if (grp == 0) {
-      *reinterpret_cast<uint4*>(const_cast<__nv_bfloat16*>(kb) + newest * p.ks[2]) = kc;
-      *reinterpret_cast<uint4*>(const_cast<__nv_bfloat16*>(vb) + newest * p.vs[2]) = vc;
-    }
-  }
-  // merge the 4 key streams of the warp (groups 8 and 16 lanes apart), then the warps
+  auto sees = [&](int d) { return RING ? d != 0 : d >= 0 && d <= p.window; };
+  auto pair = [](uint32_t v) { return make_float2(low(v), high(v)); };
+  auto splat = [](float v) { return make_float2(v, v); };
+  auto dot = [&](int r, const uint4& k) {
+    float2 t = __fmul2_rn(pair(qv[r].x), pair(k.x));
+    t = __ffma2_rn(pair(qv[r].y), pair(k.y), t);
+    t = __ffma2_rn(pair(qv[r].z), pair(k.z), t);
+    t = __ffma2_rn(pair(qv[r].w), pair(k.w), t);
+    return t.x + t.y;
+  };
+  float m[R], l[R];
+  float2 acc[R][4];
+  auto add = [&](int r, float w, const uint4& v, bool ok) {      // a masked row's values, whatever they are, count as zero
+    acc[r][0] = __ffma2_rn(splat(w), pair(ok ? v.x : 0u), acc[r][0]); acc[r][1] = __ffma2_rn(splat(w), pair(ok ? v.y : 0u), acc[r][1]);
+    acc[r][2] = __ffma2_rn(splat(w), pair(ok ? v.z : 0u), acc[r][2]); acc[r][3] = __ffma2_rn(splat(w), pair(ok ? v.w : 0u), acc[r][3]);
+  };
 #pragma unroll
   for (int r = 0; r < R; ++r) {
+    float sc[4], x = -INFINITY;
+#pragma unroll
+    for (int s = 0; s < 4; ++s) sc[s] = dot(r, kq[s]);
+#pragma unroll
+    for (int of = 1; of < 8; of <<= 1)
+#pragma unroll
+      for (int s = 0; s < 4; ++s) sc[s] += __shfl_xor_sync(0xffffffffu, sc[s], of);
+    bool ok_x = false;
+    if (extra) {                                                 // warp-uniform
+      x = dot(r, kx);
+#pragma unroll
+      for (int of = 1; of < 8; of <<= 1) x += __shfl_xor_sync(0xffffffffu, x, of);
+      const int d = RING && grp == 0 ? 0 : distance(r, last);
+      ok_x = RING && grp == 0 ? true : grp == 1 && sees(d);
+      x = ok_x ? fmaf(x, p.c2, -slope[r] * (float)d) : -INFINITY;
+    }
+    m[r] = x;
+    bool ok[4];
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      const int j = j0 + s * 4, d = distance(r, j);
+      ok[s] = j < last && sees(d);
+      sc[s] = ok[s] ? fmaf(sc[s], p.c2, -slope[r] * (float)d) : -INFINITY;
+      m[r] = fmaxf(m[r], sc[s]);
+    }
+    m[r] = fmaxf(m[r], -INFINITY);                               // NaN is not a maximum, it stays in the sum
+    const float mf = finite_max(m[r]);
+    l[r] = 0.f;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[r][e] = splat(0.f);
+    if (extra) { x = ex2(x - mf); l[r] = x; add(r, x, vx, ok_x); }
+#pragma unroll
+    for (int s = 0; s < 4; ++s) { sc[s] = ex2(sc[s] - mf); l[r] += sc[s]; add(r, sc[s], vq[s], ok[s]); }
+  }
+  if (RING && extra && grp == 0 && blockIdx.y == 0) {            // over the oldest row, which nobody uses any more
+    *reinterpret_cast<uint4*>(const_cast<__nv_bfloat16*>(kb) + newest * p.ks[2]) = kx;
+    *reinterpret_cast<uint4*>(const_cast<__nv_bfloat16*>(vb) + newest * p.vs[2]) = vx;
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r) {                                  // the four streams: one maximum, then plain sums
+    float mw = fmaxf(m[r], __shfl_xor_sync(0xffffffffu, m[r], 8));
+    mw = fmaxf(mw, __shfl_xor_sync(0xffffffffu, mw, 16));
+    const float corr = ex2(m[r] - finite_max(mw));
+    l[r] *= corr;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[r][e] = __fmul2_rn(acc[r][e], splat(corr));
 #pragma unroll
     for (int of = 8; of <= 16; of <<= 1) {
-      const float m2 = __shfl_xor_sync(0xffffffffu, st[r].m, of), l2 = __shfl_xor_sync(0xffffffffu, st[r].l, of);
-      float a2[8];
+      l[r] += __shfl_xor_sync(0xffffffffu, l[r], of);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) a2[e] = __shfl_xor_sync(0xffffffffu, st[r].acc[e], of);
-      merge(st[r], m2, l2, a2);
+      for (int e = 0; e < 4; ++e) {
+        acc[r][e].x += __shfl_xor_sync(0xffffffffu, acc[r][e].x, of);
+        acc[r][e].y += __shfl_xor_sync(0xffffffffu, acc[r][e].y, of);
+      }
     }
+    float* dst = part[warp][r];
+    if (lane == 0) { dst[0] = mw; dst[1] = l[r]; }
     if (grp == 0) {
-      if (sub == 0) { part[warp][r][0] = st[r].m; part[warp][r][1] = st[r].l; }
 #pragma unroll
-      for (int e = 0; e < 8; ++e) part[warp][r][2 + sub * 8 + e] = st[r].acc[e];
+      for (int e = 0; e < 4; ++e) *reinterpret_cast<float2*>(dst + 2 + sub * 8 + 2 * e) = acc[r][e];
     }
   }
-  __syncthreads();
-  // thread t < rows * 8 finishes 8 output columns of one row
-  if (threadIdx.x < rows * 8) {
-    const int r = threadIdx.x >> 3, s8 = threadIdx.x & 7;
-    State t;
-    t.m = -INFINITY; t.l = 0.f;
+  merge_and_store<R>(p, part, total, ctas, rank, n, hk, row0, rows);
+}
+
+// Several rounds of sixteen keys a warp: throughput counts, the next sixteen rows are on their way while these are worked on, on the tensor
+// cores (row_attn.cuh).  The extra rows are a sixteen of the first warp's, before its others: a fifth round for them made a window of 512 a
+// quarter longer.
+template <int R, bool RING>
+__global__ void __maxnreg__((WIN_REGS<R, true>))
+win_rounds_kernel(const WinParams p, int) {                      // one CTA an item
+  __shared__ WarpState<R> part[WIN_WARPS<R, true>];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, warps = blockDim.x >> 5;
+  const int n = blockIdx.x / p.Hkv, hk = blockIdx.x - n * p.Hkv;
+  const int row0 = blockIdx.y * R, rows = min(R, p.G * p.Sq - row0);
+  pdl_trigger();
+  pdl_wait();
+  const int first = max(0, p.T - p.Sq - p.window);             // keys any row can see: [first, T)
+  // Sixteens of keys: [first, last) in order, dealt out over the warps, and one with the ring's new row and the window's last row
+  const bool extra = RING || p.Sq == 1;
+  const int last = extra ? p.T - 1 : p.T;
+  const __nv_bfloat16* kb = p.k + n * p.ks[0] + hk * p.ks[1] + t * 8;
+  const __nv_bfloat16* vb = p.v + n * p.vs[0] + hk * p.vs[1] + g * 8;
+  const long long written = RING ? *p.ring : 0;
+  uint4 kq[2][2], vq[4];
+  const __nv_bfloat16 *kp = kb + (first + warp * 16 + g) * p.ks[2], *vp = vb + (first + warp * 16 + 2 * t) * p.vs[2];
+  auto load_k = [&](int j0) {
 #pragma unroll
-    for (int e = 0; e < 8; ++e) t.acc[e] = 0.f;
-    for (int w = 0; w < NWARPS; ++w) merge(t, part[w][r][0], part[w][r][1], &part[w][r][2 + s8 * 8]);
-    const float inv = t.l > 0.f ? 1.0f / t.l : 0.f;
-    const int gi = r / p.Sq, i = r - gi * p.Sq, h = hk * p.G + gi;
-    uint32_t o[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const __nv_bfloat162 b = __floats2bfloat162_rn(t.acc[2 * e] * inv, t.acc[2 * e + 1] * inv);
-      o[e] = *reinterpret_cast<const uint32_t*>(&b);
+    for (int h = 0; h < 2; ++h) {
+      const int j = j0 + row_attn::key_of_k(lane, h);
+      kq[h][0] = kq[h][1] = make_uint4(0, 0, 0, 0);
+      if (j < last) { kq[h][0] = load16(kp + h * 8 * p.ks[2]); kq[h][1] = load16(kp + h * 8 * p.ks[2] + 32); }
     }
-    *reinterpret_cast<uint4*>(p.out + n * p.os[0] + h * p.os[1] + i * p.os[2] + s8 * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+    kp += warps * 16 * p.ks[2];
+  };
+  auto load_v = [&](int j0) {
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      const int j = j0 + row_attn::key_of_v(lane, s);
+      vq[s] = make_uint4(0, 0, 0, 0);
+      if (j < last) vq[s] = load16(vp + ((s >> 1) * 8 + (s & 1)) * p.vs[2]);
+    }
+    vp += warps * 16 * p.vs[2];
+  };
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  const int span = warps * 16;
+  int jb = first + warp * 16;                  // this warp's sixteen
+  load_k(jb); load_v(jb);
+  const bool has_extra = extra && warp == 0;                     // warp-uniform
+  uint4 kx[2] = {zero, zero}, vx[2] = {zero, zero};
+  if (has_extra) {
+    const __nv_bfloat16* row = g == 1 ? kb + last * p.ks[2] : RING && g == 0 ? p.knew + n * p.ns[0] + hk * p.ns[1] + t * 8 : nullptr;
+    if (row) { kx[0] = load16(row); kx[1] = load16(row + 32); }
+    if (t == 0) {
+      if (RING) vx[0] = load16(p.vnew + n * p.ns[0] + hk * p.ns[1] + g * 8);
+      vx[1] = load16(vb + last * p.vs[2]);
+    }
+  }
+  // the query rows, and of this lane's row the ALiBi slope (in log2 units) and position
+  const __nv_bfloat16* qr[2] = {nullptr, nullptr};
+  float slope = 0.f;
+  int pos = 0, pos_of[2] = {0, 0};
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    if (r < rows) {
+      const int gi = (row0 + r) / p.Sq, i = row0 + r - gi * p.Sq, h = hk * p.G + gi;
+      qr[r] = p.q + n * p.qs[0] + h * p.qs[1] + i * p.qs[2];
+      pos_of[r] = p.T - p.Sq + i;
+      if (R == 1 || (t & 1) == r) { slope = p.slopes ? p.slopes[h] * GCA_LOG2E : 0.f; pos = pos_of[r]; }
+    }
+  if (rows < R) pos_of[R - 1] = pos_of[0];
+  const row_attn::Query q = row_attn::query<R>(qr[0], qr[1], lane);
+  // Ring: physical row `newest` is the new row's (the count stays below 2^32: caller's contract).  The linear form's newest row is the last one.
+  const int newest = RING ? (int)((unsigned)written % (unsigned)p.T) : last;
+  row_attn::State st;
+  row_attn::reset(st);
+  // a dot product as a score: how far key j lies behind this lane's row, and whether the row sees it
+  auto score = [&](float x, int j, bool there) {
+    int d = (RING ? newest : pos) - j;
+    if (RING && d < 0) d += p.T;
+    const bool sees = there && (RING ? d != 0 : d >= 0 && d <= p.window);
+    return sees ? fmaf(x, p.c2, -slope * (float)d) : -INFINITY;
+  };
+  // a key that the row does not see counts with zeros, whatever its row of V holds
+  auto blank_v = [&](int j0, int row_pos) {
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      const int d = (RING ? newest : row_pos) - (j0 + row_attn::key_of_v(lane, s));
+      if (RING ? d == 0 : d < 0 || d > p.window) vq[s] = make_uint4(0, 0, 0, 0);
+    }
+  };
+  if (has_extra) {
+    if (RING && blockIdx.y == 0) {                               // the new row over the oldest one, which nobody uses any more
+      if (g == 0) {
+        __nv_bfloat16* kd = const_cast<__nv_bfloat16*>(kb) + newest * p.ks[2];
+        *reinterpret_cast<uint4*>(kd) = kx[0]; *reinterpret_cast<uint4*>(kd + 32) = kx[1];
+      }
+      if (t == 0) *reinterpret_cast<uint4*>(const_cast<__nv_bfloat16*>(vb) + newest * p.vs[2]) = vx[0];
+    }
+    float s[2];
+    const uint4 k[2][2] = {{kx[0], kx[1]}, {zero, zero}}, v[4] = {vx[0], RING && newest == last ? zero : vx[1], zero, zero};
+    row_attn::scores(q, k, s);
+    s[0] = RING && g == 0 ? s[0] * p.c2 : score(s[0], last, g == 1);
+    s[1] = -INFINITY;
+    row_attn::accumulate<R>(st, s, v, lane);
+  }
+#pragma unroll 1
+  for (; jb < last; jb += span) {
+    float s[2];
+    row_attn::scores(q, kq, s);
+    load_k(jb + span);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) { const int j = jb + row_attn::key_of_k(lane, h); s[h] = score(s[h], j, j < last); }
+    if (RING || p.Sq > 1) blank_v(jb, pos_of[0]);
+    if (!RING && R == 2 && pos_of[0] != pos_of[R - 1] &&
+        ((jb + 15 > pos_of[0] && jb <= pos_of[R - 1]) || (jb + 15 >= pos_of[0] - p.window && jb < pos_of[R - 1] - p.window))) {
+      // a row sees a key that the other does not: first the one's, then the other's, each into its own columns only (a weight of 0 times
+      // an infinite value would not be nothing)
+#pragma unroll 1
+      for (int r = 0; r < 2; ++r) {
+        float mine[2] = {(t & 1) == r ? s[0] : -INFINITY, (t & 1) == r ? s[1] : -INFINITY}, keep[4][2];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { keep[i][0] = r ? st.acc[i][0] : st.acc[i][1]; keep[i][1] = r ? st.acc[i][2] : st.acc[i][3]; }
+        if (r) { vp -= span * p.vs[2]; load_v(jb); blank_v(jb, pos_of[R - 1]); }
+        row_attn::accumulate<R>(st, mine, vq, lane);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if (r) { st.acc[i][0] = keep[i][0]; st.acc[i][2] = keep[i][1]; }
+          else { st.acc[i][1] = keep[i][0]; st.acc[i][3] = keep[i][1]; }
+        }
+      }
+    } else {
+      row_attn::accumulate<R>(st, s, vq, lane);
+    }
+    load_v(jb + span);
+  }
+  float o[R][8];
+  row_attn::finish<R>(st, o);
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    float* dst = part[warp][r];
+    if (lane == r) { dst[0] = st.m; dst[1] = st.l; }            // lane r = row r's
+    if (t == 0) {
+#pragma unroll
+      for (int e = 0; e < 8; e += 2) *reinterpret_cast<float2*>(dst + 2 + g * 8 + e) = make_float2(o[r][e], o[r][e + 1]);
+    }
+  }
+  merge_and_store<R>(p, part, part[0], 1, 0, n, hk, row0, rows);
+}
+
+// Which kernel, and how the sixteens of an item (a kv head's row pair) are dealt out over warps and CTAs (a cluster).  All CTAs have to run at
+// once, and as few rounds as possible to follow one another.  So, the first of these that fits one wave (one row, us):
+//   once, one CTA        256 keys, 148 items 5.0 (two rounds 5.8), 256 items 6.8 (7.9)
+//   once, a cluster      of four, three or two CTAs where two have an SM to themselves: 640 keys, 4 items 4.6 (two rounds in one CTA 6.0)
+//   rounds               two, three .. in one CTA: 512 keys, 256 items three of eleven warps 9.8 (four of eight 10.9), 384 items four of eight 12.7
+// Within 1.2 % of the best of all splits on average over one and two rows x 64 .. 640 keys x 4 .. 768 items (caches from memory).  Two rows at
+// 80 registers a thread fit more warps and lose 10 % where both fit (512 keys, 148 items 8.2 against 7.4).
+struct WindowPlan { int ctas, warps; bool rounds; };
+#ifdef WINDOW_PLAN_PROBE
+WindowPlan g_probe_plan;
+#endif
+WindowPlan window_plan(long long items, int keys, int rows, int sms) {
+#ifdef WINDOW_PLAN_PROBE
+  return g_probe_plan;
+#endif
+  if (rows > 1) items *= (rows + 1) / 2;
+  auto fits = [&](int ctas, int warps, bool many) {
+    const int regs = rows > 1 ? WIN_REGS<2, true> : many ? WIN_REGS<1, true> : WIN_REGS<1, false>;
+    const int cap = rows > 1 ? WIN_WARPS<2, true> : many ? WIN_WARPS<1, true> : WIN_WARPS<1, false>;
+    return warps <= cap && items * ctas <= (long long)sms * (65536 / (32 * regs) / warps);
+  };
+  const int sixteens = std::max(1, (keys + 15) / 16);
+  if (fits(1, sixteens, false)) return {1, sixteens, false};
+  for (int ctas = 4; ctas > 1; --ctas) {
+    const int warps = (sixteens + ctas - 1) / ctas;
+    if (2 * items * ctas <= sms && fits(ctas, warps, false)) return {ctas, warps, false};
+  }
+  for (int rounds = std::max(2, (sixteens + 23) / 24);; ++rounds) {
+    const int warps = (sixteens + rounds - 1) / rounds;
+    if (warps <= 4 || fits(1, warps, true)) return {1, warps, true};
   }
 }
 
@@ -264,7 +468,7 @@ int launch_window_shift_append(const WindowAppendArgs& a, cudaStream_t stream) {
   return (int)cudaGetLastError();
 }
 
-static int launch_window(const WindowDecodeArgs& a, const WindowRingDecodeArgs* ring, cudaStream_t stream) {
+static int launch_window(const WindowDecodeArgs& a, const WindowRingDecodeArgs* ring, int sms, cudaStream_t stream) {
   WinParams p;
   p.knew = p.vnew = nullptr; p.ring = nullptr; p.ns[0] = p.ns[1] = 0;
   if (ring) {
@@ -276,18 +480,29 @@ static int launch_window(const WindowDecodeArgs& a, const WindowRingDecodeArgs* 
   for (int i = 0; i < 3; ++i) { p.qs[i] = a.q_stride[i]; p.os[i] = a.o_stride[i]; p.ks[i] = a.k_stride[i]; p.vs[i] = a.v_stride[i]; }
   p.N = a.N; p.Hq = a.Hq; p.Hkv = a.Hkv; p.G = a.Hq / a.Hkv; p.Sq = a.Sq; p.T = a.T; p.window = a.window;
   p.c2 = a.sm_scale * GCA_LOG2E;
-  const int rows = p.G * a.Sq;
-  const unsigned grid = (unsigned)(a.N * a.Hkv);
-  if (grid == 0) return 0;
-  auto run = [&](auto kernel) { return (int)launch_dependent(kernel, dim3(grid), dim3(NWARPS * 32), 0, stream, p); };
+  const int rows = p.G * a.Sq, items = a.N * a.Hkv;
+  if (items == 0) return 0;
   if (rows > 4) return GCA_ERR_SHAPE;
+  const WindowPlan plan = window_plan(items, p.T - (ring || a.Sq == 1 ? 1 : 0) - std::max(0, p.T - p.Sq - p.window), rows, sms);
+  auto run = [&](auto kernel) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(items * plan.ctas), (unsigned)((rows + 1) / 2)); cfg.blockDim = dim3((unsigned)(plan.warps * 32)); cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)plan.ctas; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = plan.ctas > 1 ? 2 : 1;
+    return (int)cudaLaunchKernelEx(&cfg, kernel, p, plan.ctas);
+  };
+  auto form = [&](auto once, auto rounds) { return plan.rounds ? run(rounds) : run(once); };
   if (ring)                                        // one new position: G rows per kv head
-    return rows <= 1 ? run(win_decode_kernel<1, true>) : rows <= 2 ? run(win_decode_kernel<2, true>) : run(win_decode_kernel<4, true>);
-  return rows <= 1 ? run(win_decode_kernel<1, false>) : rows <= 2 ? run(win_decode_kernel<2, false>) : run(win_decode_kernel<4, false>);
+    return rows <= 1 ? form(win_once_kernel<1, true>, win_rounds_kernel<1, true>) : form(win_once_kernel<2, true>, win_rounds_kernel<2, true>);
+  return rows <= 1 ? form(win_once_kernel<1, false>, win_rounds_kernel<1, false>) : form(win_once_kernel<2, false>, win_rounds_kernel<2, false>);
 }
 
-int launch_window_decode(const WindowDecodeArgs& a, cudaStream_t stream) { return launch_window(a, nullptr, stream); }
+int launch_window_decode(const WindowDecodeArgs& a, int sms, cudaStream_t stream) { return launch_window(a, nullptr, sms, stream); }
 
-int launch_window_ring_decode(const WindowRingDecodeArgs& a, cudaStream_t stream) { return launch_window(a.attn, &a, stream); }
+int launch_window_ring_decode(const WindowRingDecodeArgs& a, int sms, cudaStream_t stream) { return launch_window(a.attn, &a, sms, stream); }
 
 }  // namespace gca

@@ -206,6 +206,49 @@ def test_window_decode_against_float32(n, hq, hkv, sq, t, window, alibi):
     close(got, ref, (n, hq, hkv, sq, t, window))
 
 
+@pytest.mark.parametrize("items,g,sq,t,window", [
+    (3, 1, 1, 1, 7), (2, 1, 1, 2, 7), (4, 1, 1, 17, 16), (4, 1, 1, 18, 40),      # one warp: a single key, the last row beside one and sixteen keys
+    (5, 1, 1, 513, 512), (5, 2, 1, 641, 700), (12, 1, 1, 640, 639),              # clusters of CTAs
+    (60, 1, 1, 350, 349), (60, 2, 1, 200, 300), (148, 1, 1, 513, 512),           # one round, two rounds
+    (390, 1, 1, 200, 199), (150, 3, 1, 260, 300), (800, 2, 1, 66, 65),           # several rounds, a row pair that is half empty
+    (2, 1, 2, 40, 16), (150, 1, 2, 500, 300), (300, 2, 2, 300, 64),              # rows at two positions: each sees a key that the other does not
+])
+@pytest.mark.parametrize("poison", [False, True])
+def test_window_decode_splits(items, g, sq, t, window, poison):
+    """Every split of the keys over warps, CTAs and rounds, linear and (one position) ring; with `poison`, rows that no query may see
+    hold NaN, and one visible value is infinite: only that output column is."""
+    need_gpu()
+    from long_context_modeling_b200 import fused_ops as F
+    gen = torch.Generator().manual_seed(items + t)
+    h = 2 if items % 2 == 0 else 1
+    n = items // h
+    k, v = (torch.randn(n, h, t, 64, generator=gen).bfloat16().cuda() for _ in range(2))
+    q = torch.randn(n, h * g, sq, 64, generator=gen).bfloat16().cuda()
+    slopes = torch.linspace(0.02, 0.3, h * g).cuda()
+    k_seen, v_seen = k.clone(), v.clone()
+    if poison:
+        v[0, 0, t - sq, 5] = v_seen[0, 0, t - sq, 5] = float("inf")        # the first position's own row: every position sees it
+        if t - sq - window > 0:
+            k[:, :, :t - sq - window], v[:, :, :t - sq - window] = float("nan"), float("nan")
+    ref = _window_reference(q, k_seen, v_seen, window, slopes, 0.125)
+    forms = [F.window_decode(q, k, v, window, slopes, 0.125)]
+    if sq == 1 and t <= window + 1:
+        turn = 2 * t // 3                                          # the ring starts there; its oldest row is about to be overwritten
+        count = torch.full((1,), 5 * t + turn, dtype=torch.int64).cuda()
+        kr, vr = (torch.roll(x, turn + 1, 2) for x in (k, v))
+        if poison:
+            kr[:, :, turn], vr[:, :, turn] = float("nan"), float("nan")
+        forms.append(F.window_ring_decode(q, kr, vr, k[:, :, t - 1:].contiguous(), v[:, :, t - 1:].contiguous(), count, window, slopes, 0.125))
+        assert torch.equal(kr.roll(-(turn + 1), 2), k) and torch.equal(vr.roll(-(turn + 1), 2), v)
+    for got in forms:
+        got = got.float().cpu()
+        inf = torch.isinf(ref)
+        assert torch.equal(torch.isinf(got), inf) and not torch.isnan(got).any()
+        got, want = got.masked_fill(inf, 0.0), ref.masked_fill(inf, 0.0)
+        # bf16: eight significant bits, the error half a unit of the last place, 2^-8 of the value; float32 sums (2^-18 of the largest)
+        assert ((got - want).abs() <= want.abs() * 2.0 ** -8 + 2.0 ** -18 * want.abs().max()).all()
+
+
 def test_window_decode_reads_strided_caches():
     """k / v as (N, T, H, 64) token-major storage viewed as (N, H, T, 64): the reference's cache layout."""
     need_gpu()
