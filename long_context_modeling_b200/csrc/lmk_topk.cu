@@ -18,6 +18,7 @@
 #include <algorithm>
 
 #include "lmk_common.cuh"
+#include "sm100_ptx.cuh"
 
 namespace gca {
 // lmk_tc_sm100.cu: many query rows per sequence
@@ -100,9 +101,33 @@ __device__ __forceinline__ void select_batch(unsigned long long& mine, unsigned 
 constexpr int BATCH = 64, STREAM_WARPS = 16;
 template <int NP> constexpr int RING_ROWS = NP > 3 ? 6 : 8;       // 196 KB per SM
 
-template <int NP, bool PER_HEAD>
+// The K best of up to 32 descending lists, lane l at the head of list l: K times the best head, found by a warp-wide maximum, moves on.
+// `at(i)`: this lane's list's entry i (0 past the end of a short list); lanes without a list pass has = false.
+template <class At>
+__device__ __forceinline__ unsigned long long merge_heads(int K, bool has, int lane, At at) {
+  unsigned long long head = has ? at(0) : 0ull, next = has && K > 1 ? at(1) : 0ull, mine = 0ull;
+  int taken = 1;
+  for (int i = 0; i < K; ++i) {
+    const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(head >> 32));
+    if (hi == 0u) break;
+    const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(head >> 32) == hi ? (unsigned)head : 0u);
+    const unsigned long long best = ((unsigned long long)hi << 32) | lo;
+    if (lane == i) mine = best;
+    if (head == best) { head = next; ++taken; next = taken < K ? at(taken) : 0ull; }
+  }
+  return mine;
+}
+__device__ __forceinline__ unsigned long long ld_dsmem_u64(const unsigned long long* p, int rank) {       // the same variable in another CTA of the cluster
+  unsigned long long v;
+  asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %1, %2;\n\tld.shared::cluster.u64 %0, [a];\n\t}" : "=l"(v) : "r"(sm100::smem_u32(p)), "r"(rank) : "memory");
+  return v;
+}
+
+// FUSED: the blocks of a row are a cluster, and the first one merges their lists and writes the row's outputs: no lists in memory, no
+// second launch.  When, is said at fused().
+template <int NP, bool PER_HEAD, bool FUSED>
 __global__ void __launch_bounds__(STREAM_WARPS * 32, 1)
-lmk_stream_kernel(ScanParams p) {
+lmk_stream_kernel(ScanParams p, FinalParams fin) {
   constexpr int RING = RING_ROWS<NP>, NL = PER_HEAD ? NP * 4 : 1, MINE = (NL + STREAM_WARPS - 1) / STREAM_WARPS, ROW_BYTES = NP * 512;
   extern __shared__ __align__(16) unsigned char ring_all[];            // [STREAM_WARPS][RING][ROW_BYTES]
   __shared__ float score[2][NL][BATCH];
@@ -202,6 +227,22 @@ lmk_stream_kernel(ScanParams p) {
       }
       select_batch(mine[x], kth[x], e0 < e_hi ? orderable(s0) : 0u, e1 < e_hi ? orderable(s1) : 0u, (unsigned)(p.e_base + e_lo + b * BATCH), p.K, lane);
     }
+  }
+  if (FUSED) {
+    __shared__ unsigned long long lists[FUSED ? NL : 1][MAXK];
+#pragma unroll
+    for (int x = 0; x < MINE; ++x)
+      if (warp + x * STREAM_WARPS < NL) lists[warp + x * STREAM_WARPS][lane] = mine[x];
+    sm100::cluster_sync();
+    if (split == 0) {
+#pragma unroll 1
+      for (int l = warp; l < NL && (!PER_HEAD || l < p.H); l += STREAM_WARPS) {
+        const unsigned long long best = merge_heads(p.K, lane < p.splits, lane, [&](int i) { return ld_dsmem_u64(&lists[l][i], lane); });
+        emit_row(fin, ((long long)n * p.Cq + t0) * p.H + l, best, lane);
+      }
+    }
+    sm100::cluster_sync();                                     // nobody leaves while its lists may be read
+    return;
   }
 #pragma unroll
   for (int x = 0; x < MINE; ++x) {
@@ -356,8 +397,7 @@ __device__ void finalize_row(const FinalParams& p, long long row, const unsigned
   emit_row(p, row, m, lane);
 }
 
-// The scan's lists of a row merged by one warp (up to 32 lists; eight rows per block): lane l stands at the head of list
-// l, and K times the best head is taken by a warp-wide maximum and its list moves on.
+// The scan's lists of a row merged by one warp (up to 32 lists; eight rows per block).
 __global__ void __launch_bounds__(FIN_WARPS * 32)
 lmk_merge_rows_kernel(FinalParams p) {
   const int lane = threadIdx.x & 31;
@@ -366,17 +406,7 @@ lmk_merge_rows_kernel(FinalParams p) {
   pdl_wait();
   if (row >= p.R) return;
   const unsigned long long* src = p.keys + row * p.P + (long long)lane * p.K;
-  unsigned long long head = lane < p.lists ? src[0] : 0ull, next = lane < p.lists && p.K > 1 ? src[1] : 0ull, mine = 0ull;
-  int at = 1;
-  for (int i = 0; i < p.K; ++i) {
-    const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(head >> 32));
-    if (hi == 0u) break;
-    const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(head >> 32) == hi ? (unsigned)head : 0u);
-    const unsigned long long best = ((unsigned long long)hi << 32) | lo;
-    if (lane == i) mine = best;
-    if (head == best) { head = next; ++at; next = at < p.K ? src[at] : 0ull; }
-  }
-  emit_row(p, row, mine, lane);
+  emit_row(p, row, merge_heads(p.K, lane < p.lists, lane, [&](int i) { return src[i]; }), lane);
 }
 
 // Many lists per row (a long cache scanned by every SM): one block per row, no serial insertion.  An entry e of a
@@ -544,8 +574,9 @@ int scan_splits(const LmkTopkArgs& a, int sms) {
 
 namespace {
 
-// Landmark ranges of the streaming form: one block per SM at a time, so what counts is whole waves; a block costs about as much
-// again as reading 96 rows before and after its stream.
+// Landmark ranges of the streaming form: one block per SM at a time, so what counts is whole waves; a wave costs about as much
+// again as reading 200 rows before and after its stream (32 rows x 4,096 landmarks: one wave of 4 ranges 36 us, two of 9 41; x 8,192
+// 66 either way).
 int most_stream_splits(const LmkTopkArgs& a, int sms) { return (int)std::min<long long>((a.E + BATCH - 1) / BATCH, 2 * sms); }
 int stream_splits(const LmkTopkArgs& a, int sms) {
   const long long blocks = (long long)a.N * a.Cq;
@@ -553,7 +584,7 @@ int stream_splits(const LmkTopkArgs& a, int sms) {
   int best = 1;
   long long best_cost = -1;
   for (int s = 1; s <= most; ++s) {
-    const long long cost = (blocks * s + sms - 1) / sms * ((a.E + s - 1) / s + 96);
+    const long long cost = (blocks * s + sms - 1) / sms * ((a.E + s - 1) / s + 200);
     if (best_cost < 0 || cost < best_cost) { best = s; best_cost = cost; }
   }
   return best;
@@ -563,18 +594,36 @@ int choose_splits(const LmkTopkArgs& a, int sms) {
   return a.splits > 0 ? a.splits : pick_tq(a) == 1 ? stream_splits(a, sms) : scan_splits(a, sms);
 }
 
-template <int NP, bool PER_HEAD>
-int launch_stream(const ScanParams& sp, dim3 grid, cudaStream_t stream) {
+// A row's blocks are a cluster that merges for itself where they are at most eight anyway and all clusters find their SMs, in one group of
+// them each: 256 landmarks x 1 row 6.9 us either way (the merge kernel is on its way before the scan ends) but one launch less on
+// the host, calls in a row 9.1 -> 7.3 us; 64 landmarks 6.6 -> 5.7 us.  A cluster of eight in place of more blocks costs more than it saves
+// (1,000 landmarks: 16 blocks and a merge 6.7 us, a cluster 9.2).
+bool fused(const LmkTopkArgs& a, int splits, int sms) {
+  const int slack = splits == 1 ? 0 : splits < 5 ? 1 : splits;
+  return splits <= 8 && (long long)a.N * a.Cq * splits * (16 + slack) <= 16ll * sms;
+}
+
+template <int NP, bool PER_HEAD, bool FUSED>
+int launch_stream(const ScanParams& sp, const FinalParams& fp, dim3 grid, cudaStream_t stream) {
   constexpr int smem = STREAM_WARPS * RING_ROWS<NP> * NP * 512;
-  GCA_CUDA_CHECK(cudaFuncSetAttribute(lmk_stream_kernel<NP, PER_HEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  return (int)launch_dependent(lmk_stream_kernel<NP, PER_HEAD>, grid, dim3(STREAM_WARPS * 32), smem, stream, sp);
+  auto kernel = lmk_stream_kernel<NP, PER_HEAD, FUSED>;
+  GCA_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = dim3(STREAM_WARPS * 32); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = grid.x; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = FUSED && grid.x > 1 ? 2 : 1;
+  return (int)cudaLaunchKernelEx(&cfg, kernel, sp, fp);
 }
 
 template <int NP>
-int launch_scan(const ScanParams& sp, int tq, bool per_head, cudaStream_t stream) {
+int launch_scan(const ScanParams& sp, const FinalParams& fp, int tq, bool per_head, bool fused, cudaStream_t stream) {
   const dim3 grid((unsigned)sp.splits, (unsigned)((sp.Cq + tq - 1) / tq), (unsigned)sp.N);
-  if (per_head) return launch_stream<NP, true>(sp, grid, stream);
-  if (tq == 1) return launch_stream<NP, false>(sp, grid, stream);
+  if (per_head) return fused ? launch_stream<NP, true, true>(sp, fp, grid, stream) : launch_stream<NP, true, false>(sp, fp, grid, stream);
+  if (tq == 1) return fused ? launch_stream<NP, false, true>(sp, fp, grid, stream) : launch_stream<NP, false, false>(sp, fp, grid, stream);
   lmk_scan_kernel<NP, 4><<<grid, SCAN_WARPS * 32, 0, stream>>>(sp);
   return (int)cudaGetLastError();
 }
@@ -612,8 +661,11 @@ int launch_lmk_score_topk(const LmkTopkArgs& a, void* scratch, int sms, cudaStre
   fp.R = (int)rows; fp.P = 0; fp.K = a.K; fp.lists = 0;
   if (lmk_screen_applies(a)) return launch_lmk_screen(a, scratch, sms, fp, stream);
   const int tq = pick_tq(a), splits = choose_splits(a, sms);
+  const bool cluster = tq == 1 && fused(a, splits, sms);
+  if (a.noise == nullptr || per_head) fp.lq = nullptr;          // the keys hold the noise-free scores
+  fp.P = splits * a.K; fp.lists = splits;
   ScanParams sp;
-  sp.lq = fp.lq; sp.lk = fp.lk; sp.noise = a.noise;
+  sp.lq = (const __nv_bfloat16*)a.lmk_q; sp.lk = fp.lk; sp.noise = a.noise;
   sp.part = (unsigned long long*)scratch;
   sp.qbs = a.q_batch_stride; sp.qrs = a.q_row_stride; sp.kbs = a.k_batch_stride; sp.krs = a.k_row_stride;
   sp.q_pos0 = a.q_pos0; sp.e_base = a.e_base;
@@ -622,15 +674,14 @@ int launch_lmk_score_topk(const LmkTopkArgs& a, void* scratch, int sms, cudaStre
   sp.score_round = a.score_round; sp.scale = scale;
   int rc;
   switch ((a.D + 255) / 256) {
-    case 1: rc = launch_scan<1>(sp, tq, per_head, stream); break;
-    case 2: rc = launch_scan<2>(sp, tq, per_head, stream); break;
-    case 3: rc = launch_scan<3>(sp, tq, per_head, stream); break;
-    case 4: rc = launch_scan<4>(sp, tq, per_head, stream); break;
+    case 1: rc = launch_scan<1>(sp, fp, tq, per_head, cluster, stream); break;
+    case 2: rc = launch_scan<2>(sp, fp, tq, per_head, cluster, stream); break;
+    case 3: rc = launch_scan<3>(sp, fp, tq, per_head, cluster, stream); break;
+    case 4: rc = launch_scan<4>(sp, fp, tq, per_head, cluster, stream); break;
     default: rc = GCA_ERR_SHAPE;
   }
   if (rc) return rc;
-  if (a.noise == nullptr || per_head) fp.lq = nullptr;          // the keys hold the noise-free scores
-  fp.P = splits * a.K; fp.lists = splits;
+  if (cluster) return 0;
   // a warp per row up to 32 lists, a block per row beyond
   if (splits <= 32)
     return (int)launch_dependent(lmk_merge_rows_kernel, dim3((unsigned)((rows + FIN_WARPS - 1) / FIN_WARPS)), dim3(FIN_WARPS * 32), 0, stream, fp);

@@ -367,6 +367,23 @@ def test_tensor_core_screening_with_copies_of_landmarks(lcm, copies):
     check(res, oracle_rows(lq, lk, 8, q_pos0=260))
 
 
+@pytest.mark.parametrize("n,cq,e,d,k,per_head,noisy", [
+    (1, 1, 3, 768, 8, False, False), (1, 1, 64, 768, 1, True, False),       # one block, fewer landmarks than places
+    (2, 3, 65, 512, 32, False, True), (3, 2, 449, 256, 7, True, False),     # two and eight blocks, a last one of a single landmark, hidden landmarks
+    (5, 1, 512, 1024, 16, True, False), (12, 1, 500, 768, 8, False, True),  # clusters of eight
+    (32, 1, 200, 768, 8, False, False), (40, 1, 512, 768, 8, False, False),     # clusters of four; too many rows for clusters
+])
+def test_scan_that_merges_for_itself(lcm, n, cq, e, d, k, per_head, noisy):
+    lq, lk = cases.landmark_case(36, n, cq, e, d=d)
+    head_dim = 64 if per_head else 0
+    noise = -torch.empty(n, cq, e).exponential_(generator=torch.Generator().manual_seed(4)).log() if noisy else None
+    lk[:, e // 2] = lk[:, 0]                                   # a tie between blocks
+    res = lcm.lmk_score_topk(lq.cuda(), lk.cuda(), k, q_pos0=e - 1, noise=None if noise is None else noise.cuda(), head_dim=head_dim)
+    check(res, oracle_rows(lq, lk, k, q_pos0=e - 1, noise=noise, head_dim=head_dim))
+    apart = lcm.lmk_score_topk(lq.cuda(), lk.cuda(), k, q_pos0=e - 1, noise=None if noise is None else noise.cuda(), head_dim=head_dim, splits=9)
+    assert all(torch.equal(a, b) for a, b in zip(res, apart))
+
+
 @pytest.mark.parametrize("e,k,splits", [(9000, 32, 33), (70001, 1, 0), (5000, 7, 1024), (3000, 8, 1500)])
 def test_many_candidate_lists_per_row(lcm, e, k, splits):
     lq, lk = cases.landmark_case(32, 1, 1, e, d=128)
