@@ -453,6 +453,10 @@ typedef struct LinearBatchedArgs {
 
 int gca_linear_batched(const LinearBatchedArgs* args, void* stream);
 
+/* gca_linear_batched with rms_eps for any number of rows (one.row_scale NULL, lead_rows 0): the rows' factors come from the tiles of x as they
+ * are multiplied, or from a launch before into `scratch`, batches * one.M floats, which is the call's to write to. */
+int gca_rms_linear_batched(const LinearBatchedArgs* args, float* scratch, void* stream);
+
 /* 1 where M rows of K -> N are faster in the latency-bound form on the current device than as tiles of the tensor cores, which
  * gca_linear goes by.  with_norm: RMSNorm + projection as one call with rms_eps against gca_row_rms and a call with row_scale. */
 int gca_linear_few_rows(int64_t M, int32_t N, int32_t K, int32_t with_norm);

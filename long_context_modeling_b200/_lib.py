@@ -188,6 +188,7 @@ EXPORTS = {
     "gca_row_rms": (C.c_int, [C.POINTER(RowRmsArgs), C.c_void_p]),
     "gca_linear": (C.c_int, [C.POINTER(LinearArgs), C.c_void_p]),
     "gca_linear_batched": (C.c_int, [C.POINTER(LinearBatchedArgs), C.c_void_p]),
+    "gca_rms_linear_batched": (C.c_int, [C.POINTER(LinearBatchedArgs), C.c_void_p, C.c_void_p]),
     "gca_linear_few_rows": (C.c_int, [C.c_int64, C.c_int32, C.c_int32, C.c_int32]),
     "gca_silu_mul": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int64, C.c_int32, C.c_int64, C.c_int64, C.c_void_p]),
     "gca_window_decode": (C.c_int, [C.POINTER(WindowDecodeArgs), C.c_void_p]),

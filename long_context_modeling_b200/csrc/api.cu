@@ -15,7 +15,7 @@ int launch_cache_append(const CacheAppendArgs& a, cudaStream_t stream);
 int launch_kv_project_append(const KvProjectArgs& a, int sms, cudaStream_t stream);
 int launch_row_rms(const RowRmsArgs& a, cudaStream_t stream);
 int launch_silu_mul(const void* gu, void* out, long long M, int I, long long in_stride, long long out_stride, cudaStream_t stream);
-int launch_linear(const LinearBatchedArgs& a, int sms, cudaStream_t stream);
+int launch_linear(const LinearBatchedArgs& a, float* norm_scratch, int sms, cudaStream_t stream);
 bool few_rows(long long M, int N, int K, bool with_norm, int sms);
 int launch_layer_decode(const LayerDecodeArgs& a, int dev, cudaStream_t stream);
 int launch_window_decode(const WindowDecodeArgs& a, int sms, cudaStream_t stream);
@@ -464,7 +464,7 @@ int gca_window_ring_decode(const WindowRingDecodeArgs* a, void* stream) {
   return gca::launch_window_ring_decode(*a, gca::sm_count(scope.dev), (cudaStream_t)stream);
 }
 
-int gca_linear_batched(const LinearBatchedArgs* b, void* stream) {
+static int linear_batched(const LinearBatchedArgs* b, float* norm_scratch, void* stream) {
   if (!b) return GCA_ERR_NULL;
   const LinearArgs* a = &b->one;
   if (!a->x || !a->w || !a->out) return GCA_ERR_NULL;
@@ -478,7 +478,15 @@ int gca_linear_batched(const LinearBatchedArgs* b, void* stream) {
   if (a->M == 0 || b->batches == 0) return 0;
   gca::DeviceScope scope(a->out);
   if (scope.rc) return scope.rc;
-  return gca::launch_linear(*b, gca::sm_count(scope.dev), (cudaStream_t)stream);
+  return gca::launch_linear(*b, norm_scratch, gca::sm_count(scope.dev), (cudaStream_t)stream);
+}
+
+int gca_linear_batched(const LinearBatchedArgs* b, void* stream) { return linear_batched(b, nullptr, stream); }
+
+int gca_rms_linear_batched(const LinearBatchedArgs* b, float* scratch, void* stream) {
+  if (!b || !scratch) return GCA_ERR_NULL;
+  if (b->one.row_scale || b->lead_rows != 0) return GCA_ERR_SHAPE;
+  return linear_batched(b, scratch, stream);
 }
 
 int gca_linear_few_rows(int64_t M, int32_t N, int32_t K, int32_t with_norm) {

@@ -51,7 +51,7 @@ struct Api {
 #define GCA_API_LIST                                                                                          \
   GCA_API(gca_fwd) GCA_API(gca_decode) GCA_API(gca_bwd_stages) GCA_API(gca_bwd_workspace_bytes)               \
   GCA_API(lmk_score_topk_kept) GCA_API(lmk_topk_workspace_bytes) GCA_API(lmk_weights_backward) GCA_API(gca_kv_project_append) GCA_API(gca_row_rms) \
-  GCA_API(gca_linear) GCA_API(gca_linear_batched) GCA_API(gca_linear_few_rows) GCA_API(gca_layer_decode) GCA_API(gca_silu_mul) GCA_API(gca_window_decode)            \
+  GCA_API(gca_linear) GCA_API(gca_linear_batched) GCA_API(gca_rms_linear_batched) GCA_API(gca_linear_few_rows) GCA_API(gca_layer_decode) GCA_API(gca_silu_mul) GCA_API(gca_window_decode)            \
   GCA_API(gca_window_ring_decode) GCA_API(gca_strerror)
   GCA_API_LIST
 #undef GCA_API
@@ -466,12 +466,11 @@ Tensor linear(const Tensor& x, const Tensor& weight, const Tensor& row_scale, co
   return out;
 }
 
-// RMSNorm(x) w^T with the norm's gain in w: a few rows are one launch, more take a row reduction and the GEMM's epilogue.
+// RMSNorm(x) w^T with the norm's gain in w: a few rows take the latency-bound kernel, more the GEMM that sums the squares up on the way.
 Tensor rmsnorm_linear(const Tensor& x, const Tensor& weight, double eps) {
   at::AutoDispatchBelowADInplaceOrView below;
   const Rows r = rows_of(x);
   Launch on(x);
-  if (!api.gca_linear_few_rows(r.m, (int32_t)weight.size(0), (int32_t)x.size(-1), 1)) return linear(x, weight, row_rms(x, eps), Tensor(), Tensor());
   c10::SmallVector<int64_t, 6> shape(x.sizes().begin(), x.sizes().end());
   shape.back() = weight.size(0);
   const Tensor out = at::empty(shape, x.options());
@@ -480,7 +479,12 @@ Tensor rmsnorm_linear(const Tensor& x, const Tensor& weight, double eps) {
   lp.one.M = r.m; lp.one.N = (int32_t)weight.size(0); lp.one.K = (int32_t)x.size(-1);
   lp.one.x_stride = r.stride; lp.one.w_stride = weight.stride(0); lp.one.out_stride = weight.size(0);
   lp.batches = 1; lp.rms_eps = (float)eps;
-  call("gca_linear", [&] { return api.gca_linear_batched(&lp, on.stream); });
+  if (api.gca_linear_few_rows(r.m, (int32_t)weight.size(0), (int32_t)x.size(-1), 1))
+    call("gca_linear", [&] { return api.gca_linear_batched(&lp, on.stream); });
+  else {
+    const Tensor scratch = at::empty({r.m}, x.options().dtype(at::kFloat));
+    call("gca_linear", [&] { return api.gca_rms_linear_batched(&lp, scratch.mutable_data_ptr<float>(), on.stream); });
+  }
   return out;
 }
 
@@ -548,24 +552,19 @@ Tensor layer_fused(const Tensor& hidden_in, const Tensor& q_weight, double eps, 
   const bool few = skip == 0 && api.gca_linear_few_rows(n * rows, (int32_t)q_weight.size(0), (int32_t)dim, 1);       // the norm rides on the projection
   const Tensor q = at::empty({2, n, J, s, dim}, hidden.options());      // [0]: q, [1]: the attention's output
   void* const vals = static_cast<char*>(q.mutable_data_ptr()) + q.stride(0) * 2;
-  Tensor scale;
-  if (!few) {
-    scale = at::empty({n * chunks * s}, hidden.options().dtype(at::kFloat));
-    RowRmsArgs rr;
-    rr.x = hidden.const_data_ptr(); rr.row_scale = scale.mutable_data_ptr<float>(); rr.M = n * chunks * s; rr.x_stride = dim;
-    rr.D = (int32_t)dim; rr.eps = (float)eps;
-    call("gca_row_rms", [&] { return api.gca_row_rms(&rr, on.stream); });
-  }
   LinearBatchedArgs lp{};
   LinearArgs& a = lp.one;
   a.x = static_cast<const char*>(hidden.const_data_ptr()) + skip * s * dim * 2; a.w = q_weight.const_data_ptr(); a.out = q.mutable_data_ptr();
   a.M = rows; a.N = (int32_t)q_weight.size(0); a.K = (int32_t)dim;
   a.x_stride = dim; a.w_stride = q_weight.stride(0); a.out_stride = dim;
-  if (few) lp.rms_eps = (float)eps;
-  else a.row_scale = scale.const_data_ptr<float>() + skip * s;
+  lp.rms_eps = (float)eps;
   a.status = status_ptr(on.dev);
-  lp.batches = (int32_t)n; lp.x_batch_stride = chunks * s * dim; lp.out_batch_stride = rows * dim; lp.scale_batch_stride = chunks * s;
-  call("gca_linear", [&] { return api.gca_linear_batched(&lp, on.stream); });
+  lp.batches = (int32_t)n; lp.x_batch_stride = chunks * s * dim; lp.out_batch_stride = rows * dim;
+  if (few) call("gca_linear", [&] { return api.gca_linear_batched(&lp, on.stream); });
+  else {
+    const Tensor scratch = at::empty({n * rows}, hidden.options().dtype(at::kFloat));
+    call("gca_linear", [&] { return api.gca_rms_linear_batched(&lp, scratch.mutable_data_ptr<float>(), on.stream); });
+  }
   // q as (n, J, heads, s, head_dim) by strides
   p.qs[0] = rows * dim; p.qs[1] = s * dim; p.qs[2] = head_dim; p.qs[3] = dim;
   GcaFwdArgs f = fwd_args(p, q, k, v, idx, w, q, p.qs, nullptr, sm_scale, 0.0, GCA_ALGO_AUTO, on.dev);

@@ -25,9 +25,12 @@
 //
 // The same kernel in LINEAR mode is the projection either side of GCA (model/DRT.py:352-355,385):
 //   out[m, :] = row_scale[m] * (x[m, :] W^T) + residual[m, :]
-// row_scale = 1 / rms(x) from `row_rms_kernel` turns it into pre-norm RMSNorm + q_proj (the norm's
-// gain is folded into W's columns by the caller: RMSNorm(x) W^T = diag(1 / rms) x (W diag(g))^T, so
-// the normalised activations are never written), residual makes it o_proj + residual add.
+// row_scale = 1 / rms(x) turns it into pre-norm RMSNorm + q_proj (the norm's gain is folded into W's
+// columns by the caller: RMSNorm(x) W^T = diag(1 / rms) x (W diag(g))^T, so the normalised activations
+// are never written), residual makes it o_proj + residual add.  The factors come from the tiles of x as
+// they pass (NORM); for pairs, whose tiles arrive on the leader's barriers alone, `row_rms_kernel` reads x
+// before.  768 -> 768, 640 / 2,368 / 7,104 rows, x from memory: 6.8 / 8.1 / 14.5 us, with that launch before
+// 8.0 / 11.2 / 17.1.
 //
 // CROSS-ENTROPY mode is the LM head fused with the loss (model/DRT.py:1055-1064, inference /
 // evaluation): the 128 x 256 logit tiles stay in tensor memory, the epilogue reduces each row's tile
@@ -39,6 +42,8 @@
 #include "tc_common.cuh"
 #include "tma_host.cuh"
 
+#include <type_traits>
+
 namespace gca {
 
 namespace {
@@ -46,7 +51,7 @@ namespace {
 using namespace sm100;
 
 constexpr int BM = 128, BK = 64;                      // rows of a CTA's accumulator, K step
-constexpr int EPI_WARPS = 8, W_WARP = 2 + EPI_WARPS, NTHREADS = (3 + EPI_WARPS) * 32;
+constexpr int EPI_WARPS = 8, W_WARP = 2 + EPI_WARPS, NTHREADS = (3 + EPI_WARPS) * 32, STAT_WARPS = 4;
 
 // BN: columns of a tile.  PAIR: two CTAs share a tile of 256 rows (cta_group::2), each loading half of the weight rows.
 template <int BN, bool PAIR>
@@ -54,8 +59,9 @@ struct Cfg {
   static constexpr int B_ROWS = PAIR ? BN / 2 : BN;
   static constexpr int A_BYTES = BM * BK * 2, STAGE_BYTES = A_BYTES + B_ROWS * BK * 2;
   static constexpr int STAGES = 196608 / STAGE_BYTES;
-  static constexpr int OFF_BAR = STAGES * STAGE_BYTES, SMEM_BYTES = OFF_BAR + 256 + 1024;
-  static constexpr int FULL = 0, EMPTY = FULL + STAGES, ACC_FULL = EMPTY + STAGES, ACC_EMPTY = ACC_FULL + 2, NUM_BARS = ACC_EMPTY + 2;
+  static constexpr int OFF_BAR = STAGES * STAGE_BYTES, OFF_SCALE = OFF_BAR + 256, SMEM_BYTES = OFF_SCALE + 2 * BM * 4 + 1024;
+  static constexpr int FULL = 0, EMPTY = FULL + STAGES, ACC_FULL = EMPTY + STAGES, ACC_EMPTY = ACC_FULL + 2, SCALE_FULL = ACC_EMPTY + 2,
+                       NUM_BARS = SCALE_FULL + 2;
   static constexpr uint32_t IDESC = umma_idesc_bf16(PAIR ? 2 * BM : BM, BN, 0, 0);
   static constexpr int TM = PAIR ? 2 * BM : BM;        // rows of a tile
   static constexpr int ACC_COLS = BN > 128 ? 256 : BN;  // tensor-memory columns of an accumulator
@@ -85,6 +91,7 @@ struct ProjParams {
   __nv_bfloat16* out;
   const __nv_bfloat16* residual;      // or nullptr
   const float* row_scale;             // or nullptr
+  float rms_eps;                      // NORM: what the rows' mean squares get added
   long long out_stride, res_stride;   // elements between rows
   int ncols;                          // output columns (multiple of 16; any number in cross-entropy mode)
   // cross-entropy mode (linear mode with ce_part != nullptr): the logits never leave tensor memory
@@ -101,25 +108,30 @@ __device__ __forceinline__ void tile_of(const ProjParams& p, int t, int& which, 
   else { which = 0; tm = r; }
 }
 
-template <int BN, bool PAIR>
-__global__ void __launch_bounds__(NTHREADS, 1)
+// NORM (linear mode, no pairs): the rows are scaled by 1 / rms(x), from the tiles of x as they pass through shared memory: four warps more
+// read them beside the MMAs, each thread a row of 64 values, and hand the row's factor to the epilogue.  Every column tile sums its
+// rows up again: 16 KB of shared memory per 64-deep stage beside the 24 to 48 KB that the MMAs read.
+template <int BN, bool PAIR, bool NORM>
+__global__ void __launch_bounds__(NTHREADS + (NORM ? STAT_WARPS * 32 : 0), 1)
 kv_project_append_kernel(const __grid_constant__ ProjParams p) {
+  static_assert(!(PAIR && NORM), "a pair's tiles arrive on the leader's barriers alone");
   using C = Cfg<BN, PAIR>;
   constexpr int STAGES = C::STAGES, STAGE_BYTES = C::STAGE_BYTES, A_BYTES = C::A_BYTES, OFF_BAR = C::OFF_BAR, NUM_BARS = C::NUM_BARS;
-  constexpr int FULL = C::FULL, EMPTY = C::EMPTY, ACC_FULL = C::ACC_FULL, ACC_EMPTY = C::ACC_EMPTY, ACC_COLS = C::ACC_COLS, TMEM_COLS = 2 * ACC_COLS;
+  constexpr int FULL = C::FULL, EMPTY = C::EMPTY, ACC_FULL = C::ACC_FULL, ACC_EMPTY = C::ACC_EMPTY, SCALE_FULL = C::SCALE_FULL, ACC_COLS = C::ACC_COLS, TMEM_COLS = 2 * ACC_COLS;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + NUM_BARS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + NUM_BARS + 1);
+  float* scale = reinterpret_cast<float*>(smem + C::OFF_SCALE);           // NORM: [accumulator][row]
   const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int total = p.tiles_m * p.tiles_n * p.nmat;
   const int ksteps = p.D / BK;
   const uint32_t rank = PAIR ? cluster_rank() : 0u;
   const int first = PAIR ? blockIdx.x / 2 : blockIdx.x, step = PAIR ? gridDim.x / 2 : gridDim.x;
   if (threadIdx.x == 0) {
-    for (int i = 0; i < STAGES; ++i) { mbar_init(&bars[FULL + i], 2); mbar_init(&bars[EMPTY + i], 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&bars[ACC_FULL + i], 1); mbar_init(&bars[ACC_EMPTY + i], (PAIR ? 2 : 1) * EPI_WARPS); }
+    for (int i = 0; i < STAGES; ++i) { mbar_init(&bars[FULL + i], 2); mbar_init(&bars[EMPTY + i], NORM ? 1 + STAT_WARPS : 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&bars[SCALE_FULL + i], STAT_WARPS); mbar_init(&bars[ACC_FULL + i], 1); mbar_init(&bars[ACC_EMPTY + i], (PAIR ? 2 : 1) * EPI_WARPS); }
     *abort_flag = 0;
     fence_barrier_init();
   }
@@ -210,6 +222,38 @@ kv_project_append_kernel(const __grid_constant__ ProjParams p) {
         else umma_commit_elect(&bars[ACC_FULL + ab]);
       }
     }
+  } else if (NORM && warp > W_WARP) {
+    const int row = (warp - W_WARP - 1) * 32 + lane;
+    Ring ring; ring.init(STAGES);
+    bool ok = true;
+    uint32_t tcount = 0;
+    for (int t = first; t < total && ok; t += step, ++tcount) {
+      float2 sq[4] = {};                                   // eight sums of a row, then their sum: chains of K / 8
+      for (int ks = 0; ks < ksteps; ++ks) {
+        ok = mbar_wait_warp(&bars[FULL + ring.st], ring.ph, abort_flag, lane);
+        if (!ok) break;
+        const uint4* x = reinterpret_cast<const uint4*>(smem + ring.st * STAGE_BYTES + row * 128);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          const uint4 v = x[c ^ (row & 7)];
+          const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float2 f = make_float2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
+            sq[i] = __ffma2_rn(f, f, sq[i]);
+          }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars[EMPTY + ring.st]);
+        ring.next();
+      }
+      const uint32_t ab = tcount & 1;
+      ok = ok && mbar_wait_warp(&bars[ACC_EMPTY + ab], ((tcount >> 1) & 1) ^ 1, abort_flag, lane);       // the factors before have been read
+      if (!ok) break;
+      scale[ab * BM + row] = rsqrtf((((sq[0].x + sq[0].y) + (sq[1].x + sq[1].y)) + ((sq[2].x + sq[2].y) + (sq[3].x + sq[3].y))) / (float)p.D + p.rms_eps);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars[SCALE_FULL + ab]);
+    }
   } else {
     // epilogue: thread = accumulator lane = row of the tile
     const int quad = warp & 3, half = (warp - 2) >> 2;   // warps 2..9: every TMEM lane quarter twice, one half of the columns each
@@ -250,6 +294,7 @@ kv_project_append_kernel(const __grid_constant__ ProjParams p) {
         }
       }
       ok = mbar_wait_bounded(&bars[ACC_FULL + ab], (tcount >> 1) & 1, abort_flag);
+      if (NORM) ok = ok && mbar_wait_bounded(&bars[SCALE_FULL + ab], (tcount >> 1) & 1, abort_flag);
       if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
       tc_fence_after();
       long long m = (long long)tm * C::TM + (int)rank * BM + row_in_tile;
@@ -300,7 +345,8 @@ kv_project_append_kernel(const __grid_constant__ ProjParams p) {
         const int block = (C::TM / 64) * tm + 2 * (int)rank + (row_in_tile >> 6), b = block / p.blocks_per_batch;
         m = (block - b * p.blocks_per_batch) * 64 + (row_in_tile & 63);
         live = b < p.batches && m < p.M;
-        if (live && p.row_scale) sc = p.row_scale[b * p.scale_bs + m];
+        if (NORM) sc = scale[ab * BM + row_in_tile];
+        else if (live && p.row_scale) sc = p.row_scale[b * p.scale_bs + m];
         dst = p.out + b * p.out_bs + m * p.out_stride + tn * BN;
         if (live && p.residual) res = p.residual + b * p.res_bs + m * p.res_stride + tn * BN;
       } else {
@@ -356,13 +402,14 @@ kv_project_append_kernel(const __grid_constant__ ProjParams p) {
   if (threadIdx.x == 0 && *abort_flag && p.status) atomicOr(p.status, GCA_STATUS_TIMEOUT);
 }
 
-// row_scale[m] = rsqrt(mean(x[m, :]^2) + eps): one warp per row, 16-byte loads.
+// row_scale[m] = rsqrt(mean(x[m, :]^2) + eps): one warp per row, 16-byte loads; blockIdx.y: batch.
 __global__ void row_rms_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ row_scale, long long M, int D,
-                               long long stride, float eps) {
+                               long long stride, float eps, long long x_bs, long long scale_bs) {
   const long long m = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (m >= M) return;
   const int lane = threadIdx.x & 31;
-  const uint4* row = reinterpret_cast<const uint4*>(x + m * stride);
+  const uint4* row = reinterpret_cast<const uint4*>(x + blockIdx.y * x_bs + m * stride);
+  row_scale += blockIdx.y * scale_bs;
   float acc = 0.f;
   for (int i = lane; i < D / 8; i += 32) {
     const uint4 v = row[i];
@@ -451,20 +498,23 @@ TileChoice choose_tile(long long rows64, int ncols, int nmat, int sms) {
   return best;
 }
 
-template <int BN, bool PAIR>
+template <int BN, bool PAIR, bool NORM>
 int launch_tiles(const ProjParams& p, int sms, cudaStream_t stream) {
   using C = Cfg<BN, PAIR>;
-  GCA_CUDA_CHECK(cudaFuncSetAttribute(kv_project_append_kernel<BN, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
+  auto kernel = kv_project_append_kernel<BN, PAIR, NORM>;
+  GCA_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
   const long long tiles = (long long)p.tiles_m * p.tiles_n * p.nmat + p.lead_tiles;
+  const dim3 block(NTHREADS + (NORM ? STAT_WARPS * 32 : 0));
   if (PAIR) {
     const unsigned pairs = (unsigned)(tiles < sms / 2 ? tiles : sms / 2);
-    return (int)launch_dependent_pairs(kv_project_append_kernel<BN, PAIR>, dim3(2 * pairs), dim3(NTHREADS), C::SMEM_BYTES, stream, p);
+    return (int)launch_dependent_pairs(kernel, dim3(2 * pairs), block, C::SMEM_BYTES, stream, p);
   }
-  return (int)launch_dependent(kv_project_append_kernel<BN, PAIR>, dim3((unsigned)(tiles < sms ? tiles : sms)), dim3(NTHREADS), C::SMEM_BYTES, stream, p);
+  return (int)launch_dependent(kernel, dim3((unsigned)(tiles < sms ? tiles : sms)), block, C::SMEM_BYTES, stream, p);
 }
 
 // rows64: 64-row blocks of x (of all batches).  Fills in the tile counts; the weight maps are made here because their box is the tile's.
-int launch_product(ProjParams& p, const void* wk, const void* wv, long long w_stride, long long rows64, TileChoice tile, int sms, cudaStream_t stream) {
+int launch_product(ProjParams& p, const void* wk, const void* wv, long long w_stride, long long rows64, TileChoice tile, int sms, cudaStream_t stream,
+                   bool norm = false) {
   const int tm = tile.pair ? 4 : 2, box = tile.pair ? tile.bn / 2 : tile.bn;
   int rc;
   if ((rc = make_matrix_map(&p.tm_wk, wk, p.ncols, p.D, w_stride, box)) || (rc = make_matrix_map(&p.tm_wv, wv, p.ncols, p.D, w_stride, box))) return rc;
@@ -472,11 +522,15 @@ int launch_product(ProjParams& p, const void* wk, const void* wv, long long w_st
   p.tiles_n = (p.ncols + tile.bn - 1) / tile.bn;
   p.lead_tiles = p.lead_rows > 0 ? p.batches * p.tiles_n : 0;
   if ((long long)p.tiles_m * p.tiles_n * p.nmat + p.lead_tiles >= (1ll << 30)) return GCA_ERR_TOO_LARGE;
-  if (tile.pair) return launch_tiles<256, true>(p, sms, stream);
-  if (tile.bn == 256) return launch_tiles<256, false>(p, sms, stream);
-  if (tile.bn == 192) return launch_tiles<192, false>(p, sms, stream);
-  if (tile.bn == 128) return launch_tiles<128, false>(p, sms, stream);
-  return launch_tiles<64, false>(p, sms, stream);
+  auto width = [&](auto with) {
+    constexpr bool NORM = decltype(with)::value;
+    if (tile.bn == 256) return launch_tiles<256, false, NORM>(p, sms, stream);
+    if (tile.bn == 192) return launch_tiles<192, false, NORM>(p, sms, stream);
+    if (tile.bn == 128) return launch_tiles<128, false, NORM>(p, sms, stream);
+    return launch_tiles<64, false, NORM>(p, sms, stream);
+  };
+  if (tile.pair) return launch_tiles<256, true, false>(p, sms, stream);
+  return norm ? width(std::true_type()) : width(std::false_type());
 }
 
 }  // namespace
@@ -508,7 +562,7 @@ int launch_row_rms(const RowRmsArgs& a, cudaStream_t stream) {
   if (a.M == 0) return 0;
   const int warps = 8;
   row_rms_kernel<<<(unsigned)((a.M + warps - 1) / warps), warps * 32, 0, stream>>>(
-      (const __nv_bfloat16*)a.x, a.row_scale, a.M, a.D, a.x_stride, a.eps);
+      (const __nv_bfloat16*)a.x, a.row_scale, a.M, a.D, a.x_stride, a.eps, 0, 0);
   return (int)cudaGetLastError();
 }
 
@@ -520,17 +574,32 @@ int launch_silu_mul(const void* gu, void* out, long long M, int I, long long in_
   return (int)cudaGetLastError();
 }
 
-int launch_linear(const LinearBatchedArgs& ba, int sms, cudaStream_t stream) {
+// norm_scratch: nullptr, or where the rows' factors 1 / rms(x) may be put, batches x M values, one.row_scale being NULL.
+int launch_linear(const LinearBatchedArgs& ba, float* norm_scratch, int sms, cudaStream_t stream) {
   LinearBatchedArgs args = ba;
   LinearArgs& a = args.one;
+  const float norm_eps = args.rms_eps;
+  if (norm_scratch) { args.rms_eps = 0.f; args.scale_batch_stride = a.M; }
   // batches that lie back to back are one block of rows
   if (args.batches > 1 && args.lead_rows == 0 && args.x_batch_stride == a.M * a.x_stride && args.out_batch_stride == a.M * a.out_stride &&
       (!a.residual || args.residual_batch_stride == a.M * a.residual_stride) && (!a.row_scale || args.scale_batch_stride == a.M)) {
     a.M *= args.batches;
     args.batches = 1;
   }
-  if (args.batches == 1 && args.lead_rows == 0 && a.M <= GCA_SKINNY_ROWS && (args.rms_eps > 0.f || few_rows(a.M, a.N, a.K, false, sms)))
+  auto factors = [&]() -> int {                          // by a launch of their own
+    if (args.batches > 65535) return GCA_ERR_TOO_LARGE;
+    const int warps = 8;
+    row_rms_kernel<<<dim3((unsigned)((a.M + warps - 1) / warps), (unsigned)args.batches), warps * 32, 0, stream>>>(
+        (const __nv_bfloat16*)a.x, norm_scratch, a.M, a.K, a.x_stride, norm_eps, args.x_batch_stride, args.scale_batch_stride);
+    return (int)cudaGetLastError();
+  };
+  if (args.batches == 1 && args.lead_rows == 0 && a.M <= GCA_SKINNY_ROWS && (args.rms_eps > 0.f || few_rows(a.M, a.N, a.K, false, sms))) {
+    if (norm_scratch) {
+      if (int rc = factors()) return rc;
+      a.row_scale = norm_scratch;
+    }
     return launch_skinny_linear(a, args.rms_eps, stream);
+  }
   if (args.rms_eps > 0.f) return GCA_ERR_SHAPE;
   ProjParams p;
   if (a.M >= (1ll << 31)) return GCA_ERR_TOO_LARGE;
@@ -549,7 +618,14 @@ int launch_linear(const LinearBatchedArgs& ba, int sms, cudaStream_t stream) {
   p.ce_part = nullptr; p.ce_target = nullptr; p.targets = nullptr;
   const long long blocks = per_batch * args.batches;
   if (blocks >= (1ll << 30)) return GCA_ERR_TOO_LARGE;
-  return launch_product(p, a.w, a.w, a.w_stride, blocks, choose_tile(blocks, a.N, 1, sms), sms, stream);
+  const TileChoice tile = choose_tile(blocks, a.N, 1, sms);
+  const bool norm = norm_scratch && !tile.pair;
+  p.rms_eps = norm_eps;
+  if (norm_scratch && !norm) {
+    if ((rc = factors())) return rc;
+    p.row_scale = norm_scratch;
+  }
+  return launch_product(p, a.w, a.w, a.w_stride, blocks, tile, sms, stream, norm);
 }
 
 int launch_kv_project_append(const KvProjectArgs& a, int sms, cudaStream_t stream) {

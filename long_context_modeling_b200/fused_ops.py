@@ -52,8 +52,8 @@ def fold_gain(weight: torch.Tensor, gain: torch.Tensor) -> torch.Tensor:
 
 
 def rmsnorm_linear(x: torch.Tensor, folded_weight: torch.Tensor, eps: float) -> torch.Tensor:
-    """RMSNorm(x) @ W.T with ``folded_weight = fold_gain(W, norm.weight)``: one row reduction over x
-    and one GEMM over the raw x whose epilogue applies 1 / rms (one launch for a handful of rows)."""
+    """RMSNorm(x) @ W.T with ``folded_weight = fold_gain(W, norm.weight)``: one GEMM over the raw x whose
+    epilogue applies 1 / rms, summed up from the tiles of x (large products: by a launch before)."""
     return _lib.host().rmsnorm_linear(x, folded_weight, eps)
 
 

@@ -421,6 +421,25 @@ def test_linear_tile_widths_against_float32(m, n, k):
     assert torch.equal(y, F.linear(x, w, row_scale=sc, residual=r))
 
 
+@pytest.mark.parametrize("m,n,k", [(129, 64, 64), (200, 768, 768), (1000, 1008, 192), (2333, 512, 512), (7105, 768, 768),     # 64 .. 192 columns
+                                   (5100, 768, 64), (20001, 256, 128), (25000, 768, 768)])      # fewer K steps than stages, 256 columns, pairs
+def test_norm_from_the_tiles_of_x(m, n, k):
+    """RMSNorm + projection whose row factors are summed up beside the MMAs (or by a launch before, for pairs), against 64 bits; rows
+    of very different sizes, several tiles per CTA."""
+    need_gpu()
+    from long_context_modeling_b200 import fused_ops as F
+    import long_context_modeling_b200 as lcm
+    g = torch.Generator(device="cuda").manual_seed(m)
+    x = (torch.randn(m, k, generator=g, device="cuda") * torch.exp2(torch.randint(-20, 20, (m, 1), generator=g, device="cuda").float())).bfloat16()
+    w = (torch.randn(n, k, generator=g, device="cuda") * k ** -0.5).bfloat16()
+    got = F.rmsnorm_linear(x, w, 1e-5).double()
+    xd = x.double()
+    ref = (xd @ w.double().t()) * torch.rsqrt(xd.pow(2).mean(-1, keepdim=True) + 1e-5)
+    # the rounding to bf16, 2^-8 of the value, and float32: k terms of 2^-24 of the row's largest, the factor's 2^-22
+    assert ((got - ref).abs() <= ref.abs() * (2.0 ** -8 + 2.0 ** -22) + k * 2.0 ** -24 * ref.abs().amax(-1, keepdim=True)).all()
+    assert torch.equal(got, F.rmsnorm_linear(x, w, 1e-5).double()) and lcm.read_status() == 0
+
+
 @pytest.mark.parametrize("n,c,dim", [(1, 1, 256), (3, 5, 512), (5, 61, 768), (2, 300, 1024)])
 def test_projection_append_tile_widths(n, c, dim):
     """K, V and landmark rows of an append at a position behind earlier chunks, against float32, small and large products."""
