@@ -795,7 +795,7 @@ def window_decode_arm(args):
             "e2e": {"value": nbytes / (ms_e2e * 1e-3) / 1e9, "unit": "GB/s", "h2d_bytes_per_step": q_host.numel() * 2,
                     "d2h_bytes_per_step": q_host.numel() * 2, "ms_per_step": ms_e2e},
             "gpu_launches": steps,
-            "roofline": {"kernel": "win_decode_kernel", "bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
+            "roofline": {"kernel": "win_rounds_kernel", "bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                          "frac": achieved / peaks["hbm_gbs"], "peak_source": peaks["source"] + " copy bandwidth", "traffic": None,
                          "algorithmic_bytes_per_launch": nbytes, "us_per_launch": ms_k * 1e3,
                          "ring_form": {"us_per_launch": ms_ring * 1e3, "achieved": nbytes / (ms_ring * 1e-3) / 1e9,
