@@ -29,7 +29,7 @@
 // columns by the caller: RMSNorm(x) W^T = diag(1 / rms) x (W diag(g))^T, so the normalised activations
 // are never written), residual makes it o_proj + residual add.  The factors come from the tiles of x as
 // they pass (NORM); for pairs, whose tiles arrive on the leader's barriers alone, `row_rms_kernel` reads x
-// before.  768 -> 768, 640 / 2,368 / 7,104 rows, x from memory: 6.8 / 8.1 / 14.5 us, with that launch before
+// before.  768 -> 768, 640 / 2,368 / 7,104 rows, x from memory: 6.7 / 8.1 / 14.8 us, with that launch before
 // 8.0 / 11.2 / 17.1.
 //
 // CROSS-ENTROPY mode is the LM head fused with the loss (model/DRT.py:1055-1064, inference /
@@ -228,11 +228,13 @@ kv_project_append_kernel(const __grid_constant__ ProjParams p) {
     bool ok = true;
     uint32_t tcount = 0;
     for (int t = first; t < total && ok; t += step, ++tcount) {
-      float2 sq[4] = {};                                   // eight sums of a row, then their sum: chains of K / 8
+      float2 sq[4] = {};                                   // eight sums of a row, chains of 8 within a stage and of K / 64 over them: as close to
+                                                           // 64 bits as a lane's 24 values and the tree over 32 lanes (4e-8; chains of K / 8 1.1e-7)
       for (int ks = 0; ks < ksteps; ++ks) {
         ok = mbar_wait_warp(&bars[FULL + ring.st], ring.ph, abort_flag, lane);
         if (!ok) break;
         const uint4* x = reinterpret_cast<const uint4*>(smem + ring.st * STAGE_BYTES + row * 128);
+        float2 part[4];
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
           const uint4 v = x[c ^ (row & 7)];
@@ -240,9 +242,11 @@ kv_project_append_kernel(const __grid_constant__ ProjParams p) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const float2 f = make_float2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
-            sq[i] = __ffma2_rn(f, f, sq[i]);
+            part[i] = c == 0 ? __fmul2_rn(f, f) : __ffma2_rn(f, f, part[i]);
           }
         }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sq[i] = __fadd2_rn(sq[i], part[i]);
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars[EMPTY + ring.st]);
         ring.next();
