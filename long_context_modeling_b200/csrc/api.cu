@@ -229,18 +229,22 @@ int gca_bwd_stages(const GcaBwdArgs* a, unsigned stages, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
   gca::DeviceScope scope(a->q);
   if (scope.rc) return scope.rc;
-  gca::Csr csr;
-  size_t used = 0;
-  rc = gca::build_csr(a->indices, a->N, a->J, a->K, a->C, a->workspace, a->workspace_bytes, gca::units_by_count(*a), &csr, &used, s,
-                      (stages & GCA_BWD_STAGE_INDEX) != 0, (stages & GCA_BWD_INDEX_BY_SORT) != 0);
-  if (rc) return rc;
-  if (!(stages & (GCA_BWD_STAGE_KV | GCA_BWD_STAGE_Q))) return 0;
-  float* dw_part = reinterpret_cast<float*>(static_cast<char*>(a->workspace) + used);
-  uint4* rowterm = reinterpret_cast<uint4*>(static_cast<char*>(a->workspace) + used + dw_part_bytes(a));
   int algo = a->algo;
   const bool tc_ok = a->dtype == GCA_BF16 && a->S == 64;
   if (algo == GCA_ALGO_TC_UNPAIRED) algo = GCA_ALGO_TC;
   if (algo == GCA_ALGO_AUTO) algo = tc_ok ? GCA_ALGO_TC : GCA_ALGO_SIMT;
+  // the tensor-core passes of a pre-gathered call read no index: no launch for it where both of them run
+  const unsigned all = GCA_BWD_STAGE_INDEX | GCA_BWD_STAGE_Q | GCA_BWD_STAGE_KV;
+  const bool unread = !a->indices && algo == GCA_ALGO_TC && tc_ok && (stages & all) == all;
+  gca::Csr csr;
+  size_t used = 0;
+  rc = gca::build_csr(a->indices, a->N, a->J, a->K, a->C, a->workspace, a->workspace_bytes, gca::units_by_count(*a), &csr, &used, s,
+                      (stages & GCA_BWD_STAGE_INDEX) != 0 && !unread, (stages & GCA_BWD_INDEX_BY_SORT) != 0);
+  if (rc) return rc;
+  csr.clear = unread;
+  if (!(stages & (GCA_BWD_STAGE_KV | GCA_BWD_STAGE_Q))) return 0;
+  float* dw_part = reinterpret_cast<float*>(static_cast<char*>(a->workspace) + used);
+  uint4* rowterm = reinterpret_cast<uint4*>(static_cast<char*>(a->workspace) + used + dw_part_bytes(a));
   const bool f32_tc = a->algo == GCA_ALGO_AUTO &&
                       gca::f32_tc_takes(a->dtype, a->S, (long long)a->N * (a->J > a->C ? a->J : a->C) * a->Hq);
   if (algo == GCA_ALGO_TC)

@@ -106,6 +106,7 @@ struct Csr {
   const int4* unit_tab;
   int* tickets;
   bool overlaps;
+  bool clear = false;      // not built, nor needed but for the counters: the q-major pass clears them
 };
 
 // launch == false: only lay the index out in `workspace` (it was built by an earlier call)

@@ -141,7 +141,8 @@ bool small_path(int N, int JK, int C) {
   return C <= LIST_MAX_C && (long long)N * JK < (1ll << 31) && (long long)N * C * JK <= (1ll << 27) && N <= 65535;
 }
 
-// The pre-gathered call: chunk c of row block n is read by its slot c and nothing else.
+// The pre-gathered call: chunk c of row block n is read by its slot c and nothing else.  (For kernels that read the index; the bf16
+// tensor-core passes of one call do without: 109 row blocks x 8 heads, forward + backward, calls in a row 79.3 -> 75.8 us.)
 __global__ void csr_identity_kernel(unsigned long long* __restrict__ keys_out, int4* __restrict__ unit_tab, int* __restrict__ tickets, int NC, int C) {
   pdl_wait();
   pdl_trigger();

@@ -1,6 +1,6 @@
 // Attention of one or two query rows over rows of a bf16 cache, sixteen keys at a time in one warp, several sixteens in a row.  The bound
-// is HBM, but with a multiply-add per value the instructions were in the way of the loads: ~400 a warp for sixteen keys.  As matrix
-// instructions (m16n8k16, float32 sums) they are ~110, most of them for the softmax.
+// is HBM, but with a multiply-add per value the instructions were in the way of the loads: 384 items x 512 keys were 6.6 million warp
+// instructions, as matrix instructions (m16n8k16, float32 sums) they are 3.9 million, most of them for the softmax and around the keys.
 //
 // Lane = 4 * g + t.  Scores: the keys are the rows of A.  A lane's 16 bytes of a key row are the four registers of one A operand, as
 // they come from memory: its dims 0,1 and 4,5 stand in row g, dims 2,3 and 6,7 in row g + 8.  So the columns of B come in pairs, the

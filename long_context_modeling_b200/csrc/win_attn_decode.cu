@@ -14,8 +14,7 @@
 //
 // Bound: HBM for many items, else latency (launch, one round of loads, the merges).  Eight warps an item, one key at a time and
 // multiply-adds took, us, one row: 512 keys, 4 items 6.9, now 4.8; 64 items 8.8, now 5.8; 384 items 13.3, now 12.7 (7.7 at the
-// copy rate); two rows, 384 items 23.0, now 12.6.  With multiply-adds in the second kernel too (four keys a step) 13.9 and 13.9: they
-// were ~400 instructions a warp for sixteen keys.  The same matrix instructions in the first kernel are slower (128 keys, 148
+// copy rate); two rows, 384 items 23.0, now 12.6.  With multiply-adds in the second kernel too (four keys a step) 13.9 and 13.9.  The same matrix instructions in the first kernel are slower (128 keys, 148
 // items 4.0 us against 3.4): their chain is the longer one.
 //
 // RING form (decode of one position per sequence against a FULL window): the window buffer is a

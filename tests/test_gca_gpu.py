@@ -251,6 +251,31 @@ def test_backward_stage_by_stage_equals_one_call(lcm, algo):
     assert lcm.read_status() == 0
 
 
+@pytest.mark.parametrize("z,hq,hkv,k", [(1, 1, 1, 1), (7, 8, 4, 5), (70, 6, 6, 3), (40, 12, 12, 32)])
+def test_pre_gathered_backward_reads_no_index(lcm, z, hq, hkv, k):
+    """The pre-gathered call has no inverse index (chunk c is read by slot c): the gradients of the indexed call on the same chunks,
+    bit for bit, with whatever the workspace holds before, call after call."""
+    g = torch.Generator().manual_seed(z)
+    q, dout = (torch.randn(z, hq, 64, 64, generator=g).bfloat16().cuda() for _ in range(2))
+    kk, vv = (torch.randn(z, hkv, k, 64, 64, generator=g).bfloat16().cuda() for _ in range(2))
+    w = torch.softmax(torch.randn(z, k, generator=g), -1).cuda()
+    idx = torch.arange(k, dtype=torch.int32, device="cuda").expand(z, 1, k).contiguous()
+    cache = [t.permute(0, 2, 3, 1, 4).contiguous() for t in (kk, vv)]                   # (Z, K, L, Hkv, D)
+    want = run_indexed(lcm, q.unsqueeze(1).cpu(), cache[0].cpu(), cache[1].cpu(), idx.cpu(), w.view(z, 1, k).cpu(), 0.125, dout=dout.unsqueeze(1).cpu())
+    for _ in range(3):
+        junk = torch.full((64 << 20,), 0x7f, dtype=torch.uint8, device="cuda")
+        del junk
+        leaves = [t.clone().requires_grad_() for t in (q, kk, vv, w)]
+        out = lcm.attention(*leaves, 0.125, 0.0)
+        out.backward(dout)
+        got = [out, *(t.grad for t in leaves)]
+        assert torch.equal(got[0].view(-1).cpu(), want[0].reshape(-1).cpu())
+        assert torch.equal(got[1].view(-1).cpu(), want[1].reshape(-1).cpu()) and torch.equal(got[4].view(-1).cpu(), want[4].reshape(-1).cpu())
+        for a, b in zip(got[2:4], want[2:4]):
+            assert torch.equal(a.permute(0, 2, 3, 1, 4).reshape(-1).cpu(), b.reshape(-1).cpu())
+    assert lcm.read_status() == 0
+
+
 @pytest.mark.parametrize("shape", [(2, 14, 4, 8), (3, 40, 2, 4), (1, 70, 4, 16), (8, 256, 2, 8), (1, 1024, 2, 4)])
 def test_inverse_index_single_launch_equals_radix_sort(lcm, shape):
     """The single-launch counting sort that builds the inverse retrieval index for small problems
