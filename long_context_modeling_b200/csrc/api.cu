@@ -233,15 +233,15 @@ int gca_bwd_stages(const GcaBwdArgs* a, unsigned stages, void* stream) {
   const bool tc_ok = a->dtype == GCA_BF16 && a->S == 64;
   if (algo == GCA_ALGO_TC_UNPAIRED) algo = GCA_ALGO_TC;
   if (algo == GCA_ALGO_AUTO) algo = tc_ok ? GCA_ALGO_TC : GCA_ALGO_SIMT;
-  // the tensor-core passes of a pre-gathered call read no index: no launch for it where both of them run
+  // the index of a pre-gathered call is known: the q-major tensor-core pass writes it on its way where both passes run, no launch of its own
   const unsigned all = GCA_BWD_STAGE_INDEX | GCA_BWD_STAGE_Q | GCA_BWD_STAGE_KV;
-  const bool unread = !a->indices && algo == GCA_ALGO_TC && tc_ok && (stages & all) == all;
+  const bool on_the_way = !a->indices && (long long)a->N * a->C >= 2 && algo == GCA_ALGO_TC && tc_ok && (stages & all) == all;
   gca::Csr csr;
   size_t used = 0;
   rc = gca::build_csr(a->indices, a->N, a->J, a->K, a->C, a->workspace, a->workspace_bytes, gca::units_by_count(*a), &csr, &used, s,
-                      (stages & GCA_BWD_STAGE_INDEX) != 0 && !unread, (stages & GCA_BWD_INDEX_BY_SORT) != 0);
+                      (stages & GCA_BWD_STAGE_INDEX) != 0 && !on_the_way, (stages & GCA_BWD_INDEX_BY_SORT) != 0);
   if (rc) return rc;
-  csr.clear = unread;
+  csr.write = on_the_way;
   if (!(stages & (GCA_BWD_STAGE_KV | GCA_BWD_STAGE_Q))) return 0;
   float* dw_part = reinterpret_cast<float*>(static_cast<char*>(a->workspace) + used);
   uint4* rowterm = reinterpret_cast<uint4*>(static_cast<char*>(a->workspace) + used + dw_part_bytes(a));

@@ -146,7 +146,6 @@ struct BwdKvParams {
   const uint4* rowterm;     // (N*J, Hq, K) tiles of 64 x 16 bytes, written by the q-major pass
   const int4* unit_tab;     // units in walking order: (first entry, one past the last, chunk id n*C + c)
   const unsigned long long* sorted_keys;
-  bool identity;            // the pre-gathered call: chunk c of row block n is read by its slot c and nothing else, no table is read
   int* tickets;             // [units handed out beyond the first of every CTA, CTAs done]
   __nv_bfloat16* dk;
   __nv_bfloat16* dv;
@@ -208,7 +207,7 @@ __device__ void kv_scheduler(const BwdKvParams& p, uint8_t* smem, uint64_t* bars
         pair = x / p.C;
         row = n * p.C + x - pair * p.C;
       }
-      unit = p.identity ? make_int4(row, row + 1, row, 0) : p.unit_tab[row];
+      unit = p.unit_tab[row];
       unit.w = pair;
     }
     slots[head % ND] = unit;
@@ -265,7 +264,7 @@ __device__ void kv_producer(const BwdKvParams& p, uint8_t* smem, uint64_t* bars,
       tma_load_5d(base, &p.tm_k2, &bars[KV_FULL + kb], 0, 0, hk0, ch, n);
       tma_load_5d(base + PAIR_BYTES, &p.tm_v2, &bars[KV_FULL + kb], 0, 0, hk0, ch, n);
     }
-    unsigned long long key_next = p.identity ? (unsigned long long)ch : p.sorted_keys[beg];
+    unsigned long long key_next = p.sorted_keys[beg];
     for (int e = beg; e < end && ok; ++e) {
       const int entry = (int)(key_next & 0xffffffffull);
       if (e + 1 < end) key_next = p.sorted_keys[e + 1];
@@ -638,7 +637,7 @@ int launch_bwd_kv_tc(const GcaBwdArgs& a, const Csr& csr, const uint4* rowterm, 
       (rc = qmap(&p.tm_q1, a.q, a.q_stride, 1)) || (rc = qmap(&p.tm_do1, a.dout, a.do_stride, 1)) ||
       (rc = kmap(&p.tm_k2, a.k_cache, a.k_stride, 2)) || (rc = kmap(&p.tm_v2, a.v_cache, a.v_stride, 2)))
     return rc;
-  p.weights = a.weights; p.rowterm = rowterm; p.unit_tab = csr.unit_tab; p.sorted_keys = csr.sorted_keys; p.identity = a.indices == nullptr; p.tickets = csr.tickets;
+  p.weights = a.weights; p.rowterm = rowterm; p.unit_tab = csr.unit_tab; p.sorted_keys = csr.sorted_keys; p.tickets = csr.tickets;
   p.dk = (__nv_bfloat16*)a.dk_cache; p.dv = (__nv_bfloat16*)a.dv_cache; p.status = a.status;
   p.prof = profile_buffer();
   for (int i = 0; i < 4; ++i) { p.dks[i] = a.dk_stride[i]; p.dvs[i] = a.dv_stride[i]; }

@@ -151,7 +151,7 @@ struct BwdQParams {
                             // b0 + b1 + b2 = -Di: the kv-major pass adds them to its scores with one MMA K step
   float inv_c2;
   int32_t* status;
-  int* zero;                // two counters to clear for the kv-major pass, or nullptr (whoever built the index has)
+  Csr index;                // of a pre-gathered call, written by this kernel on its way (index.write), for the kv-major pass
   long long* prof;
   long long dqs[4];
   int units;
@@ -556,7 +556,9 @@ bwd_q_tc_kernel(const __grid_constant__ BwdQParams p) {
   __syncthreads();
   if (warp == ISSUE_S) tmem_dealloc(tmem_base, TMEM_COLS);
   if (threadIdx.x == 0 && *abort_flag && p.status) atomicOr(p.status, GCA_STATUS_TIMEOUT);
-  if (p.zero && blockIdx.x == 0 && threadIdx.x < 2) p.zero[threadIdx.x] = 0;
+  if (p.index.write) {
+    for (int i = (int)(blockIdx.x * NTHREADS + threadIdx.x); i < p.N * p.C; i += (int)gridDim.x * NTHREADS) identity_entry(p.index, i, p.C);
+  }
 }
 
 // every 64-element bf16 row of the tensor starts on a 32-byte boundary
@@ -570,7 +572,7 @@ bool rows_32b_aligned(const void* base, const int64_t* stride) {
 }  // namespace
 
 // dw_part: (N*J, Hq, K, 4) float32 partials; rowterm: (N*J, Hq, K, 64) x 16 bytes (see BwdQParams).
-int launch_bwd_q_tc(const GcaBwdArgs& a, float* dw_part, uint4* rowterm, bool beside_index, int* zero, int sms, cudaStream_t stream) {
+int launch_bwd_q_tc(const GcaBwdArgs& a, float* dw_part, uint4* rowterm, const Csr& csr, int sms, cudaStream_t stream) {
   const float c2 = a.sm_scale * GCA_LOG2E;
   int rc;
   auto qmap = [&](CUtensorMap* m, const void* base, const int64_t* st, int box) {
@@ -580,7 +582,7 @@ int launch_bwd_q_tc(const GcaBwdArgs& a, float* dw_part, uint4* rowterm, bool be
     return make_tile_map_5d(m, base, 64, 64, a.Hkv, a.C, a.N, st[2], st[3], st[1], st[0], box);
   };
   BwdQParams p;
-  p.zero = zero;
+  p.index = csr;
   if ((rc = qmap(&p.tm_q, a.q, a.q_stride, 2)) || (rc = qmap(&p.tm_do, a.dout, a.do_stride, 2)) ||
       (rc = kmap(&p.tm_k2, a.k_cache, a.k_stride, 2)) || (rc = kmap(&p.tm_v2, a.v_cache, a.v_stride, 2)) ||
       (rc = kmap(&p.tm_k1, a.k_cache, a.k_stride, 1)) || (rc = kmap(&p.tm_v1, a.v_cache, a.v_stride, 1)))
@@ -599,7 +601,7 @@ int launch_bwd_q_tc(const GcaBwdArgs& a, float* dw_part, uint4* rowterm, bool be
   if (p.units == 0) return 0;
   GCA_CUDA_CHECK(cudaFuncSetAttribute(bwd_q_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
   const unsigned grid = (unsigned)(p.units < sms ? p.units : sms);
-  p.beside_index = beside_index;
+  p.beside_index = csr.overlaps;
   return (int)launch_dependent(bwd_q_tc_kernel, dim3(grid), dim3(NTHREADS), SMEM_BYTES, stream, p);
 }
 

@@ -13,7 +13,7 @@
 namespace gca {
 
 int launch_bwd_kv_tc(const GcaBwdArgs& a, const Csr& csr, const uint4* rowterm, const float* dw_part, int sms, cudaStream_t stream);
-int launch_bwd_q_tc(const GcaBwdArgs& a, float* dw_part, uint4* rowterm, bool beside_index, int* zero, int sms, cudaStream_t stream);
+int launch_bwd_q_tc(const GcaBwdArgs& a, float* dw_part, uint4* rowterm, const Csr& csr, int sms, cudaStream_t stream);
 
 bool bwd_tc_available() { return true; }
 
@@ -27,7 +27,7 @@ int launch_bwd_tc(const GcaBwdArgs& a, const Csr& csr, float* dw_part, uint4* ro
   if (a.dtype != GCA_BF16 || a.S != 64 || a.L != 64 || a.D != 64 || a.K > 32) return GCA_ERR_ALGO;
   int rc;
   if (stages & GCA_BWD_STAGE_Q) {
-    if ((rc = launch_bwd_q_tc(a, dw_part, rowterm, csr.overlaps, csr.clear ? csr.tickets : nullptr, sms, stream))) return rc;
+    if ((rc = launch_bwd_q_tc(a, dw_part, rowterm, csr, sms, stream))) return rc;
   }
   if (stages & GCA_BWD_STAGE_KV) {
     if ((rc = launch_bwd_kv_tc(a, csr, rowterm, (stages & GCA_BWD_STAGE_Q) ? dw_part : nullptr, sms, stream))) return rc;

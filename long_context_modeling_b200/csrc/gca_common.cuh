@@ -106,8 +106,15 @@ struct Csr {
   const int4* unit_tab;
   int* tickets;
   bool overlaps;
-  bool clear = false;      // not built, nor needed but for the counters: the q-major pass clears them
+  bool write = false;      // laid out only: the q-major pass writes it
 };
+
+// The index of a pre-gathered call: chunk c of row block n is read by its slot c and nothing else.
+__device__ __forceinline__ void identity_entry(const Csr& index, int i, int C) {
+  const_cast<unsigned long long*>(index.sorted_keys)[i] = ((unsigned long long)i << 32) | (unsigned)(i % C);
+  const_cast<int4*>(index.unit_tab)[i] = make_int4(i, i + 1, i, 0);
+  if (i < 2) index.tickets[i] = 0;
+}
 
 // launch == false: only lay the index out in `workspace` (it was built by an earlier call)
 // by_count: the unit table's order (units_by_count)

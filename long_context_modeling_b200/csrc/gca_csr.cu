@@ -141,16 +141,14 @@ bool small_path(int N, int JK, int C) {
   return C <= LIST_MAX_C && (long long)N * JK < (1ll << 31) && (long long)N * C * JK <= (1ll << 27) && N <= 65535;
 }
 
-// The pre-gathered call: chunk c of row block n is read by its slot c and nothing else.  (For kernels that read the index; the bf16
-// tensor-core passes of one call do without: 109 row blocks x 8 heads, forward + backward, calls in a row 79.3 -> 75.8 us.)
-__global__ void csr_identity_kernel(unsigned long long* __restrict__ keys_out, int4* __restrict__ unit_tab, int* __restrict__ tickets, int NC, int C) {
+// For passes that do not write it themselves.  (The bf16 tensor-core passes of one call do: 109 row blocks x 8 heads, forward + backward, calls in
+// a row 79.5 -> 76.3 us.)
+__global__ void csr_identity_kernel(Csr index, int NC, int C) {
   pdl_wait();
   pdl_trigger();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < 2) tickets[i] = 0;
-  if (i >= NC) return;
-  keys_out[i] = ((unsigned long long)i << 32) | (unsigned)(i % C);
-  unit_tab[i] = make_int4(i, i + 1, i, 0);
+  if (i < 2) index.tickets[i] = 0;
+  if (i < NC) identity_entry(index, i, C);
 }
 
 size_t cub_temp_bytes(long long total) {
@@ -207,7 +205,7 @@ int build_csr(const int32_t* indices, int N, int J, int K, int C, void* workspac
   if (cbits + nbits > 32) return GCA_ERR_TOO_LARGE;
   out->overlaps = false;
   if (launch && !indices && NC > 0) {
-    GCA_CUDA_CHECK(launch_dependent(csr_identity_kernel, dim3((unsigned)((NC + 255) / 256)), dim3(256), 0, stream, keys_out, uvals_out, tickets, (int)NC, C));
+    GCA_CUDA_CHECK(launch_dependent(csr_identity_kernel, dim3((unsigned)((NC + 255) / 256)), dim3(256), 0, stream, Csr{keys_out, uvals_out, tickets, false}, (int)NC, C));
     out->overlaps = true;
   } else if (launch && NC > 0 && total > 0 && !by_sort && small_path(N, J * K, C)) {
     GCA_CUDA_CHECK(launch_dependent(csr_list_kernel, dim3((unsigned)((C + LIST_WARPS - 1) / LIST_WARPS), (unsigned)N), dim3(LIST_WARPS * 32), 0,

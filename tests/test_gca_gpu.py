@@ -252,9 +252,9 @@ def test_backward_stage_by_stage_equals_one_call(lcm, algo):
 
 
 @pytest.mark.parametrize("z,hq,hkv,k", [(1, 1, 1, 1), (7, 8, 4, 5), (70, 6, 6, 3), (40, 12, 12, 32)])
-def test_pre_gathered_backward_reads_no_index(lcm, z, hq, hkv, k):
-    """The pre-gathered call has no inverse index (chunk c is read by slot c): the gradients of the indexed call on the same chunks,
-    bit for bit, with whatever the workspace holds before, call after call."""
+def test_pre_gathered_backward_writes_its_index_on_the_way(lcm, z, hq, hkv, k):
+    """The inverse index of a pre-gathered call (chunk c is read by slot c) is written by the q-major pass: the gradients of the indexed
+    call on the same chunks, bit for bit, with whatever the workspace holds before, call after call."""
     g = torch.Generator().manual_seed(z)
     q, dout = (torch.randn(z, hq, 64, 64, generator=g).bfloat16().cuda() for _ in range(2))
     kk, vv = (torch.randn(z, hkv, k, 64, 64, generator=g).bfloat16().cuda() for _ in range(2))
