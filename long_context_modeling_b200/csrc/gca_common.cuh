@@ -150,6 +150,9 @@ inline bool units_by_count(const GcaBwdArgs& a) {
   return (long long)a.N * a.J * a.Hq * a.S * a.D * 2 * (a.dtype == GCA_F32 ? 4 : 2) <= (64ll << 20);
 }
 
+// Warps of a kernel with that many registers a thread (a multiple of eight) that an SM holds: each of its four quarters has registers of its own.
+constexpr int warps_per_sm(int regs) { return 4 * (512 / regs); }
+
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 // The entry points run on the device that HOLDS THE BUFFERS, whatever the calling thread's

@@ -452,36 +452,50 @@ decode_rows_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
 //   two warps a slot       one CTA: K = 8, 148 items 7.0 against 7.4.  In clusters only for two rows, whose chain is the longer one
 //                          (K = 16, 64 items: 7.7 against 8.6; one row 8.1 against 7.6), and for one row where a CTA cannot hold all slots
 //   a warp a slot          one CTA if it holds them (K = 13, 148 items: 8.4 against 10.2 of two CTAs), else a cluster of two to four
-//   two, three .. slots a warp, one CTA
-// Measured over rows 1, 2 x K 2 .. 32 x 4 .. 592 items (caches from memory): 1.0 % above the best of all splits on average.  Two rows at
+//   two, three .. slots a warp, one CTA: the rounds r and waves w with the least w (r + 0.9).  The bytes take the same time however they are
+//                          split; what differs is a round's latency (~3.4 us) in every wave, and a wave's start and merges (~3 us).  One
+//                          row, K = 8, 1000 items: three rounds in one wave 25.5 us, two in two 30.9, one in three 29.9
+// A CTA of a warp a slot has a multiple of four warps where that many still run at once, the last ones idle: the SM's quarters then have the same
+// number of loads in flight (one row, K = 6, 384 items: eight warps 9.0 us, six 9.8; K = 3, 700 items: four 8.8, three 10.1; two rows, K = 5, 240
+// items: eight 8.0, five 8.7).  Two rows keep an even number: six are 3 % faster than eight.
+// Measured over rows 1, 2 x K 2 .. 32 x 148 .. 3000 items (caches from memory): within 0.3 % of the best of all splits on average (3.7 % above it with
+// the first split of at most four warps a CTA beyond one wave, and 25 warps of 80 registers counted where 24 fit).  Two rows at
 // 96 registers a thread instead of 128 fit more warps and lose 12 %: they spill.  Three and four rows are two pairs, whose second reading of
 // K and V hits L2: 250 registers left 8 warps an SM (K = 8, 184 items 16.7 us as four rows, 14.2 as pairs).
 struct DecodePlan { int wps, ctas, warps; };
 DecodePlan decode_plan(long long items, int K, int rows, int sms) {
   const int cap4 = rows > 1 ? ROW_WARPS<2, 4> : ROW_WARPS<1, 4>, cap = rows > 1 ? ROW_WARPS<2, 1> : ROW_WARPS<1, 1>;
+  const int sm_warps4 = warps_per_sm(rows > 1 ? ROW_REGS<2, 4> : ROW_REGS<1, 4>), sm_warps = warps_per_sm(rows > 1 ? ROW_REGS<2, 1> : ROW_REGS<1, 1>);
   if (rows > 1) items *= (rows + 1) / 2;
   DecodePlan plan = {0, 0, 0};
-  auto one_wave = [&](int wps, int ctas, int warps) {
-    const int sm_warps = 65536 / (32 * (rows > 1 ? ROW_REGS<2, 1> : wps == 4 ? ROW_REGS<1, 4> : ROW_REGS<1, 1>));
+  auto take = [&](int wps, int ctas) {
+    const int slots = (K + ctas - 1) / ctas, warps = slots * wps;
     // clusters leave some places empty: all of a cluster's CTAs have to find theirs in one group of SMs
     const int slack = ctas == 1 ? 0 : ctas < 5 ? 1 : ctas;
-    return warps <= (wps == 4 ? cap4 : cap) && items * ctas * (16 + slack) <= 16ll * sms * (sm_warps / warps);
-  };
-  auto take = [&](int wps, int ctas) {
-    const int slots = (K + ctas - 1) / ctas;
-    if (ctas > 8 || (K + slots - 1) / slots != ctas || !one_wave(wps, ctas, slots * wps)) return false;
-    plan = {wps, ctas, slots * wps};
+    if (ctas > 8 || (K + slots - 1) / slots != ctas || warps > (wps == 4 ? cap4 : cap)) return false;
+    if (items * ctas * (16 + slack) > 16ll * sms * ((wps == 4 ? sm_warps4 : sm_warps) / warps)) return false;
+    plan = {wps, ctas, warps};
     return true;
   };
   const int by2 = (K + 1) / 2, by3 = (K + 2) / 3, by4 = (K + 3) / 4;
   if (K > 6 && items * by2 <= sms && take(4, by2)) return plan;
   if (take(4, 1) || (K > 4 && (take(4, by3) || take(4, by4))) || take(2, 1)) return plan;
   if (rows > 1 && K > 8 && take(2, by4)) return plan;
-  if (take(1, 1) || (K > 8 && (take(2, by4) || take(1, 2) || take(1, 3) || take(1, 4)))) return plan;
-  for (int rounds = 2;; ++rounds) {
+  auto quartered = [&] {
+    const int warps = (plan.warps + 3) & ~3;
+    if ((rows == 1 || plan.warps % 2) && warps <= cap && items <= (long long)sms * (sm_warps / warps)) plan.warps = warps;
+    return plan;
+  };
+  if (take(1, 1)) return quartered();
+  if (K > 8 && (take(2, by4) || take(1, 2) || take(1, 3) || take(1, 4))) return plan;
+  long long least = 0;
+  for (int rounds = (K + cap - 1) / cap; rounds <= K; ++rounds) {
     const int warps = (K + rounds - 1) / rounds;
-    if (warps <= 4 || one_wave(1, 1, warps)) return {1, 1, warps};
+    const long long wave = (long long)sms * (sm_warps / warps), cost = (items + wave - 1) / wave * (10 * rounds + 9);
+    if (least == 0 || cost < least) { least = cost; plan = {1, 1, warps}; }
+    if (items <= wave) break;                                    // one wave: more rounds only take longer
   }
+  return quartered();
 }
 
 template <int R>

@@ -550,6 +550,8 @@ def test_decode_warps_per_slot(lcm, n, hq, hkv, sq, k, obo):
     (140, 16, 1), (400, 8, 1), (140, 6, 3),  # a warp a slot in one CTA
     (90, 30, 1), (160, 16, 1), (100, 32, 1), (24, 31, 3),  # ... in clusters
     (300, 32, 1), (520, 9, 1), (300, 17, 2), (1100, 5, 4),  # several slots a warp
+    (640, 14, 1), (760, 16, 2), (1504, 2, 2),  # ... in one wave, in three, a single warp a CTA
+    (384, 6, 1), (700, 3, 1), (240, 5, 2), (300, 12, 1),  # idle warps
 ])
 def test_decode_splits(lcm, items, k, rows):
     """How the slots are dealt out over warps, CTAs and clusters does not change the result: every split the decode kernel has,
