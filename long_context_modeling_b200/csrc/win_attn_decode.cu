@@ -400,13 +400,7 @@ win_rounds_kernel(const WinParams p, int) {                      // one CTA an i
 // Within 1.2 % of the best of all splits on average over one and two rows x 64 .. 640 keys x 4 .. 768 items (caches from memory).  Two rows at
 // 80 registers a thread fit more warps and lose 10 % where both fit (512 keys, 148 items 8.2 against 7.4).
 struct WindowPlan { int ctas, warps; bool rounds; };
-#ifdef WINDOW_PLAN_PROBE
-WindowPlan g_probe_plan;
-#endif
 WindowPlan window_plan(long long items, int keys, int rows, int sms) {
-#ifdef WINDOW_PLAN_PROBE
-  return g_probe_plan;
-#endif
   if (rows > 1) items *= (rows + 1) / 2;
   auto fits = [&](int ctas, int warps, bool many) {
     const int regs = rows > 1 ? WIN_REGS<2, true> : many ? WIN_REGS<1, true> : WIN_REGS<1, false>;
