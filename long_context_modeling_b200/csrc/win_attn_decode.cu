@@ -396,27 +396,33 @@ win_rounds_kernel(const WinParams p, int) {                      // one CTA an i
 // once, and as few rounds as possible to follow one another.  So, the first of these that fits one wave (one row, us):
 //   once, one CTA        256 keys, 148 items 5.0 (two rounds 5.8), 256 items 6.8 (7.9)
 //   once, a cluster      of four, three or two CTAs where two have an SM to themselves: 640 keys, 4 items 4.6 (two rounds in one CTA 6.0)
-//   rounds               two, three .. in one CTA: 512 keys, 256 items three of eleven warps 9.8 (four of eight 10.9), 384 items four of eight 12.7
-// Within 1.2 % of the best of all splits on average over one and two rows x 64 .. 640 keys x 4 .. 768 items (caches from memory).  Two rows at
+//   rounds               two, three .. in one CTA, the rounds r and waves w with the least w (r + 1.5): 512 keys, 256 items three of eleven warps
+//                        9.8 (four of eight 10.9), 384 items four of eight 12.7, 640 items eight of four 18.4 (seven of five in two waves 24.1)
+// Over one and two rows x 64 .. 640 keys x 148 .. 3000 items (caches from memory) 0.1 % above the best of these splits on average (3.5 % with the
+// first split of at most four warps a CTA beyond one wave, and 25 warps of 80 registers counted where 24 fit).  Two rows at
 // 80 registers a thread fit more warps and lose 10 % where both fit (512 keys, 148 items 8.2 against 7.4).
 struct WindowPlan { int ctas, warps; bool rounds; };
 WindowPlan window_plan(long long items, int keys, int rows, int sms) {
   if (rows > 1) items *= (rows + 1) / 2;
-  auto fits = [&](int ctas, int warps, bool many) {
-    const int regs = rows > 1 ? WIN_REGS<2, true> : many ? WIN_REGS<1, true> : WIN_REGS<1, false>;
-    const int cap = rows > 1 ? WIN_WARPS<2, true> : many ? WIN_WARPS<1, true> : WIN_WARPS<1, false>;
-    return warps <= cap && items * ctas <= (long long)sms * (65536 / (32 * regs) / warps);
-  };
+  const int cap = rows > 1 ? WIN_WARPS<2, true> : WIN_WARPS<1, true>, cap_once = rows > 1 ? WIN_WARPS<2, false> : WIN_WARPS<1, false>;
+  const int sm_warps = warps_per_sm(rows > 1 ? WIN_REGS<2, true> : WIN_REGS<1, true>);
+  const int sm_warps_once = warps_per_sm(rows > 1 ? WIN_REGS<2, false> : WIN_REGS<1, false>);
+  auto fits_once = [&](int ctas, int warps) { return warps <= cap_once && items * ctas <= (long long)sms * (sm_warps_once / warps); };
   const int sixteens = std::max(1, (keys + 15) / 16);
-  if (fits(1, sixteens, false)) return {1, sixteens, false};
+  if (fits_once(1, sixteens)) return {1, sixteens, false};
   for (int ctas = 4; ctas > 1; --ctas) {
     const int warps = (sixteens + ctas - 1) / ctas;
-    if (2 * items * ctas <= sms && fits(ctas, warps, false)) return {ctas, warps, false};
+    if (2 * items * ctas <= sms && fits_once(ctas, warps)) return {ctas, warps, false};
   }
-  for (int rounds = std::max(2, (sixteens + 23) / 24);; ++rounds) {
+  WindowPlan plan = {1, std::min(cap, sixteens), true};
+  long long least = 0;
+  for (int rounds = std::max(2, (sixteens + cap - 1) / cap); rounds <= sixteens; ++rounds) {
     const int warps = (sixteens + rounds - 1) / rounds;
-    if (warps <= 4 || fits(1, warps, true)) return {1, warps, true};
+    const long long wave = (long long)sms * (sm_warps / warps), cost = (items + wave - 1) / wave * (2 * rounds + 3);
+    if (least == 0 || cost < least) { least = cost; plan.warps = warps; }
+    if (items <= wave) break;                                    // one wave: more rounds only take longer
   }
+  return plan;
 }
 
 // The cached window of one decode step, moved on IN PLACE: every (sequence, head) block of T rows drops

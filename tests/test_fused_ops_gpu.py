@@ -211,6 +211,7 @@ def test_window_decode_against_float32(n, hq, hkv, sq, t, window, alibi):
     (5, 1, 1, 513, 512), (5, 2, 1, 641, 700), (12, 1, 1, 640, 639),              # clusters of CTAs
     (60, 1, 1, 350, 349), (60, 2, 1, 200, 300), (148, 1, 1, 513, 512),           # one round, two rounds
     (390, 1, 1, 200, 199), (150, 3, 1, 260, 300), (800, 2, 1, 66, 65),           # several rounds, a row pair that is half empty
+    (700, 1, 1, 300, 299), (350, 4, 1, 330, 329), (1500, 2, 1, 50, 49),          # ... and waves, two pairs, a single warp a CTA
     (2, 1, 2, 40, 16), (150, 1, 2, 500, 300), (300, 2, 2, 300, 64),              # rows at two positions: each sees a key that the other does not
 ])
 @pytest.mark.parametrize("poison", [False, True])
