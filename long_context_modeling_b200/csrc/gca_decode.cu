@@ -255,10 +255,11 @@ decode_rows_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
   __shared__ bool slot_reads[WARPS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = lane >> 3, sub = lane & 7;
   const int warps = blockDim.x >> 5, slots = warps / WPS;        // of the CTA
-  const int item = blockIdx.x / ctas, rank = blockIdx.x - item * ctas;
+  const int unit = blockIdx.x / ctas, rank = blockIdx.x - unit * ctas;
+  const bool pairs = R > 1 && g.G * g.S > R;                     // three or four rows: an item's two pairs follow one another
+  const int item = pairs ? unit >> 1 : unit, row0 = pairs ? (unit & 1) * R : 0, rows = min(R, g.G * g.S - row0);      // this CTA's rows of the kv head
   const int zj = item / g.Hkv, hk = item - zj * g.Hkv;
   const int n = zj / g.J, j = zj - n * g.J;
-  const int row0 = blockIdx.y * R, rows = min(R, g.G * g.S - row0);      // this CTA's rows of the kv head
   const float c2 = g.sm_scale * GCA_LOG2E;
   const int k0 = rank * slots + warp / WPS, share = warp % WPS;
   pdl_trigger();
@@ -460,8 +461,9 @@ decode_rows_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
 // items: eight 8.0, five 8.7).  Two rows keep an even number: six are 3 % faster than eight.
 // Measured over rows 1, 2 x K 2 .. 32 x 148 .. 3000 items (caches from memory): within 0.3 % of the best of all splits on average (3.7 % above it with
 // the first split of at most four warps a CTA beyond one wave, and 25 warps of 80 registers counted where 24 fit).  Two rows at
-// 96 registers a thread instead of 128 fit more warps and lose 12 %: they spill.  Three and four rows are two pairs, whose second reading of
-// K and V hits L2: 250 registers left 8 warps an SM (K = 8, 184 items 16.7 us as four rows, 14.2 as pairs).
+// 96 registers a thread instead of 128 fit more warps and lose 12 %: they spill.  Three and four rows are two pairs: 250 registers left
+// 8 warps an SM (K = 8, 184 items 16.7 us as four rows, 14.2 as pairs).  An item's pairs are neighbours in the grid, so that the second reading
+// of its K and V hits L2 however many items there are (K = 8, 1500 items, four rows 71 us; all first pairs before all second ones 84; as four rows 103).
 struct DecodePlan { int wps, ctas, warps; };
 DecodePlan decode_plan(long long items, int K, int rows, int sms) {
   const int cap4 = rows > 1 ? ROW_WARPS<2, 4> : ROW_WARPS<1, 4>, cap = rows > 1 ? ROW_WARPS<2, 1> : ROW_WARPS<1, 1>;
@@ -532,7 +534,7 @@ int launch_decode(const GcaFwdArgs& a, int sms, cudaStream_t stream) {
     const DecodePlan plan = decode_plan(blocks, g.K, rows, sms);
     auto run = [&](auto kernel) {
       cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3((unsigned)(blocks * plan.ctas), (unsigned)((rows + 1) / 2)); cfg.blockDim = dim3((unsigned)(plan.warps * 32)); cfg.stream = stream;
+      cfg.gridDim = dim3((unsigned)(blocks * plan.ctas * ((rows + 1) / 2))); cfg.blockDim = dim3((unsigned)(plan.warps * 32)); cfg.stream = stream;
       cudaLaunchAttribute attr[2];
       attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
       attr[0].val.programmaticStreamSerializationAllowed = 1;

@@ -107,7 +107,7 @@ __device__ __forceinline__ void merge_and_store(const WinParams& p, WarpState<R>
 }
 
 // One warp for sixteen keys, in one round: latency counts.  A warp load covers FOUR key rows: 8 lanes x 16 bytes per 128-byte row; each 8-lane
-// group has a stream of four keys, the streams are merged within the warp.  R rows of the kv head (blockIdx.y: which of its row pairs).  The
+// group has a stream of four keys, the streams are merged within the warp.  R rows of the kv head (blockIdx.x: which of its row pairs).  The
 // ring's new row and the window's last row stand beside the sixteens, in the first warp: a window of 512 is 513 rows.
 template <int R, bool RING>
 __global__ void __maxnreg__((WIN_REGS<R, false>))
@@ -115,9 +115,10 @@ win_once_kernel(const WinParams p, int ctas) {
   __shared__ WarpState<R> part[WIN_WARPS<R, false>];
   __shared__ WarpState<R> total;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = lane >> 3, sub = lane & 7, warps = blockDim.x >> 5;
-  const int item = blockIdx.x / ctas, rank = blockIdx.x - item * ctas;
+  const int unit = blockIdx.x / ctas, rank = blockIdx.x - unit * ctas;
+  const bool pairs = R > 1 && p.G * p.Sq > R;                    // three or four rows: an item's two pairs follow one another
+  const int item = pairs ? unit >> 1 : unit, row0 = pairs ? (unit & 1) * R : 0, rows = min(R, p.G * p.Sq - row0);
   const int n = item / p.Hkv, hk = item - n * p.Hkv;
-  const int row0 = blockIdx.y * R, rows = min(R, p.G * p.Sq - row0);
   pdl_trigger();
   pdl_wait();
   const int last = p.T - 1;
@@ -216,7 +217,7 @@ win_once_kernel(const WinParams p, int ctas) {
 #pragma unroll
     for (int s = 0; s < 4; ++s) { sc[s] = ex2(sc[s] - mf); l[r] += sc[s]; add(r, sc[s], vq[s], ok[s]); }
   }
-  if (RING && extra && grp == 0 && blockIdx.y == 0) {            // over the oldest row, which nobody uses any more
+  if (RING && extra && grp == 0 && row0 == 0) {                  // over the oldest row, which nobody uses any more
     *reinterpret_cast<uint4*>(const_cast<__nv_bfloat16*>(kb) + newest * p.ks[2]) = kx;
     *reinterpret_cast<uint4*>(const_cast<__nv_bfloat16*>(vb) + newest * p.vs[2]) = vx;
   }
@@ -255,8 +256,9 @@ __global__ void __maxnreg__((WIN_REGS<R, true>))
 win_rounds_kernel(const WinParams p, int) {                      // one CTA an item
   __shared__ WarpState<R> part[WIN_WARPS<R, true>];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, warps = blockDim.x >> 5;
-  const int n = blockIdx.x / p.Hkv, hk = blockIdx.x - n * p.Hkv;
-  const int row0 = blockIdx.y * R, rows = min(R, p.G * p.Sq - row0);
+  const bool pairs = R > 1 && p.G * p.Sq > R;                    // three or four rows: an item's two pairs follow one another
+  const int item = pairs ? blockIdx.x >> 1 : blockIdx.x, row0 = pairs ? (blockIdx.x & 1) * R : 0, rows = min(R, p.G * p.Sq - row0);
+  const int n = item / p.Hkv, hk = item - n * p.Hkv;
   pdl_trigger();
   pdl_wait();
   const int first = max(0, p.T - p.Sq - p.window);             // keys any row can see: [first, T)
@@ -334,7 +336,7 @@ win_rounds_kernel(const WinParams p, int) {                      // one CTA an i
     }
   };
   if (has_extra) {
-    if (RING && blockIdx.y == 0) {                               // the new row over the oldest one, which nobody uses any more
+    if (RING && row0 == 0) {                                     // the new row over the oldest one, which nobody uses any more
       if (g == 0) {
         __nv_bfloat16* kd = const_cast<__nv_bfloat16*>(kb) + newest * p.ks[2];
         *reinterpret_cast<uint4*>(kd) = kx[0]; *reinterpret_cast<uint4*>(kd + 32) = kx[1];
@@ -401,6 +403,8 @@ win_rounds_kernel(const WinParams p, int) {                      // one CTA an i
 // Over one and two rows x 64 .. 640 keys x 148 .. 3000 items (caches from memory) 0.1 % above the best of these splits on average (3.5 % with the
 // first split of at most four warps a CTA beyond one wave, and 25 warps of 80 registers counted where 24 fit).  Two rows at
 // 80 registers a thread fit more warps and lose 10 % where both fit (512 keys, 148 items 8.2 against 7.4).
+// Three and four rows are two pairs, neighbours in the grid: the second reading of an item's window hits L2 (512 keys, 1500 items, four rows
+// 56 us; all first pairs before all second ones 70).
 struct WindowPlan { int ctas, warps; bool rounds; };
 WindowPlan window_plan(long long items, int keys, int rows, int sms) {
   if (rows > 1) items *= (rows + 1) / 2;
@@ -485,7 +489,7 @@ static int launch_window(const WindowDecodeArgs& a, const WindowRingDecodeArgs* 
   const WindowPlan plan = window_plan(items, p.T - (ring || a.Sq == 1 ? 1 : 0) - std::max(0, p.T - p.Sq - p.window), rows, sms);
   auto run = [&](auto kernel) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(items * plan.ctas), (unsigned)((rows + 1) / 2)); cfg.blockDim = dim3((unsigned)(plan.warps * 32)); cfg.stream = stream;
+    cfg.gridDim = dim3((unsigned)(items * plan.ctas * ((rows + 1) / 2))); cfg.blockDim = dim3((unsigned)(plan.warps * 32)); cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
