@@ -253,9 +253,9 @@ int gca_bwd_stages(const GcaBwdArgs* a, unsigned stages, void* stream) {
   else if (algo == GCA_ALGO_SIMT) rc = gca::launch_bwd_simt(*a, csr, dw_part, reinterpret_cast<float*>(rowterm), s, stages & GCA_BWD_STAGE_ALL);
   else rc = GCA_ERR_ALGO;
   if (rc) return rc;
-  if (!(stages & GCA_BWD_STAGE_Q)) return 0;
+  if (!(stages & GCA_BWD_STAGE_Q) || f32_tc) return 0;                   // float32 on the tensor cores: dw is reduced
   if (algo == GCA_ALGO_TC && (stages & GCA_BWD_STAGE_KV)) return 0;      // the kv-major kernel has reduced dw
-  return gca::launch_dw_reduce(dw_part, a->dw, a->N * a->J, a->Hq, a->K, algo == GCA_ALGO_TC ? gca::bwd_tc_dw_parts() : f32_tc ? 4 : 1, s);
+  return gca::launch_dw_reduce(dw_part, a->dw, a->N * a->J, a->Hq, a->K, algo == GCA_ALGO_TC ? gca::bwd_tc_dw_parts() : 1, s);
 }
 
 }  // extern "C"

@@ -129,7 +129,7 @@ int launch_fwd_simt(const GcaFwdArgs& a, cudaStream_t stream);
 // row_di: (N*J, Hq, K, 64) floats of scratch, Di of every row: the q-major stage writes it, the kv-major stage reads it
 int launch_bwd_simt(const GcaBwdArgs& a, const Csr& csr, float* dw_part, float* row_di, cudaStream_t stream, unsigned stages);
 
-// float32 on the tensor cores, S = L = D = 64 (same scratch; four dw partials per (row block, head, slot)).
+// float32 on the tensor cores, S = L = D = 64 (same scratch; four dw partials per (row block, head, slot), summed to dw by the q-major stage).
 bool f32_tc_takes(int dtype, int S, long long units);
 int launch_fwd_f32_tc(const GcaFwdArgs& a, cudaStream_t stream);
 int launch_bwd_f32_tc(const GcaBwdArgs& a, const Csr& csr, float* dw_part, float* row_di, cudaStream_t stream, unsigned stages);

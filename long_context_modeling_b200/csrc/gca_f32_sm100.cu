@@ -1,6 +1,7 @@
 // GCA on float32 data with tcgen05, S = L = D = 64: every float32 operand as the sum of three bf16 values.
 //
-// A float32 number is b0 + b1 + b2 with b0 = bf16(x), b1 = bf16(x - b0), b2 = bf16(x - b0 - b1), to 2^-27 of itself, so a
+// A float32 number is b0 + b1 + b2 with b0 = bf16(x), b1 = bf16(x - b0), b2 = bf16(x - b0 - b1): three times eight bits hold its 24, exactly
+// down to |x| = 2^-110, where the last of them is bf16's smallest number, 2^-133 (below, to 2^-134).  So a
 // product of two float32 tiles is the sum of the bf16 products b0 b0', b0 b1', b1 b0', b1 b1', b0 b2', b2 b0' (what is left out is
 // below 2^-26), accumulated from the smallest to the largest in ONE accumulator.  The tensor core cuts an accumulator off
 // where an FMA rounds it, so a long chain drifts: with the large product last only its four K steps count.  Measured against
@@ -22,11 +23,13 @@
 // The 16-row forms of tcgen05.ld / st spread a 16 x 64 tile over all 32 threads of a warp (thread t: rows t / 4 and t / 4 + 8,
 // columns 2 (t % 4), + 1 of every 8), and packed pairs of what a thread holds are what the 16x128b store takes.
 // Every wait is bounded (GCA_STATUS_TIMEOUT on expiry).  No atomics on results: they are bit-reproducible.
+// Infinities, NaN, sums that overflow on the way and tiles of tiny numbers are outside the range of all this: such units are found by their outputs
+// and done over again with multiply-adds (see `outside`), with the results that the CUDA-core kernels have always had.
 // 2 x 64 chunks x 12 heads, top-8: forward 115 us, q-major 171, kv-major 210 (CUDA cores: 355, 481, 588), the whole step with inputs
 // that are not in L2 541 us (1,425).  2-norm against 64 bits: o 2.2e-7 (4.4e-7), dq 2.8e-7 (4.7e-7), dk 3.0e-7 (6.9e-7), dv 2.6e-7
 // (6.8e-7).  What bounds it now: the chains; a CTA takes ~5,400 cycles per slot in the forward, of which its own products are 1,024.
 // Tried and slower: eight worker warps in the forward (the row maxima and sums then cross groups: 135 us).
-#include "gca_common.cuh"
+#include "gca_simt.cuh"
 #include "sm100_ptx.cuh"
 
 namespace gca {
@@ -73,7 +76,7 @@ __device__ __forceinline__ float2 add2(uint32_t a0, uint32_t a1, uint32_t b0, ui
   return __fadd2_rn(make_float2(__uint_as_float(a0), __uint_as_float(a1)), make_float2(__uint_as_float(b0), __uint_as_float(b1)));
 }
 // x, y -> the packed pair of their bf16 values; x, y keep what is left.  FIRST: a finite float32 past bf16's largest number must not become
-// an infinity (an infinity is left as it is, and ends as NaN like a NaN).
+// an infinity (an infinity ends as a NaN, which the unit's outputs show).
 template <bool FIRST>
 __device__ __forceinline__ uint32_t take_bf16x2(float& x, float& y) {
   uint32_t w;
@@ -139,13 +142,14 @@ __device__ __forceinline__ void load_cols32(const float* base, long long row_str
     }
   }
 }
-__device__ __forceinline__ void store_cols32(float* base, long long row_stride, int row, int lane, int group, const float* acc, float s) {
+// Returns where the thread's first value went.
+__device__ __forceinline__ float* store_cols32(float* base, long long row_stride, int row, int lane, int group, const float* acc, float s) {
+  base += row * row_stride + 32 * group + (lane & 3) * 2;
 #pragma unroll
-  for (int r = 0; r < 2; ++r) {
-    float* d = base + (row + 8 * r) * row_stride + 32 * group + (lane & 3) * 2;
+  for (int r = 0; r < 2; ++r)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) *reinterpret_cast<float2*>(d + 8 * i) = make_float2(acc[4 * i + 2 * r] * s, acc[4 * i + 2 * r + 1] * s);
-  }
+    for (int i = 0; i < 4; ++i) *reinterpret_cast<float2*>(base + 8 * r * row_stride + 8 * i) = make_float2(acc[4 * i + 2 * r] * s, acc[4 * i + 2 * r + 1] * s);
+  return base;
 }
 
 // ---------------------------------------------------------------- tiles
@@ -282,19 +286,24 @@ __device__ __forceinline__ float quad_sum(float v) {
   return v + __shfl_xor_sync(0xffffffffu, v, 2);
 }
 
-// The unit of a q-major CTA and the list of its slots that read a chunk, x = slot, y = chunk.  Late query chunks first: they have
-// the most slots, and what starts last should be short.
-struct QUnit {
-  int n, j, h, hk, nv;
+// The unit of a q-major CTA.  Late query chunks first: they have the most slots, and what starts last should be short.
+struct UnitId {
+  int n, j, h;
+  __device__ __forceinline__ UnitId(const Geom& g, int b) {
+    h = b % g.Hq;
+    n = b / g.Hq % g.N;
+    j = g.J - 1 - b / g.Hq / g.N;
+  }
+};
+// With the list of its slots that read a chunk, x = slot, y = chunk.
+struct QUnit : UnitId {
+  int hk, nv;
   long long zj;
   int first;          // chunk of the first one
   unsigned valid;
   const int2* slot;
-  __device__ __forceinline__ QUnit(const Geom& g, const int32_t* indices, int32_t* status, uint8_t* smem) {
-    const int b = blockIdx.x, lane = threadIdx.x & 31;
-    h = b % g.Hq;
-    n = b / g.Hq % g.N;
-    j = g.J - 1 - b / g.Hq / g.N;
+  __device__ __forceinline__ QUnit(const Geom& g, const int32_t* indices, int32_t* status, uint8_t* smem) : UnitId(g, blockIdx.x) {
+    const int lane = threadIdx.x & 31;
     hk = h / g.G;
     zj = (long long)n * g.J + j;
     const int idx = lane < g.K ? slot_chunk(indices, zj, g.K, lane) : -1;
@@ -310,6 +319,88 @@ struct QUnit {
     slot = list;                                   // complete behind the barrier in Frame::set_up()
   }
 };
+
+struct BwdStrides { long long dout[4], dk[4], dv[4]; };
+
+// ------------------------------------------------------------------------------------ units outside the range
+// What a warp holds of a unit's outputs lies outside the kernels' range if anything is infinite or NaN, or if nothing reaches 2^-100 (and not all
+// is zero): an infinite operand or a sum past the largest number ends as a NaN here, where multiply-adds give an infinity or, for a score
+// of -inf, a weight of zero; and of operands below 2^-110 bits are lost.  The warp then puts a NaN that no arithmetic produces in the place of its
+// first output, and a kernel behind this one does the units so marked over again with multiply-adds.  Where nothing is marked the kernels behind
+// cost 3.0 us (forward), 4.6 (q-major, which sums dw by the way; that alone took 5.2) and 3.2 (kv-major).  As a call from the kernels
+// themselves the same took registers from their loops: kv-major 205 -> 230 us, q-major 165 -> 178.
+constexpr unsigned MARK = 0x7fc5f32bu;
+template <int N>
+__device__ __forceinline__ bool outside(const float (&acc)[N]) {
+  uint32_t m = 0;
+#pragma unroll
+  for (int i = 0; i < N; ++i) m = max(m, __float_as_uint(acc[i]) & 0x7fffffffu);
+  m = __reduce_max_sync(0xffffffffu, m);
+  return m >= 0x7f800000u || (m > 0 && m < ((127u - 100u) << 23));
+}
+__device__ __forceinline__ void mark(float* first) { *reinterpret_cast<unsigned*>(first) = MARK; }
+// `warps` marks, of the four row groups and (eight) the two halves of the columns
+__device__ __forceinline__ bool marked(const float* tile, long long row_stride, int warps) {
+  bool any = false;
+  for (int w = 0; w < warps; ++w) any |= *reinterpret_cast<const volatile unsigned*>(tile + (w & 3) * 16 * row_stride + (w >> 2) * 32) == MARK;
+  return any;
+}
+// The units b, b + blocks, ...: a thread looks at one, then the block does the marked ones together.
+template <class Marked, class Unit>
+__device__ __forceinline__ void do_marked(int units, Marked is_marked, Unit unit) {
+  pdl_wait();
+  for (long long b0 = blockIdx.x; b0 < units; b0 += (long long)NTHREADS * gridDim.x) {
+    const long long mine = b0 + (long long)threadIdx.x * gridDim.x;
+    if (!__syncthreads_or(mine < units && is_marked((int)mine))) continue;
+    for (long long b = b0; b < units && b < b0 + (long long)NTHREADS * gridDim.x; b += gridDim.x)
+      if (__syncthreads_or(threadIdx.x == 0 && is_marked((int)b))) unit((int)b);
+  }
+}
+__global__ void __launch_bounds__(NTHREADS, 4)
+fwd_f32_again_kernel(const float* q, const float* kc, const float* vc, const int32_t* indices, const float* weights, float* out, float* lse, Geom g) {
+  extern __shared__ __align__(16) float smem_fma[];
+  do_marked(g.N * g.J * g.Hq, [&](int b) { const UnitId u(g, b); return marked(out + u.n * g.os[0] + u.j * g.os[1] + u.h * g.os[2], g.os[3], FWD_WORKERS); },
+            [&](int b) { const UnitId u(g, b); fwd_unit<float>(smem_fma, u.n * g.J + u.j, u.h, q, kc, vc, indices, weights, out, lse, nullptr, g); });
+}
+// One block per row block: its marked heads, then dw = the sum of its heads' partials, four heads side by side, in a fixed order.
+__global__ void __launch_bounds__(NTHREADS, 2)
+bwd_q_f32_finish_kernel(const float* q, const float* kc, const float* vc, const int32_t* indices, const float* weights, const float* dout, const float* lse,
+                        float* dq, float* dw_part, float* row_di, float* dw, Geom g, BwdStrides st) {
+  extern __shared__ __align__(16) float smem_fma[];
+  __shared__ float part[NTHREADS];
+  const int zj = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  auto is_marked = [&](int h) { return h < g.Hq && marked(dq + zj / g.J * g.os[0] + zj % g.J * g.os[1] + h * g.os[2], g.os[3], BWD_WORKERS); };
+  pdl_wait();
+  for (int h0 = 0; h0 < g.Hq; h0 += NTHREADS) {
+    if (!__syncthreads_or(is_marked(h0 + threadIdx.x))) continue;
+    for (int h = h0; h < min(h0 + NTHREADS, g.Hq); ++h)
+      if (__syncthreads_or(threadIdx.x == 0 && is_marked(h)))
+        bwd_q_unit<float, 4>(smem_fma, zj, h, q, kc, vc, indices, weights, dout, lse, dq, dw_part, row_di, g, st.dout[0], st.dout[1], st.dout[2], st.dout[3]);
+    __syncthreads();
+  }
+  float t = 0.f;
+  if (lane < g.K)
+#pragma unroll 4
+    for (int h = warp; h < g.Hq; h += NTHREADS / 32) {
+      const float4 v = *reinterpret_cast<const float4*>(dw_part + (((long long)zj * g.Hq + h) * g.K + lane) * 4);
+      t += (v.x + v.y) + (v.z + v.w);
+    }
+  part[threadIdx.x] = t;
+  __syncthreads();
+  if (threadIdx.x < g.K) dw[(long long)zj * g.K + lane] = (part[lane] + part[32 + lane]) + (part[64 + lane] + part[96 + lane]);
+}
+__global__ void __launch_bounds__(NTHREADS, 2)
+bwd_kv_f32_again_kernel(const float* q, const float* kc, const float* vc, const float* weights, const float* dout, const float* lse, const float* row_di,
+                        float* dk, float* dv, Csr csr, Geom g, BwdStrides st) {
+  extern __shared__ __align__(16) float smem_fma[];
+  do_marked(g.N * g.C * g.Hkv, [&](int b) {
+    const int hk = b % g.Hkv, nc = csr.unit_tab[b / g.Hkv].z;
+    return marked(dk + nc / g.C * st.dk[0] + nc % g.C * st.dk[1] + hk * st.dk[3], st.dk[2], BWD_WORKERS);
+  }, [&](int b) {
+    bwd_kv_unit<float>(smem_fma, csr.unit_tab[b / g.Hkv], b % g.Hkv, q, kc, vc, weights, dout, lse, row_di, dk, dv, csr, g, st.dout[0], st.dout[1],
+                       st.dout[2], st.dout[3], st.dk[0], st.dk[1], st.dk[2], st.dk[3], st.dv[0], st.dv[1], st.dv[2], st.dv[3]);
+  });
+}
 
 // ------------------------------------------------------------------------------------ forward
 // Regions: Q | scores | probabilities | product.  The next slot's scores are computed while this slot's are worked on, its product while
@@ -398,10 +489,12 @@ fwd_f32_tc_kernel(const float* __restrict__ q, const float* __restrict__ kc, con
         }
       }
     }
-    if (ok)
+    if (ok) {
+      float* first = nullptr;
 #pragma unroll
-      for (int h = 0; h < 2; ++h)
-        store_cols32(out + u.n * g.os[0] + u.j * g.os[1] + u.h * g.os[2], g.os[3], f.row, f.lane, h, acc + 16 * h, 1.0f);
+      for (int h = 1; h >= 0; --h) first = store_cols32(out + u.n * g.os[0] + u.j * g.os[1] + u.h * g.os[2], g.os[3], f.row, f.lane, h, acc + 16 * h, 1.0f);
+      if (outside(acc) && f.lane == 0) mark(first);
+    }
   } else if (f.warp < f.ISSUER) {
     if (nv > 0) {
       const int t = threadIdx.x - FWD_WORKERS * 32;
@@ -527,7 +620,10 @@ bwd_q_f32_tc_kernel(const float* __restrict__ q, const float* __restrict__ kc, c
       add_product32(f.quarter + R3, f.group, one, acc);
       f.arrive_read(O_FREE);
     }
-    if (ok) store_cols32(dq + u.n * g.os[0] + u.j * g.os[1] + u.h * g.os[2], g.os[3], f.row, f.lane, f.group, acc, g.sm_scale);
+    if (ok) {
+      float* first = store_cols32(dq + u.n * g.os[0] + u.j * g.os[1] + u.h * g.os[2], g.os[3], f.row, f.lane, f.group, acc, g.sm_scale);
+      if (outside(acc) && f.lane == 0) mark(first);
+    }
   } else if (f.warp < f.ISSUER) {
     if (nv > 0) {
       const int t = threadIdx.x - BWD_WORKERS * 32;
@@ -645,8 +741,9 @@ bwd_kv_f32_tc_kernel(const float* __restrict__ q, const float* __restrict__ kc, 
       add_product32(f.quarter + R3, f.group, one, aK);
     }
     if (ok) {
-      store_cols32(dk + n * dks0 + c * dks1 + hk * dks3, dks2, f.row, f.lane, f.group, aK, g.sm_scale);
+      float* first = store_cols32(dk + n * dks0 + c * dks1 + hk * dks3, dks2, f.row, f.lane, f.group, aK, g.sm_scale);
       store_cols32(dv + n * dvs0 + c * dvs1 + hk * dvs3, dvs2, f.row, f.lane, f.group, aV, 1.0f);
+      if ((outside(aK) | outside(aV)) && f.lane == 0) mark(first);
     }
   } else if (f.warp < f.ISSUER) {
     if (steps > 0) {
@@ -712,33 +809,48 @@ bwd_kv_f32_tc_kernel(const float* __restrict__ q, const float* __restrict__ kc, 
 // One CTA per unit along x: problems past that limit (no memory holds their q) stay with the CUDA-core kernels.
 bool f32_tc_takes(int dtype, int S, long long units) { return dtype == GCA_F32 && S == 64 && units < (1ll << 31); }
 
+// As many blocks as run at once, each with a word to read for every unit it answers for: ~2 us where nothing is marked.
+template <class... Params, class... Args>
+static int launch_again(void (*kernel)(Params...), long long units, int blocks_per_sm, int smem, cudaStream_t stream, Args... args) {
+  GCA_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  return (int)launch_dependent(kernel, dim3((unsigned)(units < 148 * blocks_per_sm ? units : 148 * blocks_per_sm)), dim3(NTHREADS), smem, stream, args...);
+}
+
 int launch_fwd_f32_tc(const GcaFwdArgs& a, cudaStream_t stream) {
   const long long units = (long long)a.N * a.J * a.Hq;
   GCA_CUDA_CHECK(cudaFuncSetAttribute(fwd_f32_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-  fwd_f32_tc_kernel<<<(unsigned)units, threads_of(FWD_WORKERS), SMEM_BYTES, stream>>>((const float*)a.q, (const float*)a.k_cache, (const float*)a.v_cache,
-                                                                       a.indices, a.weights, (float*)a.out, a.lse, a.status, make_geom(a));
-  return (int)cudaGetLastError();
+  const float *q = (const float*)a.q, *kc = (const float*)a.k_cache, *vc = (const float*)a.v_cache;
+  fwd_f32_tc_kernel<<<(unsigned)units, threads_of(FWD_WORKERS), SMEM_BYTES, stream>>>(q, kc, vc, a.indices, a.weights, (float*)a.out, a.lse, a.status,
+                                                                                      make_geom(a));
+  GCA_CUDA_CHECK(cudaGetLastError());
+  return launch_again(fwd_f32_again_kernel, units, 4, FWD_UNIT_SMEM, stream, q, kc, vc, a.indices, a.weights, (float*)a.out, a.lse, make_geom(a));
 }
 
 int launch_bwd_f32_tc(const GcaBwdArgs& a, const Csr& csr, float* dw_part, float* row_di, cudaStream_t stream, unsigned stages) {
   const Geom g = make_geom(a);
+  BwdStrides st;
+  for (int i = 0; i < 4; ++i) { st.dout[i] = a.do_stride[i]; st.dk[i] = a.dk_stride[i]; st.dv[i] = a.dv_stride[i]; }
+  const float *q = (const float*)a.q, *kc = (const float*)a.k_cache, *vc = (const float*)a.v_cache, *dout = (const float*)a.dout;
   const long long q_units = (long long)a.N * a.J * a.Hq, kv_units = (long long)a.N * a.C * a.Hkv;
   if ((stages & GCA_BWD_STAGE_Q) && q_units > 0) {
     GCA_CUDA_CHECK(cudaFuncSetAttribute(bwd_q_f32_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-    GCA_CUDA_CHECK(launch_dependent(bwd_q_f32_tc_kernel, dim3((unsigned)q_units), dim3(threads_of(BWD_WORKERS)), SMEM_BYTES, stream,
-                                    (const float*)a.q, (const float*)a.k_cache, (const float*)a.v_cache, a.indices, a.weights,
-                                    (const float*)a.dout, a.lse, (float*)a.dq, dw_part, row_di, a.status, g, (int)csr.overlaps,
+    GCA_CUDA_CHECK(launch_dependent(bwd_q_f32_tc_kernel, dim3((unsigned)q_units), dim3(threads_of(BWD_WORKERS)), SMEM_BYTES, stream, q, kc, vc,
+                                    a.indices, a.weights, dout, a.lse, (float*)a.dq, dw_part, row_di, a.status, g, (int)csr.overlaps,
                                     a.do_stride[0], a.do_stride[1], a.do_stride[2], a.do_stride[3]));
+    GCA_CUDA_CHECK(cudaFuncSetAttribute(bwd_q_f32_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BWD_Q_UNIT_SMEM));
+    GCA_CUDA_CHECK(launch_dependent(bwd_q_f32_finish_kernel, dim3((unsigned)(a.N * a.J)), dim3(NTHREADS), BWD_Q_UNIT_SMEM, stream, q, kc, vc, a.indices,
+                                    a.weights, dout, a.lse, (float*)a.dq, dw_part, row_di, (float*)a.dw, g, st));
   }
   if ((stages & GCA_BWD_STAGE_KV) && kv_units > 0) {
     GCA_CUDA_CHECK(cudaFuncSetAttribute(bwd_kv_f32_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
     bwd_kv_f32_tc_kernel<<<(unsigned)kv_units, threads_of(BWD_WORKERS), SMEM_BYTES, stream>>>(
-        (const float*)a.q, (const float*)a.k_cache, (const float*)a.v_cache, a.weights, (const float*)a.dout, a.lse, row_di,
-        (float*)a.dk_cache, (float*)a.dv_cache, a.status, csr, g,
+        q, kc, vc, a.weights, dout, a.lse, row_di, (float*)a.dk_cache, (float*)a.dv_cache, a.status, csr, g,
         a.do_stride[0], a.do_stride[1], a.do_stride[2], a.do_stride[3],
         a.dk_stride[0], a.dk_stride[1], a.dk_stride[2], a.dk_stride[3],
         a.dv_stride[0], a.dv_stride[1], a.dv_stride[2], a.dv_stride[3]);
     GCA_CUDA_CHECK(cudaGetLastError());
+    return launch_again(bwd_kv_f32_again_kernel, kv_units, 2, BWD_KV_UNIT_SMEM, stream, q, kc, vc, a.weights, dout, a.lse, row_di, (float*)a.dk_cache,
+                        (float*)a.dv_cache, csr, g, st);
   }
   return 0;
 }

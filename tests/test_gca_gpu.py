@@ -632,6 +632,50 @@ def test_float32_extremes_and_nan(lcm):
         assert torch.equal(torch.isfinite(got), torch.isfinite(want))
 
 
+OUTSIDE = {                                            # inf: +inf, huge: products past the largest number, tiny: below what three bf16 values hold
+    "v inf": lambda t: t["v"][0, 2, 11, 30].fill_(float("inf")),
+    "v -inf": lambda t: t["v"][0, 2].fill_(float("-inf")),
+    "k inf": lambda t: t["k"][0, 2, 11, 30].fill_(float("inf")),
+    "score -inf": lambda t: (t["k"][0, 2, 11, 30].fill_(float("-inf")), t["q"][..., 30].abs_().add_(0.1)),
+    "score huge": lambda t: (t["k"][0, 2, 11, 30].fill_(-1e30), t["q"][..., 30].abs_().add_(0.1).mul_(1e25)),
+    "q inf": lambda t: t["q"][0, 4, 1, 20, 3].fill_(float("-inf")),
+    "q nan": lambda t: t["q"][0, 4, 1, 20, 3].fill_(float("nan")),
+    "dout inf": lambda t: t["dout"][0, 4, 1, 20, 3].fill_(float("inf")),
+    "w nan": lambda t: t["w"][0, 4, 0].fill_(float("nan")),
+    "v tiny": lambda t: t["v"].mul_(2.0 ** -115),
+    "dout tiny": lambda t: t["dout"].mul_(2.0 ** -115),
+    "all": lambda t: [t[x].fill_(float("nan")) for x in t],
+}
+
+
+@pytest.mark.parametrize("what", list(OUTSIDE))
+@pytest.mark.parametrize("heads,token_major", [(2, False), (3, True)])
+def test_float32_outside_the_split_range_is_as_with_multiply_adds(lcm, what, heads, token_major):
+    """Infinite, NaN, overflowing and tiny operands: where the CUDA-core kernels give a number, an infinity or a NaN, so does the default, in all
+    five outputs; where they give numbers, the default is as near to 64 bits as ever."""
+    q, kc, vc, idx, w, dout = cases.gca_indexed_case(34, 1, 6, heads, 2, dtype=torch.float32)
+    if token_major:
+        q, dout = (t.transpose(2, 3).contiguous().transpose(2, 3) for t in (q, dout))
+    OUTSIDE[what](dict(q=q, k=kc, v=vc, w=w, dout=dout))
+    got, fma = (run_indexed(lcm, q, kc, vc, idx, w, 0.125, dout=dout, algo=algo, token_major_out=token_major) for algo in (0, 1))
+    for name, g_, f_ in zip(("o", "dq", "dk", "dv", "dw"), got, fma):
+        if what == "score huge" and name != "o":       # the gradients of scores of 1e54 are noise
+            continue
+        assert torch.equal(torch.isnan(g_), torch.isnan(f_)), name
+        assert torch.equal(torch.nan_to_num(g_, 0.0, 1.0, -1.0) * torch.isinf(g_), torch.nan_to_num(f_, 0.0, 1.0, -1.0) * torch.isinf(f_)), name
+        ok = torch.isfinite(f_)
+        if ok.any():
+            assert _two_norm(g_[ok], f_[ok]) <= 2 * F32_SPLIT_REL, (name, _two_norm(g_[ok], f_[ok]))     # either's own error
+    want = G.gca_indexed_grads(q, kc, vc, idx, w, 0.125, dout, work_dtype=torch.float64)
+    if what.endswith("tiny"):
+        for name, g_, r_ in zip(("o", "dq", "dk", "dv", "dw"), got, want):
+            assert _two_norm(g_, r_) <= F32_SPLIT_REL, (name, _two_norm(g_, r_))
+    elif what not in ("score huge", "all"):            # 1e25 x 1e30 is a number in 64 bits; the oracle reads chunk 0 for a slot that reads none
+        o, r = got[0].cpu(), want[0]
+        assert torch.equal(torch.isnan(o), torch.isnan(r)) and torch.equal(o == float("inf"), r == float("inf")) and torch.equal(o == float("-inf"), r == float("-inf"))
+    assert lcm.read_status() == 0
+
+
 @pytest.mark.parametrize("n,c,h,k", [(40, 30, 3, 1), (8, 60, 4, 2), (3, 30, 2, 32), (1, 3, 1, 4)])
 def test_forward_slot_records(lcm, n, c, h, k):
     """Units of one slot, of few, of 32, and fewer slots in all than there are warpgroups; a third of the units empty: the forward's roles
