@@ -613,7 +613,7 @@ def test_float32_split_products_are_no_less_precise_than_fma(lcm):
     q, kc, vc, idx, w, dout = cases.gca_indexed_case(33, 2, 20, 4, 8, dtype=torch.float32)
     ref = G.gca_indexed_grads(q, kc, vc, idx, w, 0.125, dout, work_dtype=torch.float64)
     tc, fma = (run_indexed(lcm, q, kc, vc, idx, w, 0.125, dout=dout, algo=algo) for algo in (0, 1))
-    for name, t_, f_, r_ in zip(("o", "dq", "dk", "dv"), tc, fma, ref):
+    for name, t_, f_, r_ in zip(("o", "dq", "dk", "dv", "dw"), tc, fma, ref):
         assert _two_norm(t_, r_) <= _two_norm(f_, r_), name
 
 
