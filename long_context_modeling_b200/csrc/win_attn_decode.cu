@@ -2,7 +2,7 @@
 // cached window (autoregressive decode): what the reference gets from flash-attn's
 // flash_attn_with_kvcache(q, k, v, causal=True, window_size=(W, 0), alibi_slopes=m) at
 // model/llama.py:684-688.  Per decoded token this reads 2 x (W + 1) x 128 bytes per (sequence, kv
-// head) and layer: HBM-bound, no tensor cores.
+// head) and layer: HBM-bound.
 //
 //   s[i, j] = scale * q_i . k_j  -  slope_h * (pos_i - j),   pos_i = T - Sq + i  (bottom-right aligned)
 //   visible: pos_i - W <= j <= pos_i;   out_i = softmax_j(s[i, :]) V
@@ -63,6 +63,8 @@ template <int R, bool ROUNDS> constexpr int WIN_WARPS = R > 1 ? 16 : ROUNDS ? 24
 
 template <int R> using WarpState = float[R][2 + 64];            // maximum, sum, 64 outputs of the rows
 
+// The kernels' first row: one row's is blockIdx.y, which is 0 -- as a constant it makes the 80-register kernel spill more (384 items x 512 keys 11.73
+// us, 11.62 so).
 // The warps' states (and a cluster's CTAs') to the outputs, in a fixed order.
 template <int R>
 __device__ __forceinline__ void merge_and_store(const WinParams& p, WarpState<R>* part, WarpState<R>& total, int ctas, int rank, int n, int hk, int row0, int rows) {
@@ -117,7 +119,7 @@ win_once_kernel(const WinParams p, int ctas) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = lane >> 3, sub = lane & 7, warps = blockDim.x >> 5;
   const int unit = blockIdx.x / ctas, rank = blockIdx.x - unit * ctas;
   const bool pairs = R > 1 && p.G * p.Sq > R;                    // three or four rows: an item's two pairs follow one another
-  const int item = pairs ? unit >> 1 : unit, row0 = pairs ? (unit & 1) * R : 0, rows = min(R, p.G * p.Sq - row0);
+  const int item = pairs ? unit >> 1 : unit, row0 = R == 1 ? blockIdx.y : pairs ? (unit & 1) * R : 0, rows = min(R, p.G * p.Sq - row0);
   const int n = item / p.Hkv, hk = item - n * p.Hkv;
   pdl_trigger();
   pdl_wait();
@@ -257,7 +259,8 @@ win_rounds_kernel(const WinParams p, int) {                      // one CTA an i
   __shared__ WarpState<R> part[WIN_WARPS<R, true>];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, warps = blockDim.x >> 5;
   const bool pairs = R > 1 && p.G * p.Sq > R;                    // three or four rows: an item's two pairs follow one another
-  const int item = pairs ? blockIdx.x >> 1 : blockIdx.x, row0 = pairs ? (blockIdx.x & 1) * R : 0, rows = min(R, p.G * p.Sq - row0);
+  const unsigned item = pairs ? blockIdx.x >> 1 : blockIdx.x;
+  const int row0 = R == 1 ? blockIdx.y : pairs ? (blockIdx.x & 1) * R : 0, rows = min(R, p.G * p.Sq - row0);
   const int n = item / p.Hkv, hk = item - n * p.Hkv;
   pdl_trigger();
   pdl_wait();
