@@ -166,7 +166,7 @@ int gca_fwd(const GcaFwdArgs* a, void* stream) {
     b.algo = algo;
     return gca::launch_fwd_tc(b, gca::sm_count(scope.dev), s);
   }
-  if (a->algo == GCA_ALGO_AUTO && gca::f32_tc_takes(a->dtype, a->S, (long long)a->N * a->J * a->Hq)) return gca::launch_fwd_f32_tc(*a, s);
+  if (a->algo == GCA_ALGO_AUTO && gca::f32_tc_takes(a->dtype, a->S, (long long)a->N * a->J * a->Hq)) return gca::launch_fwd_f32_tc(*a, scope.dev, s);
   if (algo == GCA_ALGO_SIMT) return gca::launch_fwd_simt(*a, s);
   return GCA_ERR_ALGO;
 }
@@ -249,7 +249,7 @@ int gca_bwd_stages(const GcaBwdArgs* a, unsigned stages, void* stream) {
                       gca::f32_tc_takes(a->dtype, a->S, (long long)a->N * (a->J > a->C ? a->J : a->C) * a->Hq);
   if (algo == GCA_ALGO_TC)
     rc = tc_ok ? gca::launch_bwd_tc(*a, csr, dw_part, rowterm, gca::sm_count(scope.dev), s, stages & GCA_BWD_STAGE_ALL) : GCA_ERR_ALGO;
-  else if (f32_tc) rc = gca::launch_bwd_f32_tc(*a, csr, dw_part, reinterpret_cast<float*>(rowterm), s, stages & GCA_BWD_STAGE_ALL);
+  else if (f32_tc) rc = gca::launch_bwd_f32_tc(*a, csr, dw_part, reinterpret_cast<float*>(rowterm), scope.dev, s, stages & GCA_BWD_STAGE_ALL);
   else if (algo == GCA_ALGO_SIMT) rc = gca::launch_bwd_simt(*a, csr, dw_part, reinterpret_cast<float*>(rowterm), s, stages & GCA_BWD_STAGE_ALL);
   else rc = GCA_ERR_ALGO;
   if (rc) return rc;

@@ -131,8 +131,8 @@ int launch_bwd_simt(const GcaBwdArgs& a, const Csr& csr, float* dw_part, float* 
 
 // float32 on the tensor cores, S = L = D = 64 (same scratch; four dw partials per (row block, head, slot), summed to dw by the q-major stage).
 bool f32_tc_takes(int dtype, int S, long long units);
-int launch_fwd_f32_tc(const GcaFwdArgs& a, cudaStream_t stream);
-int launch_bwd_f32_tc(const GcaBwdArgs& a, const Csr& csr, float* dw_part, float* row_di, cudaStream_t stream, unsigned stages);
+int launch_fwd_f32_tc(const GcaFwdArgs& a, int dev, cudaStream_t stream);
+int launch_bwd_f32_tc(const GcaBwdArgs& a, const Csr& csr, float* dw_part, float* row_di, int dev, cudaStream_t stream, unsigned stages);
 
 // tcgen05 / TMEM / TMA kernels: bf16, S = L = D = 64.
 int launch_fwd_tc(const GcaFwdArgs& a, int sms, cudaStream_t stream);

@@ -33,6 +33,7 @@
 // What bounds it now: the chains; a CTA takes ~5,400 cycles per slot in the forward, of which its own products are 1,024.
 // Tried and slower: eight worker warps in the forward (the row maxima and sums then cross groups: 135 us).
 #include "gca_simt.cuh"
+#include "per_device.cuh"
 #include "sm100_ptx.cuh"
 
 namespace gca {
@@ -815,16 +816,36 @@ bwd_kv_f32_tc_kernel(const float* __restrict__ q, const float* __restrict__ kc, 
 // One CTA per unit along x: problems past that limit (no memory holds their q) stay with the CUDA-core kernels.
 bool f32_tc_takes(int dtype, int S, long long units) { return dtype == GCA_F32 && S == 64 && units < (1ll << 31); }
 
+// The six kernels' shared memory, raised once per device: 0.4 us a call each, of ~90 of a small step.
+static int raise_limits(int dev) {
+  static PerDevice raised;
+  cudaError_t rc = cudaSuccess;
+  auto raise = [&](auto kernel, int bytes) {
+    if (rc == cudaSuccess) rc = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  };
+  int done = 0;
+  raised.get(dev, &done, [&](int* v) {
+    raise(fwd_f32_tc_kernel, SMEM_BYTES);
+    raise(bwd_q_f32_tc_kernel, SMEM_BYTES);
+    raise(bwd_kv_f32_tc_kernel, SMEM_BYTES);
+    raise(fwd_f32_again_kernel, FWD_UNIT_SMEM);
+    raise(bwd_q_f32_finish_kernel, BWD_Q_UNIT_SMEM);
+    raise(bwd_kv_f32_again_kernel, BWD_KV_UNIT_SMEM);
+    *v = 1;
+    return rc == cudaSuccess;
+  });
+  return (int)rc;
+}
+
 // As many blocks as run at once, each with a word to read for every unit it answers for: ~2 us where nothing is marked.
 template <class... Params, class... Args>
 static int launch_again(void (*kernel)(Params...), long long units, int blocks_per_sm, int smem, cudaStream_t stream, Args... args) {
-  GCA_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   return (int)launch_dependent(kernel, dim3((unsigned)(units < 148 * blocks_per_sm ? units : 148 * blocks_per_sm)), dim3(NTHREADS), smem, stream, args...);
 }
 
-int launch_fwd_f32_tc(const GcaFwdArgs& a, cudaStream_t stream) {
+int launch_fwd_f32_tc(const GcaFwdArgs& a, int dev, cudaStream_t stream) {
+  if (int rc = raise_limits(dev)) return rc;
   const long long units = (long long)a.N * a.J * a.Hq;
-  GCA_CUDA_CHECK(cudaFuncSetAttribute(fwd_f32_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
   const float *q = (const float*)a.q, *kc = (const float*)a.k_cache, *vc = (const float*)a.v_cache;
   fwd_f32_tc_kernel<<<(unsigned)units, threads_of(FWD_WORKERS), SMEM_BYTES, stream>>>(q, kc, vc, a.indices, a.weights, (float*)a.out, a.lse, a.status,
                                                                                       make_geom(a));
@@ -832,23 +853,21 @@ int launch_fwd_f32_tc(const GcaFwdArgs& a, cudaStream_t stream) {
   return launch_again(fwd_f32_again_kernel, units, 4, FWD_UNIT_SMEM, stream, q, kc, vc, a.indices, a.weights, (float*)a.out, a.lse, make_geom(a));
 }
 
-int launch_bwd_f32_tc(const GcaBwdArgs& a, const Csr& csr, float* dw_part, float* row_di, cudaStream_t stream, unsigned stages) {
+int launch_bwd_f32_tc(const GcaBwdArgs& a, const Csr& csr, float* dw_part, float* row_di, int dev, cudaStream_t stream, unsigned stages) {
+  if (int rc = raise_limits(dev)) return rc;
   const Geom g = make_geom(a);
   BwdStrides st;
   for (int i = 0; i < 4; ++i) { st.dout[i] = a.do_stride[i]; st.dk[i] = a.dk_stride[i]; st.dv[i] = a.dv_stride[i]; }
   const float *q = (const float*)a.q, *kc = (const float*)a.k_cache, *vc = (const float*)a.v_cache, *dout = (const float*)a.dout;
   const long long q_units = (long long)a.N * a.J * a.Hq, kv_units = (long long)a.N * a.C * a.Hkv;
   if ((stages & GCA_BWD_STAGE_Q) && q_units > 0) {
-    GCA_CUDA_CHECK(cudaFuncSetAttribute(bwd_q_f32_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
     GCA_CUDA_CHECK(launch_dependent(bwd_q_f32_tc_kernel, dim3((unsigned)q_units), dim3(threads_of(BWD_WORKERS)), SMEM_BYTES, stream, q, kc, vc,
                                     a.indices, a.weights, dout, a.lse, (float*)a.dq, dw_part, row_di, a.status, g, (int)csr.overlaps,
                                     a.do_stride[0], a.do_stride[1], a.do_stride[2], a.do_stride[3]));
-    GCA_CUDA_CHECK(cudaFuncSetAttribute(bwd_q_f32_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BWD_Q_UNIT_SMEM));
     GCA_CUDA_CHECK(launch_dependent(bwd_q_f32_finish_kernel, dim3((unsigned)(a.N * a.J)), dim3(NTHREADS), BWD_Q_UNIT_SMEM, stream, q, kc, vc, a.indices,
                                     a.weights, dout, a.lse, (float*)a.dq, dw_part, row_di, (float*)a.dw, g, st));
   }
   if ((stages & GCA_BWD_STAGE_KV) && kv_units > 0) {
-    GCA_CUDA_CHECK(cudaFuncSetAttribute(bwd_kv_f32_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
     bwd_kv_f32_tc_kernel<<<(unsigned)kv_units, threads_of(BWD_WORKERS), SMEM_BYTES, stream>>>(
         q, kc, vc, a.weights, dout, a.lse, row_di, (float*)a.dk_cache, (float*)a.dv_cache, a.status, csr, g,
         a.do_stride[0], a.do_stride[1], a.do_stride[2], a.do_stride[3],
