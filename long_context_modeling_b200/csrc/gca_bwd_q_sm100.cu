@@ -68,7 +68,7 @@ constexpr int NWG = GCA_Q_NWG;              // measured: 2 groups 0.653 ms, 3 gr
 static_assert(NWG >= 2 && NWG <= NBUF, "worker groups");
 // The issuers probe the NEXT slot's barriers before they issue the current slot's MMAs, so that the
 // probes' shared-memory round trip runs under the issue: 0.562 -> 0.538 ms.  (The same in the
-// forward and in the kv-major kernel was measured slower: 0.434 against 0.414 and 0.634 against
+// forward and in the kv-major kernel was measured slower: 0.398 against 0.357 and 0.634 against
 // 0.613 ms.)
 #ifndef GCA_Q_PREPROBE
 #define GCA_Q_PREPROBE 1

@@ -157,7 +157,7 @@ __device__ __forceinline__ UnitInfo unit_info(const FwdTcParams& p, int hp) {
   else { t.hk0 = t.h0 / p.G; t.share = t.two && ((t.h0 + 1) / p.G == t.hk0); }
   return t;
 }
-// Lane-parallel read of one row of retrieved indices; every role prefetches the next row.
+// Lane-parallel read of one row of retrieved indices (the Q / K producer, one row ahead).
 __device__ __forceinline__ int load_index_row(const FwdTcParams& p, int u, int zj, int lane) {
   if (u >= p.units || lane >= p.K) return -1;
   return slot_chunk(p.indices, zj, p.K, lane);
