@@ -50,7 +50,8 @@ enum GcaError {
 
 /* kernel variants (GcaFwdArgs.algo / GcaBwdArgs.algo) */
 enum GcaAlgo {
-  GCA_ALGO_AUTO = 0,        /* S=L=D=64: tensor-core kernels (fp32: each operand as three bf16 values), everything else -> SIMT */
+  GCA_ALGO_AUTO = 0,        /* S=L=D=64: tensor-core kernels (fp32: each operand as three bf16 values; where infinities, NaN, overflow or
+                               operands below 2^-110 are involved, results as from SIMT), everything else -> SIMT */
   GCA_ALGO_SIMT = 1,        /* fp32-accumulating CUDA-core kernel (bf16 or fp32 data) */
   GCA_ALGO_TC = 2,          /* tcgen05/TMEM/TMA kernel (bf16 only) */
   GCA_ALGO_TC_UNPAIRED = 3  /* forward only: the tensor-core kernel with ONE q head per work unit instead of a
