@@ -265,17 +265,21 @@ struct Frame {
     tmem = *slot;
     quarter = tmem + ((uint32_t)((warp & 3) * 32) << 16);
   }
-  // Whatever ended the CTA: no MMA is in flight any more when tensor memory is given back.
-  __device__ __forceinline__ void leave(int32_t* status) const {
+  // Whatever ended the CTA: no MMA is in flight any more when tensor memory is given back.  VOTE: true if `vote` is in some thread and no wait
+  // has run out.
+  template <bool VOTE = false>
+  __device__ __forceinline__ bool leave(int32_t* status, bool vote = false) const {
     if (warp == ISSUER && *abort_flag) {
       umma_commit_elect(&bars[DRAIN]);
       for (int i = 0; i < (1 << 20); ++i)
         if (mbar_try_wait(&bars[DRAIN], 0)) break;
     }
     tc_fence_before();
-    __syncthreads();
+    if (VOTE) vote = __syncthreads_or(vote);
+    else __syncthreads();
     if (warp == ISSUER) tmem_dealloc(tmem, TMEM_COLS);
     if (threadIdx.x == 0 && *abort_flag && status) atomicOr(status, GCA_STATUS_TIMEOUT);
+    return VOTE && vote && !*abort_flag;
   }
 };
 __device__ __forceinline__ uint8_t* aligned_smem(uint8_t* raw) {
@@ -331,8 +335,9 @@ struct BwdStrides { long long dout[4], dk[4], dv[4]; };
 // is zero): an infinite operand or a sum past the largest number ends as a NaN here, where multiply-adds give an infinity or, for a score
 // of -inf, a weight of zero; and of operands below 2^-110 bits are lost.  The warp then puts a NaN that no arithmetic produces in the place of its
 // first output, and a kernel behind this one does the units so marked over again with multiply-adds.  Where nothing is marked the kernels behind
-// cost 3.0 us (forward), 4.6 (q-major, which sums dw by the way; that alone took 5.2) and 3.2 (kv-major).  As a call from the kernels
-// themselves the same took registers from their loops: kv-major 205 -> 230 us, q-major 165 -> 178.
+// cost 3.0 us (forward), 4.6 (q-major, which sums dw by the way; that alone took 5.2) and 3.2 (kv-major).
+// HERE: the forward and the kv-major kernel do that themselves, on the spot: a launch less for short passes.  The code takes
+// registers from their loops, 2.7 % of the forward and 11 % of kv-major (205 -> 228 us; q-major 165 -> 178, which has the kernel behind for dw).
 constexpr unsigned MARK = 0x7fc5f32bu;
 template <int N>
 __device__ __forceinline__ bool outside(const float (&acc)[N]) {
@@ -349,6 +354,16 @@ __device__ __forceinline__ bool marked(const float* tile, long long row_stride, 
   for (int w = 0; w < warps; ++w) any |= *reinterpret_cast<const volatile unsigned*>(tile + (w & 3) * 16 * row_stride + (w >> 2) * 32) == MARK;
   return any;
 }
+__device__ __forceinline__ int this_block() {        // looked up again rather than kept through the kernel
+  int b;
+  asm volatile("mov.u32 %0, %%ctaid.x;" : "=r"(b));
+  return b;
+}
+__device__ __forceinline__ float* unit_smem() {
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  return reinterpret_cast<float*>(aligned_smem(smem_raw));
+}
+static_assert(FWD_UNIT_SMEM <= OFF_BAR && BWD_KV_UNIT_SMEM <= OFF_BAR, "shared memory of a unit done on the spot");
 // The units b, b + blocks, ...: a thread looks at one, then the block does the marked ones together.
 template <class Marked, class Unit>
 __device__ __forceinline__ void do_marked(int units, Marked is_marked, Unit unit) {
@@ -410,6 +425,7 @@ bwd_kv_f32_again_kernel(const float* q, const float* kc, const float* vc, const 
 // Regions: Q | scores | probabilities | product.  The next slot's scores are computed while this slot's are worked on, its product while
 // the next slot's are.  The product takes exp2(S - m) / 64; w / l is a factor of the sum over the slots.
 // Tiles: a ring, in the order of use K0 K1 V0 K2 V1 ...
+template <bool HERE>
 __global__ void __launch_bounds__(threads_of(FWD_WORKERS), 2)
 fwd_f32_tc_kernel(const float* __restrict__ q, const float* __restrict__ kc, const float* __restrict__ vc,
                   const int32_t* __restrict__ indices, const float* __restrict__ weights, float* __restrict__ out,
@@ -425,6 +441,7 @@ fwd_f32_tc_kernel(const float* __restrict__ q, const float* __restrict__ kc, con
   } else if (nv > 0 && f.warp < f.ISSUER)
     fetch_tile(kc + u.n * g.ks[0] + u.first * g.ks[1] + u.hk * g.ks[3], g.ks[2], threadIdx.x - FWD_WORKERS * 32, v);
   f.set_up(aligned_smem(smem_raw));
+  bool again = false;
 
   if (f.warp < FWD_WORKERS) {
     const long long slot0 = (u.zj * g.Hq + u.h) * g.K;
@@ -497,7 +514,8 @@ fwd_f32_tc_kernel(const float* __restrict__ q, const float* __restrict__ kc, con
       float* first = nullptr;
 #pragma unroll
       for (int h = 1; h >= 0; --h) first = store_cols32(out + u.n * g.os[0] + u.j * g.os[1] + u.h * g.os[2], g.os[3], f.row, f.lane, h, acc + 16 * h, 1.0f);
-      if (outside(acc) && f.lane == 0) mark(first);
+      again = outside(acc);
+      if (!HERE && again && f.lane == 0) mark(first);
     }
   } else if (f.warp < f.ISSUER) {
     if (nv > 0) {
@@ -542,7 +560,10 @@ fwd_f32_tc_kernel(const float* __restrict__ q, const float* __restrict__ kc, con
       if (++st == NTILES) { st = 0; ph ^= 1; }
     }
   }
-  f.leave(status);
+  if (f.leave<HERE>(status, again) && threadIdx.x < NTHREADS) {
+    const UnitId w(g, this_block());
+    fwd_unit<float>(unit_smem(), w.n * g.J + w.j, w.h, q, kc, vc, indices, weights, out, lse, nullptr, g);
+  }
 }
 
 // ------------------------------------------------------------------------------------ backward, q-major
@@ -677,6 +698,7 @@ bwd_q_f32_tc_kernel(const float* __restrict__ q, const float* __restrict__ kc, c
 // scores: rows = keys, so probabilities and their gradients are the A operands of the gradient products as they stand.
 // Regions: K | S^T, then w P^T | dP^T, then dS^T | dV of the step, then its dK.  Tiles 0: V; 1: dO of the step; 2, 3: Q of even and
 // odd steps.  V stays in shared memory (there is no fifth region), so dP^T is the one product of 64 rows.
+template <bool HERE>
 __global__ void __launch_bounds__(threads_of(BWD_WORKERS), 2)
 bwd_kv_f32_tc_kernel(const float* __restrict__ q, const float* __restrict__ kc, const float* __restrict__ vc,
                      const float* __restrict__ weights, const float* __restrict__ dout, const float* __restrict__ lse,
@@ -698,6 +720,7 @@ bwd_kv_f32_tc_kernel(const float* __restrict__ q, const float* __restrict__ kc, 
   if (steps > 0 && f.warp < BWD_WORKERS) load_cols32(kc + n * g.ks[0] + c * g.ks[1] + hk * g.ks[3], g.ks[2], f.row, f.lane, f.group, v);
   else if (steps > 0 && f.warp < f.ISSUER) fetch_tile(vc + n * g.vs[0] + c * g.vs[1] + hk * g.vs[3], g.vs[2], threadIdx.x - BWD_WORKERS * 32, v);
   f.set_up(aligned_smem(smem_raw));
+  bool again = false;
 
   if (f.warp < BWD_WORKERS) {
     if (steps > 0) {                               // a group brings its 32 columns of K
@@ -750,7 +773,8 @@ bwd_kv_f32_tc_kernel(const float* __restrict__ q, const float* __restrict__ kc, 
     if (ok) {
       float* first = store_cols32(dk + n * dks0 + c * dks1 + hk * dks3, dks2, f.row, f.lane, f.group, aK, g.sm_scale);
       store_cols32(dv + n * dvs0 + c * dvs1 + hk * dvs3, dvs2, f.row, f.lane, f.group, aV, 1.0f);
-      if ((outside(aK) | outside(aV)) && f.lane == 0) mark(first);
+      again = outside(aK) | outside(aV);
+      if (!HERE && again && f.lane == 0) mark(first);
     }
   } else if (f.warp < f.ISSUER) {
     if (steps > 0) {
@@ -808,7 +832,11 @@ bwd_kv_f32_tc_kernel(const float* __restrict__ q, const float* __restrict__ kc, 
       }
     }
   }
-  f.leave(status);
+  if (f.leave<HERE>(status, again) && threadIdx.x < NTHREADS) {
+    const int b = this_block();
+    bwd_kv_unit<float>(unit_smem(), csr.unit_tab[b / g.Hkv], b % g.Hkv, q, kc, vc, weights, dout, lse, row_di, dk, dv, csr, g, dos0, dos1, dos2, dos3,
+                       dks0, dks1, dks2, dks3, dvs0, dvs1, dvs2, dvs3);
+  }
 }
 
 }  // namespace
@@ -816,7 +844,7 @@ bwd_kv_f32_tc_kernel(const float* __restrict__ q, const float* __restrict__ kc, 
 // One CTA per unit along x: problems past that limit (no memory holds their q) stay with the CUDA-core kernels.
 bool f32_tc_takes(int dtype, int S, long long units) { return dtype == GCA_F32 && S == 64 && units < (1ll << 31); }
 
-// The six kernels' shared memory, raised once per device: 0.4 us a call each, of ~90 of a small step.
+// The kernels' shared memory, raised once per device: 0.4 us a call each, of ~90 of a small step.
 static int raise_limits(int dev) {
   static PerDevice raised;
   cudaError_t rc = cudaSuccess;
@@ -825,9 +853,11 @@ static int raise_limits(int dev) {
   };
   int done = 0;
   raised.get(dev, &done, [&](int* v) {
-    raise(fwd_f32_tc_kernel, SMEM_BYTES);
+    raise(fwd_f32_tc_kernel<false>, SMEM_BYTES);
+    raise(fwd_f32_tc_kernel<true>, SMEM_BYTES);
     raise(bwd_q_f32_tc_kernel, SMEM_BYTES);
-    raise(bwd_kv_f32_tc_kernel, SMEM_BYTES);
+    raise(bwd_kv_f32_tc_kernel<false>, SMEM_BYTES);
+    raise(bwd_kv_f32_tc_kernel<true>, SMEM_BYTES);
     raise(fwd_f32_again_kernel, FWD_UNIT_SMEM);
     raise(bwd_q_f32_finish_kernel, BWD_Q_UNIT_SMEM);
     raise(bwd_kv_f32_again_kernel, BWD_KV_UNIT_SMEM);
@@ -843,13 +873,20 @@ static int launch_again(void (*kernel)(Params...), long long units, int blocks_p
   return (int)launch_dependent(kernel, dim3((unsigned)(units < 148 * blocks_per_sm ? units : 148 * blocks_per_sm)), dim3(NTHREADS), smem, stream, args...);
 }
 
+// (query chunk, head, slot) up to which the forward and the kv-major pass do units outside the range themselves (HERE): where the launch saved, 3 us of
+// the device's time and as much of the host's, is worth the registers.  The forward at 12,096: 113.1 us against 111.5 + 3.0.  kv-major:
+// steps of 40 to 936 84 us, 90 with the launch (the host's time); 1,440 and more are the device's time, 107.4 with it, 108.2 without.
+constexpr long long FWD_HERE_SLOTS = 12288, KV_HERE_SLOTS = 1024;
+
 int launch_fwd_f32_tc(const GcaFwdArgs& a, int dev, cudaStream_t stream) {
   if (int rc = raise_limits(dev)) return rc;
   const long long units = (long long)a.N * a.J * a.Hq;
+  const bool here = units * a.K <= FWD_HERE_SLOTS;
   const float *q = (const float*)a.q, *kc = (const float*)a.k_cache, *vc = (const float*)a.v_cache;
-  fwd_f32_tc_kernel<<<(unsigned)units, threads_of(FWD_WORKERS), SMEM_BYTES, stream>>>(q, kc, vc, a.indices, a.weights, (float*)a.out, a.lse, a.status,
-                                                                                      make_geom(a));
+  auto kernel = here ? fwd_f32_tc_kernel<true> : fwd_f32_tc_kernel<false>;
+  kernel<<<(unsigned)units, threads_of(FWD_WORKERS), SMEM_BYTES, stream>>>(q, kc, vc, a.indices, a.weights, (float*)a.out, a.lse, a.status, make_geom(a));
   GCA_CUDA_CHECK(cudaGetLastError());
+  if (here) return 0;
   return launch_again(fwd_f32_again_kernel, units, 4, FWD_UNIT_SMEM, stream, q, kc, vc, a.indices, a.weights, (float*)a.out, a.lse, make_geom(a));
 }
 
@@ -868,12 +905,15 @@ int launch_bwd_f32_tc(const GcaBwdArgs& a, const Csr& csr, float* dw_part, float
                                     a.weights, dout, a.lse, (float*)a.dq, dw_part, row_di, (float*)a.dw, g, st));
   }
   if ((stages & GCA_BWD_STAGE_KV) && kv_units > 0) {
-    bwd_kv_f32_tc_kernel<<<(unsigned)kv_units, threads_of(BWD_WORKERS), SMEM_BYTES, stream>>>(
+    const bool here = q_units * a.K <= KV_HERE_SLOTS;
+    auto kernel = here ? bwd_kv_f32_tc_kernel<true> : bwd_kv_f32_tc_kernel<false>;
+    kernel<<<(unsigned)kv_units, threads_of(BWD_WORKERS), SMEM_BYTES, stream>>>(
         q, kc, vc, a.weights, dout, a.lse, row_di, (float*)a.dk_cache, (float*)a.dv_cache, a.status, csr, g,
         a.do_stride[0], a.do_stride[1], a.do_stride[2], a.do_stride[3],
         a.dk_stride[0], a.dk_stride[1], a.dk_stride[2], a.dk_stride[3],
         a.dv_stride[0], a.dv_stride[1], a.dv_stride[2], a.dv_stride[3]);
     GCA_CUDA_CHECK(cudaGetLastError());
+    if (here) return 0;
     return launch_again(bwd_kv_f32_again_kernel, kv_units, 2, BWD_KV_UNIT_SMEM, stream, q, kc, vc, a.weights, dout, a.lse, row_di, (float*)a.dk_cache,
                         (float*)a.dv_cache, csr, g, st);
   }
