@@ -50,8 +50,9 @@ enum GcaError {
 
 /* kernel variants (GcaFwdArgs.algo / GcaBwdArgs.algo) */
 enum GcaAlgo {
-  GCA_ALGO_AUTO = 0,        /* S=L=D=64: tensor-core kernels (fp32: each operand as three bf16 values; where infinities, NaN, overflow or
-                               operands below 2^-110 are involved, results as from SIMT), everything else -> SIMT */
+  GCA_ALGO_AUTO = 0,        /* S=L=D=64: tensor-core kernels (fp32: each operand as three bf16 values, exact from 2^-110 on,
+                               below that to 2^-134 absolutely; where 16 rows of a result hold infinities or
+                               NaN, or nothing that reaches 2^-100, the chunk's as from SIMT), everything else -> SIMT */
   GCA_ALGO_SIMT = 1,        /* fp32-accumulating CUDA-core kernel (bf16 or fp32 data) */
   GCA_ALGO_TC = 2,          /* tcgen05/TMEM/TMA kernel (bf16 only) */
   GCA_ALGO_TC_UNPAIRED = 3  /* forward only: the tensor-core kernel with ONE q head per work unit instead of a

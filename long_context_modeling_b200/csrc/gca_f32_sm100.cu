@@ -333,9 +333,10 @@ struct BwdStrides { long long dout[4], dk[4], dv[4]; };
 // ------------------------------------------------------------------------------------ units outside the range
 // What a warp holds of a unit's outputs lies outside the kernels' range if anything is infinite or NaN, or if nothing reaches 2^-100 (and not all
 // is zero): an infinite operand or a sum past the largest number ends as a NaN here, where multiply-adds give an infinity or, for a score
-// of -inf, a weight of zero; and of operands below 2^-110 bits are lost.  The warp then puts a NaN that no arithmetic produces in the place of its
-// first output, and a kernel behind this one does the units so marked over again with multiply-adds.  Where nothing is marked the kernels behind
-// cost 3.0 us (forward), 4.6 (q-major, which sums dw by the way; that alone took 5.2) and 3.2 (kv-major).
+// of -inf, a weight of zero; and of operands below 2^-110 bits are lost (not found: where larger ones have brought the products back above
+// 2^-100, or others of the warp's outputs lie there; the split's 2^-134 of the operand, absolutely, is then the error).  The warp puts a NaN
+// that no arithmetic produces in the place of its first output, and a kernel behind this one does the units so marked over again with
+// multiply-adds.  Where nothing is marked the kernels behind cost 3.0 us (forward), 4.6 (q-major, which sums dw by the way; that alone took 5.2) and 3.2 (kv-major).
 // HERE: the forward and the kv-major kernel do that themselves, on the spot: a launch less for short passes.  The code takes
 // registers from their loops, 2.7 % of the forward and 11 % of kv-major (205 -> 228 us; q-major 165 -> 178, which has the kernel behind for dw).
 constexpr unsigned MARK = 0x7fc5f32bu;
