@@ -15,24 +15,27 @@
 //
 // Every product is computed per head with 64-row MMAs.  A 64-row accumulator or tensor-memory
 // operand occupies lanes 0-15 of every 32-lane quarter, so head B's tiles, placed at lane offset
-// 16, share head A's columns: S and dP of a head PAIR take 128 columns, and THREE such score
-// buffers plus two dQ accumulators (64 columns each for both heads) fill the 512 columns.  A
-// buffer goes through  MMA (S, dP) -> worker -> MMA (dQ) -> release  in a few thousand cycles;
-// with three of them, and one worker warpgroup per buffer, slot g + 1 and g + 2 are computed while
-// slot g is still being worked on.  (With stacked 128-row products S and dP took 256 columns and
-// could not be double-buffered: issue of the eight MMAs, the workers' read and two barrier hops
-// formed a serial chain of ~1,900 cycles per slot.)
+// 16, share head A's columns: S and dP of a head PAIR take 64 columns each.  S is free again when its slot's
+// worker group has read P back (~3,000 cycles after the MMAs were issued), dP when the dQ product has consumed the dS in its place
+// (~4,300): three S regions, four dP regions and one dQ accumulator fill the 512 columns.
 //
 // A worker thread never holds a whole row in registers: it walks its 64 keys twice in passes of
 // 16 columns.  Pass 1 reads S and dP, accumulates Di and writes P as packed bf16 over the S
 // columns it has already read; pass 2 reads P and dP back and writes dS = P (w dP - w Di) as
 // packed bf16 over the dP columns, from where the dQ product takes it as its A operand (lane =
-// row of A = query row).  82 registers instead of 161, which is what lets three worker groups
-// and twenty warps fit.  Shared memory sees only the TMA copies and the MMAs' operand reads.
+// row of A = query row).  76 registers, which is what lets four worker groups
+// and twenty-four warps fit.  Shared memory sees only the TMA copies and the MMAs' operand reads.
 //
-// CTA = 20 warps: three worker warpgroups, one TMA producer, three MMA issuers (S, dP, dQ), and a
-// warpgroup that writes the finished dQ tiles.  No
+// CTA = 24 warps: four worker warpgroups, one TMA producer, three MMA issuers (S, dP, dQ), and a
+// warpgroup that writes the finished dQ tiles.  The producer walks the unit list and publishes one RECORD per valid slot; the
+// others follow the records and have no code that runs once per unit.  No
 // atomics: gradients are bit-reproducible.  Every wait is bounded (GCA_STATUS_TIMEOUT on expiry).
+//
+// What bounds it (event trace at 8 x 256 chunks, 12 heads, K = 8): the S and dP issuers, ~1,220 cycles a slot inside a unit and 1,330 on
+// average, of which the slot's 24 MMAs take 768.  With three groups on three shared S / dP buffers, and every role walking the units
+// by itself, it was 1,515: the groups, busy all of their 4,170 cycles a slot, and 870 cycles at each unit's end.  Each change alone gave little
+// (four groups 522 -> 511 us, records with three groups 512 -> 521, separate regions with three groups 521 -> 532), together 523 -> 506,
+// and 547 -> 540 at 1 x 1,024 chunks, K = 16.
 #include "gca_common.cuh"
 #include "sm100_ptx.cuh"
 #include "tc_common.cuh"
@@ -49,30 +52,12 @@ using namespace sm100;
 constexpr int TILE_BYTES = 64 * 64 * 2;
 constexpr int PAIR_BYTES = 2 * TILE_BYTES;
 constexpr uint32_t PAIR16 = PAIR_BYTES >> 4, TILE16 = TILE_BYTES >> 4;
-#ifndef GCA_Q_NBUF
-#define GCA_Q_NBUF 3
-#endif
-constexpr int NBUF = GCA_Q_NBUF;
-static_assert(NBUF == 2 || NBUF == 3, "score buffers");
-// One issuing warp per product.  An issuer needs ~1,300 cycles per slot (probe of its two barriers
-// ~330, eight 64-row MMAs and the commits ~600, loop bookkeeping ~300: event traces), which is what
-// bounds the kernel today; yet more issuing warps were measured SLOWER, both ways tried: one warp
-// per head (the heads of a slot share the buffer's columns) 0.835 against 0.567 ms, one warp per
-// slot parity for S and dP 1,640 against 1,390 cycles per slot -- every extra polling warp slows
-// the shared-memory path that the MMAs' operand reads already load to ~875 of those cycles.
-// Worker warpgroups: slot g goes to group g % NWG (and to buffer g % NBUF).
-#ifndef GCA_Q_NWG
-#define GCA_Q_NWG GCA_Q_NBUF
-#endif
-constexpr int NWG = GCA_Q_NWG;              // measured: 2 groups 0.653 ms, 3 groups 0.55-0.57 ms
-static_assert(NWG >= 2 && NWG <= NBUF, "worker groups");
-// The issuers probe the NEXT slot's barriers before they issue the current slot's MMAs, so that the
-// probes' shared-memory round trip runs under the issue: 0.562 -> 0.538 ms.  (The same in the
-// forward and in the kv-major kernel was measured slower: 0.398 against 0.357 and 0.634 against
-// 0.613 ms.)
-#ifndef GCA_Q_PREPROBE
-#define GCA_Q_PREPROBE 1
-#endif
+// One issuing warp per product.  More were measured SLOWER, both ways tried: one warp
+// per head (the heads of a slot share the region's columns) 0.835 against 0.567 ms, one warp per
+// slot parity for S and dP 1,640 against 1,390 cycles per slot.
+constexpr int NS = 3, NDP = 4;              // S regions, dP regions of tensor memory
+constexpr int NWG = 4;                      // worker warpgroups: slot g goes to group g % 4
+static_assert(NWG == NDP, "a group's dP region is its own");
 constexpr int PROD_WARP = 4 * NWG, ISSUE_S = PROD_WARP + 1, ISSUE_DP = ISSUE_S + 1, ISSUE_DQ = ISSUE_DP + 1;
 constexpr int WRITER_WARP = (ISSUE_DQ + 1 + 3) / 4 * 4;   // a multiple of 4: warp % 4 = its TMEM lane quarter
 constexpr int NTHREADS = (WRITER_WARP + 4) * 32;
@@ -83,29 +68,46 @@ constexpr uint32_t IDESC_DQ = umma_idesc_bf16(64, 64, 0, 1);       // A: tensor 
 constexpr int STEP_K = 2;      // K-major operand: +32 bytes (>> 4) per K step of 16
 constexpr int STEP_MN = 128;   // MN-major operand: +2048 bytes (>> 4) per K step of 16
 
-#ifndef GCA_Q_NKS
-#define GCA_Q_NKS 6
-#endif
-#ifndef GCA_Q_NVS
-#define GCA_Q_NVS 4
-#endif
-constexpr int NKS = GCA_Q_NKS, NVS = GCA_Q_NVS;
+constexpr int NKS = 6, NVS = 4;              // K / V ring stages
 constexpr int OFF_QDO = 0;                                   // [2][Q pair | dO pair]
 constexpr int OFF_K = OFF_QDO + 2 * 2 * PAIR_BYTES;          // [NKS][K pair]
 constexpr int OFF_V = OFF_K + NKS * PAIR_BYTES;              // [NVS][V pair]
 constexpr int OFF_BAR = OFF_V + NVS * PAIR_BYTES;
-constexpr int OFF_IDX = OFF_BAR + 512;
-constexpr int SMEM_BYTES = OFF_IDX + 256 + 1024;
+constexpr int OFF_REC = OFF_BAR + 512;                       // [NKS]
+constexpr int NU = 8;                                        // unit records
+constexpr int OFF_UREC = OFF_REC + NKS * 16;                 // [NU]
+constexpr int SMEM_BYTES = OFF_UREC + NU * 16 + 1024;
 static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
+// A slot's record lies in the place of its K stage.  REC_FULL[stage]: it is written; K_FULL and V_FULL say so too (the same lane
+// writes it and then arrives there), and who has seen PDS_FULL of the slot.  K_EMPTY of a stage -- dQ of the slot that had it is
+// complete -- means that every role has read that slot's record.  UREC_FULL[u % NU]: the writer's record of unit u; when it is
+// written, dP of unit u - 2 is complete, hence, with one slot a unit, dQ of unit u - 6, and the writer is past unit u - 7.
+// S_FULL, DP_FULL, PDS_FULL, DP_FREE belong to a worker group, i.e. to every fourth slot.  PDS_FULL: P is read and dS written, so dQ may run
+// and S of the slot three later may take the S region.
 enum Bar { QDO_FULL = 0, QDO_EMPTY = 2, K_FULL = 4, K_EMPTY = K_FULL + NKS, V_FULL = K_EMPTY + NKS,
-           V_EMPTY = V_FULL + NVS, SP_FULL = V_EMPTY + NVS, PDS_FULL = SP_FULL + NBUF, BUF_FREE = PDS_FULL + NBUF,
-           ACC_FULL = BUF_FREE + NBUF, ACC_EMPTY = ACC_FULL + 2, NUM_BARS = ACC_EMPTY + 2 };
+           V_EMPTY = V_FULL + NVS, S_FULL = V_EMPTY + NVS, DP_FULL = S_FULL + NWG, PDS_FULL = DP_FULL + NWG, DP_FREE = PDS_FULL + NWG,
+           ACC_FULL = DP_FREE + NWG, ACC_EMPTY = ACC_FULL + 1, REC_FULL = ACC_EMPTY + 1, UREC_FULL = REC_FULL + NKS,
+           NUM_BARS = UREC_FULL + NU };
 static_assert(NUM_BARS * 8 + 16 <= 512, "barrier block");
-// Tensor-memory columns.  Buffer b (slot g uses b = g % NBUF) = 128 columns: S at +0 and dP at
-// +64 as float32; afterwards P at +0 and dS at +64 as packed bf16 (32 columns each).  Behind the
-// buffers two dQ accumulators of 64 columns (unit u uses accumulator u % 2).
-constexpr uint32_t BUF_COLS = 128, COL_DPT = 64, COL_DQ = NBUF * BUF_COLS;
-static_assert(NBUF * BUF_COLS + 128 <= TMEM_COLS, "tensor memory");
+
+// What the other roles need to know about a slot, and the writer about a unit.
+struct SlotRec {
+  uint32_t flags;           // REC_*
+  float w;                  // retrieval weight
+  long long row_off;        // element offset of (row block, head A, this slot, row 0) in lse and rowterm; 16 times that in dw_part
+};
+struct UnitRec {
+  uint32_t flags, pad;
+  long long dq_off;         // element offset of (row block, head A, row 0) in dq
+};
+constexpr uint32_t REC_END = 1, REC_FIRST = 2, REC_LAST = 4, REC_TWO = 8, REC_SHARE = 16;     // END: no more slots; FIRST / LAST of its unit
+static_assert(sizeof(SlotRec) == 16 && sizeof(UnitRec) == 16, "records");
+__device__ __forceinline__ SlotRec* slot_recs(uint8_t* smem) { return reinterpret_cast<SlotRec*>(smem + OFF_REC); }
+__device__ __forceinline__ UnitRec* unit_recs(uint8_t* smem) { return reinterpret_cast<UnitRec*>(smem + OFF_UREC); }
+// Tensor-memory columns: three S regions (slot g: g % 3), four dP regions (g % 4), one dQ accumulator, 64 columns each.  P (packed
+// bf16, 32 columns) lands on S, dS on dP.
+constexpr uint32_t COL_DP = NS * 64, COL_DQ = COL_DP + NDP * 64;
+static_assert(COL_DQ + 64 <= TMEM_COLS, "tensor memory");
 
 // x as the sum of three bf16 values (24 mantissa bits: float32 precision).
 __device__ __forceinline__ void split3(float x, __nv_bfloat16& h, __nv_bfloat16& m, __nv_bfloat16& l) {
@@ -179,152 +181,198 @@ __device__ __forceinline__ unsigned q_valid(const BwdQParams& p, int idx) {
   return __ballot_sync(0xffffffffu, idx >= 0 && idx < p.C);
 }
 
-// One lane: Q + dO per unit, K and V per slot.
+// Walks this CTA's units: lane k publishes the record of slot k and issues its copies when its turn has come, the first valid lane the
+// unit's record and its Q and dO copies too.  What no slot will write is also written here (rare: the first K chunks of a
+// sequence): dw partials of padding slots, dQ rows of a unit without valid slots.
 __device__ void q_producer(const BwdQParams& p, uint8_t* smem, uint64_t* bars, volatile int* abort_flag, int lane) {
-  int* sidx = reinterpret_cast<int*>(smem + OFF_IDX);
+  SlotRec* recs = slot_recs(smem);
+  UnitRec* urecs = unit_recs(smem);
   PairCursor c;
   c.init(p.HP);
   Ring rk, rv; rk.init(NKS); rv.init(NVS);
-  uint32_t ucnt = 0, issued = 0;
+  uint32_t un = 0, k_issued = 0, v_issued = 0, q_issued = 0;
   bool ok = true;
+  const unsigned full = (p.K >= 32) ? 0xffffffffu : ((1u << p.K) - 1u);
   int next_idx = q_load_row(p, c.u, c.outer, lane);
-  for (; c.u < p.units; c.advance()) {
+  float next_w = (c.u < p.units && lane < p.K) ? p.weights[(long long)c.outer * p.K + lane] : 0.f;
+  for (; c.u < p.units && ok; c.advance()) {
     const int my_idx = next_idx;
-    next_idx = q_load_row(p, c.u + gridDim.x, c.next_outer(), lane);
+    const float my_w = next_w;
+    {
+      const int nzj = c.next_outer();
+      next_idx = q_load_row(p, c.u + gridDim.x, nzj, lane);
+      next_w = (c.u + gridDim.x < p.units && lane < p.K) ? p.weights[(long long)nzj * p.K + lane] : 0.f;
+    }
     const unsigned mask = q_valid(p, my_idx);
-    if (mask == 0) continue;
-    __syncwarp();
-    sidx[lane] = my_idx;
-    __syncwarp();
-    const uint32_t un = ucnt++;
-    if (lane != 0 || !ok) continue;
     const QInfo t = q_info(p, c.inner);
     const int n = c.outer / p.J, j = c.outer - n * p.J;
-    {
-      const uint32_t ub = un & 1;
-      ok = mbar_wait_bounded(&bars[QDO_EMPTY + ub], ((un >> 1) & 1) ^ 1, abort_flag);
-      if (!ok) continue;
-      uint8_t* base = smem + OFF_QDO + ub * 2 * PAIR_BYTES;
-      mbar_arrive_expect_tx(&bars[QDO_FULL + ub], 2 * PAIR_BYTES);
-      tma_load_5d(base, &p.tm_q, &bars[QDO_FULL + ub], 0, 0, t.h0, j, n);
-      tma_load_5d(base + PAIR_BYTES, &p.tm_do, &bars[QDO_FULL + ub], 0, 0, t.h0, j, n);
+    const long long head_slot = ((long long)c.outer * p.Hq + t.h0) * p.K;                   // (row block, head A, slot 0)
+    const long long dq_off = n * p.dqs[0] + j * p.dqs[1] + t.h0 * p.dqs[2];
+    if (mask != full) {
+      for (int i = lane; i < (t.two ? 8 : 4) * p.K; i += 32) {                              // [head][slot][quarter]
+        const int x = i >> 2, k = x >= p.K ? x - p.K : x;
+        if (!((mask >> k) & 1)) p.dw_part[head_slot * 4 + i] = 0.f;
+      }
+      if (mask == 0) {
+        for (int i = lane; i < (t.two ? 128 : 64) * 8; i += 32) {
+          const int r = i >> 3;
+          reinterpret_cast<uint4*>(p.dq + dq_off + (r >> 6) * p.dqs[2] + (r & 63) * p.dqs[3])[i & 7] = make_uint4(0, 0, 0, 0);
+        }
+        continue;
+      }
     }
+    const bool valid = (mask >> lane) & 1u;
+    const int nv = __popc(mask), r = __popc(mask & ((1u << lane) - 1u));                    // the slot's number inside the unit
+    const uint32_t ub = un & 1;
     const CUtensorMap* tmk = t.share ? &p.tm_k1 : &p.tm_k2;
     const CUtensorMap* tmv = t.share ? &p.tm_v1 : &p.tm_v2;
     const uint32_t bytes = t.share ? TILE_BYTES : PAIR_BYTES;
-    for (unsigned m = mask; m; m &= m - 1) {
-      const int idx = sidx[__ffs(m) - 1];
-      ok = mbar_wait_bounded(&bars[K_EMPTY + rk.st], rk.ph ^ 1, abort_flag);
-      if (!ok) break;
-      mbar_arrive_expect_tx(&bars[K_FULL + rk.st], bytes);
-      tma_load_5d(smem + OFF_K + rk.st * PAIR_BYTES, tmk, &bars[K_FULL + rk.st], 0, 0, t.hk0, idx, n);
+    const uint32_t unit_flags = (t.two ? REC_TWO : 0u) | (t.share ? REC_SHARE : 0u);
+    SlotRec rec;
+    rec.flags = unit_flags | (r == 0 ? REC_FIRST : 0u) | (r == nv - 1 ? REC_LAST : 0u);
+    rec.w = my_w;
+    rec.row_off = (head_slot + lane) * 64;
+    if (!(ok = mbar_wait_warp(&bars[QDO_EMPTY + ub], ((un >> 1) & 1) ^ 1, abort_flag, lane))) break;
+    for (int i = 0; i < nv; ++i) {
+      const bool mine = valid && r == i;
+      if (!(ok = mbar_wait_warp(&bars[K_EMPTY + rk.st], rk.ph ^ 1, abort_flag, lane))) break;
+      if (mine) {
+        if (i == 0) {
+          UnitRec u;
+          u.flags = unit_flags; u.pad = 0; u.dq_off = dq_off;
+          urecs[un % NU] = u;
+          mbar_arrive(&bars[UREC_FULL + un % NU]);
+          uint8_t* base = smem + OFF_QDO + ub * 2 * PAIR_BYTES;
+          mbar_arrive_expect_tx(&bars[QDO_FULL + ub], 2 * PAIR_BYTES);
+          tma_load_5d(base, &p.tm_q, &bars[QDO_FULL + ub], 0, 0, t.h0, j, n);
+          tma_load_5d(base + PAIR_BYTES, &p.tm_do, &bars[QDO_FULL + ub], 0, 0, t.h0, j, n);
+        }
+        recs[rk.st] = rec;               // before the arrivals on K_FULL and V_FULL: the S and dP issuers read it behind those
+        mbar_arrive(&bars[REC_FULL + rk.st]);
+        mbar_arrive_expect_tx(&bars[K_FULL + rk.st], bytes);
+        tma_load_5d(smem + OFF_K + rk.st * PAIR_BYTES, tmk, &bars[K_FULL + rk.st], 0, 0, t.hk0, my_idx, n);
+      }
+      if (i == 0) ++q_issued;
+      ++k_issued;
+      if (!(ok = mbar_wait_warp(&bars[V_EMPTY + rv.st], rv.ph ^ 1, abort_flag, lane))) break;
+      if (mine) {
+        mbar_arrive_expect_tx(&bars[V_FULL + rv.st], bytes);
+        tma_load_5d(smem + OFF_V + rv.st * PAIR_BYTES, tmv, &bars[V_FULL + rv.st], 0, 0, t.hk0, my_idx, n);
+      }
+      __syncwarp();
+      ++v_issued;
       rk.next();
-      ok = mbar_wait_bounded(&bars[V_EMPTY + rv.st], rv.ph ^ 1, abort_flag);
-      if (!ok) break;
-      mbar_arrive_expect_tx(&bars[V_FULL + rv.st], bytes);
-      tma_load_5d(smem + OFF_V + rv.st * PAIR_BYTES, tmv, &bars[V_FULL + rv.st], 0, 0, t.hk0, idx, n);
       rv.next();
-      ++issued;
     }
+    ++un;
   }
-  if (lane == 0 && *abort_flag) {
-    drain(bars, K_FULL, issued, NKS);
-    drain(bars, V_FULL, issued, NVS);
-    drain(bars, QDO_FULL, ucnt, 2);
+  // end of work, in the next record of every group and of the writer (behind the waits for the stages: their last copies have landed)
+  for (int i = 0; i < NWG && ok; ++i) {
+    if (!(ok = mbar_wait_warp(&bars[K_EMPTY + rk.st], rk.ph ^ 1, abort_flag, lane))) break;
+    if (i == 0 && !(ok = mbar_wait_warp(&bars[V_EMPTY + rv.st], rv.ph ^ 1, abort_flag, lane))) break;
+    if (lane == 0) {
+      recs[rk.st].flags = REC_END | (i == 0 ? REC_FIRST : 0u);
+      mbar_arrive(&bars[REC_FULL + rk.st]);
+      if (i == 0) {
+        mbar_arrive(&bars[K_FULL + rk.st]);
+        mbar_arrive(&bars[V_FULL + rv.st]);
+      }
+    }
+    rk.next();
+  }
+  if (lane == 0) {
+    if (ok) {
+      urecs[un % NU].flags = REC_END;
+      mbar_arrive(&bars[UREC_FULL + un % NU]);
+    }
+    if (*abort_flag) {
+      drain(bars, K_FULL, k_issued, NKS);
+      drain(bars, V_FULL, v_issued, NVS);
+      drain(bars, QDO_FULL, q_issued, 2);
+    }
   }
 }
 
 // role 0: S per slot;  role 1: dP per slot;  role 2: dQ += dS K per slot.  All 32 lanes run this
 // code; elect.sync inside the MMA / commit wrappers picks the issuing lane.
 template <int ROLE>
-__device__ void q_issuer(const BwdQParams& p, uint8_t* smem, uint64_t* bars, volatile int* abort_flag, int lane,
-                         uint32_t tmem_base) {
+__device__ void q_issuer(uint8_t* smem, uint64_t* bars, volatile int* abort_flag, int lane, uint32_t tmem_base, long long* prof) {
   const uint64_t dQDO = umma_desc_sw128(smem_u32(smem + OFF_QDO));
   const uint64_t dK = umma_desc_sw128(smem_u32(smem + OFF_K)), dV = umma_desc_sw128(smem_u32(smem + OFF_V));
   const uint64_t dKmn = umma_desc_sw128_mn_blocks(smem_u32(smem + OFF_K), TILE_BYTES);
-  PairCursor c;
-  c.init(p.HP);
-  Ring ring; ring.init(ROLE == 1 ? NVS : NKS);
-  uint32_t ucnt = 0, g = 0;
-  uint32_t b = 0, bph = 0;                                // g % NBUF and the parity of g / NBUF
-  bool ok = true;
-  int next_idx = q_load_row(p, c.u, c.outer, lane);
-  for (; c.u < p.units && ok; c.advance()) {
-    const int my_idx = next_idx;
-    next_idx = q_load_row(p, c.u + gridDim.x, c.next_outer(), lane);
-    const unsigned mask = q_valid(p, my_idx);
-    if (mask == 0) continue;
-    const uint32_t un = ucnt++;
-    const int nv = __popc(mask);
-    const QInfo t = q_info(p, c.inner);
+  constexpr uint32_t FULL = ROLE == 0 ? K_FULL : ROLE == 1 ? V_FULL : PDS_FULL;
+  const SlotRec* recs = slot_recs(smem);
+  Ring rr, rv; rr.init(NKS); rv.init(NVS);                // record and K stage; V stage
+  Ring rg, rf; rg.init(NWG); rf.init(NWG);                // the slot's group (and dP region); the group of slot g - 3
+  uint32_t sreg = 0, un = 0, g = 0;                       // S region; unit
+  bool pre_a = false, pre_b = ROLE != 1;                  // early probe results for the coming slot, and its flags
+  uint32_t pre_flags = 0;
+  for (;; ++g) {
+    // role 0, 1: the tile has landed AND the region is free -- S: its group has read P, three slots ago; dP: dQ has consumed the
+    // dS in it, four slots ago; role 2: dS is written
+    const uint32_t st = ROLE == 0 ? rr.st : ROLE == 1 ? rv.st : rg.st, ph = ROLE == 0 ? rr.ph : ROLE == 1 ? rv.ph : rg.ph;
+    if (lane == 0 && ROLE == 0) GCA_TRACE_BUF(prof, 0, g);
+    if (!mbar_wait_warp2_probed(&bars[FULL + st], ph, pre_a, &bars[ROLE == 0 ? PDS_FULL + rf.st : DP_FREE + rg.st], ROLE == 0 ? rf.ph : rg.ph ^ 1,
+                                pre_b, abort_flag)) break;
+    if (ROLE == 0 && g >= NS) rf.next();
+    if (!pre_a) pre_flags = recs[rr.st].flags;
+    const uint32_t flags = __shfl_sync(0xffffffffu, pre_flags, 0);
+    if (flags & REC_END) break;
     const uint32_t ub = un & 1, uph = (un >> 1) & 1;
-    const uint32_t kt1 = t.share ? 0u : TILE16;            // head B's K / V tile inside the stage
-    if (ROLE != 2) ok = mbar_wait_warp(&bars[QDO_FULL + ub], uph, abort_flag, lane);
-    else ok = mbar_wait_warp(&bars[ACC_EMPTY + ub], uph ^ 1, abort_flag, lane);
-    bool pre_a = false, pre_b = false;           // early probe results for the coming slot
-    for (int i = 0; i < nv && ok; ++i, ++g) {
-      const uint32_t tbuf = tmem_base + b * BUF_COLS;
-      if (ROLE != 2) {
-        if (lane == 0 && ROLE == 0) GCA_TRACE_BUF(p.prof, 0, g);
-        // the tile has landed AND the buffer's previous contents (the packed dS of slot g - NBUF)
-        // have been consumed: both barriers are probed at once (one shared-memory round trip)
-        // (probed while the previous slot's MMAs were being issued, when there was one in this unit)
-        ok = mbar_wait_warp2_probed(&bars[(ROLE == 0 ? K_FULL : V_FULL) + ring.st], ring.ph, pre_a, &bars[BUF_FREE + b], bph ^ 1,
-                                    pre_b, abort_flag);
-        if (lane == 0 && ROLE == 0) GCA_TRACE_BUF(p.prof, 3, g);
-        if (!ok) break;
-        if (lane == 0 && ROLE == 0) GCA_TRACE_BUF(p.prof, 1, g);
-        tc_fence_after();
-        pre_a = pre_b = false;
-        if (GCA_Q_PREPROBE && i + 1 < nv) {              // the next slot's two barriers
-          const uint32_t nst = ring.st + 1 == (uint32_t)ring.depth ? 0u : ring.st + 1, nph = nst ? ring.ph : ring.ph ^ 1;
-          const uint32_t nb = b + 1 == NBUF ? 0u : b + 1, nbph = nb ? bph : bph ^ 1;
-          pre_a = mbar_test_wait(&bars[(ROLE == 0 ? K_FULL : V_FULL) + nst], nph);
-          pre_b = mbar_test_wait(&bars[BUF_FREE + nb], nbph ^ 1);
-        }
-        const uint64_t a = dQDO + ub * 2 * PAIR16 + (ROLE == 0 ? 0u : PAIR16);          // Q pair | dO pair
-        const uint64_t bt = (ROLE == 0 ? dK : dV) + ring.st * PAIR16;
-        const uint32_t d = tbuf + (ROLE == 0 ? 0u : COL_DPT);
-#pragma unroll
-        for (int tl = 0; tl < 2; ++tl) {
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            umma_bf16_ss_elect(d + (tl ? LANE16 : 0u), a + tl * TILE16 + kk * STEP_K, bt + (tl ? kt1 : 0u) + kk * STEP_K,
-                               IDESC_64, (uint32_t)(kk > 0));
-        }
-        umma_commit_elect(&bars[SP_FULL + b]);            // the barrier expects both the S and the dP commit
-        if (ROLE == 1) umma_commit_elect(&bars[V_EMPTY + ring.st]);
-        if (i == nv - 1) umma_commit_elect(&bars[QDO_EMPTY + ub]);    // expects both issuers' commits
-        if (lane == 0 && ROLE == 0) GCA_TRACE_BUF(p.prof, 2, g);
-      } else {
-        ok = mbar_wait_warp2_probed(&bars[PDS_FULL + b], bph, pre_a, &bars[PDS_FULL + b], bph, true, abort_flag);
-        if (!ok) break;
-        if (lane == 0) GCA_TRACE_BUF(p.prof, 5, g);
-        tc_fence_after();
-        pre_a = false;
-        if (GCA_Q_PREPROBE && i + 1 < nv) {
-          const uint32_t nb = b + 1 == NBUF ? 0u : b + 1, nbph = nb ? bph : bph ^ 1;
-          pre_a = mbar_test_wait(&bars[PDS_FULL + nb], nbph);
-        }
-        // dQ += dS K_k per head: A = dS from tensor memory (lane = query row, 8 columns per K step
-        // of 16 keys), B = the head's K tile read N-contiguous (MN-major)
-        const uint32_t acc = tmem_base + COL_DQ + ub * 64;
-        const uint64_t bk = dKmn + ring.st * PAIR16;
-#pragma unroll
-        for (int tl = 0; tl < 2; ++tl) {
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            umma_bf16_ts_elect(acc + (tl ? LANE16 : 0u), tbuf + COL_DPT + (tl ? LANE16 : 0u) + kk * 8,
-                               bk + (tl ? kt1 : 0u) + kk * STEP_MN, IDESC_DQ, (uint32_t)(i > 0 || kk > 0));
-        }
-        umma_commit_elect(&bars[BUF_FREE + b]);
-        umma_commit_elect(&bars[K_EMPTY + ring.st]);      // the K tiles of this slot are free once dQ is done
-        if (i == nv - 1) umma_commit_elect(&bars[ACC_FULL + ub]);     // written out by the last slot's worker group
-        if (lane == 0) GCA_TRACE_BUF(p.prof, 6, g);
-      }
-      ring.next();
-      if (++b == NBUF) { b = 0; bph ^= 1; }
+    const uint32_t kt1 = (flags & REC_SHARE) ? 0u : TILE16;            // head B's K / V tile inside the stage
+    if (flags & REC_FIRST) {
+      if (!mbar_wait_warp(&bars[ROLE != 2 ? QDO_FULL + ub : ACC_EMPTY], ROLE != 2 ? uph : ub ^ 1, abort_flag, lane)) break;
     }
+    if (lane == 0 && ROLE != 1) GCA_TRACE_BUF(prof, ROLE == 0 ? 3 : 5, g);
+    tc_fence_after();
+    // The next slot's barriers and flags, between the two heads' MMAs: the probes' round trip runs under the issue.
+    auto probe = [&] {
+      Ring nr = rr, nv = rv, ng = rg;
+      nr.next(); nv.next(); ng.next();
+      pre_a = mbar_test_wait(&bars[FULL + (ROLE == 0 ? nr.st : ROLE == 1 ? nv.st : ng.st)], ROLE == 0 ? nr.ph : ROLE == 1 ? nv.ph : ng.ph);
+      if (ROLE == 0) pre_b = g + 1 < NS || mbar_test_wait(&bars[PDS_FULL + rf.st], rf.ph);
+      if (ROLE == 1) pre_b = mbar_test_wait(&bars[DP_FREE + ng.st], ng.ph ^ 1);
+      if (pre_a) pre_flags = recs[nr.st].flags;
+    };
+    if (ROLE != 2) {
+      const uint64_t a = dQDO + ub * 2 * PAIR16 + (ROLE == 0 ? 0u : PAIR16);          // Q pair | dO pair
+      const uint64_t bt = (ROLE == 0 ? dK : dV) + st * PAIR16;
+      const uint32_t d = tmem_base + (ROLE == 0 ? sreg : COL_DP + rg.st * 64);
+#pragma unroll
+      for (int tl = 0; tl < 2; ++tl) {
+        if (tl == 1) probe();
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+          umma_bf16_ss_elect(d + (tl ? LANE16 : 0u), a + tl * TILE16 + kk * STEP_K, bt + (tl ? kt1 : 0u) + kk * STEP_K,
+                             IDESC_64, (uint32_t)(kk > 0));
+      }
+      umma_commit_elect(&bars[(ROLE == 0 ? S_FULL : DP_FULL) + rg.st]);
+      if (ROLE == 1) umma_commit_elect(&bars[V_EMPTY + st]);
+      if (flags & REC_LAST) umma_commit_elect(&bars[QDO_EMPTY + ub]);    // expects both issuers' commits
+      if (lane == 0 && ROLE == 0) GCA_TRACE_BUF(prof, 2, g);
+      if ((sreg += 64) == COL_DP) sreg = 0;
+    } else {
+      // dQ += dS K_k per head: A = dS from tensor memory (lane = query row, 8 columns per K step
+      // of 16 keys), B = the head's K tile read N-contiguous (MN-major)
+      const uint32_t acc = tmem_base + COL_DQ, at = tmem_base + COL_DP + rg.st * 64, first = flags & REC_FIRST;
+      const uint64_t bk = dKmn + rr.st * PAIR16;
+#pragma unroll
+      for (int tl = 0; tl < 2; ++tl) {
+        if (tl == 1) probe();
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+          umma_bf16_ts_elect(acc + (tl ? LANE16 : 0u), at + (tl ? LANE16 : 0u) + kk * 8,
+                             bk + (tl ? kt1 : 0u) + kk * STEP_MN, IDESC_DQ, (uint32_t)(kk > 0 || !first));
+      }
+      umma_commit_elect(&bars[DP_FREE + rg.st]);
+      umma_commit_elect(&bars[K_EMPTY + rr.st]);        // the K tiles of this slot are free once dQ is done
+      if (flags & REC_LAST) umma_commit_elect(&bars[ACC_FULL]);
+      if (lane == 0) GCA_TRACE_BUF(prof, 6, g);
+    }
+    if (flags & REC_LAST) ++un;
+    rr.next();
+    rv.next();
+    rg.next();
   }
 }
 
@@ -362,150 +410,108 @@ __device__ void q_worker(const BwdQParams& p, uint8_t* smem, uint64_t* bars, vol
   // TMEM lane of this thread = 32 quad + lane = (head tile, query row) as the 64-row MMAs lay them out
   const int tile = lane >> 4;
   const int row = quad * 16 + (lane & 15);
-  const uint32_t tlane = tmem_base + ((uint32_t)(quad * 32) << 16);
+  const uint32_t tlane = tmem_base + ((uint32_t)(quad * 32) << 16), td = tlane + COL_DP + wg * 64;
   const bool elected = quad == 0 && lane == 0;
-  const int tid = quad * 32 + lane;                             // 0..127 inside the worker group
-  PairCursor c;
-  c.init(p.HP);
-  uint32_t ucnt = 0, g = 0;
-  uint32_t b = 0, bph = 0;
-  bool ok = true;
-  int next_idx = q_load_row(p, c.u, c.outer, lane);
-  float next_w = (c.u < p.units && lane < p.K) ? p.weights[(long long)c.outer * p.K + lane] : 0.f;
+  const SlotRec* recs = slot_recs(smem);
   const float2 c2v = make_float2(p.c2, p.c2);
-  for (; c.u < p.units && ok; c.advance()) {
-    const int my_idx = next_idx;
-    const float my_w = next_w;
-    {
-      const int nzj = c.next_outer();
-      next_idx = q_load_row(p, c.u + gridDim.x, nzj, lane);
-      next_w = (c.u + gridDim.x < p.units && lane < p.K) ? p.weights[(long long)nzj * p.K + lane] : 0.f;
+  uint32_t st = wg, st_ph = 0, sreg = (wg % NS) * 64;             // g % 6 and the parity of g / 6; S region
+  for (uint32_t own = 0;; ++own) {                               // slot g = wg + 4 own
+    if (!mbar_wait_warp(&bars[REC_FULL + st], st_ph, abort_flag, lane)) break;
+    const uint32_t flags = recs[st].flags;
+    if (flags & REC_END) {
+      // The group of the first slot behind the last lets the dQ issuer see the end: when that has seen the group's last dS (it
+      // has consumed it), and the S issuer too (S of the last slot waited for it)
+      if (!(flags & REC_FIRST)) break;
+      const uint32_t last = wg + NWG * own - 1;
+      if (own > 0 && !mbar_wait_warp(&bars[DP_FREE + wg], (own - 1) & 1u, abort_flag, lane)) break;
+      if (last != ~0u && !mbar_wait_warp(&bars[S_FULL + last % NWG], (last / NWG) & 1u, abort_flag, lane)) break;
+      mbar_arrive(&bars[PDS_FULL + wg]);
+      break;
     }
-    const unsigned mask = q_valid(p, my_idx);
-    const QInfo t = q_info(p, c.inner);
-    const int h = t.h0 + tile;
-    const bool live = (tile == 0 || t.two) && h < p.Hq;
-    const int n = c.outer / p.J, j = c.outer - n * p.J;
-    __nv_bfloat16* dq_row = p.dq + n * p.dqs[0] + j * p.dqs[1] + h * p.dqs[2] + row * p.dqs[3];
-    float* dwp = p.dw_part + ((long long)c.outer * p.Hq + t.h0) * p.K * 4;     // [tile][k][quarter]
-    if (wg == 0) {
-      // padding slots (and whole units without valid slots): zero dw partials, zero dQ rows
-      const unsigned full = (p.K >= 32) ? 0xffffffffu : ((1u << p.K) - 1u);
-      if (mask != full)
-        for (int i = tid; i < 8 * p.K; i += 128) {
-          const int tl = i / (4 * p.K), k = (i - tl * 4 * p.K) >> 2;
-          if (!((mask >> k) & 1) && t.h0 + tl < p.Hq) dwp[i] = 0.f;
-        }
-      if (mask == 0 && live) {
-        const uint4 z = make_uint4(0, 0, 0, 0);
-#pragma unroll
-        for (int cc = 0; cc < 8; ++cc) reinterpret_cast<uint4*>(dq_row)[cc] = z;
-      }
-    }
-    if (mask == 0) continue;
-    const uint32_t un = ucnt++;
-    const long long row_off = ((long long)c.outer * p.Hq + (live ? h : t.h0)) * p.K * 64 + row;
-    const float* lse_base = p.lse + row_off;
-    uint4* rt_base = p.rowterm + row_off;
-    for (unsigned m = mask; m; m &= m - 1, ++g) {
-      const uint32_t bb = b, pp = bph;
-      if (++b == NBUF) { b = 0; bph ^= 1; }
-      if ((int)(g % NWG) != wg) continue;
-      const int k = __ffs(m) - 1;
-      const float w = __shfl_sync(0xffffffffu, my_w, k);
-      const float lse = lse_base[k * 64];
-      ok = mbar_wait_bounded(&bars[SP_FULL + bb], pp, abort_flag);
-      if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
-      if (elected) GCA_TRACE_BUF(p.prof, 7, g);
-      tc_fence_after();
-      const uint32_t tb = tlane + bb * BUF_COLS;
-      // Pass 1 over the row's 64 keys, 16 at a time (ONE small loop body: after its first pass it
-      // is in the instruction cache):  P = exp2(S c - LSE),  Di += P dP,  P -> packed bf16 over S
-      // columns that earlier passes have already read.
-      const float2 nl = make_float2(-lse, -lse);
-      float2 dacc = make_float2(0.f, 0.f);
+    const float w = recs[st].w;
+    const bool live = tile == 0 || (flags & REC_TWO);
+    const long long block = recs[st].row_off + (tile && live ? p.K * 64 : 0);     // (row block, head, slot, row 0)
+    const float lse = p.lse[block + row];
+    if ((st += NWG) >= NKS) { st -= NKS; st_ph ^= 1; }
+    if (!mbar_wait_warp2(&bars[S_FULL + wg], own & 1u, &bars[DP_FULL + wg], own & 1u, abort_flag, lane)) break;
+    const uint32_t ts = tlane + sreg;
+    if ((sreg += 64) == COL_DP) sreg = 0;                      // 4 slots on = one region on
+    if (elected) GCA_TRACE_BUF(p.prof, 7, own * 4 + wg);
+    tc_fence_after();
+    // Pass 1 over the row's 64 keys, 16 at a time (ONE small loop body: after its first pass it
+    // is in the instruction cache):  P = exp2(S c - LSE),  Di += P dP,  P -> packed bf16 over S
+    // columns that earlier passes have already read.
+    const float2 nl = make_float2(-lse, -lse);
+    float2 dacc = make_float2(0.f, 0.f);
 #pragma unroll 1
-      for (int cpos = 0; cpos < 64; cpos += CW) {
-        uint32_t s[CW], dp[CW];
-        tmem_ld_32x32b_x16(tb + cpos, s);
-        tmem_ld_32x32b_x16(tb + COL_DPT + cpos, dp);
-        tmem_ld_wait();
-        pass1_cols(s, dp, c2v, nl, dacc, tb + cpos / 2);
-      }
-      const float di = dacc.x + dacc.y;
-      tmem_st_wait();
-      if (elected) GCA_TRACE_BUF(p.prof, 8, g);
-      // Pass 2:  dS = P (w dP - w Di)  -> packed bf16 over the dP columns already read.  (Issuing the
-      // tensor-memory read of the next 16 columns before computing the current ones was measured
-      // slower, 0.603 against 0.562 ms; so was writing dS into two regions of its own, which frees
-      // the score buffer before the dQ product has run: 0.602 against 0.558 ms.)
-      const float2 wv = make_float2(w, w), nwd = make_float2(-w * di, -w * di);
-#pragma unroll 1
-      for (int cpos = 0; cpos < 64; cpos += CW) {
-        uint32_t pk[CW / 2], dp[CW];
-        tmem_ld_32x32b_x8(tb + cpos / 2, pk);
-        tmem_ld_32x32b_x16(tb + COL_DPT + cpos, dp);
-        tmem_ld_wait();
-        pass2_cols(pk, dp, wv, nwd, tb + COL_DPT + cpos / 2);
-      }
-      tmem_st_wait();
-      tc_fence_before();
-      mbar_arrive(&bars[PDS_FULL + bb]);
-      if (elected) GCA_TRACE_BUF(p.prof, 9, g);
-      if (live) rt_base[k * 64] = row_terms((log2_abs_clamped(w) - lse) * p.inv_c2, -di);
-      // dw: sum of Di over the 16 rows this warp holds of each head's tile -> one partial per
-      // (head, 16-row quarter)
-      float dsum = di;
-#pragma unroll
-      for (int of = 8; of > 0; of >>= 1) dsum += __shfl_xor_sync(0xffffffffu, dsum, of);
-      if ((lane & 15) == 0 && live) dwp[(tile * p.K + k) * 4 + quad] = dsum;
+    for (int cpos = 0; cpos < 64; cpos += CW) {
+      uint32_t s[CW], dp[CW];
+      tmem_ld_32x32b_x16(ts + cpos, s);
+      tmem_ld_32x32b_x16(td + cpos, dp);
+      tmem_ld_wait();
+      pass1_cols(s, dp, c2v, nl, dacc, ts + cpos / 2);
     }
-    if (!ok) break;
+    const float di = dacc.x + dacc.y;
+    tmem_st_wait();
+    if (elected) GCA_TRACE_BUF(p.prof, 8, own * 4 + wg);
+    // Pass 2:  dS = P (w dP - w Di)  -> packed bf16 over the dP columns already read.  (Issuing the
+    // tensor-memory read of the next 16 columns before computing the current ones was measured
+    // slower, 0.603 against 0.562 ms.)
+    const float2 wv = make_float2(w, w), nwd = make_float2(-w * di, -w * di);
+#pragma unroll 1
+    for (int cpos = 0; cpos < 64; cpos += CW) {
+      uint32_t pk[CW / 2], dp[CW];
+      tmem_ld_32x32b_x8(ts + cpos / 2, pk);
+      tmem_ld_32x32b_x16(td + cpos, dp);
+      tmem_ld_wait();
+      pass2_cols(pk, dp, wv, nwd, td + cpos / 2);
+    }
+    tmem_st_wait();
+    tc_fence_before();
+    mbar_arrive(&bars[PDS_FULL + wg]);
+    if (elected) GCA_TRACE_BUF(p.prof, 9, own * 4 + wg);
+    if (live) p.rowterm[block + row] = row_terms((log2_abs_clamped(w) - lse) * p.inv_c2, -di);
+    // dw: sum of Di over the 16 rows this warp holds of each head's tile -> one partial per
+    // (head, 16-row quarter)
+    float dsum = di;
+#pragma unroll
+    for (int of = 8; of > 0; of >>= 1) dsum += __shfl_xor_sync(0xffffffffu, dsum, of);
+    if ((lane & 15) == 0 && live) p.dw_part[block / 16 + quad] = dsum;
   }
 }
 
 // The dQ writer: a warpgroup of its own, so that no worker group is held up by a unit's output (a
-// worker group is tied to every NBUF-th slot; while it waited for the unit's last dQ product and
+// worker group is tied to every fourth slot; while it waited for the unit's last dQ product and
 // stored the tile, ~2,000-2,800 cycles, its next slot and with it the whole ring stood still once
 // per unit: 0.571 -> 0.544 ms).  Its wait is the ordinary suspending try_wait: polling with a sleep
 // between probes (20 / 100 / 400 ns) was measured slower (0.584 / 0.574 / 0.558 ms).  Thread = TMEM
 // lane = (head tile, query row) as in the workers.
-__device__ void q_writer(const BwdQParams& p, uint64_t* bars, volatile int* abort_flag, int quad, int lane, uint32_t tmem_base) {
+__device__ void q_writer(const BwdQParams& p, uint8_t* smem, uint64_t* bars, volatile int* abort_flag, int quad, int lane, uint32_t tmem_base) {
   const int tile = lane >> 4;
   const int row = quad * 16 + (lane & 15);
   const uint32_t tlane = tmem_base + ((uint32_t)(quad * 32) << 16);
   const bool elected = quad == 0 && lane == 0;
-  PairCursor c;
-  c.init(p.HP);
-  uint32_t ucnt = 0;
-  bool ok = true;
-  int next_idx = q_load_row(p, c.u, c.outer, lane);
-  for (; c.u < p.units && ok; c.advance()) {
-    const int my_idx = next_idx;
-    next_idx = q_load_row(p, c.u + gridDim.x, c.next_outer(), lane);
-    if (q_valid(p, my_idx) == 0) continue;           // the workers zero-fill units without valid slots
-    const uint32_t un = ucnt++;
-    const uint32_t ub = un & 1;
-    const QInfo t = q_info(p, c.inner);
-    const int h = t.h0 + tile;
-    const bool live = (tile == 0 || t.two) && h < p.Hq;
-    const int n = c.outer / p.J, j = c.outer - n * p.J;
-    __nv_bfloat16* dq_row = p.dq + n * p.dqs[0] + j * p.dqs[1] + h * p.dqs[2] + row * p.dqs[3];
-    ok = mbar_wait_bounded(&bars[ACC_FULL + ub], (un >> 1) & 1, abort_flag);
-    if (!__all_sync(0xffffffffu, ok)) break;
+  const UnitRec* urecs = unit_recs(smem);
+  __nv_bfloat16* const dq_t = p.dq + tile * p.dqs[2] + row * p.dqs[3];
+  for (uint32_t un = 0;; ++un) {
+    if (!mbar_wait_warp(&bars[UREC_FULL + un % NU], (un / NU) & 1, abort_flag, lane)) break;
+    const uint32_t flags = urecs[un % NU].flags;
+    if (flags & REC_END) break;
+    const bool live = tile == 0 || (flags & REC_TWO);
+    __nv_bfloat16* dq_row = dq_t + urecs[un % NU].dq_off;
+    if (!mbar_wait_warp(&bars[ACC_FULL], un & 1, abort_flag, lane)) break;
     if (elected) GCA_TRACE_BUF(p.prof, 10, un);
     tc_fence_after();
-    // dQ leaves in four passes of one small loop body (16 columns: TMEM -> bf16 -> one 32-byte
-    // store per row)
-#pragma unroll 1
-    for (int part = 0; part < OUT_PASSES; ++part) {
-      uint32_t v[OUT_COLS];
-      tmem_ld_32x32b_x16(tlane + COL_DQ + ub * 64 + part * OUT_COLS, v);
-      tmem_ld_wait();
-      if (live) store16_bf16(reinterpret_cast<uint8_t*>(dq_row) + part * OUT_COLS * 2, v, p.sm_scale, p.wide_store);
-    }
+    // the whole row into registers, so that the accumulator is free again at once
+    uint32_t v[64];
+    tmem_ld_32x32b_x32(tlane + COL_DQ, v);
+    tmem_ld_32x32b_x32(tlane + COL_DQ + 32, v + 32);
+    tmem_ld_wait();
     tc_fence_before();
-    mbar_arrive(&bars[ACC_EMPTY + ub]);
+    mbar_arrive_warp(&bars[ACC_EMPTY], lane);
+#pragma unroll
+    for (int part = 0; part < OUT_PASSES; ++part)
+      if (live) store16_bf16(reinterpret_cast<uint8_t*>(dq_row) + part * OUT_COLS * 2, v + part * OUT_COLS, p.sm_scale, p.wide_store);
     if (elected) GCA_TRACE_BUF(p.prof, 11, un);
   }
 }
@@ -522,15 +528,14 @@ bwd_q_tc_kernel(const __grid_constant__ BwdQParams p) {
     for (int i = 0; i < 2; ++i) {
       mbar_init(&bars[QDO_FULL + i], 1);
       mbar_init(&bars[QDO_EMPTY + i], 2);                  // S issuers + dP issuers
-      mbar_init(&bars[ACC_FULL + i], 1);
-      mbar_init(&bars[ACC_EMPTY + i], 128);
     }
-    for (int i = 0; i < NBUF; ++i) {
-      mbar_init(&bars[SP_FULL + i], 2);                    // S commits + dP commits
-      mbar_init(&bars[PDS_FULL + i], 128);
-      mbar_init(&bars[BUF_FREE + i], 1);
+    mbar_init(&bars[ACC_FULL], 1);
+    mbar_init(&bars[ACC_EMPTY], 4);
+    for (int i = 0; i < NWG; ++i) {
+      mbar_init(&bars[S_FULL + i], 1); mbar_init(&bars[DP_FULL + i], 1); mbar_init(&bars[PDS_FULL + i], 128); mbar_init(&bars[DP_FREE + i], 1);
     }
-    for (int i = 0; i < NKS; ++i) { mbar_init(&bars[K_FULL + i], 1); mbar_init(&bars[K_EMPTY + i], 1); }
+    for (int i = 0; i < NKS; ++i) { mbar_init(&bars[K_FULL + i], 1); mbar_init(&bars[K_EMPTY + i], 1); mbar_init(&bars[REC_FULL + i], 1); }
+    for (int i = 0; i < NU; ++i) mbar_init(&bars[UREC_FULL + i], 1);
     for (int i = 0; i < NVS; ++i) { mbar_init(&bars[V_FULL + i], 1); mbar_init(&bars[V_EMPTY + i], 1); }
     *abort_flag = 0;
     fence_barrier_init();
@@ -547,10 +552,10 @@ bwd_q_tc_kernel(const __grid_constant__ BwdQParams p) {
   if (!p.beside_index) pdl_wait();
   if (warp < 4 * NWG) q_worker(p, smem, bars, abort_flag, warp >> 2, warp & 3, lane, tmem_base);
   else if (warp == PROD_WARP) q_producer(p, smem, bars, abort_flag, lane);
-  else if (warp >= WRITER_WARP) q_writer(p, bars, abort_flag, warp & 3, lane, tmem_base);
-  else if (warp == ISSUE_S) q_issuer<0>(p, smem, bars, abort_flag, lane, tmem_base);
-  else if (warp == ISSUE_DP) q_issuer<1>(p, smem, bars, abort_flag, lane, tmem_base);
-  else if (warp == ISSUE_DQ) q_issuer<2>(p, smem, bars, abort_flag, lane, tmem_base);
+  else if (warp >= WRITER_WARP) q_writer(p, smem, bars, abort_flag, warp & 3, lane, tmem_base);
+  else if (warp == ISSUE_S) q_issuer<0>(smem, bars, abort_flag, lane, tmem_base, p.prof);
+  else if (warp == ISSUE_DP) q_issuer<1>(smem, bars, abort_flag, lane, tmem_base, p.prof);
+  else if (warp == ISSUE_DQ) q_issuer<2>(smem, bars, abort_flag, lane, tmem_base, p.prof);
   if (p.beside_index) pdl_wait();        // the index is complete before this kernel is
   tc_fence_before();
   __syncthreads();

@@ -114,6 +114,28 @@ def test_odd_head_count_many_units(lcm, h):
     assert lcm.read_status() == 0
 
 
+@pytest.mark.parametrize("h,hkv", [(5, 5), (4, 2)])
+@pytest.mark.parametrize("k", [1, 2, 3, 4, 5, 7, 9, 13])
+def test_few_slots_per_cta(lcm, k, h, hkv):
+    """Fewer units than SMs: a CTA sees 0 to k slots in all (row blocks without a valid slot, with one, with some, with all), so the hand-over of
+    its last slots comes right behind its first ones; the four worker groups, three score regions and six tile stages meet every remainder."""
+    n, c = 2, 14
+    g = torch.Generator().manual_seed(k * 10 + h)
+    q, dout = (torch.randn(n, c, h, 64, 64, generator=g).bfloat16() for _ in range(2))
+    kc, vc = (torch.randn(n, c, 64, hkv * 64, generator=g).bfloat16() for _ in range(2))
+    idx = torch.stack([torch.stack([torch.randperm(c, generator=g)[:k] for _ in range(c)]) for _ in range(n)]).int()
+    for j in range(c):                       # the first, the last or scattered slots are padding; row blocks 0 and 7 have none
+        idx[0, j, j % (k + 1):] = -1
+        idx[1, j, torch.rand(k, generator=g) < 0.4] = -1
+    idx[:, 7] = -1
+    w = torch.rand(n, c, k, generator=g).masked_fill(idx < 0, 0.0)
+    got = run(lcm, q, kc, vc, idx, w, dout)
+    ref = G.gca_indexed_grads(q.float(), kc.float(), vc.float(), idx, w, 0.125, dout.float())
+    for name, g_, r_ in zip(NAMES, got, ref):
+        check(name, g_.reshape(r_.shape), r_, 2e-2)
+    assert lcm.read_status() == 0
+
+
 @pytest.mark.parametrize("true_off_by_one", [False, True])
 def test_cpu_reference_config_fp32(lcm, true_off_by_one):
     """The CPU-runnable configuration exactly: B = 2, H = 12, 64 chunks of 64 tokens (L = 4096),
