@@ -158,6 +158,7 @@ struct BwdQParams {
   long long dqs[4];
   int units;
   int N, J, Hq, Hkv, G, K, C, HP;
+  bool late_first;           // order of the units, see row_block_at
   int wide_store;           // dq rows are 32-byte aligned: 256-bit stores
   float c2, sm_scale;
 };
@@ -193,20 +194,19 @@ __device__ void q_producer(const BwdQParams& p, uint8_t* smem, uint64_t* bars, v
   uint32_t un = 0, k_issued = 0, v_issued = 0, q_issued = 0;
   bool ok = true;
   const unsigned full = (p.K >= 32) ? 0xffffffffu : ((1u << p.K) - 1u);
-  int next_idx = q_load_row(p, c.u, c.outer, lane);
-  float next_w = (c.u < p.units && lane < p.K) ? p.weights[(long long)c.outer * p.K + lane] : 0.f;
+  int next_zj = row_block_at(c.outer, p.N, p.J, p.late_first);
+  int next_idx = q_load_row(p, c.u, next_zj, lane);
+  float next_w = (c.u < p.units && lane < p.K) ? p.weights[(long long)next_zj * p.K + lane] : 0.f;
   for (; c.u < p.units && ok; c.advance()) {
-    const int my_idx = next_idx;
+    const int zj = next_zj, my_idx = next_idx;
     const float my_w = next_w;
-    {
-      const int nzj = c.next_outer();
-      next_idx = q_load_row(p, c.u + gridDim.x, nzj, lane);
-      next_w = (c.u + gridDim.x < p.units && lane < p.K) ? p.weights[(long long)nzj * p.K + lane] : 0.f;
-    }
+    next_zj = row_block_at(c.next_outer(), p.N, p.J, p.late_first);
+    next_idx = q_load_row(p, c.u + gridDim.x, next_zj, lane);
+    next_w = (c.u + gridDim.x < p.units && lane < p.K) ? p.weights[(long long)next_zj * p.K + lane] : 0.f;
     const unsigned mask = q_valid(p, my_idx);
     const QInfo t = q_info(p, c.inner);
-    const int n = c.outer / p.J, j = c.outer - n * p.J;
-    const long long head_slot = ((long long)c.outer * p.Hq + t.h0) * p.K;                   // (row block, head A, slot 0)
+    const int n = zj / p.J, j = zj - n * p.J;
+    const long long head_slot = ((long long)zj * p.Hq + t.h0) * p.K;                   // (row block, head A, slot 0)
     const long long dq_off = n * p.dqs[0] + j * p.dqs[1] + t.h0 * p.dqs[2];
     if (mask != full) {
       for (int i = lane; i < (t.two ? 8 : 4) * p.K; i += 32) {                              // [head][slot][quarter]
@@ -601,6 +601,7 @@ int launch_bwd_q_tc(const GcaBwdArgs& a, float* dw_part, uint4* rowterm, const C
   const long long units = (long long)a.N * a.J * p.HP;
   if (units >= (1ll << 31) - 65536) return GCA_ERR_TOO_LARGE;
   p.units = (int)units;
+  p.late_first = late_chunks_first(a);
   p.c2 = c2; p.sm_scale = a.sm_scale;
   p.wide_store = rows_32b_aligned(a.dq, a.dq_stride);
   if (p.units == 0) return 0;

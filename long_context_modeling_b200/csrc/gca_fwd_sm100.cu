@@ -30,13 +30,14 @@
 // next barriers probed in the middle of a slot (398 us: what counts is how many barrier operations there are, not where their
 // latency falls), probes by one elected lane (+9 %), a fourth softmax group (+28 %, with registers moved to it from the other warps).
 // Ring stages are released by tcgen05.commit straight onto the producers' barriers.  CTAs are persistent and
-// walk the units in (n, j, head pair) order so that concurrently running CTAs touch the cache
+// walk the units in an order (late_chunks_first) in which concurrently running CTAs touch the cache
 // of few sequences (L2 reuse of chunks retrieved many times).  Every mbarrier wait is bounded;
 // on expiry the CTA flags GCA_STATUS_TIMEOUT, drains its copies and unwinds.
 #include <cstdlib>
 
 #include "gca_common.cuh"
 #include "sm100_ptx.cuh"
+#include "tc_common.cuh"
 #include "tma_host.cuh"
 
 namespace gca {
@@ -112,6 +113,7 @@ struct FwdTcParams {
   long long os[4];
   int units;
   int N, J, Hq, Hkv, G, K, C, HP;
+  bool late_first;           // order of the units, see row_block_at
   int pair;                 // 1: a unit is a pair of q heads; 0: a single head (GCA_ALGO_TC_UNPAIRED)
   int dbg;                  // profile builds only: bit mask of work to skip (timing experiments)
   int wide_store;           // every output row is 32-byte aligned: 256-bit stores
@@ -134,20 +136,6 @@ struct FwdTcParams {
 #define GCA_DBG(bit) 0
 #endif
 
-// Incremental walk over this CTA's units u = blockIdx.x, +gridDim.x, ...: unit u is
-// (zj, hp) = (u / HP, u % HP); no division after the first step.
-struct UnitCursor {
-  int u, zj, hp, dzj, dhp;
-  __device__ __forceinline__ void init(const FwdTcParams& p) {
-    u = blockIdx.x; zj = u / p.HP; hp = u - zj * p.HP;
-    dzj = gridDim.x / p.HP; dhp = gridDim.x - dzj * p.HP;
-  }
-  __device__ __forceinline__ void advance(const FwdTcParams& p) {
-    u += gridDim.x; zj += dzj; hp += dhp;
-    if (hp >= p.HP) { hp -= p.HP; ++zj; }
-  }
-  __device__ __forceinline__ int next_zj(const FwdTcParams& p) const { return zj + dzj + ((hp + dhp >= p.HP) ? 1 : 0); }
-};
 struct UnitInfo { int h0, hk0; bool two, share; };
 __device__ __forceinline__ UnitInfo unit_info(const FwdTcParams& p, int hp) {
   UnitInfo t;
@@ -165,14 +153,6 @@ __device__ __forceinline__ int load_index_row(const FwdTcParams& p, int u, int z
 __device__ __forceinline__ unsigned valid_mask(const FwdTcParams& p, int idx) {
   return __ballot_sync(0xffffffffu, idx >= 0 && idx < p.C);
 }
-
-// Running slot counters of a ring / double buffer (no div or mod in the slot loops).
-struct Ring {
-  uint32_t st, ph;
-  int depth;
-  __device__ __forceinline__ void init(int d) { st = 0; ph = 0; depth = d; }
-  __device__ __forceinline__ void next() { if (++st == (uint32_t)depth) { st = 0; ph ^= 1; } }
-};
 
 __device__ __forceinline__ SlotRec* slot_recs(uint8_t* smem) { return reinterpret_cast<SlotRec*>(smem + OFF_REC); }
 
@@ -193,27 +173,26 @@ __device__ __forceinline__ void drain_ring(uint64_t* bars, int full0, uint32_t i
 // valid slots, zero lse of padding slots, the bad-index status bit.
 __device__ void kproducer_role(const FwdTcParams& p, uint8_t* smem, uint64_t* bars, volatile int* abort_flag, int lane) {
   SlotRec* recs = slot_recs(smem);
-  UnitCursor c;
-  c.init(p);
+  PairCursor c;
+  c.init(p.HP);
   Ring ring; ring.init(NK);
   Ring rr; rr.init(NR);
   uint32_t un = 0, issued = 0, q_issued = 0;
   bool ok = true;
   const unsigned full = (p.K >= 32) ? 0xffffffffu : ((1u << p.K) - 1u);
-  int next_idx = load_index_row(p, c.u, c.zj, lane);
-  float next_w = (c.u < p.units && lane < p.K) ? p.weights[(long long)c.zj * p.K + lane] : 0.f;
-  for (; c.u < p.units && ok; c.advance(p)) {
-    const int my_idx = next_idx;
+  int next_zj = row_block_at(c.outer, p.N, p.J, p.late_first);
+  int next_idx = load_index_row(p, c.u, next_zj, lane);
+  float next_w = (c.u < p.units && lane < p.K) ? p.weights[(long long)next_zj * p.K + lane] : 0.f;
+  for (; c.u < p.units && ok; c.advance()) {
+    const int zj = next_zj, my_idx = next_idx;
     const float my_w = next_w;
-    {
-      const int nzj = c.next_zj(p);
-      next_idx = load_index_row(p, c.u + gridDim.x, nzj, lane);
-      next_w = (c.u + gridDim.x < p.units && lane < p.K) ? p.weights[(long long)nzj * p.K + lane] : 0.f;
-    }
+    next_zj = row_block_at(c.next_outer(), p.N, p.J, p.late_first);
+    next_idx = load_index_row(p, c.u + gridDim.x, next_zj, lane);
+    next_w = (c.u + gridDim.x < p.units && lane < p.K) ? p.weights[(long long)next_zj * p.K + lane] : 0.f;
     const unsigned mask = valid_mask(p, my_idx);
-    const UnitInfo t = unit_info(p, c.hp);
-    const int n = c.zj / p.J, j = c.zj - n * p.J;
-    const long long lse_off = ((long long)c.zj * p.Hq + t.h0) * p.K * 64;
+    const UnitInfo t = unit_info(p, c.inner);
+    const int n = zj / p.J, j = zj - n * p.J;
+    const long long lse_off = ((long long)zj * p.Hq + t.h0) * p.K * 64;
     const long long out_off = n * p.os[0] + j * p.os[1] + t.h0 * p.os[2];
     if (__any_sync(0xffffffffu, my_idx >= p.C) && p.status && lane == 0) atomicOr(p.status, GCA_STATUS_BAD_INDEX);
     if (mask != full) {
@@ -376,12 +355,6 @@ __device__ void issuer_role(const FwdTcParams& p, uint8_t* smem, uint64_t* bars,
 }
 
 // ----------------------------------------------------------------------------- softmax + epilogue
-__device__ __forceinline__ float fmax3(float a, float b, float c) {
-  float r;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-  return r;
-}
-
 __device__ void softmax_role(const FwdTcParams& p, uint8_t* smem, uint64_t* bars, volatile int* abort_flag, int wg,
                              int quad, int lane, uint32_t tmem_base) {
   // lane 32 quad + lane of tensor memory = (head, query row) as the 64-row MMAs lay them out
@@ -595,6 +568,7 @@ int launch_fwd_tc(const GcaFwdArgs& a, int sms, cudaStream_t stream) {
   p.indices = a.indices; p.weights = a.weights; p.out = (__nv_bfloat16*)a.out; p.lse = a.lse; p.status = a.status;
   for (int i = 0; i < 4; ++i) p.os[i] = a.o_stride[i];
   p.N = a.N; p.J = a.J; p.Hq = a.Hq; p.Hkv = a.Hkv; p.G = a.Hq / a.Hkv; p.K = a.K; p.C = a.C;
+  p.late_first = late_chunks_first(a);
   p.pair = a.algo == GCA_ALGO_TC_UNPAIRED ? 0 : 1;
   p.dbg = 0;
 #ifdef GCA_DBGKNOBS

@@ -24,6 +24,14 @@ struct PairCursor {
   __device__ __forceinline__ int next_outer() const { return outer + douter + ((inner + dinner >= modulus) ? 1 : 0); }
 };
 
+// The row block (n, j) at place v of the order in which the forward and the q-major pass take them.  `late_first`: the query chunks of all
+// sequences side by side, the last first (see late_chunks_first); else sequence by sequence.
+__device__ __forceinline__ int row_block_at(int v, int N, int J, bool late_first) {
+  if (!late_first) return v;
+  const int x = v / N;
+  return (v - x * N) * J + J - 1 - x;
+}
+
 // Running stage / phase of a ring of `depth` buffers (no div or mod in the hot loops).
 struct Ring {
   uint32_t st, ph;
