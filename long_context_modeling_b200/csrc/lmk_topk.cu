@@ -100,6 +100,14 @@ __device__ __forceinline__ void select_batch(unsigned long long& mine, unsigned 
 // merge).
 constexpr int BATCH = 64, STREAM_WARPS = 16;
 template <int NP> constexpr int RING_ROWS = NP > 3 ? 6 : 8;       // 196 KB per SM
+template <int NP> constexpr int ROWS_AT_ONCE = NP > 3 ? 2 : 4;    // of a warp
+
+// One step of the butterfly over the lanes for two rows at a time: lanes whose bit `of` is clear go on with the sum of row a, the others with
+// that of row b.  The same sums as a step for each (a sum of two does not depend on their order) for half the shuffles.
+__device__ __forceinline__ float fold_rows(float a, float b, int of, int lane) {
+  const bool up = lane & of;
+  return (up ? b : a) + __shfl_xor_sync(0xffffffffu, up ? a : b, of);
+}
 
 // The K best of up to 32 descending lists, lane l at the head of list l: K times the best head, found by a warp-wide maximum, moves on.
 // `at(i)`: this lane's list's entry i (0 past the end of a short list); lanes without a list pass has = false.
@@ -128,7 +136,7 @@ __device__ __forceinline__ unsigned long long ld_dsmem_u64(const unsigned long l
 template <int NP, bool PER_HEAD, bool FUSED>
 __global__ void __launch_bounds__(STREAM_WARPS * 32, 1)
 lmk_stream_kernel(ScanParams p, FinalParams fin) {
-  constexpr int RING = RING_ROWS<NP>, NL = PER_HEAD ? NP * 4 : 1, MINE = (NL + STREAM_WARPS - 1) / STREAM_WARPS, ROW_BYTES = NP * 512;
+  constexpr int RING = RING_ROWS<NP>, U = ROWS_AT_ONCE<NP>, NL = PER_HEAD ? NP * 4 : 1, MINE = (NL + STREAM_WARPS - 1) / STREAM_WARPS, ROW_BYTES = NP * 512;
   extern __shared__ __align__(16) unsigned char ring_all[];            // [STREAM_WARPS][RING][ROW_BYTES]
   __shared__ float score[2][NL][BATCH];
   pdl_trigger();
@@ -141,24 +149,27 @@ lmk_stream_kernel(ScanParams p, FinalParams fin) {
   const long long seen = p.q_pos0 + t0 - p.e_base;
   const int e_hi = (int)max((long long)e_lo, min((long long)min(p.E, e_lo + p.e_per_split), seen));
   const __nv_bfloat16* kb = p.lk + n * p.kbs + lane * 8;
-  // this warp's i-th row is e_lo + 16 i + warp
-  auto fetch = [&](int i) {
-    const int e = e_lo + i * STREAM_WARPS + warp;
-    if (e < e_hi) {
-      const __nv_bfloat16* src = kb + (long long)e * p.krs;
-      const unsigned dst = (unsigned)__cvta_generic_to_shared(ring + (i % RING) * ROW_BYTES);
+  // this warp's i-th row is e_lo + 16 i + warp; rows are asked for in order, U at a time
+  const __nv_bfloat16* next_src = kb + (long long)(e_lo + warp) * p.krs;
+  const long long src_step = p.krs * STREAM_WARPS;
+  int next_e = e_lo + warp;
+  auto fetch = [&](int slot) {                                // into the ring's places slot .. slot + U - 1
+    const unsigned dst = (unsigned)__cvta_generic_to_shared(ring + slot * ROW_BYTES);
 #pragma unroll
-      for (int pp = 0; pp < NP; ++pp)
-        if (lane + 32 * pp < pieces) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + pp * 512), "l"(src + pp * 256) : "memory");
+    for (int u = 0; u < U; ++u) {
+      if (next_e < e_hi)
+#pragma unroll
+        for (int pp = 0; pp < NP; ++pp)
+          if (lane + 32 * pp < pieces)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + u * ROW_BYTES + pp * 512), "l"(next_src + pp * 256) : "memory");
+      next_e += STREAM_WARPS;
+      next_src += src_step;
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
   };
   pdl_wait();
 #pragma unroll
-  for (int i = 0; i < RING; i += 2) {
-    fetch(i);
-    fetch(i + 1);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  }
+  for (int i = 0; i < RING; i += U) fetch(i);
   float qf[NP][8];
 #pragma unroll
   for (int pp = 0; pp < NP; ++pp) {
@@ -172,47 +183,52 @@ lmk_stream_kernel(ScanParams p, FinalParams fin) {
   for (int x = 0; x < MINE; ++x) mine[x] = kth[x] = 0ull;
 
   const int batches = (e_hi - e_lo + BATCH - 1) / BATCH;
+  int slot = 0;
   for (int b = 0; b < batches; ++b) {
     float (*sc)[BATCH] = score[b & 1];
-#pragma unroll 2
-    for (int i = 0; i < BATCH / STREAM_WARPS; i += 2) {
-      asm volatile("cp.async.wait_group %0;" ::"n"(RING / 2 - 1) : "memory");       // a lane reads only what it copied itself
-      const int i0 = b * (BATCH / STREAM_WARPS) + i;
-      uint4 kv[2][NP];
 #pragma unroll
-      for (int u = 0; u < 2; ++u)
+    for (int i = 0; i < BATCH / STREAM_WARPS; i += U) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(RING / U - 1) : "memory");       // a lane reads only what it copied itself
+      constexpr int X = PER_HEAD ? NP : 1;
+      float2 acc[U / 2][X];                                  // of two rows
 #pragma unroll
-        for (int pp = 0; pp < NP; ++pp)
-          kv[u][pp] = lane + 32 * pp < pieces ? *reinterpret_cast<const uint4*>(ring + ((i0 + u) % RING) * ROW_BYTES + pp * 512) : make_uint4(0, 0, 0, 0);
-      float acc[2][PER_HEAD ? NP : 1];
+      for (int u = 0; u < U; u += 2) {
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-#pragma unroll
-        for (int x = 0; x < (PER_HEAD ? NP : 1); ++x) acc[u][x] = 0.f;
+        for (int x = 0; x < X; ++x) acc[u / 2][x] = make_float2(0.f, 0.f);
 #pragma unroll
         for (int pp = 0; pp < NP; ++pp) {                    // absent pieces add 0 * 0: the sums never are -0
-          float kf[8];
-          unpack8(kv[u][pp], kf);
+          const unsigned char* at = ring + (slot + u) * ROW_BYTES + pp * 512;
+          const bool there = lane + 32 * pp < pieces;
+          float k0[8], k1[8];
+          unpack8(there ? *reinterpret_cast<const uint4*>(at) : make_uint4(0, 0, 0, 0), k0);
+          unpack8(there ? *reinterpret_cast<const uint4*>(at + ROW_BYTES) : make_uint4(0, 0, 0, 0), k1);
+          float2& s = acc[u / 2][PER_HEAD ? pp : 0];
 #pragma unroll
-          for (int jj = 0; jj < 8; ++jj) acc[u][PER_HEAD ? pp : 0] = fmaf(qf[pp][jj], kf[jj], acc[u][PER_HEAD ? pp : 0]);
+          for (int jj = 0; jj < 8; ++jj) s = __ffma2_rn(make_float2(qf[pp][jj], qf[pp][jj]), make_float2(k0[jj], k1[jj]), s);
         }
       }
-      fetch(i0 + RING);
-      fetch(i0 + RING + 1);
-      asm volatile("cp.async.commit_group;" ::: "memory");
+      fetch(slot);
+      if ((slot += U) == RING) slot = 0;
+      constexpr int TOP = PER_HEAD ? 4 : 16;                 // the butterfly starts at this distance
+      float sum[X];
+      int row = 0;                                           // of the U: the one whose score this lane ends up with
 #pragma unroll
-      for (int of = PER_HEAD ? 4 : 16; of > 0; of >>= 1)
+      for (int x = 0; x < X; ++x) {
+        if (U == 4) {
+          const float s0 = fold_rows(acc[0][x].x, acc[U / 2 - 1][x].x, TOP, lane), s1 = fold_rows(acc[0][x].y, acc[U / 2 - 1][x].y, TOP, lane);
+          sum[x] = fold_rows(s0, s1, TOP / 2, lane);
+          row = (lane & TOP ? 2 : 0) + (lane & (TOP / 2) ? 1 : 0);
+        } else {
+          sum[x] = fold_rows(acc[0][x].x, acc[0][x].y, TOP, lane);
+          row = lane & TOP ? 1 : 0;
+        }
 #pragma unroll
-        for (int u = 0; u < 2; ++u)
+        for (int of = U == 4 ? TOP / 4 : TOP / 2; of > 0; of >>= 1) sum[x] += __shfl_xor_sync(0xffffffffu, sum[x], of);
+        sum[x] = p.score_round ? round_bf16(round_bf16(sum[x]) * p.scale) : sum[x] * p.scale;
+      }
+      if ((lane & (U == 4 ? TOP / 4 : TOP / 2) * 2 - 1) == 0)
 #pragma unroll
-          for (int x = 0; x < (PER_HEAD ? NP : 1); ++x) acc[u][x] += __shfl_xor_sync(0xffffffffu, acc[u][x], of);
-      if ((lane & (PER_HEAD ? 7 : 31)) == 0)
-#pragma unroll
-        for (int u = 0; u < 2; ++u)
-#pragma unroll
-          for (int x = 0; x < (PER_HEAD ? NP : 1); ++x)
-            sc[PER_HEAD ? x * 4 + (lane >> 3) : 0][(i + u) * STREAM_WARPS + warp] =
-                p.score_round ? round_bf16(round_bf16(acc[u][x]) * p.scale) : acc[u][x] * p.scale;
+        for (int x = 0; x < X; ++x) sc[PER_HEAD ? x * 4 + (lane >> 3) : 0][(i + row) * STREAM_WARPS + warp] = sum[x];
     }
     __syncthreads();
     const int e0 = e_lo + b * BATCH + lane, e1 = e0 + 32;
@@ -413,20 +429,34 @@ lmk_merge_rows_kernel(FinalParams p) {
 // list can be among the K best only if fewer than K - e list heads are better than its own; so the heads are ranked by counting,
 // the K best lists are lined up by rank, and their K (K + 1) / 2 possible entries are ranked by counting again.
 // 296 lists, K = 8: 12.9 us of warp-serial insertions before.
-constexpr int RANK_LISTS = 1024;
+constexpr int RANK_LISTS = 1024, RANK_KEYS = 1664;           // keys in shared memory: the heads alone, or all of them behind the heads (one trip for both);
+                                                             // 18 KB, so that a block finds its place beside one of the scan
 
 __global__ void __launch_bounds__(FIN_WARPS * 32)
 lmk_rank_merge_kernel(FinalParams p) {
-  __shared__ __align__(16) unsigned long long heads[RANK_LISTS];
+  __shared__ __align__(16) unsigned long long heads[RANK_KEYS];
   __shared__ int by_rank[MAXK];
   __shared__ unsigned long long cand[MAXK * (MAXK + 1) / 2 + 1], best[MAXK];
   const int tid = threadIdx.x, lists = p.lists, K = p.K;
   const int padded = (lists + 1) & ~1;
   const unsigned long long* src = p.keys + (long long)blockIdx.x * p.P;
+  static_assert(RANK_LISTS <= RANK_KEYS, "the heads fit");
   if (tid < MAXK) { by_rank[tid] = -1; best[tid] = 0ull; }
   pdl_trigger();
   pdl_wait();
-  for (int i = tid; i < padded; i += FIN_WARPS * 32) heads[i] = i < lists ? src[(long long)i * K] : 0ull;
+  const bool whole = padded + lists * K <= RANK_KEYS;
+  unsigned long long* all = heads + padded;
+  if (whole) {
+    if (tid == 0 && padded > lists) heads[lists] = 0ull;
+#pragma unroll 4
+    for (int i = tid; i < lists * K; i += FIN_WARPS * 32) {
+      const unsigned long long key = src[i];
+      all[i] = key;
+      if (i % K == 0) heads[i / K] = key;
+    }
+  } else {
+    for (int i = tid; i < padded; i += FIN_WARPS * 32) heads[i] = i < lists ? src[(long long)i * K] : 0ull;
+  }
   __syncthreads();
   for (int i = tid; i < lists; i += FIN_WARPS * 32) {
     const unsigned long long mine = heads[i];
@@ -443,7 +473,7 @@ lmk_rank_merge_kernel(FinalParams p) {
   const int total = K * (K + 1) / 2;
   for (int i = tid; i < K * K; i += FIN_WARPS * 32) {
     const int r = i / K, e = i - r * K;
-    if (r + e < K) cand[r * K - r * (r - 1) / 2 + e] = by_rank[r] >= 0 ? src[(long long)by_rank[r] * K + e] : 0ull;
+    if (r + e < K) cand[r * K - r * (r - 1) / 2 + e] = by_rank[r] < 0 ? 0ull : whole ? all[by_rank[r] * K + e] : src[(long long)by_rank[r] * K + e];
   }
   __syncthreads();
   for (int i = tid; i < total; i += FIN_WARPS * 32) {
