@@ -45,14 +45,14 @@ struct ScanParams {
   float scale;
 };
 
-// Merge a batch of 64 scores (lane i: ids id0 + i and id0 + 32 + i; orderable, 0 = none; all ids above those of the list) into a
-// list of K keys held one per lane; `kth` is the list's K-th key.
-__device__ __forceinline__ void select_batch(unsigned long long& mine, unsigned long long& kth, unsigned o0, unsigned o1, unsigned id0, int K,
-                                             int lane) {
+// Merge 64 scores (lane i: ids id0 + i and id0 + 32 + i; orderable, 0 = none; all ids above those of the list) into a
+// list of K keys held one per lane, whatever scores are equal; `kth` is the list's K-th key.
+struct TopList { unsigned long long mine, kth; };
+__device__ __noinline__ TopList select_64(unsigned long long mine, unsigned long long kth, unsigned o0, unsigned o1, unsigned id0, int K, int lane) {
   const unsigned th = (unsigned)(kth >> 32);                 // 0 while the list is not full
   unsigned b0 = __ballot_sync(0xffffffffu, o0 > th), b1 = __ballot_sync(0xffffffffu, o1 > th);
   const int found = __popc(b0) + __popc(b1);
-  if (found == 0) return;
+  if (found == 0) return {mine, kth};
   if (found < K) {                                           // a few: one insertion each, lower ids first
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
@@ -68,7 +68,7 @@ __device__ __forceinline__ void select_batch(unsigned long long& mine, unsigned 
         }
       }
     }
-    return;
+    return {mine, kth};
   }
   unsigned long long run = mine, best_mine = 0ull;           // many: the K best of list and batch by K warp-wide maxima
   for (int k = 0; k < K; ++k) {
@@ -85,20 +85,70 @@ __device__ __forceinline__ void select_batch(unsigned long long& mine, unsigned 
     if (lane == k) best_mine = best;
   }
   mine = lane < K ? best_mine : 0ull;
-  kth = __shfl_sync(0xffffffffu, mine, K - 1);
+  return {mine, __shfl_sync(0xffffffffu, mine, K - 1)};
+}
+
+constexpr int BATCH = 128;
+// The same for a batch of 128 (o[i]: id id0 + 32 i + lane).  One or two that beat the list's K-th score are inserted; more, and the K best
+// come out by K warp-wide maxima of the 32-bit scores: whoever holds the maximum strikes it out and notes its key, which is all that the
+// next round waits for (~45 cycles; with the owner found by votes and its key shuffled to its place ~110, and an insertion as much).
+// Equal scores are struck out together: more struck out than rounds, and the batch is done over again the careful way.
+__device__ __forceinline__ void select_batch(unsigned long long& mine, unsigned long long& kth, const unsigned o[4], unsigned id0, int K, int lane,
+                                             unsigned long long* note) {
+  const unsigned th = (unsigned)(kth >> 32);                 // 0 while the list is not full
+  unsigned b[4];
+  int found = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) { b[i] = __ballot_sync(0xffffffffu, o[i] > th); found += __popc(b[i]); }
+  if (found == 0) return;
+  if (found <= 2) {                                          // lower ids first; what the first one pushes below the K-th place stays there
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      for (unsigned m = b[i]; m; m &= m - 1) {
+        const int src = __ffs(m) - 1;
+        list_insert(mine, ((unsigned long long)__shfl_sync(0xffffffffu, o[i], src) << 32) | (0xffffffffu - (id0 + 32 * i + src)), lane);
+      }
+    kth = __shfl_sync(0xffffffffu, mine, K - 1);
+    return;
+  }
+  unsigned r = (unsigned)(mine >> 32), v[4] = {o[0], o[1], o[2], o[3]};
+  const unsigned first = 0xffffffffu - (id0 + lane);
+  int k = 0, struck = 0;
+  for (; k < K; ++k) {
+    const unsigned m = __reduce_max_sync(0xffffffffu, max(max(max(r, v[0]), max(v[1], v[2])), v[3]));
+    if (m == 0u) break;
+    unsigned low = (unsigned)mine;
+    bool hit = r == m;
+    if (hit) { r = 0u; ++struck; }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (v[i] == m) { v[i] = 0u; low = first - 32 * i; hit = true; ++struck; }
+    if (hit) note[k] = ((unsigned long long)m << 32) | low;
+  }
+  if (__reduce_add_sync(0xffffffffu, struck) == k) {
+    __syncwarp();
+    mine = lane < k ? note[lane] : 0ull;
+    __syncwarp();
+    kth = __shfl_sync(0xffffffffu, mine, K - 1);
+    return;
+  }
+  TopList t = select_64(mine, kth, o[0], o[1], id0, K, lane);
+  t = select_64(t.mine, t.kth, o[2], o[3], id0 + 64, K, lane);
+  mine = t.mine;
+  kth = t.kth;
 }
 
 // ---------------------------------------------------------------------------------------------
 // One query row (a decode step), or one row and head at a time: the landmarks are streamed once, HBM-bound.
 //
 // Every lane copies the 16-byte pieces it will need itself to shared memory (cp.async), RING rows ahead of the
-// arithmetic, so 196 KB per SM are on their way without a register or a barrier.  Scores of 64 rows at a time go to shared
-// memory; list l (one per head, or the only one) is kept by warp l % 16, which looks at the 64 scores with two
-// votes and inserts what beats its K-th entry: one list per block instead of one per warp to merge at the end, and
+// arithmetic, so 196 KB per SM are on their way without a register or a barrier.  Scores of 128 rows at a time go to shared
+// memory; list l (one per head, or the only one) is kept by warp l % 16, which merges
+// the 128 scores into it (select_batch): one list per block instead of one per warp to merge at the end, and
 // no list code in the scoring loop (per head it was 12 lists in every warp, each with a serial insertion: 60 us for
 // 2 x 16,411 landmarks, now 16; 262,144 landmarks, one list: 68 -> 63 us = 6.3 TB/s for the scan alone, 69.4 us = 5.8 TB/s with its
 // merge).
-constexpr int BATCH = 64, STREAM_WARPS = 16;
+constexpr int SPLIT_ROWS = 64, STREAM_WARPS = 16;                // rows that a block takes at least
 template <int NP> constexpr int RING_ROWS = NP > 3 ? 6 : 8;       // 196 KB per SM
 template <int NP> constexpr int ROWS_AT_ONCE = NP > 3 ? 2 : 4;    // of a warp
 
@@ -139,6 +189,7 @@ lmk_stream_kernel(ScanParams p, FinalParams fin) {
   constexpr int RING = RING_ROWS<NP>, U = ROWS_AT_ONCE<NP>, NL = PER_HEAD ? NP * 4 : 1, MINE = (NL + STREAM_WARPS - 1) / STREAM_WARPS, ROW_BYTES = NP * 512;
   extern __shared__ __align__(16) unsigned char ring_all[];            // [STREAM_WARPS][RING][ROW_BYTES]
   __shared__ float score[2][NL][BATCH];
+  __shared__ unsigned long long note[NL < STREAM_WARPS ? NL : STREAM_WARPS][MAXK];
   pdl_trigger();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int split = blockIdx.x, t0 = blockIdx.y, n = blockIdx.z;
@@ -149,6 +200,11 @@ lmk_stream_kernel(ScanParams p, FinalParams fin) {
   const long long seen = p.q_pos0 + t0 - p.e_base;
   const int e_hi = (int)max((long long)e_lo, min((long long)min(p.E, e_lo + p.e_per_split), seen));
   const __nv_bfloat16* kb = p.lk + n * p.kbs + lane * 8;
+  // NP = ceil(D / 256): only a lane's last piece can be absent.  Nothing is ever copied to its place, which holds zeros.
+  const bool last_piece = lane + 32 * (NP - 1) < pieces;
+  if (!last_piece)
+#pragma unroll
+    for (int r = 0; r < RING; ++r) *reinterpret_cast<uint4*>(ring + r * ROW_BYTES + (NP - 1) * 512) = make_uint4(0, 0, 0, 0);
   // this warp's i-th row is e_lo + 16 i + warp; rows are asked for in order, U at a time
   const __nv_bfloat16* next_src = kb + (long long)(e_lo + warp) * p.krs;
   const long long src_step = p.krs * STREAM_WARPS;
@@ -160,7 +216,7 @@ lmk_stream_kernel(ScanParams p, FinalParams fin) {
       if (next_e < e_hi)
 #pragma unroll
         for (int pp = 0; pp < NP; ++pp)
-          if (lane + 32 * pp < pieces)
+          if (pp + 1 < NP || last_piece)
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + u * ROW_BYTES + pp * 512), "l"(next_src + pp * 256) : "memory");
       next_e += STREAM_WARPS;
       next_src += src_step;
@@ -188,6 +244,7 @@ lmk_stream_kernel(ScanParams p, FinalParams fin) {
     float (*sc)[BATCH] = score[b & 1];
 #pragma unroll
     for (int i = 0; i < BATCH / STREAM_WARPS; i += U) {
+      if (e_lo + b * BATCH + i * STREAM_WARPS >= e_hi) break;
       asm volatile("cp.async.wait_group %0;" ::"n"(RING / U - 1) : "memory");       // a lane reads only what it copied itself
       constexpr int X = PER_HEAD ? NP : 1;
       float2 acc[U / 2][X];                                  // of two rows
@@ -198,10 +255,9 @@ lmk_stream_kernel(ScanParams p, FinalParams fin) {
 #pragma unroll
         for (int pp = 0; pp < NP; ++pp) {                    // absent pieces add 0 * 0: the sums never are -0
           const unsigned char* at = ring + (slot + u) * ROW_BYTES + pp * 512;
-          const bool there = lane + 32 * pp < pieces;
           float k0[8], k1[8];
-          unpack8(there ? *reinterpret_cast<const uint4*>(at) : make_uint4(0, 0, 0, 0), k0);
-          unpack8(there ? *reinterpret_cast<const uint4*>(at + ROW_BYTES) : make_uint4(0, 0, 0, 0), k1);
+          unpack8(*reinterpret_cast<const uint4*>(at), k0);
+          unpack8(*reinterpret_cast<const uint4*>(at + ROW_BYTES), k1);
           float2& s = acc[u / 2][PER_HEAD ? pp : 0];
 #pragma unroll
           for (int jj = 0; jj < 8; ++jj) s = __ffma2_rn(make_float2(qf[pp][jj], qf[pp][jj]), make_float2(k0[jj], k1[jj]), s);
@@ -231,17 +287,19 @@ lmk_stream_kernel(ScanParams p, FinalParams fin) {
         for (int x = 0; x < X; ++x) sc[PER_HEAD ? x * 4 + (lane >> 3) : 0][(i + row) * STREAM_WARPS + warp] = sum[x];
     }
     __syncthreads();
-    const int e0 = e_lo + b * BATCH + lane, e1 = e0 + 32;
+    const int e0 = e_lo + b * BATCH + lane;
 #pragma unroll
     for (int x = 0; x < MINE; ++x) {
       const int l = warp + x * STREAM_WARPS;
       if (l >= NL || (PER_HEAD && l >= p.H)) continue;
-      float s0 = sc[l][lane], s1 = sc[l][lane + 32];
-      if (p.noise) {
-        if (e0 < e_hi) s0 += p.noise[((long long)n * p.Cq + t0) * p.E + e0];
-        if (e1 < e_hi) s1 += p.noise[((long long)n * p.Cq + t0) * p.E + e1];
+      unsigned o[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float s = sc[l][lane + 32 * i];
+        if (p.noise && e0 + 32 * i < e_hi) s += p.noise[((long long)n * p.Cq + t0) * p.E + e0 + 32 * i];
+        o[i] = e0 + 32 * i < e_hi ? orderable(s) : 0u;
       }
-      select_batch(mine[x], kth[x], e0 < e_hi ? orderable(s0) : 0u, e1 < e_hi ? orderable(s1) : 0u, (unsigned)(p.e_base + e_lo + b * BATCH), p.K, lane);
+      select_batch(mine[x], kth[x], o, (unsigned)(p.e_base + e_lo + b * BATCH), p.K, lane, note[warp]);
     }
   }
   if (FUSED) {
@@ -607,7 +665,7 @@ namespace {
 // Landmark ranges of the streaming form: one block per SM at a time, so what counts is whole waves; a wave costs about as much
 // again as reading 200 rows before and after its stream (32 rows x 4,096 landmarks: one wave of 4 ranges 36 us, two of 9 41; x 8,192
 // 66 either way).
-int most_stream_splits(const LmkTopkArgs& a, int sms) { return (int)std::min<long long>((a.E + BATCH - 1) / BATCH, 2 * sms); }
+int most_stream_splits(const LmkTopkArgs& a, int sms) { return (int)std::min<long long>((a.E + SPLIT_ROWS - 1) / SPLIT_ROWS, 2 * sms); }
 int stream_splits(const LmkTopkArgs& a, int sms) {
   const long long blocks = (long long)a.N * a.Cq;
   const int most = most_stream_splits(a, sms);
