@@ -117,6 +117,19 @@ def test_per_head_mode(lcm):
     check(res, oracle_rows(lq, lk, 8, head_dim=64))
 
 
+@pytest.mark.parametrize("splits", [1, 3, 20, 40, 160, 161])
+@pytest.mark.parametrize("d,head_dim", [(768, 0), (768, 64), (72, 0), (520, 0), (1024, 64), (1000, 0)])
+def test_equal_scores_in_every_batch_and_list(lcm, d, head_dim, splits):
+    """Five distinct landmarks over and over: every maximum of a batch, and of the lists that are merged, is held by many at once (a plain cache
+    in front, so that lists are full of distinct scores before).  Also widths whose last piece not every lane has, and 0 landmarks in a block."""
+    g = torch.Generator().manual_seed(d + splits)
+    e, k = 161 * 9 + 4, 8 if splits != 20 else 21
+    lq, lk = cases.landmark_case(d, 1, 1, e, d=d)
+    lk[:, 700:] = lk[:, :5][:, torch.randint(0, 5, (e - 700,), generator=g)]
+    res = lcm.lmk_score_topk(lq.cuda(), lk.cuda(), k, q_pos0=e - 2, head_dim=head_dim, splits=splits)
+    check(res, oracle_rows(lq, lk, k, q_pos0=e - 2, head_dim=head_dim))
+
+
 def test_noise_selects_but_weights_stay_noise_free(lcm):
     """Training: Gumbel noise perturbs the selection only (DRT.py:616-626)."""
     n, c, d, k = 2, 20, 768, 4
