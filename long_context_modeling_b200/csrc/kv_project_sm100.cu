@@ -19,7 +19,7 @@
 // weight rows: per product a third less shared-memory and L2 traffic than 128 x 256, and power is what a large
 // product is bound by (SM clock 1.3-1.6 GHz of 1.97 within milliseconds).  8 x 260 chunks x 64 rows, 768 -> 2 x 768, as the call with the
 // allocation of its cache: 252 us after a rest, 289 in a row; cuBLAS, in the same run, 285 / 294 us for the bare product (with
-// 128 x 256 tiles in place of pairs the call took 7 % more).  Smaller products take the width of 64, 128, 192 or 256 columns
+// 128 x 256 tiles in place of pairs the call took 7 % more).  Other products take the width of 64, 128, 192 or 256 columns
 // whose waves cost least: 6,912 rows 768 -> 768 on 148 SMs are 162 tiles of 256 columns (two waves, the second nearly
 // empty) but 216 of 192: 33 -> 19 us.
 //
@@ -30,7 +30,8 @@
 // are never written), residual makes it o_proj + residual add.  The factors come from the tiles of x as
 // they pass (NORM); for pairs, whose tiles arrive on the leader's barriers alone, `row_rms_kernel` reads x
 // before.  768 -> 768, 640 / 2,368 / 7,104 rows, x from memory: 6.7 / 8.1 / 14.8 us, with that launch before
-// 8.0 / 11.2 / 17.1.
+// 8.0 / 11.2 / 17.1.  The residual is read two passes of 32 columns ahead of its use; read in the pass itself, an L2 trip each, 1,152 / 3,456 / 7,104 /
+// 16,384 rows took 7.3 / 11.4 / 16.1 / 27.4 us, now 6.2 / 9.8 / 14.8 / 25.4.
 //
 // CROSS-ENTROPY mode is the LM head fused with the loss (model/DRT.py:1055-1064, inference /
 // evaluation): the 128 x 256 logit tiles stay in tensor memory, the epilogue reduces each row's tile
@@ -297,18 +298,53 @@ kv_project_append_kernel(const __grid_constant__ ProjParams p) {
           for (int v = lane; v < vecs; v += 32) p.lmk[n * p.lmk_bs + (p.pos + c) * vecs + v] = p.x_rows[last * vecs + v];
         }
       }
+      // this thread's row: linear mode out = scale * acc + residual, append mode a cache row (zeros for a landmark row)
+      struct Row { __nv_bfloat16* dst; const __nv_bfloat16* res; float sc; bool live, zero; };
+      auto row_of = [&] {
+        Row o = {nullptr, nullptr, 1.0f, false, false};
+        if (p.nmat == 1) {
+          const int block = (C::TM / 64) * tm + 2 * (int)rank + (row_in_tile >> 6), b = block / p.blocks_per_batch;
+          const long long m = (block - b * p.blocks_per_batch) * 64 + (row_in_tile & 63);
+          o.live = b < p.batches && m < p.M;
+          if (!NORM && o.live && p.row_scale) o.sc = p.row_scale[b * p.scale_bs + m];
+          o.dst = p.out + b * p.out_bs + m * p.out_stride + tn * BN;
+          if (o.live && p.residual) o.res = p.residual + b * p.res_bs + m * p.res_stride + tn * BN;
+        } else {
+          const long long m = (long long)tm * C::TM + (int)rank * BM + row_in_tile;
+          o.live = m < p.M;
+          const int n = o.live ? (int)(m / p.rows_per_seq) : 0;
+          const int r = o.live ? (int)(m - (long long)n * p.rows_per_seq) : 0;       // (chunk, row) inside the appended block
+          o.zero = p.zero_landmark && (r & 63) == 63;
+          o.dst = (which ? p.v_cache : p.k_cache) + n * p.cache_bs + ((long long)p.pos * 64 + r) * p.D + tn * BN;
+        }
+        return o;
+      };
+      // Passes of 32 columns (or the last 16) of one small loop body.  A pass's residual is asked for two passes ahead, that of the first two
+      // before the accumulator is waited for.
+      const int cols = min(BN, p.ncols - tn * BN);       // not every width divides every matrix: the last tile may be a narrow one
+      const int c_begin = half * (BN / 2), c_end = min(cols, c_begin + BN / 2);
+      const bool ce = p.nmat == 1 && p.ce_part;
+      const Row row = ce ? Row{nullptr, nullptr, 1.0f, false, false} : row_of();
+      int ask_c = c_begin;
+      const bool with_res = p.nmat == 1 && p.residual;
+      auto ask = [&](uint4 (&r)[4]) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) r[i] = (row.res && ask_c + 8 * i < c_end) ? *reinterpret_cast<const uint4*>(row.res + ask_c + 8 * i) : make_uint4(0, 0, 0, 0);
+        ask_c += 32;
+      };
+      uint4 rr[4] = {}, rr_next[4];
+      if (with_res) { ask(rr); ask(rr_next); }
       ok = mbar_wait_bounded(&bars[ACC_FULL + ab], (tcount >> 1) & 1, abort_flag);
       if (NORM) ok = ok && mbar_wait_bounded(&bars[SCALE_FULL + ab], (tcount >> 1) & 1, abort_flag);
       if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
       tc_fence_after();
-      long long m = (long long)tm * C::TM + (int)rank * BM + row_in_tile;
-      bool live = m < p.M;
-      if (p.nmat == 1 && p.ce_part) {
+      if (ce) {
+        const long long m = (long long)tm * C::TM + (int)rank * BM + row_in_tile;
+        const bool live = m < p.M;
         if (half) { release(ab); continue; }             // a row's tile is reduced by one thread
         // cross-entropy mode: per row, the maximum and the sum of exponentials of this column
         // tile's logits (base 2, logits scaled by log2 e) and the target's logit if it lies here
         const float sc = ((live && p.row_scale) ? p.row_scale[m] : 1.0f) * GCA_LOG2E;
-        const int cols = min(BN, p.ncols - tn * BN);
         const long long tgt = live ? p.targets[m] - (long long)tn * BN : -1;
         float mx = -INFINITY, sum = 0.f;
 #pragma unroll 1
@@ -339,56 +375,37 @@ kv_project_append_kernel(const __grid_constant__ ProjParams p) {
         release(ab);
         continue;
       }
-      // a row of the output: linear mode out = scale * acc + residual, append mode a cache row (zeros for a landmark row)
-      __nv_bfloat16* dst;
-      const __nv_bfloat16* res = nullptr;
-      float sc = 1.0f;
-      bool zero = false;
-      const int cols = min(BN, p.ncols - tn * BN);       // 192 does not divide every width: the last tile is a narrow one
-      if (p.nmat == 1) {
-        const int block = (C::TM / 64) * tm + 2 * (int)rank + (row_in_tile >> 6), b = block / p.blocks_per_batch;
-        m = (block - b * p.blocks_per_batch) * 64 + (row_in_tile & 63);
-        live = b < p.batches && m < p.M;
-        if (NORM) sc = scale[ab * BM + row_in_tile];
-        else if (live && p.row_scale) sc = p.row_scale[b * p.scale_bs + m];
-        dst = p.out + b * p.out_bs + m * p.out_stride + tn * BN;
-        if (live && p.residual) res = p.residual + b * p.res_bs + m * p.res_stride + tn * BN;
-      } else {
-        const int n = live ? (int)(m / p.rows_per_seq) : 0;
-        const int r = live ? (int)(m - (long long)n * p.rows_per_seq) : 0;       // (chunk, row) inside the appended block
-        zero = p.zero_landmark && (r & 63) == 63;
-        dst = (which ? p.v_cache : p.k_cache) + n * p.cache_bs + ((long long)p.pos * 64 + r) * p.D + tn * BN;
-      }
-      // passes of 32 columns (or the last 16) of one small loop body; the residual is asked for before the accumulator
-      const int c_end = min(cols, (half + 1) * (BN / 2));
+      const float sc = NORM ? scale[ab * BM + row_in_tile] : row.sc;
 #pragma unroll 1
-      for (int c0 = half * (BN / 2); c0 < c_end; c0 += 32) {
-        uint32_t v[32];
-        uint4 rr[4];
+      for (int c0 = c_begin; c0 < c_end; c0 += 32) {
+        uint32_t v[32], w[16];
         const bool two = c0 + 16 < c_end;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) rr[i] = (res && (i < 2 || two)) ? *reinterpret_cast<const uint4*>(res + c0 + 8 * i) : make_uint4(0, 0, 0, 0);
         tmem_ld_32x32b_x32(tlane + ab * ACC_COLS + c0, v);
+        const uint32_t rw[16] = {rr[0].x, rr[0].y, rr[0].z, rr[0].w, rr[1].x, rr[1].y, rr[1].z, rr[1].w,
+                                 rr[2].x, rr[2].y, rr[2].z, rr[2].w, rr[3].x, rr[3].y, rr[3].z, rr[3].w};
         tmem_ld_wait();
-        if (zero) {
+        if (row.zero) {
 #pragma unroll
           for (int i = 0; i < 32; ++i) v[i] = 0u;
         }
-        if (!live) continue;
-        const uint32_t rw[16] = {rr[0].x, rr[0].y, rr[0].z, rr[0].w, rr[1].x, rr[1].y, rr[1].z, rr[1].w,
-                                 rr[2].x, rr[2].y, rr[2].z, rr[2].w, rr[3].x, rr[3].y, rr[3].z, rr[3].w};
-        uint32_t w[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i)
           w[i] = pack_bf16x2(fmaf(__uint_as_float(v[2 * i]), sc, __uint_as_float(rw[i] << 16)),
                              fmaf(__uint_as_float(v[2 * i + 1]), sc, __uint_as_float(rw[i] & 0xffff0000u)));
+        if (with_res) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) rr[i] = rr_next[i];
+          ask(rr_next);
+        }
+        if (!row.live) continue;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           if (h && !two) break;
-          if (p.wide) st_global_256(dst + c0 + 16 * h, w[8 * h], w[8 * h + 1], w[8 * h + 2], w[8 * h + 3], w[8 * h + 4], w[8 * h + 5], w[8 * h + 6], w[8 * h + 7]);
+          __nv_bfloat16* dst = row.dst + c0 + 16 * h;
+          if (p.wide) st_global_256(dst, w[8 * h], w[8 * h + 1], w[8 * h + 2], w[8 * h + 3], w[8 * h + 4], w[8 * h + 5], w[8 * h + 6], w[8 * h + 7]);
           else {
-            reinterpret_cast<uint4*>(dst + c0 + 16 * h)[0] = make_uint4(w[8 * h], w[8 * h + 1], w[8 * h + 2], w[8 * h + 3]);
-            reinterpret_cast<uint4*>(dst + c0 + 16 * h)[1] = make_uint4(w[8 * h + 4], w[8 * h + 5], w[8 * h + 6], w[8 * h + 7]);
+            reinterpret_cast<uint4*>(dst)[0] = make_uint4(w[8 * h], w[8 * h + 1], w[8 * h + 2], w[8 * h + 3]);
+            reinterpret_cast<uint4*>(dst)[1] = make_uint4(w[8 * h + 4], w[8 * h + 5], w[8 * h + 6], w[8 * h + 7]);
           }
         }
       }
@@ -487,17 +504,25 @@ bool few_rows(long long M, int N, int K, bool with_norm, int sms);
 
 namespace {
 
-// Which tile: wide pairs once every pair of SMs has one (they read the least shared memory and L2 per product, and power is what a
-// large product runs into), else the width whose waves cost least.  In units of column-steps of one CTA: a tile costs its
-// width plus ~64 for its prologue and epilogue tail.
+// Which tile: the width, or the pairs, whose waves cost least.
+//   APPEND (and cross-entropy): in units of column-steps of one CTA a tile costs its width plus ~64 for its prologue and epilogue tail; wide pairs, which read
+// the least shared memory and L2 per product, ~48 (power is what a large product runs into).
+//   LINEAR, 768 -> 768 with a residual, us a wave: 64 columns 3.0, 128 3.8, 192 5.4, 256 7.0.  Pairs never better than 256 columns: 12,288 rows 19.3 us
+// against 18.8, 24,576 39.9 / 37.6, 133,120 197 / 185 (power limit), 1,024 -> 1,024 with 49,152 rows 111 / 108, 512 -> 512 with 65,536 67 / 56.
+//   NORM, us a wave: 4.6, 4.9, 5.7, 6.5.  Pairs need a launch before for the rows' factors: 12,288 rows 22.7 us against 16.8 with 256 columns, 133,120 200 / 178;
+// 512 -> 512, 6,912 rows 13.9 / 9.1.  From K = 1,024 and six waves on the factors in every column tile cost more: 24,576 rows 60.2 / 62.7, 49,152 109 / 119.
+enum class Product { APPEND, LINEAR, NORM };
 struct TileChoice { int bn; bool pair; };
-TileChoice choose_tile(long long rows64, int ncols, int nmat, int sms) {
+TileChoice choose_tile(Product product, long long rows64, int ncols, int k, int nmat, int sms) {
   auto ceil_div = [](long long a, long long b) { return (a + b - 1) / b; };
+  const long long pair_waves = ceil_div(ceil_div(rows64, 4) * ceil_div(ncols, 256) * nmat, sms / 2);
+  const bool pairs = product == Product::APPEND || (product == Product::NORM && k >= 1024 && pair_waves >= 6);
   TileChoice best = {256, true};
-  long long best_cost = ceil_div(ceil_div(rows64, 4) * ceil_div(ncols, 256) * nmat, sms / 2) * (256 + 48);
+  long long best_cost = pairs ? pair_waves * (256 + (product == Product::NORM ? 240 : 48)) : -1;
   for (int bn : {256, 192, 128, 64}) {
-    const long long cost = ceil_div(ceil_div(rows64, 2) * ceil_div(ncols, bn) * nmat, sms) * (bn + 64);
-    if (cost < best_cost) { best_cost = cost; best = {bn, false}; }
+    const int tile = product == Product::APPEND ? bn + 64 : product == Product::LINEAR ? (bn == 64 ? 120 : bn + 24) : bn + 260;
+    const long long cost = ceil_div(ceil_div(rows64, 2) * ceil_div(ncols, bn) * nmat, sms) * tile;
+    if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = {bn, false}; }
   }
   return best;
 }
@@ -553,7 +578,7 @@ int launch_linear_ce(const LinearCeArgs& a, int sms, cudaStream_t stream) {
   p.ce_part = reinterpret_cast<float2*>(a.workspace);
   p.ce_target = reinterpret_cast<float*>(p.ce_part + a.M * tiles);
   p.targets = reinterpret_cast<const long long*>(a.targets);
-  TileChoice tile = choose_tile((a.M + 63) / 64, a.N, 1, sms);
+  TileChoice tile = choose_tile(Product::APPEND, (a.M + 63) / 64, a.N, a.K, 1, sms);
   tile.bn = 256;                                       // the workspace counts 256-column tiles
   if ((rc = launch_product(p, a.w, a.w, a.w_stride, (a.M + 63) / 64, tile, sms, stream))) return rc;
   const int warps = 8;
@@ -622,7 +647,7 @@ int launch_linear(const LinearBatchedArgs& ba, float* norm_scratch, int sms, cud
   p.ce_part = nullptr; p.ce_target = nullptr; p.targets = nullptr;
   const long long blocks = per_batch * args.batches;
   if (blocks >= (1ll << 30)) return GCA_ERR_TOO_LARGE;
-  const TileChoice tile = choose_tile(blocks, a.N, 1, sms);
+  const TileChoice tile = choose_tile(norm_scratch ? Product::NORM : Product::LINEAR, blocks, a.N, a.K, 1, sms);
   const bool norm = norm_scratch && !tile.pair;
   p.rms_eps = norm_eps;
   if (norm_scratch && !norm) {
@@ -645,7 +670,7 @@ int launch_kv_project_append(const KvProjectArgs& a, int sms, cudaStream_t strea
   p.batches = 1; p.blocks_per_batch = 0; p.lead_rows = 0; p.out_bs = p.res_bs = p.scale_bs = 0;
   p.wide = 1;                                          // the entry point asks for 32-byte aligned caches
   p.x_rows = (const uint4*)a.x; p.lmk = (uint4*)a.lmk_cache; p.lmk_bs = a.lmk_cache_batch_stride / 8;
-  return launch_product(p, a.wk, a.wv, a.D, M / 64, choose_tile(M / 64, a.D, 2, sms), sms, stream);
+  return launch_product(p, a.wk, a.wv, a.D, M / 64, choose_tile(Product::APPEND, M / 64, a.D, a.D, 2, sms), sms, stream);
 }
 
 }  // namespace gca

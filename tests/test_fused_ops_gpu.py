@@ -441,6 +441,23 @@ def test_norm_from_the_tiles_of_x(m, n, k):
     assert torch.equal(got, F.rmsnorm_linear(x, w, 1e-5).double()) and lcm.read_status() == 0
 
 
+@pytest.mark.parametrize("m,n,k", [(130, 80, 64), (2333, 512, 512), (7105, 784, 192), (12400, 768, 512), (25000, 1024, 1024)])
+def test_residual_read_ahead_and_norm_tiles(m, n, k):
+    """The residual is read two passes ahead of the stores: adding onto it in place gives what a residual of its own gives, in 1 to 4 passes of a thread's
+    columns, a last one of 16.  The same sizes with the norm: 64 to 256 columns in up to six waves, and pairs behind a launch for the factors."""
+    need_gpu()
+    from long_context_modeling_b200 import fused_ops as F
+    g = torch.Generator(device="cuda").manual_seed(m)
+    x, w, r = ((torch.randn(*s, generator=g, device="cuda") * c).bfloat16() for s, c in (((m, k), 1.0), ((n, k), k ** -0.5), ((m, n), 1.0)))
+    y = F.linear(x, w, residual=r)
+    close(y, x.float() @ w.float().t() + r.float())
+    there = r.clone()
+    F.linear(x, w, residual=there, out=there)
+    assert torch.equal(there, y)
+    xf = x.float()
+    close(F.rmsnorm_linear(x, w, 1e-5), (xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + 1e-5)) @ w.float().t())
+
+
 @pytest.mark.parametrize("n,c,dim", [(1, 1, 256), (3, 5, 512), (5, 61, 768), (2, 300, 1024)])
 def test_projection_append_tile_widths(n, c, dim):
     """K, V and landmark rows of an append at a position behind earlier chunks, against float32, small and large products."""
