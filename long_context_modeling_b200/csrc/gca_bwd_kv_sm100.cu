@@ -67,23 +67,17 @@ constexpr uint32_t PAIR16 = PAIR_BYTES >> 4, TILE16 = TILE_BYTES >> 4;
 #ifndef GCA_KV_SPLIT
 #define GCA_KV_SPLIT 1
 #endif
-#ifndef GCA_KV_GRAD2
-#define GCA_KV_GRAD2 1
-#endif
 constexpr int NBUF = GCA_KV_NBUF, SPLIT = GCA_KV_SPLIT, NG = NBUF * SPLIT;
-constexpr int GRAD_ISSUERS = GCA_KV_GRAD2 ? 2 : 1;       // dV and dK from one warp, or from a warp each
+constexpr int GRAD_ISSUERS = 2;                          // dV and dK from a warp each
 static_assert(NBUF == 2 || NBUF == 3, "score buffers");
-// One issuing warp per product (two for the gradients with GRAD2).  Measured slower: one issuing
+// One issuing warp per product.  Measured slower: one issuing
 // warp per HEAD (0.955 against 0.615 ms: both heads of an iteration share the buffer's columns, and
 // every extra polling warp loads the shared-memory path); a warpgroup of its own that writes dK /
 // dV so that no worker group is held up by a unit's output (0.668 ms, 0.70-0.81 with sleeping
 // waits: with single accumulators the gradient issuers wait for the writer either way, and four
-// more resident warps cost more than the freed worker group gains).
-// Probing the next iteration's barriers before the current iteration's MMAs are issued (a 7 % gain in the
-// q-major kernel) was measured slower here: 0.634 against 0.613 ms.
-#ifndef GCA_KV_PREPROBE
-#define GCA_KV_PREPROBE 0
-#endif
+// more resident warps cost more than the freed worker group gains); the two tiles through the groups of the last two iterations, which frees the
+// accumulators in half the time (0.657 against 0.635); probing the next iteration's barriers before the current iteration's MMAs are issued,
+// a gain in the q-major kernel (0.634 against 0.613).
 constexpr int PROD_WARP = 4 * NG, ISSUE_S = PROD_WARP + 1, ISSUE_DP = ISSUE_S + 1, ISSUE_DV = ISSUE_DP + 1;       // dK issuer (GRAD2): ISSUE_DV + 1
 constexpr int SCHED_WARP = ISSUE_DV + GRAD_ISSUERS;
 constexpr int NTHREADS = (SCHED_WARP + 1) * 32;
@@ -309,17 +303,18 @@ __host__ __device__ constexpr uint32_t packed_col(int kk) {
   return (uint32_t)((16 * kk) / WCOLS * WCOLS + ((16 * kk) % WCOLS) / 2);
 }
 
-// role 0: S^T per iteration;  role 1: dP^T per iteration;  role 2: dV (and dK when there is one
-// gradient issuer);  role 3: dK.  All 32 lanes run this code; elect.sync inside the MMA / commit
-// wrappers picks the issuing lane.
-template <int ROLE>
+// SCORES: S^T per iteration (second: dP^T); else dV (second: dK).  All 32 lanes run this
+// code; elect.sync inside the MMA / commit wrappers picks the issuing lane.  The two warps of a kind run the SAME code, told apart by
+// `second`: the roles of this kernel do not fit the instruction cache together, and a copy of this loop for each product cost 8 x 256 chunks, K = 8
+// 626 us instead of 611, 1 x 1,024, K = 16 580 instead of 556, pre-gathered 109 x 8 heads (units of two iterations) 33.8 instead of 28.7.
+template <bool SCORES>
 __device__ void kv_issuer(const BwdKvParams& p, uint8_t* smem, uint64_t* bars, volatile int* abort_flag, int lane,
-                          uint32_t tmem_base) {
+                          uint32_t tmem_base, uint32_t second) {
   const uint64_t dKV = umma_desc_sw128(smem_u32(smem + OFF_KV));
   const uint64_t dQDO = umma_desc_sw128(smem_u32(smem + OFF_QDO));
   const uint64_t dQDOmn = umma_desc_sw128_mn_blocks(smem_u32(smem + OFF_QDO), TILE_BYTES);
   const uint32_t zero_addr = smem_u32(smem + OFF_ZERO);
-  const uint32_t ones_addr = smem_u32(smem + (ROLE == 0 ? OFF_ONES_S : OFF_ONES_DP));
+  const uint32_t ones_addr = smem_u32(smem + (second ? OFF_ONES_DP : OFF_ONES_S));
   const uint64_t dOnes = umma_desc_nosw_k(ones_addr, zero_addr - ones_addr, 128);
   const float* sw = reinterpret_cast<const float*>(smem + OFF_W);
   Ring ring, ur; ring.init(NQ); ur.init(ND);
@@ -334,31 +329,20 @@ __device__ void kv_issuer(const BwdKvParams& p, uint8_t* smem, uint64_t* bars, v
     if (niter == 0) continue;
     const uint32_t un = ucnt++;
     const uint32_t kb = un % NKV;
-    if (ROLE < 2) ok = mbar_wait_warp(&bars[KV_FULL + kb], (un / NKV) & 1, abort_flag, lane);
+    if (SCORES) ok = mbar_wait_warp(&bars[KV_FULL + kb], (un / NKV) & 1, abort_flag, lane);
     else ok = mbar_wait_warp(&bars[ACC_EMPTY], (un & 1) ^ 1, abort_flag, lane);
-    bool pre_a = false, pre_b = false;           // early probe results for the coming iteration
     for (int i = 0; i < niter && ok; ++i, ++g) {
       const uint64_t stage = ring.st * 2 * PAIR16;
       const uint32_t tbuf = tmem_base + b * BUF_COLS;
-      if (ROLE < 2) {
+      if (SCORES) {
         // the tiles have landed AND the buffer's previous contents (the packed A operands of iteration
         // g - NBUF) have been consumed: both barriers are probed at once (one shared-memory round trip)
-        if (lane == 0 && ROLE == 0) GCA_TRACE_BUF(p.prof, 1, g);
-        // (probed while the previous iteration's MMAs were being issued, when there was one in this unit)
-        ok = mbar_wait_warp2_probed(&bars[QDO_FULL + ring.st], ring.ph, pre_a, &bars[BUF_FREE + b], bph ^ 1, pre_b, abort_flag);
+        ok = mbar_wait_warp2(&bars[QDO_FULL + ring.st], ring.ph, &bars[BUF_FREE + b], bph ^ 1, abort_flag, lane);
         if (!ok) break;
-        if (lane == 0 && ROLE == 0) GCA_TRACE_BUF(p.prof, 2, g);
         tc_fence_after();
-        pre_a = pre_b = false;
-        if (GCA_KV_PREPROBE && i + 1 < niter) {          // the next iteration's two barriers: their shared-memory round
-          const uint32_t nst = ring.st + 1 == (uint32_t)ring.depth ? 0u : ring.st + 1, nph = nst ? ring.ph : ring.ph ^ 1;   // trip runs under the MMA issue
-          const uint32_t nb = b + 1 == NBUF ? 0u : b + 1, nbph = nb ? bph : bph ^ 1;
-          pre_a = mbar_test_wait(&bars[QDO_FULL + nst], nph);
-          pre_b = mbar_test_wait(&bars[BUF_FREE + nb], nbph ^ 1);
-        }
-        const uint64_t a = dKV + kb * 2 * PAIR16 + (ROLE == 0 ? 0u : PAIR16);       // K pair | V pair
-        const uint64_t bq = dQDO + stage + (ROLE == 0 ? 0u : PAIR16);               // Q pair | dO pair
-        const uint32_t d = tbuf + (ROLE == 0 ? 0u : COL_DPT);
+        const uint64_t a = dKV + kb * 2 * PAIR16 + second * PAIR16;       // K pair | V pair
+        const uint64_t bq = dQDO + stage + second * PAIR16;               // Q pair | dO pair
+        const uint32_t d = tbuf + second * COL_DPT;
         // fifth K step: A = the constant ones tile, B = the head's row-term tile of this stage
         const uint32_t rt = smem_u32(smem + OFF_RT + ring.st * 2 * RT_BYTES);
 #pragma unroll
@@ -371,43 +355,26 @@ __device__ void kv_issuer(const BwdKvParams& p, uint8_t* smem, uint64_t* bars, v
                              IDESC_64, 1u);
         }
         umma_commit_elect(&bars[SP_FULL + b]);            // the barrier expects both the S^T and the dP^T commit
-        if (lane == 0) GCA_TRACE_BUF(p.prof, 3 + ROLE, g);
       } else {
-        ok = mbar_wait_warp2_probed(&bars[PDS_FULL + b], bph, pre_a, &bars[PDS_FULL + b], bph, true, abort_flag);
+        ok = mbar_wait_warp(&bars[PDS_FULL + b], bph, abort_flag, lane);
         if (!ok) break;
-        if (lane == 0 && ROLE == 2) GCA_TRACE_BUF(p.prof, 5, g);
         tc_fence_after();
-        pre_a = false;
-        if (GCA_KV_PREPROBE && i + 1 < niter) {
-          const uint32_t nb = b + 1 == NBUF ? 0u : b + 1, nbph = nb ? bph : bph ^ 1;
-          pre_a = mbar_test_wait(&bars[PDS_FULL + nb], nbph);
-        }
         // the workers produced |w| P^T and |w| dS^T: a negative weight negates both A operands
         const uint32_t idesc = IDESC_GRAD | (sw[ring.st] < 0.f ? IDESC_NEG_A : 0u);
         // dV += (w P)^T dO, dK += dS^T Q, per head: A from tensor memory (lane = key row, 8 columns
         // per K step of 16 query rows), B = the head's dO / Q tile read N-contiguous (MN-major)
-        if (ROLE == 2) {
+        const uint32_t acc = tmem_base + (second ? COL_DK : COL_DV), at = tbuf + second * COL_DPT;
+        const uint64_t bg = dQDOmn + stage + (second ? 0u : PAIR16);
 #pragma unroll
-          for (int tl = 0; tl < 2; ++tl) {
-  #pragma unroll
-            for (int kk = 0; kk < 4; ++kk)
-              umma_bf16_ts_elect(tmem_base + COL_DV + (tl ? LANE16 : 0u), tbuf + (tl ? LANE16 : 0u) + packed_col(kk),
-                                 dQDOmn + stage + PAIR16 + tl * TILE16 + kk * STEP_MN, idesc, (uint32_t)(i > 0 || kk > 0));
-          }
-        }
-        if (ROLE == 3 || GRAD_ISSUERS == 1) {
+        for (int tl = 0; tl < 2; ++tl) {
 #pragma unroll
-          for (int tl = 0; tl < 2; ++tl) {
-  #pragma unroll
-            for (int kk = 0; kk < 4; ++kk)
-              umma_bf16_ts_elect(tmem_base + COL_DK + (tl ? LANE16 : 0u), tbuf + COL_DPT + (tl ? LANE16 : 0u) + packed_col(kk),
-                                 dQDOmn + stage + tl * TILE16 + kk * STEP_MN, idesc, (uint32_t)(i > 0 || kk > 0));
-          }
+          for (int kk = 0; kk < 4; ++kk)
+            umma_bf16_ts_elect(acc + (tl ? LANE16 : 0u), at + (tl ? LANE16 : 0u) + packed_col(kk), bg + tl * TILE16 + kk * STEP_MN, idesc,
+                               (uint32_t)(i > 0 || kk > 0));
         }
         umma_commit_elect(&bars[BUF_FREE + b]);
         umma_commit_elect(&bars[QDO_EMPTY + ring.st]);   // Q / dO of this iteration are free once dV, dK are done
         if (i == niter - 1) umma_commit_elect(&bars[ACC_FULL + b]);   // written out by the last iteration's worker groups
-        if (lane == 0 && ROLE == 2) GCA_TRACE_BUF(p.prof, 6, g);
       }
       ring.next();
       if (++b == NBUF) { b = 0; bph ^= 1; }
@@ -591,10 +558,8 @@ bwd_kv_tc_kernel(const __grid_constant__ BwdKvParams p) {
   const uint32_t tmem_base = *tmem_slot;
   // The order of the roles is the order of their code, and the time depends on where the hot loops lie: 8 x 256 chunks, forward +
   // backward, 1543 us with the issuers in front, 1565 with the workers in front, 1600 with scheduler and producer in front.
-  if (warp == ISSUE_S) kv_issuer<0>(p, smem, bars, abort_flag, lane, tmem_base);
-  else if (warp == ISSUE_DP) kv_issuer<1>(p, smem, bars, abort_flag, lane, tmem_base);
-  else if (warp == ISSUE_DV) kv_issuer<2>(p, smem, bars, abort_flag, lane, tmem_base);
-  else if (GRAD_ISSUERS == 2 && warp == ISSUE_DV + 1) kv_issuer<3>(p, smem, bars, abort_flag, lane, tmem_base);
+  if (warp == ISSUE_S || warp == ISSUE_DP) kv_issuer<true>(p, smem, bars, abort_flag, lane, tmem_base, (uint32_t)(warp - ISSUE_S));
+  else if (warp == ISSUE_DV || warp == ISSUE_DV + 1) kv_issuer<false>(p, smem, bars, abort_flag, lane, tmem_base, (uint32_t)(warp - ISSUE_DV));
   else if (warp < 4 * NG) {
     reduce_dw(p);                        // while the first tiles are on their way
     kv_worker(p, smem, bars, abort_flag, warp >> 2, warp & 3, lane, tmem_base);

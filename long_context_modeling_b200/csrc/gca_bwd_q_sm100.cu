@@ -35,7 +35,7 @@
 // average, of which the slot's 24 MMAs take 768.  With three groups on three shared S / dP buffers, and every role walking the units
 // by itself, it was 1,515: the groups, busy all of their 4,170 cycles a slot, and 870 cycles at each unit's end.  Each change alone gave little
 // (four groups 522 -> 511 us, records with three groups 512 -> 521, separate regions with three groups 521 -> 532), together 523 -> 506,
-// and 547 -> 540 at 1 x 1,024 chunks, K = 16.
+// with one code for the S and dP issuers 500; at 1 x 1,024 chunks, K = 16 539 -> 529.
 #include "gca_common.cuh"
 #include "sm100_ptx.cuh"
 #include "tc_common.cuh"
@@ -293,51 +293,49 @@ __device__ void q_producer(const BwdQParams& p, uint8_t* smem, uint64_t* bars, v
   }
 }
 
-// role 0: S per slot;  role 1: dP per slot;  role 2: dQ += dS K per slot.  All 32 lanes run this
+// SCORES: S per slot, or dP (dp = 1), the two warps with ONE code between them (a copy each: 507 instead of 500 us at 8 x 256 chunks, K = 8; the roles do not fit the
+// instruction cache together); else dQ += dS K per slot.  All 32 lanes run this
 // code; elect.sync inside the MMA / commit wrappers picks the issuing lane.
-template <int ROLE>
-__device__ void q_issuer(uint8_t* smem, uint64_t* bars, volatile int* abort_flag, int lane, uint32_t tmem_base, long long* prof) {
+template <bool SCORES>
+__device__ void q_issuer(uint8_t* smem, uint64_t* bars, volatile int* abort_flag, int lane, uint32_t tmem_base, uint32_t dp, long long* prof) {
   const uint64_t dQDO = umma_desc_sw128(smem_u32(smem + OFF_QDO));
   const uint64_t dK = umma_desc_sw128(smem_u32(smem + OFF_K)), dV = umma_desc_sw128(smem_u32(smem + OFF_V));
   const uint64_t dKmn = umma_desc_sw128_mn_blocks(smem_u32(smem + OFF_K), TILE_BYTES);
-  constexpr uint32_t FULL = ROLE == 0 ? K_FULL : ROLE == 1 ? V_FULL : PDS_FULL;
+  const uint32_t FULL = !SCORES ? PDS_FULL : dp ? V_FULL : K_FULL;
   const SlotRec* recs = slot_recs(smem);
   Ring rr, rv; rr.init(NKS); rv.init(NVS);                // record and K stage; V stage
   Ring rg, rf; rg.init(NWG); rf.init(NWG);                // the slot's group (and dP region); the group of slot g - 3
   uint32_t sreg = 0, un = 0, g = 0;                       // S region; unit
-  bool pre_a = false, pre_b = ROLE != 1;                  // early probe results for the coming slot, and its flags
+  bool pre_a = false, pre_b = !SCORES || !dp;                 // early probe results for the coming slot, and its flags
   uint32_t pre_flags = 0;
   for (;; ++g) {
-    // role 0, 1: the tile has landed AND the region is free -- S: its group has read P, three slots ago; dP: dQ has consumed the
-    // dS in it, four slots ago; role 2: dS is written
-    const uint32_t st = ROLE == 0 ? rr.st : ROLE == 1 ? rv.st : rg.st, ph = ROLE == 0 ? rr.ph : ROLE == 1 ? rv.ph : rg.ph;
-    if (lane == 0 && ROLE == 0) GCA_TRACE_BUF(prof, 0, g);
-    if (!mbar_wait_warp2_probed(&bars[FULL + st], ph, pre_a, &bars[ROLE == 0 ? PDS_FULL + rf.st : DP_FREE + rg.st], ROLE == 0 ? rf.ph : rg.ph ^ 1,
+    // S, dP: the tile has landed AND the region is free -- S: its group has read P, three slots ago; dP: dQ has consumed the
+    // dS in it, four slots ago; dQ: dS is written
+    const uint32_t st = !SCORES ? rg.st : dp ? rv.st : rr.st, ph = !SCORES ? rg.ph : dp ? rv.ph : rr.ph;
+    if (!mbar_wait_warp2_probed(&bars[FULL + st], ph, pre_a, &bars[dp ? DP_FREE + rg.st : PDS_FULL + rf.st], dp ? rg.ph ^ 1 : rf.ph,
                                 pre_b, abort_flag)) break;
-    if (ROLE == 0 && g >= NS) rf.next();
+    if (SCORES && g >= NS) rf.next();
     if (!pre_a) pre_flags = recs[rr.st].flags;
     const uint32_t flags = __shfl_sync(0xffffffffu, pre_flags, 0);
     if (flags & REC_END) break;
     const uint32_t ub = un & 1, uph = (un >> 1) & 1;
     const uint32_t kt1 = (flags & REC_SHARE) ? 0u : TILE16;            // head B's K / V tile inside the stage
     if (flags & REC_FIRST) {
-      if (!mbar_wait_warp(&bars[ROLE != 2 ? QDO_FULL + ub : ACC_EMPTY], ROLE != 2 ? uph : ub ^ 1, abort_flag, lane)) break;
+      if (!mbar_wait_warp(&bars[SCORES ? QDO_FULL + ub : ACC_EMPTY], SCORES ? uph : ub ^ 1, abort_flag, lane)) break;
     }
-    if (lane == 0 && ROLE != 1) GCA_TRACE_BUF(prof, ROLE == 0 ? 3 : 5, g);
     tc_fence_after();
     // The next slot's barriers and flags, between the two heads' MMAs: the probes' round trip runs under the issue.
     auto probe = [&] {
       Ring nr = rr, nv = rv, ng = rg;
       nr.next(); nv.next(); ng.next();
-      pre_a = mbar_test_wait(&bars[FULL + (ROLE == 0 ? nr.st : ROLE == 1 ? nv.st : ng.st)], ROLE == 0 ? nr.ph : ROLE == 1 ? nv.ph : ng.ph);
-      if (ROLE == 0) pre_b = g + 1 < NS || mbar_test_wait(&bars[PDS_FULL + rf.st], rf.ph);
-      if (ROLE == 1) pre_b = mbar_test_wait(&bars[DP_FREE + ng.st], ng.ph ^ 1);
+      pre_a = mbar_test_wait(&bars[FULL + (!SCORES ? ng.st : dp ? nv.st : nr.st)], !SCORES ? ng.ph : dp ? nv.ph : nr.ph);
+      if (SCORES) pre_b = mbar_test_wait(&bars[dp ? DP_FREE + ng.st : PDS_FULL + rf.st], dp ? ng.ph ^ 1 : rf.ph) || (!dp && g + 1 < NS);
       if (pre_a) pre_flags = recs[nr.st].flags;
     };
-    if (ROLE != 2) {
-      const uint64_t a = dQDO + ub * 2 * PAIR16 + (ROLE == 0 ? 0u : PAIR16);          // Q pair | dO pair
-      const uint64_t bt = (ROLE == 0 ? dK : dV) + st * PAIR16;
-      const uint32_t d = tmem_base + (ROLE == 0 ? sreg : COL_DP + rg.st * 64);
+    if (SCORES) {
+      const uint64_t a = dQDO + ub * 2 * PAIR16 + dp * PAIR16;          // Q pair | dO pair
+      const uint64_t bt = (dp ? dV : dK) + st * PAIR16;
+      const uint32_t d = tmem_base + (dp ? COL_DP + rg.st * 64 : sreg);
 #pragma unroll
       for (int tl = 0; tl < 2; ++tl) {
         if (tl == 1) probe();
@@ -346,10 +344,9 @@ __device__ void q_issuer(uint8_t* smem, uint64_t* bars, volatile int* abort_flag
           umma_bf16_ss_elect(d + (tl ? LANE16 : 0u), a + tl * TILE16 + kk * STEP_K, bt + (tl ? kt1 : 0u) + kk * STEP_K,
                              IDESC_64, (uint32_t)(kk > 0));
       }
-      umma_commit_elect(&bars[(ROLE == 0 ? S_FULL : DP_FULL) + rg.st]);
-      if (ROLE == 1) umma_commit_elect(&bars[V_EMPTY + st]);
+      umma_commit_elect(&bars[(dp ? DP_FULL : S_FULL) + rg.st]);
+      if (dp) umma_commit_elect(&bars[V_EMPTY + st]);
       if (flags & REC_LAST) umma_commit_elect(&bars[QDO_EMPTY + ub]);    // expects both issuers' commits
-      if (lane == 0 && ROLE == 0) GCA_TRACE_BUF(prof, 2, g);
       if ((sreg += 64) == COL_DP) sreg = 0;
     } else {
       // dQ += dS K_k per head: A = dS from tensor memory (lane = query row, 8 columns per K step
@@ -367,7 +364,6 @@ __device__ void q_issuer(uint8_t* smem, uint64_t* bars, volatile int* abort_flag
       umma_commit_elect(&bars[DP_FREE + rg.st]);
       umma_commit_elect(&bars[K_EMPTY + rr.st]);        // the K tiles of this slot are free once dQ is done
       if (flags & REC_LAST) umma_commit_elect(&bars[ACC_FULL]);
-      if (lane == 0) GCA_TRACE_BUF(prof, 6, g);
     }
     if (flags & REC_LAST) ++un;
     rr.next();
@@ -553,9 +549,8 @@ bwd_q_tc_kernel(const __grid_constant__ BwdQParams p) {
   if (warp < 4 * NWG) q_worker(p, smem, bars, abort_flag, warp >> 2, warp & 3, lane, tmem_base);
   else if (warp == PROD_WARP) q_producer(p, smem, bars, abort_flag, lane);
   else if (warp >= WRITER_WARP) q_writer(p, smem, bars, abort_flag, warp & 3, lane, tmem_base);
-  else if (warp == ISSUE_S) q_issuer<0>(smem, bars, abort_flag, lane, tmem_base, p.prof);
-  else if (warp == ISSUE_DP) q_issuer<1>(smem, bars, abort_flag, lane, tmem_base, p.prof);
-  else if (warp == ISSUE_DQ) q_issuer<2>(smem, bars, abort_flag, lane, tmem_base, p.prof);
+  else if (warp == ISSUE_S || warp == ISSUE_DP) q_issuer<true>(smem, bars, abort_flag, lane, tmem_base, (uint32_t)(warp - ISSUE_S), p.prof);
+  else if (warp == ISSUE_DQ) q_issuer<false>(smem, bars, abort_flag, lane, tmem_base, 0u, p.prof);
   if (p.beside_index) pdl_wait();        // the index is complete before this kernel is
   tc_fence_before();
   __syncthreads();

@@ -72,20 +72,26 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
 #ifndef GCA_WAIT_LIMIT
 #define GCA_WAIT_LIMIT (1u << 22)
 #endif
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
-                                                  uint32_t limit = GCA_WAIT_LIMIT) {
-#ifndef GCA_NO_FAST_PROBE
-  if (mbar_test_wait(bar, parity)) return true;
-#endif
-  for (uint32_t i = 0; i < limit; ++i) {
+// GCA_WAIT_OUT_OF_LINE (a file's choice, before this header): the polling loop is a function of its own.  All roles of a kernel share an instruction cache
+// that their code does not fit, so a loop less at every wait can be worth the call behind a failed first probe.
+__device__ __forceinline__ bool mbar_poll(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  for (uint32_t i = 0; i < GCA_WAIT_LIMIT; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
-#ifdef GCA_WAIT_SLEEP_NS
-    __nanosleep(GCA_WAIT_SLEEP_NS);
-#endif
     if ((i & 255u) == 255u && *abort_flag) return false;
   }
   *abort_flag = 1;
   return false;
+}
+#ifdef GCA_WAIT_OUT_OF_LINE
+static __device__ __noinline__ bool mbar_poll_far(uint64_t* bar, uint32_t parity, volatile int* abort_flag) { return mbar_poll(bar, parity, abort_flag); }
+#endif
+__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  if (mbar_test_wait(bar, parity)) return true;
+#ifdef GCA_WAIT_OUT_OF_LINE
+  return mbar_poll_far(bar, parity, abort_flag);
+#else
+  return mbar_poll(bar, parity, abort_flag);
+#endif
 }
 
 // Warp-level forms.  An mbarrier is one shared-memory word: 128 threads arriving on it, or 128
