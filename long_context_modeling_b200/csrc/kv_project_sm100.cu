@@ -320,7 +320,8 @@ kv_project_append_kernel(const __grid_constant__ ProjParams p) {
         return o;
       };
       // Passes of 32 columns (or the last 16) of one small loop body.  A pass's residual is asked for two passes ahead, that of the first two
-      // before the accumulator is waited for.
+      // before the accumulator is waited for.  Not by pairs: they have a residual behind a norm alone, and the append pays for the code (8 x 60 chunks,
+      // 512 wide, 36.2 -> 36.8 us).
       const int cols = min(BN, p.ncols - tn * BN);       // not every width divides every matrix: the last tile may be a narrow one
       const int c_begin = half * (BN / 2), c_end = min(cols, c_begin + BN / 2);
       const bool ce = p.nmat == 1 && p.ce_part;
@@ -333,7 +334,7 @@ kv_project_append_kernel(const __grid_constant__ ProjParams p) {
         ask_c += 32;
       };
       uint4 rr[4] = {}, rr_next[4];
-      if (with_res) { ask(rr); ask(rr_next); }
+      if (!PAIR && with_res) { ask(rr); ask(rr_next); }
       ok = mbar_wait_bounded(&bars[ACC_FULL + ab], (tcount >> 1) & 1, abort_flag);
       if (NORM) ok = ok && mbar_wait_bounded(&bars[SCALE_FULL + ab], (tcount >> 1) & 1, abort_flag);
       if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
@@ -380,6 +381,7 @@ kv_project_append_kernel(const __grid_constant__ ProjParams p) {
       for (int c0 = c_begin; c0 < c_end; c0 += 32) {
         uint32_t v[32], w[16];
         const bool two = c0 + 16 < c_end;
+        if (PAIR && with_res) { ask_c = c0; ask(rr); }
         tmem_ld_32x32b_x32(tlane + ab * ACC_COLS + c0, v);
         const uint32_t rw[16] = {rr[0].x, rr[0].y, rr[0].z, rr[0].w, rr[1].x, rr[1].y, rr[1].z, rr[1].w,
                                  rr[2].x, rr[2].y, rr[2].z, rr[2].w, rr[3].x, rr[3].y, rr[3].z, rr[3].w};
@@ -392,7 +394,7 @@ kv_project_append_kernel(const __grid_constant__ ProjParams p) {
         for (int i = 0; i < 16; ++i)
           w[i] = pack_bf16x2(fmaf(__uint_as_float(v[2 * i]), sc, __uint_as_float(rw[i] << 16)),
                              fmaf(__uint_as_float(v[2 * i + 1]), sc, __uint_as_float(rw[i] & 0xffff0000u)));
-        if (with_res) {
+        if (!PAIR && with_res) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) rr[i] = rr_next[i];
           ask(rr_next);
