@@ -25,8 +25,8 @@
 // Every wait is bounded (GCA_STATUS_TIMEOUT on expiry).  No atomics on results: they are bit-reproducible.
 // Infinities, NaN, sums that overflow on the way and tiles of tiny numbers are outside the range of all this: such units are found by their outputs
 // and done over again with multiply-adds (see `outside`), with the results that the CUDA-core kernels have always had.
-// 2 x 64 chunks x 12 heads, top-8: forward 111 us, q-major 165, kv-major 205 (CUDA cores: 355, 481, 588), the whole step with inputs
-// that are not in L2 545 us (1,425).  2-norm against 64 bits, N(0,1): o 2.2e-7 (4.4e-7), dq 2.8e-7 (4.7e-7), dk 3.0e-7 (6.9e-7), dv 2.6e-7
+// 2 x 64 chunks x 12 heads, top-8: forward 110 us, q-major 154, kv-major 200 (CUDA cores: 355, 481, 588), the whole step with inputs
+// that are not in L2 515 us (1,425).  2-norm against 64 bits, N(0,1): o 2.2e-7 (4.4e-7), dq 2.8e-7 (4.7e-7), dk 3.0e-7 (6.9e-7), dv 2.6e-7
 // (6.8e-7), dw 2.6e-7 (3.3e-7); the largest errors over the rms, as means over 63 drawn sizes: o 4.3e-6 (7.5e-6), dq 5.9e-6 (8.9e-6), dk 7.0e-6
 // (2.0e-5), dv 6.7e-6 (1.8e-5), dw 8.6e-7 (1.1e-6), a single size now and then the other way round.  With q x 10 still closer in all five but
 // dv (1.3e-6, 1.2e-6), q x 100: dq 6.7e-5 (7.6e-5), dv 1.3e-5 (6.9e-6): the kv-major pass's scores are not the forward's to the last bit.
@@ -194,10 +194,11 @@ __device__ __forceinline__ void tile_ready(uint64_t* bar, int lane) {
 
 // ---------------------------------------------------------------- products (all lanes of the issuing warp)
 // D = A B with A the operand in tensor-memory region `a`: (b0 | b1) b1', (b0 | b1) b2', b2 b0', (b0 | b1) b0', in this order: the first
-// writes both halves, the large one comes last.  Rolled, because all roles share an instruction cache.
+// writes both halves, the large one comes last.  Unrolled: an instruction is 32 cycles of the pipe, and a loop around four of them did not keep up (q-major 166 us
+// against 154, kv-major 205 / 200, forward 114 / 112; around each one 202, 235, 142; as a function 187, 222, 130; with one lane elected for all 16 161, 209, 121).
 template <bool MN>
 __device__ __forceinline__ void product_ts(uint32_t d, uint32_t a, uint64_t b) {
-#pragma unroll 1
+#pragma unroll
   for (int q = 0; q < 4; ++q) {
     const uint32_t aq = a + (q == 2 ? 16u : 0u);
     const uint64_t bq = b + (q == 0 ? PIECE16 : q == 1 ? 2 * PIECE16 : 0u);
@@ -209,7 +210,7 @@ __device__ __forceinline__ void product_ts(uint32_t d, uint32_t a, uint64_t b) {
 // D = A B^T, both tiles in shared memory, K-major, 64 rows (lanes 0-15): nibble q of PA, PB is the piece.
 __device__ __forceinline__ void product_ss(uint32_t d, uint64_t a, uint64_t b) {
   constexpr uint32_t PA = 0x001102u, PB = 0x010120u;
-#pragma unroll 1
+#pragma unroll
   for (int q = 0; q < 6; ++q) {
     const uint64_t aq = a + ((PA >> (4 * q)) & 15u) * PIECE16, bq = b + ((PB >> (4 * q)) & 15u) * PIECE16;
 #pragma unroll
