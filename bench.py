@@ -34,7 +34,7 @@ N_SEQ, CHUNKS, HEADS, TOPK, HEAD_DIM, CHUNK = 8, 256, 12, 8, 64, 64
 FWD_FLOP_PER_SLOT = 4 * CHUNK * CHUNK * HEAD_DIM          # QK^T + PV for one (query chunk, head, slot)
 FWD_BWD_FACTOR = 3.5                                      # backward counted as 2.5 x forward (ltriton/gca.py:1091-1092)
 # dram__bytes_read.sum + dram__bytes_write.sum per launch, ncu capture of `--n-seq 2` (see profiles/)
-TRAFFIC_2SEQ = {"fwd": 140.7e6 + 47.7e6, "bwd_kv": 256.5e6 + 69.0e6, "bwd_q": 211.5e6 + 81.9e6}
+TRAFFIC_2SEQ = {"fwd": 139.6e6 + 47.9e6, "bwd_kv": 254.2e6 + 72.5e6, "bwd_q": 211.5e6 + 84.5e6}
 
 
 def valid_slots(chunks: int, topk: int) -> int:

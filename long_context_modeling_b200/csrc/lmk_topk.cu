@@ -146,7 +146,7 @@ __device__ __forceinline__ void select_batch(unsigned long long& mine, unsigned 
 // memory; list l (one per head, or the only one) is kept by warp l % 16, which merges
 // the 128 scores into it (select_batch): one list per block instead of one per warp to merge at the end, and
 // no list code in the scoring loop (per head it was 12 lists in every warp, each with a serial insertion: 60 us for
-// 2 x 16,411 landmarks, now 16; 262,144 landmarks, one list: 68 -> 63 us = 6.3 TB/s for the scan alone, 69.4 us = 5.8 TB/s with its
+// 2 x 16,411 landmarks, now 15.5 with its merge; 262,144 landmarks, one list: 66.2 us = 6.1 TB/s with its
 // merge).
 constexpr int SPLIT_ROWS = 64, STREAM_WARPS = 16;                // rows that a block takes at least
 template <int NP> constexpr int RING_ROWS = NP > 3 ? 6 : 8;       // 196 KB per SM
