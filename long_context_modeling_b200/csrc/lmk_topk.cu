@@ -188,7 +188,11 @@ __global__ void __launch_bounds__(STREAM_WARPS * 32, 1)
 lmk_stream_kernel(ScanParams p, FinalParams fin) {
   constexpr int RING = RING_ROWS<NP>, U = ROWS_AT_ONCE<NP>, NL = PER_HEAD ? NP * 4 : 1, MINE = (NL + STREAM_WARPS - 1) / STREAM_WARPS, ROW_BYTES = NP * 512;
   extern __shared__ __align__(16) unsigned char ring_all[];            // [STREAM_WARPS][RING][ROW_BYTES]
-  __shared__ float score[2][NL][BATCH];
+  // A store's four heads in banks of their own (2 x 16,411 landmarks 15.2 -> 14.7 us).  The arrays stay a multiple of 128 bytes: the ring behind them would
+  // not lie on the lines that are copied into it otherwise (262,144 landmarks, one list: 64.9 -> 67.5).
+  constexpr int PITCH = PER_HEAD ? BATCH + 4 : BATCH;
+  static_assert(2 * NL * PITCH * 4 % 128 == 0, "alignment of the ring");
+  __shared__ float score[2][NL][PITCH];
   __shared__ unsigned long long note[NL < STREAM_WARPS ? NL : STREAM_WARPS][MAXK];
   pdl_trigger();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -241,7 +245,7 @@ lmk_stream_kernel(ScanParams p, FinalParams fin) {
   const int batches = (e_hi - e_lo + BATCH - 1) / BATCH;
   int slot = 0;
   for (int b = 0; b < batches; ++b) {
-    float (*sc)[BATCH] = score[b & 1];
+    float (*sc)[PITCH] = score[b & 1];
 #pragma unroll
     for (int i = 0; i < BATCH / STREAM_WARPS; i += U) {
       if (e_lo + b * BATCH + i * STREAM_WARPS >= e_hi) break;
