@@ -89,9 +89,10 @@ __device__ __noinline__ TopList select_64(unsigned long long mine, unsigned long
 }
 
 constexpr int BATCH = 128;
-// The same for a batch of 128 (o[i]: id id0 + 32 i + lane).  One or two that beat the list's K-th score are inserted; more, and the K best
-// come out by K warp-wide maxima of the 32-bit scores: whoever holds the maximum strikes it out and notes its key, which is all that the
-// next round waits for (~45 cycles; with the owner found by votes and its key shuffled to its place ~110, and an insertion as much).
+// The same for a batch of 128 (o[i]: id id0 + 32 i + lane).  Fewer than K that beat the list's K-th score are inserted, one after the other; K or more, and
+// the K best come out by K warp-wide maxima of the 32-bit scores: whoever holds the maximum strikes it out and notes its key, which is all that the
+// next round waits for (with the owner found by votes and its key shuffled to its place a round takes more than twice as long).  K rounds from the third
+// of a batch on cost 32 x 7,200 landmarks of 1,024, per head, K = 32 119 us (now 90), 32 x 7,200 of 768 93 (69), 4 x 37,000 57.6 (47.4), K = 16 45.2 (43.3).
 // Equal scores are struck out together: more struck out than rounds, and the batch is done over again the careful way.
 __device__ __forceinline__ void select_batch(unsigned long long& mine, unsigned long long& kth, const unsigned o[4], unsigned id0, int K, int lane,
                                              unsigned long long* note) {
@@ -101,7 +102,7 @@ __device__ __forceinline__ void select_batch(unsigned long long& mine, unsigned 
 #pragma unroll
   for (int i = 0; i < 4; ++i) { b[i] = __ballot_sync(0xffffffffu, o[i] > th); found += __popc(b[i]); }
   if (found == 0) return;
-  if (found <= 2) {                                          // lower ids first; what the first one pushes below the K-th place stays there
+  if (found < max(K, 3)) {                                   // lower ids first; what the first ones push below the K-th place stays there
 #pragma unroll
     for (int i = 0; i < 4; ++i)
       for (unsigned m = b[i]; m; m &= m - 1) {

@@ -130,6 +130,27 @@ def test_equal_scores_in_every_batch_and_list(lcm, d, head_dim, splits):
     check(res, oracle_rows(lq, lk, k, q_pos0=e - 2, head_dim=head_dim))
 
 
+@pytest.mark.parametrize("head_dim", [0, 64])
+@pytest.mark.parametrize("k", [1, 2, 3, 4, 16, 31, 32])
+def test_batches_that_change_a_list_by_any_number_of_entries(lcm, k, head_dim):
+    """From batch to batch 0 to 128 scores beat all that the list holds, K - 1, K and K + 1 among them: inserted one by one or taken by maxima.  Scores are
+    the sums of two products, so no two of them are equal; the last batch is a short one."""
+    d, counts = 512, [5, 0, 1, 2, 3, k - 1, k, k + 1, 128, 1, 20]
+    g = torch.Generator().manual_seed(k)
+    lk = torch.zeros(1, 128 * len(counts), d)
+    fine = torch.randperm(lk.shape[1], generator=g)
+    for b, m in enumerate(counts):
+        at = 128 * b + torch.randperm(128, generator=g)
+        lk[0, at, 0] = torch.where(torch.arange(128) < m, 1.0 + b, -1.0 - b)
+    lk[0, :, 1] = (fine % 128) / 128.0
+    lk[0, :, 2] = (fine // 128) / 4096.0
+    lk = lk[:, :-90].repeat_interleave(d // 64 if head_dim else 1, 0)
+    lk = (torch.stack([torch.roll(lk[h], 64 * h, 1) for h in range(lk.shape[0])]).sum(0, keepdim=True) if head_dim else lk).bfloat16()
+    lq = torch.ones(1, 1, d).bfloat16()
+    res = lcm.lmk_score_topk(lq.cuda(), lk.cuda(), k, q_pos0=lk.shape[1], head_dim=head_dim, splits=1)
+    check(res, oracle_rows(lq, lk, k, q_pos0=lk.shape[1], head_dim=head_dim))
+
+
 def test_noise_selects_but_weights_stay_noise_free(lcm):
     """Training: Gumbel noise perturbs the selection only (DRT.py:616-626)."""
     n, c, d, k = 2, 20, 768, 4
