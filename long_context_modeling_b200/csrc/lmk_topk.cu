@@ -488,80 +488,106 @@ lmk_merge_rows_kernel(FinalParams p) {
   emit_row(p, row, merge_heads(p.K, lane < p.lists, lane, [&](int i) { return src[i]; }), lane);
 }
 
-// Many lists per row (a long cache scanned by every SM): one block per row, no serial insertion.  All lists come to shared memory in one trip where
-// they fit.  Up to 160 of them are then merged by one warp, five a lane: K warp-wide maxima of the heads' 32-bit scores, whose owner notes the
-// key and moves on (equal scores move on together: more noted than rounds, and the general way does it).
-// In general an entry e of a list can be among the K best only if fewer than K - e list heads are better than its own; so the heads are ranked
-// by counting, the K best lists are lined up by rank, and their K (K + 1) / 2 possible entries are ranked by counting again.
-// 296 lists, K = 8: 12.9 us of warp-serial insertions before.
-// 18 KB and 128 threads: a block finds its place beside one of the scan (192 KB + 15, 512 threads of up to 112 registers) and is there when the scan
-// ends.  With 256 threads it did not: 1 x 32,768 landmarks per head on all 148 SMs 20.4 us, on 128 of them 16.1.
-constexpr int RANK_LISTS = 1024, RANK_KEYS = 1664, RANK_THREADS = 128, WARP_LISTS = 160;
+// Many lists per row (a long cache scanned by every SM), up to 160: one block per row.  All keys come to shared memory, 1,664 of them a trip, then one warp
+// merges the lists, five a lane, by K warp-wide maxima of the heads' 32-bit scores: whose head it is notes the key and moves on.
+// Equal scores move on together: more noted than rounds, and the warp starts again with the lowest id of each maximum (a second maximum a round).
+// 128 threads and 8 bytes a key: up to a width of 768 and K = 10 a block finds its place beside one of the scan (192 KB + 15, 512 threads of up to 112
+// registers) and is there when the scan ends.  With 256 threads it did not: 1 x 32,768 landmarks per head on all 148 SMs 20.4 us, on 128 of them 16.1.  Wider
+// rows and longer lists leave it no place, and it starts when blocks of the scan have left; several of a launch then share an SM, so they must be
+// short: ranked by counting as below, K = 32 took 30 us of 128 threads (20 of 256).  1 x 7,400 x 768, K = 16 / 32: 10.8 / 31.2 us, now 9.6 / 13.5;
+// 1 x 266,400 per head, K = 32, x 768 97 (now 78), x 1,024 182 (101).
+constexpr int WARP_LISTS = 160, MERGE_THREADS = 128, MERGE_LOADS = 13;
 
-__global__ void __launch_bounds__(RANK_THREADS)
+__global__ void __launch_bounds__(MERGE_THREADS)
+lmk_warp_merge_kernel(FinalParams p) {
+  extern __shared__ unsigned long long all[];                            // [lists][K]
+  __shared__ unsigned long long best[MAXK];
+  const int tid = threadIdx.x, K = p.K, keys = p.lists * K;
+  const unsigned long long* src = p.keys + (long long)blockIdx.x * p.P;
+  if (tid < MAXK) best[tid] = 0ull;
+  pdl_trigger();
+  pdl_wait();
+  for (int i0 = tid; i0 < keys; i0 += MERGE_LOADS * MERGE_THREADS) {
+    unsigned long long v[MERGE_LOADS];
+#pragma unroll
+    for (int i = 0; i < MERGE_LOADS; ++i) v[i] = i0 + i * MERGE_THREADS < keys ? src[i0 + i * MERGE_THREADS] : 0ull;
+#pragma unroll
+    for (int i = 0; i < MERGE_LOADS; ++i)
+      if (i0 + i * MERGE_THREADS < keys) all[i0 + i * MERGE_THREADS] = v[i];
+  }
+  __syncthreads();
+  if (tid >= 32) return;
+  constexpr int MINE = WARP_LISTS / 32;
+  unsigned h[MINE];
+  int at[MINE];
+  auto start = [&] {
+#pragma unroll
+    for (int i = 0; i < MINE; ++i) {
+      at[i] = (tid + 32 * i) * K;
+      h[i] = tid + 32 * i < p.lists ? (unsigned)(all[at[i]] >> 32) : 0u;
+    }
+  };
+  auto highest = [&] {
+    unsigned top = h[0];
+#pragma unroll
+    for (int i = 1; i < MINE; ++i) top = max(top, h[i]);
+    return __reduce_max_sync(0xffffffffu, top);
+  };
+  auto take = [&](int i, int k) {                                        // the head of this lane's list i is the k-th best
+    best[k] = all[at[i]];
+    ++at[i];
+    h[i] = at[i] < (tid + 32 * i + 1) * K ? (unsigned)(all[at[i]] >> 32) : 0u;
+  };
+  start();
+  int k = 0, noted = 0;
+  for (; k < K; ++k) {
+    const unsigned m = highest();
+    if (m == 0u) break;
+#pragma unroll
+    for (int i = 0; i < MINE; ++i)
+      if (h[i] == m) { take(i, k); ++noted; }
+  }
+  if (__reduce_add_sync(0xffffffffu, noted) != k) {
+    __syncwarp();
+    start();
+    for (k = 0; k < K; ++k) {
+      const unsigned m = highest();
+      if (m == 0u) break;
+      unsigned low = 0u;                                                 // ~id
+#pragma unroll
+      for (int i = 0; i < MINE; ++i)
+        if (h[i] == m) low = max(low, (unsigned)all[at[i]]);
+      const unsigned first = __reduce_max_sync(0xffffffffu, low);
+#pragma unroll
+      for (int i = 0; i < MINE; ++i)
+        if (h[i] == m && (unsigned)all[at[i]] == first) take(i, k);
+    }
+    if (tid >= k) best[tid] = 0ull;
+  }
+  __syncwarp();
+  emit_row(p, blockIdx.x, tid < K ? best[tid] : 0ull, tid);
+}
+
+// More lists than that: no serial insertion either.  An entry e of a
+// list can be among the K best only if fewer than K - e list heads are better than its own; so the heads are ranked by counting,
+// the K best lists are lined up by rank, and their K (K + 1) / 2 possible entries are ranked by counting again.
+// 296 lists, K = 8: 12.9 us of warp-serial insertions before.
+constexpr int RANK_LISTS = 1024;
+
+__global__ void __launch_bounds__(FIN_WARPS * 32)
 lmk_rank_merge_kernel(FinalParams p) {
-  __shared__ __align__(16) unsigned long long heads[RANK_KEYS];          // the heads (padded to an even number), then all keys if they fit
-  __shared__ int by_rank[MAXK], equal;
+  __shared__ __align__(16) unsigned long long heads[RANK_LISTS];
+  __shared__ int by_rank[MAXK];
   __shared__ unsigned long long cand[MAXK * (MAXK + 1) / 2 + 1], best[MAXK];
   const int tid = threadIdx.x, lists = p.lists, K = p.K;
   const int padded = (lists + 1) & ~1;
   const unsigned long long* src = p.keys + (long long)blockIdx.x * p.P;
-  static_assert(RANK_LISTS <= RANK_KEYS, "the heads fit");
-  const bool whole = padded + lists * K <= RANK_KEYS;
-  unsigned long long* all = heads + padded;
   if (tid < MAXK) { by_rank[tid] = -1; best[tid] = 0ull; }
   pdl_trigger();
   pdl_wait();
-  if (whole) {
-    constexpr int LOADS = RANK_KEYS / RANK_THREADS;
-    unsigned long long v[LOADS];
-#pragma unroll
-    for (int i = 0; i < LOADS; ++i) v[i] = tid + i * RANK_THREADS < lists * K ? src[tid + i * RANK_THREADS] : 0ull;
-#pragma unroll
-    for (int i = 0; i < LOADS; ++i)
-      if (tid + i * RANK_THREADS < lists * K) all[tid + i * RANK_THREADS] = v[i];
-    __syncthreads();
-    if (lists <= WARP_LISTS) {
-      if (tid < 32) {
-        constexpr int MINE = WARP_LISTS / 32;
-        unsigned h[MINE];
-        int at[MINE];
-#pragma unroll
-        for (int i = 0; i < MINE; ++i) {
-          at[i] = (tid + 32 * i) * K;
-          h[i] = tid + 32 * i < lists ? (unsigned)(all[at[i]] >> 32) : 0u;
-        }
-        int k = 0, noted = 0;
-        for (; k < K; ++k) {
-          unsigned top = h[0];
-#pragma unroll
-          for (int i = 1; i < MINE; ++i) top = max(top, h[i]);
-          const unsigned m = __reduce_max_sync(0xffffffffu, top);
-          if (m == 0u) break;
-#pragma unroll
-          for (int i = 0; i < MINE; ++i)
-            if (h[i] == m) {
-              best[k] = all[at[i]];
-              ++noted;
-              ++at[i];
-              h[i] = at[i] < (tid + 32 * i + 1) * K ? (unsigned)(all[at[i]] >> 32) : 0u;
-            }
-        }
-        const bool distinct = __reduce_add_sync(0xffffffffu, noted) == k;
-        __syncwarp();
-        if (distinct) emit_row(p, blockIdx.x, tid < K ? best[tid] : 0ull, tid);
-        else best[tid] = 0ull;
-        if (tid == 0) equal = !distinct;
-      }
-      __syncthreads();
-      if (!equal) return;
-    }
-    for (int i = tid; i < padded; i += RANK_THREADS) heads[i] = i < lists ? all[i * K] : 0ull;
-  } else {
-    for (int i = tid; i < padded; i += RANK_THREADS) heads[i] = i < lists ? src[(long long)i * K] : 0ull;
-  }
+  for (int i = tid; i < padded; i += FIN_WARPS * 32) heads[i] = i < lists ? src[(long long)i * K] : 0ull;
   __syncthreads();
-  for (int i = tid; i < lists; i += RANK_THREADS) {
+  for (int i = tid; i < lists; i += FIN_WARPS * 32) {
     const unsigned long long mine = heads[i];
     if (mine == 0ull) continue;
     int rank = 0;
@@ -574,12 +600,12 @@ lmk_rank_merge_kernel(FinalParams p) {
   __syncthreads();
   // candidate (r, e), r + e < K, at position e of the list of rank r
   const int total = K * (K + 1) / 2;
-  for (int i = tid; i < K * K; i += RANK_THREADS) {
+  for (int i = tid; i < K * K; i += FIN_WARPS * 32) {
     const int r = i / K, e = i - r * K;
-    if (r + e < K) cand[r * K - r * (r - 1) / 2 + e] = by_rank[r] < 0 ? 0ull : whole ? all[by_rank[r] * K + e] : src[(long long)by_rank[r] * K + e];
+    if (r + e < K) cand[r * K - r * (r - 1) / 2 + e] = by_rank[r] >= 0 ? src[(long long)by_rank[r] * K + e] : 0ull;
   }
   __syncthreads();
-  for (int i = tid; i < total; i += RANK_THREADS) {
+  for (int i = tid; i < total; i += FIN_WARPS * 32) {
     const unsigned long long mine = cand[i];
     if (mine == 0ull) continue;
     int rank = 0;
@@ -822,7 +848,9 @@ int launch_lmk_score_topk(const LmkTopkArgs& a, void* scratch, int sms, cudaStre
   // a warp per row up to 32 lists, a block per row beyond
   if (splits <= 32)
     return (int)launch_dependent(lmk_merge_rows_kernel, dim3((unsigned)((rows + FIN_WARPS - 1) / FIN_WARPS)), dim3(FIN_WARPS * 32), 0, stream, fp);
-  if (splits <= RANK_LISTS) return (int)launch_dependent(lmk_rank_merge_kernel, dim3((unsigned)rows), dim3(RANK_THREADS), 0, stream, fp);
+  if (splits <= WARP_LISTS)
+    return (int)launch_dependent(lmk_warp_merge_kernel, dim3((unsigned)rows), dim3(MERGE_THREADS), (size_t)splits * a.K * sizeof(unsigned long long), stream, fp);
+  if (splits <= RANK_LISTS) return (int)launch_dependent(lmk_rank_merge_kernel, dim3((unsigned)rows), dim3(FIN_WARPS * 32), 0, stream, fp);
   lmk_finalize_kernel<<<(unsigned)rows, FIN_WARPS * 32, 0, stream>>>(fp);
   return (int)cudaGetLastError();
 }

@@ -151,6 +151,21 @@ def test_batches_that_change_a_list_by_any_number_of_entries(lcm, k, head_dim):
     check(res, oracle_rows(lq, lk, k, q_pos0=lk.shape[1], head_dim=head_dim))
 
 
+@pytest.mark.parametrize("splits", [33, 64, 65, 148, 160, 161])
+@pytest.mark.parametrize("k", [1, 10, 13, 27, 32])
+def test_merge_of_many_lists(lcm, splits, k):
+    """33 to 160 lists a row are merged by a warp, in one to four trips of its block; more are ranked by counting.  Full lists and lists that end before K,
+    scores that all differ and scores that are each held by landmarks of many lists, one row and a row per head."""
+    g = torch.Generator().manual_seed(splits + k)
+    for rows, distinct, head_dim in [(40, 0, 0), (40, 6, 0), (9, 0, 64), (9, 40, 64), (2, 3, 0)]:
+        e = rows * splits - 1
+        lq, lk = cases.landmark_case(splits, 1, 1, e, d=256)
+        if distinct:
+            lk = lk[:, :distinct][:, torch.randint(0, distinct, (e,), generator=g)]
+        res = lcm.lmk_score_topk(lq.cuda(), lk.cuda(), k, q_pos0=e, head_dim=head_dim, splits=splits)
+        check(res, oracle_rows(lq, lk, k, q_pos0=e, head_dim=head_dim))
+
+
 def test_noise_selects_but_weights_stay_noise_free(lcm):
     """Training: Gumbel noise perturbs the selection only (DRT.py:616-626)."""
     n, c, d, k = 2, 20, 768, 4
