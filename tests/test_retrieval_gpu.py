@@ -166,6 +166,19 @@ def test_merge_of_many_lists(lcm, splits, k):
         check(res, oracle_rows(lq, lk, k, q_pos0=e, head_dim=head_dim))
 
 
+@pytest.mark.parametrize("d,head_dim", [(768, 0), (776, 0), (1024, 64)])
+@pytest.mark.parametrize("n,e", [(1, 9473), (1, 19000), (4, 2369), (4, 4737), (9, 1025), (32, 257)])
+def test_ranges_in_steps_of_the_rows_taken_at_once(lcm, n, e, d, head_dim):
+    """Ranges as the library cuts them, just past one, two and four steps of a block (of 64 rows, of 32 beyond a width of 768), with as many lists as a warp
+    merges and one more: the result does not depend on the cut."""
+    lq, lk = cases.landmark_case(e, n, 1, e, d=d)
+    lq, lk = lq.cuda(), lk.cuda()
+    got = lcm.lmk_score_topk(lq, lk, 16, q_pos0=e, head_dim=head_dim)
+    one = lcm.lmk_score_topk(lq, lk, 16, q_pos0=e, head_dim=head_dim, splits=1)
+    assert torch.equal(got.indices, one.indices) and torch.equal(got.scores, one.scores) and torch.equal(got.weights, one.weights)
+    check(lcm.Retrieval(*(t[:1] for t in got)), oracle_rows(lq[:1].cpu(), lk[:1].cpu(), 16, q_pos0=e, head_dim=head_dim))
+
+
 def test_noise_selects_but_weights_stay_noise_free(lcm):
     """Training: Gumbel noise perturbs the selection only (DRT.py:616-626)."""
     n, c, d, k = 2, 20, 768, 4
