@@ -19,7 +19,7 @@
 // weight rows: per product a third less shared-memory and L2 traffic than 128 x 256, and power is what a large
 // product is bound by (SM clock 1.3-1.6 GHz of 1.97 within milliseconds).  8 x 260 chunks x 64 rows, 768 -> 2 x 768, as the call with the
 // allocation of its cache: 252 us after a rest, 289 in a row; cuBLAS, in the same run, 285 / 294 us for the bare product (with
-// 128 x 256 tiles in place of pairs the call took 7 % more).  Other products take the width of 64, 128, 192 or 256 columns
+// 128 x 256 tiles in place of pairs the call took 7 % more).  Smaller products take the width of 64, 128, 192 or 256 columns
 // whose waves cost least: 6,912 rows 768 -> 768 on 148 SMs are 162 tiles of 256 columns (two waves, the second nearly
 // empty) but 216 of 192: 33 -> 19 us.
 //
@@ -320,8 +320,7 @@ kv_project_append_kernel(const __grid_constant__ ProjParams p) {
         return o;
       };
       // Passes of 32 columns (or the last 16) of one small loop body.  A pass's residual is asked for two passes ahead, that of the first two
-      // before the accumulator is waited for.  Not by pairs: they have a residual behind a norm alone, and the append pays for the code (8 x 60 chunks,
-      // 512 wide, 36.2 -> 36.8 us).
+      // before the accumulator is waited for.  Not by pairs, whose code the append shares and pays for (8 x 60 chunks, 512 wide, 36.2 -> 36.8 us).
       const int cols = min(BN, p.ncols - tn * BN);       // not every width divides every matrix: the last tile may be a narrow one
       const int c_begin = half * (BN / 2), c_end = min(cols, c_begin + BN / 2);
       const bool ce = p.nmat == 1 && p.ce_part;
@@ -509,22 +508,28 @@ namespace {
 // Which tile: the width, or the pairs, whose waves cost least.
 //   APPEND (and cross-entropy): in units of column-steps of one CTA a tile costs its width plus ~64 for its prologue and epilogue tail; wide pairs, which read
 // the least shared memory and L2 per product, ~48 (power is what a large product runs into).
-//   LINEAR, 768 -> 768 with a residual, us a wave: 64 columns 3.0, 128 3.8, 192 5.4, 256 7.0.  Pairs never better than 256 columns: 12,288 rows 19.3 us
-// against 18.8, 24,576 39.9 / 37.6, 133,120 197 / 185 (power limit), 1,024 -> 1,024 with 49,152 rows 111 / 108, 512 -> 512 with 65,536 67 / 56.
-//   NORM, us a wave: 4.6, 4.9, 5.7, 6.5.  Pairs need a launch before for the rows' factors: 12,288 rows 22.7 us against 16.8 with 256 columns, 133,120 200 / 178;
-// 512 -> 512, 6,912 rows 13.9 / 9.1.  From K = 1,024 and six waves on the factors in every column tile cost more: 24,576 rows 60.2 / 62.7, 49,152 109 / 119.
-enum class Product { APPEND, LINEAR, NORM };
+//   The linear products, in ns: once, a wave, and a wave's stage (64 of K), fitted to 1,400 to 1,600 sizes of each (300 to 131,072 rows, 256 to 4,096 columns,
+// K 128 to 4,096, x from memory).  The choice is the fastest of the five or within 0.3 % of it on average, 5 % in 99 of 100.  A residual costs pairs more, which read
+// it in the pass itself: 24,576 rows 2,048 -> 1,024 take pairs with one (74.7 us, 256 columns 91.4, 128 columns 98.8) and without, 12,288 rows 768 -> 2,048
+// only without (34.3, 256 columns 38.2; with a residual 51.5, 192 columns 47.2).  NORM: every column tile sums up the factors from the tiles of x again; for pairs a
+// launch before reads x (0.75 ns for 64 x 64 values of it): 24,576 rows 768 -> 4,096 121.1 us, 256 columns 144.4, but 3,072 -> 256 66.0 and 52.3.
+enum class Product { APPEND, PLAIN, RESIDUAL, NORM };
 struct TileChoice { int bn; bool pair; };
+struct TileCost { TileChoice tile; int once, wave, stage; };
+constexpr TileCost TILE_COSTS[4][5] = {
+    {{{256, true}, 0, 304, 0}, {{256, false}, 0, 320, 0}, {{192, false}, 0, 256, 0}, {{128, false}, 0, 192, 0}, {{64, false}, 0, 128, 0}},
+    {{{256, true}, 1100, 2440, 275}, {{256, false}, 600, 1610, 371}, {{192, false}, 500, 1110, 332}, {{128, false}, 110, 1050, 223}, {{64, false}, 0, 560, 197}},
+    {{{256, true}, 2510, 5180, 216}, {{256, false}, 690, 3910, 329}, {{192, false}, 450, 2390, 289}, {{128, false}, 0, 1700, 238}, {{64, false}, 40, 1010, 153}},
+    {{{256, true}, 2900, 2470, 318}, {{256, false}, 600, 2240, 398}, {{192, false}, 130, 1870, 377}, {{128, false}, 560, 1230, 361}, {{64, false}, 90, 750, 320}}};
 TileChoice choose_tile(Product product, long long rows64, int ncols, int k, int nmat, int sms) {
   auto ceil_div = [](long long a, long long b) { return (a + b - 1) / b; };
-  const long long pair_waves = ceil_div(ceil_div(rows64, 4) * ceil_div(ncols, 256) * nmat, sms / 2);
-  const bool pairs = product == Product::APPEND || (product == Product::NORM && k >= 1024 && pair_waves >= 6);
-  TileChoice best = {256, true};
-  long long best_cost = pairs ? pair_waves * (256 + (product == Product::NORM ? 240 : 48)) : -1;
-  for (int bn : {256, 192, 128, 64}) {
-    const int tile = product == Product::APPEND ? bn + 64 : product == Product::LINEAR ? (bn == 64 ? 120 : bn + 24) : bn + 260;
-    const long long cost = ceil_div(ceil_div(rows64, 2) * ceil_div(ncols, bn) * nmat, sms) * tile;
-    if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = {bn, false}; }
+  TileChoice best = {};
+  long long best_cost = -1;
+  for (const TileCost& c : TILE_COSTS[(int)product]) {
+    const long long tiles = ceil_div(rows64, c.tile.pair ? 4 : 2) * ceil_div(ncols, c.tile.bn) * nmat;
+    const long long factors = product == Product::NORM && c.tile.pair ? rows64 * (k / BK) * 3 / 4 : 0;
+    const long long cost = c.once + factors + ceil_div(tiles, c.tile.pair ? sms / 2 : sms) * (c.wave + (long long)(k / BK) * c.stage);
+    if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = c.tile; }
   }
   return best;
 }
@@ -649,7 +654,7 @@ int launch_linear(const LinearBatchedArgs& ba, float* norm_scratch, int sms, cud
   p.ce_part = nullptr; p.ce_target = nullptr; p.targets = nullptr;
   const long long blocks = per_batch * args.batches;
   if (blocks >= (1ll << 30)) return GCA_ERR_TOO_LARGE;
-  const TileChoice tile = choose_tile(norm_scratch ? Product::NORM : Product::LINEAR, blocks, a.N, a.K, 1, sms);
+  const TileChoice tile = choose_tile(norm_scratch ? Product::NORM : a.residual ? Product::RESIDUAL : Product::PLAIN, blocks, a.N, a.K, 1, sms);
   const bool norm = norm_scratch && !tile.pair;
   p.rms_eps = norm_eps;
   if (norm_scratch && !norm) {

@@ -458,6 +458,78 @@ def test_residual_read_ahead_and_norm_tiles(m, n, k):
     close(F.rmsnorm_linear(x, w, 1e-5), (xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + 1e-5)) @ w.float().t())
 
 
+def exactly(got, ref, k):
+    """Against 64 bits: the rounding to bf16, 2^-8 of the value, and float32: k terms of 2^-24 of the row's largest, the factor's 2^-22."""
+    bound = ref.abs() * (2.0 ** -8 + 2.0 ** -22) + k * 2.0 ** -24 * ref.abs().amax(-1, keepdim=True)
+    assert ((got.double() - ref).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("m,n,k", [(9100, 1808, 2048), (4100, 4112, 1024), (49153, 528, 4096), (24580, 1040, 2048)])
+def test_pairs_of_ctas_in_linear_products(m, n, k):
+    """Sizes whose tiles are shared by two CTAs, ragged in rows and in columns: row scale, residual in a place of its own and in the output's, and the norm
+    whose factors a launch before sums up, rows of very different sizes."""
+    need_gpu()
+    import long_context_modeling_b200 as lcm
+    from long_context_modeling_b200 import fused_ops as F
+    g = torch.Generator(device="cuda").manual_seed(m)
+    x = (torch.randn(m, k, generator=g, device="cuda") * torch.exp2(torch.randint(-20, 20, (m, 1), generator=g, device="cuda").float())).bfloat16()
+    w = (torch.randn(n, k, generator=g, device="cuda") * k ** -0.5).bfloat16()
+    r = torch.randn(m, n, generator=g, device="cuda").bfloat16()
+    sc = torch.rand(m, generator=g, device="cuda") + 0.5
+    product, factor = x.double() @ w.double().t(), torch.rsqrt(x.double().pow(2).mean(-1, keepdim=True) + 1e-5)
+    exactly(F.linear(x, w), product, k)
+    exactly(F.linear(x, w, row_scale=sc), product * sc.double()[:, None], k)
+    exactly(F.rmsnorm_linear(x, w, 1e-5), product * factor, k)
+    y = F.linear(x, w, row_scale=sc, residual=r)
+    # a sum that cancels keeps the error of its terms
+    ref, terms = product * sc.double()[:, None] + r.double(), (product * sc.double()[:, None]).abs() + r.double().abs()
+    assert ((y.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + (k * 2.0 ** -24) * terms.amax(-1, keepdim=True)).all()
+    there = r.clone()
+    F.linear(x, w, row_scale=sc, residual=there, out=there)
+    assert torch.equal(there, y) and lcm.read_status() == 0
+
+
+@pytest.mark.parametrize("norm", [False, True])
+@pytest.mark.parametrize("residual", [None, "own", "in place"])
+def test_pairs_of_ctas_over_batches(norm, residual):
+    """The C entries over blocks of rows with a gap between them, whose 256-row tiles hold rows of two blocks; lead rows get the residual alone, or zeros."""
+    need_gpu()
+    import ctypes as C
+    from long_context_modeling_b200 import _lib
+    b, m, n, k, lead = 3, 3033, 1808, 2048, 0 if norm else 64
+    g = torch.Generator(device="cuda").manual_seed(7)
+    x, w, r = ((torch.randn(*s, generator=g, device="cuda") * c).bfloat16() for s, c in (((b, m + 64, k), 3.0), ((n, k), k ** -0.5), ((b, m + 64, n), 1.0)))
+    out = r.clone() if residual == "in place" else torch.full_like(r, 7.0)
+    res = out if residual == "in place" else r if residual else None
+    a = _lib.LinearBatchedArgs()
+    o, esize = a.one, 2
+    o.x, o.w, o.out = x.data_ptr() + 64 * k * esize, w.data_ptr(), out.data_ptr() + 64 * n * esize
+    if res is not None:
+        o.residual, o.residual_stride, a.residual_batch_stride = res.data_ptr() + 64 * n * esize, n, (m + 64) * n
+    o.M, o.N, o.K, o.x_stride, o.w_stride, o.out_stride = m, n, k, k, k, n
+    a.x_batch_stride, a.out_batch_stride, a.batches, a.lead_rows = (m + 64) * k, (m + 64) * n, b, lead
+    stream = torch.cuda.current_stream().cuda_stream
+    if norm:
+        a.rms_eps = 1e-5
+        scratch = torch.empty(b * m, device="cuda")
+        _lib.call("gca_rms_linear_batched", C.byref(a), scratch.data_ptr(), stream)
+    else:
+        _lib.call("gca_linear_batched", C.byref(a), stream)
+    xd = x[:, 64:].double()
+    ref = xd @ w.double().t()
+    if norm:
+        ref = ref * torch.rsqrt(xd.pow(2).mean(-1, keepdim=True) + 1e-5)
+    terms = ref.abs()
+    if residual:
+        ref, terms = ref + r[:, 64:].double(), terms + r[:, 64:].double().abs()
+    assert ((out[:, 64:].double() - ref).abs() <= ref.abs() * (2.0 ** -8 + 2.0 ** -22) + k * 2.0 ** -24 * terms.amax(-1, keepdim=True)).all()
+    untouched = r if residual == "in place" else torch.full_like(r, 7.0)
+    if lead:
+        assert torch.equal(out[:, :64], r[:, :64] if residual else torch.zeros_like(r[:, :64]))
+    else:
+        assert torch.equal(out[:, :64], untouched[:, :64])
+
+
 @pytest.mark.parametrize("n,c,dim", [(1, 1, 256), (3, 5, 512), (5, 61, 768), (2, 300, 1024)])
 def test_projection_append_tile_widths(n, c, dim):
     """K, V and landmark rows of an append at a position behind earlier chunks, against float32, small and large products."""
