@@ -61,13 +61,7 @@ constexpr int PAIR_BYTES = 2 * TILE_BYTES;
 constexpr uint32_t PAIR16 = PAIR_BYTES >> 4, TILE16 = TILE_BYTES >> 4;
 // Worker arrangement: NBUF score buffers, SPLIT worker warpgroups per buffer, each taking
 // 64 / SPLIT of the query columns of every key row of its buffer's iterations.
-#ifndef GCA_KV_NBUF
-#define GCA_KV_NBUF 3
-#endif
-#ifndef GCA_KV_SPLIT
-#define GCA_KV_SPLIT 1
-#endif
-constexpr int NBUF = GCA_KV_NBUF, SPLIT = GCA_KV_SPLIT, NG = NBUF * SPLIT;
+constexpr int NBUF = 3, SPLIT = 1, NG = NBUF * SPLIT;
 constexpr int GRAD_ISSUERS = 2;                          // dV and dK from a warp each
 static_assert(NBUF == 2 || NBUF == 3, "score buffers");
 // One issuing warp per product.  Measured slower: one issuing
@@ -78,7 +72,7 @@ static_assert(NBUF == 2 || NBUF == 3, "score buffers");
 // more resident warps cost more than the freed worker group gains); the two tiles through the groups of the last two iterations, which frees the
 // accumulators in half the time (0.657 against 0.635); probing the next iteration's barriers before the current iteration's MMAs are issued,
 // a gain in the q-major kernel (0.634 against 0.613).
-constexpr int PROD_WARP = 4 * NG, ISSUE_S = PROD_WARP + 1, ISSUE_DP = ISSUE_S + 1, ISSUE_DV = ISSUE_DP + 1;       // dK issuer (GRAD2): ISSUE_DV + 1
+constexpr int PROD_WARP = 4 * NG, ISSUE_S = PROD_WARP + 1, ISSUE_DP = ISSUE_S + 1, ISSUE_DV = ISSUE_DP + 1;       // dK issuer: ISSUE_DV + 1
 constexpr int SCHED_WARP = ISSUE_DV + GRAD_ISSUERS;
 constexpr int NTHREADS = (SCHED_WARP + 1) * 32;
 constexpr int WCOLS = 64 / SPLIT;                        // query columns of a key row that one group handles
@@ -304,7 +298,8 @@ __host__ __device__ constexpr uint32_t packed_col(int kk) {
 }
 
 // SCORES: S^T per iteration (second: dP^T); else dV (second: dK).  All 32 lanes run this
-// code; elect.sync inside the MMA / commit wrappers picks the issuing lane.  The two warps of a kind run the SAME code, told apart by
+// code; elect.sync inside the MMA / commit wrappers picks the issuing lane.  Event trace, by iteration: S^T 1 / 2 / 3 (before the waits, behind them, issued),
+// dP^T 4 (issued), dV 5 / 6 (behind the wait, issued).  The two warps of a kind run the SAME code, told apart by
 // `second`: the roles of this kernel do not fit the instruction cache together, and a copy of this loop for each product cost 8 x 256 chunks, K = 8
 // 626 us instead of 611, 1 x 1,024, K = 16 580 instead of 556, pre-gathered 109 x 8 heads (units of two iterations) 33.8 instead of 28.7.
 template <bool SCORES>
@@ -337,8 +332,10 @@ __device__ void kv_issuer(const BwdKvParams& p, uint8_t* smem, uint64_t* bars, v
       if (SCORES) {
         // the tiles have landed AND the buffer's previous contents (the packed A operands of iteration
         // g - NBUF) have been consumed: both barriers are probed at once (one shared-memory round trip)
+        if (lane == 0 && !second) GCA_TRACE_BUF(p.prof, 1, g);
         ok = mbar_wait_warp2(&bars[QDO_FULL + ring.st], ring.ph, &bars[BUF_FREE + b], bph ^ 1, abort_flag, lane);
         if (!ok) break;
+        if (lane == 0 && !second) GCA_TRACE_BUF(p.prof, 2, g);
         tc_fence_after();
         const uint64_t a = dKV + kb * 2 * PAIR16 + second * PAIR16;       // K pair | V pair
         const uint64_t bq = dQDO + stage + second * PAIR16;               // Q pair | dO pair
@@ -355,9 +352,11 @@ __device__ void kv_issuer(const BwdKvParams& p, uint8_t* smem, uint64_t* bars, v
                              IDESC_64, 1u);
         }
         umma_commit_elect(&bars[SP_FULL + b]);            // the barrier expects both the S^T and the dP^T commit
+        if (lane == 0) GCA_TRACE_BUF(p.prof, second ? 4 : 3, g);
       } else {
         ok = mbar_wait_warp(&bars[PDS_FULL + b], bph, abort_flag, lane);
         if (!ok) break;
+        if (lane == 0 && !second) GCA_TRACE_BUF(p.prof, 5, g);
         tc_fence_after();
         // the workers produced |w| P^T and |w| dS^T: a negative weight negates both A operands
         const uint32_t idesc = IDESC_GRAD | (sw[ring.st] < 0.f ? IDESC_NEG_A : 0u);
@@ -375,6 +374,7 @@ __device__ void kv_issuer(const BwdKvParams& p, uint8_t* smem, uint64_t* bars, v
         umma_commit_elect(&bars[BUF_FREE + b]);
         umma_commit_elect(&bars[QDO_EMPTY + ring.st]);   // Q / dO of this iteration are free once dV, dK are done
         if (i == niter - 1) umma_commit_elect(&bars[ACC_FULL + b]);   // written out by the last iteration's worker groups
+        if (lane == 0 && !second) GCA_TRACE_BUF(p.prof, 6, g);
       }
       ring.next();
       if (++b == NBUF) { b = 0; bph ^= 1; }

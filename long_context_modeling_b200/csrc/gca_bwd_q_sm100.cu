@@ -295,7 +295,8 @@ __device__ void q_producer(const BwdQParams& p, uint8_t* smem, uint64_t* bars, v
 
 // SCORES: S per slot, or dP (dp = 1), the two warps with ONE code between them (a copy each: 507 instead of 500 us at 8 x 256 chunks, K = 8; the roles do not fit the
 // instruction cache together); else dQ += dS K per slot.  All 32 lanes run this
-// code; elect.sync inside the MMA / commit wrappers picks the issuing lane.
+// code; elect.sync inside the MMA / commit wrappers picks the issuing lane.  Event trace, by slot: S 0 / 1 / 2, dP 3 / 4 / 12 (before the waits, behind
+// them, issued), dQ 5 / 6 (behind the waits, issued).
 template <bool SCORES>
 __device__ void q_issuer(uint8_t* smem, uint64_t* bars, volatile int* abort_flag, int lane, uint32_t tmem_base, uint32_t dp, long long* prof) {
   const uint64_t dQDO = umma_desc_sw128(smem_u32(smem + OFF_QDO));
@@ -312,6 +313,7 @@ __device__ void q_issuer(uint8_t* smem, uint64_t* bars, volatile int* abort_flag
     // S, dP: the tile has landed AND the region is free -- S: its group has read P, three slots ago; dP: dQ has consumed the
     // dS in it, four slots ago; dQ: dS is written
     const uint32_t st = !SCORES ? rg.st : dp ? rv.st : rr.st, ph = !SCORES ? rg.ph : dp ? rv.ph : rr.ph;
+    if (SCORES && lane == 0) GCA_TRACE_BUF(prof, dp ? 3 : 0, g);
     if (!mbar_wait_warp2_probed(&bars[FULL + st], ph, pre_a, &bars[dp ? DP_FREE + rg.st : PDS_FULL + rf.st], dp ? rg.ph ^ 1 : rf.ph,
                                 pre_b, abort_flag)) break;
     if (SCORES && g >= NS) rf.next();
@@ -323,6 +325,7 @@ __device__ void q_issuer(uint8_t* smem, uint64_t* bars, volatile int* abort_flag
     if (flags & REC_FIRST) {
       if (!mbar_wait_warp(&bars[SCORES ? QDO_FULL + ub : ACC_EMPTY], SCORES ? uph : ub ^ 1, abort_flag, lane)) break;
     }
+    if (lane == 0) GCA_TRACE_BUF(prof, !SCORES ? 5 : dp ? 4 : 1, g);
     tc_fence_after();
     // The next slot's barriers and flags, between the two heads' MMAs: the probes' round trip runs under the issue.
     auto probe = [&] {
@@ -365,6 +368,7 @@ __device__ void q_issuer(uint8_t* smem, uint64_t* bars, volatile int* abort_flag
       umma_commit_elect(&bars[K_EMPTY + rr.st]);        // the K tiles of this slot are free once dQ is done
       if (flags & REC_LAST) umma_commit_elect(&bars[ACC_FULL]);
     }
+    if (lane == 0) GCA_TRACE_BUF(prof, !SCORES ? 6 : dp ? 12 : 2, g);
     if (flags & REC_LAST) ++un;
     rr.next();
     rv.next();

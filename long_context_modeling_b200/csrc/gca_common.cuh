@@ -153,8 +153,8 @@ inline bool units_by_count(const GcaBwdArgs& a) {
 // Order of the forward's and the q-major pass's units.  The first query chunks of a sequence have few or no chunks behind them to
 // retrieve: taken last, these short units even the CTAs out, where a last, partial wave in ascending order is made of the longest.  That pays
 // where a CTA has few units (3 x 37 chunks, 12 heads, K = 8, 4.4 units a CTA: the forward's kernel 34.9 -> 32.4 us).  Side by
-// side the sequences have to share L2, hence the line at half of its 126 MB for their K and V; above it, sequence by sequence, the last
-// query chunk first: 8 x 256 chunks 1711 -> 1749 us forward + backward, the forward at 1 x 1,024 chunks, K = 16 364 -> 377.
+// side the sequences have to share L2, hence the line at half of its 126 MB for their K and V; above it, sequence by sequence in ascending order: the last
+// query chunk first cost 8 x 256 chunks 1711 -> 1749 us forward + backward, the forward at 1 x 1,024 chunks, K = 16 364 -> 377.
 template <class Args>
 inline bool late_chunks_first(const Args& a) {
   return (long long)a.N * a.C * a.Hkv * a.L * a.D * 2 * 2 <= (64ll << 20);

@@ -307,8 +307,8 @@ lmk_stream_kernel(ScanParams p, FinalParams fin) {
       select_batch(mine[x], kth[x], o, (unsigned)(p.e_base + e_lo + b * BATCH), p.K, lane, note[warp]);
     }
   }
-  if (FUSED) {
-    __shared__ unsigned long long lists[FUSED ? NL : 1][MAXK];
+  if constexpr (FUSED) {
+    __shared__ unsigned long long lists[NL][MAXK];
 #pragma unroll
     for (int x = 0; x < MINE; ++x)
       if (warp + x * STREAM_WARPS < NL) lists[warp + x * STREAM_WARPS][lane] = mine[x];
@@ -321,14 +321,14 @@ lmk_stream_kernel(ScanParams p, FinalParams fin) {
       }
     }
     sm100::cluster_sync();                                     // nobody leaves while its lists may be read
-    return;
-  }
+  } else {
 #pragma unroll
-  for (int x = 0; x < MINE; ++x) {
-    const int l = warp + x * STREAM_WARPS;
-    if (l >= NL || (PER_HEAD && l >= p.H)) continue;
-    const long long row = ((long long)n * p.Cq + t0) * p.H + l;
-    if (lane < p.K) p.part[(row * p.splits + split) * p.K + lane] = mine[x];
+    for (int x = 0; x < MINE; ++x) {
+      const int l = warp + x * STREAM_WARPS;
+      if (l >= NL || (PER_HEAD && l >= p.H)) continue;
+      const long long row = ((long long)n * p.Cq + t0) * p.H + l;
+      if (lane < p.K) p.part[(row * p.splits + split) * p.K + lane] = mine[x];
+    }
   }
 }
 

@@ -64,7 +64,7 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Bounded wait: gives up after `limit` polls or as soon as *abort_flag is set (by another
+// Bounded wait: gives up after the first probe and GCA_WAIT_LIMIT polls, or as soon as *abort_flag is set (by another
 // role that already gave up).  Returns false on give-up; the caller must then unwind.
 // The first probe is the non-blocking test_wait: most waits of the MMA-issuing warps find their
 // barrier already complete, and the potentially-suspending try_wait costs a few hundred cycles
