@@ -45,57 +45,16 @@ struct ScanParams {
   float scale;
 };
 
-// Merge 64 scores (lane i: ids id0 + i and id0 + 32 + i; orderable, 0 = none; all ids above those of the list) into a
-// list of K keys held one per lane, whatever scores are equal; `kth` is the list's K-th key.
-struct TopList { unsigned long long mine, kth; };
-__device__ __noinline__ TopList select_64(unsigned long long mine, unsigned long long kth, unsigned o0, unsigned o1, unsigned id0, int K, int lane) {
-  const unsigned th = (unsigned)(kth >> 32);                 // 0 while the list is not full
-  unsigned b0 = __ballot_sync(0xffffffffu, o0 > th), b1 = __ballot_sync(0xffffffffu, o1 > th);
-  const int found = __popc(b0) + __popc(b1);
-  if (found == 0) return {mine, kth};
-  if (found < K) {                                           // a few: one insertion each, lower ids first
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      unsigned b = h ? b1 : b0;
-      while (b) {
-        const int src = __ffs(b) - 1;
-        b &= b - 1;
-        const unsigned o = __shfl_sync(0xffffffffu, h ? o1 : o0, src);
-        const unsigned long long key = ((unsigned long long)o << 32) | (0xffffffffu - (id0 + 32 * h + src));
-        if (key > kth) {
-          list_insert(mine, key, lane);
-          kth = __shfl_sync(0xffffffffu, mine, K - 1);
-        }
-      }
-    }
-    return {mine, kth};
-  }
-  unsigned long long run = mine, best_mine = 0ull;           // many: the K best of list and batch by K warp-wide maxima
-  for (int k = 0; k < K; ++k) {
-    const unsigned rh = (unsigned)(run >> 32);
-    const unsigned m = __reduce_max_sync(0xffffffffu, max(rh, max(o0, o1)));
-    if (m == 0u) break;
-    const unsigned br = __ballot_sync(0xffffffffu, rh == m);
-    b0 = __ballot_sync(0xffffffffu, o0 == m);
-    b1 = __ballot_sync(0xffffffffu, o1 == m);
-    const int src = __ffs(br ? br : b0 ? b0 : b1) - 1;       // equal scores: the lower id first
-    unsigned long long best = __shfl_sync(0xffffffffu, run, src);
-    if (!br) best = ((unsigned long long)m << 32) | (0xffffffffu - (id0 + src + (b0 ? 0 : 32)));
-    if (lane == src) { if (br) run = 0ull; else if (b0) o0 = 0u; else o1 = 0u; }
-    if (lane == k) best_mine = best;
-  }
-  mine = lane < K ? best_mine : 0ull;
-  return {mine, __shfl_sync(0xffffffffu, mine, K - 1)};
-}
-
 constexpr int BATCH = 128;
-// The same for a batch of 128 (o[i]: id id0 + 32 i + lane).  Fewer than K that beat the list's K-th score are inserted, one after the other; K or more, and
-// the K best come out by K warp-wide maxima of the 32-bit scores: whoever holds the maximum strikes it out and notes its key, which is all that the
-// next round waits for (with the owner found by votes and its key shuffled to its place a round takes more than twice as long).  K rounds from the third
-// of a batch on cost 32 x 7,200 landmarks of 1,024, per head, K = 32 119 us (now 90), 32 x 7,200 of 768 93 (69), 4 x 37,000 57.6 (47.4), K = 16 45.2 (43.3).
-// Equal scores are struck out together: more struck out than rounds, and the batch is done over again the careful way.
+// Merge a batch of 128 scores (o[i]: id id0 + 32 i + lane; orderable, 0 = none; all ids above those of the list) into a list of K keys held one per lane;
+// `kth` is the list's K-th key.  Fewer than K that beat the list's K-th score are inserted, one after the other; K or more, and the K best come out
+// by K warp-wide maxima of the 32-bit scores: whoever holds the maximum strikes it out and notes its key, which is all that the next round waits for (with
+// the owner found by votes and its key shuffled to its place a round takes more than twice as long, with a vote on how many hold it nearly twice).
+// Equal scores are struck out together: more struck out than rounds, and it is done over again with a second maximum a round, which finds the lowest
+// id; at once where scores are rounded to 16 bits (`often_equal`).  K rounds from the third of a batch on cost 32 x 7,200 landmarks of 1,024, per
+// head, K = 32 119 us (now 90), 32 x 7,200 of 768 93 (69), 4 x 37,000 57.6 (47.4), K = 16 45.2 (43.3).
 __device__ __forceinline__ void select_batch(unsigned long long& mine, unsigned long long& kth, const unsigned o[4], unsigned id0, int K, int lane,
-                                             unsigned long long* note) {
+                                             bool often_equal, unsigned long long* note) {
   const unsigned th = (unsigned)(kth >> 32);                 // 0 while the list is not full
   unsigned b[4];
   int found = 0;
@@ -114,9 +73,10 @@ __device__ __forceinline__ void select_batch(unsigned long long& mine, unsigned 
   }
   unsigned r = (unsigned)(mine >> 32), v[4] = {o[0], o[1], o[2], o[3]};
   const unsigned first = 0xffffffffu - (id0 + lane);
-  int k = 0, struck = 0;
-  for (; k < K; ++k) {
-    const unsigned m = __reduce_max_sync(0xffffffffu, max(max(max(r, v[0]), max(v[1], v[2])), v[3]));
+  auto highest = [&] { return __reduce_max_sync(0xffffffffu, max(max(max(r, v[0]), max(v[1], v[2])), v[3])); };
+  int k = 0, struck = often_equal;
+  for (; k < K && !often_equal; ++k) {
+    const unsigned m = highest();
     if (m == 0u) break;
     unsigned low = (unsigned)mine;
     bool hit = r == m;
@@ -126,17 +86,34 @@ __device__ __forceinline__ void select_batch(unsigned long long& mine, unsigned 
       if (v[i] == m) { v[i] = 0u; low = first - 32 * i; hit = true; ++struck; }
     if (hit) note[k] = ((unsigned long long)m << 32) | low;
   }
-  if (__reduce_add_sync(0xffffffffu, struck) == k) {
+  if (__reduce_add_sync(0xffffffffu, struck) != k) {
     __syncwarp();
-    mine = lane < k ? note[lane] : 0ull;
-    __syncwarp();
-    kth = __shfl_sync(0xffffffffu, mine, K - 1);
-    return;
+    r = (unsigned)(mine >> 32);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = o[i];
+#pragma unroll 1
+    for (k = 0; k < K; ++k) {
+      const unsigned m = highest();
+      if (m == 0u) break;
+      unsigned low = 0u;                                     // ~id of this lane's first with that score
+#pragma unroll
+      for (int i = 3; i >= 0; --i)
+        if (v[i] == m) low = first - 32 * i;
+      if (r == m) low = (unsigned)mine;
+      const unsigned lowest = __reduce_max_sync(0xffffffffu, low);
+      if (low != lowest) continue;
+      note[k] = ((unsigned long long)m << 32) | low;
+      if (r == m) r = 0u;
+      else
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (low == first - 32 * i) v[i] = 0u;
+    }
   }
-  TopList t = select_64(mine, kth, o[0], o[1], id0, K, lane);
-  t = select_64(t.mine, t.kth, o[2], o[3], id0 + 64, K, lane);
-  mine = t.mine;
-  kth = t.kth;
+  __syncwarp();
+  mine = lane < k ? note[lane] : 0ull;
+  __syncwarp();
+  kth = __shfl_sync(0xffffffffu, mine, K - 1);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -147,7 +124,7 @@ __device__ __forceinline__ void select_batch(unsigned long long& mine, unsigned 
 // memory; list l (one per head, or the only one) is kept by warp l % 16, which merges
 // the 128 scores into it (select_batch): one list per block instead of one per warp to merge at the end, and
 // no list code in the scoring loop (per head it was 12 lists in every warp, each with a serial insertion: 60 us for
-// 2 x 16,411 landmarks, now 15.5 with its merge; 262,144 landmarks, one list: 66.2 us = 6.1 TB/s with its
+// 2 x 16,411 landmarks, now 14.8 with its merge; 262,144 landmarks, one list: 66.2 us = 6.1 TB/s with its
 // merge).
 constexpr int SPLIT_ROWS = 64, STREAM_WARPS = 16;                // rows that a block takes at least
 template <int NP> constexpr int RING_ROWS = NP > 3 ? 6 : 8;       // 196 KB per SM
@@ -304,7 +281,7 @@ lmk_stream_kernel(ScanParams p, FinalParams fin) {
         if (p.noise && e0 + 32 * i < e_hi) s += p.noise[((long long)n * p.Cq + t0) * p.E + e0 + 32 * i];
         o[i] = e0 + 32 * i < e_hi ? orderable(s) : 0u;
       }
-      select_batch(mine[x], kth[x], o, (unsigned)(p.e_base + e_lo + b * BATCH), p.K, lane, note[warp]);
+      select_batch(mine[x], kth[x], o, (unsigned)(p.e_base + e_lo + b * BATCH), p.K, lane, p.score_round != 0, note[warp]);
     }
   }
   if constexpr (FUSED) {
@@ -492,8 +469,11 @@ lmk_merge_rows_kernel(FinalParams p) {
 
 // Many lists per row (a long cache scanned by every SM), up to 160: one block per row.  All keys come to shared memory, 1,664 of them a trip, then one warp
 // merges the lists, five a lane, by K warp-wide maxima of the heads' 32-bit scores: whose head it is notes the key and moves on.
-// Equal scores move on together: more noted than rounds, and the warp starts again with the lowest id of each maximum (a second maximum a round).
-// 128 threads and 8 bytes a key: up to a width of 768 and K = 10 a block finds its place beside one of the scan (192 KB + 15, 512 threads of up to 112
+// Equal scores move on together: more noted than rounds (looked at after two of them and at the end), and the warp starts again with the lowest id of each
+// maximum, a second maximum a round; at once where scores are rounded to 16 bits, which are often equal.  (A vote in every round: K = 16 4 % more for distinct
+// scores.  Lists an odd number of keys apart, in banks of their own: 3 % more, by the sums for it.)  1 x 5,000 of 768 per head, K = 16: distinct scores 10.0 us,
+// rounded ones 11.6 (15.8 with the general way for equal scores, 10.7 when that had 256 threads), all equal 11.8 (16.3, 9.9).
+// 128 threads and 8 bytes a key: up to a width of 768 and K = 15 a block finds its place beside one of the scan (192 KB + 15, 512 threads of up to 112
 // registers) and is there when the scan ends.  With 256 threads it did not: 1 x 32,768 landmarks per head on all 148 SMs 20.4 us, on 128 of them 16.1.  Wider
 // rows and longer lists leave it no place, and it starts when blocks of the scan have left; several of a launch then share an SM, so they must be
 // short: ranked by counting as below, K = 32 took 30 us of 128 threads (20 of 256).  1 x 7,400 x 768, K = 16 / 32: 10.8 / 31.2 us, now 9.6 / 13.5;
@@ -541,28 +521,37 @@ lmk_warp_merge_kernel(FinalParams p) {
     h[i] = at[i] < (tid + 32 * i + 1) * K ? (unsigned)(all[at[i]] >> 32) : 0u;
   };
   start();
-  int k = 0, noted = 0;
-  for (; k < K; ++k) {
-    const unsigned m = highest();
-    if (m == 0u) break;
+  int k = 0, noted = p.score_round != 0;
+  if (!p.score_round) {
+    auto rounds = [&](int end) {
+      for (; k < end; ++k) {
+        const unsigned m = highest();
+        if (m == 0u) return;
 #pragma unroll
-    for (int i = 0; i < MINE; ++i)
-      if (h[i] == m) { take(i, k); ++noted; }
+        for (int i = 0; i < MINE; ++i)
+          if (h[i] == m) { take(i, k); ++noted; }
+      }
+    };
+    rounds(min(K, 2));
+    if (__reduce_add_sync(0xffffffffu, noted) == k) rounds(K);
   }
   if (__reduce_add_sync(0xffffffffu, noted) != k) {
     __syncwarp();
     start();
+    unsigned low[MINE];                                                  // ~id of each head
+#pragma unroll
+    for (int i = 0; i < MINE; ++i) low[i] = h[i] ? (unsigned)all[at[i]] : 0u;
+#pragma unroll 1
     for (k = 0; k < K; ++k) {
       const unsigned m = highest();
       if (m == 0u) break;
-      unsigned low = 0u;                                                 // ~id
+      unsigned mine = 0u;
+#pragma unroll
+      for (int i = 0; i < MINE; ++i) mine = max(mine, h[i] == m ? low[i] : 0u);
+      if (mine != __reduce_max_sync(0xffffffffu, mine)) continue;
 #pragma unroll
       for (int i = 0; i < MINE; ++i)
-        if (h[i] == m) low = max(low, (unsigned)all[at[i]]);
-      const unsigned first = __reduce_max_sync(0xffffffffu, low);
-#pragma unroll
-      for (int i = 0; i < MINE; ++i)
-        if (h[i] == m && (unsigned)all[at[i]] == first) take(i, k);
+        if (low[i] == mine) { take(i, k); low[i] = h[i] ? (unsigned)all[at[i]] : 0u; }
     }
     if (tid >= k) best[tid] = 0ull;
   }

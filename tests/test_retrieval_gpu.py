@@ -179,6 +179,17 @@ def test_ranges_in_steps_of_the_rows_taken_at_once(lcm, n, e, d, head_dim):
     check(lcm.Retrieval(*(t[:1] for t in got)), oracle_rows(lq[:1].cpu(), lk[:1].cpu(), 16, q_pos0=e, head_dim=head_dim))
 
 
+@pytest.mark.parametrize("splits", [1, 7, 40, 160])
+@pytest.mark.parametrize("head_dim", [0, 64])
+@pytest.mark.parametrize("k", [1, 8, 17, 32])
+def test_scores_rounded_to_16_bits_are_often_equal(lcm, k, head_dim, splits):
+    """Equal scores within a batch, between a batch and the list, and between the lists that are merged: the lowest id each time."""
+    e = 160 * 13 + 5
+    lq, lk = cases.landmark_case(k, 1, 1, e, d=256)
+    res = lcm.lmk_score_topk(lq.cuda(), lk.cuda(), k, q_pos0=e, head_dim=head_dim, splits=splits, score_round="bf16")
+    check(res, oracle_rows(lq, lk, k, q_pos0=e, head_dim=head_dim, score_round="bf16"))
+
+
 def test_noise_selects_but_weights_stay_noise_free(lcm):
     """Training: Gumbel noise perturbs the selection only (DRT.py:616-626)."""
     n, c, d, k = 2, 20, 768, 4
