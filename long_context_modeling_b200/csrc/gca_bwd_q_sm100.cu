@@ -31,11 +31,12 @@
 // others follow the records and have no code that runs once per unit.  No
 // atomics: gradients are bit-reproducible.  Every wait is bounded (GCA_STATUS_TIMEOUT on expiry).
 //
-// What bounds it (event trace at 8 x 256 chunks, 12 heads, K = 8): the S and dP issuers, ~1,220 cycles a slot inside a unit and 1,330 on
-// average, of which the slot's 24 MMAs take 768.  With three groups on three shared S / dP buffers, and every role walking the units
+// What bounds it (event trace at 8 x 256 chunks, 12 heads, K = 8): the S and dP issuers, ~1,280 cycles a slot inside a unit and 1,380 on
+// average -- 660 and 710 of issue, 430 and 380 of waiting for tile and region -- of which the slot's 24 MMAs take 768; and close to that the regions, S 3,280
+// cycles over three, dP 4,210 over four.  With three groups on three shared S / dP buffers, and every role walking the units
 // by itself, it was 1,515: the groups, busy all of their 4,170 cycles a slot, and 870 cycles at each unit's end.  Each change alone gave little
 // (four groups 522 -> 511 us, records with three groups 512 -> 521, separate regions with three groups 521 -> 532), together 523 -> 506,
-// with one code for the S and dP issuers 500; at 1 x 1,024 chunks, K = 16 539 -> 529.
+// with one code for the S and dP issuers 500 to 507; at 1 x 1,024 chunks, K = 16 539 -> 512 to 529.
 #include "gca_common.cuh"
 #include "sm100_ptx.cuh"
 #include "tc_common.cuh"

@@ -26,7 +26,7 @@
 // Infinities, NaN, sums that overflow on the way and tiles of tiny numbers are outside the range of all this: such units are found by their outputs
 // and done over again with multiply-adds (see `outside`), with the results that the CUDA-core kernels have always had.
 // 2 x 64 chunks x 12 heads, top-8: forward 110 us, q-major 154, kv-major 200 (CUDA cores: 355, 481, 588), the whole step with inputs
-// that are not in L2 515 us (1,425).  2-norm against 64 bits, N(0,1): o 2.2e-7 (4.4e-7), dq 2.8e-7 (4.7e-7), dk 3.0e-7 (6.9e-7), dv 2.6e-7
+// that are not in L2 520 us (1,425).  2-norm against 64 bits, N(0,1): o 2.2e-7 (4.4e-7), dq 2.8e-7 (4.7e-7), dk 3.0e-7 (6.9e-7), dv 2.6e-7
 // (6.8e-7), dw 2.6e-7 (3.3e-7); the largest errors over the rms, as means over 63 drawn sizes: o 4.3e-6 (7.5e-6), dq 5.9e-6 (8.9e-6), dk 7.0e-6
 // (2.0e-5), dv 6.7e-6 (1.8e-5), dw 8.6e-7 (1.1e-6), a single size now and then the other way round.  With q x 10 still closer in all five but
 // dv (1.3e-6, 1.2e-6), q x 100: dq 6.7e-5 (7.6e-5), dv 1.3e-5 (6.9e-6): the kv-major pass's scores are not the forward's to the last bit.

@@ -26,7 +26,7 @@
 // All other roles follow the records, slot by slot, and have no code that runs once per unit: that code is never in the instruction
 // cache and costs a warp ~10 cycles an instruction (an event trace of the form with one descriptor per unit: 1,500 cycles between
 // a group's last slot of a unit and its first of the next, of ~10,000 per unit).
-// 12 heads: 8 x 256 chunks, K = 8: 390 -> 357 us (345 with the polling loops out of line), 1 x 1,024, K = 16: 389 -> 364 (353).  Tried on this form and slower: Q in tensor
+// 12 heads: 8 x 256 chunks, K = 8: 390 -> 357 us (345 to 352 with the polling loops out of line), 1 x 1,024, K = 16: 389 -> 364 (353 to 368).  Tried on this form and slower: Q in tensor
 // memory so that both issuers run one code (363), one copy of the output code (357), the next record and the
 // next barriers probed in the middle of a slot (398 us: what counts is how many barrier operations there are, not where their
 // latency falls), probes by one elected lane (+9 %), a fourth softmax group (+28 %, with registers moved to it from the other warps).
